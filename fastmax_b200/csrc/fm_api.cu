@@ -116,9 +116,15 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   // times the share of chunks that build and read states.  The two families then break even near 9 300 keys,
   // as measured (score against moment family for the same number of token-heads, 8192 keys: 20.3 / 22.8 ms;
   // 9216: 22.6 / 23.0; 10000: 60.9 / 54.5).
-  const double rate_score = tc_ok ? 800e12 : 25e12;
-  const double rate_state = p.p == 2 ? (moments_tc_supports(p) ? 930e12 : 20e12) : (first_tc_supports(p) ? 450e12 : 20e12);
-  const double rate_chunk = tc_ok ? 0.58 * rate_score : rate_score;
+  // float32 (fm_dense_split.cu, moment states on the CUDA cores), per token and head and step: the score form takes
+  // 4.2 / 5.8 ps per key at d = 32 / 64, the states and read-outs 4.5 / 10.5 ns at p = 1 (256 heads of 1024 tokens)
+  // and 25 / 190 ns at p = 2, so the moment family starts near 2 400 / 3 900 causal keys at p = 1 and 12 000 /
+  // 65 000 at p = 2.
+  const bool split = dense_split_supports(p);
+  const double rate_score = tc_ok ? 800e12 : (split ? (p.d == 32 ? 108e12 : 156e12) : 25e12);
+  const double rate_first = first_tc_supports(p) ? 450e12 : (split ? (p.d == 32 ? 3.3e12 : 5.5e12) : 20e12);
+  const double rate_state = p.p == 2 ? (moments_tc_supports(p) ? 930e12 : 20e12) : rate_first;
+  const double rate_chunk = tc_ok || split ? 0.58 * rate_score : rate_score;
   // Unmasked with nq != nk: the score form costs nq * nk pairs, the moment form one state per key and one
   // read-out per query row (and the mirror image backward), so per token of the mean length the score form
   // sees nq * nk / mean(nq, nk) keys.  Few query rows against many keys therefore stay on the score family.
@@ -183,6 +189,16 @@ static BwdWs bwd_layout(const fastmax_problem& p) {
   return w;
 }
 // the workspace must serve whichever family AUTO picks
+// Backward workspace of the split-operand float32 kernels: [dots][parts and row dots]
+static size_t split_bwd_off(const fastmax_problem& p) { return bwd_layout(p).delta_off; }
+static size_t split_bwd_bytes(const fastmax_problem& p) { return split_bwd_off(p) + dense_split_bwd_bytes(p); }
+// Whether the float32 score family's call runs on the tensor cores: the operands are read by TMA and in 16-byte
+// pieces, and their parts need room.  A call with less workspace or unaligned tensors runs on the CUDA cores.
+static bool use_split(const fastmax_problem& p, size_t need, const void* workspace, size_t workspace_bytes,
+                      std::initializer_list<const void*> ptrs) {
+  return dense_split_supports(p) && workspace && workspace_bytes >= need && ((uintptr_t)workspace & 255) == 0 &&
+         aligned16(ptrs);
+}
 static size_t fwd_ws_bytes(const fastmax_problem& p) {
   return moments_supports(p) ? moments_fwd_layout(p).bytes : 0;
 }
@@ -214,6 +230,7 @@ int fastmax_b200_device_status(int* status, void* stream) {
   if (!a) a = w;
   if ((rc = moments_tc_status(&b, (cudaStream_t)stream))) return rc;
   if ((rc = first_tc_status(&f, (cudaStream_t)stream))) return rc;
+  if (!f && (rc = split_status(&f, (cudaStream_t)stream))) return rc;
   *status = a ? a : (b ? b : f);
   return FASTMAX_OK;
 }
@@ -225,6 +242,7 @@ int fastmax_b200_device_status_reset(void* stream) {
   if ((rc = tc_wide_status_reset(s))) return rc;
   if ((rc = tc_dkdv128_status_reset(s))) return rc;
   if ((rc = moments_tc_status_reset(s))) return rc;
+  if ((rc = split_status_reset(s))) return rc;
   return first_tc_status_reset(s);
 }
 
@@ -303,14 +321,18 @@ size_t fastmax_b200_forward_workspace_bytes(const fastmax_problem* p) {
   if (validate(p)) return 0;
   int impl;
   if (pick_impl(*p, false, &impl)) return 0;
-  return impl == FASTMAX_IMPL_MOMENTS ? fwd_ws_bytes(*p) : 0;
+  if (impl == FASTMAX_IMPL_MOMENTS) return fwd_ws_bytes(*p);
+  return impl == FASTMAX_IMPL_DENSE_FFMA && dense_split_supports(*p) ? dense_split_fwd_bytes(*p) : 0;
 }
 
 size_t fastmax_b200_backward_workspace_bytes(const fastmax_problem* p) {
   if (validate(p)) return 0;
   int impl;
   if (pick_impl(*p, false, &impl)) return 0;
-  return impl == FASTMAX_IMPL_MOMENTS ? bwd_ws_bytes(*p) : bwd_layout(*p).total;
+  if (impl == FASTMAX_IMPL_MOMENTS) return bwd_ws_bytes(*p);
+  const size_t plain = bwd_layout(*p).total;
+  if (impl != FASTMAX_IMPL_DENSE_FFMA || !dense_split_supports(*p)) return plain;
+  return plain > split_bwd_bytes(*p) ? plain : split_bwd_bytes(*p);
 }
 
 // Whether a problem can take its result and upstream gradient in the (batch, n, heads, d) layout:
@@ -347,7 +369,9 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   c.out_heads = heads_per_batch;
   if (p.normalize && (rc = launch_rowmax(c, q, k, (stat_t*)stats))) return rc;
   if (impl == FASTMAX_IMPL_MOMENTS) {
-    const size_t need = moments_fwd_layout(p).bytes;
+    const MomFwdWs w = moments_fwd_layout(p);
+    const size_t need = w.split;
+    if (use_split(p, w.bytes, workspace, workspace_bytes, {q, k, v, o.out})) c.split_ws = (char*)workspace + w.split;
     if (!workspace || workspace_bytes < need)
       return fail(FASTMAX_E_WORKSPACE, "forward workspace too small: need %zu bytes, got %zu", need,
                   workspace_bytes);
@@ -356,6 +380,8 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   }
   if (impl == FASTMAX_IMPL_DENSE_TC)
     return dense_tc_forward(c, q, k, v, (const stat_t*)stats, o.out, o.den);
+  if (use_split(p, dense_split_fwd_bytes(p), workspace, workspace_bytes, {q, k, v, o.out}))
+    return dense_split_forward(c, q, k, v, (const stat_t*)stats, o, workspace);
   return dense_ffma_forward(c, q, k, v, (const stat_t*)stats, o);
 }
 
@@ -407,18 +433,22 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
     impl = FASTMAX_IMPL_DENSE_FFMA;
   if (heads_per_batch && (rc = bt_layout_ok(p, heads_per_batch, impl))) return rc;
   BwdWs w = bwd_layout(p);
-  const size_t need = impl == FASTMAX_IMPL_MOMENTS ? moments_bwd_layout(p).bytes : w.total;
+  const MomBwdWs mw = impl == FASTMAX_IMPL_MOMENTS ? moments_bwd_layout(p) : MomBwdWs{};
+  const size_t need = impl == FASTMAX_IMPL_MOMENTS ? mw.split : w.total;
   if (need > 0 && (!workspace || workspace_bytes < need))
     return fail(FASTMAX_E_WORKSPACE, "backward workspace too small: need %zu bytes, got %zu", need,
                 workspace_bytes);
   if ((rc = check_device())) return rc;
   Ctx c{p, (cudaStream_t)stream};
   c.out_heads = heads_per_batch;
-  if (impl == FASTMAX_IMPL_MOMENTS)
+  if (impl == FASTMAX_IMPL_MOMENTS) {
+    if (use_split(p, mw.bytes, workspace, workspace_bytes, {q, k, v, out, grad_out, grad_q, grad_k, grad_v}))
+      c.split_ws = (char*)workspace + mw.split;
     return moments_backward(c, q, k, v, out, den, (const stat_t*)stats, grad_out, grad_q, grad_k, grad_v,
                             workspace,
                             (stats && keeps_total(p, impl)) ? (const float*)((const char*)stats + stats_words_bytes(p))
                                                             : nullptr);
+  }
   float* dots = (float*)((char*)workspace + w.dots_off);
   float* delta = (float*)((char*)workspace + w.delta_off);
   if (p.normalize)
@@ -428,6 +458,11 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
     if ((rc = launch_gprep(c, grad_out, out, den, gs, delta))) return rc;
     if ((rc = dense_tc_backward(c, q, k, v, gs, delta, (const stat_t*)stats, dots, grad_q, grad_k,
                                 grad_v)))
+      return rc;
+  } else if (use_split(p, split_bwd_bytes(p), workspace, workspace_bytes,
+                       {q, k, v, out, grad_out, grad_q, grad_k, grad_v})) {
+    if ((rc = dense_split_backward(c, q, k, v, out, den, (const stat_t*)stats, grad_out, dots, grad_q, grad_k, grad_v,
+                                   (char*)workspace + split_bwd_off(p))))
       return rc;
   } else {
     if ((rc = launch_delta(c, grad_out, out, delta))) return rc;

@@ -81,6 +81,9 @@ struct Ctx {
   // without a read-out.  -1: no such chunk.  Honoured by the tensor-core moment kernels.
   int skip_chunk = -1;
   int zero_chunk = -1;
+  // float32 moment family: room for the operand parts of the in-chunk score kernels (dense_split_*_bytes), or
+  // null where the tensors do not allow them
+  void* split_ws = nullptr;
 };
 // Row of head `head`, token `row` in a (heads, n, .) array, or in a (batch, n, out_heads, .) array
 __host__ __device__ __forceinline__ size_t out_row(int head, int row, int n, int out_heads) {
@@ -167,6 +170,19 @@ int dense_ffma_backward(const Ctx& c, const void* q, const void* k, const void* 
                         const float* delta, float* dots, void* grad_q, void* grad_k,
                         void* grad_v, const ChunkAdd& ca = ChunkAdd());
 
+// float32 score form on the tensor cores, operands split into three bf16 parts (fm_dense_split.cu): the default of
+// the float32 score family for head dimensions 32 and 64.
+bool dense_split_supports(const fastmax_problem& p);
+size_t dense_split_fwd_bytes(const fastmax_problem& p);
+size_t dense_split_bwd_bytes(const fastmax_problem& p);
+int dense_split_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats, const FwdOut& o,
+                        void* workspace, const ChunkAdd* ca = nullptr);
+int dense_split_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* out, const float* den,
+                         const stat_t* stats, const void* grad_out, float* dots, void* grad_q, void* grad_k,
+                         void* grad_v, void* workspace, const ChunkAdd* ca = nullptr);
+int split_status(int* out, cudaStream_t stream);
+int split_status_reset(cudaStream_t stream);
+
 // ---- moment-state form (fm_moments_ffma.cu) ---------------------------------------
 struct MomentDims {
   int f;    // state rows that are stored: d*d + d + 1, or d + 1 when p == 1
@@ -216,8 +232,8 @@ int first_tc_readout(const Ctx& c, int type_b, int heads, int n, int chunk, int 
 int first_tc_status(int* out, cudaStream_t stream);
 int first_tc_status_reset(cudaStream_t stream);
 // host orchestration of the moment family (fm_moments.cu)
-struct MomFwdWs { size_t states, total, o_add, den_add, s16, bytes; };
-struct MomBwdWs { size_t dots, delta, dvec, gs, states, total, gq_add, gk_add, gv_add, s16, bytes; };
+struct MomFwdWs { size_t states, total, o_add, den_add, s16, split, bytes; };
+struct MomBwdWs { size_t dots, delta, dvec, gs, states, total, gq_add, gk_add, gv_add, s16, split, bytes; };
 int moments_chunk(const fastmax_problem& p);
 bool moments_supports(const fastmax_problem& p);
 size_t moment_state_bytes(const fastmax_problem& p, int n);

@@ -60,7 +60,8 @@ MomFwdWs moments_fwd_layout(const fastmax_problem& p) {
   w.o_add = w.total + moment_total_bytes(p);
   w.den_add = w.o_add + up256(sizeof(float) * (size_t)p.bh * p.nq * p.d);
   w.s16 = w.den_add + up256(sizeof(float) * (size_t)p.bh * p.nq);
-  w.bytes = w.s16 + state16_bytes(p, p.nk);
+  w.split = w.s16 + state16_bytes(p, p.nk);
+  w.bytes = w.split + (p.mask && dense_split_supports(p) ? dense_split_fwd_bytes(p) : 0);
   return w;
 }
 // Workspace of the one-call backward:
@@ -77,7 +78,8 @@ MomBwdWs moments_bwd_layout(const fastmax_problem& p) {
   w.gk_add = w.gq_add + up256(sizeof(float) * (size_t)p.bh * p.nq * p.d);
   w.gv_add = w.gk_add + up256(sizeof(float) * (size_t)p.bhkv * p.nk * p.d);
   w.s16 = w.gv_add + up256(sizeof(float) * (size_t)p.bhkv * p.nk * p.d);
-  w.bytes = w.s16 + state16_bytes(p, p.nk > p.nq ? p.nk : p.nq);
+  w.split = w.s16 + state16_bytes(p, p.nk > p.nq ? p.nk : p.nq);
+  w.bytes = w.split + (p.mask && dense_split_supports(p) ? dense_split_bwd_bytes(p) : 0);
   return w;
 }
 
@@ -194,6 +196,7 @@ int moments_forward_finish(const Ctx& c, const void* q, const void* k, const voi
   ca.out_add = o_add;
   ca.den_add = den_add;
   if (dense_tc_supports(p) && !o.out_f32) return dense_tc_forward(c, q, k, v, stats, o.out, o.den, &ca);
+  if (c.split_ws) return dense_split_forward(c, q, k, v, stats, o, c.split_ws, &ca);
   return dense_ffma_forward(c, q, k, v, stats, o, ca);
 }
 
@@ -348,6 +351,8 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
     ca.gk_add = gk_add;
     ca.gv_add = gv_add;
     if (tc) rc = dense_tc_backward(c, q, k, v, gs, dvec, stats, dots, grad_q, grad_k, grad_v, &ca);
+    else if (c.split_ws)
+      rc = dense_split_backward(c, q, k, v, out, den, stats, grad_out, dots, grad_q, grad_k, grad_v, c.split_ws, &ca);
     else rc = dense_ffma_backward(c, q, k, v, den, stats, grad_out, delta, dots, grad_q, grad_k, grad_v, ca);
     if (rc) return rc;
   } else {

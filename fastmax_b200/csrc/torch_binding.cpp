@@ -134,8 +134,14 @@ torch::Tensor forward_impl(const torch::Tensor& q, const torch::Tensor& k, const
   auto o = buf.narrow(0, 0, elems).view({q.size(0), q.size(1), q.size(2) + 1});
   void* stats = (char*)buf.data_ptr() + stats_offset;
   auto stream = at::cuda::getCurrentCUDAStream().stream();
+  // the float32 score kernels keep their operand parts in a workspace (the packed layout is always score form)
+  int32_t impl = 0;
+  size_t wsb = 0;
+  if (fastmax_b200_selected_impl(&pr, &impl) == FASTMAX_OK && impl == FASTMAX_IMPL_DENSE_FFMA)
+    wsb = fastmax_b200_forward_workspace_bytes(&pr);
+  auto ws = torch::empty({(int64_t)wsb}, q.options().dtype(torch::kUInt8));
   check_rc(fastmax_b200_forward_packed(&pr, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr<float>(), stats,
-                                       nullptr, 0, stream),
+                                       ws.data_ptr(), wsb, stream),
            "fastmax forwardpass");
   if (dropout > 0.0) {
     TORCH_CHECK(drop_noise.has_value() && drop_noise->defined(), "dropout > 0 needs drop_noise");
