@@ -19,38 +19,46 @@
 // (fastmax_cuda_forward.cu:109, 132-150 with nq = 1).
 //
 // The state is fp32, F = (d^2 +) d + 1 rows of d+1 floats (second-order rows first, the
-// constant row last) after a 4-word header {max |k|^2, token count (int32 bits), 0, 0} per key/value head.
-// A step reads and writes it once: HBM-bound, 2 * 4 * F * (d+1) bytes per key/value head
-// per token, independent of the length.  A thread owns one column c of one block of rows
-// (a CTA's threads cover whole rows, so state accesses are contiguous), keeps the block
-// in registers across the tokens of a call, and adds its share of the read-out to a small
-// fp32 array with one atomicAdd per (query head, column, CTA).  Measured on B200 (1024
-// heads, d = 64, p = 2, bf16 inputs): 0.50 ms per token for the 1.11 GB state, 4.4 TB/s.
+// constant row last) after a 4-word header {max |k|^2, token count (int32 bits), arrival count of a
+// running step (0 between calls), 0} per key/value head.  S2 is symmetric in (a, b), so only its
+// upper triangle of tiles is computed; every result is written to both of its rows.
+//
+// Two kernels:
+//   step_kernel    few tokens (one per decode step): bound by the state's traffic.  The lower
+//                  triangle is written but never read: 4 F (d+1) x (1 + 0.56) bytes at d = 64.
+//                  1024 heads, d = 64, p = 2, bf16: 356 us for 1.73 GB = 4.9 TB/s (487 us when every row
+//                  was read, a fill and a division kernel went with each step); 8 key/value heads of 4
+//                  query heads: 13 us (18).
+//   append_kernel  many tokens (prompt): bound by the FMA pipe; see there.
 #include "fm_common.cuh"
+#include "fm_sm100.cuh"
 
 namespace fm {
 namespace {
 
-constexpr int kBlockA = 4;      // a thread's block of state rows: 4 values of a ...
-constexpr int kBlockB = 16;     // ... times 16 consecutive values of b
-constexpr int kTokBatch = 32;   // tokens staged in shared memory per pass (prompt processing)
+constexpr int kTile = 8;        // step_kernel: a thread's block is half (4 x 8) of an 8 x 8 tile of second-order rows ...
+constexpr int kHalf = 4;
+constexpr int kLinear = kHalf * kTile;   // ... or 32 first-order rows, or the constant row
+constexpr int kTokBatch = 32;   // tokens staged in shared memory per pass
+constexpr int kQueries = 4;     // query heads of a group that are read out together
 constexpr int kHeader = 4;
 
 struct DecArgs {
   int bh, bhkv, ratio, p, normalize;
   float a0, a1, a2, lim;
   long long n_new;       // tokens to add
-  int rows;              // F
   long long head_floats; // kHeader + F * (d + 1)
 };
 
 template <int D> struct DecCfg {
   static constexpr int DV = D + 1;
-  static constexpr int RPB = 256 / DV;          // row blocks per CTA
+  static constexpr int RPB = (D == 128) ? 2 : 256 / DV;           // row blocks per CTA
+  static constexpr int PER_SM = (D == 64) ? 4 : 3;                // CTAs per SM, a compromise with spills
   static constexpr int THREADS = RPB * DV;
-  static constexpr int KS = D + 16;             // (k, 1, 0 x 15): a 16-float window may start at D
-  static constexpr int NB2 = (D / kBlockA) * (D / kBlockB);   // second-order blocks per head
-  static constexpr int NB1 = D / kBlockB;                     // first-order blocks per head
+  static constexpr int NT = D / kTile;
+  static constexpr int NB2 = NT * (NT + 1);                       // second-order half tiles per head
+  static constexpr int NB1 = (D + kLinear - 1) / kLinear;         // first-order blocks per head
+  __host__ __device__ static constexpr int ctas(int p) { return ((p == 2 ? NB2 : 0) + NB1 + 1 + RPB - 1) / RPB; }
 };
 
 // Sum of squares of x[0..D) by one warp; the result is valid in every lane.
@@ -79,23 +87,41 @@ __device__ __forceinline__ void load16_to_f32(const __nv_bfloat16* src, float* d
   }
 }
 
-// Row order of a head's state: the d*d second-order rows (a, b) first (p = 2), then the d
-// first-order rows, then the constant row.  A thread owns one column c of one block of rows:
-// (a0..a0+3) x (b0..b0+15) of the second order, or 16 first-order rows, or the constant row.
-// feature(a, b) = kx[a] * kx[b] with kx = (k, 1, 0, ...): per token the thread forms four
-// products kx[a] * vt[c] and reads 16 values kx[b] (five 16-byte shared-memory loads and one
-// scalar one) for its 64 multiply-adds, so prompt processing is bound by the FMA pipe rather
-// than by shared memory; a decode step just streams the 64 accumulators through once.
+// 16 bytes of T held in registers to shared memory as fp32 values.
+template <typename T>
+__device__ __forceinline__ void store16_as_f32(const uint4& w, float* dst) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<uint4*>(dst) = w;
+  } else {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w.x << 16, w.x & 0xFFFF0000u, w.y << 16, w.y & 0xFFFF0000u);
+    *reinterpret_cast<uint4*>(dst + 4) = make_uint4(w.z << 16, w.z & 0xFFFF0000u, w.w << 16, w.w & 0xFFFF0000u);
+  }
+}
+
+// A tile of the upper triangle, counted row by row: (ta, tb) with ta <= tb < nt.
+__device__ __forceinline__ void upper_tile(int idx, int nt, int& ta, int& tb) {
+  ta = 0;
+  while (idx >= nt - ta) { idx -= nt - ta; ++ta; }
+  tb = ta + idx;
+}
+
+// A thread owns one column c of one block of rows, so a CTA's accesses are runs of whole rows: half of an
+// 8 x 8 tile of the second order on or above the diagonal, 32 first-order rows, or the constant row.  READ: the
+// blocks' shares of the read-out go to scratch[query head][CTA][column]; the CTA of a head that arrives last
+// (a counter in the head's header) adds them in CTA order, divides and writes the output row.
 template <typename T, int D, bool READ>
-__global__ void __launch_bounds__(DecCfg<D>::THREADS) decode_kernel(const DecArgs a, const T* __restrict__ q,
-                                                                    const T* __restrict__ k, const T* __restrict__ v,
-                                                                    float* __restrict__ state, float* __restrict__ num) {
+__global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_kernel(const DecArgs a, const T* __restrict__ q,
+                                                                  const T* __restrict__ k, const T* __restrict__ v,
+                                                                  float* __restrict__ state, float* __restrict__ scratch,
+                                                                  T* __restrict__ out) {
   typedef DecCfg<D> C;
-  __shared__ __align__(16) float ks[kTokBatch][C::KS];
+  __shared__ __align__(16) float ks[kTokBatch][D];
   __shared__ float vs[kTokBatch][D + 1];   // (v, 1)
-  __shared__ float red[C::RPB][C::DV];
-  __shared__ float s_q2;
+  __shared__ float qs[kQueries][D];
+  __shared__ float red[kQueries][C::RPB][C::DV];
+  __shared__ float s_q2[kQueries];
   __shared__ int s_kmax2_bits;   // max |k|^2 as its bit pattern: non-negative floats order like integers
+  __shared__ int s_last;
   const int tid = threadIdx.x, r = tid / C::DV, c = tid - r * C::DV, lane = tid & 31;
   const int head = blockIdx.y;
   float* hs = state + head * a.head_floats;
@@ -103,26 +129,28 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS) decode_kernel(const DecArg
   // this thread's block
   const int nb2 = (a.p == 2) ? C::NB2 : 0, n2rows = (a.p == 2) ? D * D : 0;
   const int sb = blockIdx.x * C::RPB + r;
-  int a0 = D, b0 = D, kind = 0, nu = 0, ni = 0;   // nu x ni valid rows
-  int row00 = 0, ustride = 0;                     // row of (u, i) = row00 + u * ustride + i
+  bool diagonal = false;
+  int a0 = 0, b0 = 0, kind = -1, count = 0;      // kind 2, 1, 0: order of the block; count: its first-order rows
   if (sb < nb2) {
-    a0 = (sb / C::NB1) * kBlockA; b0 = (sb % C::NB1) * kBlockB; kind = 2; nu = kBlockA; ni = kBlockB;
-    row00 = a0 * D + b0; ustride = D;
+    upper_tile(sb >> 1, C::NT, a0, b0);
+    diagonal = a0 == b0;
+    a0 = a0 * kTile + (sb & 1) * kHalf; b0 *= kTile; kind = 2;
   } else if (sb < nb2 + C::NB1) {
-    b0 = (sb - nb2) * kBlockB; kind = 1; nu = 1; ni = kBlockB; row00 = n2rows + b0;
+    a0 = (sb - nb2) * kLinear; kind = 1; count = D - a0 < kLinear ? D - a0 : kLinear;
   } else if (sb == nb2 + C::NB1) {
-    nu = 1; ni = 1; row00 = n2rows + D;           // the constant row: kx[D] * kx[D] = 1
+    kind = 0;
   }
-
-  float* const base = hs + kHeader + (long long)row00 * C::DV + c;   // row (u, i) at base[(u * ustride + i) * DV]
-  const int ustep = ustride * C::DV;
-  float s[kBlockA][kBlockB];
+  // row (u, i) at base[(u * ustride + i * istride)]; a second-order tile's mirror image at base2
+  float* base = hs + kHeader + c + (long long)C::DV * (kind == 2 ? a0 * D + b0 : n2rows + (kind == 1 ? a0 : D));
+  float* base2 = hs + kHeader + c + (long long)C::DV * (b0 * D + a0);
+  const int ustride = (kind == 2 ? D : kTile) * C::DV;
+  float s[kHalf][kTile];
+  // rows of this thread's block that exist: all 32, `count` of them, or one
+  const int live = kind == 2 ? kHalf * kTile : (kind == 1 ? count : (kind == 0 ? 1 : 0));
 #pragma unroll
-  for (int u = 0; u < kBlockA; ++u) {
-    const float* pu = base + u * ustep;
+  for (int u = 0; u < kHalf; ++u)
 #pragma unroll
-    for (int i = 0; i < kBlockB; ++i) s[u][i] = (u < nu && i < ni) ? pu[i * C::DV] : 0.0f;
-  }
+    for (int i = 0; i < kTile; ++i) s[u][i] = (u * kTile + i < live) ? base[u * ustride + i * C::DV] : 0.0f;
   if (tid == 0) s_kmax2_bits = __float_as_int(hs[0]);
   __syncthreads();
 
@@ -130,20 +158,16 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS) decode_kernel(const DecArg
   const T* vh = v + (long long)head * a.n_new * D;
   for (long long t0 = 0; t0 < a.n_new; t0 += kTokBatch) {
     const int nt = (int)((a.n_new - t0 < kTokBatch) ? a.n_new - t0 : kTokBatch);
-    // stage the batch: 16-byte loads of k and v, converted to fp32; then the (1, 0, ...) tails
+    // stage the batch: 16-byte loads of k and v, converted to fp32
     constexpr int EPV = 16 / (int)sizeof(T), VPT = D / EPV;   // elements per load, loads per token
     for (int e = tid; e < nt * VPT; e += C::THREADS) {
       const int tok = e / VPT, x = (e - tok * VPT) * EPV;
       load16_to_f32(kh + (t0 + tok) * D + x, &ks[tok][x]);
       load16_to_f32(vh + (t0 + tok) * D + x, &vs[tok][x]);
-    }
-    for (int e = tid; e < nt * 16; e += C::THREADS) {
-      const int tok = e >> 4, j = e & 15;
-      ks[tok][D + j] = j == 0 ? 1.0f : 0.0f;
-      if (j == 0) vs[tok][D] = 1.0f;
+      if (x == 0) vs[tok][D] = 1.0f;
     }
     __syncthreads();
-    {   // running maximum of |k|^2, the tokens spread over the CTA's full warps
+    if (READ || blockIdx.x == 0) {   // running maximum of |k|^2, the tokens spread over the CTA's full warps
       constexpr int kFullWarps = C::THREADS / 32;
       const int warp = tid >> 5;
       if (warp < kFullWarps) {
@@ -154,76 +178,288 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS) decode_kernel(const DecArg
     }
     for (int tok = 0; tok < nt; ++tok) {
       const float vc = vs[tok][c];
-      const float4 ka = *reinterpret_cast<const float4*>(&ks[tok][a0]);   // (1, 0, 0, 0) when a0 == D
-      const float t[kBlockA] = {ka.x * vc, ka.y * vc, ka.z * vc, ka.w * vc};
-      const float4* kb = reinterpret_cast<const float4*>(&ks[tok][b0]);
+      if (kind == 2) {
+        float kb[kTile];
 #pragma unroll
-      for (int i4 = 0; i4 < kBlockB / 4; ++i4) {
-        const float4 b4 = kb[i4];
+        for (int i = 0; i < kTile; ++i) kb[i] = ks[tok][b0 + i];
 #pragma unroll
-        for (int u = 0; u < kBlockA; ++u) {
-          s[u][4 * i4 + 0] = fmaf(t[u], b4.x, s[u][4 * i4 + 0]);
-          s[u][4 * i4 + 1] = fmaf(t[u], b4.y, s[u][4 * i4 + 1]);
-          s[u][4 * i4 + 2] = fmaf(t[u], b4.z, s[u][4 * i4 + 2]);
-          s[u][4 * i4 + 3] = fmaf(t[u], b4.w, s[u][4 * i4 + 3]);
+        for (int u = 0; u < kHalf; ++u) {
+          const float ka = ks[tok][a0 + u];
+#pragma unroll
+          for (int i = 0; i < kTile; ++i) s[u][i] = fmaf(ka * kb[i], vc, s[u][i]);
         }
+      } else if (kind == 1) {
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+          for (int i = 0; i < kTile; ++i)
+            if (u * kTile + i < count) s[u][i] = fmaf(ks[tok][a0 + u * kTile + i], vc, s[u][i]);
+      } else if (kind == 0) {
+        s[0][0] += vc;
       }
     }
     __syncthreads();
   }
 
 #pragma unroll
-  for (int u = 0; u < kBlockA; ++u) {
-    float* pu = base + u * ustep;
+  for (int u = 0; u < kHalf; ++u)
 #pragma unroll
-    for (int i = 0; i < kBlockB; ++i)
-      if (u < nu && i < ni) pu[i * C::DV] = s[u][i];
+    for (int i = 0; i < kTile; ++i)
+      if (u * kTile + i < live) base[u * ustride + i * C::DV] = s[u][i];
+  if (kind == 2 && !diagonal) {
+#pragma unroll
+    for (int i = 0; i < kTile; ++i)
+#pragma unroll
+      for (int u = 0; u < kHalf; ++u) base2[(i * D + u) * C::DV] = s[u][i];
   }
-  // every CTA of the head holds the same maximum; the first one records it
-  if (blockIdx.x == 0 && tid == 0) {
-    hs[0] = __int_as_float(s_kmax2_bits);
-    // the token count is an integer bit pattern in the float slot: exact past 2^24 tokens
-    hs[1] = __int_as_float(__float_as_int(hs[1]) + (int)a.n_new);
+  if (!READ) {
+    if (blockIdx.x == 0 && tid == 0) {
+      hs[0] = __int_as_float(s_kmax2_bits);
+      // the token count is an integer bit pattern in the float slot: exact past 2^24 tokens
+      hs[1] = __int_as_float(__float_as_int(hs[1]) + (int)a.n_new);
+    }
+    return;
   }
-  if (!READ) return;
 
-  float* qx = &ks[0][0];   // (q, 1, 0 x 15), reusing the key staging
-  for (int g = 0; g < a.ratio; ++g) {
-    const int qh = head * a.ratio + g;
+  // the group's query heads, kQueries at a time
+  for (int g0 = 0; g0 < a.ratio; g0 += kQueries) {
+    const int ng = a.ratio - g0 < kQueries ? a.ratio - g0 : kQueries;
+    const long long qh = (long long)head * a.ratio + g0;
     __syncthreads();
-    for (int x = tid; x < C::KS; x += C::THREADS) qx[x] = x < D ? ldf(q + (long long)qh * D + x) : (x == D ? 1.0f : 0.0f);
+    for (int x = tid; x < ng * D; x += C::THREADS) qs[x / D][x % D] = ldf(q + qh * D + x);
     __syncthreads();
-    if (tid < 32) {
-      const float n2 = warp_norm2<D>(qx, lane);
-      if (lane == 0) s_q2 = n2;
+    if (tid < ng * 32) {
+      const float n2 = warp_norm2<D>(qs[tid >> 5], lane);
+      if (lane == 0) s_q2[tid >> 5] = n2;
     }
     __syncthreads();
-    const float sc = a.normalize ? (a.lim * rsqrtf(s_q2)) * (a.lim * rsqrtf(__int_as_float(s_kmax2_bits))) : 1.0f;
-    const float coef = kind == 0 ? a.a0 : (kind == 1 ? a.a1 * sc : a.a2 * sc * sc);
-    float part = 0.0f;
+    for (int g = 0; g < ng; ++g) {
+      const float* qx = qs[g];
+      const float sc = a.normalize ? (a.lim * rsqrtf(s_q2[g])) * (a.lim * rsqrtf(__int_as_float(s_kmax2_bits))) : 1.0f;
+      float part = 0.0f;
+      if (kind == 2) {
+        // a tile above the diagonal stands for its mirror image too
+        const float coef = a.a2 * sc * sc * (diagonal ? 1.0f : 2.0f);
 #pragma unroll
-    for (int u = 0; u < kBlockA; ++u) {
-      const float cu = coef * qx[a0 + u];
+        for (int u = 0; u < kHalf; ++u) {
+          float row = 0.0f;
 #pragma unroll
-      for (int i = 0; i < kBlockB; ++i) part = fmaf((u < nu && i < ni) ? cu * qx[b0 + i] : 0.0f, s[u][i], part);
+          for (int i = 0; i < kTile; ++i) row = fmaf(qx[b0 + i], s[u][i], row);
+          part = fmaf(coef * qx[a0 + u], row, part);
+        }
+      } else if (kind == 1) {
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+          for (int i = 0; i < kTile; ++i)
+            if (u * kTile + i < count) part = fmaf(a.a1 * sc * qx[a0 + u * kTile + i], s[u][i], part);
+      } else {
+        part = a.a0 * s[0][0];
+      }
+      red[g][r][c] = part;
     }
-    red[r][c] = part;
     __syncthreads();
-    if (r == 0) {
+    for (int x = tid; x < ng * C::DV; x += C::THREADS) {
+      const int g = x / C::DV, cc = x - g * C::DV;
       float tot = 0.0f;
 #pragma unroll
-      for (int rr = 0; rr < C::RPB; ++rr) tot += red[rr][c];
-      atomicAdd(num + (long long)qh * C::DV + c, tot);
+      for (int rr = 0; rr < C::RPB; ++rr) tot += red[g][rr][cc];
+      __stcg(scratch + ((qh + g) * gridDim.x + blockIdx.x) * C::DV + cc, tot);
     }
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    const int before = atomicAdd(reinterpret_cast<int*>(hs + 2), 1);
+    s_last = before == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) {
+    hs[0] = __int_as_float(s_kmax2_bits);
+    hs[1] = __int_as_float(__float_as_int(hs[1]) + (int)a.n_new);
+    hs[2] = 0.0f;
+  }
+  for (int g0 = 0; g0 < a.ratio; g0 += kQueries) {
+    const int ng = a.ratio - g0 < kQueries ? a.ratio - g0 : kQueries;
+    const long long qh = (long long)head * a.ratio + g0;
+    for (int g = 0; g < ng; ++g) {
+      float tot = 0.0f;
+      const float* src = scratch + (qh + g) * gridDim.x * C::DV + c;
+#pragma unroll 8
+      for (int b = r; b < (int)gridDim.x; b += C::RPB) tot += __ldcg(src + (long long)b * C::DV);
+      red[g][r][c] = tot;
+    }
+    __syncthreads();
+    for (int x = tid; x < ng * D; x += C::THREADS) {
+      const int g = x / D, cc = x - g * D;
+      float num = 0.0f, den = 0.0f;
+#pragma unroll
+      for (int rr = 0; rr < C::RPB; ++rr) { num += red[g][rr][cc]; den += red[g][rr][D]; }
+      stf(out + qh * D + x, num / den);
+    }
+    __syncthreads();
   }
 }
 
+// Prompt processing: S += sum over tokens of kx[a] kx[b] (v, 1)[c], kx = (k, 1, 0, 0, 0).
+// A thread owns 4 x 4 pairs (a, b) of the upper triangle (of kx, so the first-order rows and the constant row
+// are its last column of tiles) times 8 value columns, as 64 packed accumulators, and a share of the tile's
+// normaliser column.  Per token it reads 4 + 4 + 8 floats of shared memory for 128 multiply-adds; with fewer
+// pairs or columns per thread the loads would take the time (an LDS.128 moves 512 bytes per warp, four cycles
+// of the SM's 128-byte port, against 32 for the multiply-adds).  The next batch's tokens are fetched into
+// registers while the current one is processed.  64 heads x 4000 tokens, d = 64, bf16: 2.22 ms = 16 TFMA/s (5.59 ms
+// when all ordered pairs were summed, 64 multiply-adds for 5 loads); the grid's last wave is nearly empty there.
+template <int D> struct AppCfg {
+  static constexpr int NT = D / 4 + 1;                       // tile rows of kx
+  static constexpr int CG = D / 8;                           // column groups
+  static constexpr int PE = 16 / CG;                         // pairs per thread of the normaliser column
+  static constexpr int BPC = 128 / CG;                       // tiles per CTA
+  static constexpr int THREADS = BPC * CG;
+  __host__ __device__ static constexpr int tiles(int p) { return p == 2 ? NT * (NT + 1) / 2 : NT; }
+  __host__ __device__ static constexpr int ctas(int p) { return (tiles(p) + BPC - 1) / BPC; }
+};
+
 template <typename T, int D>
-__global__ void decode_finish_kernel(const float* __restrict__ num, T* __restrict__ out, int bh) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= bh * D) return;
-  const int h = idx / D, c = idx - h * D;
-  stf(out + idx, num[(long long)h * (D + 1) + c] / num[(long long)h * (D + 1) + D]);
+__global__ void __launch_bounds__(AppCfg<D>::THREADS, 2) append_kernel(const DecArgs a, const T* __restrict__ k,
+                                                                       const T* __restrict__ v,
+                                                                       float* __restrict__ state) {
+  using namespace sm100;
+  typedef AppCfg<D> C;
+  constexpr int DV = D + 1, KS = D + 4;
+  constexpr int TB = 64 / (int)sizeof(T) * (D >= 128 ? 1 : 2) / 2;      // tokens per batch: 32 / 16 (D = 128: half)
+  constexpr int EPV = 16 / (int)sizeof(T), VPT = D / EPV;
+  constexpr int NLD = (TB * VPT + C::THREADS - 1) / C::THREADS;         // 16-byte loads per thread, k and v each
+  __shared__ __align__(16) float ks[TB][KS];
+  __shared__ __align__(16) float vs[TB][D];
+  __shared__ int s_kmax2_bits;
+  const int tid = threadIdx.x, cg = tid % C::CG, head = blockIdx.y, lane = tid & 31;
+  const int tile = blockIdx.x * C::BPC + tid / C::CG;
+  const bool on = tile < C::tiles(a.p);
+  int ta = 0, tb = C::NT - 1;
+  if (a.p == 2) upper_tile(on ? tile : 0, C::NT, ta, tb);
+  else ta = on ? tile : 0;
+  const int a0 = ta * 4, b0 = tb * 4, c0 = cg * 8;
+  const int ea = a0 + cg * C::PE / 4, eb = b0 + cg * C::PE % 4;         // this thread's first normaliser pair
+  float* hs = state + head * a.head_floats;
+  if (tid == 0) s_kmax2_bits = __float_as_int(hs[0]);
+
+  uint64_t acc[4][2][8];            // [a][b pair][column]
+  float acce[C::PE];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[u][i][c] = 0ull;
+#pragma unroll
+  for (int e = 0; e < C::PE; ++e) acce[e] = 0.f;
+  for (int e = tid; e < TB * 4; e += C::THREADS) ks[e >> 2][D + (e & 3)] = (e & 3) == 0 ? 1.0f : 0.0f;
+
+  const T* kh = k + (long long)head * a.n_new * D;
+  const T* vh = v + (long long)head * a.n_new * D;
+  uint4 kr[NLD], vr[NLD];
+  auto fetch = [&](long long t0) {   // tokens past the end read as zero: they add nothing
+#pragma unroll
+    for (int i = 0; i < NLD; ++i) {
+      const int e = tid + i * C::THREADS;
+      const bool ok = e < TB * VPT && t0 + e / VPT < a.n_new;
+      const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+      kr[i] = ok ? __ldg(reinterpret_cast<const uint4*>(kh + t0 * D) + e) : zero;
+      vr[i] = ok ? __ldg(reinterpret_cast<const uint4*>(vh + t0 * D) + e) : zero;
+    }
+  };
+  fetch(0);
+  for (long long t0 = 0; t0 < a.n_new; t0 += TB) {
+    const int nt = (int)((a.n_new - t0 < TB) ? a.n_new - t0 : TB);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NLD; ++i) {
+      const int e = tid + i * C::THREADS;
+      if (e < TB * VPT) {
+        store16_as_f32<T>(kr[i], &ks[e / VPT][(e % VPT) * EPV]);
+        store16_as_f32<T>(vr[i], &vs[e / VPT][(e % VPT) * EPV]);
+      }
+    }
+    __syncthreads();
+    if (t0 + TB < a.n_new) fetch(t0 + TB);
+    if (blockIdx.x == 0) {
+      const int warp = tid >> 5;
+      if (warp < C::THREADS / 32) {
+        float m = 0.0f;
+        for (int tok = warp; tok < nt; tok += C::THREADS / 32) m = fmaxf(m, warp_norm2<D>(ks[tok], lane));
+        if (lane == 0) atomicMax(&s_kmax2_bits, __float_as_int(m));
+      }
+    }
+    if (!on) continue;
+#pragma unroll 2
+    for (int tok = 0; tok < nt; ++tok) {
+      const float4 ka = *reinterpret_cast<const float4*>(&ks[tok][a0]);
+      const ulonglong2 kb = *reinterpret_cast<const ulonglong2*>(&ks[tok][b0]);
+      const float4 v0 = *reinterpret_cast<const float4*>(&vs[tok][c0]), v1 = *reinterpret_cast<const float4*>(&vs[tok][c0 + 4]);
+      const float kau[4] = {ka.x, ka.y, ka.z, ka.w}, vc[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+      uint64_t vv[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) vv[c] = pack2(vc[c], vc[c]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint64_t kk = pack2(kau[u], kau[u]);
+        const uint64_t t0p = mul2(kk, kb.x), t1p = mul2(kk, kb.y);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          acc[u][0][c] = fma2(t0p, vv[c], acc[u][0][c]);
+          acc[u][1][c] = fma2(t1p, vv[c], acc[u][1][c]);
+        }
+      }
+      const float ke = ks[tok][ea];
+#pragma unroll
+      for (int e = 0; e < C::PE; ++e) acce[e] = fmaf(ke, ks[tok][eb + e], acce[e]);
+    }
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && tid == 0) {
+    hs[0] = __int_as_float(s_kmax2_bits);
+    hs[1] = __int_as_float(__float_as_int(hs[1]) + (int)a.n_new);
+  }
+  if (!on) return;
+  const int n2rows = (a.p == 2) ? D * D : 0;
+  float* st = hs + kHeader;
+  // the row of pair (a, b) and, off the diagonal of tiles, its mirror image; -1: a padding row of kx
+  auto row_of = [&](int x, int y) -> int {
+    if (y < D) return x * D + y;
+    return (y == D && x <= D) ? n2rows + x : -1;
+  };
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int x = a0 + u, y = b0 + i, row = row_of(x, y);
+      if (row < 0 || (x == D && y < D)) continue;
+      float f[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        float lo, hi;
+        unpack2(acc[u][i >> 1][c], lo, hi);
+        f[c] = (i & 1) ? hi : lo;
+      }
+      float* r1 = st + (long long)row * DV + c0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) { f[c] += r1[c]; r1[c] = f[c]; }
+      if (y < D && ta != tb) {
+        float* r2 = st + (long long)(y * D + x) * DV + c0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) r2[c] = f[c];
+      }
+    }
+#pragma unroll
+  for (int e = 0; e < C::PE; ++e) {
+    const int x = ea, y = eb + e, row = row_of(x, y);
+    if (row < 0 || (x == D && y < D)) continue;
+    const float f = acce[e] + st[(long long)row * DV + D];
+    st[(long long)row * DV + D] = f;
+    if (y < D && ta != tb) st[(long long)(y * D + x) * DV + D] = f;
+  }
 }
 
 int rows_of(const fastmax_problem& p) { return 1 + p.d + (p.p == 2 ? p.d * p.d : 0); }
@@ -236,32 +472,40 @@ int check_decode(const fastmax_problem* prob) {
   return FASTMAX_OK;
 }
 
+// CTAs per head of step_kernel: each leaves one partial row per query head in the scratch.
+int step_ctas(const fastmax_problem& p) {
+  if (p.d == 32) return DecCfg<32>::ctas(p.p);
+  if (p.d == 64) return DecCfg<64>::ctas(p.p);
+  return DecCfg<128>::ctas(p.p);
+}
+
+// Below this many tokens the state's traffic decides and step_kernel, whose accesses are whole rows, is faster.
+constexpr long long kAppendMin = 64;
+
 template <typename T, int D, bool READ>
 int launch_decode(const fastmax_problem& p, const void* q, const void* k, const void* v, long long n_new,
-                  float* state, float* num, void* out, cudaStream_t st) {
-  typedef DecCfg<D> C;
-  DecArgs a{p.bh, p.bhkv, p.bhkv ? p.bh / p.bhkv : 1, p.p, p.normalize, p.a0, p.a1, p.a2, p.lim, n_new, rows_of(p),
+                  float* state, float* scratch, void* out, cudaStream_t st) {
+  DecArgs a{p.bh, p.bhkv, p.bhkv ? p.bh / p.bhkv : 1, p.p, p.normalize, p.a0, p.a1, p.a2, p.lim, n_new,
             kHeader + (long long)rows_of(p) * (D + 1)};
   if (p.bhkv == 0) return FASTMAX_OK;
-  if (READ) FM_CUDA_TRY(cudaMemsetAsync(num, 0, sizeof(float) * (size_t)p.bh * (D + 1), st));
-  const int blocks_per_head = (p.p == 2 ? C::NB2 : 0) + C::NB1 + 1;
-  dim3 grid((blocks_per_head + C::RPB - 1) / C::RPB, p.bhkv);
-  FM_LAUNCH(READ ? "fm_decode_step" : "fm_decode_append", st,
-            (decode_kernel<T, D, READ><<<grid, C::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state, num)));
-  FM_CUDA_TRY(cudaGetLastError());
-  if (READ) {
-    const int total = p.bh * D;
-    FM_LAUNCH("fm_decode_finish", st,
-              (decode_finish_kernel<T, D><<<(total + 255) / 256, 256, 0, st>>>(num, (T*)out, p.bh)));
-    FM_CUDA_TRY(cudaGetLastError());
+  if (!READ && n_new >= kAppendMin) {
+    dim3 grid(AppCfg<D>::ctas(p.p), p.bhkv);
+    FM_LAUNCH("fm_decode_append", st,
+              (append_kernel<T, D><<<grid, AppCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));
+  } else {
+    dim3 grid(DecCfg<D>::ctas(p.p), p.bhkv);
+    FM_LAUNCH(READ ? "fm_decode_step" : "fm_decode_append", st,
+              (step_kernel<T, D, READ><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
+                                                                            scratch, (T*)out)));
   }
+  FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
 
 template <bool READ>
 int dispatch_decode(const fastmax_problem& p, const void* q, const void* k, const void* v, long long n_new,
-                    float* state, float* num, void* out, cudaStream_t st) {
-#define FM_DEC(TT, DD) return launch_decode<TT, DD, READ>(p, q, k, v, n_new, state, num, out, st)
+                    float* state, float* scratch, void* out, cudaStream_t st) {
+#define FM_DEC(TT, DD) return launch_decode<TT, DD, READ>(p, q, k, v, n_new, state, scratch, out, st)
   if (p.dtype == FASTMAX_F32) {
     if (p.d == 32) FM_DEC(float, 32);
     if (p.d == 64) FM_DEC(float, 64);
@@ -285,7 +529,7 @@ size_t fastmax_b200_decode_state_bytes(const fastmax_problem* prob) {
 
 size_t fastmax_b200_decode_scratch_bytes(const fastmax_problem* prob) {
   if (!prob || prob->bh < 0 || prob->d <= 0) return 0;
-  return sizeof(float) * (size_t)prob->bh * (prob->d + 1);
+  return sizeof(float) * (size_t)prob->bh * step_ctas(*prob) * (prob->d + 1);
 }
 
 int fastmax_b200_decode_append(const fastmax_problem* prob, const void* k, const void* v, long long n_new,
