@@ -29,7 +29,8 @@
 //                  1024 heads, d = 64, p = 2, bf16: 356 us for 1.73 GB = 4.9 TB/s (487 us when every row
 //                  was read, a fill and a division kernel went with each step); 8 key/value heads of 4
 //                  query heads: 13 us (18).
-//   append_kernel  many tokens (prompt): bound by the FMA pipe; see there.
+//   append_kernel  many tokens (prompt), float32 or d = 32: bound by the FMA pipe; see there.  bf16 prompts of
+//                  d 64 and 128 go to the tensor cores (fm_decode_tc.cu).
 #include "fm_common.cuh"
 #include "fm_sm100.cuh"
 
@@ -479,7 +480,8 @@ int step_ctas(const fastmax_problem& p) {
   return DecCfg<128>::ctas(p.p);
 }
 
-// Below this many tokens the state's traffic decides and step_kernel, whose accesses are whole rows, is faster.
+// Below this many tokens the state's traffic decides and step_kernel is as fast (64 heads, d = 64: 68 us at 40 tokens;
+// 70 us on the tensor cores and 71 us in append_kernel at 64).
 constexpr long long kAppendMin = 64;
 
 template <typename T, int D, bool READ>
@@ -488,6 +490,7 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
   DecArgs a{p.bh, p.bhkv, p.bhkv ? p.bh / p.bhkv : 1, p.p, p.normalize, p.a0, p.a1, p.a2, p.lim, n_new,
             kHeader + (long long)rows_of(p) * (D + 1)};
   if (p.bhkv == 0) return FASTMAX_OK;
+  if (!READ && n_new >= kAppendMin && decode_append_tc_supports(p)) return decode_append_tc(p, k, v, n_new, state, st);
   if (!READ && n_new >= kAppendMin) {
     dim3 grid(AppCfg<D>::ctas(p.p), p.bhkv);
     FM_LAUNCH("fm_decode_append", st,
