@@ -140,6 +140,15 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
                            void* grad_k, void* grad_v, const ChunkAdd* ca = nullptr);
 int dense_tc_wide_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                           void* out, float* den, const ChunkAdd* ca = nullptr);
+// The same sums for rows that see few columns, two row tiles per SM (fm_dense_tc_short.cu).
+int dense_tc_short_dq(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
+                      const stat_t* stats, float* dots, void* grad_q, const ChunkAdd* ca);
+int dense_tc_short_dkdv(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
+                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd* ca);
+int dense_tc_short_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
+                           void* out, float* den, const ChunkAdd* ca = nullptr);
+int tc_short_status(int* out, cudaStream_t stream);
+int tc_short_status_reset(cudaStream_t stream);
 int tc_wide_status(int* out, cudaStream_t stream);
 int tc_wide_status_reset(cudaStream_t stream);
 // backward for d == 128: grad_q, and grad_k / grad_v in one kernel (fm_dense_tc_dkdv128.cu)

@@ -618,6 +618,22 @@ bool dense_tc_wide_supports(const fastmax_problem& p) {
   return !off && p.dtype == FASTMAX_BF16 && p.d == 64 && p.bhkv > 0 && p.bh % p.bhkv == 0;
 }
 
+// Whether the short-row kernels (two row tiles per SM) serve a pass better than these, which overlap more inside one
+// row tile but leave its ends uncovered.  Both measured for 256 heads, us, short / wide: forward 102.9 / 120.8 at 1200
+// causal columns, 211 / 224 at 2048, 668 / 619 at 4096, unmasked 217 / 223 at 1600, 320 / 301 at 2048; grad_q 254 / 291
+// at 2048 causal, 392 / 406 at 2048 unmasked, 826 / 820 at 4096; grad_k + grad_v 179 / 187 at 1200 causal, 271 / 267 at
+// 1600, 264 / 277 at 1200 unmasked, 435 / 410 at 1600 -- but 845 / 921 in the moment family's chunks of 2048, whose
+// epilogues read fp32 rows too.  So the line is drawn at the mean number of columns a row tile walks.  With no more
+// row tiles than SMs there is nothing to overlap and the wide kernels' larger tiles win (8 heads of 1024: 16.3 / 12.4).
+static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
+  const bool chunked = ca && ca->chunk > 0;
+  const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
+  if ((long long)(pass == 2 ? p.bhkv : p.bh) * ((rows + BM - 1) / BM) <= 148) return false;
+  const int seen = chunked ? ca->chunk / 2 : (p.mask ? cols / 2 : cols);
+  const int most[3] = {1500, 1900, chunked ? 1100 : (p.mask ? 700 : 1300)};
+  return seen * (pass == 2 ? p.bh / p.bhkv : 1) <= most[pass];
+}
+
 int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* gs,
                            const float* dvec, const stat_t* stats, float* dots, void* grad_q,
                            void* grad_k, void* grad_v, const ChunkAdd* ca) {
@@ -638,7 +654,10 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
   a.o = grad_q;
   a.dots = p.normalize ? dots : nullptr;
   a.o_add = ca ? ca->gq_add : nullptr;
-  if ((rc = launch_wide<MODE_DQ>(c, "fm_dense_tc_dq", q, gs, k, v, p.nq, p.nk, a))) return rc;
+  if (short_rows(p, ca, 1)) rc = dense_tc_short_dq(c, q, k, v, gs, dvec, stats, dots, grad_q, ca);
+  else rc = launch_wide<MODE_DQ>(c, "fm_dense_tc_dq", q, gs, k, v, p.nq, p.nk, a);
+  if (rc) return rc;
+  if (short_rows(p, ca, 2)) return dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, ca);
   // grad_k and grad_v: rows = keys, columns = queries
   a.o = grad_k;
   a.o2 = grad_v;
@@ -651,6 +670,7 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
 int dense_tc_wide_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                           void* out, float* den, const ChunkAdd* ca) {
   const fastmax_problem& p = c.p;
+  if (short_rows(p, ca, 0)) return dense_tc_short_forward(c, q, k, v, stats, out, den, ca);
   WArgs a = {};
   a.stat_q = p.normalize ? stats : nullptr;
   a.stat_k = p.normalize ? stats + p.bh : nullptr;
