@@ -109,6 +109,20 @@ static int check_device() {
 // number of keys a row sees, the moment form is constant plus its own chunk in score form.
 static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   if (!moments_supports(p)) return false;
+  if (p.p == 1 && p.mask && (p.d == 64 || (tc_ok && p.d == 128) || (!tc_ok && p.d == 32 && p.dtype == FASTMAX_F32))) {
+    // First order, causal.  The score form's time per token and head grows by `slope` ns per token of length (a line
+    // through its measured times), the moment form's is flat; they meet at `meet` tokens.  The moment form's extra
+    // launches cost some 30 us of host time, so what it saves has to exceed that.  Measured per step, score / moment:
+    //   bf16 d = 64   256 heads: 0.255 / 0.293 ms at 768, 0.360 / 0.369 at 1024, 0.483 / 0.446 at 1280, 2.80 / 1.30 at 4096
+    //                 64 heads: 0.137 / 0.159 at 1024, 0.298 / 0.235 at 2048; 8 heads: 0.098 / 0.126 at 2048, 0.163 / 0.127 at 4096
+    //   bf16 d = 128  256 heads: 1.55 / 1.88 at 2048, 2.20 / 2.37 at 2560, 2.94 / 2.81 at 3072, 5.1 / 3.65 at 4096
+    //   float32 d = 32   64 heads: 0.60 / 0.80 at 2048, 1.12 / 1.11 at 3072, 1.80 / 1.52 at 4096
+    //   float32 d = 64   32 heads: 1.10 / 1.31 at 3072, 1.75 / 1.67 at 4096, 3.59 / 2.67 at 6144
+    const bool bf16 = p.dtype == FASTMAX_BF16;
+    const double slope = bf16 ? (p.d == 64 ? 0.42e-3 : 0.82e-3) : (p.d == 64 ? 2.44e-3 : 1.11e-3);
+    const double meet = bf16 ? (p.d == 64 ? 1000 : 2750) : (p.d == 64 ? 3950 : 3100);
+    return p.nk > moments_chunk(p) && (double)p.bh * p.nk * slope * ((double)p.nk - meet) > 30e3;
+  }
   const double d = p.d, F = d + (p.p == 2 ? d * d : 0.0);
   // Constants fitted to this library's kernels on a B200 (bf16, d = 64, p = 2, causal): the score family takes
   // 5.6 ns per token and head at 10^4 keys; the moment family 4.1 ns for its states and read-outs plus 2.0 ns
@@ -172,6 +186,13 @@ static bool aligned16(std::initializer_list<const void*> ptrs) {
   for (const void* q : ptrs)
     if (((uintptr_t)q & 15) != 0) return false;
   return true;
+}
+
+// First-order causal problems go to the moment family at almost any length; unlike the second-order ones, which
+// get there only where nothing else is fast enough, their calls with unaligned tensors are served too.
+static bool first_order_unaligned(const fastmax_problem& p, int impl, std::initializer_list<const void*> ptrs) {
+  return p.impl == FASTMAX_IMPL_AUTO && impl == FASTMAX_IMPL_MOMENTS && p.p == 1 && p.mask && dense_tc_supports(p) &&
+         !aligned16(ptrs);
 }
 
 // Backward workspace: [dots: bh+bhkv floats][delta or dvec: bh*nq floats]
@@ -368,10 +389,22 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   if ((rc = pick_impl(p, o.out_f32 != 0, &impl))) return rc;
   if (p.impl == FASTMAX_IMPL_AUTO && impl == FASTMAX_IMPL_DENSE_TC && !aligned16({q, k, v, o.out}))
     impl = FASTMAX_IMPL_DENSE_FFMA;
-  if (heads_per_batch && (rc = bt_layout_ok(p, heads_per_batch, impl))) return rc;
+  const bool first_unaligned = first_order_unaligned(p, impl, {q, k, v, o.out});
+  if (heads_per_batch && (rc = bt_layout_ok(p, heads_per_batch, first_unaligned ? FASTMAX_IMPL_DENSE_FFMA : impl)))
+    return rc;
   Ctx c{p, (cudaStream_t)stream};
   c.out_heads = heads_per_batch;
   if (p.normalize && (rc = launch_rowmax(c, q, k, (stat_t*)stats))) return rc;
+  if (first_unaligned) {
+    // a backward call whose tensors are aligned (copies of these) still finds the states it expects
+    if (stats && keeps_total(p, impl)) {
+      float* keep = (float*)((char*)stats + stats_words_bytes(p));
+      const int L = moments_chunk(p);
+      if ((rc = moments_chunk_state(c, p.bh, p.nk, L, k, v, nullptr, nullptr, 0, keep))) return rc;
+      if ((rc = moments_prefix(c, p.bh, (p.nk + L - 1) / L, keep, nullptr, nullptr, 0, 1))) return rc;
+    }
+    return dense_ffma_forward(c, q, k, v, (const stat_t*)stats, o);
+  }
   if (impl == FASTMAX_IMPL_MOMENTS) {
     const MomFwdWs w = moments_fwd_layout(p);
     const size_t need = w.split;
@@ -435,6 +468,7 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
   if (p.impl == FASTMAX_IMPL_AUTO && impl == FASTMAX_IMPL_DENSE_TC &&
       !aligned16({q, k, v, out, grad_out, grad_q, grad_k, grad_v}))
     impl = FASTMAX_IMPL_DENSE_FFMA;
+  if (first_order_unaligned(p, impl, {q, k, v, out, grad_out, grad_q, grad_k, grad_v})) impl = FASTMAX_IMPL_DENSE_FFMA;
   if (heads_per_batch && (rc = bt_layout_ok(p, heads_per_batch, impl))) return rc;
   BwdWs w = bwd_layout(p);
   const MomBwdWs mw = impl == FASTMAX_IMPL_MOMENTS ? moments_bwd_layout(p) : MomBwdWs{};

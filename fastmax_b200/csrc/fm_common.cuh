@@ -140,13 +140,22 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
                            void* grad_k, void* grad_v, const ChunkAdd* ca = nullptr);
 int dense_tc_wide_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                           void* out, float* den, const ChunkAdd* ca = nullptr);
+// First-order running sums that the short-row kernels read themselves (causal, p = 1): fp32 states of every (head,
+// chunk), their bf16 copies scaled by the first-order coefficient (first_tc_convert), and the chunk without any.
+struct FirstState {
+  const float* states;
+  const void* s1b;
+  int zero_chunk;
+};
 // The same sums for rows that see few columns, two row tiles per SM (fm_dense_tc_short.cu).
 int dense_tc_short_dq(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
-                      const stat_t* stats, float* dots, void* grad_q, const ChunkAdd* ca);
+                      const stat_t* stats, float* dots, void* grad_q, const ChunkAdd* ca,
+                      const FirstState* fs = nullptr);
 int dense_tc_short_dkdv(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
-                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd* ca);
+                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd* ca,
+                        const FirstState* fs = nullptr);
 int dense_tc_short_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
-                           void* out, float* den, const ChunkAdd* ca = nullptr);
+                           void* out, float* den, const ChunkAdd* ca = nullptr, const FirstState* fs = nullptr);
 int tc_short_status(int* out, cudaStream_t stream);
 int tc_short_status_reset(cudaStream_t stream);
 int tc_wide_status(int* out, cudaStream_t stream);
@@ -240,7 +249,8 @@ bool first_tc_supports(const fastmax_problem& p);
 size_t first_tc_copy_bytes(const fastmax_problem& p, int mats);
 int first_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void* y, const void* z,
                          const float* dvec, float* state);
-int first_tc_convert(const Ctx& c, int mats, const float* state, void* s1b);
+int first_tc_convert(const Ctx& c, int mats, const float* state, void* s1b, int nchunk = 0,
+                     const stat_t* stats = nullptr);   // nchunk > 0: scaled by a1 and the head's statistics
 int first_tc_readout(const Ctx& c, int type_b, int heads, int n, int chunk, int per_chunk, const void* tile,
                      const void* x, const float* uvec, const float* state, const void* s1b,
                      const stat_t* stats, float* o_add, float* den_add, int accumulate, int final = 0,

@@ -13,6 +13,12 @@
 //                DKDV S 64 | W 64 | grad_k 64 | grad_v 64, with E over S and P over W: the 16 columns a warp has just
 //                read hold its 8 packed columns, so the next tile's scores wait for this tile's products
 // All waits are bounded.
+//
+// FIRST: the first-order moment family's chunks.  What a token takes from everything before its chunk (or, DKDV, after
+// it) is one more product per row tile with the d x d state S1 -- FWD x S1, DQ gs S1^T, DKDV v S1^T and k S1 -- so it
+// goes into the same accumulators before the chunk's own products, from a bf16 copy of S1 already scaled by the
+// first-order coefficient; the state's vectors (constant row, normaliser column) are added in the epilogue.  No fp32
+// rows travel between a read-out kernel and this one.
 #include "fm_common.cuh"
 #include "fm_sm100.cuh"
 
@@ -39,17 +45,22 @@ struct ShortArgs {
   const stat_t* stat_k;
   int nrows, ncols, off, mask, ntr, chunk, ratio, o_heads;
   float a0, a1, a2, lim;
+  // FIRST: running sums of the states, rows [y_a | 1] of `dvp` floats, d + 1 rows per (head, chunk)
+  const float* st;
+  int dvp, nchunk, zero_chunk;    // zero_chunk: the chunk whose running sum is empty (-1: none)
 };
 
 constexpr int BM = 128, BN = 64, D = 64;
 constexpr int kThreads = 352, kComputeWarps = 8, kProducerWarp = 8, kIssuerWarp = 9, kAccIssuerWarp = 10;
 constexpr int ROW_TILE = BM * 128, COL_TILE = BN * 128, STAGE = 2 * COL_TILE;
 
-template <int MODE>
+template <int MODE, bool FIRST>
 struct SH {
   static constexpr int NS = 3;
   static constexpr int OFF_U = ROW_TILE, OFF_ST = (MODE == MODE_FWD ? 1 : 2) * ROW_TILE;
-  static constexpr int OFF_VEC = OFF_ST + NS * STAGE;      // per compute warp 2 x 32 floats; row sums (FWD)
+  static constexpr int OFF_S1 = OFF_ST + NS * STAGE;       // FIRST: the chunk's 64 x 64 state copy
+  static constexpr int OFF_STV = OFF_S1 + (FIRST ? 8192 : 0);   // FIRST: normaliser column 64, constant row 65 (+ 3)
+  static constexpr int OFF_VEC = OFF_STV + (FIRST ? 132 * 4 : 0);   // per compute warp 2 x 32 floats; row sums (FWD)
   static constexpr int OFF_BAR = OFF_VEC + kComputeWarps * 2 * 32 * 4;
   static constexpr int NBAR = 2 + 2 * NS + 4;
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
@@ -86,11 +97,53 @@ __device__ __forceinline__ void issue_acc(uint32_t acc, uint32_t a_tmem, int ste
   for (int ks = 0; ks < BN / 16; ++ks) umma_ts_1(acc, a_tmem + ks * step, b_mn + ks * 128, idesc, ks > 0 ? 1u : accumulate);
 }
 
-template <int MODE>
+// One thread's row segment: (accumulator + mul * vec) * scale -> bf16, vec NC floats of shared memory; returns its
+// dot product with the x row when wanted (store_row of fm_sm100.cuh with a vector in place of fp32 rows).
+template <int NC>
+__device__ __forceinline__ float store_row_vec(uint32_t taddr, bool row_ok, __nv_bfloat16* dst, uint32_t vec_s, float mul,
+                                               const __nv_bfloat16* xr, float scale) {
+  float part = 0.f;
+  const bool wide = (((uintptr_t)dst | (uintptr_t)xr) & 31) == 0;
+#pragma unroll
+  for (int c0 = 0; c0 < NC; c0 += 16) {
+    uint32_t ov[16];
+    tmem_ld16(taddr + c0, ov);
+    tmem_wait_ld();
+    if (row_ok) {
+      float f[16];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const ulonglong2 v = lds_v2(vec_s + (c0 + 4 * e) * 4);
+        float w[4];
+        unpack2(v.x, w[0], w[1]);
+        unpack2(v.y, w[2], w[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[4 * e + i] = fmaf(mul, w[i], __uint_as_float(ov[4 * e + i])) * scale;
+      }
+      uint32_t w[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) w[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+      stg32(dst + c0, w, wide);
+      if (xr) {
+        uint32_t xw[8];
+        ldg32(xr + c0, xw, wide);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          part = fmaf(f[2 * e], __uint_as_float(xw[e] << 16), part);
+          part = fmaf(f[2 * e + 1], __uint_as_float(xw[e] & 0xFFFF0000u), part);
+        }
+      }
+    }
+  }
+  return part;
+}
+
+template <int MODE, bool FIRST>
 __global__ void __launch_bounds__(kThreads, 2)
 short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
-             const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmZ, const ShortArgs a) {
-  using C = SH<MODE>;
+             const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmZ,
+             const __grid_constant__ CUtensorMap tmS, const ShortArgs a) {
+  using C = SH<MODE, FIRST>;
   constexpr int NS = C::NS;
   constexpr bool rev = MODE == MODE_DKDV, FWD = MODE == MODE_FWD, HAS_U = !FWD;
   extern __shared__ uint8_t smem_raw[];
@@ -127,6 +180,8 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     if (++cp.t >= tb + Jh && rev) { cp.t = tb; ++cp.h; }
   };
 
+  const int chunk = FIRST ? r0 / a.chunk : 0;
+  const bool has_state = FIRST && chunk != a.zero_chunk;
   if (tid == 0) {
     mbar_init(BAR_X, 1);
     mbar_init(BAR_DONE, 1);
@@ -147,9 +202,10 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   if (warp == kProducerWarp) {
     // ================= TMA producer =================
     if (lane == 0 && J > 0) {
-      mbar_expect_tx(BAR_X, (HAS_U ? 2 : 1) * ROW_TILE);
+      mbar_expect_tx(BAR_X, (HAS_U ? 2 : 1) * ROW_TILE + (has_state ? 8192 : 0));
       tma_load_3d(sbase, &tmX, BAR_X, 0, r0, head);
       if (HAS_U) tma_load_3d(sbase + C::OFF_U, &tmU, BAR_X, 0, r0, head);
+      if (has_state) tma_load_3d(sbase + C::OFF_S1, &tmS, BAR_X, 0, 0, head * a.nchunk + chunk);
     }
     ColPos pc = pos0;
     for (int j = 0; j < J; ++j, advance(pc)) {
@@ -190,14 +246,27 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     // ================= issuer of the accumulating products =================
     if (J > 0) {
       const uint32_t st_mn = desc_lo(sbase + C::OFF_ST, COL_TILE);   // stage 0, MN-major view
-      for (int j = 0; j < J; ++j) {
+      bool ok = true;
+      if (has_state) {
+        ok = mbar_wait_warp(BAR_X, 0);
+        if (!ok) report(76);
+        tc_fence_after();
+        const uint32_t x_lo = desc_lo(sbase, 16), u_lo = desc_lo(sbase + C::OFF_U, 16);
+        const uint32_t s_k = desc_lo(sbase + C::OFF_S1, 16), s_mn = desc_lo(sbase + C::OFF_S1, 8192);
+        if (ok && elect_one()) {
+          if (!FWD) umma_ss_k64(tmem + C::T_A1, u_lo, s_k, idesc_bf16(BM, D, 0, 0));
+          if (FWD || rev) umma_ss_kmn_steps<4>(tmem + (FWD ? C::T_A1 : C::T_A2), x_lo, s_mn, idesc_bf16(BM, D, 0, 1), 0u);
+        }
+        __syncwarp();
+      }
+      for (int j = 0; ok && j < J; ++j) {
         const int s = j % NS;
         if (!mbar_wait_warp(BAR_P, (uint32_t)(j & 1))) { report(75); break; }
         tc_fence_after();
         const uint32_t y_mn = st_mn + (uint32_t)s * (STAGE >> 4), z_mn = y_mn + (COL_TILE >> 4);
         if (elect_one()) {
-          issue_acc(tmem + C::T_A1, tmem + C::T_E, C::INPLACE ? 16 : 8, FWD ? z_mn : y_mn, j > 0 ? 1u : 0u);
-          if (rev) issue_acc(tmem + C::T_A2, tmem + C::T_P, 16, z_mn, j > 0 ? 1u : 0u);
+          issue_acc(tmem + C::T_A1, tmem + C::T_E, C::INPLACE ? 16 : 8, FWD ? z_mn : y_mn, j > 0 || has_state ? 1u : 0u);
+          if (rev) issue_acc(tmem + C::T_A2, tmem + C::T_P, 16, z_mn, j > 0 || has_state ? 1u : 0u);
           umma_commit(BAR_PV);
           umma_commit(BAR_EMPTY(s));
           if (j + 1 == J) umma_commit(BAR_DONE);
@@ -240,6 +309,12 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       const int col = cp.t * BN + cpart * 32 + lane;
       return (col < a.ncols) ? -__ldg(a.dvec + (size_t)cp.h * a.ncols + col) : 0.f;
     };
+    float* const stv = (float*)(smem + C::OFF_STV);
+    if (FIRST) {    // read after the barrier in the epilogue
+      const float* st = a.st + (size_t)(head * a.nchunk + chunk) * (D + 1) * a.dvp;
+      for (int i = tid; i < 129; i += 256)
+        stv[i] = !has_state ? 0.f : (i < 64 ? __ldg(st + (size_t)i * a.dvp + D) : __ldg(st + (size_t)D * a.dvp + (i - 64)));
+    }
     uint64_t rs2 = 0ull;
     ColPos pc = pos0;
     float nxt = rev ? fetch_vec(0, pc) : 0.f;
@@ -333,10 +408,36 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     tc_fence_after();
     // ---- epilogue: FWD and DQ 32 of the 64 columns per warp; DKDV grad_k by warps 0-3, grad_v by warps 4-7 ----
     float scale = 1.f, rowsum = 0.f;
+    const uint32_t stv_s = sbase + C::OFF_STV;
+    float A1 = 0.f;
+    if (FIRST) {
+      float unused;
+      unpack2(A1v, A1, unused);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
     if (FWD) {
       float lo, hi;
       unpack2(rs2, lo, hi);
-      rows_sum[cpart * BM + qd * 32 + lane] = lo + hi;
+      lo += hi;
+      if (FIRST && has_state && ok && J > 0) {
+        // the state's share of the row sum: x . (normaliser column), half of the row per warp, read from its tile
+        if (!mbar_wait(BAR_X, 0)) report(78);
+        const int r = qd * 32 + lane;
+        float dot = 0.f;
+#pragma unroll
+        for (int pc = 0; pc < 4; ++pc) {
+          const ulonglong2 xv = lds_v2(sbase + r * 128 + (((cpart * 4 + pc) ^ (r & 7)) << 4));
+          const uint32_t xw[4] = {(uint32_t)xv.x, (uint32_t)(xv.x >> 32), (uint32_t)xv.y, (uint32_t)(xv.y >> 32)};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float* nc = stv + cpart * 32 + 8 * pc + 2 * e;
+            dot = fmaf(__uint_as_float(xw[e] << 16), nc[0], dot);
+            dot = fmaf(__uint_as_float(xw[e] & 0xFFFF0000u), nc[1], dot);
+          }
+        }
+        lo += A1 * dot + (cpart == 0 ? a.a0 * stv[128] : 0.f);
+      }
+      rows_sum[cpart * BM + qd * 32 + lane] = lo;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       rowsum = rows_sum[qd * 32 + lane] + rows_sum[BM + qd * 32 + lane];
       if (a.den_add && row_ok) rowsum += a.den_add[(size_t)head * a.nrows + row];
@@ -346,7 +447,19 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       const size_t grow = (size_t)head * a.nrows + (row_ok ? row : 0);
       float part = 0.f;
       const bool dots_here = !FWD && a.dots != nullptr && !(rev && cpart == 1);
-      if constexpr (rev) {
+      if constexpr (FIRST && rev) {
+        const bool second = cpart == 1;
+        part = store_row_vec<64>(tl + (second ? C::T_A2 : C::T_A1), row_ok,
+                                 (__nv_bfloat16*)(second ? a.o2 : a.o1) + grow * D, second ? stv_s + 256 : stv_s,
+                                 second ? a.a0 : A1, dots_here ? (const __nv_bfloat16*)a.x + grow * D : nullptr, 1.f);
+      } else if constexpr (FIRST) {
+        const int cc = cpart * 32;
+        const size_t orow = FWD ? out_row(head, row_ok ? row : 0, a.nrows, a.o_heads) : grow;
+        part = store_row_vec<32>(tl + C::T_A1 + cc, row_ok, (__nv_bfloat16*)a.o1 + orow * D + cc,
+                                 stv_s + (FWD ? 256 : 0) + cc * 4, FWD ? a.a0 : -A1 * dl_row,
+                                 dots_here ? (const __nv_bfloat16*)a.x + grow * D + cc : nullptr, scale);
+        if (FWD && cpart == 0 && row_ok) a.den_out[grow] = rowsum;
+      } else if constexpr (rev) {
         const bool second = cpart == 1;
         const float* add = second ? a.o2_add : a.o1_add;
         part = store_row<64>(tl + (second ? C::T_A2 : C::T_A1), row_ok, (__nv_bfloat16*)(second ? a.o2 : a.o1) + grow * D,
@@ -377,12 +490,12 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
 
 template <int MODE>
 int launch(const Ctx& c, const char* name, const void* x, const void* u, const void* y, const void* z, int nrows,
-           int ncols, ShortArgs a) {
+           int ncols, ShortArgs a, const FirstState* fs = nullptr) {
   constexpr bool rev = MODE == MODE_DKDV;
   const fastmax_problem& p = c.p;
   const int heads = rev ? p.bhkv : p.bh, col_heads = rev ? p.bh : p.bhkv;
   if (heads == 0 || nrows == 0) return FASTMAX_OK;
-  CUtensorMap tx, tu, ty, tz;
+  CUtensorMap tx, tu, ty, tz, ts;
   int rc;
   if ((rc = tma_map_bf16(&tx, x, heads, nrows, D, BM))) return rc;
   if ((rc = tma_map_bf16(&tu, u ? u : x, heads, nrows, D, BM))) return rc;
@@ -399,9 +512,21 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
   a.a1 = p.a1;
   a.a2 = (p.p == 2) ? p.a2 : 0.f;
   a.lim = p.lim;
-  FM_CUDA_TRY(cudaFuncSetAttribute(short_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH<MODE>::SMEM));
   dim3 grid((unsigned)((size_t)heads * a.ntr));
-  FM_LAUNCH(name, c.stream, (short_kernel<MODE><<<grid, kThreads, SH<MODE>::SMEM, c.stream>>>(tx, tu, ty, tz, a)));
+  if (fs) {
+    a.nchunk = (nrows + a.chunk - 1) / a.chunk;
+    a.st = fs->states;
+    a.dvp = moment_dims(D, 1).dvp;
+    a.zero_chunk = fs->zero_chunk;
+    if ((rc = tma_map_bf16(&ts, fs->s1b, (size_t)heads * a.nchunk, D, D, D))) return rc;
+    using C = SH<MODE, true>;
+    FM_CUDA_TRY(cudaFuncSetAttribute(short_kernel<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    FM_LAUNCH(name, c.stream, (short_kernel<MODE, true><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, ts, a)));
+  } else {
+    using C = SH<MODE, false>;
+    FM_CUDA_TRY(cudaFuncSetAttribute(short_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    FM_LAUNCH(name, c.stream, (short_kernel<MODE, false><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, tx, a)));
+  }
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
@@ -409,7 +534,7 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
 }  // namespace
 
 int dense_tc_short_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats, void* out,
-                           float* den, const ChunkAdd* ca) {
+                           float* den, const ChunkAdd* ca, const FirstState* fs) {
   const fastmax_problem& p = c.p;
   ShortArgs a = {};
   a.stat_q = p.normalize ? stats : nullptr;
@@ -418,7 +543,7 @@ int dense_tc_short_forward(const Ctx& c, const void* q, const void* k, const voi
   a.den_out = den;
   a.o_heads = c.out_heads;
   if (ca) { a.chunk = ca->chunk; a.o1_add = ca->out_add; a.den_add = ca->den_add; }
-  return launch<MODE_FWD>(c, "fm_dense_tc_fwd", q, nullptr, k, v, p.nq, p.nk, a);
+  return launch<MODE_FWD>(c, "fm_dense_tc_fwd", q, nullptr, k, v, p.nq, p.nk, a, fs);
 }
 
 static ShortArgs backward_args(const fastmax_problem& p, const float* dvec, const stat_t* stats, const ChunkAdd* ca) {
@@ -431,23 +556,23 @@ static ShortArgs backward_args(const fastmax_problem& p, const float* dvec, cons
 }
 
 int dense_tc_short_dq(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
-                      const stat_t* stats, float* dots, void* grad_q, const ChunkAdd* ca) {
+                      const stat_t* stats, float* dots, void* grad_q, const ChunkAdd* ca, const FirstState* fs) {
   ShortArgs a = backward_args(c.p, dvec, stats, ca);
   a.o1 = grad_q;
   a.dots = c.p.normalize ? dots : nullptr;
   a.o1_add = ca ? ca->gq_add : nullptr;
-  return launch<MODE_DQ>(c, "fm_dense_tc_dq", q, gs, k, v, c.p.nq, c.p.nk, a);
+  return launch<MODE_DQ>(c, "fm_dense_tc_dq", q, gs, k, v, c.p.nq, c.p.nk, a, fs);
 }
 
 int dense_tc_short_dkdv(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
-                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd* ca) {
+                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd* ca, const FirstState* fs) {
   ShortArgs a = backward_args(c.p, dvec, stats, ca);
   a.o1 = grad_k;
   a.o2 = grad_v;
   a.dots = c.p.normalize ? dots + c.p.bh : nullptr;
   a.o1_add = ca ? ca->gk_add : nullptr;
   a.o2_add = ca ? ca->gv_add : nullptr;
-  return launch<MODE_DKDV>(c, "fm_dense_tc_dkdv", k, v, q, gs, c.p.nk, c.p.nq, a);
+  return launch<MODE_DKDV>(c, "fm_dense_tc_dkdv", k, v, q, gs, c.p.nk, c.p.nq, a, fs);
 }
 
 int tc_short_status(int* out, cudaStream_t stream) {

@@ -493,13 +493,17 @@ first_readout_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_const
   }
 }
 
-// bf16 copy of the first-order block: out[m][a][c] = state[m][f_lin + a][c], a, c < D
+// bf16 copy of the first-order block: out[m][a][c] = state[m][f_lin + a][c], a, c < D; with nchunk > 0 times the
+// first-order coefficient of the matrix's head
 __global__ void __launch_bounds__(256) s1_to_bf16_kernel(const float* __restrict__ state,
                                                          __nv_bfloat16* __restrict__ out, int d, int dvp,
-                                                         int rows, int f_lin) {
+                                                         int rows, int f_lin, int nchunk, const stat_t* stat_q,
+                                                         const stat_t* stat_k, float a1, float lim) {
+  const int head = nchunk > 0 ? blockIdx.x / nchunk : 0;
+  const float scale = nchunk > 0 ? a1 * (stat_scale(stat_q, head, lim) * stat_scale(stat_k, head, lim)) : 1.f;
   const float* src = state + (size_t)blockIdx.x * rows * dvp + (size_t)f_lin * dvp;
   __nv_bfloat16* dst = out + (size_t)blockIdx.x * d * d;
-  for (int i = threadIdx.x; i < d * d; i += 256) dst[i] = __float2bfloat16_rn(src[(size_t)(i / d) * dvp + i % d]);
+  for (int i = threadIdx.x; i < d * d; i += 256) dst[i] = __float2bfloat16_rn(scale * src[(size_t)(i / d) * dvp + i % d]);
 }
 
 }  // namespace
@@ -557,13 +561,14 @@ int first_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void* 
 }
 
 // bf16 copies of the first-order blocks of `mats` prefix (or total) states
-int first_tc_convert(const Ctx& c, int mats, const float* state, void* s1b) {
+int first_tc_convert(const Ctx& c, int mats, const float* state, void* s1b, int nchunk, const stat_t* stats) {
   if (mats == 0) return FASTMAX_OK;
   const fastmax_problem& p = c.p;
   const MomentDims m = moment_dims(p.d, p.p);
   FM_LAUNCH("fm_first_state_bf16", c.stream,
             (s1_to_bf16_kernel<<<mats, 256, 0, c.stream>>>(state, (__nv_bfloat16*)s1b, p.d, m.dvp, m.f,
-                                                           p.d * p.d - m.f0)));
+                                                           p.d * p.d - m.f0, nchunk, p.normalize ? stats : nullptr,
+                                                           p.normalize ? stats + p.bh : nullptr, p.a1, p.lim)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }

@@ -9,10 +9,15 @@ namespace fm {
 
 static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
+// Tokens per chunk.  Second order: 2048, measured best for the tensor-core kernels (8.9 ms at 1024, 7.8 at 2048,
+// 8.2 at 4096 per step for 8 heads of 65536 tokens): a chunk's state is as large as its tokens, so fewer, larger
+// chunks mean fewer states to build, scan and convert.  First order, causal: a state is d + 1 rows (17 KB at
+// d = 64 against 131 KB of tokens in 512), so a short chunk wins -- what a token costs there is its own chunk in score
+// form (256 heads x 4096, d = 64, bf16: 1.91 ms at 256, 1.80 at 512, 1.97 at 1024, 2.41 at 2048; float32 at d = 32,
+// 8 heads x 4096: 0.31, 0.42, 0.64, 1.06).  First order, unmasked: there is no in-chunk part and every chunk only
+// adds a state to sum.
 int moments_chunk(const fastmax_problem& p) {
-  // 2048 tokens per chunk: measured best for the tensor-core kernels (8.9 ms at 1024, 7.8 at 2048, 8.2 at
-  // 4096 per step for 8 heads of 65536 tokens); fewer, larger chunks mean fewer states to build, scan and convert
-  int L = p.chunk > 0 ? p.chunk : 2048;
+  int L = p.chunk > 0 ? p.chunk : (p.p == 1 && p.mask ? (p.dtype == FASTMAX_BF16 ? 512 : 256) : 2048);
   L = (L + 255) / 256 * 256;
   return L;
 }
@@ -154,6 +159,12 @@ static int read_first_final(const Ctx& c, int type_b, int n, const void* tile, c
                           nullptr, 0, final, out, den_out, dots);
 }
 
+// Causal p = 1 at d = 64: the score kernels of the chunks read the states themselves, so there is no read-out pass
+// and no fp32 rows between two kernels.
+static bool first_fused(const fastmax_problem& p) {
+  return p.p == 1 && p.mask && p.d == 64 && p.nq == p.nk && first_tc_supports(p) && dense_tc_wide_supports(p);
+}
+
 // Exclusive running sums over the chunks of every head (per-chunk mode).  With `fuse` and the tensor-core
 // second-order part, the second-order rows go straight to their bf16 transposed copies at `second16` in one
 // pass over the raw states and stay raw in `states` (nothing else reads them); only the first-order rows are
@@ -187,6 +198,13 @@ int moments_forward_finish(const Ctx& c, const void* q, const void* k, const voi
   // second16 != null: the caller does not need the fp32 second-order prefixes (see prefix_states)
   bool ready;
   if ((rc = prefix_states(c, nchunk, kv_states, s_base, 0, second16 != nullptr, second16, &ready))) return rc;
+  if (first_fused(p) && !o.out_f32) {
+    if ((rc = first_tc_convert(c, p.bh * nchunk, kv_states, s16, nchunk, stats))) return rc;
+    ChunkAdd own;
+    own.chunk = L;
+    const FirstState fs = {kv_states, s16, s_base ? -1 : 0};
+    return dense_tc_short_forward(c, q, k, v, stats, o.out, o.den, &own, &fs);
+  }
   // without a base the tokens of the first chunk have nothing before them
   if ((rc = read_states(zeroing(c, s_base ? -1 : 0), 0, p.nq, 1, q, nullptr, nullptr, nullptr, 0, nullptr, nullptr,
                         kv_states, s16, stats, o_add, den_add, nullptr, ready ? second16 : nullptr)))
@@ -334,6 +352,20 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
       if (ready) kv16 = s16;
     } else if (moment_kept16_bytes(p) > 0) {
       kv16 = (const char*)kv_total_kept + moment_state_bytes(p, p.nk);
+    }
+    if (first_fused(p)) {
+      const float* kv = kv_total_kept ? kv_total_kept : states;
+      ChunkAdd own;
+      own.chunk = L;
+      if ((rc = first_tc_convert(c, p.bh * nck, kv, s16, nck, stats))) return rc;
+      const FirstState before = {kv, s16, 0};
+      if ((rc = dense_tc_short_dq(c, q, k, v, gs, dvec, stats, dots, grad_q, &own, &before))) return rc;
+      if ((rc = moments_build_states(skipping(c, 0), p.nq, q, grad_out, den, delta, 1, gs, dvec, states))) return rc;
+      if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, s16, &ready))) return rc;
+      if ((rc = first_tc_convert(c, p.bh * ncq, states, s16, ncq, stats))) return rc;
+      const FirstState after = {states, s16, ncq - 1};
+      if ((rc = dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, &own, &after))) return rc;
+      return p.normalize ? launch_norm_fixup(c, q, k, stats, dots, grad_q, grad_k) : FASTMAX_OK;
     }
     // grad_q: the first chunk's tokens have no keys before their chunk; grad_k, grad_v: the last chunk's
     // tokens no queries after theirs, and nothing reads the query/gradient state of the first chunk
