@@ -489,11 +489,11 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
   }
   float* dots = (float*)((char*)workspace + w.dots_off);
   float* delta = (float*)((char*)workspace + w.delta_off);
-  if (p.normalize)
-    FM_CUDA_TRY(cudaMemsetAsync(dots, 0, sizeof(float) * (size_t)(p.bh + p.bhkv), c.stream));
+  const int dot_count = p.normalize ? p.bh + p.bhkv : 0;   // added to with atomics: zeroed by the preparation pass
   if (impl == FASTMAX_IMPL_DENSE_TC) {
     void* gs = (char*)workspace + w.gs_off;
-    if ((rc = launch_gprep(c, grad_out, out, den, gs, delta))) return rc;
+    if ((rc = launch_gprep(c, grad_out, out, den, gs, delta, dots, dot_count))) return rc;
+    if (p.nq == 0 && dot_count) FM_CUDA_TRY(cudaMemsetAsync(dots, 0, sizeof(float) * (size_t)dot_count, c.stream));
     if ((rc = dense_tc_backward(c, q, k, v, gs, delta, (const stat_t*)stats, dots, grad_q, grad_k,
                                 grad_v)))
       return rc;
@@ -503,6 +503,7 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
                                    (char*)workspace + split_bwd_off(p))))
       return rc;
   } else {
+    if (dot_count) FM_CUDA_TRY(cudaMemsetAsync(dots, 0, sizeof(float) * (size_t)dot_count, c.stream));
     if ((rc = launch_delta(c, grad_out, out, delta))) return rc;
     if ((rc = dense_ffma_backward(c, q, k, v, den, (const stat_t*)stats, grad_out, delta, dots,
                                   grad_q, grad_k, grad_v)))

@@ -16,74 +16,113 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // the scale lim/max is applied inside the attention kernels instead of
 // rewriting q and k in place (reference apply_norm, :255-269).
 // Each warp owns rows; a row of D elements is read by D/VEC lanes, so a warp
-// covers 32*VEC/D rows per load and every load is a full 128-byte line.
+// covers 32*VEC/D rows per load and every load is a full 128-byte line; UNROLL
+// independent loads per lane are in flight, because one at a time left HBM at
+// 45 % (256 heads x 4096 x 64 bf16: 45.5 us per tensor before, 134 MB each).
+// q and k go in one launch (blockIdx.x: query heads, then key heads).  A head that one CTA covers
+// is written directly, so small problems need no zero fill either.
+struct RowmaxArgs {
+  const void* q;
+  const void* k;
+  int bh, nq, nk, rows_per_block, row_offset, direct;
+};
+
 template <typename T, int D, bool WIDE>
-__global__ void __launch_bounds__(256) rowmax_kernel(const T* __restrict__ x, int n,
-                                                     int rows_per_block, int row_offset,
-                                                     stat_t* __restrict__ stats) {
-  // elements per lane: 16 bytes for the wide bf16 rows, else 4 (or 1) elements
-  // (WIDE needs 16-byte aligned rows; the launcher checks the base pointer)
-  constexpr int VEC = WIDE ? 8 : ((D >= 32) ? 4 : 1);
+__global__ void __launch_bounds__(256) rowmax_kernel(const RowmaxArgs a, stat_t* __restrict__ stats) {
+  // elements per lane: 16 bytes in one load for aligned tensors, else 4 (or 1) elements one by one
+  // (WIDE needs 16-byte aligned rows; the launcher checks the base pointers)
+  constexpr int VEC = !WIDE ? ((D >= 32) ? 4 : 1) : (sizeof(T) == 2 ? 8 : 4);
   constexpr int LPR = D / VEC;                 // lanes per row
-  constexpr int RPW = 32 / LPR;                // rows per warp per step
+  constexpr int RPW = 32 / LPR;                // rows per warp per load
+  constexpr int UNROLL = 4;
   static_assert(D % VEC == 0 && LPR <= 32 && 32 % LPR == 0, "bad head dimension");
   const int head = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / LPR, off = (lane % LPR) * VEC;
-  const int row0 = blockIdx.y * rows_per_block;
-  const int row1 = min(n, row0 + rows_per_block);
-  const T* base = x + (size_t)head * n * D;
+  const bool is_q = head < a.bh;
+  const int n = is_q ? a.nq : a.nk;
+  const T* base = is_q ? (const T*)a.q + (size_t)head * n * D : (const T*)a.k + (size_t)(head - a.bh) * n * D;
+  const int row0 = blockIdx.y * a.rows_per_block;
+  const int row1 = min(n, row0 + a.rows_per_block);
   float best = -1.0f;
   int best_row = 0;
   // the loop bound is warp-uniform: every lane takes part in every shuffle
-  for (int rb = row0 + warp * RPW; rb < row1; rb += 8 * RPW) {
-    const int r = rb + sub;
-    float s = 0.f;
-    if (r < row1) {
-      const T* p = base + (size_t)r * D + off;
-      if constexpr (VEC == 8) {
-        const uint4 w = __ldg((const uint4*)p);
-        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+  for (int rb = row0 + warp * RPW; rb < row1; rb += 8 * RPW * UNROLL) {
+    float s[UNROLL];
+    if constexpr (WIDE) {
+      uint4 w[UNROLL];
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        const int r = rb + u * 8 * RPW + sub;
+        w[u] = r < row1 ? __ldg((const uint4*)(base + (size_t)r * D + off)) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        const uint32_t ww[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+        s[u] = 0.f;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float lo = __uint_as_float(ww[e] << 16), hi = __uint_as_float(ww[e] & 0xFFFF0000u);
-          s = fmaf(lo, lo, fmaf(hi, hi, s));
+          if constexpr (sizeof(T) == 2) {
+            const float lo = __uint_as_float(ww[e] << 16), hi = __uint_as_float(ww[e] & 0xFFFF0000u);
+            s[u] = fmaf(lo, lo, fmaf(hi, hi, s[u]));
+          } else {
+            s[u] = fmaf(__uint_as_float(ww[e]), __uint_as_float(ww[e]), s[u]);
+          }
         }
-      } else {
+      }
+    } else {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-          float t = ldf(p + e);
-          s = fmaf(t, t, s);
+      for (int u = 0; u < UNROLL; ++u) {
+        const int r = rb + u * 8 * RPW + sub;
+        s[u] = 0.f;
+        if (r < row1) {
+          const T* p = base + (size_t)r * D + off;
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) {
+            const float t = ldf(p + e);
+            s[u] = fmaf(t, t, s[u]);
+          }
         }
       }
     }
 #pragma unroll
-    for (int m = LPR / 2; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-    if (r < row1 && s > best) { best = s; best_row = r; }
+    for (int u = 0; u < UNROLL; ++u) {
+      const int r = rb + u * 8 * RPW + sub;
+#pragma unroll
+      for (int m = LPR / 2; m >= 1; m >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], m);
+      if (r < row1 && s[u] > best) { best = s[u]; best_row = r; }
+    }
   }
   // NaN norms never compare greater, so they are ignored as a maximum.
-  if (best >= 0.f && (lane % LPR) == 0) {
-    stat_t w = ((stat_t)__float_as_uint(best) << 32) | (stat_t)(0xFFFFFFFFu - (unsigned)(best_row + row_offset));
-    atomicMax(&stats[head], w);
+  stat_t w = best >= 0.f ? ((stat_t)__float_as_uint(best) << 32) | (stat_t)(0xFFFFFFFFu - (unsigned)(best_row + a.row_offset))
+                         : 0ull;
+  __shared__ stat_t warp_best[8];
+#pragma unroll
+  for (int m = 16; m >= 1; m >>= 1) {
+    const stat_t o = __shfl_xor_sync(0xffffffffu, w, m);
+    w = o > w ? o : w;
+  }
+  if (lane == 0) warp_best[warp] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) w = warp_best[i] > w ? warp_best[i] : w;
+    if (a.direct) stats[head] = w;
+    else if (w) atomicMax(&stats[head], w);
   }
 }
 
 template <typename T>
-static int rowmax_one(const Ctx& c, const T* x, int heads, int n, stat_t* stats, int row_offset) {
-  if (heads == 0 || n == 0) return FASTMAX_OK;
-  // enough blocks per head to fill the GPU, at least 256 rows each
-  int splits = max(1, min((n + 255) / 256, (148 * 8 + heads - 1) / heads));
-  int rpb = (n + splits - 1) / splits;
-  dim3 grid(heads, (n + rpb - 1) / rpb);
+static int rowmax_both(const Ctx& c, const RowmaxArgs& a, int heads, int splits, stat_t* stats) {
+  dim3 grid(heads, splits);
+  const bool wide = (((uintptr_t)a.q | (uintptr_t)a.k) & 15) == 0;
   switch (c.p.d) {
 #define FM_CASE(DD) \
   case DD:                                                                              \
-    if (sizeof(T) == 2 && DD >= 64 && ((uintptr_t)x & 15) == 0)                           \
-      FM_LAUNCH("fm_rowmax", c.stream,                                                    \
-                (rowmax_kernel<T, DD, (sizeof(T) == 2 && DD >= 64)><<<grid, 256, 0, c.stream>>>(x, n, rpb, row_offset, stats))); \
+    if (wide && DD * (int)sizeof(T) >= 16)                                              \
+      FM_LAUNCH("fm_rowmax", c.stream, (rowmax_kernel<T, DD, true><<<grid, 256, 0, c.stream>>>(a, stats)));  \
     else                                                                                  \
-      FM_LAUNCH("fm_rowmax", c.stream,                                                    \
-                (rowmax_kernel<T, DD, false><<<grid, 256, 0, c.stream>>>(x, n, rpb, row_offset, stats)));      \
+      FM_LAUNCH("fm_rowmax", c.stream, (rowmax_kernel<T, DD, false><<<grid, 256, 0, c.stream>>>(a, stats))); \
     break;
     FM_CASE(8) FM_CASE(16) FM_CASE(32) FM_CASE(64) FM_CASE(128)
 #undef FM_CASE
@@ -95,14 +134,15 @@ static int rowmax_one(const Ctx& c, const T* x, int heads, int n, stat_t* stats,
 
 int launch_rowmax(const Ctx& c, const void* q, const void* k, stat_t* stats, int row_offset) {
   const fastmax_problem& p = c.p;
-  FM_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(stat_t) * (size_t)(p.bh + p.bhkv), c.stream));
-  int rc;
-  if (p.dtype == FASTMAX_F32) {
-    if ((rc = rowmax_one<float>(c, (const float*)q, p.bh, p.nq, stats, row_offset))) return rc;
-    return rowmax_one<float>(c, (const float*)k, p.bhkv, p.nk, stats + p.bh, row_offset);
-  }
-  if ((rc = rowmax_one<__nv_bfloat16>(c, (const __nv_bfloat16*)q, p.bh, p.nq, stats, row_offset))) return rc;
-  return rowmax_one<__nv_bfloat16>(c, (const __nv_bfloat16*)k, p.bhkv, p.nk, stats + p.bh, row_offset);
+  const int heads = p.bh + p.bhkv, n = p.nq > p.nk ? p.nq : p.nk;
+  if (heads == 0) return FASTMAX_OK;
+  // enough blocks per head to fill the GPU, at least 512 rows each
+  int splits = max(1, min((n + 511) / 512, (148 * 8 + heads - 1) / heads));
+  RowmaxArgs a{q, k, p.bh, p.nq, p.nk, (n + splits - 1) / splits, row_offset, splits == 1};
+  if (n == 0 || splits > 1) FM_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(stat_t) * (size_t)heads, c.stream));
+  if (n == 0) return FASTMAX_OK;
+  if (p.dtype == FASTMAX_F32) return rowmax_both<float>(c, a, heads, splits, stats);
+  return rowmax_both<__nv_bfloat16>(c, a, heads, splits, stats);
 }
 
 // ---------------------------------------------------------------------------
@@ -196,7 +236,11 @@ __global__ void __launch_bounds__(256) gprep_kernel(const __nv_bfloat16* __restr
                                                     const __nv_bfloat16* __restrict__ out,
                                                     const float* __restrict__ den, size_t rows,
                                                     __nv_bfloat16* __restrict__ gs,
-                                                    float* __restrict__ dvec, int n, int out_heads) {
+                                                    float* __restrict__ dvec, int n, int out_heads,
+                                                    float* __restrict__ zero, int zeros) {
+  // the per-head dots that the gradient kernels after this one add to
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < zeros; i += 256) zero[i] = 0.f;
   constexpr int LPR = D / 8;        // lanes per row, 16 bytes (8 elements) each
   constexpr int RPW = 32 / LPR;     // rows per warp and step
   constexpr int STEPS = 2;          // independent steps per warp: more bytes in flight
@@ -243,7 +287,7 @@ __global__ void __launch_bounds__(256) gprep_kernel(const __nv_bfloat16* __restr
 }
 
 int launch_gprep(const Ctx& c, const void* go, const void* out, const float* den, void* gs,
-                 float* dvec) {
+                 float* dvec, float* zero, int zeros) {
   size_t rows = (size_t)c.p.bh * c.p.nq;
   if (rows == 0) return FASTMAX_OK;
   if ((c.p.d != 64 && c.p.d != 128) || c.p.dtype != FASTMAX_BF16)
@@ -257,12 +301,12 @@ int launch_gprep(const Ctx& c, const void* go, const void* out, const float* den
     FM_LAUNCH("fm_gprep", c.stream,
               (gprep_kernel<64><<<blocks, 256, 0, c.stream>>>((const __nv_bfloat16*)go,
                                                               (const __nv_bfloat16*)out, den, rows,
-                                                              (__nv_bfloat16*)gs, dvec, c.p.nq, c.out_heads)));
+                                                              (__nv_bfloat16*)gs, dvec, c.p.nq, c.out_heads, zero, zeros)));
   else
     FM_LAUNCH("fm_gprep", c.stream,
               (gprep_kernel<128><<<blocks, 256, 0, c.stream>>>((const __nv_bfloat16*)go,
                                                                (const __nv_bfloat16*)out, den, rows,
-                                                               (__nv_bfloat16*)gs, dvec, c.p.nq, c.out_heads)));
+                                                               (__nv_bfloat16*)gs, dvec, c.p.nq, c.out_heads, zero, zeros)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }

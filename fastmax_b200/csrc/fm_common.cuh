@@ -114,8 +114,9 @@ struct FwdOut {
 };
 
 // gs[h,i,:] = grad_out[h,i,:] / den[h,i]  (bf16) and dvec[h,i] = (grad_out[h,i,:] . out[h,i,:]) / den[h,i]
+// and zeroes the `zeros` floats at `zero` (the per-head dots of the kernels that follow)
 int launch_gprep(const Ctx& c, const void* grad_out, const void* out, const float* den, void* gs,
-                 float* dvec);
+                 float* dvec, float* zero = nullptr, int zeros = 0);
 // true when every stage of the moment family runs on tensor cores for this problem (then grad_out
 // and out are read by the gradient preparation pass only)
 bool moments_all_tc(const fastmax_problem& p);

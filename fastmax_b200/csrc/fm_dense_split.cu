@@ -612,12 +612,18 @@ struct SplitJob {
   const float* out;
   float* dvec;
 };
-struct SplitJobs { SplitJob j[4]; };
+struct SplitJobs {
+  SplitJob j[4];
+  float* zero;      // `zeros` floats set to zero (the per-head dots of the kernels that follow)
+  int zeros;
+};
 
 template <int D>
 __global__ void __launch_bounds__(256) split3_kernel(const SplitJobs jobs) {
   constexpr int TPR = D / 8;                    // threads per row
   const SplitJob& jb = jobs.j[blockIdx.y];
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < jobs.zeros; i += 256) jobs.zero[i] = 0.f;
   const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x, row = idx / TPR;
   const int part = (int)(idx % TPR);
   if (row - (size_t)(threadIdx.x & 31) / TPR >= jb.rows) return;      // whole warps leave together
@@ -757,6 +763,10 @@ int dense_split_backward(const Ctx& c, const void* q, const void* k, const void*
   jobs.j[1] = {(const float*)k, k3, (size_t)p.bhkv * p.nk, nullptr, nullptr, nullptr};
   jobs.j[2] = {(const float*)v, v3, (size_t)p.bhkv * p.nk, nullptr, nullptr, nullptr};
   jobs.j[3] = {(const float*)grad_out, g3, (size_t)p.bh * p.nq, den, (const float*)out, dvec};
+  if (p.normalize && !ca) {      // with `ca` other kernels have added to the dots already
+    jobs.zero = dots;
+    jobs.zeros = p.bh + p.bhkv;
+  }
   int rc;
   if ((rc = launch_split3(c, jobs, 4))) return rc;
   SplitArgs a = {};
