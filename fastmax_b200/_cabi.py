@@ -6,7 +6,9 @@ or a call fails, a ``RuntimeError`` is raised.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import functools
 import os
 
 import torch
@@ -184,21 +186,57 @@ def make_problem(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl="a
 
 
 def _require(q, k, v, *more):
+    if q.is_cuda and (q.dim() != 3 or k.dim() != 3 or v.dim() != 3):
+        raise ValueError("q, k and v must be (b*h, n, d) here")
+    _require_any(q, k, v, *more)
+
+
+def _require_any(q, k, v, *more):
     if not q.is_cuda:
         raise RuntimeError("fastmax_b200 runs on CUDA tensors only (there is no CPU path)")
-    if q.dim() != 3 or k.dim() != 3 or v.dim() != 3:
-        raise ValueError("q, k and v must be (b*h, n, d) here")
-    if k.shape != v.shape or q.shape[2] != k.shape[2]:
+    if k.shape != v.shape or q.shape[-1] != k.shape[-1]:
         raise ValueError(f"shape mismatch: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
+    device, dtype = q.device, q.dtype
     for t in (q, k, v) + more:
-        if t.device != q.device or t.dtype != q.dtype:
+        if t.device != device or t.dtype != dtype:
             raise ValueError("all tensors must share one device and dtype")
         if not t.is_contiguous():
             raise ValueError("tensors must be contiguous")
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
+_HERE_ALREADY = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context in which ``device`` is current.  Most calls are made with it current already; entering and
+    leaving ``torch.cuda.device`` then costs more host time (5 us) than the rest of a small call's set-up."""
+    return _HERE_ALREADY if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+@functools.lru_cache(maxsize=256)
+def _plan(dtype, bh, bhkv, nq, nk, d, mask, normalize, p, impl, a0, a1, a2, lim, temperature, chunk):
+    """(problem, forward workspace, backward workspace, stats bytes) of one problem: host arithmetic that depends
+    on nothing but these values."""
+    L = lib()
+    prob = Problem(dtype, bh, bhkv, nq, nk, d, mask, normalize, p, impl, a0, a1, a2, lim, temperature, chunk)
+    return (prob, L.fastmax_b200_forward_workspace_bytes(prob), L.fastmax_b200_backward_workspace_bytes(prob),
+            max(L.fastmax_b200_stats_bytes(prob), 8))
+
+
+def _heads_of(t):
+    return t.shape[0] if t.dim() == 3 else t.shape[0] * t.shape[1]
+
+
+def _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk):
+    if p not in (1, 2):
+        raise ValueError(f"p must be 1 or 2, got: {p}")
+    return _plan(_dtype_code(q), _heads_of(q), _heads_of(k), q.shape[-2], k.shape[-2], q.shape[-1], int(bool(mask)), int(bool(normalize)), int(p),
+                 IMPL[impl] if isinstance(impl, str) else int(impl), float(a0), float(a1), float(a2), float(lim),
+                 float(temperature), int(chunk))
 
 
 def _workspace(nbytes: int, device) -> torch.Tensor:
@@ -212,21 +250,26 @@ def forward(q, k, v, *, mask, normalize, temperature=1.0, a0=1.0, a1=1.0, a2=0.5
     ``buffers`` may hold preallocated ``out``, ``den``, ``stats`` and ``workspace`` tensors
     (see ``forward_buffers``); otherwise they are allocated here."""
     _require(q, k, v)
+    return forward_any(q, k, v, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk, buffers)
+
+
+def forward_any(q, k, v, mask, normalize, temperature, a0, a1, a2, lim, p, impl="auto", chunk=0, buffers=None):
+    """``forward`` on contiguous (b*h, n, d) or (b, h, n, d) tensors; out has q's shape."""
+    _require_any(q, k, v)
     L = lib()
-    prob = make_problem(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
-    with torch.cuda.device(q.device):
-        wsb = L.fastmax_b200_forward_workspace_bytes(prob)
+    prob, wsb, _, stats_bytes = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    with _on(q.device):
         if buffers is None:
             out = torch.empty_like(q)
-            den = torch.empty(q.shape[:2], dtype=torch.float32, device=q.device)
-            stats = torch.empty(max(L.fastmax_b200_stats_bytes(prob), 8), dtype=torch.uint8, device=q.device)
-            ws = _workspace(wsb, q.device)
+            den = torch.empty(prob.bh, prob.nq, dtype=torch.float32, device=q.device)
+            stats = torch.empty(stats_bytes, dtype=torch.uint8, device=q.device)
+            ws = _workspace(wsb, q.device) if wsb else None
         else:
             out, den, stats, ws = buffers["out"], buffers["den"], buffers["stats"], buffers["workspace"]
             if ws.numel() < wsb:
                 raise ValueError("preallocated forward workspace is too small")
         rc = L.fastmax_b200_forward(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                    den.data_ptr(), stats.data_ptr(), ws.data_ptr(), wsb, _stream(q))
+                                    den.data_ptr(), stats.data_ptr(), _ptr(ws), wsb, _stream(q))
     _check(rc, "fastmax_b200_forward")
     return out, den, stats
 
@@ -245,13 +288,12 @@ def forward_bt(q, k, v, heads_per_batch, *, mask, normalize, temperature=1.0, a0
     takes after a ``view`` -- written in that layout by the attention kernel itself."""
     _require(q, k, v)
     L = lib()
-    prob = make_problem(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    prob, wsb, _, stats_bytes = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
     bh, nq, d = q.shape
-    with torch.cuda.device(q.device):
-        wsb = L.fastmax_b200_forward_workspace_bytes(prob)
+    with _on(q.device):
         out = torch.empty(bh // heads_per_batch, nq, heads_per_batch, d, dtype=q.dtype, device=q.device)
         den = torch.empty(bh, nq, dtype=torch.float32, device=q.device)
-        stats = torch.empty(max(L.fastmax_b200_stats_bytes(prob), 8), dtype=torch.uint8, device=q.device)
+        stats = torch.empty(stats_bytes, dtype=torch.uint8, device=q.device)
         ws = _workspace(wsb, q.device)
         rc = L.fastmax_b200_forward_bt(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                                        den.data_ptr(), stats.data_ptr(), int(heads_per_batch), ws.data_ptr(), wsb,
@@ -268,9 +310,8 @@ def backward_bt(q, k, v, out_bt, den, stats, grad_out_bt, heads_per_batch, *, ma
         if t.device != q.device or t.dtype != q.dtype or not t.is_contiguous() or t.numel() != q.numel():
             raise ValueError("out and grad_out must be contiguous (batch, nq, heads, d) tensors of q's dtype")
     L = lib()
-    prob = make_problem(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
-    with torch.cuda.device(q.device):
-        wsb = L.fastmax_b200_backward_workspace_bytes(prob)
+    prob, _, wsb, _ = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    with _on(q.device):
         gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         ws = _workspace(wsb, q.device)
         rc = L.fastmax_b200_backward_bt(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out_bt.data_ptr(),
@@ -322,10 +363,17 @@ def backward(q, k, v, out, den, stats, grad_out, *, mask, normalize, temperature
     """Gradients (grad_q, grad_k, grad_v) in the dtype of the inputs; ``buffers`` as in ``forward``
     with ``grad_q``, ``grad_k``, ``grad_v`` and ``workspace``."""
     _require(q, k, v, out, grad_out)
+    return backward_any(q, k, v, out, den, stats, grad_out, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk,
+                        buffers)
+
+
+def backward_any(q, k, v, out, den, stats, grad_out, mask, normalize, temperature, a0, a1, a2, lim, p, impl="auto",
+                 chunk=0, buffers=None):
+    """``backward`` for ``forward_any``'s tensors."""
+    _require_any(q, k, v, out, grad_out)
     L = lib()
-    prob = make_problem(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
-    with torch.cuda.device(q.device):
-        wsb = L.fastmax_b200_backward_workspace_bytes(prob)
+    prob, _, wsb, _ = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    with _on(q.device):
         if buffers is None:
             gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
             ws = _workspace(wsb, q.device)
@@ -369,7 +417,7 @@ def qkv_split_rope(qkv, cos, sin, rope_n):
     q = torch.empty(b * g * qper, n, d, dtype=qkv.dtype, device=qkv.device)
     k = torch.empty(b * g, n, d, dtype=qkv.dtype, device=qkv.device)
     v = torch.empty_like(k)
-    with torch.cuda.device(qkv.device):
+    with _on(qkv.device):
         rc = lib().fastmax_b200_qkv_split_rope(qkv.data_ptr(), _ptr(cs), _ptr(sn), q.data_ptr(), k.data_ptr(),
                                                v.data_ptr(), b, n, g, qper, d, rope_n, _dtype_code(qkv),
                                                _stream(qkv))
@@ -389,7 +437,7 @@ def qkv_merge_rope_grad(gq, gk, gv, cos, sin, rope_n, batch):
         raise ValueError("head counts do not match the batch size")
     cs, sn = _rope_tables(cos, sin, n, rope_n, gq.device)
     out = torch.empty(batch, n, g, qper + 2, d, dtype=gq.dtype, device=gq.device)
-    with torch.cuda.device(gq.device):
+    with _on(gq.device):
         rc = lib().fastmax_b200_qkv_merge_rope_grad(gq.data_ptr(), gk.data_ptr(), gv.data_ptr(), _ptr(cs), _ptr(sn),
                                                     out.data_ptr(), batch, n, g, qper, d, rope_n,
                                                     _dtype_code(gq), _stream(gq))
@@ -403,7 +451,7 @@ def swap_middle_axes(x):
         raise ValueError("expected a contiguous CUDA tensor (B, X, Y, hs)")
     b, nx, ny, d = x.shape
     out = torch.empty(b, ny, nx, d, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib().fastmax_b200_swap_middle_axes(x.data_ptr(), out.data_ptr(), b, nx, ny, d, _dtype_code(x),
                                                  _stream(x))
     _check(rc, "fastmax_b200_swap_middle_axes")
@@ -416,7 +464,7 @@ def scale_by_noise(x, noise, dropout, out=None):
             or noise.dtype != x.dtype or noise.device != x.device:
         raise ValueError("x and noise must be contiguous CUDA tensors of one shape and dtype")
     out = torch.empty_like(x) if out is None else out
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib().fastmax_b200_scale_by_noise(x.data_ptr(), noise.data_ptr(), out.data_ptr(), float(dropout),
                                                x.numel(), _dtype_code(x), _stream(x))
     _check(rc, "fastmax_b200_scale_by_noise")

@@ -30,10 +30,8 @@ __all__ = ["FASTMultiHeadAttention_Function", "FASTMultiHeadAttention", "fastmax
            "rpe_matrix_creator"]
 
 
-def _to3d(t: torch.Tensor) -> torch.Tensor:
-    if t.dim() == 4:
-        return t.reshape(t.shape[0] * t.shape[1], t.shape[2], t.shape[3]).contiguous()
-    if t.dim() == 3:
+def _contiguous_heads(t: torch.Tensor) -> torch.Tensor:
+    if t.dim() in (3, 4):
         return t.contiguous()
     raise ValueError("q, k, and v should be either 3 or 4 dimensional tensors. "
                      "If 3D: (b*h,n,d), if 4D: (b,h,n,d).")
@@ -65,36 +63,38 @@ class FASTMultiHeadAttention_Function(torch.autograd.Function):
             raise ValueError(f"dropout must be non-negative, got: {dropout}")
         if dropout > 0.0 and (drop_noise is None or drop_noise.shape != q.shape):
             raise ValueError("dropout > 0 needs drop_noise with the shape of q")
-        shape_q, shape_k = q.shape, k.shape
-        q3, k3, v3 = _to3d(q), _to3d(k), _to3d(v)
-        kw = dict(mask=bool(mask), normalize=bool(normalize), temperature=temperature,
-                  a0=a0, a1=a1, a2=a2, lim=lim, p=p, impl=impl)
-        out, den, stats = _cabi.forward(q3, k3, v3, **kw)
+        shapes = None
+        if k.dim() != v.dim():           # one of them has its batch and head axes merged
+            shapes = k.shape, v.shape
+            k, v = [t.flatten(0, 1) if t.dim() == 4 else t for t in (k, v)]
+        q, k, v = _contiguous_heads(q), _contiguous_heads(k), _contiguous_heads(v)
+        args = (bool(mask), bool(normalize), temperature, a0, a1, a2, lim, p, impl)
+        out, den, stats = _cabi.forward_any(q, k, v, *args)
         noise = None
         if dropout > 0.0:
-            noise = _to3d(drop_noise.to(q3.dtype))
-        ctx.save_for_backward(q3, k3, v3, out, den, stats, noise)
-        ctx.kw = kw
+            noise = _contiguous_heads(drop_noise.to(q.dtype))
+        ctx.save_for_backward(q, k, v, out, den, stats, noise)
+        ctx.args, ctx.shapes = args, shapes
         ctx.dropout = float(dropout)
-        ctx.shape_q, ctx.shape_k = shape_q, shape_k
         if noise is not None:
             out = _cabi.scale_by_noise(out, noise, ctx.dropout)
-        return out.reshape(shape_q)
+        return out
 
     @staticmethod
     def backward(ctx, grad_output):
-        q3, k3, v3, out, den, stats, noise = ctx.saved_tensors
-        go = grad_output.reshape(q3.shape).contiguous()
-        if go.dtype != q3.dtype:
-            go = go.to(q3.dtype)
+        q, k, v, out, den, stats, noise = ctx.saved_tensors
+        go = grad_output.contiguous()
+        if go.dtype != q.dtype:
+            go = go.to(q.dtype)
         if noise is not None:
             go = _cabi.scale_by_noise(go, noise, ctx.dropout)
-        gq, gk, gv = _cabi.backward(q3, k3, v3, out, den, stats, go, **ctx.kw)
-        t = ctx.kw["temperature"]
+        gq, gk, gv = _cabi.backward_any(q, k, v, out, den, stats, go, *ctx.args)
+        t = ctx.args[2]
         if t != 1.0:
             gk = gk / t
-        return (gq.reshape(ctx.shape_q), gk.reshape(ctx.shape_k), gv.reshape(ctx.shape_k),
-                None, None, None, None, None, None, None, None, None, None, None)
+        if ctx.shapes is not None:
+            gk, gv = gk.view(ctx.shapes[0]), gv.view(ctx.shapes[1])
+        return (gq, gk, gv, None, None, None, None, None, None, None, None, None, None, None)
 
 
 def fastmax_function(q, k, v, mask=0, dropout_rate=0.0, normalize=0, temperature=1, a0=1, a1=1,

@@ -62,7 +62,7 @@ class FastmaxDecodeState:
         self._check(v, self.bhkv, "v")
         if k.shape != v.shape:
             raise ValueError("k and v differ in shape")
-        with torch.cuda.device(self.device):
+        with _cabi._on(self.device):
             rc = _cabi.lib().fastmax_b200_decode_append(self.prob, k.data_ptr(), v.data_ptr(), k.shape[1],
                                                         self.state.data_ptr(), _cabi._stream(k))
         _cabi._check(rc, "fastmax_b200_decode_append")
@@ -76,7 +76,7 @@ class FastmaxDecodeState:
         if q.shape[1] != 1 or k.shape[1] != 1 or v.shape[1] != 1:
             raise ValueError("step takes exactly one token")
         out = torch.empty_like(q)
-        with torch.cuda.device(self.device):
+        with _cabi._on(self.device):
             rc = _cabi.lib().fastmax_b200_decode_step(self.prob, q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                                       self.state.data_ptr(), self.scratch.data_ptr(),
                                                       out.data_ptr(), _cabi._stream(q))
