@@ -64,6 +64,17 @@ __device__ __forceinline__ float stat_scale(const stat_t* st, int head, float li
   return st ? lim / sqrtf(stat_norm2(st[head])) : 1.0f;
 }
 
+// Order of the row tiles in a score kernel's grid.  Long grids go head by head, so that a head's column tiles stay in
+// L2.  A causal grid of a few waves goes tile by tile over all heads (`by_tile` = number of row heads): the longest row
+// tiles of every head start first and the last wave is made of the shortest ones.
+inline int rows_by_tile(bool causal, long long heads, long long tiles, int ctas_per_sm) {
+  return causal && tiles > 1 && heads * tiles > 148 * ctas_per_sm && heads * tiles <= 8LL * 148 * ctas_per_sm ? (int)heads : 0;
+}
+__device__ __forceinline__ void row_tile_of(int cta, int by_tile, int tiles, int& head, int& tile) {
+  head = by_tile > 0 ? cta % by_tile : cta / tiles;
+  tile = by_tile > 0 ? cta / by_tile : cta % tiles;
+}
+
 // FASTMAX_OK if the problem description is valid, else the error code (message recorded).
 int check_problem(const fastmax_problem* p);
 

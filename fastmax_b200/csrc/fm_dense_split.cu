@@ -59,7 +59,7 @@ struct SplitArgs {
   float* dots;            // per row head: sum of o1 . x, or null
   const stat_t* stat_q;
   const stat_t* stat_k;
-  int nrows, ncols, off, mask, ntr, chunk, ratio;
+  int nrows, ncols, off, mask, ntr, chunk, ratio, by_tile;
   int o_stride, den_stride;   // FWD: floats per row of out and den (the packed layout interleaves them)
   float a0, a1, a2, lim;
 };
@@ -256,8 +256,9 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_TMEM);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // consecutive CTAs work on one head (its column tiles stay in L2); longest rows first
-  const int head = blockIdx.x / a.ntr, pidx = blockIdx.x % a.ntr;
+  // longest rows first (row_tile_of)
+  int head, pidx;
+  row_tile_of(blockIdx.x, a.by_tile, a.ntr, head, pidx);
   const int r0 = (rev ? pidx : a.ntr - 1 - pidx) * BM;
 
   const int ntile = (a.ncols + BN - 1) / BN;
@@ -689,6 +690,7 @@ int launch_mode(const Ctx& c, const char* name, const void* x, const void* u, co
   a.nrows = nrows;
   a.ncols = ncols;
   a.ntr = (nrows + BM - 1) / BM;
+  a.by_tile = rows_by_tile(p.mask && a.chunk == 0, heads, a.ntr, 1);
   a.ratio = p.bh / p.bhkv;
   a.off = p.nk - p.nq;
   a.mask = p.mask;

@@ -52,7 +52,7 @@ struct TcArgs {
   float* dots;          // OP_B: per head sum of o . x  (null when not normalised)
   const stat_t* stat_q;
   const stat_t* stat_k;
-  int nrows, ncols, off, mask, rev, fwd_div, npairs;
+  int nrows, ncols, off, mask, rev, fwd_div, npairs, by_tile;
   float a0, a1, a2, lim;
   int ratio;             // query heads per key/value head (forward-direction modes only)
   int chunk;             // > 0: only the columns of the row pair's own chunk
@@ -118,10 +118,9 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_TMEM);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // consecutive CTAs work on the same head, so its K/V (or Q/G) tiles stay in L2 while the
-  // row tiles that share them are in flight; causal row pairs are issued longest first
-  const int head = blockIdx.x / a.npairs;
-  const int pidx = blockIdx.x % a.npairs;
+  // causal row pairs are issued longest first (row_tile_of)
+  int head, pidx;
+  row_tile_of(blockIdx.x, a.by_tile, a.npairs, head, pidx);
   const int pair = a.rev ? pidx : a.npairs - 1 - pidx;
   const int r0 = pair * C::NG * BM;
   const bool colvec = (MODE == OP_B) && a.rev;
@@ -509,6 +508,7 @@ int launch_tc_d(const Ctx& c, const char* name, const void* x, const void* u, co
   FM_CUDA_TRY(cudaFuncSetAttribute(dense_tc_kernel<MODE, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    C::SMEM));
   a.npairs = (nrows + C::NG * BM - 1) / (C::NG * BM);
+  a.by_tile = rows_by_tile(a.mask && a.chunk == 0, heads, a.npairs, 1);
   dim3 grid((unsigned)((size_t)heads * a.npairs));
   FM_LAUNCH(name, c.stream,
             (dense_tc_kernel<MODE, DD><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, a)));

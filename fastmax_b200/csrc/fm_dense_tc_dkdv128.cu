@@ -40,7 +40,7 @@ struct KArgs {
   float* dots;           // per head sum of gk . x, or null
   const stat_t* stat_q;
   const stat_t* stat_k;
-  int nrows, ncols, off, mask, ntr, chunk;
+  int nrows, ncols, off, mask, ntr, chunk, by_tile;
   int ratio;             // query heads per key/value head (grouped k/v heads)
   float a0, a1, a2, lim;
 };
@@ -90,10 +90,10 @@ dkdv128_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + OFF_TMEM);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // consecutive CTAs work on one head (its column tiles stay in L2); longest rows first
+  // longest rows first (row_tile_of)
   constexpr bool rev = FUSED;
-  const int head = blockIdx.x / a.ntr;
-  const int pidx = blockIdx.x % a.ntr;
+  int head, pidx;
+  row_tile_of(blockIdx.x, a.by_tile, a.ntr, head, pidx);
   const int r0 = (rev ? pidx : a.ntr - 1 - pidx) * BM;
 
   const int ntile = (a.ncols + BN - 1) / BN;
@@ -406,6 +406,7 @@ int launch128(const Ctx& c, const char* name, const void* x, const void* u, cons
   a.off = p.nk - p.nq;
   a.mask = p.mask;
   a.ntr = (nrows + BM - 1) / BM;
+  a.by_tile = rows_by_tile(p.mask && a.chunk == 0, heads, a.ntr, 1);
   a.a0 = p.a0;
   a.a1 = p.a1;
   a.a2 = (p.p == 2) ? p.a2 : 0.f;

@@ -54,7 +54,7 @@ struct WArgs {
   float* dots;           // per head sum of o . x, or null
   const stat_t* stat_q;
   const stat_t* stat_k;
-  int nrows, ncols, off, mask, ntr, chunk;
+  int nrows, ncols, off, mask, ntr, chunk, by_tile;
   float a0, a1, a2, lim;
   int o_heads;           // MODE_FWD: > 0 writes out as (batch, nrows, o_heads, 64)
 };
@@ -141,9 +141,9 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool rev = FUSED;
-  // consecutive CTAs work on one head (its column tiles stay in L2); longest rows first
-  const int head = blockIdx.x / a.ntr;
-  const int pidx = blockIdx.x % a.ntr;
+  // longest rows first (row_tile_of)
+  int head, pidx;
+  row_tile_of(blockIdx.x, a.by_tile, a.ntr, head, pidx);
   const int rt = rev ? pidx : a.ntr - 1 - pidx;
   const int r0 = rt * BM;
 
@@ -584,6 +584,7 @@ int launch_wide(const Ctx& c, const char* name, const void* x, const void* u, co
   a.ncols = ncols;
   a.x = x;
   a.ntr = (nrows + BM - 1) / BM;
+  a.by_tile = rows_by_tile(a.mask && a.chunk == 0, heads, a.ntr, 1);
   dim3 grid((unsigned)((size_t)heads * a.ntr));
   if (MODE == MODE_DKDV && kv_ratio == 1 && a.a2 > 0.f) {
     FM_CUDA_TRY(cudaFuncSetAttribute(dense_tc_wide_kernel<MODE, false, MODE == MODE_DKDV>,
