@@ -480,9 +480,14 @@ int step_ctas(const fastmax_problem& p) {
   return DecCfg<128>::ctas(p.p);
 }
 
-// Below this many tokens the state's traffic decides and step_kernel is as fast (64 heads, d = 64: 68 us at 40 tokens;
-// 70 us on the tensor cores and 71 us in append_kernel at 64).
-constexpr long long kAppendMin = 64;
+// From how many tokens on a prompt's kernels beat step_kernel, which reads and writes whole rows but walks the tokens
+// one by one.  Measured, us, step_kernel / prompt kernel (64 heads): d = 64, p = 2: 56 / 67 at 33 tokens, 69.5 / 67 at 44
+// (bf16), 69 / 70 at 44 (float32); p = 1: 15.0 / 10.4 at 33, 10.4 / 10.4 at 20; d = 128, p = 2: 462 / 391 at 44 (float32),
+// 582 / 663 at 63 (bf16).
+long long append_min(const fastmax_problem& p) {
+  if (p.p == 1) return 24;
+  return p.d == 128 && p.dtype == FASTMAX_BF16 ? 64 : 40;
+}
 
 template <typename T, int D, bool READ>
 int launch_decode(const fastmax_problem& p, const void* q, const void* k, const void* v, long long n_new,
@@ -490,8 +495,8 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
   DecArgs a{p.bh, p.bhkv, p.bhkv ? p.bh / p.bhkv : 1, p.p, p.normalize, p.a0, p.a1, p.a2, p.lim, n_new,
             kHeader + (long long)rows_of(p) * (D + 1)};
   if (p.bhkv == 0) return FASTMAX_OK;
-  if (!READ && n_new >= kAppendMin && decode_append_tc_supports(p)) return decode_append_tc(p, k, v, n_new, state, st);
-  if (!READ && n_new >= kAppendMin) {
+  if (!READ && n_new >= append_min(p) && decode_append_tc_supports(p)) return decode_append_tc(p, k, v, n_new, state, st);
+  if (!READ && n_new >= append_min(p)) {
     dim3 grid(AppCfg<D>::ctas(p.p), p.bhkv);
     FM_LAUNCH("fm_decode_append", st,
               (append_kernel<T, D><<<grid, AppCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));

@@ -19,9 +19,9 @@
 // the transposed stores and the row reads are both free of bank conflicts), then a thread forms its lane's 32 products
 // (half of the block: two warps share a lane quarter), splits them and stores them as the A operand in tensor memory;
 // B is the value tile as TMA delivered it.  The normaliser column is the sum of the thread's own products.
-// 64 heads x 4000 tokens, d = 64, p = 2: 567 us (append_kernel 2.22 ms).  Per block of 64 tokens the generator's chain --
-// transposed stores, barrier, row reads, products and splits, tcgen05.st -- takes about 4 000 cycles of which the two
-// tiles' products need 520: warps issue in 40 % of the cycles and wait mostly for shared memory.
+// 64 heads x 4000 tokens, d = 64, p = 2: 0.39 ms (append_kernel 2.22 ms; 0.57 ms with a block's 32 operand words held at
+// once, which spilled).  Per block of 64 tokens the generator's chain -- transposed stores, barrier, row reads, products
+// and splits, tcgen05.st -- takes some 3 000 cycles of which the two tiles' products need 520.
 // The result goes through shared memory, because a lane is a row of 65 floats: whole rows are read, added and written
 // to both places of the pair.
 #include "fm_common.cuh"
@@ -65,6 +65,22 @@ struct AppArgs {
 };
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_dec_status, 0, code); }
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+      "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      : "memory");
+}
 
 // Byte offset of token chunk c (8 tokens) of row f inside a transposed block.
 __device__ __forceinline__ uint32_t yt_off(int f, int c) { return (uint32_t)(f * 128 + ((c ^ (f & 7) ^ ((f >> 3) & 7)) << 4)); }
@@ -157,11 +173,14 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const AppArgs a) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) run[i] = 0ull;
     auto promote = [&]() {
-      uint32_t v[32];
-      tmem_ld32(tl + hf * 32, v);
-      tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) run[i] = add2(run[i], pack2u(v[2 * i], v[2 * i + 1]));
+      for (int h = 0; h < 2; ++h) {
+        uint32_t v[16];
+        tmem_ld16(tl + hf * 32 + h * 16, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) run[8 * h + i] = add2(run[8 * h + i], pack2u(v[2 * i], v[2 * i + 1]));
+      }
     };
     // 16 bytes (8 features) of one token per thread and load; tokens past the end read as zero
     constexpr int VPT = D / 8, NLD = TB * VPT / kGenThreads;
@@ -222,28 +241,32 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const AppArgs a) {
       asm volatile("bar.sync 1, 512;" ::: "memory");
       fetch(j + 1);
       if (!on) continue;
-      uint32_t hi[16], lo[16];
+      // two chunks of 8 tokens at a time: their 16 operand words and the 32 running sums fit the registers
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const ulonglong2 x = lds_v2(yt_s + yt_off(fx, hf * 4 + c)), y = lds_v2(yt_s + yt_off(fy, hf * 4 + c));
-        const uint32_t xw[4] = {(uint32_t)x.x, (uint32_t)(x.x >> 32), (uint32_t)x.y, (uint32_t)(x.y >> 32)};
-        const uint32_t yw[4] = {(uint32_t)y.x, (uint32_t)(y.x >> 32), (uint32_t)y.y, (uint32_t)(y.y >> 32)};
+      for (int half = 0; half < 2; ++half) {
+        uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint64_t pr = mul2(pack2u(xw[q] << 16, xw[q] & 0xFFFF0000u), pack2u(yw[q] << 16, yw[q] & 0xFFFF0000u));
-          e2 = add2(e2, pr);
-          const uint32_t h = pack_bf16_2(pr);
-          hi[4 * c + q] = h;
-          lo[4 * c + q] = pack_bf16_2(fma2(pack2u(h << 16, h & 0xFFFF0000u), 0xBF800000BF800000ull, pr));
+        for (int c = 0; c < 2; ++c) {
+          const ulonglong2 x = lds_v2(yt_s + yt_off(fx, hf * 4 + half * 2 + c)), y = lds_v2(yt_s + yt_off(fy, hf * 4 + half * 2 + c));
+          const uint32_t xw[4] = {(uint32_t)x.x, (uint32_t)(x.x >> 32), (uint32_t)x.y, (uint32_t)(x.y >> 32)};
+          const uint32_t yw[4] = {(uint32_t)y.x, (uint32_t)(y.x >> 32), (uint32_t)y.y, (uint32_t)(y.y >> 32)};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint64_t pr = mul2(pack2u(xw[q] << 16, xw[q] & 0xFFFF0000u), pack2u(yw[q] << 16, yw[q] & 0xFFFF0000u));
+            e2 = add2(e2, pr);
+            const uint32_t h = pack_bf16_2(pr);
+            hi[4 * c + q] = h;
+            lo[4 * c + q] = pack_bf16_2(fma2(pack2u(h << 16, h & 0xFFFF0000u), 0xBF800000BF800000ull, pr));
+          }
         }
+        if (half == 0 && j > 0) {     // the previous block's products are done: take its sums over, reuse the operand
+          if (ok && !mbar_wait(BAR_DONE(t), (uint32_t)((j - 1) & 1))) { report(64); ok = false; }
+          tc_fence_after();
+          promote();
+        }
+        tmem_st8(tl + 64 + hf * 16 + half * 8, hi);
+        tmem_st8(tl + 96 + hf * 16 + half * 8, lo);
       }
-      if (j > 0) {
-        if (ok && !mbar_wait(BAR_DONE(t), (uint32_t)((j - 1) & 1))) { report(64); ok = false; }
-        tc_fence_after();
-        promote();
-      }
-      tmem_st16(tl + 64 + hf * 16, hi);
-      tmem_st16(tl + 96 + hf * 16, lo);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
