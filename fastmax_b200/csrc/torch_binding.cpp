@@ -199,6 +199,9 @@ std::vector<torch::Tensor> backwardpass(torch::Tensor q, torch::Tensor k, torch:
     stats = (const char*)o.storage().data() + rec.stats_offset;
   }
   fastmax_problem pr = make_problem(q, k, mask, normalize, 1.0, a0, a1, a2, lim, p);
+  // the packed forward leaves statistics but no moment states behind them: one chunk as long as the sequence keeps the
+  // backward on the score form, which reads the statistics only
+  if (stats) pr.chunk = (int32_t)((k.size(1) + 255) / 256 * 256);
   auto out = o.slice(2, 0, d).to(q.scalar_type()).contiguous();
   auto den = o.select(2, d).contiguous();
   auto go = grad_output.to(q.scalar_type()).contiguous();
