@@ -13,9 +13,9 @@ static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 // 8.2 at 4096 per step for 8 heads of 65536 tokens): a chunk's state is as large as its tokens, so fewer, larger
 // chunks mean fewer states to build, scan and convert.  First order, causal: a state is d + 1 rows (17 KB at
 // d = 64 against 131 KB of tokens in 512), so a short chunk wins -- what a token costs there is its own chunk in score
-// form (256 heads x 4096, d = 64, bf16: 1.91 ms at 256, 1.80 at 512, 1.97 at 1024, 2.41 at 2048; float32 at d = 32,
-// 8 heads x 4096: 0.31, 0.42, 0.64, 1.06).  First order, unmasked: there is no in-chunk part and every chunk only
-// adds a state to sum.
+// form (256 heads x 4096, bf16, ms: d = 64 1.30 at 256 and 512, with separate read-outs 1.97 at 1024 and 2.41 at 2048;
+// d = 128 4.19, 3.65, 3.79, 4.60; float32 at d = 32, 8 heads x 4096: 0.31, 0.42, 0.64, 1.06).  First order, unmasked:
+// there is no in-chunk part and every chunk only adds a state to sum.
 int moments_chunk(const fastmax_problem& p) {
   int L = p.chunk > 0 ? p.chunk : (p.p == 1 && p.mask ? (p.dtype == FASTMAX_BF16 ? 512 : 256) : 2048);
   L = (L + 255) / 256 * 256;

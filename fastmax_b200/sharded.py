@@ -270,7 +270,7 @@ def fastmax_sequence_parallel(q, k, v, *, mask=True, normalize=False, a0=1.0, a1
     (CUDA, float32 or bfloat16).
 
     Rank r of ``group`` must hold tokens ``[r*n_local, (r+1)*n_local)``, the same ``n_local`` on every rank
-    (chunks of ``chunk`` tokens, default 2048, are laid out from the start of each shard).  Differentiable;
+    (chunks of ``chunk`` tokens, by default 2048 for p = 2 and 256 to 512 for causal p = 1, are laid out from the start of each shard).  Differentiable;
     gradients come back sharded the same way.
     """
     if backend is None:

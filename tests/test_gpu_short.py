@@ -60,3 +60,21 @@ def test_grouped_heads_against_expanded_heads(mask):
     assert _cabi.device_status() == 0
     for a, b, name in zip(res["dense_tc"], res["dense_ffma"], ("out", "dq", "dk", "dv")):
         assert float((a.float() - b.float()).abs().max() / b.float().abs().max()) < 2e-2, name
+
+
+def test_first_order_shards_read_the_base_of_earlier_shards():
+    """Two sequence shards one after the other: the second one's chunks start from the first one's total."""
+    from fastmax_b200.sharded import CudaShardBackend
+    g = torch.Generator(device="cuda").manual_seed(5)
+    bh, nl = 3, 640
+    q, k, v = [torch.randn(bh, 2 * nl, 64, generator=g, device="cuda").bfloat16() for _ in range(3)]
+    want, wden, _ = _cabi.forward(q, k, v, mask=True, normalize=True, p=1, impl="dense_ffma")
+    be = CudaShardBackend(normalize=True, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=1, chunk=256)
+    sh = lambda t, r: t[:, r * nl:(r + 1) * nl].contiguous()  # noqa: E731
+    st = torch.stack([be.rowmax(sh(q, r), sh(k, r), r * nl) for r in range(2)]).max(0).values
+    kv = [be.kv_state(sh(k, r), sh(v, r)) for r in range(2)]
+    outs = [be.forward(sh(q, r), sh(k, r), sh(v, r), st, kv[r][0], kv[0][1] if r else None) for r in range(2)]
+    assert _cabi.device_status() == 0
+    out, den = torch.cat([o for o, _ in outs], 1), torch.cat([d for _, d in outs], 1)
+    assert float((out.float() - want.float()).abs().max() / want.float().abs().max()) < 2e-2
+    assert float((den - wden).abs().max() / wden.abs().max()) < 1e-2
