@@ -615,6 +615,9 @@ def roofline_of(per, cfg, bh, peaks, lib_version, chunk=0):
         achieved = flops / (ms * 1e-3) / 1e12
         if dt == "bf16":
             peak, src, bound = peaks["bf16_tflops_sustained"], peaks["source"] + " (sustained cuBLAS bf16)", "tensor"
+        elif dom.startswith("fm_dense_split"):   # float32 operands as three bf16 parts: six bf16 products each
+            peak = peaks["bf16_tflops_sustained"] / 6
+            src, bound = peaks["source"] + " (sustained cuBLAS bf16) / 6 products", "tensor"
         else:
             peak, src, bound = FFMA_TFLOPS_NOMINAL, "nominal FP32 FFMA at the maximum SM clock (no measured figure)", "fp32-ffma"
         traffic = None
