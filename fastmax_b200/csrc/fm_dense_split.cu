@@ -711,12 +711,14 @@ size_t parts_bytes(const fastmax_problem& p, int heads, int n) { return up256((s
 
 }  // namespace
 
-// float32, d 32 or 64: every problem of these types, as the default of the float32 score family and of the chunks
-// of the float32 moment family (the families that name the CUDA cores, FASTMAX_IMPL_DENSE_FFMA and _MOMENTS_FFMA,
-// stay on them).
+// float32, d 32 or 64, as the default of the float32 score family and of the chunks of the float32 moment family (the
+// families that name the CUDA cores, FASTMAX_IMPL_DENSE_FFMA and _MOMENTS_FFMA, stay on them).  The parts take one and a
+// half times the memory of the tensors they are made of.  Problems whose parts would need more than 48 GiB -- tensors of
+// 8 GB each, eight of which autograd and the caller hold -- stay on the CUDA cores, so that what fitted a device without
+// a workspace still does.
 bool dense_split_supports(const fastmax_problem& p) {
-  return (p.impl == FASTMAX_IMPL_AUTO || p.impl == FASTMAX_IMPL_MOMENTS) && p.dtype == FASTMAX_F32 && (p.d == 32 || p.d == 64) &&
-         p.bhkv > 0 && p.nq > 0 && p.nk > 0;
+  return (p.impl == FASTMAX_IMPL_AUTO || p.impl == FASTMAX_IMPL_MOMENTS) && p.dtype == FASTMAX_F32 &&
+         (p.d == 32 || p.d == 64) && p.bhkv > 0 && p.nq > 0 && p.nk > 0 && dense_split_bwd_bytes(p) <= (size_t)48 << 30;
 }
 
 // Workspace: forward [q | k | v], backward [q | k | v | gs | dvec], parts of 3 d bf16 per row.
