@@ -322,6 +322,12 @@ static size_t kept_bytes(const fastmax_problem& p) {
 static bool keeps_total(const fastmax_problem& p, int impl) {
   return impl == FASTMAX_IMPL_MOMENTS && kept_bytes(p) > 0;
 }
+// Where in a stats buffer they lie; null where nothing is kept, in the forward and in the backward alike.  The states
+// are read 16 bytes at a time; the statistic words alone may lie at any multiple of 8.
+static float* kept_states(const fastmax_problem& p, int impl, const void* stats) {
+  if (!stats || ((uintptr_t)stats & 15) || !keeps_total(p, impl)) return nullptr;
+  return (float*)((char*)const_cast<void*>(stats) + stats_words_bytes(p));
+}
 
 size_t fastmax_b200_stats_bytes(const fastmax_problem* p) {
   if (!p || p->bh < 0 || p->bhkv < 0) return 0;
@@ -395,16 +401,15 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   Ctx c{p, (cudaStream_t)stream};
   c.out_heads = heads_per_batch;
   if (p.normalize && (rc = launch_rowmax(c, q, k, (stat_t*)stats))) return rc;
-  if (first_unaligned) {
-    // a backward call whose tensors are aligned (copies of these) still finds the states it expects
-    if (stats && keeps_total(p, impl)) {
-      float* keep = (float*)((char*)stats + stats_words_bytes(p));
-      const int L = moments_chunk(p);
-      if ((rc = moments_chunk_state(c, p.bh, p.nk, L, k, v, nullptr, nullptr, 0, keep))) return rc;
-      if ((rc = moments_prefix(c, p.bh, (p.nk + L - 1) / L, keep, nullptr, nullptr, 0, 1))) return rc;
-    }
-    return dense_ffma_forward(c, q, k, v, (const stat_t*)stats, o);
-  }
+  // The backward picks its family from the problem alone.  Where that is the moment family and this forward is not on
+  // it (the packed layout, unaligned tensors), the states it will look for behind the statistics are left all the same.
+  int plain = impl;
+  if (o.out_f32 && (rc = pick_impl(p, false, &plain))) return rc;
+  float* keep = kept_states(p, plain, stats);
+  if ((o.out_f32 || first_unaligned) && keep &&
+      (rc = moments_leave_states(c, k, v, aligned16({k, v}), workspace, workspace_bytes, keep)))
+    return rc;
+  if (first_unaligned) return dense_ffma_forward(c, q, k, v, (const stat_t*)stats, o);
   if (impl == FASTMAX_IMPL_MOMENTS) {
     const MomFwdWs w = moments_fwd_layout(p);
     const size_t need = w.split;
@@ -412,7 +417,6 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
     if (!workspace || workspace_bytes < need)
       return fail(FASTMAX_E_WORKSPACE, "forward workspace too small: need %zu bytes, got %zu", need,
                   workspace_bytes);
-    float* keep = (stats && keeps_total(p, impl)) ? (float*)((char*)stats + stats_words_bytes(p)) : nullptr;
     return moments_forward(c, q, k, v, (const stat_t*)stats, o, workspace, keep);
   }
   if (impl == FASTMAX_IMPL_DENSE_TC)
@@ -483,9 +487,7 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
     if (use_split(p, mw.bytes, workspace, workspace_bytes, {q, k, v, out, grad_out, grad_q, grad_k, grad_v}))
       c.split_ws = (char*)workspace + mw.split;
     return moments_backward(c, q, k, v, out, den, (const stat_t*)stats, grad_out, grad_q, grad_k, grad_v,
-                            workspace,
-                            (stats && keeps_total(p, impl)) ? (const float*)((const char*)stats + stats_words_bytes(p))
-                                                            : nullptr);
+                            workspace, kept_states(p, impl, stats));
   }
   float* dots = (float*)((char*)workspace + w.dots_off);
   float* delta = (float*)((char*)workspace + w.delta_off);

@@ -282,6 +282,8 @@ MomFwdWs moments_fwd_layout(const fastmax_problem& p);
 MomBwdWs moments_bwd_layout(const fastmax_problem& p);
 int moments_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                     const FwdOut& o, void* workspace, float* total_keep = nullptr);
+int moments_leave_states(const Ctx& c, const void* k, const void* v, bool aligned, void* workspace,
+                         size_t workspace_bytes, float* total_keep);
 int moments_forward_finish(const Ctx& c, const void* q, const void* k, const void* v,
                            const stat_t* stats, float* kv_states, const float* s_base,
                            float* o_add, float* den_add, void* s16, const FwdOut& o,

@@ -251,6 +251,28 @@ int moments_forward(const Ctx& c, const void* q, const void* k, const void* v, c
   return moments_forward_total(c, q, stats, total, o_add, den_add, s16, o);
 }
 
+// What moments_forward leaves at total_keep, for a forward of another family.  The tensor-core state kernels read k and
+// v by TMA, so unaligned tensors take the CUDA-core ones.  Unmasked, the chunk states need a workspace; without one
+// the total is summed as a single chunk, in less parallel but next to a forward that is quadratic in the length.
+int moments_leave_states(const Ctx& c, const void* k, const void* v, bool aligned, void* workspace,
+                         size_t workspace_bytes, float* total_keep) {
+  const fastmax_problem& p = c.p;
+  const int L = moments_chunk(p), nchunk = (p.nk + L - 1) / L;
+  const size_t need = moment_state_bytes(p, p.nk);
+  const bool room = workspace && workspace_bytes >= need && ((uintptr_t)workspace & 15) == 0;
+  if (!p.mask && !room) return moments_chunk_state(c, p.bh, p.nk, p.nk, k, v, nullptr, nullptr, 0, total_keep);
+  float* states = p.mask ? total_keep : (float*)workspace;
+  int rc;
+  if (aligned)
+    rc = moments_build_states(p.mask ? skipping(c, nchunk - 1) : c, p.nk, k, v, nullptr, nullptr, 0, nullptr, nullptr, states);
+  else
+    rc = moments_chunk_state(c, p.bh, p.nk, L, k, v, nullptr, nullptr, 0, states);
+  if (rc) return rc;
+  if (!p.mask) return moments_prefix(c, p.bh, nchunk, states, nullptr, total_keep, 0, 0);
+  bool ready;
+  return prefix_states(c, nchunk, states, nullptr, 0, true, (char*)total_keep + need, &ready);
+}
+
 // Unmasked forward from a given total state (this device's keys, or the sum over all shards).
 int moments_forward_total(const Ctx& c, const void* q, const stat_t* stats, const float* total, float* o_add,
                           float* den_add, void* s16, const FwdOut& o) {

@@ -175,7 +175,12 @@ int fastmax_b200_backward_bt(const fastmax_problem* prob,
 /* Forward pass in the reference's packed layout: o is (bh, nq, d+1) float32
  * whose channels 0..d-1 hold the divided output and channel d the denominator
  * (reference fastmax_cuda_forward.cu:347, 199-210; the reference wrapper
- * slices o[:, :, :d], example.py:47).  stats may be NULL when normalize == 0. */
+ * slices o[:, :, :d], example.py:47).  stats may be NULL when normalize == 0.
+ * The layout is written by the score form at any length; for problems whose
+ * plain-layout calls run on the moment family it also leaves the states in
+ * stats that fastmax_b200_backward will look for there.  float32 with d 32 or 64
+ * runs on the tensor cores when given a workspace of
+ * fastmax_b200_forward_workspace_bytes, on the CUDA cores without one. */
 int fastmax_b200_forward_packed(const fastmax_problem* prob,
                                 const void* q, const void* k, const void* v,
                                 float* o_packed, void* stats,
