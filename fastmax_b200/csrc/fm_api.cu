@@ -109,7 +109,7 @@ static int check_device() {
 // number of keys a row sees, the moment form is constant plus its own chunk in score form.
 static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   if (!moments_supports(p)) return false;
-  if (p.p == 1 && p.mask && (p.d == 64 || (tc_ok && p.d == 128) || (!tc_ok && p.d == 32 && p.dtype == FASTMAX_F32))) {
+  if (first_order_measured(p)) {
     // First order, causal.  The score form's time per token and head grows by `slope` ns per token of length (a line
     // through its measured times), the moment form's is flat; they meet at `meet` tokens.  The moment form's extra
     // launches cost some 30 us of host time, so what it saves has to exceed that.  Measured per step, score / moment:
@@ -132,8 +132,8 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   // 9216: 22.6 / 23.0; 10000: 60.9 / 54.5).
   // float32 (fm_dense_split.cu, moment states on the CUDA cores), per token and head and step: the score form takes
   // 4.2 / 5.8 ps per key at d = 32 / 64, the states and read-outs 4.5 / 10.5 ns at p = 1 (256 heads of 1024 tokens)
-  // and 25 / 190 ns at p = 2, so the moment family starts near 2 400 / 3 900 causal keys at p = 1 and 12 000 /
-  // 65 000 at p = 2.
+  // and 25 / 190 ns at p = 2, so the moment family starts near 2 064 / 2 928 unmasked keys at p = 1 and, at p = 2,
+  // 8 160 unmasked and 13 500 causal keys at d = 32 and beyond 20 000 at d = 64.
   const bool split = dense_split_supports(p);
   const double rate_score = tc_ok ? 800e12 : (split ? (p.d == 32 ? 108e12 : 156e12) : 25e12);
   const double rate_first = first_tc_supports(p) ? 450e12 : (split ? (p.d == 32 ? 3.3e12 : 5.5e12) : 20e12);

@@ -9,6 +9,14 @@ namespace fm {
 
 static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
+// Causal first-order problems whose chunk length and whose line to the score form were measured: bf16 with every kernel
+// on the tensor cores and float32 with the split score kernels.  The other shapes (float32 at d 8, 16 and 128 or too
+// large for the split kernels' operands, bf16 up to d = 32) run their states on the CUDA cores, whose cost per chunk
+// nobody measured at short chunks; they keep chunks of 2048 and the rate model of moments_faster.
+bool first_order_measured(const fastmax_problem& p) {
+  return p.p == 1 && p.mask && (p.dtype == FASTMAX_BF16 ? first_tc_supports(p) : dense_split_supports(p));
+}
+
 // Tokens per chunk.  Second order: 2048, measured best for the tensor-core kernels (8.9 ms at 1024, 7.8 at 2048,
 // 8.2 at 4096 per step for 8 heads of 65536 tokens): a chunk's state is as large as its tokens, so fewer, larger
 // chunks mean fewer states to build, scan and convert.  First order, causal: a state is d + 1 rows (17 KB at
@@ -17,7 +25,7 @@ static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 // d = 128 4.19, 3.65, 3.79, 4.60; float32 at d = 32, 8 heads x 4096: 0.31, 0.42, 0.64, 1.06).  First order, unmasked:
 // there is no in-chunk part and every chunk only adds a state to sum.
 int moments_chunk(const fastmax_problem& p) {
-  int L = p.chunk > 0 ? p.chunk : (p.p == 1 && p.mask ? (p.dtype == FASTMAX_BF16 ? 512 : 256) : 2048);
+  int L = p.chunk > 0 ? p.chunk : (first_order_measured(p) ? (p.dtype == FASTMAX_BF16 ? 512 : 256) : 2048);
   L = (L + 255) / 256 * 256;
   return L;
 }

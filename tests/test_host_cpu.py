@@ -75,6 +75,25 @@ def test_family_selection_follows_the_measured_break_even_points():
         pick(impl=_cabi.IMPL["dense_tc"], dtype=_cabi.F32, d=32)
 
 
+FIRST_ORDER_LINES = [   # dtype, d, heads, longest length in score form, shortest on the moment family
+    (_cabi.BF16, 64, 256, 1216, 1248), (_cabi.BF16, 64, 8, 3520, 3552), (_cabi.BF16, 128, 256, 2800, 2832),
+    (_cabi.F32, 32, 256, 3120, 3152), (_cabi.F32, 64, 256, 3952, 3984),
+    # shapes whose states run on the CUDA cores: nothing below one default chunk of 2048
+    (_cabi.F32, 8, 256, 2048, 2064), (_cabi.F32, 16, 256, 2064, 2080), (_cabi.F32, 128, 256, 2208, 2224),
+    (_cabi.BF16, 8, 256, 2048, 2064), (_cabi.BF16, 16, 256, 2064, 2080), (_cabi.BF16, 32, 256, 2080, 2096),
+    # operand parts above 48 GiB: no split kernels, so the line of the CUDA-core kernels
+    (_cabi.F32, 64, 40000, 2128, 2144)]
+
+
+@pytest.mark.parametrize("dtype,d,heads,below,above", FIRST_ORDER_LINES)
+def test_causal_first_order_lines_between_the_families(dtype, d, heads, below, above):
+    def pick(n):
+        return _cabi.selected_impl(_cabi.Problem(dtype=dtype, bh=heads, bhkv=heads, nq=n, nk=n, d=d, mask=1, normalize=1,
+                                                 p=1, impl=0, a0=1, a1=1, a2=0.5, lim=1, temperature=1))
+    dense = "dense_tc" if dtype == _cabi.BF16 and d >= 64 else "dense_ffma"
+    assert [pick(n) for n in (272, 600, below, above, 4 * above)] == [dense] * 3 + ["moments"] * 2
+
+
 def test_bad_arguments_are_rejected_before_any_launch():
     L = _cabi.lib()
     prob = _cabi.Problem(dtype=0, bh=2, bhkv=2, nq=4, nk=4, d=32, mask=1, normalize=0, p=3, impl=0,
