@@ -166,7 +166,7 @@ static int pick_impl(const fastmax_problem& p, bool packed, int* impl) {
   if (want == FASTMAX_IMPL_MOMENTS || want == FASTMAX_IMPL_MOMENTS_FFMA) {
     if (!moments_supports(p) || packed)
       return fail(FASTMAX_E_UNSUPPORTED,
-                  "the moment family needs bh == bhkv, nq == nk when causal, and the plain output layout");
+                  "the moment family needs bh == bhkv <= 65535, nq == nk when causal, and the plain output layout");
     *impl = FASTMAX_IMPL_MOMENTS;   // callers branch on the family; the state kernels look at p.impl
     return FASTMAX_OK;
   }
@@ -537,8 +537,8 @@ int fastmax_b200_backward_bt(const fastmax_problem* prob, const void* q, const v
 static int validate_shard(const fastmax_problem* prob) {
   int rc = validate(prob);
   if (rc) return rc;
-  if (prob->nq != prob->nk || prob->bh != prob->bhkv)
-    return fail(FASTMAX_E_ARG, "a sequence shard needs nq == nk and bh == bhkv");
+  if (prob->nq != prob->nk || prob->bh != prob->bhkv || prob->bh > 65535)
+    return fail(FASTMAX_E_ARG, "a sequence shard needs nq == nk and bh == bhkv <= 65535");
   return check_device();
 }
 static size_t shard_s16_bytes(const fastmax_problem& p) { return state16_bytes(p, p.nq); }

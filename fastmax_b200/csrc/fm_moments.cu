@@ -61,8 +61,10 @@ bool moments_all_tc(const fastmax_problem& p) {
   return dense_tc_supports(p) && first_tc_supports(p) && (p.p == 1 || moments_tc_supports(p));
 }
 
+// Heads are the y or z dimension of several of the family's grids, which ends at 65535; the score families have
+// one-dimensional grids.
 bool moments_supports(const fastmax_problem& p) {
-  return p.bh == p.bhkv && (!p.mask || p.nq == p.nk);
+  return p.bh == p.bhkv && p.bh <= 65535 && (!p.mask || p.nq == p.nk);
 }
 
 // Workspace of the one-call forward: [states][total][o_add][den_add]

@@ -94,6 +94,15 @@ def test_causal_first_order_lines_between_the_families(dtype, d, heads, below, a
     assert [pick(n) for n in (272, 600, below, above, 4 * above)] == [dense] * 3 + ["moments"] * 2
 
 
+@pytest.mark.parametrize("dtype,d,n,mask,chunk", [(_cabi.BF16, 64, 1100, 1, 0), (_cabi.BF16, 64, 8000, 0, 0), (_cabi.F32, 8, 300, 1, 256)])
+def test_more_heads_than_a_grid_dimension_stay_in_score_form(dtype, d, n, mask, chunk):
+    def pick(heads):
+        return _cabi.selected_impl(_cabi.Problem(dtype=dtype, bh=heads, bhkv=heads, nq=n, nk=n, d=d, mask=mask, normalize=1,
+                                                 p=1, impl=0, a0=1, a1=1, a2=0.5, lim=1, temperature=1, chunk=chunk))
+    assert pick(65535) == "moments"
+    assert pick(65536) == pick(70000) == ("dense_tc" if dtype == _cabi.BF16 else "dense_ffma")
+
+
 def test_bad_arguments_are_rejected_before_any_launch():
     L = _cabi.lib()
     prob = _cabi.Problem(dtype=0, bh=2, bhkv=2, nq=4, nk=4, d=32, mask=1, normalize=0, p=3, impl=0,
