@@ -67,20 +67,28 @@ bool moments_supports(const fastmax_problem& p) {
   return p.bh == p.bhkv && p.bh <= 65535 && (!p.mask || p.nq == p.nk);
 }
 
-// Workspace of the one-call forward: [states][total][o_add][den_add]
+// Causal p = 1 at d = 64: the score kernels of the chunks read the states themselves, so there is no read-out pass
+// and no fp32 rows between two kernels.
+static bool first_fused(const fastmax_problem& p) {
+  return p.p == 1 && p.mask && p.d == 64 && p.nq == p.nk && first_tc_supports(p) && dense_tc_wide_supports(p);
+}
+
+// Workspace of the one-call forward: [states][total][o_add][den_add][bf16 copies][float32 operand parts].  The fused
+// first-order path has no fp32 rows between two kernels and no total (256 heads x 2048, bf16: 27 MB instead of 167).
 MomFwdWs moments_fwd_layout(const fastmax_problem& p) {
   MomFwdWs w;
   w.states = 0;
   w.total = w.states + moment_state_bytes(p, p.nk);
-  w.o_add = w.total + moment_total_bytes(p);
-  w.den_add = w.o_add + up256(sizeof(float) * (size_t)p.bh * p.nq * p.d);
-  w.s16 = w.den_add + up256(sizeof(float) * (size_t)p.bh * p.nq);
+  const size_t rows = first_fused(p) ? 0 : (size_t)p.bh * p.nq;
+  w.o_add = w.total + (rows ? moment_total_bytes(p) : 0);
+  w.den_add = w.o_add + up256(sizeof(float) * rows * p.d);
+  w.s16 = w.den_add + up256(sizeof(float) * rows);
   w.split = w.s16 + state16_bytes(p, p.nk);
   w.bytes = w.split + (p.mask && dense_split_supports(p) ? dense_split_fwd_bytes(p) : 0);
   return w;
 }
 // Workspace of the one-call backward:
-// [dots][delta][dvec][gs][states][total][gq_add][gk_add][gv_add]
+// [dots][delta][dvec][gs][states][total][gq_add][gk_add][gv_add][bf16 copies][float32 operand parts]
 MomBwdWs moments_bwd_layout(const fastmax_problem& p) {
   MomBwdWs w;
   w.dots = 0;
@@ -89,10 +97,11 @@ MomBwdWs moments_bwd_layout(const fastmax_problem& p) {
   w.gs = w.dvec + up256(sizeof(float) * (size_t)p.bh * p.nq);
   w.states = w.gs + (dense_tc_supports(p) ? up256((size_t)2 * p.bh * p.nq * p.d) : 0);
   w.total = w.states + moment_state_bytes(p, p.nk > p.nq ? p.nk : p.nq);
-  w.gq_add = w.total + moment_total_bytes(p);
-  w.gk_add = w.gq_add + up256(sizeof(float) * (size_t)p.bh * p.nq * p.d);
-  w.gv_add = w.gk_add + up256(sizeof(float) * (size_t)p.bhkv * p.nk * p.d);
-  w.s16 = w.gv_add + up256(sizeof(float) * (size_t)p.bhkv * p.nk * p.d);
+  const bool fused = first_fused(p);    // as in the forward: 98 MB instead of 505
+  w.gq_add = w.total + (fused ? 0 : moment_total_bytes(p));
+  w.gk_add = w.gq_add + (fused ? 0 : up256(sizeof(float) * (size_t)p.bh * p.nq * p.d));
+  w.gv_add = w.gk_add + (fused ? 0 : up256(sizeof(float) * (size_t)p.bhkv * p.nk * p.d));
+  w.s16 = w.gv_add + (fused ? 0 : up256(sizeof(float) * (size_t)p.bhkv * p.nk * p.d));
   w.split = w.s16 + state16_bytes(p, p.nk > p.nq ? p.nk : p.nq);
   w.bytes = w.split + (p.mask && dense_split_supports(p) ? dense_split_bwd_bytes(p) : 0);
   return w;
@@ -167,12 +176,6 @@ static int read_first_final(const Ctx& c, int type_b, int n, const void* tile, c
   if ((rc = first_tc_convert(c, c.p.bh, total, s16))) return rc;
   return first_tc_readout(c, type_b, c.p.bh, n, moments_chunk(c.p), 0, tile, x, uvec, total, s16, stats, nullptr,
                           nullptr, 0, final, out, den_out, dots);
-}
-
-// Causal p = 1 at d = 64: the score kernels of the chunks read the states themselves, so there is no read-out pass
-// and no fp32 rows between two kernels.
-static bool first_fused(const fastmax_problem& p) {
-  return p.p == 1 && p.mask && p.d == 64 && p.nq == p.nk && first_tc_supports(p) && dense_tc_wide_supports(p);
 }
 
 // Exclusive running sums over the chunks of every head (per-chunk mode).  With `fuse` and the tensor-core

@@ -1,5 +1,6 @@
-"""Workspace sizes of the float32 score kernels (host arithmetic, no device): the operand parts take 6 bytes per element;
-very large problems and the families that name the CUDA cores need none, as before."""
+"""Workspace sizes (host arithmetic, no device).  The operand parts of the float32 score kernels take 6 bytes per element;
+very large problems and the families that name the CUDA cores need none.  The fused first-order path needs room for
+its states and their bf16 copies, and backward for the scaled gradient, but for no fp32 rows."""
 import pytest
 
 from fastmax_b200 import _cabi
@@ -26,3 +27,13 @@ def test_other_problems_need_no_forward_workspace(kw):
     fwd, bwd = sizes(**kw)
     rows = kw.get("bh", 16) * kw.get("nq", 1000)
     assert fwd == 0 and bwd <= 4 * rows + 8 * kw.get("bh", 16) + 1024
+
+
+@pytest.mark.parametrize("heads,n", [(256, 2048), (256, 1233), (64, 8192)])
+def test_fused_first_order_needs_no_fp32_rows(heads, n):
+    fwd, bwd = sizes(dtype=_cabi.BF16, bh=heads, bhkv=heads, nq=n, nk=n, d=64, p=1)
+    tensor = 2 * heads * n * 64
+    # states: 65 rows of 68 floats per 512 tokens, copies: 64 x 64 bf16; a last partial chunk counts as a whole one
+    states = heads * -(-n // 512) * (65 * 68 * 4 + 64 * 64 * 2)
+    assert fwd <= states + 4096
+    assert bwd <= tensor + states + 2 * 4 * heads * n + 8 * heads + 4096
