@@ -22,6 +22,7 @@ IMPL = {"auto": 0, "dense_ffma": 1, "dense_tc": 2, "moments": 3, "moments_ffma":
 EXPORTS = (
     "fastmax_b200_version", "fastmax_b200_last_error", "fastmax_b200_stats_bytes", "fastmax_b200_selected_impl",
     "fastmax_b200_forward_workspace_bytes", "fastmax_b200_backward_workspace_bytes",
+    "fastmax_b200_forward_workspace_least_bytes", "fastmax_b200_backward_workspace_least_bytes",
     "fastmax_b200_forward", "fastmax_b200_forward_packed", "fastmax_b200_backward",
     "fastmax_b200_forward_bt", "fastmax_b200_backward_bt", "fastmax_b200_bt_layout_supported",
     "fastmax_b200_launch_count", "fastmax_b200_profile_enable", "fastmax_b200_profile_count",
@@ -63,7 +64,8 @@ def lib() -> ctypes.CDLL:
         vp, sz, pp = ctypes.c_void_p, ctypes.c_size_t, ctypes.POINTER(Problem)
         L.fastmax_b200_version.restype = ctypes.c_int
         L.fastmax_b200_last_error.restype = ctypes.c_char_p
-        for f in ("stats_bytes", "forward_workspace_bytes", "backward_workspace_bytes"):
+        for f in ("stats_bytes", "forward_workspace_bytes", "backward_workspace_bytes", "forward_workspace_least_bytes",
+                  "backward_workspace_least_bytes"):
             fn = getattr(L, "fastmax_b200_" + f)
             fn.restype, fn.argtypes = sz, [pp]
         L.fastmax_b200_selected_impl.restype = ctypes.c_int
@@ -219,12 +221,18 @@ def _on(device):
 
 @functools.lru_cache(maxsize=256)
 def _plan(dtype, bh, bhkv, nq, nk, d, mask, normalize, p, impl, a0, a1, a2, lim, temperature, chunk):
-    """(problem, forward workspace, backward workspace, stats bytes) of one problem: host arithmetic that depends
-    on nothing but these values."""
+    """(problem, forward workspace, backward workspace, stats bytes) of one problem, a workspace as (wanted, least)
+    bytes: host arithmetic that depends on nothing but these values."""
     L = lib()
     prob = Problem(dtype, bh, bhkv, nq, nk, d, mask, normalize, p, impl, a0, a1, a2, lim, temperature, chunk)
-    return (prob, L.fastmax_b200_forward_workspace_bytes(prob), L.fastmax_b200_backward_workspace_bytes(prob),
+    return (prob, _forward_sizes(prob),
+            (L.fastmax_b200_backward_workspace_bytes(prob), L.fastmax_b200_backward_workspace_least_bytes(prob)),
             max(L.fastmax_b200_stats_bytes(prob), 8))
+
+
+def _forward_sizes(prob):
+    L = lib()
+    return L.fastmax_b200_forward_workspace_bytes(prob), L.fastmax_b200_forward_workspace_least_bytes(prob)
 
 
 def _heads_of(t):
@@ -234,13 +242,22 @@ def _heads_of(t):
 def _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk):
     if p not in (1, 2):
         raise ValueError(f"p must be 1 or 2, got: {p}")
-    return _plan(_dtype_code(q), _heads_of(q), _heads_of(k), q.shape[-2], k.shape[-2], q.shape[-1], int(bool(mask)), int(bool(normalize)), int(p),
+    return _plan(_dtype_code(q), _heads_of(q), _heads_of(k), q.shape[-2], k.shape[-2], q.shape[-1], int(bool(mask)),
+                 int(bool(normalize)), int(p),
                  IMPL[impl] if isinstance(impl, str) else int(impl), float(a0), float(a1), float(a2), float(lim),
                  float(temperature), int(chunk))
 
 
-def _workspace(nbytes: int, device) -> torch.Tensor:
-    return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
+def _workspace(sizes, device) -> torch.Tensor:
+    """Scratch of the wanted size, or of the least the call runs with -- more slowly -- where the device has no room
+    for more (float32: without the operand parts of the tensor-core kernels, on the CUDA cores)."""
+    want, least = sizes
+    try:
+        return torch.empty(max(want, 1), dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        if least >= want:
+            raise
+    return torch.empty(max(least, 1), dtype=torch.uint8, device=device)
 
 
 def forward(q, k, v, *, mask, normalize, temperature=1.0, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=2,
@@ -257,19 +274,20 @@ def forward_any(q, k, v, mask, normalize, temperature, a0, a1, a2, lim, p, impl=
     """``forward`` on contiguous (b*h, n, d) or (b, h, n, d) tensors; out has q's shape."""
     _require_any(q, k, v)
     L = lib()
-    prob, wsb, _, stats_bytes = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    prob, sizes, _, stats_bytes = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
     with _on(q.device):
         if buffers is None:
             out = torch.empty_like(q)
             den = torch.empty(prob.bh, prob.nq, dtype=torch.float32, device=q.device)
             stats = torch.empty(stats_bytes, dtype=torch.uint8, device=q.device)
-            ws = _workspace(wsb, q.device) if wsb else None
+            ws = _workspace(sizes, q.device) if sizes[0] else None
         else:
             out, den, stats, ws = buffers["out"], buffers["den"], buffers["stats"], buffers["workspace"]
-            if ws.numel() < wsb:
+            if ws.numel() < sizes[1]:
                 raise ValueError("preallocated forward workspace is too small")
         rc = L.fastmax_b200_forward(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                    den.data_ptr(), stats.data_ptr(), _ptr(ws), wsb, _stream(q))
+                                    den.data_ptr(), stats.data_ptr(), _ptr(ws), 0 if ws is None else ws.numel(),
+                                    _stream(q))
     _check(rc, "fastmax_b200_forward")
     return out, den, stats
 
@@ -288,16 +306,16 @@ def forward_bt(q, k, v, heads_per_batch, *, mask, normalize, temperature=1.0, a0
     takes after a ``view`` -- written in that layout by the attention kernel itself."""
     _require(q, k, v)
     L = lib()
-    prob, wsb, _, stats_bytes = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    prob, sizes, _, stats_bytes = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
     bh, nq, d = q.shape
     with _on(q.device):
         out = torch.empty(bh // heads_per_batch, nq, heads_per_batch, d, dtype=q.dtype, device=q.device)
         den = torch.empty(bh, nq, dtype=torch.float32, device=q.device)
         stats = torch.empty(stats_bytes, dtype=torch.uint8, device=q.device)
-        ws = _workspace(wsb, q.device)
+        ws = _workspace(sizes, q.device)
         rc = L.fastmax_b200_forward_bt(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                       den.data_ptr(), stats.data_ptr(), int(heads_per_batch), ws.data_ptr(), wsb,
-                                       _stream(q))
+                                       den.data_ptr(), stats.data_ptr(), int(heads_per_batch), ws.data_ptr(),
+                                       ws.numel(), _stream(q))
     _check(rc, "fastmax_b200_forward_bt")
     return out, den, stats
 
@@ -310,14 +328,14 @@ def backward_bt(q, k, v, out_bt, den, stats, grad_out_bt, heads_per_batch, *, ma
         if t.device != q.device or t.dtype != q.dtype or not t.is_contiguous() or t.numel() != q.numel():
             raise ValueError("out and grad_out must be contiguous (batch, nq, heads, d) tensors of q's dtype")
     L = lib()
-    prob, _, wsb, _ = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    prob, _, sizes, _ = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
     with _on(q.device):
         gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        ws = _workspace(wsb, q.device)
+        ws = _workspace(sizes, q.device)
         rc = L.fastmax_b200_backward_bt(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out_bt.data_ptr(),
                                         den.data_ptr(), stats.data_ptr(), grad_out_bt.data_ptr(),
                                         int(heads_per_batch), gq.data_ptr(), gk.data_ptr(), gv.data_ptr(),
-                                        ws.data_ptr(), wsb, _stream(q))
+                                        ws.data_ptr(), ws.numel(), _stream(q))
     _check(rc, "fastmax_b200_backward_bt")
     return gq, gk, gv
 
@@ -331,10 +349,9 @@ def forward_packed(q, k, v, *, mask, normalize, temperature=1.0, a0=1.0, a1=1.0,
     with torch.cuda.device(q.device):
         o = torch.empty(q.shape[0], q.shape[1], q.shape[2] + 1, dtype=torch.float32, device=q.device)
         stats = torch.empty(max(L.fastmax_b200_stats_bytes(prob), 8), dtype=torch.uint8, device=q.device)
-        wsb = L.fastmax_b200_forward_workspace_bytes(prob)
-        ws = _workspace(wsb, q.device)
+        ws = _workspace(_forward_sizes(prob), q.device)
         rc = L.fastmax_b200_forward_packed(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
-                                           stats.data_ptr(), ws.data_ptr(), wsb, _stream(q))
+                                           stats.data_ptr(), ws.data_ptr(), ws.numel(), _stream(q))
     _check(rc, "fastmax_b200_forward_packed")
     return o, stats
 
@@ -358,6 +375,14 @@ def workspace_bytes(q, k, **kw):
             max(L.fastmax_b200_stats_bytes(prob), 8))
 
 
+def shared_workspace_sizes(q, k, **kw):
+    """((wanted, least) bytes of one workspace for both passes, stats bytes) for a problem of these shapes."""
+    _, fwd, bwd, stats = _plan_of(q, k, kw["mask"], kw["normalize"], kw.get("temperature", 1.0), kw.get("a0", 1.0),
+                                  kw.get("a1", 1.0), kw.get("a2", 0.5), kw.get("lim", 1.0), kw.get("p", 2),
+                                  kw.get("impl", "auto"), kw.get("chunk", 0))
+    return (max(fwd[0], bwd[0]), max(fwd[1], bwd[1])), stats
+
+
 def backward(q, k, v, out, den, stats, grad_out, *, mask, normalize, temperature=1.0, a0=1.0, a1=1.0,
              a2=0.5, lim=1.0, p=2, impl="auto", chunk=0, buffers=None):
     """Gradients (grad_q, grad_k, grad_v) in the dtype of the inputs; ``buffers`` as in ``forward``
@@ -372,19 +397,19 @@ def backward_any(q, k, v, out, den, stats, grad_out, mask, normalize, temperatur
     """``backward`` for ``forward_any``'s tensors."""
     _require_any(q, k, v, out, grad_out)
     L = lib()
-    prob, _, wsb, _ = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
+    prob, _, sizes, _ = _plan_of(q, k, mask, normalize, temperature, a0, a1, a2, lim, p, impl, chunk)
     with _on(q.device):
         if buffers is None:
             gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-            ws = _workspace(wsb, q.device)
+            ws = _workspace(sizes, q.device)
         else:
             gq, gk, gv, ws = buffers["grad_q"], buffers["grad_k"], buffers["grad_v"], buffers["workspace"]
-            if ws.numel() < wsb:
+            if ws.numel() < sizes[1]:
                 raise ValueError("preallocated backward workspace is too small")
         rc = L.fastmax_b200_backward(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                                      den.data_ptr(), stats.data_ptr(), grad_out.data_ptr(),
-                                     gq.data_ptr(), gk.data_ptr(), gv.data_ptr(), ws.data_ptr(), wsb,
-                                     _stream(q))
+                                     gq.data_ptr(), gk.data_ptr(), gv.data_ptr(), ws.data_ptr(),
+                                     ws.numel(), _stream(q))
     _check(rc, "fastmax_b200_backward")
     return gq, gk, gv
 

@@ -209,7 +209,6 @@ static BwdWs bwd_layout(const fastmax_problem& p) {
   if (dense_tc_supports(p)) w.total += align_up((size_t)2 * p.bh * p.nq * p.d, 256);
   return w;
 }
-// the workspace must serve whichever family AUTO picks
 // Backward workspace of the split-operand float32 kernels: [dots][parts and row dots]
 static size_t split_bwd_off(const fastmax_problem& p) { return bwd_layout(p).delta_off; }
 static size_t split_bwd_bytes(const fastmax_problem& p) { return split_bwd_off(p) + dense_split_bwd_bytes(p); }
@@ -220,13 +219,16 @@ static bool use_split(const fastmax_problem& p, size_t need, const void* workspa
   return dense_split_supports(p) && workspace && workspace_bytes >= need && ((uintptr_t)workspace & 255) == 0 &&
          aligned16(ptrs);
 }
-static size_t fwd_ws_bytes(const fastmax_problem& p) {
-  return moments_supports(p) ? moments_fwd_layout(p).bytes : 0;
+// Moment family, with the operand parts or without (`least`).  The backward's also serves the score form, where
+// unaligned first-order tensors go.
+static size_t fwd_ws_bytes(const fastmax_problem& p, bool least) {
+  const MomFwdWs w = moments_fwd_layout(p);
+  return least ? w.split : w.bytes;
 }
-static size_t bwd_ws_bytes(const fastmax_problem& p) {
-  size_t a = bwd_layout(p).total;
-  if (moments_supports(p)) { size_t b = moments_bwd_layout(p).bytes; if (b > a) a = b; }
-  return a;
+static size_t bwd_ws_bytes(const fastmax_problem& p, bool least) {
+  const MomBwdWs w = moments_bwd_layout(p);
+  const size_t a = bwd_layout(p).total, b = least ? w.split : w.bytes;
+  return a > b ? a : b;
 }
 
 }  // namespace fm
@@ -347,24 +349,28 @@ int fastmax_b200_selected_impl(const fastmax_problem* p, int32_t* impl) {
   return FASTMAX_OK;
 }
 
-// Sized for the family the call will run: the moment family needs room for its states.
-size_t fastmax_b200_forward_workspace_bytes(const fastmax_problem* p) {
+// Sized for the family the call will run: the moment family needs room for its states, the float32 tensor-core kernels
+// for their operand parts -- which the `least` sizes leave out (use_split then says no).
+static size_t forward_bytes(const fastmax_problem* p, bool least) {
   if (validate(p)) return 0;
   int impl;
   if (pick_impl(*p, false, &impl)) return 0;
-  if (impl == FASTMAX_IMPL_MOMENTS) return fwd_ws_bytes(*p);
-  return impl == FASTMAX_IMPL_DENSE_FFMA && dense_split_supports(*p) ? dense_split_fwd_bytes(*p) : 0;
+  if (impl == FASTMAX_IMPL_MOMENTS) return fwd_ws_bytes(*p, least);
+  return !least && impl == FASTMAX_IMPL_DENSE_FFMA && dense_split_supports(*p) ? dense_split_fwd_bytes(*p) : 0;
 }
-
-size_t fastmax_b200_backward_workspace_bytes(const fastmax_problem* p) {
+static size_t backward_bytes(const fastmax_problem* p, bool least) {
   if (validate(p)) return 0;
   int impl;
   if (pick_impl(*p, false, &impl)) return 0;
-  if (impl == FASTMAX_IMPL_MOMENTS) return bwd_ws_bytes(*p);
+  if (impl == FASTMAX_IMPL_MOMENTS) return bwd_ws_bytes(*p, least);
   const size_t plain = bwd_layout(*p).total;
-  if (impl != FASTMAX_IMPL_DENSE_FFMA || !dense_split_supports(*p)) return plain;
+  if (least || impl != FASTMAX_IMPL_DENSE_FFMA || !dense_split_supports(*p)) return plain;
   return plain > split_bwd_bytes(*p) ? plain : split_bwd_bytes(*p);
 }
+size_t fastmax_b200_forward_workspace_bytes(const fastmax_problem* p) { return forward_bytes(p, false); }
+size_t fastmax_b200_backward_workspace_bytes(const fastmax_problem* p) { return backward_bytes(p, false); }
+size_t fastmax_b200_forward_workspace_least_bytes(const fastmax_problem* p) { return forward_bytes(p, true); }
+size_t fastmax_b200_backward_workspace_least_bytes(const fastmax_problem* p) { return backward_bytes(p, true); }
 
 // Whether a problem can take its result and upstream gradient in the (batch, n, heads, d) layout:
 // the last kernel of the forward must be a tensor-core score kernel and grad_out / out must be read

@@ -82,6 +82,17 @@ void check_rc(int rc, const char* what) {
   TORCH_CHECK(rc == FASTMAX_OK, what, " failed (code ", rc, "): ", fastmax_b200_last_error());
 }
 
+// Workspace of the wanted size, or of the least the call runs with where the device has no room for more.
+torch::Tensor scratch(size_t want, size_t least, const torch::Tensor& like) {
+  const auto opt = like.options().dtype(torch::kUInt8);
+  try {
+    return torch::empty({(int64_t)want}, opt);
+  } catch (const c10::OutOfMemoryError&) {
+    if (least >= want) throw;
+  }
+  return torch::empty({(int64_t)least}, opt);
+}
+
 // What forwardpass did, for the backwardpass that will be handed its result.
 struct FwdRecord {
   int64_t bh, bhkv, nq, nk, d;
@@ -139,9 +150,9 @@ torch::Tensor forward_impl(const torch::Tensor& q, const torch::Tensor& k, const
   size_t wsb = 0;
   if (fastmax_b200_selected_impl(&pr, &impl) == FASTMAX_OK && impl == FASTMAX_IMPL_DENSE_FFMA)
     wsb = fastmax_b200_forward_workspace_bytes(&pr);
-  auto ws = torch::empty({(int64_t)wsb}, q.options().dtype(torch::kUInt8));
+  auto ws = scratch(wsb, 0, q);
   check_rc(fastmax_b200_forward_packed(&pr, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr<float>(), stats,
-                                       ws.data_ptr(), wsb, stream),
+                                       ws.data_ptr(), ws.numel(), stream),
            "fastmax forwardpass");
   if (dropout > 0.0) {
     TORCH_CHECK(drop_noise.has_value() && drop_noise->defined(), "dropout > 0 needs drop_noise");
@@ -206,11 +217,11 @@ std::vector<torch::Tensor> backwardpass(torch::Tensor q, torch::Tensor k, torch:
   auto den = o.select(2, d).contiguous();
   auto go = grad_output.to(q.scalar_type()).contiguous();
   auto gq = torch::empty_like(q), gk = torch::empty_like(k), gv = torch::empty_like(v);
-  const size_t wsb = fastmax_b200_backward_workspace_bytes(&pr);
-  auto ws = torch::empty({(int64_t)std::max<size_t>(wsb, 1)}, q.options().dtype(torch::kUInt8));
+  auto ws = scratch(std::max<size_t>(fastmax_b200_backward_workspace_bytes(&pr), 1),
+                    fastmax_b200_backward_workspace_least_bytes(&pr), q);
   check_rc(fastmax_b200_backward(&pr, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                                  den.data_ptr<float>(), stats, go.data_ptr(), gq.data_ptr(), gk.data_ptr(),
-                                 gv.data_ptr(), ws.data_ptr(), wsb, at::cuda::getCurrentCUDAStream().stream()),
+                                 gv.data_ptr(), ws.data_ptr(), ws.numel(), at::cuda::getCurrentCUDAStream().stream()),
            "fastmax backwardpass");
   return {gq, gk, gv};
 }

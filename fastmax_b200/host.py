@@ -59,7 +59,7 @@ class HostPipeline:
         g = self.group
         with torch.cuda.device(self.dev):
             probe = torch.empty(g, n, d, dtype=dtype, device=self.dev)
-            fwd_b, bwd_b, st_b = _cabi.workspace_bytes(probe, probe, **self.kw)
+            scratch, st_b = _cabi.shared_workspace_sizes(probe, probe, **self.kw)
             self.sets = []
             for _ in range(self.SETS):
                 t = lambda: torch.empty(g, n, d, dtype=dtype, device=self.dev)
@@ -67,7 +67,7 @@ class HostPipeline:
                     q=t(), k=t(), v=t(), go=t(), out=t(), grad_q=t(), grad_k=t(), grad_v=t(),
                     den=torch.empty(g, n, dtype=torch.float32, device=self.dev),
                     stats=torch.empty(st_b, dtype=torch.uint8, device=self.dev),
-                    workspace=torch.empty(max(fwd_b, bwd_b, 1), dtype=torch.uint8, device=self.dev)))
+                    workspace=_cabi._workspace(scratch, self.dev)))
             self.s_in, self.s_cmp, self.s_out = (torch.cuda.Stream(self.dev) for _ in range(3))
             self.ev_in = [torch.cuda.Event() for _ in range(self.SETS)]
             self.ev_cmp = [torch.cuda.Event() for _ in range(self.SETS)]

@@ -137,9 +137,13 @@ size_t fastmax_b200_stats_bytes(const fastmax_problem* prob);
  * fastmax_cuda_forward.cu:384-391). */
 int fastmax_b200_selected_impl(const fastmax_problem* prob, int32_t* impl);
 
-/* Bytes of scratch the forward / backward pass needs (may be 0). */
+/* Bytes of scratch the forward / backward pass works with (may be 0), and the least each still runs with: float32
+ * with d 32 or 64 takes 6 bytes per element of q, k and v (backward: and grad_out) for the operands of its tensor-core
+ * kernels and runs on the CUDA cores, several times slower, in a workspace without that room. */
 size_t fastmax_b200_forward_workspace_bytes(const fastmax_problem* prob);
 size_t fastmax_b200_backward_workspace_bytes(const fastmax_problem* prob);
+size_t fastmax_b200_forward_workspace_least_bytes(const fastmax_problem* prob);
+size_t fastmax_b200_backward_workspace_least_bytes(const fastmax_problem* prob);
 
 /* Forward pass.  Replaces forward_cuda (reference fastmax_cuda_forward.cu:
  * 297-411): normalisation (223-269), moment/score kernels (25-197, and the

@@ -78,3 +78,39 @@ def test_less_workspace_or_unaligned_tensors_run_on_the_cuda_cores():
     rc = _cabi.lib().fastmax_b200_forward(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), den.data_ptr(),
                                           stats.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream)
     assert rc == 0 and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("p", [1, 2])
+def test_no_room_for_the_operand_parts(p):
+    """Where the device has no room for the operand parts, a call runs on the CUDA cores in the least workspace."""
+    bh, n, d = 512, 4096, 32
+    q, k, v, go = [torch.randn(bh, n, d, device="cuda") for _ in range(4)]
+    kw = dict(mask=True, normalize=True, p=p)
+    tensor = q.numel() * 4
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def run(room_fwd=None, room_bwd=None):
+        def leave(room):
+            torch.cuda.empty_cache()
+            if room is not None:
+                torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room * tensor) / total)
+        _cabi.profile(True)
+        try:
+            leave(room_fwd)
+            out, den, st = _cabi.forward(q, k, v, **kw)
+            leave(room_bwd)
+            got = (out,) + tuple(_cabi.backward(q, k, v, out, den, st, go, **kw))
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        names = {n_ for n_, _ in _cabi.profile_records()}
+        _cabi.profile(False)
+        return got, names
+
+    want, names = run()
+    assert any("split" in n_ for n_ in names), names
+    # forward: the result, and either 4.5 tensors of parts or none (first order: one of fp32 rows); backward: three
+    # gradients, and 6 tensors of parts or none (first order: three of fp32 rows)
+    got, names = run(3, 7.5)
+    assert not any("split" in n_ for n_ in names), names
+    for x, r, name in zip(got, want, ("out", "dq", "dk", "dv")):
+        assert float((x - r).abs().max() / r.abs().max()) < BOUND, name

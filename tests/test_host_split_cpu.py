@@ -29,6 +29,22 @@ def test_other_problems_need_no_forward_workspace(kw):
     assert fwd == 0 and bwd <= 4 * rows + 8 * kw.get("bh", 16) + 1024
 
 
+@pytest.mark.parametrize("kw", [dict(), dict(d=64, p=1, nq=8000, nk=8000), dict(d=32, mask=0, p=1, nq=4000, nk=4000),
+                                dict(dtype=_cabi.BF16, d=64)], ids=["score", "moments", "unmasked moments", "bf16"])
+def test_least_workspace_leaves_out_the_operand_parts(kw):
+    base = dict(dtype=_cabi.F32, bh=16, bhkv=16, nq=1000, nk=1000, d=32, mask=1, normalize=1, p=2, impl=0, a0=1, a1=1, a2=0.5,
+                lim=1, temperature=1)
+    prob, L = _cabi.Problem(**{**base, **kw}), _cabi.lib()
+    fwd, bwd = sizes(**kw)
+    least = (L.fastmax_b200_forward_workspace_least_bytes(prob), L.fastmax_b200_backward_workspace_least_bytes(prob))
+    element = prob.bh * prob.nq * prob.d
+    parts = 6 * element if prob.dtype == _cabi.F32 and prob.mask else 0
+    assert fwd - least[0] == 3 * parts
+    moments = _cabi.selected_impl(prob) == "moments"
+    # score form: the parts take the place of the CUDA-core kernels' row dots
+    assert 4 * parts <= bwd - least[1] <= 4 * parts + (4 * prob.bh * prob.nq + 256) * (moments and parts > 0)
+
+
 @pytest.mark.parametrize("heads,n", [(256, 2048), (256, 1233), (64, 8192)])
 def test_fused_first_order_needs_no_fp32_rows(heads, n):
     fwd, bwd = sizes(dtype=_cabi.BF16, bh=heads, bhkv=heads, nq=n, nk=n, d=64, p=1)
