@@ -78,6 +78,11 @@ fastmax_problem make_problem(const torch::Tensor& q, const torch::Tensor& k, boo
   return pr;
 }
 
+// The packed forward always runs the score form.  With one chunk as long as the sequence the library's sizes and the
+// backward are of the score form too: statistics without moment states (which `o` would carry as long as it lives),
+// and the float32 kernels' workspace at every length.
+void one_chunk(fastmax_problem* pr) { pr->chunk = (pr->nk + 255) / 256 * 256; }
+
 void check_rc(int rc, const char* what) {
   TORCH_CHECK(rc == FASTMAX_OK, what, " failed (code ", rc, "): ", fastmax_b200_last_error());
 }
@@ -136,6 +141,7 @@ torch::Tensor forward_impl(const torch::Tensor& q, const torch::Tensor& k, const
   TORCH_CHECK(dropout >= 0.0, "dropout must be non-negative, got: ", dropout);
   c10::cuda::CUDAGuard guard(q.device());
   fastmax_problem pr = make_problem(q, k, mask, normalize, temperature, a0, a1, a2, lim, p);
+  one_chunk(&pr);
   // one storage: the (bh, nq, d+1) result, then (256-byte aligned) the statistics of this call
   const int64_t elems = q.size(0) * q.size(1) * (q.size(2) + 1);
   const size_t stats_offset = ((size_t)elems * sizeof(float) + 255) / 256 * 256;
@@ -145,12 +151,7 @@ torch::Tensor forward_impl(const torch::Tensor& q, const torch::Tensor& k, const
   auto o = buf.narrow(0, 0, elems).view({q.size(0), q.size(1), q.size(2) + 1});
   void* stats = (char*)buf.data_ptr() + stats_offset;
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  // the float32 score kernels keep their operand parts in a workspace (the packed layout is always score form)
-  int32_t impl = 0;
-  size_t wsb = 0;
-  if (fastmax_b200_selected_impl(&pr, &impl) == FASTMAX_OK && impl == FASTMAX_IMPL_DENSE_FFMA)
-    wsb = fastmax_b200_forward_workspace_bytes(&pr);
-  auto ws = scratch(wsb, 0, q);
+  auto ws = scratch(fastmax_b200_forward_workspace_bytes(&pr), fastmax_b200_forward_workspace_least_bytes(&pr), q);
   check_rc(fastmax_b200_forward_packed(&pr, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr<float>(), stats,
                                        ws.data_ptr(), ws.numel(), stream),
            "fastmax forwardpass");
@@ -210,9 +211,7 @@ std::vector<torch::Tensor> backwardpass(torch::Tensor q, torch::Tensor k, torch:
     stats = (const char*)o.storage().data() + rec.stats_offset;
   }
   fastmax_problem pr = make_problem(q, k, mask, normalize, 1.0, a0, a1, a2, lim, p);
-  // the packed forward leaves statistics but no moment states behind them: one chunk as long as the sequence keeps the
-  // backward on the score form, which reads the statistics only
-  if (stats) pr.chunk = (int32_t)((k.size(1) + 255) / 256 * 256);
+  if (stats) one_chunk(&pr);   // as forwardpass asked for them
   auto out = o.slice(2, 0, d).to(q.scalar_type()).contiguous();
   auto den = o.select(2, d).contiguous();
   auto go = grad_output.to(q.scalar_type()).contiguous();
