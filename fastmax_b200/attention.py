@@ -64,7 +64,7 @@ class FASTMultiHeadAttention_Function(torch.autograd.Function):
         if dropout > 0.0 and (drop_noise is None or drop_noise.shape != q.shape):
             raise ValueError("dropout > 0 needs drop_noise with the shape of q")
         shapes = None
-        if k.dim() != v.dim():           # one of them has its batch and head axes merged
+        if k.shape != v.shape:           # batch and head axes merged in one of them, or split in another way
             shapes = k.shape, v.shape
             k, v = [t.flatten(0, 1) if t.dim() == 4 else t for t in (k, v)]
         q, k, v = _contiguous_heads(q), _contiguous_heads(k), _contiguous_heads(v)

@@ -155,6 +155,27 @@ def test_module_interface_matches_oracle_4d_and_3d():
         assert_close(got, ref, torch.float32, f"module flat={flat}")
 
 
+def test_batch_and_head_axes_may_be_split_differently():
+    """Only the product of the batch and head axes counts, tensor by tensor; each gradient has its tensor's shape."""
+    n, d = 70, 32
+    q, k, v, go = [randn(16, n, d, seed=s) for s in range(4)]
+    mod = fastmax_b200.FASTMultiHeadAttention()
+
+    def run(sq, sk, sv):
+        t = [x.reshape(*s, n, d).cuda().requires_grad_(True) for x, s in ((q, sq), (k, sk), (v, sv))]
+        out = mod(*t, mask=True, normalize=True, p=2)
+        out.backward(go.reshape(*sq, n, d).cuda())
+        assert out.shape == t[0].shape and all(x.grad.shape == x.shape for x in t)
+        return [x.detach().reshape(16, n, d) for x in (out, *[x.grad for x in t])]
+
+    want = run((16,), (16,), (16,))
+    for shapes in (((2, 8), (2, 8), (1, 16)), ((4, 4), (16, 1), (2, 8)), ((2, 8), (16,), (4, 4)), ((16,), (4, 4), (16,))):
+        for a, b in zip(run(*shapes), want):
+            assert float((a - b).abs().max() / b.abs().max()) < 1e-5, shapes
+    with pytest.raises(ValueError):
+        mod(q.view(2, 8, n, d).cuda(), k.view(2, 8, n, d).cuda(), v[:8].view(1, 8, n, d).cuda())
+
+
 def test_errors_surface_as_python_exceptions():
     q = torch.randn(2, 16, 32, device="cuda")
     with pytest.raises(ValueError):
