@@ -496,6 +496,10 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
   const fastmax_problem& p = c.p;
   const int heads = rev ? p.bhkv : p.bh, col_heads = rev ? p.bh : p.bhkv;
   if (heads == 0 || nrows == 0) return FASTMAX_OK;
+  // the first-order chunks come here without passing dense_tc_forward / _backward, which check this for the others:
+  // TMA reads the operands, rows are stored and read back 16 bytes at a time
+  const uintptr_t bases = (uintptr_t)x | (uintptr_t)u | (uintptr_t)y | (uintptr_t)z | (uintptr_t)a.o1 | (uintptr_t)a.o2;
+  if (bases & 15) return fail(FASTMAX_E_ARG, "the tensor-core family needs 16-byte aligned tensors");
   CUtensorMap tx, tu, ty, tz, ts;
   int rc;
   if ((rc = tma_map_bf16(&tx, x, heads, nrows, D, BM))) return rc;

@@ -78,3 +78,38 @@ def test_first_order_shards_read_the_base_of_earlier_shards():
     out, den = torch.cat([o for o, _ in outs], 1), torch.cat([d for _, d in outs], 1)
     assert float((out.float() - want.float()).abs().max() / want.float().abs().max()) < 2e-2
     assert float((den - wden).abs().max() / wden.abs().max()) < 1e-2
+
+
+def test_first_order_chunks_refuse_unaligned_results():
+    """Forced onto the moment family (AUTO takes such tensors elsewhere), and as a sequence shard: an argument error before
+    the kernel that would write the rows, forward and backward."""
+    bh, n = 3, 600
+    size = bh * n * 64
+    q, k, v, go = [torch.randn(bh, n, 64, device="cuda").bfloat16() for _ in range(4)]
+    odd = lambda: torch.empty(size + 1, dtype=torch.bfloat16, device="cuda")[1:].view(bh, n, 64)  # noqa: E731
+    kw = dict(mask=True, normalize=True, p=1, impl="moments", chunk=256)
+    fwd, bwd, stats = _cabi.workspace_bytes(q, k, **kw)
+    scratch = lambda m: torch.empty(m, dtype=torch.uint8, device="cuda")  # noqa: E731
+    with pytest.raises(ValueError, match="16-byte aligned"):
+        _cabi.forward(q, k, v, buffers=dict(out=odd(), den=torch.empty(bh, n, device="cuda"), stats=scratch(stats),
+                                            workspace=scratch(fwd)), **kw)
+    out, den, st = _cabi.forward(q, k, v, **kw)
+    want = _cabi.backward(q, k, v, out, den, st, go, **kw)
+    for name in ("grad_q", "grad_k", "grad_v"):
+        grads = {g: torch.empty_like(q) for g in ("grad_q", "grad_k", "grad_v")}
+        with pytest.raises(ValueError, match="16-byte aligned"):
+            _cabi.backward(q, k, v, out, den, st, go, buffers={**grads, name: odd(), "workspace": scratch(bwd)}, **kw)
+    got = _cabi.backward(q, k, v, out, den, st, go, **kw)
+    assert all(torch.equal(a, b) for a, b in zip(got[2:], want[2:]))     # no atomics behind grad_v
+    L = _cabi.lib()
+    prob = _cabi.make_problem(q, k, True, False, 1.0, 1.0, 1.0, 0.5, 1.0, 1, "auto", 256)
+    states = torch.empty(L.fastmax_b200_moment_state_bytes(prob), dtype=torch.uint8, device="cuda")
+    total = torch.empty(L.fastmax_b200_moment_total_bytes(prob), dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    assert L.fastmax_b200_shard_kv_state(prob, k.data_ptr(), v.data_ptr(), states.data_ptr(), total.data_ptr(), stream) == 0
+    ws = scratch(L.fastmax_b200_shard_forward_workspace_bytes(prob))
+    rc = L.fastmax_b200_shard_forward(prob, q.data_ptr(), k.data_ptr(), v.data_ptr(), None, states.data_ptr(), None,
+                                      odd().data_ptr(), den.data_ptr(), ws.data_ptr(), ws.numel(), stream)
+    assert rc == -1 and b"16-byte aligned" in L.fastmax_b200_last_error()
+    torch.cuda.synchronize()
+    assert _cabi.device_status() == 0
