@@ -1,5 +1,6 @@
 """GPU parity of the short-row score kernels (bf16, d = 64, two row tiles per SM) against the CPU oracle: enough heads
-that the dispatch picks them, row and column tile edges, grouped heads, more keys than queries, both orders, and the
+that the dispatch picks them (checked by kernel name in a test of its own, since launches of the short and the wide
+kernels carry the same labels), row and column tile edges, grouped heads, more keys than queries, both orders, and the
 chunks of the moment family.  Tolerance: the bf16 one of the other tests (2e-2 of the largest value)."""
 import pytest
 import torch
@@ -33,6 +34,39 @@ def test_short_rows_against_dense_oracle(cfg):
     assert _cabi.device_status() == 0
     ref = oracle(q, k, v, go, torch.bfloat16, dense=True, **kw)
     assert_close(got, ref, torch.bfloat16, str(cfg), floor=1.0 if nk == 1 else 1e-2)
+
+
+def kernel_names(call):
+    """Functions of the kernels that ``call`` launches, from the CUDA activity trace."""
+    call()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages()]
+
+
+def test_sizes_of_these_tests_reach_the_short_kernels():
+    kw = dict(mask=True, normalize=True, p=2)
+
+    def step(heads, kv, n, **more):
+        q, go = [torch.randn(heads, n, 64, device="cuda").bfloat16() for _ in range(2)]
+        k, v = [torch.randn(kv, n, 64, device="cuda").bfloat16() for _ in range(2)]
+
+        def call():
+            out, den, st = _cabi.forward(q, k, v, **{**kw, **more})
+            _cabi.backward(q, k, v, out, den, st, go, **{**kw, **more})
+        return kernel_names(call)
+
+    seen = {"score": step(150, 150, 65, impl="dense_tc"), "two row tiles": step(75, 75, 129, impl="dense_tc"),
+            "grouped": step(180, 60, 150, impl="dense_tc"), "chunks": step(40, 40, 520, impl="moments", chunk=256),
+            "first order": step(40, 40, 700, impl="moments", chunk=256, p=1)}
+    if not any(seen.values()):
+        pytest.skip("no CUDA activity trace on this machine")
+    for what, names in seen.items():
+        short = [n_ for n_ in names if "short_kernel<" in n_]
+        # grouped: the 120 row tiles of 60 key/value heads are fewer than the SMs, so that pass stays on the wide kernel
+        assert len(short) == (2 if what == "grouped" else 3), (what, names)
+        assert any("dense_tc_wide_kernel" in n_ for n_ in names) == (what == "grouped"), (what, names)
 
 
 @pytest.mark.parametrize("p,chunk,n", [(1, 256, 700), (1, 512, 1537), (2, 256, 520), (1, 0, 1100)])
@@ -113,3 +147,33 @@ def test_first_order_chunks_refuse_unaligned_results():
     assert rc == -1 and b"16-byte aligned" in L.fastmax_b200_last_error()
     torch.cuda.synchronize()
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("d,heads,n", [(64, 96, 1700), (128, 16, 4300)])
+@pytest.mark.parametrize("back_aligned", [False, True], ids=["unaligned backward", "aligned backward"])
+def test_unaligned_tensors_at_lengths_of_the_moment_family(d, heads, n, back_aligned):
+    """AUTO serves causal first-order tensors that TMA cannot read on the CUDA cores; a backward on aligned copies runs on the
+    moment family and finds the states it expects behind the statistics (filled with NaN before)."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    size = heads * n * d
+    flat = [torch.randn(size + 1, generator=g, device="cuda").bfloat16() for _ in range(4)]
+    q, k, v, go = [t[1:].view(heads, n, d) for t in flat]
+    assert q.data_ptr() % 16
+    kw = dict(mask=True, normalize=True, p=1)
+    assert _cabi.selected_impl(_cabi.make_problem(q, k, True, True, 1.0, 1.0, 1.0, 0.5, 1.0, 1)) == "moments"
+    aligned = [t.clone() for t in (q, k, v, go)]
+    out, den, st = _cabi.forward(*aligned[:3], **kw)
+    want = (out,) + tuple(_cabi.backward(*aligned[:3], out, den, st, aligned[3], **kw))
+    fwd, _, stats = _cabi.workspace_bytes(q, k, **kw)
+    bufs = dict(out=torch.empty_like(aligned[0]), den=torch.empty_like(den),
+                stats=torch.full((stats,), 255, dtype=torch.uint8, device="cuda"),
+                workspace=torch.empty(fwd, dtype=torch.uint8, device="cuda"))
+    _cabi.profile(True)
+    out, den, st = _cabi.forward(q, k, v, buffers=bufs, **kw)
+    t = aligned if back_aligned else (q, k, v, go)
+    got = (out,) + tuple(_cabi.backward(*t[:3], out, den, st, t[3], **kw))
+    names = {n_ for n_, _ in _cabi.profile_records()}
+    _cabi.profile(False)
+    assert "fm_dense_ffma_fwd" in names and ("fm_dense_ffma_dq" in names) != back_aligned, names
+    for a, b, name in zip(got, want, ("out", "dq", "dk", "dv")):
+        assert float((a.float() - b.float()).abs().max() / b.float().abs().max()) < 2e-2, name
