@@ -621,7 +621,10 @@ def roofline_of(per, cfg, bh, peaks, lib_version, chunk=0):
         else:
             peak, src, bound = FFMA_TFLOPS_NOMINAL, "nominal FP32 FFMA at the maximum SM clock (no measured figure)", "fp32-ffma"
         traffic = None
-        if dom in NCU_BYTES_PER_TOKEN_HEAD and D == 64 and dt == "bf16" and lib_version == TRAFFIC_LIB_VERSION:
+        # the capture is of the wide kernels on whole rows; short rows (at most 1900 columns on average) and the chunks of
+        # the moment family run on other kernels under the same labels
+        wide = (N / 2 if mask else N) > 1900 and not any(n.startswith(("fm_moments", "fm_first")) for n in per)
+        if dom in NCU_BYTES_PER_TOKEN_HEAD and D == 64 and dt == "bf16" and wide and lib_version == TRAFFIC_LIB_VERSION:
             traffic = NCU_BYTES_PER_TOKEN_HEAD[dom] * bh * N
         return {"bound": bound, "kernel": dom, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": traffic,

@@ -103,8 +103,6 @@ static int check_device() {
   return FASTMAX_OK;
 }
 
-// Family actually used for a problem.  `packed` = forward into the reference's
-// float32 (d+1)-channel layout, which only the CUDA-core family writes.
 // Rough time of one pass per (token, head) in arbitrary units: score form grows with the
 // number of keys a row sees, the moment form is constant plus its own chunk in score form.
 static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
@@ -156,6 +154,8 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   return t_mom < t_score && p.nk > moments_chunk(p);
 }
 
+// Family actually used for a problem.  `packed` = forward into the reference's float32 (d+1)-channel layout, which the
+// CUDA-core score kernels write and, for float32 at d 32 and 64, the split ones (use_split).
 static int pick_impl(const fastmax_problem& p, bool packed, int* impl) {
   int want = p.impl;
   const bool tc_ok = dense_tc_supports(p) && !packed;
@@ -188,8 +188,9 @@ static bool aligned16(std::initializer_list<const void*> ptrs) {
   return true;
 }
 
-// First-order causal problems go to the moment family at almost any length; unlike the second-order ones, which
-// get there only where nothing else is fast enough, their calls with unaligned tensors are served too.
+// bf16 first-order causal problems go to the moment family from some 1000 (d = 64) or 2750 (d = 128) tokens on, where
+// the score form would serve unaligned tensors on the CUDA cores; they go on being served there.  Second-order
+// ones get to the moment family near 9 500 tokens and are refused.
 static bool first_order_unaligned(const fastmax_problem& p, int impl, std::initializer_list<const void*> ptrs) {
   return p.impl == FASTMAX_IMPL_AUTO && impl == FASTMAX_IMPL_MOMENTS && p.p == 1 && p.mask && dense_tc_supports(p) &&
          !aligned16(ptrs);

@@ -214,7 +214,6 @@ int split_status(int* out, cudaStream_t stream);
 int split_status_reset(cudaStream_t stream);
 
 // decode state: prompt processing on the tensor cores (fm_decode_tc.cu), bf16, d 64 or 128
-bool decode_append_tc_supports(const fastmax_problem& p);
 int decode_append_tc(const fastmax_problem& p, const void* k, const void* v, long long n_new, float* state,
                      cudaStream_t st);
 int decode_tc_status(int* out, cudaStream_t stream);

@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(AppCfg<D>::THREADS, 2) append_kernel(const Dec
   using namespace sm100;
   typedef AppCfg<D> C;
   constexpr int DV = D + 1, KS = D + 4;
-  constexpr int TB = 64 / (int)sizeof(T) * (D >= 128 ? 1 : 2) / 2;      // tokens per batch: 32 / 16 (D = 128: half)
+  constexpr int TB = 64 / (int)sizeof(T) * (D >= 128 ? 1 : 2) / 2;      // tokens per batch: bf16 32, float32 16 (D = 128: 8)
   constexpr int EPV = 16 / (int)sizeof(T), VPT = D / EPV;
   constexpr int NLD = (TB * VPT + C::THREADS - 1) / C::THREADS;         // 16-byte loads per thread, k and v each
   __shared__ __align__(16) float ks[TB][KS];
@@ -495,11 +495,14 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
   DecArgs a{p.bh, p.bhkv, p.bhkv ? p.bh / p.bhkv : 1, p.p, p.normalize, p.a0, p.a1, p.a2, p.lim, n_new,
             kHeader + (long long)rows_of(p) * (D + 1)};
   if (p.bhkv == 0) return FASTMAX_OK;
-  if (!READ && n_new >= append_min(p) && decode_append_tc_supports(p)) return decode_append_tc(p, k, v, n_new, state, st);
   if (!READ && n_new >= append_min(p)) {
-    dim3 grid(AppCfg<D>::ctas(p.p), p.bhkv);
-    FM_LAUNCH("fm_decode_append", st,
-              (append_kernel<T, D><<<grid, AppCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));
+    if constexpr (sizeof(T) == 2 && D >= 64) {
+      return decode_append_tc(p, k, v, n_new, state, st);
+    } else {
+      dim3 grid(AppCfg<D>::ctas(p.p), p.bhkv);
+      FM_LAUNCH("fm_decode_append", st,
+                (append_kernel<T, D><<<grid, AppCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));
+    }
   } else {
     dim3 grid(DecCfg<D>::ctas(p.p), p.bhkv);
     FM_LAUNCH(READ ? "fm_decode_step" : "fm_decode_append", st,

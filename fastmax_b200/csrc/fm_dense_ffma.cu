@@ -1,8 +1,10 @@
 // Fastmax attention in tiled score form on CUDA cores (fp32 math, fp32 or bf16
 // storage).  This family covers every supported head dimension, both
-// polynomial orders, causal and unmasked, grouped k/v heads and nq != nk; it is
-// the fp32 product path at short sequences and the on-device cross-check for
-// the tensor-core families.
+// polynomial orders, causal and unmasked, grouped k/v heads and nq != nk.  It is
+// the product path of the shapes without a tensor-core kernel (float32 at d 8, 16
+// and 128, bf16 up to d = 32), serves float32 calls without room for operand
+// parts (fm_dense_split.cu) and unaligned tensors, and is the on-device
+// cross-check for the tensor-core families.
 //
 // One kernel template serves all three passes.  A 64-row tile owns its outputs
 // and walks 64-column tiles; for each tile pair it forms S = X Y^T (and, for the

@@ -30,7 +30,9 @@
 //    64 heads x 4000 unmasked, d = 64: 1.07 / 1.81 / 3.08  (7.96 / 11.7 / 15.6)
 // Error against float64 (2-norm, outputs and gradients): 0.8-3.7e-7 for 64 to 10 000 tokens where the CUDA-core
 // family has 0.9e-7 to 2.4e-6.  What bounds it: the chain of hand-offs per 64-column tile (scores -> registers ->
-// operand parts -> products -> sums), 2 000-2 300 cycles at d = 32 against 780 (forward) of tensor-pipe time.
+// operand parts -> products -> sums), 2 000-2 300 cycles at d = 32 against 780 (forward) of tensor-pipe time.  DKDV holds
+// 32 columns of S and W and six arrays of parts at once and is the one that spills at 168 registers (246 bytes of
+// stores at d = 64, 44 at d = 32).
 //
 // Operands: split3_kernel writes each tensor once as rows of [h | m | l] (3 d bf16); a tile of them in shared
 // memory is a set of 64-element (128-byte) swizzle atoms -- d = 64: one atom per part; d = 32: [h | m] and
@@ -171,16 +173,6 @@ __device__ __forceinline__ void split3(uint64_t v, uint32_t& h, uint32_t& m, uin
   const uint64_t r = fma2(pack2u(h << 16, h & 0xFFFF0000u), neg1, v);
   m = pack_bf16_2(r);
   l = pack_bf16_2(fma2(pack2u(m << 16, m & 0xFFFF0000u), neg1, r));
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
 }
 
 // Adds this warp's half of the features of one tile's accumulator to the running sums (packed pairs).

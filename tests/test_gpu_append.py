@@ -1,6 +1,6 @@
 """Prompt processing of the decode state at the sizes where its kernels change: the tensor-core kernel's blocks of 64
-tokens (bf16, d 64 and 128), the CUDA-core kernel's batches, and the few-token kernel below 64 tokens; onto an empty
-and onto a filled state, against float64 sums.
+tokens (bf16, d 64 and 128), the CUDA-core kernel's batches, and the few-token kernel (below 24 tokens at p = 1, 64 at
+p = 2 for bf16 with d = 128, else 40); onto an empty and onto a filled state, against float64 sums.
 
 Bound: products are exact (bf16) or rounded once (float32) and sums of up to n terms are accumulated in float32, so
 the error of an element is within n * 2^-24 of the sum of its terms' magnitudes; elements of a state of N(0,1) keys
