@@ -107,7 +107,7 @@ static int check_device() {
 // number of keys a row sees, the moment form is constant plus its own chunk in score form.
 static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   if (!moments_supports(p)) return false;
-  if (first_order_measured(p)) {
+  if (first_order_chunk(p) > 0) {
     // First order, causal.  The score form's time per token and head grows by `slope` ns per token of length (a line
     // through its measured times), the moment form's is flat; they meet at `meet` tokens.  The moment form's extra
     // launches cost some 30 us of host time, so what it saves has to exceed that.  Measured per step, score / moment:
@@ -117,8 +117,21 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
     //   float32 d = 32   64 heads: 0.60 / 0.80 at 2048, 1.12 / 1.11 at 3072, 1.80 / 1.52 at 4096
     //   float32 d = 64   32 heads: 1.10 / 1.31 at 3072, 1.75 / 1.67 at 4096, 3.59 / 2.67 at 6144
     const bool bf16 = p.dtype == FASTMAX_BF16;
-    const double slope = bf16 ? (p.d == 64 ? 0.42e-3 : 0.82e-3) : (p.d == 64 ? 2.44e-3 : 1.11e-3);
-    const double meet = bf16 ? (p.d == 64 ? 1000 : 2750) : (p.d == 64 ? 3950 : 3100);
+    if (bf16 ? p.d <= 32 : (p.d != 32 && p.d != 64)) {
+      // Both families on the CUDA cores.  With few heads the score form is a chain of column tiles, one CTA after
+      // another, that does not get shorter with less work: beyond 1100 tokens (d = 128: 880) the moment form wins with
+      // any number of heads.  Measured, ms, score / moment:
+      //   float32 d = 8    256 heads: 0.58 / 0.57 at 500, 1.29 / 0.83 at 800; 64: 0.29 / 0.28 at 600; 8: 0.20 / 0.19 at 1000; 1: 0.19 / 0.20 at 800
+      //   float32 d = 16   256 heads: 0.60 / 0.67 at 500, 0.86 / 0.79 at 600; 64: 0.30 / 0.32 at 600; 8: 0.19 / 0.20 at 1000; 1: 0.19 / 0.20 at 1000
+      //   float32 d = 128  256 heads: 8.34 / 8.80 at 800, 12.2 / 10.6 at 1000; 64: 2.38 / 2.49 at 800; 1: 0.62 / 0.67 at 800, 0.75 / 0.68 at 1000
+      //   bf16 d = 32      256 heads: 0.90 / 1.04 at 500, 1.31 / 1.23 at 600; 64: 0.43 / 0.46 at 600; 8: 0.27 / 0.29 at 1000
+      //   (bf16 d = 8 and 16 as float32)
+      if (p.nk > (p.d == 128 ? 880 : 1100)) return p.nk > moments_chunk(p);
+      if (p.d == 128) return false;
+    }
+    const double slope = bf16 ? (p.d == 64 ? 0.42e-3 : (p.d == 128 ? 0.82e-3 : (p.d == 32 ? 9.8e-3 : 6.2e-3)))
+                              : (p.d == 64 ? 2.44e-3 : (p.d == 32 ? 1.11e-3 : 6.2e-3));
+    const double meet = p.d == 64 ? (bf16 ? 1000 : 3950) : (p.d == 128 ? 2750 : (p.d == 32 ? (bf16 ? 550 : 3100) : (p.d == 16 ? 550 : 500)));
     return p.nk > moments_chunk(p) && (double)p.bh * p.nk * slope * ((double)p.nk - meet) > 30e3;
   }
   const double d = p.d, F = d + (p.p == 2 ? d * d : 0.0);

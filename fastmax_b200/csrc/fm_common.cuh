@@ -272,7 +272,7 @@ int first_tc_status_reset(cudaStream_t stream);
 struct MomFwdWs { size_t states, total, o_add, den_add, s16, split, bytes; };
 struct MomBwdWs { size_t dots, delta, dvec, gs, states, total, gq_add, gk_add, gv_add, s16, split, bytes; };
 int moments_chunk(const fastmax_problem& p);
-bool first_order_measured(const fastmax_problem& p);
+int first_order_chunk(const fastmax_problem& p);
 bool moments_supports(const fastmax_problem& p);
 size_t moment_state_bytes(const fastmax_problem& p, int n);
 size_t moment_total_bytes(const fastmax_problem& p);

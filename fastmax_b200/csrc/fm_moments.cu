@@ -9,23 +9,26 @@ namespace fm {
 
 static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Causal first-order problems whose chunk length and whose line to the score form were measured: bf16 with every kernel
-// on the tensor cores and float32 with the split score kernels.  The other shapes (float32 at d 8, 16 and 128 or too
-// large for the split kernels' operands, bf16 up to d = 32) run their states on the CUDA cores, whose cost per chunk
-// nobody measured at short chunks; they keep chunks of 2048 and the rate model of moments_faster.
-bool first_order_measured(const fastmax_problem& p) {
-  return p.p == 1 && p.mask && (p.dtype == FASTMAX_BF16 ? first_tc_supports(p) : dense_split_supports(p));
+// Tokens per chunk of causal first-order problems, for the kernels it was measured with; 0 for the others (tensor cores
+// switched off, float32 operands too large for the split kernels), which keep 2048 and the rate model of moments_faster.
+// What a token costs is its own chunk in score form, so short chunks win.  Measured, ms per step at 256 / 512 / 1024 / 2048:
+//   bf16 on the tensor cores, 256 heads x 4096: d = 64 1.30, 1.30, 1.97, 2.41 (the last two with separate read-outs); d = 128
+//   4.19, 3.65, 3.79, 4.60.  float32 with the split score kernels, d = 32, 8 heads x 4096: 0.31, 0.42, 0.64, 1.06.
+//   Everything on the CUDA cores, 256 heads x 2000: float32 d = 16 2.39, 3.21, 4.96, 8.19; d = 128 20.8, 25.6, 35.8, 55.7;
+//   bf16 d = 32 3.81, 5.10, 7.67, 12.8.
+int first_order_chunk(const fastmax_problem& p) {
+  if (p.p != 1 || !p.mask) return 0;
+  if (p.dtype == FASTMAX_BF16) return first_tc_supports(p) ? 512 : (p.d <= 32 ? 256 : 0);
+  return dense_split_supports(p) || (p.d != 32 && p.d != 64) ? 256 : 0;
 }
 
 // Tokens per chunk.  Second order: 2048, measured best for the tensor-core kernels (8.9 ms at 1024, 7.8 at 2048,
 // 8.2 at 4096 per step for 8 heads of 65536 tokens): a chunk's state is as large as its tokens, so fewer, larger
-// chunks mean fewer states to build, scan and convert.  First order, causal: a state is d + 1 rows (17 KB at
-// d = 64 against 131 KB of tokens in 512), so a short chunk wins -- what a token costs there is its own chunk in score
-// form (256 heads x 4096, bf16, ms: d = 64 1.30 at 256 and 512, with separate read-outs 1.97 at 1024 and 2.41 at 2048;
-// d = 128 4.19, 3.65, 3.79, 4.60; float32 at d = 32, 8 heads x 4096: 0.31, 0.42, 0.64, 1.06).  First order, unmasked:
-// there is no in-chunk part and every chunk only adds a state to sum.
+// chunks mean fewer states to build, scan and convert.  First order, causal: first_order_chunk; unmasked: there is no
+// in-chunk part and every chunk only adds a state to sum.
 int moments_chunk(const fastmax_problem& p) {
-  int L = p.chunk > 0 ? p.chunk : (first_order_measured(p) ? (p.dtype == FASTMAX_BF16 ? 512 : 256) : 2048);
+  int L = p.chunk > 0 ? p.chunk : first_order_chunk(p);
+  if (L == 0) L = 2048;
   L = (L + 255) / 256 * 256;
   return L;
 }

@@ -271,7 +271,7 @@ def fastmax_sequence_parallel(q, k, v, *, mask=True, normalize=False, a0=1.0, a1
 
     Rank r of ``group`` must hold tokens ``[r*n_local, (r+1)*n_local)``, the same ``n_local`` on every rank
     (chunks of ``chunk`` tokens are laid out from the start of each shard; by default 2048, for causal p = 1 512 in
-    bfloat16 at head size 64 or 128 and 256 in float32 at 32 or 64).  Differentiable;
+    bfloat16 at head size 64 or 128 and 256 elsewhere).  Differentiable;
     gradients come back sharded the same way.
     """
     if backend is None:

@@ -78,10 +78,11 @@ def test_family_selection_follows_the_measured_break_even_points():
 FIRST_ORDER_LINES = [   # dtype, d, heads, longest length in score form, shortest on the moment family
     (_cabi.BF16, 64, 256, 1216, 1248), (_cabi.BF16, 64, 8, 3520, 3552), (_cabi.BF16, 128, 256, 2800, 2832),
     (_cabi.F32, 32, 256, 3120, 3152), (_cabi.F32, 64, 256, 3952, 3984),
-    # shapes whose states run on the CUDA cores: nothing below one default chunk of 2048
-    (_cabi.F32, 8, 256, 2048, 2064), (_cabi.F32, 16, 256, 2064, 2080), (_cabi.F32, 128, 256, 2208, 2224),
-    (_cabi.BF16, 8, 256, 2048, 2064), (_cabi.BF16, 16, 256, 2064, 2080), (_cabi.BF16, 32, 256, 2080, 2096),
-    # operand parts above 48 GiB: no split kernels, so the line of the CUDA-core kernels
+    # both families on the CUDA cores: by what is saved, and beyond 1100 (d = 128: 880) tokens for any number of heads
+    (_cabi.F32, 8, 256, 528, 544), (_cabi.F32, 16, 256, 576, 592), (_cabi.F32, 16, 64, 656, 672), (_cabi.F32, 16, 1, 1100, 1101),
+    (_cabi.BF16, 8, 256, 528, 544), (_cabi.BF16, 16, 8, 1088, 1101), (_cabi.BF16, 32, 256, 560, 576), (_cabi.BF16, 32, 8, 944, 960),
+    (_cabi.F32, 128, 256, 880, 881), (_cabi.F32, 128, 1, 880, 881),
+    # operand parts above 48 GiB: no split kernels, so the rate model of the CUDA-core kernels, beyond one chunk of 2048
     (_cabi.F32, 64, 40000, 2128, 2144)]
 
 
@@ -91,10 +92,10 @@ def test_causal_first_order_lines_between_the_families(dtype, d, heads, below, a
         return _cabi.selected_impl(_cabi.Problem(dtype=dtype, bh=heads, bhkv=heads, nq=n, nk=n, d=d, mask=1, normalize=1,
                                                  p=1, impl=0, a0=1, a1=1, a2=0.5, lim=1, temperature=1))
     dense = "dense_tc" if dtype == _cabi.BF16 and d >= 64 else "dense_ffma"
-    assert [pick(n) for n in (272, 600, below, above, 4 * above)] == [dense] * 3 + ["moments"] * 2
+    assert [pick(n) for n in (272, 500, below, above, 4 * above)] == [dense] * 3 + ["moments"] * 2
 
 
-@pytest.mark.parametrize("dtype,d,n,mask,chunk", [(_cabi.BF16, 64, 1100, 1, 0), (_cabi.BF16, 64, 8000, 0, 0), (_cabi.F32, 8, 300, 1, 256)])
+@pytest.mark.parametrize("dtype,d,n,mask,chunk", [(_cabi.BF16, 64, 1100, 1, 0), (_cabi.BF16, 64, 8000, 0, 0), (_cabi.F32, 8, 600, 1, 0)])
 def test_more_heads_than_a_grid_dimension_stay_in_score_form(dtype, d, n, mask, chunk):
     def pick(heads):
         return _cabi.selected_impl(_cabi.Problem(dtype=dtype, bh=heads, bhkv=heads, nq=n, nk=n, d=d, mask=mask, normalize=1,
