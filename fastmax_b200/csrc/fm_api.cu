@@ -134,6 +134,18 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
     const double meet = p.d == 64 ? (bf16 ? 1000 : 3950) : (p.d == 128 ? 2750 : (p.d == 32 ? (bf16 ? 550 : 3100) : (p.d == 16 ? 550 : 500)));
     return p.nk > moments_chunk(p) && (double)p.bh * p.nk * slope * ((double)p.nk - meet) > 30e3;
   }
+  if (p.p == 1 && !p.mask && dense_split_supports(p)) {
+    // First order, unmasked, float32: pairs on the tensor cores (with few heads a chain of column tiles) against states
+    // and read-outs on the CUDA cores, whose one chain over a chunk of 2048 tokens is there with any number of heads.
+    // Measured per step, ms, score / moment:
+    //   d = 32  64 heads: 1.01 / 1.08 at 2050; 32: 0.85 / 0.98 at 2900; 8: 0.15 / 0.77 at 2050, 0.75 / 0.84 at 5000; 1: 0.67 / 0.77 at 14000
+    //   d = 64  128 heads: 3.42 / 3.52 at 2050, 3.92 / 3.62 at 2300; 64: 2.00 / 2.31 at 2300, 2.87 / 2.53 at 2600; 32: 1.56 / 2.02
+    //           at 2900, 2.25 / 2.12 at 3300; 8: 0.25 / 1.26 at 2050, 1.45 / 1.50 at 5000; 1: 0.80 / 1.23 at 9000
+    const double pairs = (double)p.bh * p.nq * p.nk, tokens = 0.5 * p.bh * ((double)p.nq + p.nk);
+    const double us_pairs = pairs * (p.d == 32 ? 3.6e-6 : 6.4e-6), us_chain = p.nk * (p.d == 32 ? 0.055 : 0.1);
+    const double us_moment = (p.d == 32 ? 750 + 2.9e-3 * tokens : 1200 + 8.2e-3 * tokens);
+    return p.nk > moments_chunk(p) && us_moment < (us_pairs > us_chain ? us_pairs : us_chain);
+  }
   const double d = p.d, F = d + (p.p == 2 ? d * d : 0.0);
   // Constants fitted to this library's kernels on a B200 (bf16, d = 64, p = 2, causal): the score family takes
   // 5.6 ns per token and head at 10^4 keys; the moment family 4.1 ns for its states and read-outs plus 2.0 ns
@@ -141,14 +153,12 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   // times the share of chunks that build and read states.  The two families then break even near 9 300 keys,
   // as measured (score against moment family for the same number of token-heads, 8192 keys: 20.3 / 22.8 ms;
   // 9216: 22.6 / 23.0; 10000: 60.9 / 54.5).
-  // float32 (fm_dense_split.cu, moment states on the CUDA cores), per token and head and step: the score form takes
-  // 4.2 / 5.8 ps per key at d = 32 / 64, the states and read-outs 4.5 / 10.5 ns at p = 1 (256 heads of 1024 tokens)
-  // and 25 / 190 ns at p = 2, so the moment family starts near 2 064 / 2 928 unmasked keys at p = 1 and, at p = 2,
+  // float32, second order (fm_dense_split.cu, moment states on the CUDA cores), per token and head and step: the score form
+  // takes 4.2 / 5.8 ps per key at d = 32 / 64, the states and read-outs 25 / 190 ns, so the moment family starts near
   // 8 160 unmasked and 13 500 causal keys at d = 32 and beyond 20 000 at d = 64.
   const bool split = dense_split_supports(p);
   const double rate_score = tc_ok ? 800e12 : (split ? (p.d == 32 ? 108e12 : 156e12) : 25e12);
-  const double rate_first = first_tc_supports(p) ? 450e12 : (split ? (p.d == 32 ? 3.3e12 : 5.5e12) : 20e12);
-  const double rate_state = p.p == 2 ? (moments_tc_supports(p) ? 930e12 : 20e12) : rate_first;
+  const double rate_state = p.p == 2 ? (moments_tc_supports(p) ? 930e12 : 20e12) : (first_tc_supports(p) ? 450e12 : 20e12);
   const double rate_chunk = tc_ok || split ? 0.58 * rate_score : rate_score;
   // Unmasked with nq != nk: the score form costs nq * nk pairs, the moment form one state per key and one
   // read-out per query row (and the mirror image backward), so per token of the mean length the score form

@@ -29,7 +29,7 @@ def test_other_problems_need_no_forward_workspace(kw):
     assert fwd == 0 and bwd <= 4 * rows + 8 * kw.get("bh", 16) + 1024
 
 
-@pytest.mark.parametrize("kw", [dict(), dict(d=64, p=1, nq=8000, nk=8000), dict(d=32, mask=0, p=1, nq=4000, nk=4000),
+@pytest.mark.parametrize("kw", [dict(), dict(d=64, p=1, nq=8000, nk=8000), dict(d=32, mask=0, p=1, nq=8000, nk=8000),
                                 dict(dtype=_cabi.BF16, d=64)], ids=["score", "moments", "unmasked moments", "bf16"])
 def test_least_workspace_leaves_out_the_operand_parts(kw):
     base = dict(dtype=_cabi.F32, bh=16, bhkv=16, nq=1000, nk=1000, d=32, mask=1, normalize=1, p=2, impl=0, a0=1, a1=1, a2=0.5,
