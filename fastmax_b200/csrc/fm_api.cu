@@ -129,9 +129,10 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
       if (p.nk > (p.d == 128 ? 880 : 1100)) return p.nk > moments_chunk(p);
       if (p.d == 128) return false;
     }
-    const double slope = bf16 ? (p.d == 64 ? 0.42e-3 : (p.d == 128 ? 0.82e-3 : (p.d == 32 ? 9.8e-3 : 6.2e-3)))
-                              : (p.d == 64 ? 2.44e-3 : (p.d == 32 ? 1.11e-3 : 6.2e-3));
-    const double meet = p.d == 64 ? (bf16 ? 1000 : 3950) : (p.d == 128 ? 2750 : (p.d == 32 ? (bf16 ? 550 : 3100) : (p.d == 16 ? 550 : 500)));
+    double slope = 6.2e-3, meet = p.d == 16 ? 550 : 500;      // CUDA cores, d 8 and 16
+    if (p.d == 32) { slope = bf16 ? 9.8e-3 : 1.11e-3; meet = bf16 ? 550 : 3100; }
+    if (p.d == 64) { slope = bf16 ? 0.42e-3 : 2.44e-3; meet = bf16 ? 1000 : 3950; }
+    if (p.d == 128) { slope = 0.82e-3; meet = 2750; }         // bf16; float32 has left above
     return p.nk > moments_chunk(p) && (double)p.bh * p.nk * slope * ((double)p.nk - meet) > 30e3;
   }
   if (p.p == 1 && !p.mask && dense_split_supports(p)) {

@@ -123,7 +123,8 @@ int fastmax_b200_wait_selftest(long long limit_clocks, void* stream);
  * copies of their running sums that the read-out multiplies, about 1.6 times
  * the size of q + k + v + out at d = 64).  backward must be given the buffer the
  * forward call of the same problem filled; with normalize == 0 it may be NULL,
- * and backward then recomputes what it needs.  Replaces the reference's
+ * and backward then recomputes what it needs (as it does where the buffer is
+ * not 16-byte aligned; 8 bytes suffice for the words).  Replaces the reference's
  * qnorms/knorms/qmaxes/kmaxes temporaries (reference fastmax_cuda_forward.cu:
  * 349-358), which it needs because it rescales q and k in place. */
 size_t fastmax_b200_stats_bytes(const fastmax_problem* prob);
