@@ -70,13 +70,9 @@ TRAFFIC_LIB_VERSION = 200
 # profiles/dense_tc_small_case_ncu_full.md, scaled by heads x tokens
 NCU_BYTES_PER_TOKEN_HEAD = {"fm_dense_tc_fwd": 487.0, "fm_dense_tc_dq": 622.7, "fm_dense_tc_dkdv": 722.1,
                             # per token whose chunk builds a state (profiles/moments_tc_small_case_ncu_full.md)
-                            "fm_moments_tc_state": 717.5,
-                            # per token that is read out (same file, section on the read-outs' traffic)
-                            "fm_moments_tc_readout_a": 608.2, "fm_moments_tc_readout_b": 742.4,
-                            "fm_moments_tc_readout_ab": 976.1}
+                            "fm_moments_tc_state": 717.5}
 # Labels that are launches of one kernel function: the roofline record is of the function with the largest share.
-KERNEL_OF_LABEL = {"fm_moments_tc_readout_a": "readout_tc_kernel", "fm_moments_tc_readout_b": "readout_tc_kernel",
-                   "fm_moments_tc_readout_ab": "readout_tc_kernel"}
+KERNEL_OF_LABEL = {}
 
 
 def cfg_of(name):
@@ -561,17 +557,18 @@ def seq_leg(hz, args, cfg, steps, warmup, sample_clocks=False):
 def moment_kernel_flops(name, D, N, mask, chunk):
     """Products one launch of a tensor-core moment kernel needs, per batch*head unit (None: another kernel).
     The state build forms each unordered pair of features once: D (D + 1) / 2 feature rows by D value columns
-    per token (the normaliser column comes from another kernel).  A read-out contracts a token's D x D features
-    with D + 1 columns.  Causal: one chunk builds no state and one reads none."""
+    per token (the normaliser column comes from another kernel).  A read-out of type A multiplies a token with the
+    blocks of 16 features on and below the diagonal, one of type B with each unordered pair, D + 1 columns each.
+    Causal: one chunk builds no state and one reads none."""
     L = chunk or 2048
     nchunk = -(-N // L)
     if name == "fm_moments_tc_state":
         tokens = min(N, (nchunk - 1) * L) if mask else N
         return 2 * (D * (D + 1) // 2) * D * tokens
-    reads = {"fm_moments_tc_readout_a": 1, "fm_moments_tc_readout_b": 1, "fm_moments_tc_readout_ab": 2}
-    if name in reads:
+    pairs = {"fm_moments_tc_readout_a": D * (D + 16) // 2, "fm_moments_tc_readout_b": D * (D + 1) // 2}
+    if name in pairs:
         tokens = max(N - L, 0) if mask else N
-        return reads[name] * 2 * D * D * (D + 1) * tokens
+        return 2 * pairs[name] * (D + 1) * tokens
     return None
 
 
@@ -604,8 +601,8 @@ def roofline_of(per, cfg, bh, peaks, lib_version, chunk=0):
                 "traffic_source": "ncu dram bytes of a small case scaled by heads x tokens" if traffic else None,
                 "peak_source": peaks["source"] + " (sustained cuBLAS bf16)", "ms_per_launch": ms,
                 "alg_flops_per_launch": flops,
-                "note": "products this kernel's own formulation needs (read-out: ordered feature pairs; state build: "
-                        "unordered ones), averaged over its launches of the step; the step's rate is alg_tflops_per_gpu"}
+                "note": "products this kernel's own formulation needs (read-out of type A: blocks of 16 features; type B and "
+                        "state build: unordered pairs), averaged over its launches; the step's rate is alg_tflops_per_gpu"}
     ff, fq, fkv = alg_flops_per_token_head(D, p)
     flops_of = {"fwd": ff, "dq": fq, "dkdv": fkv, "dk": fkv * 2 // 3, "dv": fkv // 3}
     kind = dom.rsplit("_", 1)[-1]

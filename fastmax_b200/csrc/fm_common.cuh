@@ -92,6 +92,9 @@ struct Ctx {
   // without a read-out.  -1: no such chunk.  Honoured by the tensor-core moment kernels.
   int skip_chunk = -1;
   int zero_chunk = -1;
+  // The chunk states built next are only read by moments_tc_prefix_convert, which needs 10 of 16 second-order rows
+  // (the tensor-core state kernel leaves the others as they are).
+  bool lower_rows = false;
   // float32 moment family: room for the operand parts of the in-chunk score kernels (dense_split_*_bytes), or
   // null where the tensors do not allow them
   void* split_ws = nullptr;
@@ -242,18 +245,27 @@ int moments_readout(const Ctx& c, int mode_b, int heads, int n, int chunk, int s
 
 // second-order part on tensor cores (fm_moments_tc.cu): bf16, d == 64, p == 2
 bool moments_tc_supports(const fastmax_problem& p);
-size_t moments_tc_state_bytes(int mats);
 int moments_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void* y, const void* z,
                            const float* dvec, float* state);
-int moments_tc_convert(const Ctx& c, int mats, const float* state, void* state_bf16);
-int moments_tc_prefix_convert(const Ctx& c, int heads, int nchunk, const float* state, const float* base,
-                              int reverse, void* state_bf16);
-int moments_tc_readout(const Ctx& c, int mode, int heads, int n, int chunk, int state_per_chunk,
-                       const void* x, const void* u, const float* uvec, const void* state_bf16,
-                       const stat_t* stats, float* out_a, float* den_a, float* out_b,
-                       const float* state_f32 = nullptr);
 int moments_tc_status(int* out, cudaStream_t stream);
 int moments_tc_status_reset(cudaStream_t stream);
+// its read-out (fm_readout.cu).  The states are multiplied as bf16 copies in two layouts, one per kind of read-out; a
+// null pointer is a layout nobody wants.
+struct StateCopies {
+  void* a = nullptr;
+  void* b = nullptr;
+};
+size_t moments_tc_copy_a_bytes(int mats);
+size_t moments_tc_copy_b_bytes(int mats);
+int moments_tc_convert(const Ctx& c, int mats, const float* state, const StateCopies& to);
+int moments_tc_prefix_convert(const Ctx& c, int heads, int nchunk, const float* state, const float* base, int reverse,
+                              const StateCopies& to);
+int moments_tc_readout_a(const Ctx& c, int heads, int n, int chunk, int state_per_chunk, const void* x,
+                         const void* copies_a, const stat_t* stats, const float* state, float* out, float* den);
+int moments_tc_readout_b(const Ctx& c, int heads, int n, int chunk, int state_per_chunk, const void* x, const void* u,
+                         const float* uvec, const void* copies_b, const stat_t* stats, const float* state, float* out);
+int readout_status(int* out, cudaStream_t stream);
+int readout_status_reset(cudaStream_t stream);
 
 // first-order part on tensor cores (fm_first_tc.cu): bf16, d in {64, 128}
 bool first_tc_supports(const fastmax_problem& p);
@@ -277,7 +289,7 @@ bool moments_supports(const fastmax_problem& p);
 size_t moment_state_bytes(const fastmax_problem& p, int n);
 size_t moment_total_bytes(const fastmax_problem& p);
 size_t state16_bytes(const fastmax_problem& p, int n);   // bf16 operand copies of the states of n tokens
-size_t moment_kept16_bytes(const fastmax_problem& p);    // bf16 second-order copies kept beside the fp32 states
+size_t moment_kept16_bytes(const fastmax_problem& p);    // bf16 second-order copies (type B) kept beside the fp32 states
 MomFwdWs moments_fwd_layout(const fastmax_problem& p);
 MomBwdWs moments_bwd_layout(const fastmax_problem& p);
 int moments_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
@@ -287,7 +299,7 @@ int moments_leave_states(const Ctx& c, const void* k, const void* v, bool aligne
 int moments_forward_finish(const Ctx& c, const void* q, const void* k, const void* v,
                            const stat_t* stats, float* kv_states, const float* s_base,
                            float* o_add, float* den_add, void* s16, const FwdOut& o,
-                           void* second16 = nullptr);
+                           bool fuse = false, void* keep_b = nullptr);
 // chunk states of (y, z | e) with the best kernels for the problem; gs/dvec are the bf16
 // gradient rows and grad_out.out/den when ext == 1 and the tensor-core path is used
 int moments_build_states(const Ctx& c, int n, const void* y, const void* z, const float* den,

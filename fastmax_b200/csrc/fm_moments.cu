@@ -43,21 +43,30 @@ size_t moment_total_bytes(const fastmax_problem& p) {
   return up256(sizeof(float) * (size_t)p.bh * m.f * m.dvp);
 }
 
-// bf16 transposed copy of the second-order block of every chunk state (tensor-core read-out)
-// layout: [second-order copies (tensor-core read-out)][first-order copies]
-static size_t state16_second(const fastmax_problem& p, int mats) {
-  return moments_tc_supports(p) ? up256(moments_tc_state_bytes(mats)) : 0;
+// bf16 copies of the chunk states that the tensor-core read-outs multiply:
+// [second order, type A][second order, type B][first order]
+static size_t copies_a_bytes(const fastmax_problem& p, int mats) {
+  return moments_tc_supports(p) ? up256(moments_tc_copy_a_bytes(mats)) : 0;
+}
+static size_t copies_b_bytes(const fastmax_problem& p, int mats) {
+  return moments_tc_supports(p) ? up256(moments_tc_copy_b_bytes(mats)) : 0;
+}
+static StateCopies copies_at(const fastmax_problem& p, void* s16, int mats) {
+  StateCopies c;
+  c.a = s16;
+  c.b = (char*)s16 + copies_a_bytes(p, mats);
+  return c;
 }
 size_t state16_bytes(const fastmax_problem& p, int n) {
   const int L = moments_chunk(p);
   const int mats = p.bh * ((n + L - 1) / L);
-  return state16_second(p, mats) + (first_tc_supports(p) ? up256(first_tc_copy_bytes(p, mats)) : 0);
+  return copies_a_bytes(p, mats) + copies_b_bytes(p, mats) + (first_tc_supports(p) ? up256(first_tc_copy_bytes(p, mats)) : 0);
 }
 
-// second-order bf16 copies of the key/value chunk prefixes that a causal forward leaves for the backward
+// the type B copies of the key/value chunk prefixes, which a causal forward leaves for the backward's grad_q
 size_t moment_kept16_bytes(const fastmax_problem& p) {
   const int L = moments_chunk(p);
-  return state16_second(p, p.bh * ((p.nk + L - 1) / L));
+  return copies_b_bytes(p, p.bh * ((p.nk + L - 1) / L));
 }
 
 bool moments_all_tc(const fastmax_problem& p) {
@@ -127,11 +136,11 @@ int moments_build_states(const Ctx& c, int n, const void* y, const void* z, cons
 }
 
 // read-out of prefix (or total) states for n tokens; mode 0: type A, 1: type B, 2: both on x
-// second16 (may be null): second-order bf16 copies that exist already (prefix_states, or kept by the forward)
+// ready (may be null): second-order copies that exist already (prefix_states, or kept by the forward)
 static int read_states(const Ctx& c, int mode, int n, int per_chunk, const void* x, const void* u,
                        const float* den, const float* delta, int ext, const void* gs, const float* dvec,
                        const float* states, void* s16, const stat_t* stats, float* out_a, float* den_a,
-                       float* out_b, const void* second16 = nullptr) {
+                       float* out_b, const StateCopies* ready = nullptr) {
   const fastmax_problem& p = c.p;
   const int L = moments_chunk(p);
   int rc;
@@ -139,14 +148,25 @@ static int read_states(const Ctx& c, int mode, int n, int per_chunk, const void*
   const bool tc1 = first_tc_supports(p) && (p.p == 1 || tc2);
   const int mats = p.bh * (per_chunk ? (n + L - 1) / L : 1);
   if (tc2) {
-    if (!second16 && (rc = moments_tc_convert(c, mats, states, s16))) return rc;
-    // both kinds come out complete: the first-order and constant terms ride on the copy's last rows
-    return moments_tc_readout(c, mode, p.bh, n, L, per_chunk, x, ext ? gs : u, ext ? dvec : nullptr,
-                              second16 ? second16 : s16, stats, out_a, den_a, out_b, states);
+    // both kinds come out complete: the first-order and constant terms ride along
+    StateCopies cp = copies_at(p, s16, mats);
+    if (ready) {
+      cp = *ready;
+    } else {
+      if (mode == 0) cp.b = nullptr;
+      if (mode == 1) cp.a = nullptr;
+      if ((rc = moments_tc_convert(c, mats, states, cp))) return rc;
+    }
+    if (mode != 1 && (rc = moments_tc_readout_a(c, p.bh, n, L, per_chunk, x, cp.a, stats, states, out_a, den_a)))
+      return rc;
+    if (mode != 0 && (rc = moments_tc_readout_b(c, p.bh, n, L, per_chunk, x, ext ? gs : u, ext ? dvec : nullptr, cp.b,
+                                                stats, states, out_b)))
+      return rc;
+    return FASTMAX_OK;
   }
   if (tc1) {
     // first-order part on tensor cores; it adds to the second-order part when there is one
-    void* s1b = (char*)s16 + state16_second(p, mats);
+    void* s1b = (char*)s16 + copies_a_bytes(p, mats) + copies_b_bytes(p, mats);
     if ((rc = first_tc_convert(c, mats, states, s1b))) return rc;
     if ((mode == 0 || mode == 2) && !tc2)
       if ((rc = first_tc_readout(c, 0, p.bh, n, L, per_chunk, x, x, nullptr, states, s1b, stats, out_a, den_a,
@@ -181,24 +201,25 @@ static int read_first_final(const Ctx& c, int type_b, int n, const void* tile, c
                           nullptr, 0, final, out, den_out, dots);
 }
 
-// Exclusive running sums over the chunks of every head (per-chunk mode).  With `fuse` and the tensor-core
-// second-order part, the second-order rows go straight to their bf16 transposed copies at `second16` in one
-// pass over the raw states and stay raw in `states` (nothing else reads them); only the first-order rows are
-// summed in place.  *ready tells whether `second16` holds the copies.
+// Exclusive running sums over the chunks of every head (per-chunk mode).  With `fuse` and the tensor-core second-order
+// part, the second-order rows go straight to the bf16 copies `to` in one pass over the raw states and stay raw in
+// `states` (nothing else reads them); only the first-order rows are summed in place.  *ready tells whether `to` holds
+// the copies.
 static int prefix_states(const Ctx& c, int nchunk, float* states, const float* base, int reverse, bool fuse,
-                         void* second16, bool* ready) {
+                         const StateCopies& to, bool* ready) {
   const fastmax_problem& p = c.p;
   *ready = fuse && p.p == 2 && moments_tc_supports(p);
   if (!*ready) return moments_prefix(c, p.bh, nchunk, states, base, nullptr, reverse, 1);
   int rc;
-  // first the first-order rows in place: the copies carry them too (their last 64 rows)
+  // first the first-order rows in place: the copies carry them too
   if ((rc = moments_prefix(c, p.bh, nchunk, states, base, nullptr, reverse, 1, p.d * p.d))) return rc;
-  return moments_tc_prefix_convert(c, p.bh, nchunk, states, base, reverse, second16);
+  return moments_tc_prefix_convert(c, p.bh, nchunk, states, base, reverse, to);
 }
 
 // Copies of the context that tell the tensor-core moment kernels which chunk's state nothing will read,
 // and whose tokens read an empty running sum (see Ctx).
-static Ctx skipping(const Ctx& c, int chunk) { Ctx r = c; r.skip_chunk = chunk; return r; }
+// (the states that skipping() builds go to prefix_states with `fuse`)
+static Ctx skipping(const Ctx& c, int chunk) { Ctx r = c; r.skip_chunk = chunk; r.lower_rows = true; return r; }
 static Ctx zeroing(const Ctx& c, int chunk) { Ctx r = c; r.zero_chunk = chunk; return r; }
 
 // ---- forward -----------------------------------------------------------------------
@@ -206,14 +227,18 @@ static Ctx zeroing(const Ctx& c, int chunk) { Ctx r = c; r.zero_chunk = chunk; r
 // totals of all earlier shards or null.  Turns the states into prefixes in place.
 int moments_forward_finish(const Ctx& c, const void* q, const void* k, const void* v,
                            const stat_t* stats, float* kv_states, const float* s_base,
-                           float* o_add, float* den_add, void* s16, const FwdOut& o, void* second16) {
+                           float* o_add, float* den_add, void* s16, const FwdOut& o, bool fuse, void* keep_b) {
   const fastmax_problem& p = c.p;
   const int L = moments_chunk(p);
   const int nchunk = (p.nk + L - 1) / L;
   int rc;
-  // second16 != null: the caller does not need the fp32 second-order prefixes (see prefix_states)
+  // fuse: the caller does not need the fp32 second-order prefixes (see prefix_states); the type A copies are used up
+  // here, type B ones are written at keep_b when the backward will want them
   bool ready;
-  if ((rc = prefix_states(c, nchunk, kv_states, s_base, 0, second16 != nullptr, second16, &ready))) return rc;
+  StateCopies cp;
+  cp.a = s16;
+  cp.b = keep_b;
+  if ((rc = prefix_states(c, nchunk, kv_states, s_base, 0, fuse, cp, &ready))) return rc;
   if (first_fused(p) && !o.out_f32) {
     if ((rc = first_tc_convert(c, p.bh * nchunk, kv_states, s16, nchunk, stats))) return rc;
     ChunkAdd own;
@@ -223,7 +248,7 @@ int moments_forward_finish(const Ctx& c, const void* q, const void* k, const voi
   }
   // without a base the tokens of the first chunk have nothing before them
   if ((rc = read_states(zeroing(c, s_base ? -1 : 0), 0, p.nq, 1, q, nullptr, nullptr, nullptr, 0, nullptr, nullptr,
-                        kv_states, s16, stats, o_add, den_add, nullptr, ready ? second16 : nullptr)))
+                        kv_states, s16, stats, o_add, den_add, nullptr, ready ? &cp : nullptr)))
     return rc;
   ChunkAdd ca;
   ca.chunk = L;
@@ -256,10 +281,9 @@ int moments_forward(const Ctx& c, const void* q, const void* k, const void* v, c
                                  states)))
     return rc;
   if (p.mask) {
-    // second-order prefixes go straight to their bf16 copies: behind the kept fp32 states when the
-    // backward will want them again, else in the workspace
-    void* second16 = total_keep ? (void*)((char*)total_keep + moment_state_bytes(p, p.nk)) : s16;
-    return moments_forward_finish(c, q, k, v, stats, states, nullptr, o_add, den_add, s16, o, second16);
+    // second-order prefixes go straight to their bf16 copies; those for the backward lie behind the kept fp32 states
+    void* keep_b = total_keep ? (void*)((char*)total_keep + moment_state_bytes(p, p.nk)) : nullptr;
+    return moments_forward_finish(c, q, k, v, stats, states, nullptr, o_add, den_add, s16, o, true, keep_b);
   }
   // unmasked: every query reads the total of all keys
   const int nchunk = (p.nk + L - 1) / L;
@@ -286,7 +310,9 @@ int moments_leave_states(const Ctx& c, const void* k, const void* v, bool aligne
   if (rc) return rc;
   if (!p.mask) return moments_prefix(c, p.bh, nchunk, states, nullptr, total_keep, 0, 0);
   bool ready;
-  return prefix_states(c, nchunk, states, nullptr, 0, true, (char*)total_keep + need, &ready);
+  StateCopies cp;
+  cp.b = (char*)total_keep + need;
+  return prefix_states(c, nchunk, states, nullptr, 0, true, cp, &ready);
 }
 
 // Unmasked forward from a given total state (this device's keys, or the sum over all shards).
@@ -335,9 +361,10 @@ int moments_backward_finish(const Ctx& c, const void* q, const void* k, const vo
   // grad_k and grad_v read the suffix sums of the query/gradient states
   // (nothing reads r_states after this call, so their second-order rows may stay raw: prefix_states)
   bool ready;
-  if ((rc = prefix_states(c, nchunk, r_states, r_base, 1, true, s16, &ready))) return rc;
+  const StateCopies cp = copies_at(p, s16, p.bh * nchunk);
+  if ((rc = prefix_states(c, nchunk, r_states, r_base, 1, true, cp, &ready))) return rc;
   if ((rc = read_states(zeroing(c, r_base ? -1 : nchunk - 1), 2, p.nk, 1, k, v, nullptr, nullptr, 0, nullptr, nullptr,
-                        r_states, s16, stats, gv_add, nullptr, gk_add, ready ? s16 : nullptr)))
+                        r_states, s16, stats, gv_add, nullptr, gk_add, ready ? &cp : nullptr)))
     return rc;
   ChunkAdd ca;
   ca.chunk = L;
@@ -382,24 +409,25 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
     // the key/value prefixes are rebuilt (the forward does not keep them), used for grad_q,
     // then the buffer is reused for the query/gradient states
     bool ready = false;
-    const void* kv16 = nullptr;   // second-order bf16 copies of the key/value prefixes, where they exist already
+    StateCopies kv;               // second-order bf16 copies of the key/value prefixes, where they exist already
     if (!kv_total_kept) {
       if ((rc = moments_build_states(skipping(c, nck - 1), p.nk, k, v, nullptr, nullptr, 0, nullptr, nullptr, states)))
         return rc;
-      if ((rc = prefix_states(c, nck, states, nullptr, 0, true, s16, &ready))) return rc;
-      if (ready) kv16 = s16;
+      kv.b = s16;
+      if ((rc = prefix_states(c, nck, states, nullptr, 0, true, kv, &ready))) return rc;
     } else if (moment_kept16_bytes(p) > 0) {
-      kv16 = (const char*)kv_total_kept + moment_state_bytes(p, p.nk);
+      kv.b = (char*)const_cast<float*>(kv_total_kept) + moment_state_bytes(p, p.nk);
+      ready = true;
     }
     if (first_fused(p)) {
-      const float* kv = kv_total_kept ? kv_total_kept : states;
+      const float* sums = kv_total_kept ? kv_total_kept : states;
       ChunkAdd own;
       own.chunk = L;
-      if ((rc = first_tc_convert(c, p.bh * nck, kv, s16, nck, stats))) return rc;
-      const FirstState before = {kv, s16, 0};
+      if ((rc = first_tc_convert(c, p.bh * nck, sums, s16, nck, stats))) return rc;
+      const FirstState before = {sums, s16, 0};
       if ((rc = dense_tc_short_dq(c, q, k, v, gs, dvec, stats, dots, grad_q, &own, &before))) return rc;
       if ((rc = moments_build_states(skipping(c, 0), p.nq, q, grad_out, den, delta, 1, gs, dvec, states))) return rc;
-      if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, s16, &ready))) return rc;
+      if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, kv, &ready))) return rc;
       if ((rc = first_tc_convert(c, p.bh * ncq, states, s16, ncq, stats))) return rc;
       const FirstState after = {states, s16, ncq - 1};
       if ((rc = dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, &own, &after))) return rc;
@@ -408,12 +436,14 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
     // grad_q: the first chunk's tokens have no keys before their chunk; grad_k, grad_v: the last chunk's
     // tokens no queries after theirs, and nothing reads the query/gradient state of the first chunk
     if ((rc = read_states(zeroing(c, 0), 1, p.nq, 1, q, grad_out, den, delta, 1, gs, dvec,
-                          kv_total_kept ? kv_total_kept : states, s16, stats, nullptr, nullptr, gq_add, kv16)))
+                          kv_total_kept ? kv_total_kept : states, s16, stats, nullptr, nullptr, gq_add,
+                          ready ? &kv : nullptr)))
       return rc;
     if ((rc = moments_build_states(skipping(c, 0), p.nq, q, grad_out, den, delta, 1, gs, dvec, states))) return rc;
-    if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, s16, &ready))) return rc;
+    const StateCopies qg = copies_at(p, s16, p.bh * ncq);
+    if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, qg, &ready))) return rc;
     if ((rc = read_states(zeroing(c, ncq - 1), 2, p.nk, 1, k, v, nullptr, nullptr, 0, nullptr, nullptr, states, s16,
-                          stats, gv_add, nullptr, gk_add, ready ? s16 : nullptr)))
+                          stats, gv_add, nullptr, gk_add, ready ? &qg : nullptr)))
       return rc;
     ChunkAdd ca;
     ca.chunk = L;

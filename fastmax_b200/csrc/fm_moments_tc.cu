@@ -1,26 +1,10 @@
-// Second-order part of the moment-state form on the tcgen05 tensor cores (bf16
-// operands, fp32 accumulation), head dimension 64.  Two kernels:
-//
-// readout  -- for a tile of 128 tokens x and a prefix state S2[a][b][c] (symmetric in
-//   a, b; c = 0..63 value columns, c = 64 the normaliser column):
-//       T[i][c][b] = sum_a x_i[a] S2[a][b][c]                   tensor cores
-//       type A:  r_i[c] = A2   sum_b x_i[b] T[i][c][b]          (numerator | denominator, grad_v)
-//       type B:  r_i[b] = 2 A2 sum_c ut_i[c] T[i][c][b]         (grad_q, grad_k)
-//   The state is read as bf16 rows (c*64 + b) of 64 a-values -- a K-major B operand
-//   streamed by TMA -- and T never leaves the SM: each 128-column slice of it is
-//   produced in tensor memory and contracted by the CUDA cores straight from there.
-//   This replaces the d*d-wide feature contraction of the reference
-//   (`old stuff/fastmax_cuda_forward_quad.cu`:111-135, 240-268 and the matching
-//   backward loops) by a GEMM of the raw token tile against the state.
-//
-// state    -- T2[(a,b)][c] = sum_j y_j[a] y_j[b] z_j[c] over the tokens of a chunk: the
-//   features y_a y_b (each unordered pair once) are formed on the CUDA cores and written
-//   to tensor memory as the A operand, the value tile is the MN-major B operand delivered
-//   by TMA, and the accumulators stay in tensor memory for the whole chunk.
-//
-// The normaliser column of the state build is a third, small tensor-core kernel here; the
-// first-order and constant rows of the state stay on the kernels of fm_first_tc.cu and
-// fm_moments_ffma.cu.
+// Chunk states of the moment-state form, second-order rows, on the tcgen05 tensor cores (bf16 operands, fp32
+// accumulation), head dimension 64 (the read-out is fm_readout.cu):
+//   T2[(a,b)][c] = sum_j y_j[a] y_j[b] z_j[c] over the tokens of a chunk: the features y_a y_b (each unordered pair
+//   once) are formed on the CUDA cores and written to tensor memory as the A operand, the value tile is the MN-major
+//   B operand delivered by TMA, and the accumulators stay in tensor memory for the whole chunk.
+// The normaliser column is a second, small tensor-core kernel here; the first-order and constant rows of the state stay
+// on the kernels of fm_first_tc.cu and fm_moments_ffma.cu.
 #include <cstdlib>
 
 #include "fm_common.cuh"
@@ -34,8 +18,6 @@ namespace {
 using namespace sm100;
 
 constexpr int D = 64;
-constexpr int NROWS_T = 65 * 64;          // rows (c, b) of the transposed bf16 state
-constexpr int NROWS_TP = 34 * 128;        // the first-order blocks (see first_rows_to_bf16t) and padding to whole 128-row tiles
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_mtc_status, 0, code); }
 // 16 bytes from / 4 bytes to shared memory by shared-window address (keeps the access off the generic path)
@@ -46,430 +28,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t saddr) {
 }
 __device__ __forceinline__ void sts32(uint32_t saddr, uint32_t v) {
   asm volatile("st.shared.b32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory");
-}
-
-// =====================================================================================
-// readout
-// =====================================================================================
-struct RtArgs {
-  const void* x;       // (heads, n, 64) bf16 tokens
-  const void* u;       // type B: (heads, n, 64) bf16 second operand (gs or v)
-  const float* uvec;   // type B: (heads, n) dvec, whose negative is the 65th entry of ut; null = 1
-  float* out_a;        // type A result (heads, n, 64) fp32
-  float* den_a;        // type A normaliser column (heads, n), may be null
-  float* out_b;        // type B result (heads, n, 64) fp32
-  const stat_t* stat_q;
-  const stat_t* stat_k;
-  float a2, lim;
-  int n, chunk, nchunk, state_per_chunk;
-  int wide_io;         // out_a / out_b are 32-byte aligned
-  int zero_chunk;      // tokens of this chunk read an empty state: zeros are written, nothing is multiplied (-1: none)
-  // Type A also adds the first-order and constant terms when state_f32 is given: x . S1 comes out of the last
-  // slice (the copy's rows 65*64..), the constant row and S1's normaliser column are read from the fp32 state.
-  const float* state_f32;
-  size_t per_state;
-  int dvp;
-  float a0, a1;
-  // Type B does the same with one more slice: u . S1[a][0..63] from the tensor core (the copy's rows 66*64..,
-  // the u tile as the A operand) plus e * S1[a][64] from the fp32 state.
-  int first_b;
-  int mode;            // 0: type A on two token tiles, 1: type B on two token tiles,
-                       // 2: one token tile, group 0 type A and group 1 type B
-};
-
-constexpr int RT_THREADS = 352;   // warps 0-3 group 0, 4-7 group 1, 8 TMA producer, 9 and 10 MMA issuers
-constexpr int RT_NS = 4;          // state-tile ring stages
-constexpr int RT_TILE = 128 * D * 2;
-constexpr int RT_OFF_X = 0;                         // two token tiles
-constexpr int RT_OFF_ST = 2 * RT_TILE;              // ring
-constexpr int RT_OFF_U = RT_OFF_ST + RT_NS * RT_TILE;    // two u tiles (type B with the first-order slice)
-constexpr int RT_OFF_UT = RT_OFF_U + 2 * RT_TILE;        // [2][128][66] fp32 (type B operand rows)
-constexpr int RT_UT_LD = 66;
-constexpr int RT_OFF_BAR = RT_OFF_UT + 2 * 128 * RT_UT_LD * 4;
-constexpr int RT_NBAR = 1 + 2 * RT_NS + 8;
-constexpr int RT_OFF_TMEM = RT_OFF_BAR + RT_NBAR * 8;
-constexpr int RT_OFF_VEC = RT_OFF_TMEM + 16;        // per type-A group: constant row [65] | S1 normaliser column [64]
-constexpr int RT_VEC = 132;
-constexpr int RT_SMEM = RT_OFF_VEC + 2 * RT_VEC * 4 + 1024;
-constexpr int RT_NT = 33;                           // slices of 128 columns of T; slice 33 is type B's first-order one
-
-__global__ void __launch_bounds__(RT_THREADS, 1)
-readout_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmS,
-                  const __grid_constant__ CUtensorMap tmU, const RtArgs a) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar0 = sbase + RT_OFF_BAR;
-  // barriers: x | st_full[NS] | st_empty[NS] | t_full[tile][buf] (4) | t_free[tile][buf] (4)
-  auto BAR_X = [&]() { return bar0; };
-  auto BAR_FULL = [&](int s) { return bar0 + 8u * (1 + s); };
-  auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (1 + RT_NS + s); };
-  auto BAR_TFULL = [&](int t, int b) { return bar0 + 8u * (1 + 2 * RT_NS + t * 2 + b); };
-  auto BAR_TFREE = [&](int t, int b) { return bar0 + 8u * (5 + 2 * RT_NS + t * 2 + b); };
-  volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + RT_OFF_TMEM);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_per_cta = (a.mode == 2) ? 1 : 2;
-  const int ctas_per_head = (a.n + 128 * tiles_per_cta - 1) / (128 * tiles_per_cta);
-  const int head = blockIdx.x / ctas_per_head;
-  const int tok0 = (blockIdx.x % ctas_per_head) * 128 * tiles_per_cta;
-  const int ntile = (tiles_per_cta == 2 && tok0 + 128 < a.n) ? 2 : 1;   // token tiles that have rows
-  const int chunk = a.state_per_chunk ? tok0 / a.chunk : 0;
-  const int srow = head * (a.state_per_chunk ? a.nchunk : 1) + chunk;   // index of the state matrix
-  const int readers = (a.mode == 2) ? 8 : 4;                            // warps that read each T buffer
-  const int nslice = RT_NT + (a.first_b ? 1 : 0);
-  if (a.state_per_chunk && chunk == a.zero_chunk) {
-    // the whole CTA lies in one chunk (chunks are multiples of 256 tokens): zero rows, no products
-    const int rows = min(128 * tiles_per_cta, a.n - tok0);
-    for (int i = tid; i < rows * (D / 4); i += RT_THREADS) {
-      const size_t e = ((size_t)head * a.n + tok0) * D + (size_t)i * 4;
-      if (a.mode != 1) *(float4*)(a.out_a + e) = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (a.mode != 0) *(float4*)(a.out_b + e) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    if (a.mode != 1 && a.den_a)
-      for (int i = tid; i < rows; i += RT_THREADS) a.den_a[(size_t)head * a.n + tok0 + i] = 0.f;
-    return;
-  }
-
-  if (tid == 0) {
-    mbar_init(BAR_X(), 1);
-    for (int s = 0; s < RT_NS; ++s) { mbar_init(BAR_FULL(s), 1); mbar_init(BAR_EMPTY(s), a.mode == 2 ? 1 : ntile); }
-    for (int t = 0; t < 2; ++t)
-      for (int b = 0; b < 2; ++b) { mbar_init(BAR_TFULL(t, b), 1); mbar_init(BAR_TFREE(t, b), readers); }
-    mbar_fence_init();
-  }
-  if (warp == 9) tmem_alloc(smem_u32((const void*)tmem_slot), 512);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-
-  if (warp == 8) {
-    // ---------------- TMA producer: token tiles once, then the 33 state tiles ----------------
-    if (lane == 0) {
-      tma_prefetch_desc(&tmX);
-      tma_prefetch_desc(&tmS);
-      mbar_expect_tx(BAR_X(), (a.first_b ? 2 : 1) * ntile * RT_TILE);
-      for (int t = 0; t < ntile; ++t) tma_load_3d(sbase + RT_OFF_X + t * RT_TILE, &tmX, BAR_X(), 0, tok0 + t * 128, head);
-      if (a.first_b) {
-        tma_prefetch_desc(&tmU);
-        for (int t = 0; t < ntile; ++t) tma_load_3d(sbase + RT_OFF_U + t * RT_TILE, &tmU, BAR_X(), 0, tok0 + t * 128, head);
-      }
-    }
-    for (int n = 0; n < nslice; ++n) {
-      const int s = n % RT_NS;
-      if (!mbar_wait(BAR_EMPTY(s), (((n / RT_NS) & 1) ^ 1))) { report(21); break; }
-      if (lane == 0) {
-        mbar_expect_tx(BAR_FULL(s), RT_TILE);
-        tma_load_3d(sbase + RT_OFF_ST + s * RT_TILE, &tmS, BAR_FULL(s), 0, n * 128, srow);
-      }
-    }
-  } else if (warp >= 9) {
-    // ---------------- MMA issuers: the whole warp runs the loop, one elected lane issues ----------------
-    // Two warps, so that the barrier checks of one overlap the products of the other (the
-    // tensor pipe's queue is short: a single issuer leaves it idle between slices).  With two
-    // token tiles issuer w owns tile w; with one tile the issuers take alternate slices, so
-    // each owns one T buffer and the ring stages of its parity.
-    const int w = warp - 9;
-    const bool one_tile = a.mode == 2;
-    if (one_tile || w < ntile) {
-      constexpr uint32_t idesc = idesc_bf16(128, 128, 0, 0);
-      bool ok = mbar_wait_warp(BAR_X(), 0);
-      if (!ok) report(22);
-      tc_fence_after();
-      const uint32_t st0 = desc_lo(sbase + RT_OFF_ST, 16);
-      const int t = one_tile ? 0 : w;
-      const uint32_t x_lo = desc_lo(sbase + RT_OFF_X + t * RT_TILE, 16);
-      const uint32_t u_lo = desc_lo(sbase + RT_OFF_U + t * RT_TILE, 16);
-      for (int n = one_tile ? w : 0; ok && n < nslice; n += one_tile ? 2 : 1) {
-        const int s = n % RT_NS, buf = n & 1;
-        if (!mbar_wait_warp(BAR_FULL(s), (uint32_t)((n / RT_NS) & 1))) { report(23); break; }
-        // the buffer was last used by slice n-2
-        if (n >= 2 && !mbar_wait_warp(BAR_TFREE(t, buf), (uint32_t)(((n >> 1) - 1) & 1))) { report(24); break; }
-        tc_fence_after();
-        if (elect_one()) {
-          umma_ss_k64(tmem + t * 256 + buf * 128, n < RT_NT ? x_lo : u_lo, st0 + (uint32_t)s * (RT_TILE >> 4), idesc);
-          umma_commit(BAR_TFULL(t, buf));
-          umma_commit(BAR_EMPTY(s));
-        }
-        __syncwarp();
-      }
-    }
-    __syncwarp();
-  } else {
-    // ---------------- contraction groups ----------------
-    const int g = warp >> 2, qd = warp & 3;
-    const int t = (a.mode == 2) ? 0 : g;                 // token tile this group reads
-    const bool type_b = (a.mode == 1) || (a.mode == 2 && g == 1);
-    if (t < ntile) {
-      const int tok = tok0 + t * 128 + qd * 32 + lane;
-      const bool tok_ok = tok < a.n;
-      const size_t grow = (size_t)head * a.n + (tok_ok ? tok : 0);
-      const float c = stat_scale(a.stat_q, head, a.lim) * stat_scale(a.stat_k, head, a.lim);
-      const float A2 = a.a2 * c * c;
-      const uint32_t tbase = tmem + t * 256 + ((uint32_t)(qd * 32) << 16);
-      // 32 packed fp32 pairs per thread: type A keeps its token row here, type B its 64 running sums
-      // (one array for both, so that neither kind carries the other's registers through the loop)
-      uint64_t xa[32];
-      if (!type_b) {
-        const uint4* xr = (const uint4*)((const __nv_bfloat16*)a.x + grow * D);
-#pragma unroll
-        for (int v8 = 0; v8 < 8; ++v8) {
-          uint4 w = tok_ok ? __ldg(xr + v8) : make_uint4(0, 0, 0, 0);
-          const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            xa[v8 * 4 + e] = pack2(__uint_as_float(ww[e] << 16), __uint_as_float(ww[e] & 0xFFFF0000u));
-        }
-      }
-      float* ut = (float*)(smem + RT_OFF_UT) + ((size_t)g * 128 + qd * 32 + lane) * RT_UT_LD;
-      if (type_b) {
-        // ut row = [u_0 .. u_63 | e]; only this thread reads it back
-        const uint4* ur = (const uint4*)((const __nv_bfloat16*)a.u + grow * D);
-#pragma unroll
-        for (int v8 = 0; v8 < 8; ++v8) {
-          uint4 w = tok_ok ? __ldg(ur + v8) : make_uint4(0, 0, 0, 0);
-          const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            ut[v8 * 8 + 2 * e] = __uint_as_float(ww[e] << 16);
-            ut[v8 * 8 + 2 * e + 1] = __uint_as_float(ww[e] & 0xFFFF0000u);
-          }
-        }
-        ut[64] = tok_ok ? (a.uvec ? -a.uvec[grow] : 1.0f) : 0.f;
-#pragma unroll
-        for (int e = 0; e < 32; ++e) xa[e] = pack2(0.f, 0.f);
-      }
-      const bool first_too = !type_b && a.state_f32 != nullptr;
-      const bool first_b = type_b && a.first_b != 0;
-      const float A1f = a.a1 * c;
-      float k_out = 2.f * A2;                                  // type B: factor of the running sums at the end
-      float* vec = (float*)(smem + RT_OFF_VEC) + g * RT_VEC;   // crow[0..64] | ncol[0..63]
-      if (first_too || first_b) {
-        // the group's 128 threads stage the two vectors of this CTA's state (all of them reach the barrier:
-        // a group is of one kind)
-        const float* fs = a.state_f32 + (size_t)srow * a.per_state + (size_t)(64 * 64) * a.dvp;   // first-order rows
-        const int i = qd * 32 + lane;
-        if (i < 65) vec[i] = __ldg(fs + (size_t)64 * a.dvp + i);               // constant row
-        if (i < 64) vec[65 + i] = __ldg(fs + (size_t)i * a.dvp + 64);           // S1[a][64]
-        if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-        else asm volatile("bar.sync 2, 128;" ::: "memory");
-      }
-      bool ok = true;
-      for (int n = 0; n < nslice; ++n) {
-        const int buf = n & 1;
-        if (n == RT_NT && !type_b) break;     // the last slice is type B's alone (nothing waits for its release)
-        if (!mbar_wait(BAR_TFULL(t, buf), (uint32_t)((n >> 1) & 1))) { report(25); ok = false; break; }
-        tc_fence_after();
-        if (n == RT_NT) {
-          // first-order slice: T1[a] = u . S1[a][0..63] in the first 64 columns; the running sums take their
-          // final factor here and the first-order term joins them
-          uint32_t tv[64];
-          tmem_ld64(tbase + buf * 128, tv);
-          tmem_wait_ld();
-          const float ue = ut[64];
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            float f0, f1;
-            unpack2(xa[e], f0, f1);
-            f0 = fmaf(k_out, f0, A1f * fmaf(ue, vec[65 + 2 * e], __uint_as_float(tv[2 * e])));
-            f1 = fmaf(k_out, f1, A1f * fmaf(ue, vec[66 + 2 * e], __uint_as_float(tv[2 * e + 1])));
-            xa[e] = pack2(f0, f1);
-          }
-          k_out = 1.f;
-          break;
-        }
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          const int cidx = 2 * n + hf;       // column c of the state this half belongs to
-          uint32_t tv[64];
-          tmem_ld64(tbase + buf * 128 + hf * 64, tv);
-          tmem_wait_ld();
-          if (hf == 1) {                      // both halves are in registers or consumed: release
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(BAR_TFREE(t, buf));
-          }
-          if (cidx > 64) {                    // the last 64 rows of the copy: the first-order block
-            if (first_too) {
-              // T1[c] = x . S1[:, c] in this half; the normaliser column's first-order part is a dot on the CUDA cores
-#pragma unroll
-              for (int cc = 0; cc < 64; ++cc) ut[cc] += fmaf(A1f, __uint_as_float(tv[cc]), a.a0 * vec[cc]);
-              uint64_t s4[4] = {pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f)};
-#pragma unroll
-              for (int e = 0; e < 32; ++e) s4[e & 3] = fma2(xa[e], pack2(vec[65 + 2 * e], vec[66 + 2 * e]), s4[e & 3]);
-              float lo, hi;
-              unpack2(add2(add2(s4[0], s4[1]), add2(s4[2], s4[3])), lo, hi);
-              ut[64] += fmaf(A1f, lo + hi, a.a0 * vec[64]);
-            }
-            continue;
-          }
-          if (!type_b) {
-            uint64_t s4[4] = {pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f)};
-#pragma unroll
-            for (int e = 0; e < 32; ++e) s4[e & 3] = fma2(xa[e], pack2u(tv[2 * e], tv[2 * e + 1]), s4[e & 3]);
-            float lo, hi;
-            unpack2(add2(add2(s4[0], s4[1]), add2(s4[2], s4[3])), lo, hi);
-            ut[cidx] = A2 * (lo + hi);      // staged in this thread's row, written out at the end
-          } else {
-            const float uc = ut[cidx];
-            const uint64_t u2 = pack2(uc, uc);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) xa[e] = fma2(u2, pack2u(tv[2 * e], tv[2 * e + 1]), xa[e]);
-          }
-        }
-      }
-      if (ok && !type_b && tok_ok) {
-        // a thread owns its 256-byte row: 32-byte stores write whole sectors
-        float* dst = a.out_a + grow * D;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          uint32_t w[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) w[q] = __float_as_uint(ut[8 * e + q]);
-          stg32(dst + 8 * e, w, a.wide_io != 0);
-        }
-        if (a.den_a) a.den_a[grow] = ut[64];
-      }
-      if (ok && type_b && tok_ok) {
-        const float k2 = k_out;
-        float* dst = a.out_b + grow * D;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          uint32_t w[8];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            float f0, f1;
-            unpack2(xa[4 * e + q], f0, f1);
-            w[2 * q] = __float_as_uint(k2 * f0);
-            w[2 * q + 1] = __float_as_uint(k2 * f1);
-          }
-          stg32(dst + 8 * e, w, a.wide_io != 0);
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 9) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 512);
-  }
-}
-
-// =====================================================================================
-// bf16 transposed copy of the second-order block of fp32 prefix states:
-//   out[m][c*64 + b][a] = state[m][(b*64 + a)][c]      (S2 is symmetric in a, b)
-// one CTA per (state matrix m, b).  The 64 rows past 65*64 hold the first-order block the same way,
-//   out[m][65*64 + c][a] = state[m][64*64 + a][c],  c < 64
-// so that the read-out's last slice yields x . S1 beside the normaliser column's second-order part, and the
-// 64 rows after those hold it untransposed,
-//   out[m][66*64 + a][c] = state[m][64*64 + a][c],  c < 64
-// the B operand of type B's first-order slice (u . S1[a][:]).  The remaining 64 rows of the last tile are
-// never written; the columns of T they produce are never read.
-// =====================================================================================
-// rows 65*64 .. 65*64 + 63 of one copy from the (summed) first-order rows of its fp32 state
-__device__ __forceinline__ void first_rows_to_bf16t(const float* __restrict__ st, __nv_bfloat16* __restrict__ o,
-                                                    int dvp, float (*blk)[69], int t) {
-  const float* src = st + (size_t)64 * 64 * dvp;     // rows 4096 + a, a = 0..63
-  for (int i = t; i < 64 * dvp; i += 256) blk[i / dvp][i % dvp] = src[i];
-  __syncthreads();
-  uint32_t* ow = (uint32_t*)(o + (size_t)NROWS_T * 64);
-  for (int w = t; w < 64 * 32; w += 256) {
-    const int cc = w >> 5, ap = (w & 31) * 2;
-    ow[64 * 32 + w] = pack_bf16(blk[cc][ap], blk[cc][ap + 1]);     // rows 66*64 + a: S1[a][c], c contiguous (type B)
-    ow[cc * 32 + (w & 31)] = pack_bf16(blk[ap][cc], blk[ap + 1][cc]);
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(256) state_to_bf16t_kernel(const float* __restrict__ state,
-                                                             __nv_bfloat16* __restrict__ out, int dvp,
-                                                             size_t per_state) {
-  __shared__ float blk[64][69];
-  const int m = blockIdx.y, b = blockIdx.x;
-  if (b == 64) {  // the first-order rows (the fp32 state holds running sums already)
-    first_rows_to_bf16t(state + (size_t)m * per_state, out + (size_t)m * NROWS_TP * 64, dvp, blk, threadIdx.x);
-    return;
-  }
-  const float* src = state + (size_t)m * per_state + (size_t)b * 64 * dvp;   // rows (b, a = 0..63)
-  for (int i = threadIdx.x; i < 64 * dvp; i += 256) blk[i / dvp][i % dvp] = src[i];
-  __syncthreads();
-  __nv_bfloat16* o = out + (size_t)m * NROWS_TP * 64;
-  for (int i = threadIdx.x; i < 65 * 64; i += 256) {
-    const int c = i / 64, aa = i % 64;
-    o[((size_t)c * 64 + b) * 64 + aa] = __float2bfloat16_rn(blk[aa][c]);
-  }
-}
-
-// =====================================================================================
-// Running sum over the chunks of a head and the bf16 transposed copy in one pass, second-order
-// rows only:  out[m][c*64 + b][a] = bf16( base[(b*64 + a)][c] + sum of state[m'][(b*64 + a)][c] over
-// the chunks m' before m (after m when reverse) ).  One CTA per (head, b) keeps its 64 x 68 block of
-// the running sum in registers, in fp32, walks the chunks in order and reads every raw chunk state
-// once; the fp32 states are left as they are.  The block with b == 64 copies the first-order rows
-// (already summed in place) into the last 64 rows of every copy.
-// =====================================================================================
-__global__ void __launch_bounds__(256) prefix_bf16t_kernel(const float* __restrict__ state,
-                                                           const float* __restrict__ base,
-                                                           __nv_bfloat16* __restrict__ out, int nchunk, int dvp,
-                                                           size_t per_state, int reverse) {
-  __shared__ float blk[64][69];
-  const int head = blockIdx.y, b = blockIdx.x, t = threadIdx.x;
-  if (b == 64) {
-    // the first-order rows: their running sums were formed in place in the fp32 states before this launch
-    for (int i = 0; i < nchunk; ++i)
-      first_rows_to_bf16t(state + (size_t)(head * nchunk + i) * per_state,
-                          out + (size_t)(head * nchunk + i) * NROWS_TP * 64, dvp, blk, t);
-    return;
-  }
-  constexpr int NV = 64 * 68 / 4;                    // float4 pieces of the block (dvp == 68)
-  const size_t blk_off = (size_t)b * 64 * dvp;       // rows (b, a = 0..63) are contiguous
-  float4 run[5], nxt[5];
-#pragma unroll
-  for (int u = 0; u < 5; ++u) {
-    const int v = t + u * 256;
-    run[u] = (base && v < NV) ? *(const float4*)(base + (size_t)head * per_state + blk_off + 4 * v)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  auto load = [&](int i, float4 (&r)[5]) {
-    const int c = reverse ? nchunk - 1 - i : i;
-    const float* src = state + (size_t)(head * nchunk + c) * per_state + blk_off;
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-      const int v = t + u * 256;
-      // the last chunk in scan order is never added to anything that is written (and may not have been built)
-      r[u] = (i + 1 < nchunk && v < NV) ? __ldcs((const float4*)(src + 4 * v)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  load(0, nxt);
-  for (int i = 0; i < nchunk; ++i) {
-    const int c = reverse ? nchunk - 1 - i : i;
-    // the exclusive running sum of this chunk, transposed through shared memory
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-      const int v = t + u * 256;
-      if (v < NV) {
-        const int e = 4 * v, aa = e / 68, cc = e % 68;   // 68 is a multiple of 4: a piece never straddles rows
-        blk[aa][cc] = run[u].x; blk[aa][cc + 1] = run[u].y; blk[aa][cc + 2] = run[u].z; blk[aa][cc + 3] = run[u].w;
-      }
-    }
-    float4 cur[5];
-#pragma unroll
-    for (int u = 0; u < 5; ++u) cur[u] = nxt[u];
-    load(i + 1, nxt);                                  // in flight during the transposed write
-    __syncthreads();
-    uint32_t* o = (uint32_t*)(out + (size_t)(head * nchunk + c) * NROWS_TP * 64);
-    for (int w = t; w < 65 * 32; w += 256) {
-      const int cc = w >> 5, ap = (w & 31) * 2;
-      o[((size_t)cc * 64 + b) * 32 + (w & 31)] = pack_bf16(blk[ap][cc], blk[ap + 1][cc]);
-    }
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-      run[u].x += cur[u].x; run[u].y += cur[u].y; run[u].z += cur[u].z; run[u].w += cur[u].w;
-    }
-    __syncthreads();
-  }
 }
 
 // =====================================================================================
@@ -501,6 +59,7 @@ struct StArgs {
   int n, chunk, nchunk, dvp;
   size_t per_state;
   int skip_chunk;    // this chunk's state is not wanted (-1: none)
+  int lower;         // only rows (b, a) with a / 16 <= b / 16 are wanted: all that the read-out's copies are made from
 };
 
 constexpr int ST_GEN_WARPS = 16;
@@ -761,8 +320,9 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
         tmem_ld64(tmem + m * 64 + ((uint32_t)(qd * 32) << 16), tv);
         tmem_wait_ld();
       }
-      // the pair's row goes to both of its places in the state, (b, other) and (other, b)
+      // the pair's row goes to both of its places in the state, (b, other) and (other, b), or to those that are read
       for (int side = 0; mine && side < (o == b ? 1 : 2); ++side) {
+      if (a.lower && (side == 0 ? (o >> 4) > (b >> 4) : (b >> 4) > (o >> 4))) continue;
       const int f = side == 0 ? b * 64 + o : o * 64 + b;
       float* dst = st + (size_t)f * a.dvp;
       const uint32_t ecol = ecols[side];
@@ -995,36 +555,6 @@ bool moments_tc_supports(const fastmax_problem& p) {
   return !off && p.impl != FASTMAX_IMPL_MOMENTS_FFMA && p.dtype == FASTMAX_BF16 && p.d == 64 && p.p == 2 && p.bh == p.bhkv;
 }
 
-size_t moments_tc_state_bytes(int mats) { return (size_t)mats * NROWS_TP * 64 * 2; }
-
-int moments_tc_convert(const Ctx& c, int mats, const float* state, void* state_bf16) {
-  if (mats == 0) return FASTMAX_OK;
-  const MomentDims m = moment_dims(64);
-  dim3 grid(65, mats);
-  FM_LAUNCH("fm_moments_state_bf16", c.stream,
-            (state_to_bf16t_kernel<<<grid, 256, 0, c.stream>>>(state, (__nv_bfloat16*)state_bf16, m.dvp,
-                                                               (size_t)m.f * m.dvp)));
-  FM_CUDA_TRY(cudaGetLastError());
-  return FASTMAX_OK;
-}
-
-// Exclusive running sums over chunks (from `base`, per head, may be null) of the second-order rows,
-// written as the read-out's bf16 transposed copies; the fp32 states stay raw.  The first-order rows
-// are the caller's business (moments_prefix with a row range).
-int moments_tc_prefix_convert(const Ctx& c, int heads, int nchunk, const float* state, const float* base,
-                              int reverse, void* state_bf16) {
-  if (heads == 0 || nchunk == 0) return FASTMAX_OK;
-  const MomentDims m = moment_dims(64);
-  if ((((uintptr_t)state | (uintptr_t)base) & 15) != 0)
-    return fail(FASTMAX_E_ARG, "moment states and totals must be 16-byte aligned");
-  dim3 grid(65, heads);
-  FM_LAUNCH("fm_moments_prefix_bf16", c.stream,
-            (prefix_bf16t_kernel<<<grid, 256, 0, c.stream>>>(state, base, (__nv_bfloat16*)state_bf16, nchunk,
-                                                             m.dvp, (size_t)m.f * m.dvp, reverse)));
-  FM_CUDA_TRY(cudaGetLastError());
-  return FASTMAX_OK;
-}
-
 // Second-order rows of the chunk states of (y, z | e) on the tensor cores: columns 0..63 by
 // state_tc_kernel, the e column (e = 1 when dvec is null, else -dvec) by state_ecol_tc_kernel.
 // The first-order and constant rows are NOT valid afterwards (they held the e column's scratch
@@ -1042,6 +572,7 @@ int moments_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void
   a.y = y; a.state = state; a.n = n; a.chunk = chunk; a.nchunk = nchunk; a.dvp = m.dvp;
   a.per_state = (size_t)m.f * m.dvp;
   a.skip_chunk = c.skip_chunk;
+  a.lower = c.lower_rows ? 1 : 0;
   // the normaliser column first: the state kernel picks it up in its epilogue
   CUtensorMap ty;
   if ((rc = make_map(&ty, y, heads, n))) return rc;
@@ -1053,42 +584,6 @@ int moments_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void
   FM_CUDA_TRY(cudaFuncSetAttribute(state_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
   FM_LAUNCH("fm_moments_tc_state", c.stream,
             (state_tc_kernel<<<(unsigned)((size_t)heads * nchunk * ST_SPLIT), ST_THREADS, ST_SMEM, c.stream>>>(tz, a)));
-  FM_CUDA_TRY(cudaGetLastError());
-  return FASTMAX_OK;
-}
-
-// mode 0: type A on x -> out_a (+ den_a);  mode 1: type B on (x, u, uvec) -> out_b;
-// mode 2: both on the same tokens.  Results overwrite; type B holds the second-order part only, type A the
-// whole result when state_f32 (the fp32 states with summed first-order rows) is given.
-int moments_tc_readout(const Ctx& c, int mode, int heads, int n, int chunk, int state_per_chunk,
-                       const void* x, const void* u, const float* uvec, const void* state_bf16,
-                       const stat_t* stats, float* out_a, float* den_a, float* out_b, const float* state_f32) {
-  if (heads == 0 || n == 0) return FASTMAX_OK;
-  const fastmax_problem& p = c.p;
-  const int nchunk = (n + chunk - 1) / chunk;
-  CUtensorMap tx, ts, tu;
-  int rc;
-  const bool first_b = mode != 0 && state_f32 != nullptr && u != nullptr;
-  if ((rc = make_map(&tx, x, heads, n))) return rc;
-  if ((rc = make_map(&tu, first_b ? u : x, heads, n))) return rc;
-  if ((rc = make_map(&ts, state_bf16, (size_t)heads * (state_per_chunk ? nchunk : 1), NROWS_TP))) return rc;
-  RtArgs a;
-  a.first_b = first_b ? 1 : 0;
-  a.x = x; a.u = u; a.uvec = uvec; a.out_a = out_a; a.den_a = den_a; a.out_b = out_b;
-  a.stat_q = p.normalize ? stats : nullptr;
-  a.stat_k = p.normalize ? stats + p.bh : nullptr;
-  a.a2 = p.a2; a.lim = p.lim;
-  a.n = n; a.chunk = chunk; a.nchunk = nchunk; a.state_per_chunk = state_per_chunk; a.mode = mode;
-  a.wide_io = (((uintptr_t)out_a | (uintptr_t)out_b) & 31) == 0;
-  a.zero_chunk = state_per_chunk ? c.zero_chunk : -1;
-  const MomentDims md = moment_dims(64);
-  a.state_f32 = state_f32; a.per_state = (size_t)md.f * md.dvp; a.dvp = md.dvp; a.a0 = p.a0; a.a1 = p.a1;
-  const int per_cta = (mode == 2) ? 128 : 256;
-  const unsigned grid = (unsigned)((size_t)heads * ((n + per_cta - 1) / per_cta));
-  FM_CUDA_TRY(cudaFuncSetAttribute(readout_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM));
-  static const char* const names[3] = {"fm_moments_tc_readout_a", "fm_moments_tc_readout_b",
-                                       "fm_moments_tc_readout_ab"};
-  FM_LAUNCH(names[mode], c.stream, (readout_tc_kernel<<<grid, RT_THREADS, RT_SMEM, c.stream>>>(tx, ts, tu, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
