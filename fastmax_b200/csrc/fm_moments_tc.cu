@@ -50,11 +50,15 @@ __device__ __forceinline__ void sts32(uint32_t saddr, uint32_t v) {
 // is feature x fixed feature, the warp's 32 rows rotated where it is a distance around the
 // ring); warp w covers the TMEM lane quarter w % 4 and 32 tokens.  Shared-memory traffic per
 // block is the transposition, the row reads and the tensor core's reads of the value tile, a
-// fraction of what feature tiles staged in shared memory cost.  The y rows come straight from global memory into
-// registers two blocks ahead; the producer warp asks for them in L2 earlier still.
+// fraction of what feature tiles staged in shared memory cost.  The y tile comes by TMA beside
+// the value tile and is transposed one block ahead, between the stores of a pair of tiles and their hand-over.
+//   What bounds it: the chain of a block (row reads, products, TMEM stores, hand-over) and the load/store unit, 1 500
+// cycles a block for rotated rows.  Measured, 1024 heads x 8192 tokens of chunks with a state, a launch: 3.7 ms; 4.7 ms
+// with the rows read from global memory by the threads that transpose them (32 lines a request kept the load/store unit
+// 75-80 % busy); 3.85 ms with the transposition at the head of its own block, 4.5 ms with the second pair handed over at
+// the start of the next block.
 // =====================================================================================
 struct StArgs {
-  const void* y;     // (heads, n, 64) bf16 feature source
   float* state;      // (heads, nchunk, F, DVP) fp32; rows a*64+b and b*64+a of each pair, columns 0..64 and padding
   int n, chunk, nchunk, dvp;
   size_t per_state;
@@ -66,22 +70,22 @@ constexpr int ST_GEN_WARPS = 16;
 constexpr int ST_THREADS = (ST_GEN_WARPS + 3) * 32;   // warps 0-15: generators; 16: TMA; 17, 18: MMA issuers
 constexpr int ST_TILES = 4;           // accumulator tiles (and feature buffers) per CTA
 constexpr int ST_SPLIT = 5;            // CTAs per (head, chunk): four of four tiles and one of one tile
-constexpr int ST_NZ = 3;              // value-tile ring
+constexpr int ST_NZ = 3;              // ring of value and feature tiles
 constexpr int ST_ZTILE = 128 * 128;
+constexpr int ST_STAGE = 2 * ST_ZTILE;  // z tile, y tile
 constexpr int ST_YT_LD = 272;         // bytes per yT row: 128 tokens + 16 (conflict-free 16-byte reads down a column)
 constexpr int ST_YT = 64 * ST_YT_LD;
 constexpr int ST_OFF_Z = 0;
-constexpr int ST_OFF_YT = ST_NZ * ST_ZTILE;          // two transposed blocks
+constexpr int ST_OFF_YT = ST_NZ * ST_STAGE;          // two transposed blocks
 constexpr int ST_OFF_BAR = ST_OFF_YT + 2 * ST_YT;
 constexpr int ST_NBAR = 5 * ST_TILES + 2 * ST_NZ + 1;
 constexpr int ST_OFF_TMEM = ST_OFF_BAR + ST_NBAR * 8;
 constexpr int ST_SMEM = ST_OFF_TMEM + 16 + 1024;
 constexpr int ST_TM_A = 64 * ST_TILES;               // first TMEM column of the feature buffers
-constexpr int ST_L2_AHEAD = 5;                       // blocks between the L2 request and the use of y rows
 static_assert(ST_TILES == 4 && ST_GEN_WARPS == 16, "the epilogue gives one tile to each group of four warps");
 
 __global__ void __launch_bounds__(ST_THREADS, 1)
-state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
+state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmY, const StArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -105,13 +109,12 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
   const int t_begin = chunk * a.chunk, t_end = min(a.n, t_begin + a.chunk);
   const int nblk = (t_end - t_begin + 127) / 128;
   const int ntile = part == 4 ? 1 : ST_TILES;
-  const __nv_bfloat16* ybase = (const __nv_bfloat16*)a.y + (size_t)head * a.n * D;
 
   if (tid == 0) {
     for (int m = 0; m < ST_TILES; ++m)
       for (int h = 0; h < 2; ++h) { mbar_init(BAR_AFULL(m, h), ST_GEN_WARPS / 2); mbar_init(BAR_AEMPTY(m, h), 1); }
     for (int m = 0; m < ST_TILES; ++m) mbar_init(BAR_START(m), 1);
-    for (int s = 0; s < ST_NZ; ++s) { mbar_init(BAR_ZFULL(s), 1); mbar_init(BAR_ZEMPTY(s), 2); }
+    for (int s = 0; s < ST_NZ; ++s) { mbar_init(BAR_ZFULL(s), 1); mbar_init(BAR_ZEMPTY(s), 2 + ST_GEN_WARPS); }
     mbar_init(BAR_DONE(), 2);
     mbar_fence_init();
   }
@@ -122,25 +125,16 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
   const uint32_t tmem = *tmem_slot;
 
   if (warp == ST_GEN_WARPS) {
-    // ---- producer: value tiles by TMA, and L2 requests for the y rows of later blocks ----
-    if (lane == 0) tma_prefetch_desc(&tmZ);
-    auto ask_l2 = [&](int k) {
-      if (k >= nblk) return;
-      for (int i = lane; i < 128; i += 32) {
-        const int tok = t_begin + k * 128 + i;
-        if (tok < t_end) asm volatile("prefetch.global.L2 [%0];" ::"l"(ybase + (size_t)tok * D));
-      }
-    };
-    for (int k = 2; k < ST_L2_AHEAD; ++k) ask_l2(k);
+    // ---- producer: value and feature tiles by TMA ----
+    if (lane == 0) { tma_prefetch_desc(&tmZ); tma_prefetch_desc(&tmY); }
     for (int k = 0; k < nblk; ++k) {
       const int s = k % ST_NZ;
-      ask_l2(k + ST_L2_AHEAD);
       if (!mbar_wait(BAR_ZEMPTY(s), (((k / ST_NZ) & 1) ^ 1))) { report(31); break; }
       if (lane == 0) {
-        mbar_expect_tx(BAR_ZFULL(s), ST_ZTILE);
-        // rows past the end of the sequence are zero-filled by TMA; rows past the end of the
-        // chunk but inside the sequence are cancelled by zero features
-        tma_load_3d(sbase + ST_OFF_Z + s * ST_ZTILE, &tmZ, BAR_ZFULL(s), 0, t_begin + k * 128, head);
+        mbar_expect_tx(BAR_ZFULL(s), ST_STAGE);
+        // rows past the end of the sequence are zero-filled; chunks are whole multiples of 128 tokens
+        tma_load_3d(sbase + ST_OFF_Z + s * ST_STAGE, &tmZ, BAR_ZFULL(s), 0, t_begin + k * 128, head);
+        tma_load_3d(sbase + ST_OFF_Z + s * ST_STAGE + ST_ZTILE, &tmY, BAR_ZFULL(s), 0, t_begin + k * 128, head);
       }
     }
   } else if (warp > ST_GEN_WARPS) {
@@ -154,7 +148,7 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
     for (int k = 0; ok && k < nblk; ++k) {
       const int s = k % ST_NZ;
       if (!mbar_wait_warp(BAR_ZFULL(s), (uint32_t)((k / ST_NZ) & 1))) { report(32); ok = false; break; }
-      const uint32_t z_lo = desc_lo(sbase + ST_OFF_Z + s * ST_ZTILE, ST_ZTILE) + (uint32_t)w * (4 * 128);
+      const uint32_t z_lo = desc_lo(sbase + ST_OFF_Z + s * ST_STAGE, ST_ZTILE) + (uint32_t)w * (4 * 128);
       if (ntile == 1) {
         // one tile: its four feature buffers are a ring over blocks, so that the threads that form the
         // features run ahead of the products instead of waiting for each one
@@ -205,39 +199,55 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
     const int tok_off = h * 64 + tq * 32;           // first of this warp's 32 tokens in the block
     // transposition duty inside the half: token pair jp (of 32) and 8 features from fg * 8
     const int jp = tid & 31, fg = (tid >> 5) & 7;
-    auto load_rows = [&](int k, uint4 (&r)[2]) {
-      const int tok = t_begin + k * 128 + h * 64 + 2 * jp;
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-        r[t] = (k < nblk && tok + t < t_end) ? __ldg((const uint4*)(ybase + (size_t)(tok + t) * D + fg * 8))
-                                             : make_uint4(0, 0, 0, 0);
-    };
-    uint4 rows[2], rows_next[2];
-    load_rows(0, rows);
-    load_rows(1, rows_next);
-    const uint32_t ta = tmem + ST_TM_A + h * 32 + tq * 16 + ((uint32_t)(qd * 32) << 16);   // this warp's part of feature buffer 0
+    // Its two rows of block k, 16 bytes each, from the y tile.  The lanes of every other group of four read the odd row
+    // first: eight neighbouring lanes then meet eight different rows modulo 8, so eight different 16-byte banks.
+    const uint32_t swap = (uint32_t)(jp >> 2) & 1;
     bool ok = true;
+    uint4 rows[2];
+    auto load_rows = [&](int k) {
+      if (k >= nblk || !ok) return;
+      const int s = k % ST_NZ;
+      if (!mbar_wait(BAR_ZFULL(s), (uint32_t)((k / ST_NZ) & 1))) { report(37); ok = false; return; }
+      const uint32_t r0 = h * 64 + 2 * jp + swap, r1 = r0 ^ 1;
+      const uint32_t tile = sbase + ST_OFF_Z + s * ST_STAGE + ST_ZTILE;
+      rows[0] = lds128(tile + r0 * 128 + ((fg ^ (r0 & 7)) << 4));
+      rows[1] = lds128(tile + r1 * 128 + ((fg ^ (r1 & 7)) << 4));
+    };
+    // ... and into yT: word (feature f, token pair) = two consecutive tokens of feature f
+    auto transpose = [&](int k) {
+      if (k >= nblk) return;
+      const uint4 even = swap ? rows[1] : rows[0], odd = swap ? rows[0] : rows[1];
+      const uint32_t t0[4] = {even.x, even.y, even.z, even.w};
+      const uint32_t t1[4] = {odd.x, odd.y, odd.z, odd.w};
+      const uint32_t col = sbase + ST_OFF_YT + (k & 1) * ST_YT + (fg * 8) * ST_YT_LD + (h * 32 + jp) * 4;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        sts32(col + (2 * e) * ST_YT_LD, __byte_perm(t0[e], t1[e], 0x5410));
+        sts32(col + (2 * e + 1) * ST_YT_LD, __byte_perm(t0[e], t1[e], 0x7632));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_ZEMPTY(k % ST_NZ));   // the y tile has been read
+    };
+    // the warp's stores to feature buffers m0 and m1 are complete: hand them over
+    auto hand_over = [&](int m0, int m1) {
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(BAR_AFULL(m0, h));
+        if (m1 >= 0) mbar_arrive(BAR_AFULL(m1, h));
+      }
+    };
+    load_rows(0);
+    transpose(0);
+    const uint32_t ta = tmem + ST_TM_A + h * 32 + tq * 16 + ((uint32_t)(qd * 32) << 16);   // this warp's part of feature buffer 0
     for (int k = 0; k < nblk; ++k) {   // every generator thread takes part in every block's barrier
       const uint32_t yt = sbase + ST_OFF_YT + (k & 1) * ST_YT;
-      {
-        // word (feature f, token pair) = two consecutive tokens of feature f
-        const uint32_t t0[4] = {rows[0].x, rows[0].y, rows[0].z, rows[0].w};
-        const uint32_t t1[4] = {rows[1].x, rows[1].y, rows[1].z, rows[1].w};
-        const uint32_t col = yt + (fg * 8) * ST_YT_LD + (h * 32 + jp) * 4;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          sts32(col + (2 * e) * ST_YT_LD, __byte_perm(t0[e], t1[e], 0x5410));
-          sts32(col + (2 * e + 1) * ST_YT_LD, __byte_perm(t0[e], t1[e], 0x7632));
-        }
-      }
-      rows[0] = rows_next[0];
-      rows[1] = rows_next[1];
-      load_rows(k + 2, rows_next);                  // two blocks ahead
       if (h == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
       else asm volatile("bar.sync 2, 256;" ::: "memory");
-      // Reuse of a yT buffer two blocks later needs no second barrier: a thread that writes block
-      // k + 2 has passed the barrier of block k + 1, which every thread of its half reaches only
-      // after its reads of block k (a half reads only the token columns it wrote).
+      // Block k is transposed, and every thread of the half is done with its reads of block k - 1: its buffer takes block
+      // k + 1 below, while the products of block k are formed (a half reads only the token columns it wrote).
+      load_rows(k + 1);
       if (!ok) continue;
       uint32_t yb[16];
       {
@@ -273,10 +283,8 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
         if (!mbar_wait(BAR_AEMPTY(fb, h), (uint32_t)(((k >> 2) & 1) ^ 1))) { report(34); ok = false; continue; }
         tc_fence_after();
         tmem_st16(ta + 64 * fb, p0);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(BAR_AFULL(fb, h));
+        transpose(k + 1);
+        hand_over(fb, -1);
         continue;
       }
       products(1, p1);
@@ -284,20 +292,15 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const StArgs a) {
       tc_fence_after();
       tmem_st16(ta, p0);
       tmem_st16(ta + 64, p1);
+      transpose(k + 1);
       products(2, p2);
       products(3, p3);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(BAR_AFULL(0, h)); mbar_arrive(BAR_AFULL(1, h)); }
+      hand_over(0, 1);
       if (!mbar_wait(BAR_AEMPTY(3, h), (uint32_t)((k & 1) ^ 1))) { report(34); ok = false; continue; }
       tc_fence_after();
       tmem_st16(ta + 128, p2);
       tmem_st16(ta + 192, p3);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(BAR_AFULL(2, h)); mbar_arrive(BAR_AFULL(3, h)); }
+      hand_over(2, 3);
     }
     // ---- epilogue: accumulator rows -> fp32 state (columns 0..63), the normaliser column from the
     // block state_ecol_tc_kernel left in the first-order rows, zero padding ----
@@ -569,7 +572,7 @@ int moments_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void
   int rc;
   if ((rc = make_map(&tz, z, heads, n))) return rc;
   StArgs a;
-  a.y = y; a.state = state; a.n = n; a.chunk = chunk; a.nchunk = nchunk; a.dvp = m.dvp;
+  a.state = state; a.n = n; a.chunk = chunk; a.nchunk = nchunk; a.dvp = m.dvp;
   a.per_state = (size_t)m.f * m.dvp;
   a.skip_chunk = c.skip_chunk;
   a.lower = c.lower_rows ? 1 : 0;
@@ -583,7 +586,7 @@ int moments_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void
   FM_CUDA_TRY(cudaGetLastError());
   FM_CUDA_TRY(cudaFuncSetAttribute(state_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
   FM_LAUNCH("fm_moments_tc_state", c.stream,
-            (state_tc_kernel<<<(unsigned)((size_t)heads * nchunk * ST_SPLIT), ST_THREADS, ST_SMEM, c.stream>>>(tz, a)));
+            (state_tc_kernel<<<(unsigned)((size_t)heads * nchunk * ST_SPLIT), ST_THREADS, ST_SMEM, c.stream>>>(tz, ty, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
