@@ -20,14 +20,12 @@
 //   scale_by_noise      y = x * (1 + dropout * noise), the reference's output
 //                       dropout (fastmax_cuda_forward.cu:271-280).
 //
-// All four are HBM-bound copies: 16-byte accesses where the shapes allow (a
-// rotated width that is only a multiple of 8 falls back to 8-byte accesses in
-// bf16, so that a piece never straddles the two halves of the rotation), two
-// to four pieces loaded per thread before the first store, 32-bit index
-// arithmetic inside a token, grid-stride over a grid sized to the SM count.
-// Measured on B200 in bf16 (B=8, T=4096, H=32, hs=64): split and merge move
-// 806 MB in 0.23-0.24 ms (3.4-3.5 TB/s; 4.0 TB/s at hs=128), the axis swap and
-// the noise scaling run at 5.4-5.6 TB/s.
+// All four are HBM-bound copies: 16-byte accesses where the shapes allow (bf16 whose rotated width or head size is only a
+// multiple of 8 falls back to 8-byte accesses, so that a piece never straddles the two halves of the rotation), several
+// pieces loaded per thread before the first store, grid-stride over a grid sized to the SM count.
+// Measured on B200 in bf16 (B=8, T=4096, H=32, hs=64): split and merge move 806 MB in 0.141 and 0.130 ms (5.7 and
+// 6.2 TB/s; 0.234 and 0.229 ms when a CTA took one token, each piece loaded its partner too and read its table entries
+// again for every head), the axis swap and the noise scaling run at 5.4-5.6 TB/s.
 #include "fm_common.cuh"
 
 namespace fm {
@@ -86,73 +84,78 @@ __device__ __forceinline__ T* head_row(T* q, T* k, T* v, const SiteArgs& a, long
   return base + ((b * a.groups + g) * a.n + t) * a.d;
 }
 
-constexpr int kInFlight = 2;  // pieces a thread loads before it computes and stores
+constexpr int kInFlight = 4;  // vectors a warp loads before it computes and stores
 
 // GRAD = false: per-head arrays <- packed projection, rotation R(t).
 // GRAD = true : packed gradient <- per-head gradients, rotation R(t)^T.
 // With x = (x1, x2) the two halves of the rotated features, cos = (c1, c2), sin = (s1, s2):
 //   y1 = x1 c1 - x2 s1,  y2 = x2 c2 + x1 s2       (model.py:812-825)
 //   gx1 = gy1 c1 + gy2 s2,  gx2 = gy2 c2 - gy1 s1
-// One token (b, t) per CTA pass: its G*(Q+2) vectors are contiguous in the packed array, so the
-// index arithmetic inside a token is 32-bit and the packed side is one contiguous run.
+// A lane keeps one slot of one token: two pieces of V elements that are rotated with each other, or two pieces that are
+// only copied.  Its table entries stay in registers while the warp walks the vectors (heads) of its tokens, so a vector
+// costs two loads and two stores a lane.  A warp's tokens are neighbours (8 of 64 bf16 features): on the head side it
+// moves a run of 1 KB, and the CTA's warps together take whole tokens of the packed side.
 template <typename T, int V, bool GRAD>
-__global__ void __launch_bounds__(256) qkv_site_kernel(const T* __restrict__ packed_in, T* __restrict__ packed_out,
-                                                       T* __restrict__ q, T* __restrict__ k, T* __restrict__ v,
-                                                       const float* __restrict__ cs, const float* __restrict__ sn,
-                                                       const SiteArgs a) {
-  const int qd = a.d / V, total = a.qper + 2, half = a.rope / 2;
-  const int per_tok = a.groups * total * qd;  // V-element pieces per token
-  const long long tokens = a.batch * a.n;
-  for (long long bt = blockIdx.x; bt < tokens; bt += gridDim.x) {
-    const long long b = bt / a.n, t = bt - b * a.n;
-    const long long pbase = bt * (long long)per_tok * V;
-    const float* ct = cs + t * a.rope;
-    const float* st = sn + t * a.rope;
-    for (int w0 = threadIdx.x; w0 < per_tok; w0 += kInFlight * blockDim.x) {
-      Pack<T, V> x[kInFlight], y[kInFlight];
-      T* dst[kInFlight];
-      int c[kInFlight];
-      bool rot[kInFlight], live[kInFlight];
+__global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ packed_in, T* __restrict__ packed_out,
+                                                          T* __restrict__ q, T* __restrict__ k, T* __restrict__ v,
+                                                          const float* __restrict__ cs, const float* __restrict__ sn,
+                                                          const SiteArgs a) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int total = a.qper + 2, vecs = a.groups * total;
+  const int slots = a.d / V / 2, width = slots < 32 ? slots : 32, tpw = 32 / width;   // lanes and tokens of a warp
+  const int pairs = a.rope / 2 / V, half = a.rope / 2;
+  const long long tgroups = (a.n + tpw - 1) / tpw, units = a.batch * tgroups;
+  for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    const long long b = unit / tgroups, t = (unit - b * tgroups) * tpw + lane / width;
+    for (int s0 = 0; s0 < slots; s0 += width) {
+      const int slot = s0 + lane % width;
+      const bool ok = t < a.n && lane / width < tpw && slot < slots, rot = ok && slot < pairs;
+      const int lo = (slot < pairs ? slot : 2 * slot) * V, hi = slot < pairs ? lo + half : lo + V;
+      float c1[V], c2[V], s1[V], s2[V];
 #pragma unroll
-      for (int u = 0; u < kInFlight; ++u) {
-        const int w = w0 + u * blockDim.x;
-        live[u] = w < per_tok;
-        rot[u] = false;
-        if (!live[u]) continue;
-        const int vec = w / qd;
-        c[u] = (w - vec * qd) * V;
-        const int g = vec / total, j = vec - g * total;
-        T* hrow = head_row(q, k, v, a, b, t, g, j);
-        const long long pvec = pbase + (long long)vec * a.d;  // start of the vector in the packed array
-        const T* src = GRAD ? hrow : packed_in + pvec;
-        dst[u] = (GRAD ? packed_out + pvec : hrow) + c[u];
-        x[u].load(src + c[u]);
-        rot[u] = c[u] < a.rope && j <= a.qper;
-        if (rot[u]) y[u].load(src + (c[u] < half ? c[u] + half : c[u] - half));
+      for (int e = 0; e < V; e += 4) {
+        const long long row = t * a.rope + e;
+        *reinterpret_cast<float4*>(c1 + e) = rot ? *reinterpret_cast<const float4*>(cs + row + lo) : make_float4(1.f, 1.f, 1.f, 1.f);
+        *reinterpret_cast<float4*>(c2 + e) = rot ? *reinterpret_cast<const float4*>(cs + row + hi) : make_float4(1.f, 1.f, 1.f, 1.f);
+        *reinterpret_cast<float4*>(s1 + e) = rot ? *reinterpret_cast<const float4*>(sn + row + lo) : make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(s2 + e) = rot ? *reinterpret_cast<const float4*>(sn + row + hi) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+      const long long pbase = (b * a.n + t) * vecs * a.d;
+      const int step = 8 * gridDim.y;
+      for (int v0 = warp + 8 * blockIdx.y; v0 < vecs; v0 += kInFlight * step) {
+        Pack<T, V> x[kInFlight], y[kInFlight];
+        T* dst[kInFlight];
+        bool turn[kInFlight];
 #pragma unroll
-      for (int u = 0; u < kInFlight; ++u) {
-        if (!live[u]) continue;
-        if (rot[u]) {
-          const bool lo = c[u] < half;
-          const int pc = lo ? c[u] + half : c[u] - half;
-          float xf[V], yf[V], cc[V], ss[V];
-          x[u].get(xf);
-          y[u].get(yf);
-          // cos at the feature's own index; sin at its own index going forward, at the partner's going back
-#pragma unroll
-          for (int e = 0; e < V; e += 4) {
-            const float4 c4 = *reinterpret_cast<const float4*>(ct + c[u] + e);
-            const float4 s4 = *reinterpret_cast<const float4*>(st + (GRAD ? pc : c[u]) + e);
-            cc[e] = c4.x; cc[e + 1] = c4.y; cc[e + 2] = c4.z; cc[e + 3] = c4.w;
-            ss[e] = s4.x; ss[e + 1] = s4.y; ss[e + 2] = s4.z; ss[e + 3] = s4.w;
-          }
-          const float sign = (lo != GRAD) ? -1.0f : 1.0f;
-#pragma unroll
-          for (int e = 0; e < V; ++e) xf[e] = xf[e] * cc[e] + sign * yf[e] * ss[e];
-          x[u].set(xf);
+        for (int u = 0; u < kInFlight; ++u) {
+          const int vec = v0 + u * step;
+          if (vec >= vecs) continue;
+          const int g = vec / total, j = vec - g * total;
+          T* hrow = head_row(q, k, v, a, b, t, g, j);
+          const long long pvec = pbase + (long long)vec * a.d;
+          const T* src = GRAD ? hrow : packed_in + pvec;
+          dst[u] = GRAD ? packed_out + pvec : hrow;
+          turn[u] = rot && j <= a.qper;
+          if (ok) { x[u].load(src + lo); y[u].load(src + hi); }
         }
-        x[u].store(dst[u]);
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) {
+          if (v0 + u * step >= vecs || !ok) continue;
+          if (turn[u]) {
+            float xf[V], yf[V], xo[V], yo[V];
+            x[u].get(xf);
+            y[u].get(yf);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+              xo[e] = GRAD ? xf[e] * c1[e] + yf[e] * s2[e] : xf[e] * c1[e] - yf[e] * s1[e];
+              yo[e] = GRAD ? yf[e] * c2[e] - xf[e] * s1[e] : yf[e] * c2[e] + xf[e] * s2[e];
+            }
+            x[u].set(xo);
+            y[u].set(yo);
+          }
+          x[u].store(dst[u] + lo);
+          y[u].store(dst[u] + hi);
+        }
       }
     }
   }
@@ -271,18 +274,27 @@ int launch_site(const void* packed_in, void* packed_out, void* q, void* k, void*
   }
   SiteArgs a{batch, n, groups, qper, d, rope};
   if (batch * n == 0) return FASTMAX_OK;
+  // 16-byte pieces where a vector has an even number of them and the rotation's halves are whole pieces (bf16: else 8 bytes)
+  const int V = dtype == FASTMAX_F32 ? 4 : (rope % 16 == 0 && d % 16 == 0 ? 8 : 4);
+  const int slots = d / V / 2, tpw = 32 / (slots < 32 ? slots : 32);
+  const long long units = batch * ((n + tpw - 1) / tpw);
   int blocks;
-  if ((rc = grid_for(batch * n * 256, &blocks))) return rc;   // one CTA per token, grid-stride beyond the cap
+  if ((rc = grid_for(units * 256, &blocks))) return rc;        // one CTA per group of tokens, grid-stride beyond the cap
+  // few tokens: several CTAs share the vectors of a group (a warp keeps at least one)
+  const int vecs8 = (groups * (qper + 2) + 7) / 8;
+  int split = (int)(units < 296 ? 296 / units : 1);
+  if (split > vecs8) split = vecs8;
+  const dim3 grid(blocks, split < 1 ? 1 : split);
   const char* name = GRAD ? "fm_qkv_merge_rope_grad" : "fm_qkv_split_rope";
   typedef __nv_bfloat16 bf;
   if (dtype == FASTMAX_F32)
-    FM_LAUNCH(name, st, (qkv_site_kernel<float, 4, GRAD><<<blocks, 256, 0, st>>>(
+    FM_LAUNCH(name, st, (qkv_site_kernel<float, 4, GRAD><<<grid, 256, 0, st>>>(
                             (const float*)packed_in, (float*)packed_out, (float*)q, (float*)k, (float*)v, cs, sn, a)));
-  else if (rope % 16 == 0)   // both halves of the rotated features are multiples of 8: 16-byte accesses
-    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 8, GRAD><<<blocks, 256, 0, st>>>(
+  else if (V == 8)
+    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 8, GRAD><<<grid, 256, 0, st>>>(
                             (const bf*)packed_in, (bf*)packed_out, (bf*)q, (bf*)k, (bf*)v, cs, sn, a)));
   else
-    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 4, GRAD><<<blocks, 256, 0, st>>>(
+    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 4, GRAD><<<grid, 256, 0, st>>>(
                             (const bf*)packed_in, (bf*)packed_out, (bf*)q, (bf*)k, (bf*)v, cs, sn, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
