@@ -23,12 +23,15 @@
 // running step (0 between calls), 0} per key/value head.  S2 is symmetric in (a, b), so only its
 // upper triangle of tiles is computed; every result is written to both of its rows.
 //
-// Two kernels:
-//   step_kernel    few tokens (one per decode step): bound by the state's traffic.  The lower
-//                  triangle is written but never read: 4 F (d+1) x (1 + 0.56) bytes at d = 64.
-//                  1024 heads, d = 64, p = 2, bf16: 356 us for 1.73 GB = 4.9 TB/s (487 us when every row
-//                  was read, a fill and a division kernel went with each step); 8 key/value heads of 4
-//                  query heads: 13 us (18).
+// Three kernels:
+//   step_kernel    one token and its read-out: bound by the state's traffic with many heads, by a chain of latencies with
+//                  few.  The lower triangle is written but never read: 4 F (d+1) x (1 + 0.56) bytes at d = 64.  Measured, us,
+//                  p = 2: 1024 heads, d = 64, bf16: 350 for 1.73 GB = 4.9 TB/s; 8 key/value heads of 4 query heads 9.3 (11.8
+//                  when the queries were asked for after the update, the arriving CTA fenced its 24 KB of state and the
+//                  last one read the queries' shares in turn); 4 heads, float32: 6.1 (7.0); d = 128, 128 heads: 328 (354).
+//                  Two other arrangements for many heads were slower: several groups of blocks to a CTA 397 us, five CTAs
+//                  to an SM 377.
+//   few_kernel     the same update for a few tokens of a prompt.
 //   append_kernel  many tokens (prompt), float32 or d = 32: bound by the FMA pipe; see there.  bf16 prompts of
 //                  d 64 and 128 go to the tensor cores (fm_decode_tc.cu).
 #include "fm_common.cuh"
@@ -106,52 +109,262 @@ __device__ __forceinline__ void upper_tile(int idx, int nt, int& ta, int& tb) {
   tb = ta + idx;
 }
 
-// A thread owns one column c of one block of rows, so a CTA's accesses are runs of whole rows: half of an
-// 8 x 8 tile of the second order on or above the diagonal, 32 first-order rows, or the constant row.  READ: the
-// blocks' shares of the read-out go to scratch[query head][CTA][column]; the CTA of a head that arrives last
-// (a counter in the head's header) adds them in CTA order, divides and writes the output row.
-template <typename T, int D, bool READ>
+// A thread owns one column c of one block of rows, so a CTA's accesses are runs of whole rows: half of an 8 x 8 tile of
+// the second order on or above the diagonal, 32 first-order rows, or the constant row.
+template <int D> struct Block {
+  typedef DecCfg<D> C;
+  int a0, b0, kind, live, ustride;        // kind 2, 1, 0: order of the block (-1: none); live: rows of it that exist
+  bool diagonal;
+  float *base, *base2;                    // row (u, i) at base[u * ustride + i * DV]; a tile's mirror image at base2
+  float s[kHalf][kTile];
+
+  // block sb of the head whose rows start at `rows`, column c
+  __device__ __forceinline__ void place(int sb, int p, float* rows, int c) {
+    const int nb2 = p == 2 ? C::NB2 : 0, n2rows = p == 2 ? D * D : 0;
+    diagonal = false;
+    a0 = b0 = 0;
+    kind = -1;
+    live = 0;
+    if (sb < nb2) {
+      upper_tile(sb >> 1, C::NT, a0, b0);
+      diagonal = a0 == b0;
+      a0 = a0 * kTile + (sb & 1) * kHalf;
+      b0 *= kTile;
+      kind = 2;
+      live = kHalf * kTile;
+    } else if (sb < nb2 + C::NB1) {
+      a0 = (sb - nb2) * kLinear;
+      kind = 1;
+      live = D - a0 < kLinear ? D - a0 : kLinear;
+    } else if (sb == nb2 + C::NB1) {
+      kind = 0;
+      live = 1;
+    }
+    base = rows + c + (long long)C::DV * (kind == 2 ? a0 * D + b0 : n2rows + (kind == 1 ? a0 : D));
+    base2 = rows + c + (long long)C::DV * (b0 * D + a0);
+    ustride = (kind == 2 ? D : kTile) * C::DV;
+  }
+  __device__ __forceinline__ void load() {
+#pragma unroll
+    for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+      for (int i = 0; i < kTile; ++i) s[u][i] = (u * kTile + i < live) ? base[u * ustride + i * C::DV] : 0.0f;
+  }
+  // one token: k, and this column's value
+  __device__ __forceinline__ void add(const float* k, float vc) {
+    if (kind == 2) {
+      float kb[kTile];
+#pragma unroll
+      for (int i = 0; i < kTile; ++i) kb[i] = k[b0 + i];
+#pragma unroll
+      for (int u = 0; u < kHalf; ++u) {
+        const float ka = k[a0 + u];
+#pragma unroll
+        for (int i = 0; i < kTile; ++i) s[u][i] = fmaf(ka * kb[i], vc, s[u][i]);
+      }
+    } else if (kind == 1) {
+#pragma unroll
+      for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+        for (int i = 0; i < kTile; ++i)
+          if (u * kTile + i < live) s[u][i] = fmaf(k[a0 + u * kTile + i], vc, s[u][i]);
+    } else if (kind == 0) {
+      s[0][0] += vc;
+    }
+  }
+  // the block's share of a read-out: query row q, scale sc of its products with keys
+  __device__ __forceinline__ float read(const DecArgs& a, const float* q, float sc) const {
+    float part = 0.0f;
+    if (kind == 2) {
+      // a tile above the diagonal stands for its mirror image too
+      const float coef = a.a2 * sc * sc * (diagonal ? 1.0f : 2.0f);
+#pragma unroll
+      for (int u = 0; u < kHalf; ++u) {
+        float row = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kTile; ++i) row = fmaf(q[b0 + i], s[u][i], row);
+        part = fmaf(coef * q[a0 + u], row, part);
+      }
+    } else if (kind == 1) {
+#pragma unroll
+      for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+        for (int i = 0; i < kTile; ++i)
+          if (u * kTile + i < live) part = fmaf(a.a1 * sc * q[a0 + u * kTile + i], s[u][i], part);
+    } else if (kind == 0) {
+      part = a.a0 * s[0][0];
+    }
+    return part;
+  }
+  __device__ __forceinline__ void store() const {
+#pragma unroll
+    for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+      for (int i = 0; i < kTile; ++i)
+        if (u * kTile + i < live) base[u * ustride + i * C::DV] = s[u][i];
+    if (kind == 2 && !diagonal) {
+#pragma unroll
+      for (int i = 0; i < kTile; ++i)
+#pragma unroll
+        for (int u = 0; u < kHalf; ++u) base2[(i * D + u) * C::DV] = s[u][i];
+    }
+  }
+};
+
+// One token per head and its read-out.  A CTA takes one group of RPB blocks of its head and leaves their share of the
+// read-out in scratch[query head][CTA][column]; the CTA of a head that arrives last (a counter in the head's header) adds
+// the shares in CTA order, divides and writes the output row.
+template <typename T, int D>
 __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_kernel(const DecArgs a, const T* __restrict__ q,
                                                                   const T* __restrict__ k, const T* __restrict__ v,
                                                                   float* __restrict__ state, float* __restrict__ scratch,
                                                                   T* __restrict__ out) {
   typedef DecCfg<D> C;
-  __shared__ __align__(16) float ks[kTokBatch][D];
-  __shared__ float vs[kTokBatch][D + 1];   // (v, 1)
+  __shared__ float ks[D], vs[D + 1];       // the token; (v, 1)
   __shared__ float qs[kQueries][D];
   __shared__ float red[kQueries][C::RPB][C::DV];
   __shared__ float s_q2[kQueries];
-  __shared__ int s_kmax2_bits;   // max |k|^2 as its bit pattern: non-negative floats order like integers
+  __shared__ float s_kmax2;
   __shared__ int s_last;
   const int tid = threadIdx.x, r = tid / C::DV, c = tid - r * C::DV, lane = tid & 31;
   const int head = blockIdx.y;
   float* hs = state + head * a.head_floats;
+  auto stage_queries = [&](long long qh, int ng) {
+    for (int x = tid; x < ng * D; x += C::THREADS) qs[x / D][x % D] = ldf(q + qh * D + x);
+  };
+  auto norms = [&](int ng) {               // of the staged queries, one warp each
+    if (tid < ng * 32) {
+      const float n2 = warp_norm2<D>(qs[tid >> 5], lane);
+      if (lane == 0) s_q2[tid >> 5] = n2;
+    }
+  };
 
-  // this thread's block
-  const int nb2 = (a.p == 2) ? C::NB2 : 0, n2rows = (a.p == 2) ? D * D : 0;
-  const int sb = blockIdx.x * C::RPB + r;
-  bool diagonal = false;
-  int a0 = 0, b0 = 0, kind = -1, count = 0;      // kind 2, 1, 0: order of the block; count: its first-order rows
-  if (sb < nb2) {
-    upper_tile(sb >> 1, C::NT, a0, b0);
-    diagonal = a0 == b0;
-    a0 = a0 * kTile + (sb & 1) * kHalf; b0 *= kTile; kind = 2;
-  } else if (sb < nb2 + C::NB1) {
-    a0 = (sb - nb2) * kLinear; kind = 1; count = D - a0 < kLinear ? D - a0 : kLinear;
-  } else if (sb == nb2 + C::NB1) {
-    kind = 0;
+  // the token and the first queries travel with the block's rows (a step of one sequence is a chain of latencies)
+  static_assert(C::THREADS >= 2 * D, "a thread an element of the token");
+  const int ng0 = a.ratio < kQueries ? a.ratio : kQueries;
+  const float tok = tid < D ? ldf(k + (long long)head * D + tid) : (tid < 2 * D ? ldf(v + (long long)head * D + tid - D) : 0.0f);
+  constexpr int QPT = (kQueries * D + C::THREADS - 1) / C::THREADS;
+  float q_first[QPT];
+#pragma unroll
+  for (int i = 0; i < QPT; ++i) {
+    const int x = tid + i * C::THREADS;
+    q_first[i] = x < ng0 * D ? ldf(q + (long long)head * a.ratio * D + x) : 0.0f;
   }
-  // row (u, i) at base[(u * ustride + i * istride)]; a second-order tile's mirror image at base2
-  float* base = hs + kHeader + c + (long long)C::DV * (kind == 2 ? a0 * D + b0 : n2rows + (kind == 1 ? a0 : D));
-  float* base2 = hs + kHeader + c + (long long)C::DV * (b0 * D + a0);
-  const int ustride = (kind == 2 ? D : kTile) * C::DV;
-  float s[kHalf][kTile];
-  // rows of this thread's block that exist: all 32, `count` of them, or one
-  const int live = kind == 2 ? kHalf * kTile : (kind == 1 ? count : (kind == 0 ? 1 : 0));
+  const float kmax2 = hs[0];
+  Block<D> blk;
+  blk.place(blockIdx.x * C::RPB + r, a.p, hs + kHeader, c);
+  blk.load();
+  if (tid < D) ks[tid] = tok;
+  else if (tid < 2 * D) vs[tid - D] = tok;
+  if (tid == 0) vs[D] = 1.0f;
 #pragma unroll
-  for (int u = 0; u < kHalf; ++u)
+  for (int i = 0; i < QPT; ++i) {
+    const int x = tid + i * C::THREADS;
+    if (x < ng0 * D) qs[x / D][x % D] = q_first[i];
+  }
+  __syncthreads();
+  norms(ng0);
+  constexpr int kLastWarp = C::THREADS / 32 - 1;         // a full warp; the queries have the first ones
+  if ((tid >> 5) == kLastWarp) {
+    const float n2 = warp_norm2<D>(ks, lane);
+    if (lane == 0) s_kmax2 = fmaxf(kmax2, n2);
+  }
+  blk.add(ks, vs[c]);
+  __syncthreads();
+  auto scale = [&](int g) {
+    return a.normalize ? (a.lim * rsqrtf(s_q2[g])) * (a.lim * rsqrtf(s_kmax2)) : 1.0f;
+  };
+
+  // this CTA's rows of the scratch, kQueries queries at a time
+#pragma unroll 1
+  for (int g0 = 0; g0 < a.ratio; g0 += kQueries) {
+    const int ng = a.ratio - g0 < kQueries ? a.ratio - g0 : kQueries;
+    const long long qh = (long long)head * a.ratio + g0;
+    if (g0 > 0) {
+      __syncthreads();
+      stage_queries(qh, ng);
+      __syncthreads();
+      norms(ng);
+      __syncthreads();
+    }
+#pragma unroll 1
+    for (int g = 0; g < ng; ++g) red[g][r][c] = blk.read(a, qs[g], scale(g));
+    __syncthreads();
+    for (int x = tid; x < ng * C::DV; x += C::THREADS) {
+      const int g = x / C::DV, cc = x - g * C::DV;
+      float tot = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kTile; ++i) s[u][i] = (u * kTile + i < live) ? base[u * ustride + i * C::DV] : 0.0f;
+      for (int rr = 0; rr < C::RPB; ++rr) tot += red[g][rr][cc];
+      __stcg(scratch + ((qh + g) * gridDim.x + blockIdx.x) * C::DV + cc, tot);
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    const int before = atomicAdd(reinterpret_cast<int*>(hs + 2), 1);
+    s_last = before == (int)gridDim.x - 1;
+  }
+  // The block is written only now: the fence above need not wait for it, and a CTA leaves with its stores in flight.
+  blk.store();
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) {
+    hs[0] = s_kmax2;
+    // the token count is an integer bit pattern in the float slot: exact past 2^24 tokens
+    hs[1] = __int_as_float(__float_as_int(hs[1]) + 1);
+    hs[2] = 0.0f;
+  }
+  for (int g0 = 0; g0 < a.ratio; g0 += kQueries) {
+    const int ng = a.ratio - g0 < kQueries ? a.ratio - g0 : kQueries;
+    const long long qh = (long long)head * a.ratio + g0;
+    // all queries' rows at once: one wait for memory instead of one a query
+    float tot[kQueries];
+#pragma unroll
+    for (int g = 0; g < kQueries; ++g) tot[g] = 0.0f;
+    const float* src = scratch + qh * gridDim.x * C::DV + c;
+    const long long per_query = (long long)gridDim.x * C::DV;
+    if (ng == 1) {
+#pragma unroll 8
+      for (int b = r; b < (int)gridDim.x; b += C::RPB) tot[0] += __ldcg(src + (long long)b * C::DV);
+    } else {
+#pragma unroll 4
+      for (int b = r; b < (int)gridDim.x; b += C::RPB) {
+#pragma unroll
+        for (int g = 0; g < kQueries; ++g)
+          if (g < ng) tot[g] += __ldcg(src + g * per_query + (long long)b * C::DV);
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < kQueries; ++g)
+      if (g < ng) red[g][r][c] = tot[g];
+    __syncthreads();
+    for (int x = tid; x < ng * D; x += C::THREADS) {
+      const int g = x / D, cc = x - g * D;
+      float num = 0.0f, den = 0.0f;
+#pragma unroll
+      for (int rr = 0; rr < C::RPB; ++rr) { num += red[g][rr][cc]; den += red[g][rr][D]; }
+      stf(out + qh * D + x, num / den);
+    }
+    __syncthreads();
+  }
+}
+
+// A few tokens of a prompt: one group of blocks per CTA, the tokens one after another.
+template <typename T, int D>
+__global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) few_kernel(const DecArgs a, const T* __restrict__ k,
+                                                                                    const T* __restrict__ v,
+                                                                                    float* __restrict__ state) {
+  typedef DecCfg<D> C;
+  __shared__ __align__(16) float ks[kTokBatch][D];
+  __shared__ float vs[kTokBatch][D + 1];   // (v, 1)
+  __shared__ int s_kmax2_bits;   // max |k|^2 as its bit pattern: non-negative floats order like integers
+  const int tid = threadIdx.x, r = tid / C::DV, c = tid - r * C::DV, lane = tid & 31;
+  const int head = blockIdx.y;
+  float* hs = state + head * a.head_floats;
+  Block<D> blk;
+  blk.place(blockIdx.x * C::RPB + r, a.p, hs + kHeader, c);
+  blk.load();
   if (tid == 0) s_kmax2_bits = __float_as_int(hs[0]);
   __syncthreads();
 
@@ -168,7 +381,7 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
       if (x == 0) vs[tok][D] = 1.0f;
     }
     __syncthreads();
-    if (READ || blockIdx.x == 0) {   // running maximum of |k|^2, the tokens spread over the CTA's full warps
+    if (blockIdx.x == 0) {   // running maximum of |k|^2, the tokens spread over the CTA's full warps
       constexpr int kFullWarps = C::THREADS / 32;
       const int warp = tid >> 5;
       if (warp < kFullWarps) {
@@ -177,130 +390,13 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
         if (lane == 0) atomicMax(&s_kmax2_bits, __float_as_int(m));
       }
     }
-    for (int tok = 0; tok < nt; ++tok) {
-      const float vc = vs[tok][c];
-      if (kind == 2) {
-        float kb[kTile];
-#pragma unroll
-        for (int i = 0; i < kTile; ++i) kb[i] = ks[tok][b0 + i];
-#pragma unroll
-        for (int u = 0; u < kHalf; ++u) {
-          const float ka = ks[tok][a0 + u];
-#pragma unroll
-          for (int i = 0; i < kTile; ++i) s[u][i] = fmaf(ka * kb[i], vc, s[u][i]);
-        }
-      } else if (kind == 1) {
-#pragma unroll
-        for (int u = 0; u < kHalf; ++u)
-#pragma unroll
-          for (int i = 0; i < kTile; ++i)
-            if (u * kTile + i < count) s[u][i] = fmaf(ks[tok][a0 + u * kTile + i], vc, s[u][i]);
-      } else if (kind == 0) {
-        s[0][0] += vc;
-      }
-    }
+    for (int tok = 0; tok < nt; ++tok) blk.add(ks[tok], vs[tok][c]);
     __syncthreads();
   }
-
-#pragma unroll
-  for (int u = 0; u < kHalf; ++u)
-#pragma unroll
-    for (int i = 0; i < kTile; ++i)
-      if (u * kTile + i < live) base[u * ustride + i * C::DV] = s[u][i];
-  if (kind == 2 && !diagonal) {
-#pragma unroll
-    for (int i = 0; i < kTile; ++i)
-#pragma unroll
-      for (int u = 0; u < kHalf; ++u) base2[(i * D + u) * C::DV] = s[u][i];
-  }
-  if (!READ) {
-    if (blockIdx.x == 0 && tid == 0) {
-      hs[0] = __int_as_float(s_kmax2_bits);
-      // the token count is an integer bit pattern in the float slot: exact past 2^24 tokens
-      hs[1] = __int_as_float(__float_as_int(hs[1]) + (int)a.n_new);
-    }
-    return;
-  }
-
-  // the group's query heads, kQueries at a time
-  for (int g0 = 0; g0 < a.ratio; g0 += kQueries) {
-    const int ng = a.ratio - g0 < kQueries ? a.ratio - g0 : kQueries;
-    const long long qh = (long long)head * a.ratio + g0;
-    __syncthreads();
-    for (int x = tid; x < ng * D; x += C::THREADS) qs[x / D][x % D] = ldf(q + qh * D + x);
-    __syncthreads();
-    if (tid < ng * 32) {
-      const float n2 = warp_norm2<D>(qs[tid >> 5], lane);
-      if (lane == 0) s_q2[tid >> 5] = n2;
-    }
-    __syncthreads();
-    for (int g = 0; g < ng; ++g) {
-      const float* qx = qs[g];
-      const float sc = a.normalize ? (a.lim * rsqrtf(s_q2[g])) * (a.lim * rsqrtf(__int_as_float(s_kmax2_bits))) : 1.0f;
-      float part = 0.0f;
-      if (kind == 2) {
-        // a tile above the diagonal stands for its mirror image too
-        const float coef = a.a2 * sc * sc * (diagonal ? 1.0f : 2.0f);
-#pragma unroll
-        for (int u = 0; u < kHalf; ++u) {
-          float row = 0.0f;
-#pragma unroll
-          for (int i = 0; i < kTile; ++i) row = fmaf(qx[b0 + i], s[u][i], row);
-          part = fmaf(coef * qx[a0 + u], row, part);
-        }
-      } else if (kind == 1) {
-#pragma unroll
-        for (int u = 0; u < kHalf; ++u)
-#pragma unroll
-          for (int i = 0; i < kTile; ++i)
-            if (u * kTile + i < count) part = fmaf(a.a1 * sc * qx[a0 + u * kTile + i], s[u][i], part);
-      } else {
-        part = a.a0 * s[0][0];
-      }
-      red[g][r][c] = part;
-    }
-    __syncthreads();
-    for (int x = tid; x < ng * C::DV; x += C::THREADS) {
-      const int g = x / C::DV, cc = x - g * C::DV;
-      float tot = 0.0f;
-#pragma unroll
-      for (int rr = 0; rr < C::RPB; ++rr) tot += red[g][rr][cc];
-      __stcg(scratch + ((qh + g) * gridDim.x + blockIdx.x) * C::DV + cc, tot);
-    }
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const int before = atomicAdd(reinterpret_cast<int*>(hs + 2), 1);
-    s_last = before == (int)gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (tid == 0) {
+  blk.store();
+  if (blockIdx.x == 0 && tid == 0) {
     hs[0] = __int_as_float(s_kmax2_bits);
     hs[1] = __int_as_float(__float_as_int(hs[1]) + (int)a.n_new);
-    hs[2] = 0.0f;
-  }
-  for (int g0 = 0; g0 < a.ratio; g0 += kQueries) {
-    const int ng = a.ratio - g0 < kQueries ? a.ratio - g0 : kQueries;
-    const long long qh = (long long)head * a.ratio + g0;
-    for (int g = 0; g < ng; ++g) {
-      float tot = 0.0f;
-      const float* src = scratch + (qh + g) * gridDim.x * C::DV + c;
-#pragma unroll 8
-      for (int b = r; b < (int)gridDim.x; b += C::RPB) tot += __ldcg(src + (long long)b * C::DV);
-      red[g][r][c] = tot;
-    }
-    __syncthreads();
-    for (int x = tid; x < ng * D; x += C::THREADS) {
-      const int g = x / D, cc = x - g * D;
-      float num = 0.0f, den = 0.0f;
-#pragma unroll
-      for (int rr = 0; rr < C::RPB; ++rr) { num += red[g][rr][cc]; den += red[g][rr][D]; }
-      stf(out + qh * D + x, num / den);
-    }
-    __syncthreads();
   }
 }
 
@@ -480,8 +576,8 @@ int step_ctas(const fastmax_problem& p) {
   return DecCfg<128>::ctas(p.p);
 }
 
-// From how many tokens on a prompt's kernels beat step_kernel, which reads and writes whole rows but walks the tokens
-// one by one.  Measured, us, step_kernel / prompt kernel (64 heads): d = 64, p = 2: 56 / 67 at 33 tokens, 69.5 / 67 at 44
+// From how many tokens on a prompt's kernels beat few_kernel, which reads and writes whole rows but walks the tokens
+// one by one.  Measured, us, few_kernel / prompt kernel (64 heads): d = 64, p = 2: 56 / 67 at 33 tokens, 69.5 / 67 at 44
 // (bf16), 69 / 70 at 44 (float32); p = 1: 15.0 / 10.4 at 33, 10.4 / 10.4 at 20; d = 128, p = 2: 462 / 391 at 44 (float32),
 // 582 / 663 at 63 (bf16).
 long long append_min(const fastmax_problem& p) {
@@ -504,10 +600,14 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
                 (append_kernel<T, D><<<grid, AppCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));
     }
   } else {
-    dim3 grid(DecCfg<D>::ctas(p.p), p.bhkv);
-    FM_LAUNCH(READ ? "fm_decode_step" : "fm_decode_append", st,
-              (step_kernel<T, D, READ><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
-                                                                            scratch, (T*)out)));
+    const dim3 grid(DecCfg<D>::ctas(p.p), p.bhkv);
+    if constexpr (READ)
+      FM_LAUNCH("fm_decode_step", st,
+                (step_kernel<T, D><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
+                                                                        scratch, (T*)out)));
+    else
+      FM_LAUNCH("fm_decode_append", st,
+                (few_kernel<T, D><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));
   }
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
