@@ -24,7 +24,7 @@ import math
 
 import torch
 
-from . import _cabi
+from . import _cabi, _native
 
 __all__ = ["FASTMultiHeadAttention_Function", "FASTMultiHeadAttention", "fastmax_function",
            "rpe_matrix_creator"]
@@ -180,6 +180,12 @@ class FASTMultiHeadAttention(torch.nn.Module):
     def forward(self, q, k, v, drop_noise=None, mask=False, dropout=0.0, normalize=False,
                 temperature=1.0, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=2, rpe_matrix=None):
         if self.use_custom_gradient:
+            # the plain case as one C++ autograd function; everything else, and every error, in Python
+            if (not dropout and _native.plain_tensors(q, k, v) and (p == 1 or p == 2)
+                    and _native.plain_numbers(temperature, a0, a1, a2, lim) and _native.host() and _native.plain_mode()):
+                out = _native.host().attention(q, k, v, bool(mask), bool(normalize), temperature, a0, a1, a2, lim, int(p))
+                if out is not None:
+                    return out
             return FASTMultiHeadAttention_Function.apply(q, k, v, drop_noise, mask, dropout, normalize,
                                                          temperature, a0, a1, a2, lim, p)
         if q.dim() == 3:

@@ -4,9 +4,10 @@
 
 * ``fastmax_b200/libfastmax_b200.so`` -- the CUDA kernels and the C ABI declared
   in ``include/fastmax_b200.h`` (plain nvcc, no torch dependency), and
-* ``fastmax_cuda*.so`` -- the torch C++ extension that exposes the reference's
-  ``forwardpass`` / ``backwardpass`` entry points on top of that C ABI
-  (only with ``--torch-ext``; it needs the torch headers and takes a minute).
+* with ``--torch-ext`` (they need the torch headers and take a minute), the torch
+  C++ extensions ``fastmax_cuda*.so``, which exposes the reference's
+  ``forwardpass`` / ``backwardpass`` entry points on top of that C ABI, and
+  ``fastmax_b200/_host*.so``, the host side of the package's frequent calls.
 
 nvcc cross-compiles without a GPU, so the build runs anywhere the CUDA toolkit
 is installed.
@@ -64,29 +65,38 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_torch_extension(force: bool = False) -> str:
-    """Compile the ``fastmax_cuda`` torch extension next to the package."""
+    """Compile the ``fastmax_cuda`` extension next to the package and ``_host`` inside it; returns the former's path."""
+    import sysconfig
+
+    build_library()
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    targets = [("torch_binding.cpp", "fastmax_cuda", ROOT, "$ORIGIN/fastmax_b200"), ("host_binding.cpp", "_host", PKG, "$ORIGIN")]
+    procs = []
+    for source, name, folder, rpath in targets:
+        src, target = os.path.join(CSRC, source), os.path.join(folder, name + suffix)
+        if force or not _newer(target, [src, os.path.join(ROOT, "include", "fastmax_b200.h")]):
+            procs.append(subprocess.Popen(_extension_command(src, name, target, rpath)))
+    for pr in procs:
+        if pr.wait():
+            raise subprocess.CalledProcessError(pr.returncode, pr.args)
+    return os.path.join(ROOT, "fastmax_cuda" + suffix)
+
+
+def _extension_command(src: str, name: str, target: str, rpath: str):
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension
 
-    build_library()
-    src = os.path.join(CSRC, "torch_binding.cpp")
-    suffix = sysconfig.get_config_var("EXT_SUFFIX")
-    target = os.path.join(ROOT, "fastmax_cuda" + suffix)
-    if not force and _newer(target, [src, os.path.join(ROOT, "include", "fastmax_b200.h")]):
-        return target
     inc = cpp_extension.include_paths("cuda")
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=fastmax_cuda",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={name}",
            "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I" + os.path.join(ROOT, "include"), "-I" + sysconfig.get_paths()["include"]]
     cmd += ["-I" + p for p in inc]
-    cmd += [src, "-o", target, "-L" + tlib, "-L" + PKG, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
-            "-ltorch", "-ltorch_python", "-l:libfastmax_b200.so", "-L/usr/local/cuda/lib64", "-lcudart",
-            "-Wl,-rpath,$ORIGIN/fastmax_b200", "-Wl,-rpath," + tlib]
-    subprocess.check_call(cmd)
-    return target
+    return cmd + [src, "-o", target, "-L" + tlib, "-L" + PKG, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+                  "-ltorch", "-ltorch_python", "-l:libfastmax_b200.so", "-L/usr/local/cuda/lib64", "-lcudart",
+                  "-Wl,-rpath," + rpath, "-Wl,-rpath," + tlib]
 
 
 if __name__ == "__main__":

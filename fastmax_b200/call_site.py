@@ -22,7 +22,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _cabi
+from . import _cabi, _native
 
 __all__ = ["fastmax_attention_from_qkv"]
 
@@ -81,6 +81,13 @@ def fastmax_attention_from_qkv(qkv, cos, sin, n_head, n_query_groups, head_size,
         raise ValueError(f"qkv width {width} does not match the head configuration")
     if not qkv.is_cuda:
         raise RuntimeError("fastmax_attention_from_qkv needs CUDA tensors (there is no CPU path)")
+    if (impl == "auto" and _native.plain_tensors(qkv, cos, sin) and (p == 1 or p == 2)
+            and _native.plain_numbers(temperature, a0, a1, a2, lim) and _native.host() and _native.plain_mode()):
+        # the plain case as one C++ autograd function (float32 tables on the device); everything else below
+        y = _native.host().from_qkv(qkv, cos, sin, n_query_groups, qper, head_size, int(rope_n_elem), bool(mask),
+                                    bool(normalize), temperature, a0, a1, a2, lim, int(p))
+        if y is not None:
+            return y
     kw = dict(mask=bool(mask), normalize=bool(normalize), temperature=temperature, a0=a0, a1=a1, a2=a2,
               lim=lim, p=p, impl=impl)
     qkv5 = qkv.contiguous().view(b, n, n_query_groups, qper + 2, head_size)

@@ -10,9 +10,11 @@ library (``fastmax_b200_decode_*``); there is no CPU path.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
-from . import _cabi
+from . import _cabi, _native
 
 __all__ = ["FastmaxDecodeState"]
 
@@ -70,6 +72,11 @@ class FastmaxDecodeState:
 
     def step(self, q, k, v):
         """Add one token and return the attention row of q (bh, 1, d) over all tokens so far."""
+        if _native.plain_tensors(q, k, v) and _native.host() and _native.plain_mode():
+            out = _native.host().decode_step(ctypes.addressof(self.prob), q, k, v, self.state, self.scratch)
+            if out is not None:
+                self.tokens += 1
+                return out
         self._check(q, self.bh, "q")
         self._check(k, self.bhkv, "k")
         self._check(v, self.bhkv, "v")

@@ -1,0 +1,109 @@
+"""The C++ host side of the frequent calls: the same results, errors and autograd behaviour as the Python functions."""
+import pytest
+import torch
+
+import fastmax_b200
+from fastmax_b200 import _native
+from fastmax_b200.attention import FASTMultiHeadAttention_Function
+
+pytestmark = pytest.mark.gpu
+KW = dict(mask=True, normalize=True, temperature=2.0, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=2)
+
+
+def _inputs(dtype=torch.float32, heads=4, kv=4, n=70, d=32):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    t = [torch.randn(1, h, n, d, generator=g, device="cuda").to(dtype) for h in (heads, kv, kv, heads)]
+    return [x.requires_grad_(True) for x in t[:3]] + [t[3]]
+
+
+def _python(q, k, v):
+    return FASTMultiHeadAttention_Function.apply(q, k, v, None, KW["mask"], 0.0, KW["normalize"], KW["temperature"], 1.0,
+                                                 1.0, 0.5, 1.0, 2)
+
+
+def test_module_is_here():
+    assert _native.host() is not None and _native.plain_mode()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kv", [4, 2])
+def test_same_as_the_python_function(dtype, kv):
+    q, k, v, go = _inputs(dtype, kv=kv)
+    mod = fastmax_b200.FASTMultiHeadAttention()
+    a, b = mod(q, k, v, **KW), _python(q, k, v)
+    assert a.grad_fn is not None and torch.equal(a, b)
+    # the dots of the normalisation gradient are summed by atomics: one row a head may differ by its last bits
+    tol = dict(rtol=0, atol=1e-5 if dtype == torch.float32 else 2e-2)
+    for x, y in zip(torch.autograd.grad(a, (q, k, v), go), torch.autograd.grad(b, (q, k, v), go)):
+        assert torch.allclose(x, y, **tol)
+    # a transposed input and an upstream gradient of another layout
+    qt = q.detach().transpose(2, 3).contiguous().transpose(2, 3).requires_grad_(True)
+    gx = torch.autograd.grad(mod(qt, k, v, **KW), qt, go.transpose(2, 3).contiguous().transpose(2, 3))[0]
+    assert torch.allclose(gx, torch.autograd.grad(_python(q, k, v), q, go)[0], **tol)
+
+
+def test_graph_rules():
+    q, k, v, go = _inputs()
+    mod = fastmax_b200.FASTMultiHeadAttention()
+    out = mod(q, k, v, **KW)
+    out.backward(go)
+    with pytest.raises(RuntimeError):
+        out.backward(go)                                     # saved tensors are freed
+    out = mod(q, k, v, **KW)
+    with torch.no_grad():
+        k.mul_(2.0)
+    with pytest.raises(RuntimeError):
+        out.backward(go)                                     # a saved input was modified
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.shape) or t.clone(), lambda t: t):
+        out = mod(q, k, v, **KW)
+    out.backward(go)
+    assert len(seen) == 6
+    with torch.no_grad():
+        assert mod(q, k, v, **KW).grad_fn is None
+    mod(q.detach(), k.detach(), v, **KW).backward(go)
+
+
+@pytest.mark.parametrize("change,error", [
+    (dict(p=3), ValueError), (dict(k=lambda t: t[:, :, :, :16]), ValueError), (dict(k=lambda t: t.double()), ValueError),
+    (dict(q=lambda t: t.cpu()), RuntimeError)])
+def test_errors_are_those_of_the_python_function(change, error):
+    q, k, v, _ = _inputs()
+    kw = dict(KW, p=change.get("p", 2))
+    q, k = change.get("q", lambda t: t)(q), change.get("k", lambda t: t)(k)
+    with pytest.raises(error):
+        fastmax_b200.FASTMultiHeadAttention()(q, k, v, **kw)
+
+
+def test_transforms_take_the_python_function():
+    q, k, v, go = _inputs()
+    mod = fastmax_b200.FASTMultiHeadAttention()
+    for f in (lambda: torch.func.vmap(lambda a: mod(a, k[0], v[0], **KW))(q),
+              lambda: torch.func.grad(lambda a: mod(a, k, v, **KW).sum())(q)):
+        with pytest.raises(RuntimeError):
+            f()
+
+
+def test_call_site_and_decode(monkeypatch):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    qkv = torch.randn(2, 45, 8 * 64, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    cos, sin = [torch.randn(45, 32, generator=g, device="cuda") for _ in range(2)]
+    go = torch.randn(2, 45, 4 * 64, generator=g, device="cuda").bfloat16()
+
+    def site():
+        y = fastmax_b200.fastmax_attention_from_qkv(qkv, cos, sin, 4, 2, 64, 32)
+        return y, torch.autograd.grad(y, qkv, go)[0]
+
+    def decode():
+        st = fastmax_b200.FastmaxDecodeState(4, 2, 64, torch.bfloat16, "cuda")
+        rows = [torch.randn(h, 1, 64, generator=torch.Generator(device="cuda").manual_seed(h), device="cuda").bfloat16()
+                for h in (4, 2, 2)]
+        with pytest.raises(ValueError):
+            st.step(rows[0][:2], rows[1], rows[2])
+        return st.step(*rows), st.state.clone(), st.tokens
+
+    a, da = site(), decode()
+    monkeypatch.setattr(_native, "host", lambda: None)
+    b, db = site(), decode()
+    assert torch.equal(a[0], b[0]) and torch.allclose(a[1], b[1], rtol=0, atol=2e-2)
+    assert torch.equal(da[0], db[0]) and torch.equal(da[1], db[1]) and da[2] == db[2] == 1
