@@ -280,6 +280,7 @@ int fastmax_b200_device_status(int* status, void* stream) {
   if ((rc = first_tc_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = tc_short_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = split_status(&f, (cudaStream_t)stream))) return rc;
+  if (!f && (rc = split_moments_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = readout_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = decode_tc_status(&f, (cudaStream_t)stream))) return rc;
   *status = a ? a : (b ? b : f);
@@ -294,6 +295,7 @@ int fastmax_b200_device_status_reset(void* stream) {
   if ((rc = tc_dkdv128_status_reset(s))) return rc;
   if ((rc = moments_tc_status_reset(s))) return rc;
   if ((rc = split_status_reset(s))) return rc;
+  if ((rc = split_moments_status_reset(s))) return rc;
   if ((rc = readout_status_reset(s))) return rc;
   if ((rc = tc_short_status_reset(s))) return rc;
   if ((rc = decode_tc_status_reset(s))) return rc;
@@ -383,7 +385,9 @@ static size_t forward_bytes(const fastmax_problem* p, bool least) {
   int impl;
   if (pick_impl(*p, false, &impl)) return 0;
   if (impl == FASTMAX_IMPL_MOMENTS) return fwd_ws_bytes(*p, least);
-  return !least && impl == FASTMAX_IMPL_DENSE_FFMA && dense_split_supports(*p) ? dense_split_fwd_bytes(*p) : 0;
+  if (least || impl != FASTMAX_IMPL_DENSE_FFMA || !dense_split_supports(*p)) return 0;
+  const size_t parts = dense_split_fwd_bytes(*p), sums = split_moments_faster(*p) ? split_moments_bytes(*p) : 0;
+  return parts > sums ? parts : sums;
 }
 static size_t backward_bytes(const fastmax_problem* p, bool least) {
   if (validate(p)) return 0;
@@ -454,6 +458,10 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   }
   if (impl == FASTMAX_IMPL_DENSE_TC)
     return dense_tc_forward(c, q, k, v, (const stat_t*)stats, o.out, o.den);
+  // (the packed layout and calls with less room keep the score form)
+  if (!o.out_f32 && split_moments_faster(p) &&
+      use_split(p, split_moments_bytes(p), workspace, workspace_bytes, {q, k, v, o.out}))
+    return split_moments_forward(c, q, k, v, (const stat_t*)stats, o, workspace);
   if (use_split(p, dense_split_fwd_bytes(p), workspace, workspace_bytes, {q, k, v, o.out}))
     return dense_split_forward(c, q, k, v, (const stat_t*)stats, o, workspace);
   return dense_ffma_forward(c, q, k, v, (const stat_t*)stats, o);

@@ -213,6 +213,16 @@ int dense_split_forward(const Ctx& c, const void* q, const void* k, const void* 
 int dense_split_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* out, const float* den,
                          const stat_t* stats, const void* grad_out, float* dots, void* grad_q, void* grad_k,
                          void* grad_v, void* workspace, const ChunkAdd* ca = nullptr);
+// rows of d float32 -> rows of [h | m | l], 3 d bf16, for two tensors
+int split3_rows(const Ctx& c, const void* a, void* a3, size_t rows_a, const void* b, void* b3, size_t rows_b);
+// Unmasked second-order forward of the float32 score family in moment form (fm_split_moments.cu): whether it is the
+// faster one for the problem's sizes, its workspace, and the call.
+bool split_moments_faster(const fastmax_problem& p);
+size_t split_moments_bytes(const fastmax_problem& p);
+int split_moments_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats, const FwdOut& o,
+                          void* workspace);
+int split_moments_status(int* out, cudaStream_t stream);
+int split_moments_status_reset(cudaStream_t stream);
 int split_status(int* out, cudaStream_t stream);
 int split_status_reset(cudaStream_t stream);
 

@@ -166,15 +166,6 @@ __device__ __forceinline__ void issue_acc(uint32_t acc, uint32_t a_tmem, uint32_
   }
 }
 
-// Two float32 values as three packed bf16 pairs whose sums are the values.
-__device__ __forceinline__ void split3(uint64_t v, uint32_t& h, uint32_t& m, uint32_t& l) {
-  const uint64_t neg1 = 0xBF800000BF800000ull;
-  h = pack_bf16_2(v);
-  const uint64_t r = fma2(pack2u(h << 16, h & 0xFFFF0000u), neg1, v);
-  m = pack_bf16_2(r);
-  l = pack_bf16_2(fma2(pack2u(m << 16, m & 0xFFFF0000u), neg1, r));
-}
-
 // Adds this warp's half of the features of one tile's accumulator to the running sums (packed pairs).
 template <int D>
 __device__ __forceinline__ void promote(uint64_t (&run)[D / 4], uint32_t taddr, int cpart) {
@@ -785,6 +776,13 @@ int dense_split_backward(const Ctx& c, const void* q, const void* k, const void*
   a.dots = p.normalize ? dots + p.bh : nullptr;
   if (p.d == 32) return launch_mode<32, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, p.nk, p.nq, a);
   return launch_mode<64, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, p.nk, p.nq, a);
+}
+
+int split3_rows(const Ctx& c, const void* a, void* a3, size_t rows_a, const void* b, void* b3, size_t rows_b) {
+  SplitJobs jobs = {};
+  jobs.j[0] = {(const float*)a, (__nv_bfloat16*)a3, rows_a, nullptr, nullptr, nullptr};
+  jobs.j[1] = {(const float*)b, (__nv_bfloat16*)b3, rows_b, nullptr, nullptr, nullptr};
+  return launch_split3(c, jobs, 2);
 }
 
 int split_status(int* out, cudaStream_t stream) {

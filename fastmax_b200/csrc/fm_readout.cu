@@ -22,35 +22,18 @@
 // suspended waits (no change).
 // (Replaces the d*d-wide feature contraction of the reference, `old stuff/fastmax_cuda_forward_quad.cu`:111-135, 240-268
 // and the matching backward loops.)
-#include "fm_common.cuh"
-#include "fm_sm100.cuh"
+#include "fm_readout.cuh"
 
 namespace fm {
 
 __device__ int g_readout_status = 0;  // first protocol error seen by a kernel of this file
 
 namespace {
-using namespace sm100;
-
-constexpr int D = 64;
-constexpr int TILE = 128 * D * 2;         // 128 rows of 64 bf16
+using namespace rdo;
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_readout_status, 0, code); }
 
 // ---- operand copies of one state ---------------------------------------------------------------------------
-// Type A: 17 steps, streamed in this order.  Step 0 (16 KB, 128-byte swizzle): rows 0..63 S1 transposed (row c, a along
-// K), rows 64..127 E (row b, a along K).  Step 1 + 4 g + j holds two slices, the sixteen value columns of group g against
-// the features b of octet j, then of octet 7 - j, so that every step has five K steps in all.  The 128 rows of a slice are
-// (c / 8 % 2) * 64 + b % 8 * 8 + c % 8.  A slice is unswizzled K-major: per K step of 16 features two halves of 2048
-// bytes, in them 128-byte groups of eight rows.  One feature b and eight value columns are one such group, which is what
-// the CTA that owns b writes.
-constexpr int A_STEPS = 17;
-constexpr int A_STAGE = 5 * 4096;
-constexpr int A_BYTES = TILE + 16 * A_STAGE;
-__device__ __forceinline__ int a_slice(int g, int oct) {
-  const int j = oct < 4 ? oct : 7 - oct;
-  return TILE + (g * 4 + j) * A_STAGE + (oct < 4 ? 0 : ((j >> 1) + 1) * 4096);
-}
 // Type B: 19 slices of 128 rows with c along K (128-byte swizzle).  Slices 0..17 hold two 8 x 8 blocks (alpha <= beta)
 // of pairs each, block beta (beta + 1) / 2 + alpha; slice 18 has S1 (row a, c along K) and E (row a, b along K).
 // Rows of a block are ordered for packed arithmetic: two neighbouring columns of M are the pairs (2i, 2k), (2i+1, 2k+1)
@@ -60,11 +43,8 @@ constexpr int B_BYTES = B_SLICES * TILE;
 __host__ __device__ constexpr int b_col(int a8, int b8) {
   return (((a8 >> 1) * 4 + (b8 >> 1)) * 2 + ((a8 ^ b8) & 1)) * 2 + (b8 & 1);
 }
-__device__ __forceinline__ int swz(int row, int byte) { return row * 128 + (byte ^ ((row & 7) << 4)); }
-
 // The 64 x 65 block S2[a][b][:] of feature b (rows a < 16 (b / 16 + 1) are enough) -> its places in the copies, 16 bytes
 // a thread: a warp writes 128-byte runs in both layouts.
-constexpr int BLK_LD = 68;
 __device__ __forceinline__ void write_feature(const float (*blk)[BLK_LD], int b, char* ca, char* cb, int t) {
   const int bb = b >> 4, warp = t >> 5, lane = t & 31;
   if (ca)
@@ -194,47 +174,6 @@ __global__ void __launch_bounds__(256, 3) prefix_copies_kernel(const float* __re
   }
 }
 
-// ---- read-outs -----------------------------------------------------------------------------------------------
-struct RdArgs {
-  const char* copies;     // A_BYTES or B_BYTES per state
-  const float* state;     // fp32 states, for the constant row and S1's normaliser column
-  const float* uvec;      // type B: (heads, n) dvec, whose negative is e; null: e = 1
-  float* out;             // (heads, n, 64) fp32
-  float* den;             // type A: (heads, n), may be null
-  const stat_t* stat_q;
-  const stat_t* stat_k;
-  float a0, a1, a2, lim;
-  size_t per_state;
-  int dvp, heads, n;
-  int items;              // heads * groups
-  int chunk, nchunk;      // chunk 0: one state per head
-  int per_chunk;          // groups of a chunk
-  int first, groups;      // groups of 256 tokens of a head that are read out: first .. first + groups - 1
-  int zero_first, zero_groups;   // groups whose state is empty: zeros are written
-  int wide_io;            // out is 32-byte aligned
-};
-// A CTA's walk over the items blockIdx.x, blockIdx.x + gridDim.x, ...: head, first token and state of the present one.
-struct Walk {
-  int left, head, grp, dhead, dgrp;
-  __device__ __forceinline__ explicit Walk(const RdArgs& a) {
-    left = (a.items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    head = blockIdx.x / a.groups;
-    grp = blockIdx.x % a.groups;
-    dhead = gridDim.x / a.groups;
-    dgrp = gridDim.x % a.groups;
-  }
-  __device__ __forceinline__ bool more() const { return left > 0; }
-  __device__ __forceinline__ void next(const RdArgs& a) {
-    --left;
-    head += dhead;
-    grp += dgrp;
-    if (grp >= a.groups) { grp -= a.groups; ++head; }
-  }
-  __device__ __forceinline__ int tok0(const RdArgs& a) const { return (a.first + grp) * 256; }
-  __device__ __forceinline__ int state(const RdArgs& a) const {
-    return a.chunk > 0 ? head * a.nchunk + (a.first + grp) / a.per_chunk : head;
-  }
-};
 // zero rows of the groups with an empty state, by `threads` threads of this CTA
 __device__ __forceinline__ void write_zeros(const RdArgs& a, int t, int threads) {
   for (int w = blockIdx.x; w < a.heads * a.zero_groups; w += gridDim.x) {
@@ -246,51 +185,6 @@ __device__ __forceinline__ void write_zeros(const RdArgs& a, int t, int threads)
       for (int i = t; i < rows; i += threads) a.den[(size_t)head * a.n + tok0 + i] = 0.f;
   }
 }
-// contiguous global -> shared copy (both 16-byte aligned, size a multiple of 16)
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ uint4 lds128(uint32_t saddr) {
-  uint4 r;
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(saddr));
-  return r;
-}
-// wait for the loads of tensor memory in flight; the registers they fill pass through, so no use moves ahead of it
-template <int N> __device__ __forceinline__ void pass_through(uint32_t (&r)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
-}
-__device__ __forceinline__ void wait_ld64(uint32_t (&r)[64]) { tmem_wait_ld(); pass_through(r); }
-__device__ __forceinline__ void wait_ld128(uint32_t (&r)[128]) { tmem_wait_ld(); pass_through(r); }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-// K steps of D[tmem] = A[smem] B[smem]^T, A in the 128-byte swizzle (32 bytes per step), B unswizzled in the layout of
-// the type A slices (4096 bytes per step, K halves 2048 bytes apart, groups of eight rows 128 bytes apart)
-constexpr uint32_t kDescHiFlat = (128u >> 4) | (1u << 14);
-__device__ __forceinline__ void mma_steps(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, int steps) {
-  for (int ks = 0; ks < steps; ++ks)
-    asm volatile(
-        "{\n"
-        ".reg .b64 da, db;\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %6, 0;\n"
-        "mov.b64 da, {%1, %3};\n"
-        "mov.b64 db, {%2, %4};\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_lo + ks * 2), "r"(b_lo + ks * (4096 >> 4)), "r"(kDescHi), "r"(kDescHiFlat), "r"(idesc),
-          "r"(ks > 0 ? 1u : 0u)
-        : "memory");
-}
-
 // ---- type A ---------------------------------------------------------------------------------------------------
 // Two token tiles of 128 rows with two 128-column T buffers each.  Eight warps and one issuer warp per tile: the two sets
 // of four warps take one half of the columns of every slice, that is eight of its sixteen value columns.  A thread
@@ -312,8 +206,6 @@ static_assert(RA_SMEM <= 227 * 1024, "shared memory");
 // registers a thread after the split; its sum must not pass that of the launch (or the block never starts)
 constexpr int RA_REGS = 104, RA_REGS_REST = 64, RB_REGS = 232, RB_REGS_REST = 40;
 static_assert(4 * RA_REGS + RA_REGS_REST <= 5 * 96 && 2 * RB_REGS + RB_REGS_REST <= 3 * 168, "register split");
-template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 __global__ void __launch_bounds__(RA_THREADS, 1)
 readout_a_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a) {

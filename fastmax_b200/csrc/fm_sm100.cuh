@@ -457,6 +457,14 @@ __device__ __forceinline__ uint32_t pack_bf16_2(uint64_t v) {
   unpack2(v, lo, hi);
   return pack_bf16(lo, hi);
 }
+// Two float32 values as three packed bf16 pairs whose sums are the values.
+__device__ __forceinline__ void split3(uint64_t v, uint32_t& h, uint32_t& m, uint32_t& l) {
+  const uint64_t neg1 = 0xBF800000BF800000ull;
+  h = pack_bf16_2(v);
+  const uint64_t r = fma2(pack2u(h << 16, h & 0xFFFF0000u), neg1, v);
+  m = pack_bf16_2(r);
+  l = pack_bf16_2(fma2(pack2u(m << 16, m & 0xFFFF0000u), neg1, r));
+}
 
 // 32 bytes to / from global memory in one access where the address allows it (one full sector per lane:
 // a thread owns a whole row here, so its accesses never coalesce with its neighbours'), else two of 16.
