@@ -11,7 +11,7 @@
 //   readout3_kernel    the type A read-out with six products to a slice, and the division.  Bound by the products: 504 K
 //                      steps of 128 x 128 x 16 per 128 rows, 32 600 cycles.
 // 64 heads x 10 000: sums 1.32 ms, copies 0.03, read-out 0.90, operand parts 0.12, where the score form takes 7.1 ms; 2-norm
-// error against float64 2.4e-7 (score form 2.6e-7).
+// error against float64 2.4e-7 (score form 2.6e-7).  The transposed key block written one block ahead: no change.
 #include "fm_readout.cuh"
 
 namespace fm {
@@ -596,8 +596,10 @@ int split_moments_status_reset(cudaStream_t stream) {
 }
 
 // The score form costs 1.05 ps a pair.  The moment form: 1.45 ns a query row, 2.1 us per block of 64 keys and wave of CTAs
-// (nine a key head), and its launches.  Measured, us, score / moment: 64 heads x 10 000 7 030 / 2 450, 8 x 10 000 840 / 540,
-// 32 on 8 key heads x 4000 540 / 400; 64 x 2000 280 against 490 by the line, 8 x 4000 135 / 250.
+// (nine a key head), and its launches.  Measured, all kernels of a forward, us, score / moment:
+//   64 heads: 6267 / 2471 at 10 000, 1357 / 1106 at 4200, 1090 / 968 at 3600; 16: 556 / 393 at 5000; 8: 875 / 541 at 10 000,
+//   569 / 411 at 7500, 323 / 354 at 6000; 2: 1101 / 791 at 20 000; 1: 1065 / 1144 at 30 000
+//   32 on 8 key heads: 585 / 400 at 4000, 397 / 315 at 3000; 8 on 2, 40 000 queries: 790 / 609 for 2000 keys
 bool split_moments_faster(const fastmax_problem& p) {
   if (!dense_split_supports(p) || p.mask || p.p != 2 || p.d != 64 || p.bh % p.bhkv || p.bhkv > 65535) return false;
   const double us_pairs = 1.05e-6 * p.bh * p.nq * p.nk;
