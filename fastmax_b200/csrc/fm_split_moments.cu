@@ -600,8 +600,25 @@ int split_moments_status_reset(cudaStream_t stream) {
 //   64 heads: 6267 / 2471 at 10 000, 1357 / 1106 at 4200, 1090 / 968 at 3600; 16: 556 / 393 at 5000; 8: 875 / 541 at 10 000,
 //   569 / 411 at 7500, 323 / 354 at 6000; 2: 1101 / 791 at 20 000; 1: 1065 / 1144 at 30 000
 //   32 on 8 key heads: 585 / 400 at 4000, 397 / 315 at 3000; 8 on 2, 40 000 queries: 790 / 609 for 2000 keys
+//
+// And only where the terms of f(s) = a0 + a1 s + a2 s^2 cannot cancel to less than a fifth of their sizes.  The sums over
+// feature pairs are rounded relative to a2 |q|^2 |k|^2, whatever the score is; the score form's are relative to f.  With
+// normalised rows |s| <= |q| |k| <= lim^2, which bounds the loss; without nothing does.  2-norm errors against float64, 64 heads
+// x 4097, score / moment: keys that share a direction of norm 80 which the queries do not see, not normalised, 4.4e-7 / 1.6e-5,
+// of norm 800 3.9e-6 / 1.6e-3; normalised, the usual coefficients (1, 1, 0.5), N(0,1) 1.8e-7 / 1.7e-7, q and k along one direction
+// 1.9e-7 / 1.2e-7, along opposite ones (where f is a fifth) 1.9e-7 / 3.8e-7; (1, 0, -1), a tenth, 2.0e-7 / 3.1e-7; (1, -1.5, 0.5),
+// no bound, 7.0e-7 / 4.8e-6; (1, 1, 0.5) and lim 4, a hundredth and less, 1.9e-7 / 4.0e-7.
+static bool terms_hardly_cancel(const fastmax_problem& p) {
+  if (!p.normalize) return false;
+  const double a0 = p.a0, a1 = p.a1, a2 = p.a2, most = (double)p.lim * p.lim;
+  auto f = [&](double s) { return a0 + s * (a1 + s * a2); };
+  double least = f(-most) < f(most) ? f(-most) : f(most);
+  if (a2 > 0 && fabs(a1) < 2 * a2 * most && f(-a1 / (2 * a2)) < least) least = f(-a1 / (2 * a2));
+  return fabs(a0) + most * (fabs(a1) + most * fabs(a2)) <= 5 * least;
+}
 bool split_moments_faster(const fastmax_problem& p) {
   if (!dense_split_supports(p) || p.mask || p.p != 2 || p.d != 64 || p.bh % p.bhkv || p.bhkv > 65535) return false;
+  if (!terms_hardly_cancel(p)) return false;
   const double us_pairs = 1.05e-6 * p.bh * p.nq * p.nk;
   const double us_moment = 60 + 1.45e-3 * p.bh * p.nq + ((9 * p.bhkv + 147) / 148) * (p.nk / 64.0) * 2.1;
   return us_moment < us_pairs;

@@ -29,13 +29,11 @@ def reference(q, k, v, norm, a):
 
 # query heads, key heads, nq, nk, normalize, scale of the keys
 @pytest.mark.parametrize("bh,bhkv,nq,nk,norm,scale", [
-    (8, 8, 9999, 9999, 1, 1.0), (8, 2, 40001, 2111, 1, 1e17), (16, 4, 4097, 8191, 0, 0.1), (64, 64, 4001, 4033, 1, 1e-17)])
+    (8, 8, 9999, 9999, 1, 1.0), (8, 2, 40001, 2111, 1, 1e17), (16, 4, 4097, 8191, 1, 0.1), (64, 64, 4001, 4033, 1, 1e-17)])
 def test_moment_form_forward_against_float64(bh, bhkv, nq, nk, norm, scale):
     g = torch.Generator(device="cuda").manual_seed(nq)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
     q, k, v = rnd(bh, nq, 64), rnd(bhkv, nk, 64) * scale, rnd(bhkv, nk, 64)
-    if not norm:
-        q = q * 0.1
     _cabi.profile(True)
     out, den, _ = _cabi.forward(q, k, v, mask=0, normalize=norm, p=2, a0=1.0, a1=0.7, a2=0.4, lim=1.0)
     names = {n for n, _ in _cabi.profile_records()}
@@ -45,3 +43,21 @@ def test_moment_form_forward_against_float64(bh, bhkv, nq, nk, norm, scale):
     ref = reference(q, k, v, norm, (1.0, 0.7, 0.4))
     err = float((out.double() - ref).norm() / ref.norm())
     assert err < 1e-6, err
+
+
+@pytest.mark.parametrize("offset", [80.0, 800.0])
+def test_unnormalised_keys_with_a_common_direction_keep_the_score_form(offset):
+    """Keys share a direction that the queries do not see: scores near 8 from norms of 8 and `offset`.  A score is a sum of 64
+    products of up to |q| |k| / 8, rounded to 2^-24 of the largest partial sum, which f = 1 + s + s^2 / 2 doubles: a bound of
+    2^-23 (8 + offset) beside the 1e-6 of the sums over the keys, of which random signs leave about a twentieth.  Sums over
+    feature pairs would be rounded to 2^-24 |q|^2 |k|^2 / 2, 1.6e-5 and 1.6e-3 on these inputs."""
+    heads, n = 64, 4097
+    g = torch.Generator(device="cuda").manual_seed(int(offset))
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v, u = rnd(heads, n, 64), rnd(heads, n, 64), rnd(heads, n, 64), rnd(heads, 1, 64)
+    u = u / u.norm(dim=2, keepdim=True)
+    q, k = q - (q * u).sum(2, keepdim=True) * u, k + offset * u
+    out, _, _ = _cabi.forward(q, k, v, mask=0, normalize=0, p=2, a0=1.0, a1=1.0, a2=0.5, lim=1.0)
+    ref = reference(q, k, v, 0, (1.0, 1.0, 0.5))
+    err = float((out.double() - ref).norm() / ref.norm())
+    assert err < 1e-6 + 2.0 ** -23 * (8 + offset) / 8, err

@@ -53,3 +53,19 @@ def test_fused_first_order_needs_no_fp32_rows(heads, n):
     states = heads * -(-n // 512) * (65 * 68 * 4 + 64 * 64 * 2)
     assert fwd <= states + 4096
     assert bwd <= tensor + states + 2 * 4 * heads * n + 8 * heads + 4096
+
+
+@pytest.mark.parametrize("kw,moment", [
+    (dict(), True), (dict(normalize=0), False), (dict(a1=-1.0), True), (dict(a1=1.01), False), (dict(a1=-1.01), False),
+    (dict(a2=2.3), True), (dict(a2=2.6), False), (dict(a1=0.0, a2=4.0), True), (dict(a1=0.0, a2=4.01), False),
+    (dict(a1=0.0, a2=-0.66), True), (dict(a1=0.0, a2=-0.67), False), (dict(a1=0.5, a2=-0.5), False),
+    (dict(a0=2.0, a1=2.0, a2=1.0), True), (dict(lim=0.5), True), (dict(lim=-1.0), True), (dict(lim=1.01), False),
+    (dict(lim=0.0), True), (dict(a0=0.0), False), (dict(a0=-1.0, a1=-1.0, a2=-0.5), False), (dict(a0=0.9), False),
+    (dict(a1=float("nan")), False), (dict(a2=float("nan")), False), (dict(lim=float("inf")), False)])
+def test_moment_form_forward_only_where_the_terms_hardly_cancel(kw, moment):
+    """Its sums round relative to a2 |q|^2 |k|^2, whatever the scores are: on |s| <= lim^2 the polynomial has to stay above a
+    fifth of the sizes of its terms.  The workspace tells which form is planned."""
+    heads, nq, nk = 64, 4000, 4033
+    fwd, _ = sizes(**{**dict(bh=heads, bhkv=heads, nq=nq, nk=nk, d=64, mask=0), **kw})
+    parts = 6 * 64 * heads * (nq + 2 * nk)
+    assert (fwd > parts + 1024) == moment
