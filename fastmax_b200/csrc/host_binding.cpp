@@ -235,6 +235,7 @@ std::optional<Tensor> decode_step(uintptr_t problem, const Tensor& q, const Tens
            t.device() == state.device() && t.is_contiguous();
   };
   if (!row_ok(q, pr.bh) || !row_ok(k, pr.bhkv) || !row_ok(v, pr.bhkv)) return std::nullopt;
+  py::gil_scoped_release no_gil;       // a launch waits while the device's queue is full
   const c10::cuda::CUDAGuard guard(state.device());
   Tensor out = at::empty(q.sizes(), q.options());
   check_rc(fastmax_b200_decode_step(&pr, q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(), scratch.data_ptr(),

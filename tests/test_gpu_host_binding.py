@@ -107,3 +107,36 @@ def test_call_site_and_decode(monkeypatch):
     b, db = site(), decode()
     assert torch.equal(a[0], b[0]) and torch.allclose(a[1], b[1], rtol=0, atol=2e-2)
     assert torch.equal(da[0], db[0]) and torch.equal(da[1], db[1]) and da[2] == db[2] == 1
+
+
+def test_decode_step_lets_other_threads_run():
+    """A launch waits once the device's queue is full (some 1000 kernels); other Python threads go on meanwhile."""
+    import threading
+    import time
+
+    st = fastmax_b200.FastmaxDecodeState(4, 4, 64, torch.bfloat16, "cuda")
+    row = torch.randn(4, 1, 64, device="cuda").bfloat16()
+    st.step(row, row, row)
+    torch.cuda.synchronize()
+    gaps, done = [0.0], threading.Event()
+
+    def watch():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    t = threading.Thread(target=watch)
+    t.start()
+    start = time.perf_counter()
+    torch.cuda._sleep(1_500_000_000)        # clocks: 0.75 s and more
+    for _ in range(3000):
+        st.step(row, row, row)
+    issued = time.perf_counter() - start
+    done.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert issued > 0.5, issued             # the queue was full for most of the pause
+    assert max(gaps) < 0.25, max(gaps)
