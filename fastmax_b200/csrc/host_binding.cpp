@@ -173,7 +173,8 @@ struct FromQKV : public torch::autograd::Function<FromQKV> {
     const fastmax_problem pr = problem_of(q, k, a);
     const bool bt = fastmax_b200_bt_layout_supported(&pr, (int)heads) != 0;    // the attention kernel writes (B, T, H, hs) itself
     auto [out, den, stats] = run_forward(q, k, v, a, bt ? (int)heads : 0);
-    ctx->save_for_backward({q, k, v, out, den, stats, cs, sn});
+    // without a rotation the tables are not part of the problem: the caller may go on changing them
+    ctx->save_for_backward({q, k, v, out, den, stats, rope ? cs : Tensor(), rope ? sn : Tensor()});
     keep(ctx, a);
     ctx->saved_data["d"] = std::vector<int64_t>{b, n, groups, qper, d, rope, bt ? 1 : 0};
     if (bt) return out.view({b, n, heads * d});

@@ -140,3 +140,14 @@ def test_decode_step_lets_other_threads_run():
     torch.cuda.synchronize()
     assert issued > 0.5, issued             # the queue was full for most of the pause
     assert max(gaps) < 0.25, max(gaps)
+
+
+def test_tables_that_no_rotation_reads_may_change():
+    g = torch.Generator(device="cuda").manual_seed(6)
+    qkv = torch.randn(2, 45, 8 * 64, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    cos, sin = torch.zeros(45, 64, device="cuda"), torch.zeros(45, 64, device="cuda")
+    y = fastmax_b200.fastmax_attention_from_qkv(qkv, cos, sin, 4, 2, 64, 0)
+    cos.add_(1.0)
+    sin.add_(1.0)
+    y.sum().backward()
+    assert torch.isfinite(qkv.grad).all()
