@@ -1,11 +1,14 @@
 """Access to ``_host``, the C++ host side of the package's frequent calls (``csrc/host_binding.cpp``).
 
 ``host()`` is the module, or None where it was not built; ``plain_mode()`` says whether nothing is active that the Python
-autograd functions take part in and C++ ones do not: tracing, compilation, functorch transforms, dispatch modes.
+autograd functions take part in and C++ ones do not: tracing, compilation, functorch transforms, dispatch and function
+modes.
 """
 from __future__ import annotations
 
 import torch
+from torch.overrides import _get_current_function_mode_stack as _function_modes
+from torch.utils._device import DeviceContext as _DeviceContext
 
 _module = None
 _looked = False
@@ -29,8 +32,11 @@ def host():
 
 def plain_mode() -> bool:
     c = torch._C
-    return (c._functorch.peek_interpreter_stack() is None and c._get_tracing_state() is None
-            and c._len_torch_dispatch_stack() == 0 and not torch.compiler.is_compiling())
+    if (c._functorch.peek_interpreter_stack() is not None or c._get_tracing_state() is not None
+            or c._len_torch_dispatch_stack() or torch.compiler.is_compiling()):
+        return False
+    # a default device is a function mode too, but every allocation here names its device
+    return not c._len_torch_function_stack() or all(type(m) is _DeviceContext for m in _function_modes())
 
 
 def plain_tensors(*tensors) -> bool:

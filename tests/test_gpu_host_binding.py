@@ -151,3 +151,25 @@ def test_tables_that_no_rotation_reads_may_change():
     sin.add_(1.0)
     y.sum().backward()
     assert torch.isfinite(qkv.grad).all()
+
+
+def test_function_modes_see_the_calls_inside(monkeypatch):
+    """A torch function mode takes the Python function, as with the module absent; a default device is no such mode."""
+    class Record(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            self.seen.append(getattr(func, "__name__", str(func)))
+            return func(*args, **(kwargs or {}))
+
+    q, k, v, _ = _inputs()
+    mod = fastmax_b200.FASTMultiHeadAttention()
+    seen = []
+    for present in (True, False):
+        if not present:
+            monkeypatch.setattr(_native, "host", lambda: None)
+        with Record() as mode:
+            mode.seen = []
+            mod(q, k, v, **KW)
+        seen.append(mode.seen)
+    assert "contiguous" in seen[0] and seen[0] == seen[1]
+    with torch.device("cuda"):
+        assert _native.plain_mode()
