@@ -2,18 +2,25 @@
 
 ``host()`` is the module, or None where it was not built; ``plain_mode()`` says whether nothing is active that the Python
 autograd functions take part in and C++ ones do not: tracing, compilation, functorch transforms, dispatch and function
-modes.
+modes.  A torch that does not offer these queries counts as one in which something is active.
 """
 from __future__ import annotations
 
 import torch
-from torch.overrides import _get_current_function_mode_stack as _function_modes
-from torch.utils._device import DeviceContext as _DeviceContext
 
 _module = None
 _looked = False
 _TENSORS = (torch.Tensor, torch.nn.Parameter)
 _NUMBERS = (int, float)
+
+try:
+    from torch.overrides import _get_current_function_mode_stack as _function_modes
+    from torch.utils._device import DeviceContext as _DeviceContext
+
+    _queries = (torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state, torch._C._len_torch_dispatch_stack,
+                torch._C._len_torch_function_stack)
+except (ImportError, AttributeError):
+    _queries = None
 
 
 def host():
@@ -31,12 +38,13 @@ def host():
 
 
 def plain_mode() -> bool:
-    c = torch._C
-    if (c._functorch.peek_interpreter_stack() is not None or c._get_tracing_state() is not None
-            or c._len_torch_dispatch_stack() or torch.compiler.is_compiling()):
+    if torch.compiler.is_compiling() or _queries is None:
+        return False
+    transforms, tracing, dispatch_modes, function_modes = _queries
+    if transforms() is not None or tracing() is not None or dispatch_modes():
         return False
     # a default device is a function mode too, but every allocation here names its device
-    return not c._len_torch_function_stack() or all(type(m) is _DeviceContext for m in _function_modes())
+    return not function_modes() or all(type(m) is _DeviceContext for m in _function_modes())
 
 
 def plain_tensors(*tensors) -> bool:

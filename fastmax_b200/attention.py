@@ -182,7 +182,7 @@ class FASTMultiHeadAttention(torch.nn.Module):
         if self.use_custom_gradient:
             # the plain case as one C++ autograd function; everything else, and every error, in Python
             if (not dropout and _native.plain_tensors(q, k, v) and (p == 1 or p == 2)
-                    and _native.plain_numbers(temperature, a0, a1, a2, lim) and _native.host() and _native.plain_mode()):
+                    and _native.plain_numbers(temperature, a0, a1, a2, lim) and _native.plain_mode() and _native.host()):
                 out = _native.host().attention(q, k, v, bool(mask), bool(normalize), temperature, a0, a1, a2, lim, int(p))
                 if out is not None:
                     return out

@@ -82,7 +82,7 @@ def fastmax_attention_from_qkv(qkv, cos, sin, n_head, n_query_groups, head_size,
     if not qkv.is_cuda:
         raise RuntimeError("fastmax_attention_from_qkv needs CUDA tensors (there is no CPU path)")
     if (impl == "auto" and _native.plain_tensors(qkv, cos, sin) and (p == 1 or p == 2)
-            and _native.plain_numbers(temperature, a0, a1, a2, lim) and _native.host() and _native.plain_mode()):
+            and _native.plain_numbers(temperature, a0, a1, a2, lim) and _native.plain_mode() and _native.host()):
         # the plain case as one C++ autograd function (float32 tables on the device); everything else below
         y = _native.host().from_qkv(qkv, cos, sin, n_query_groups, qper, head_size, int(rope_n_elem), bool(mask),
                                     bool(normalize), temperature, a0, a1, a2, lim, int(p))

@@ -72,7 +72,7 @@ class FastmaxDecodeState:
 
     def step(self, q, k, v):
         """Add one token and return the attention row of q (bh, 1, d) over all tokens so far."""
-        if _native.plain_tensors(q, k, v) and _native.host() and _native.plain_mode():
+        if _native.plain_tensors(q, k, v) and _native.plain_mode() and _native.host():
             out = _native.host().decode_step(ctypes.addressof(self.prob), q, k, v, self.state, self.scratch)
             if out is not None:
                 self.tokens += 1

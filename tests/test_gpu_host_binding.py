@@ -173,3 +173,9 @@ def test_function_modes_see_the_calls_inside(monkeypatch):
     assert "contiguous" in seen[0] and seen[0] == seen[1]
     with torch.device("cuda"):
         assert _native.plain_mode()
+
+
+def test_without_the_queries_of_torch_the_python_function_serves(monkeypatch):
+    q, k, v, _ = _inputs()
+    monkeypatch.setattr(_native, "_queries", None)
+    assert torch.equal(fastmax_b200.FASTMultiHeadAttention()(q, k, v, **KW), _python(q, k, v))
