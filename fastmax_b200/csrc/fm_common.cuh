@@ -63,6 +63,13 @@ __host__ __device__ __forceinline__ int stat_row(stat_t s) {
 __device__ __forceinline__ float stat_scale(const stat_t* st, int head, float lim) {
   return st ? lim / sqrtf(stat_norm2(st[head])) : 1.0f;
 }
+// The power of two below a normal positive s (1 for any other).  Rows taken times that of their scale, which is exact, have
+// norms near lim wherever the inputs lie, so that products of several of their features stay in range; what reads the
+// products applies the rest of the scale.
+__device__ __forceinline__ float pow2_of(float s) {
+  const uint32_t e = __float_as_uint(s) & 0x7F800000u;
+  return e == 0u || e == 0x7F800000u ? 1.f : __uint_as_float(e);
+}
 
 // Order of the row tiles in a score kernel's grid.  Long grids go head by head, so that a head's column tiles stay in
 // L2.  A causal grid of a few waves goes tile by tile over all heads (`by_tile` = number of row heads): the longest row
@@ -213,8 +220,8 @@ int dense_split_forward(const Ctx& c, const void* q, const void* k, const void* 
 int dense_split_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* out, const float* den,
                          const stat_t* stats, const void* grad_out, float* dots, void* grad_q, void* grad_k,
                          void* grad_v, void* workspace, const ChunkAdd* ca = nullptr);
-// rows of d float32 -> rows of [h | m | l], 3 d bf16, for two tensors
-int split3_rows(const Ctx& c, const void* a, void* a3, size_t rows_a, const void* b, void* b3, size_t rows_b);
+// rows of d float32 -> rows of [h | m | l], 3 d bf16, of q and v; q times pow2_of its head's scale first (exact)
+int split3_scaled_q(const Ctx& c, const void* q, void* q3, const void* v, void* v3, const stat_t* stats);
 // Unmasked second-order forward of the float32 score family in moment form (fm_split_moments.cu): whether it is the
 // faster one for the problem's sizes, its workspace, and the call.
 bool split_moments_faster(const fastmax_problem& p);

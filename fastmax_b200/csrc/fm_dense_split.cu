@@ -595,6 +595,9 @@ struct SplitJob {
   const float* den;
   const float* out;
   float* dvec;
+  const stat_t* stat;     // rows are taken times pow2_of the scale of their head, `n` rows each, or null
+  int n;
+  float lim;
 };
 struct SplitJobs {
   SplitJob j[4];
@@ -636,6 +639,11 @@ __global__ void __launch_bounds__(256) split3_kernel(const SplitJobs jobs) {
     for (int e = 0; e < 8; ++e) f[e] *= inv;
   }
   if (!ok) return;
+  if (jb.stat) {
+    const float s = pow2_of(stat_scale(jb.stat, (int)(row / jb.n), jb.lim));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] *= s;
+  }
   uint32_t h[4], m[4], l[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) split3(pack2(f[2 * e], f[2 * e + 1]), h[e], m[e], l[e]);
@@ -778,10 +786,11 @@ int dense_split_backward(const Ctx& c, const void* q, const void* k, const void*
   return launch_mode<64, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, p.nk, p.nq, a);
 }
 
-int split3_rows(const Ctx& c, const void* a, void* a3, size_t rows_a, const void* b, void* b3, size_t rows_b) {
+int split3_scaled_q(const Ctx& c, const void* q, void* q3, const void* v, void* v3, const stat_t* stats) {
+  const fastmax_problem& p = c.p;
   SplitJobs jobs = {};
-  jobs.j[0] = {(const float*)a, (__nv_bfloat16*)a3, rows_a, nullptr, nullptr, nullptr};
-  jobs.j[1] = {(const float*)b, (__nv_bfloat16*)b3, rows_b, nullptr, nullptr, nullptr};
+  jobs.j[0] = {(const float*)q, (__nv_bfloat16*)q3, (size_t)p.bh * p.nq, nullptr, nullptr, nullptr, stats, p.nq, p.lim};
+  jobs.j[1] = {(const float*)v, (__nv_bfloat16*)v3, (size_t)p.bhkv * p.nk, nullptr, nullptr, nullptr};
   return launch_split3(c, jobs, 2);
 }
 

@@ -23,13 +23,6 @@ using namespace rdo;
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_smom_status, 0, code); }
 
-// The power of two below a normal positive s.  Normalised keys are taken times that of their scale (exact), so that their
-// squares stay in range wherever the keys lie; the read-out applies the rest of the scale.
-__device__ __forceinline__ float pow2_of(float s) {
-  const uint32_t e = __float_as_uint(s) & 0x7F800000u;
-  return e == 0u || e == 0x7F800000u ? 1.f : __uint_as_float(e);
-}
-
 // ---- sums over the keys ---------------------------------------------------------------------------------------
 // Rows as in fm_decode_tc.cu: lane L of tile t is the pair (b, b + s mod 64), b = L % 64, s = 2 t + L / 64, s = 0..32 (half
 // of s = 32); row 64 of the transposed block is ones (the first-order rows and the constant row), row 65 zeros.
@@ -144,7 +137,7 @@ pair_sums_kernel(const __grid_constant__ CUtensorMap tmV, const float* __restric
     };
     // four features of one token per thread and load, two loads a block; tokens past the end read as zero
     const float* kh = k + (size_t)head * n * D;
-    const float ks = stat_k ? pow2_of(stat_scale(stat_k, head, lim)) : 1.f;
+    const float ks = pow2_of(stat_scale(stat_k, head, lim));
     float4 kr[2];
     auto fetch = [&](int j) {
 #pragma unroll
@@ -436,8 +429,8 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
     auto first_rows = [&](const Walk& w) { return a.state + (size_t)(w.head / ratio) * a.per_state + (size_t)(64 * 64) * a.dvp; };
     auto const_of = [&](const Walk& w) { return w.more() && row <= 64 ? __ldg(first_rows(w) + (size_t)64 * a.dvp + row) : 0.f; };
     auto norm_of = [&](const Walk& w) { return w.more() && h && row < 64 ? __ldg(first_rows(w) + (size_t)row * a.dvp + 64) : 0.f; };
-    auto q_of = [&](const Walk& w) { return a.stat_q && w.more() ? a.stat_q[w.head] : (stat_t)0; };
-    auto k_of = [&](const Walk& w) { return a.stat_k && w.more() ? a.stat_k[w.head / ratio] : (stat_t)0; };
+    auto q_of = [&](const Walk& w) { return w.more() ? a.stat_q[w.head] : (stat_t)0; };
+    auto k_of = [&](const Walk& w) { return w.more() ? a.stat_k[w.head / ratio] : (stat_t)0; };
     Walk w(a);
     float s0next = const_of(w), n1next = norm_of(w);
     stat_t qnext = q_of(w), knext = k_of(w);
@@ -453,11 +446,9 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
       if (lane == 0) mbar_arrive(BAR_TFREE(t, buf));
     };
     for (; w.more(); ++k) {
-      float c = 1.f;
-      if (a.stat_q) {
-        const float sk = stat_scale(&knext, 0, a.lim);
-        c = stat_scale(&qnext, 0, a.lim) * (sk / pow2_of(sk));
-      }
+      // what pow2_of has left of the scales of the queries and of the keys
+      const float sq = stat_scale(&qnext, 0, a.lim), sk = stat_scale(&knext, 0, a.lim);
+      const float c = (sq / pow2_of(sq)) * (sk / pow2_of(sk));
       const float A1 = a.a1 * c, A2 = a.a2 * c * c;
       const int tok = w.tok0(a) + t * 128 + row;
       const bool tok_ok = tok < a.n;
@@ -634,14 +625,14 @@ int split_moments_forward(const Ctx& c, const void* q, const void* k, const void
   char* ws = (char*)workspace;
   float* state = (float*)(ws + l.state);
   int rc;
-  if ((rc = split3_rows(c, q, ws + l.q3, (size_t)p.bh * p.nq, v, ws + l.v3, (size_t)p.bhkv * p.nk))) return rc;
+  if ((rc = split3_scaled_q(c, q, ws + l.q3, v, ws + l.v3, stats))) return rc;
   CUtensorMap tv, tx;
   if ((rc = tma_map_bf16(&tv, ws + l.v3, p.bhkv, p.nk, 3 * 64, TB))) return rc;
   if ((rc = tma_map_bf16(&tx, ws + l.q3, p.bh, p.nq, 3 * 64, 128))) return rc;
   FM_CUDA_TRY(cudaFuncSetAttribute(pair_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM));
   const dim3 sums((PS_TILES + 1) / 2, p.bhkv);
   FM_LAUNCH("fm_split_pair_sums", c.stream, (pair_sums_kernel<<<sums, PS_THREADS, PS_SMEM, c.stream>>>(
-                                                tv, (const float*)k, p.normalize ? stats + p.bh : nullptr, p.lim, state, p.nk, m.dvp, (size_t)m.f * m.dvp)));
+                                                tv, (const float*)k, stats + p.bh, p.lim, state, p.nk, m.dvp, (size_t)m.f * m.dvp)));
   FM_CUDA_TRY(cudaGetLastError());
   const dim3 grid(65, p.bhkv);
   FM_LAUNCH("fm_split_state_copies", c.stream,
@@ -652,8 +643,8 @@ int split_moments_forward(const Ctx& c, const void* q, const void* k, const void
   a.state = state;
   a.out = (float*)o.out;
   a.den = o.den;
-  a.stat_q = p.normalize ? stats : nullptr;
-  a.stat_k = p.normalize ? stats + p.bh : nullptr;
+  a.stat_q = stats;
+  a.stat_k = stats + p.bh;
   a.a0 = p.a0; a.a1 = p.a1; a.a2 = p.a2; a.lim = p.lim;
   a.per_state = (size_t)m.f * m.dvp;
   a.dvp = m.dvp;

@@ -1,6 +1,6 @@
 """float32 unmasked second-order forward in moment form against float64: last groups of 1, 15, 65 and 161 of 256 query rows,
-last key blocks of 1, 15 and 63 of 64, grouped heads, more query groups than SMs, keys whose squares alone would leave
-float32's range.
+last key blocks of 1, 15 and 63 of 64, grouped heads, more query groups than SMs, keys and queries whose squares alone would
+leave float32's range.
 
 Bound: operands and products are exact to 2^-24; a sum over n keys is rounded to nearest once per 64 keys, a random walk of
 sqrt(n / 64) steps of 2^-25 of it, 13 steps at 10 000 keys, and the rows average 4 160 such sums.  1e-6 in the 2-norm is
@@ -27,20 +27,21 @@ def reference(q, k, v, norm, a):
     return out
 
 
-# query heads, key heads, nq, nk, normalize, scale of the keys
-@pytest.mark.parametrize("bh,bhkv,nq,nk,norm,scale", [
-    (8, 8, 9999, 9999, 1, 1.0), (8, 2, 40001, 2111, 1, 1e17), (16, 4, 4097, 8191, 1, 0.1), (64, 64, 4001, 4033, 1, 1e-17)])
-def test_moment_form_forward_against_float64(bh, bhkv, nq, nk, norm, scale):
+# query heads, key heads, nq, nk, scale of the keys, of the queries
+@pytest.mark.parametrize("bh,bhkv,nq,nk,kscale,qscale", [
+    (8, 8, 9999, 9999, 1.0, 1.0), (8, 2, 40001, 2111, 1e17, 1e-18), (16, 4, 4097, 8191, 0.1, 1e18),
+    (64, 64, 4001, 4033, 1e-17, 1e18)])
+def test_moment_form_forward_against_float64(bh, bhkv, nq, nk, kscale, qscale):
     g = torch.Generator(device="cuda").manual_seed(nq)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
-    q, k, v = rnd(bh, nq, 64), rnd(bhkv, nk, 64) * scale, rnd(bhkv, nk, 64)
+    q, k, v = rnd(bh, nq, 64) * qscale, rnd(bhkv, nk, 64) * kscale, rnd(bhkv, nk, 64)
     _cabi.profile(True)
-    out, den, _ = _cabi.forward(q, k, v, mask=0, normalize=norm, p=2, a0=1.0, a1=0.7, a2=0.4, lim=1.0)
+    out, den, _ = _cabi.forward(q, k, v, mask=0, normalize=1, p=2, a0=1.0, a1=0.7, a2=0.4, lim=1.0)
     names = {n for n, _ in _cabi.profile_records()}
     _cabi.profile(False)
     assert "fm_split_readout" in names, names
     assert _cabi.device_status() == 0
-    ref = reference(q, k, v, norm, (1.0, 0.7, 0.4))
+    ref = reference(q, k, v, 1, (1.0, 0.7, 0.4))
     err = float((out.double() - ref).norm() / ref.norm())
     assert err < 1e-6, err
 
