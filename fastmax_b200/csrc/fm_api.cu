@@ -220,6 +220,14 @@ static bool first_order_unaligned(const fastmax_problem& p, int impl, std::initi
          !aligned16(ptrs);
 }
 
+// The tensor-core state kernels and read-outs move states, their bf16 copies and result rows 16 bytes at a time, by TMA among
+// others, and all of those lie in workspaces or buffers of the caller.
+static int check_state_alignment(const fastmax_problem& p, std::initializer_list<const void*> ptrs) {
+  if ((moments_tc_supports(p) || first_tc_supports(p)) && !aligned16(ptrs))
+    return fail(FASTMAX_E_ARG, "workspaces, moment states and totals must be 16-byte aligned");
+  return FASTMAX_OK;
+}
+
 // Backward workspace: [dots: bh+bhkv floats][delta or dvec: bh*nq floats]
 // [gs: bh*nq*d bf16, tensor-core family only], 256-byte aligned parts.
 struct BwdWs {
@@ -427,7 +435,6 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   if (p.bh == 0 || p.nq == 0) return FASTMAX_OK;
   if (!q || !k || !v || !o.out || !o.den) return fail(FASTMAX_E_ARG, "NULL tensor pointer");
   if (p.normalize && !stats) return fail(FASTMAX_E_ARG, "normalize needs a stats buffer");
-  if ((rc = check_device())) return rc;
   int impl;
   if ((rc = pick_impl(p, o.out_f32 != 0, &impl))) return rc;
   if (p.impl == FASTMAX_IMPL_AUTO && impl == FASTMAX_IMPL_DENSE_TC && !aligned16({q, k, v, o.out}))
@@ -435,6 +442,8 @@ static int forward_impl(const fastmax_problem* prob, const void* q, const void* 
   const bool first_unaligned = first_order_unaligned(p, impl, {q, k, v, o.out});
   if (heads_per_batch && (rc = bt_layout_ok(p, heads_per_batch, first_unaligned ? FASTMAX_IMPL_DENSE_FFMA : impl)))
     return rc;
+  if (impl == FASTMAX_IMPL_MOMENTS && !first_unaligned && (rc = check_state_alignment(p, {workspace}))) return rc;
+  if ((rc = check_device())) return rc;
   Ctx c{p, (cudaStream_t)stream};
   c.out_heads = heads_per_batch;
   if (p.normalize && (rc = launch_rowmax(c, q, k, (stat_t*)stats))) return rc;
@@ -521,6 +530,7 @@ static int backward_impl(const fastmax_problem* prob, const void* q, const void*
   if (need > 0 && (!workspace || workspace_bytes < need))
     return fail(FASTMAX_E_WORKSPACE, "backward workspace too small: need %zu bytes, got %zu", need,
                 workspace_bytes);
+  if (impl == FASTMAX_IMPL_MOMENTS && (rc = check_state_alignment(p, {workspace}))) return rc;
   if ((rc = check_device())) return rc;
   Ctx c{p, (cudaStream_t)stream};
   c.out_heads = heads_per_batch;
@@ -575,11 +585,13 @@ int fastmax_b200_backward_bt(const fastmax_problem* prob, const void* q, const v
 }
 
 // ---- sequence sharding ------------------------------------------------------------------
-static int validate_shard(const fastmax_problem* prob) {
+// ptrs: the call's states, totals and workspace
+static int validate_shard(const fastmax_problem* prob, std::initializer_list<const void*> ptrs = {}) {
   int rc = validate(prob);
   if (rc) return rc;
   if (prob->nq != prob->nk || prob->bh != prob->bhkv || prob->bh > 65535)
     return fail(FASTMAX_E_ARG, "a sequence shard needs nq == nk and bh == bhkv <= 65535");
+  if ((rc = check_state_alignment(*prob, ptrs))) return rc;
   return check_device();
 }
 static size_t shard_s16_bytes(const fastmax_problem& p) { return state16_bytes(p, p.nq); }
@@ -630,7 +642,7 @@ int fastmax_b200_shard_rowmax(const fastmax_problem* prob, const void* q, const 
 
 int fastmax_b200_shard_kv_state(const fastmax_problem* prob, const void* k, const void* v,
                                 float* kv_states, float* kv_total, void* stream) {
-  int rc = validate_shard(prob);
+  int rc = validate_shard(prob, {kv_states, kv_total});
   if (rc) return rc;
   if (!k || !v || !kv_states || !kv_total) return fail(FASTMAX_E_ARG, "NULL tensor pointer");
   const fastmax_problem& p = *prob;
@@ -644,7 +656,7 @@ int fastmax_b200_shard_forward(const fastmax_problem* prob, const void* q, const
                                const void* v, const void* stats, float* kv_states,
                                const float* s_base, void* out, float* den, void* workspace,
                                size_t workspace_bytes, void* stream) {
-  int rc = validate_shard(prob);
+  int rc = validate_shard(prob, {kv_states, s_base, workspace});
   if (rc) return rc;
   const fastmax_problem& p = *prob;
   if (!q || !k || !v || !out || !den) return fail(FASTMAX_E_ARG, "NULL tensor pointer");
@@ -669,7 +681,7 @@ int fastmax_b200_shard_qg_state(const fastmax_problem* prob, const void* q, cons
                                 const float* den, const void* grad_out, float* delta,
                                 float* qg_states, float* qg_total, void* workspace,
                                 size_t workspace_bytes, void* stream) {
-  int rc = validate_shard(prob);
+  int rc = validate_shard(prob, {qg_states, qg_total, workspace});
   if (rc) return rc;
   const fastmax_problem& p = *prob;
   if (!q || !out || !den || !grad_out || !delta || !qg_states || !qg_total)
@@ -695,7 +707,7 @@ int fastmax_b200_shard_backward(const fastmax_problem* prob, const void* q, cons
                                 const float* kv_states, float* qg_states, const float* r_base,
                                 float* dots, void* grad_q, void* grad_k, void* grad_v,
                                 int32_t dq_far_done, void* workspace, size_t workspace_bytes, void* stream) {
-  int rc = validate_shard(prob);
+  int rc = validate_shard(prob, {kv_states, qg_states, r_base, workspace});
   if (rc) return rc;
   const fastmax_problem& p = *prob;
   if (!q || !k || !v || !out || !den || !grad_out || !delta || !kv_states || !dots || !grad_q || !grad_k ||
@@ -730,7 +742,7 @@ int fastmax_b200_shard_backward(const fastmax_problem* prob, const void* q, cons
 int fastmax_b200_shard_dq_far(const fastmax_problem* prob, const void* q, const float* den, const void* stats,
                               const void* grad_out, const float* delta, const float* kv_states, void* workspace,
                               size_t workspace_bytes, void* stream) {
-  int rc = validate_shard(prob);
+  int rc = validate_shard(prob, {kv_states, workspace});
   if (rc) return rc;
   const fastmax_problem& p = *prob;
   if (!p.mask) return fail(FASTMAX_E_ARG, "shard_dq_far applies to causal shards only");

@@ -724,6 +724,8 @@ size_t moments_tc_copy_b_bytes(int mats) { return (size_t)mats * B_BYTES; }
 int moments_tc_convert(const Ctx& c, int mats, const float* state, const StateCopies& to) {
   if (mats == 0) return FASTMAX_OK;
   const MomentDims m = moment_dims(64);
+  if ((((uintptr_t)to.a | (uintptr_t)to.b) & 15) != 0)
+    return fail(FASTMAX_E_ARG, "the copies of the moment states must be 16-byte aligned");
   dim3 grid(65, mats);
   FM_LAUNCH("fm_moments_state_bf16", c.stream,
             (copies_kernel<<<grid, 256, 0, c.stream>>>(state, (char*)to.a, (char*)to.b, m.dvp, (size_t)m.f * m.dvp)));
@@ -738,8 +740,8 @@ int moments_tc_prefix_convert(const Ctx& c, int heads, int nchunk, const float* 
                               const StateCopies& to) {
   if (heads == 0 || nchunk == 0) return FASTMAX_OK;
   const MomentDims m = moment_dims(64);
-  if ((((uintptr_t)state | (uintptr_t)base) & 15) != 0)
-    return fail(FASTMAX_E_ARG, "moment states and totals must be 16-byte aligned");
+  if ((((uintptr_t)state | (uintptr_t)base | (uintptr_t)to.a | (uintptr_t)to.b) & 15) != 0)
+    return fail(FASTMAX_E_ARG, "moment states, totals and copies must be 16-byte aligned");
   dim3 grid(65, heads);
   FM_LAUNCH("fm_moments_prefix_bf16", c.stream,
             (prefix_copies_kernel<<<grid, 256, 0, c.stream>>>(state, base, (char*)to.a, (char*)to.b, nchunk, m.dvp,

@@ -140,7 +140,11 @@ int fastmax_b200_selected_impl(const fastmax_problem* prob, int32_t* impl);
 
 /* Bytes of scratch the forward / backward pass works with (may be 0), and the least each still runs with: float32
  * with d 32 or 64 takes 6 bytes per element of q, k and v (backward: and grad_out) for the operands of its tensor-core
- * kernels and runs on the CUDA cores, several times slower, in a workspace without that room. */
+ * kernels and runs on the CUDA cores, several times slower, in a workspace without that room.
+ * Alignment: workspaces, moment states and totals should start at multiples of 16 bytes.  bf16 calls whose kernels move
+ * them in such pieces (the moment family at d 64 and 128, shards included; the gradients of the tensor-core score family)
+ * are refused with FASTMAX_E_ARG otherwise.  The float32 tensor-core kernels run in workspaces that start at multiples of
+ * 256 bytes; a call with another one runs on the CUDA cores. */
 size_t fastmax_b200_forward_workspace_bytes(const fastmax_problem* prob);
 size_t fastmax_b200_backward_workspace_bytes(const fastmax_problem* prob);
 size_t fastmax_b200_forward_workspace_least_bytes(const fastmax_problem* prob);

@@ -120,6 +120,38 @@ def test_bad_arguments_are_rejected_before_any_launch():
     assert L.fastmax_b200_forward(prob, 1, 1, 1, 1, 1, 1, None, 0, None) == -1
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="made-up addresses, which only a machine without a device may see")
+@pytest.mark.parametrize("p", [1, 2])
+@pytest.mark.parametrize("mask", [0, 1])
+def test_unaligned_state_buffers_are_an_argument_error(p, mask):
+    """The bf16 moment kernels move states, their copies and result rows 16 bytes at a time, all of them in the caller's
+    workspace: an unaligned one is refused before any launch, as are unaligned states and totals of a shard."""
+    L, good, bad, big = _cabi.lib(), 1 << 20, (1 << 20) + 8, 1 << 40
+    prob = _cabi.Problem(dtype=_cabi.BF16, bh=2, bhkv=2, nq=5000, nk=5000, d=64, mask=mask, normalize=1, p=p, impl=3, a0=1,
+                         a1=1, a2=0.5, lim=1, temperature=1)
+
+    def codes(ws, state):
+        g = good
+        yield L.fastmax_b200_forward(prob, g, g, g, g, g, g, ws, big, None)
+        yield L.fastmax_b200_backward(prob, g, g, g, g, g, g, g, g, g, g, ws, big, None)
+        if mask:
+            yield L.fastmax_b200_forward_bt(prob, g, g, g, g, g, g, 2, ws, big, None)
+            yield L.fastmax_b200_backward_bt(prob, g, g, g, g, g, g, g, 2, g, g, g, ws, big, None)
+            yield L.fastmax_b200_shard_dq_far(prob, g, g, g, g, g, state, ws, big, None)
+        yield L.fastmax_b200_shard_forward(prob, g, g, g, g, state, state, g, g, ws, big, None)
+        yield L.fastmax_b200_shard_qg_state(prob, g, g, g, g, g, state, state, ws, big, None)
+        yield L.fastmax_b200_shard_backward(prob, g, g, g, g, g, g, g, g, state, state, state, g, g, g, g, 0, ws, big, None)
+
+    for ws, state in ((bad, good), (bad, bad)):
+        for rc in codes(ws, state):
+            assert rc == -1 and b"16-byte aligned" in L.fastmax_b200_last_error(), (rc, L.fastmax_b200_last_error())
+    for rc in (L.fastmax_b200_shard_kv_state(prob, good, good, bad, good, None),
+               L.fastmax_b200_shard_kv_state(prob, good, good, good, bad, None),
+               L.fastmax_b200_shard_forward(prob, good, good, good, good, bad, bad, good, good, good, big, None)):
+        assert rc == -1
+    assert all(rc not in (0, -1) for rc in codes(good, good))       # nothing else is wrong with these calls: no device here
+
+
 def test_custom_path_refuses_cpu_tensors():
     q = torch.randn(1, 2, 8, 8)
     with pytest.raises(RuntimeError):
