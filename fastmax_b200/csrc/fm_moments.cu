@@ -43,24 +43,35 @@ size_t moment_total_bytes(const fastmax_problem& p) {
   return up256(sizeof(float) * (size_t)p.bh * m.f * m.dvp);
 }
 
-// bf16 copies of the chunk states that the tensor-core read-outs multiply:
-// [second order, type A][second order, type B][first order]
+// bf16 copies of the chunk states that the tensor-core read-outs multiply: second order, in one layout for read-outs of type
+// A and one for type B, or first order.  The room for them holds one layout.
 static size_t copies_a_bytes(const fastmax_problem& p, int mats) {
   return moments_tc_supports(p) ? up256(moments_tc_copy_a_bytes(mats)) : 0;
 }
 static size_t copies_b_bytes(const fastmax_problem& p, int mats) {
   return moments_tc_supports(p) ? up256(moments_tc_copy_b_bytes(mats)) : 0;
 }
-static StateCopies copies_at(const fastmax_problem& p, void* s16, int mats) {
+// Where the copies of `mats` states go that are read out in one kind (mode 0: A, 1: B) or both (2): `s16`, and for both kinds
+// the type B ones lie in the rows of n tokens that the type A read-out will write, which therefore comes second.  Chunks
+// that are too short for that (of less than 1216 tokens) use s16 for one kind after the other: c.a == c.b.
+static StateCopies copies_at(const fastmax_problem& p, int mode, void* s16, float* rows_a, int n, int mats) {
   StateCopies c;
-  c.a = s16;
-  c.b = (char*)s16 + copies_a_bytes(p, mats);
+  if (mode != 1) c.a = s16;
+  if (mode != 0) c.b = s16;
+  if (mode == 2 && copies_b_bytes(p, mats) <= sizeof(float) * (size_t)p.bh * n * p.d) c.b = rows_a;
+  return c;
+}
+// the layouts of `c` that can be written at once
+static StateCopies at_once(StateCopies c) {
+  if (c.a == c.b) c.a = nullptr;
   return c;
 }
 size_t state16_bytes(const fastmax_problem& p, int n) {
   const int L = moments_chunk(p);
   const int mats = p.bh * ((n + L - 1) / L);
-  return copies_a_bytes(p, mats) + copies_b_bytes(p, mats) + (first_tc_supports(p) ? up256(first_tc_copy_bytes(p, mats)) : 0);
+  const size_t a = copies_a_bytes(p, mats), b = copies_b_bytes(p, mats);
+  if (a > 0) return a > b ? a : b;
+  return first_tc_supports(p) ? up256(first_tc_copy_bytes(p, mats)) : 0;
 }
 
 // the type B copies of the key/value chunk prefixes, which a causal forward leaves for the backward's grad_q
@@ -149,32 +160,30 @@ static int read_states(const Ctx& c, int mode, int n, int per_chunk, const void*
   const int mats = p.bh * (per_chunk ? (n + L - 1) / L : 1);
   if (tc2) {
     // both kinds come out complete: the first-order and constant terms ride along
-    StateCopies cp = copies_at(p, s16, mats);
-    if (ready) {
-      cp = *ready;
-    } else {
-      if (mode == 0) cp.b = nullptr;
-      if (mode == 1) cp.a = nullptr;
-      if ((rc = moments_tc_convert(c, mats, states, cp))) return rc;
-    }
-    if (mode != 1 && (rc = moments_tc_readout_a(c, p.bh, n, L, per_chunk, x, cp.a, stats, states, out_a, den_a)))
-      return rc;
+    const StateCopies cp = ready ? *ready : copies_at(p, mode, s16, out_a, n, mats);
+    if (!ready && (rc = moments_tc_convert(c, mats, states, at_once(cp)))) return rc;
     if (mode != 0 && (rc = moments_tc_readout_b(c, p.bh, n, L, per_chunk, x, ext ? gs : u, ext ? dvec : nullptr, cp.b,
                                                 stats, states, out_b)))
+      return rc;
+    if (!ready && mode == 2 && cp.a == cp.b) {
+      StateCopies then;
+      then.a = cp.a;
+      if ((rc = moments_tc_convert(c, mats, states, then))) return rc;
+    }
+    if (mode != 1 && (rc = moments_tc_readout_a(c, p.bh, n, L, per_chunk, x, cp.a, stats, states, out_a, den_a)))
       return rc;
     return FASTMAX_OK;
   }
   if (tc1) {
     // first-order part on tensor cores; it adds to the second-order part when there is one
-    void* s1b = (char*)s16 + copies_a_bytes(p, mats) + copies_b_bytes(p, mats);
-    if ((rc = first_tc_convert(c, mats, states, s1b))) return rc;
+    if ((rc = first_tc_convert(c, mats, states, s16))) return rc;
     if ((mode == 0 || mode == 2) && !tc2)
-      if ((rc = first_tc_readout(c, 0, p.bh, n, L, per_chunk, x, x, nullptr, states, s1b, stats, out_a, den_a,
+      if ((rc = first_tc_readout(c, 0, p.bh, n, L, per_chunk, x, x, nullptr, states, s16, stats, out_a, den_a,
                                  tc2)))
         return rc;
     if (mode == 1 || mode == 2)
       if ((rc = first_tc_readout(c, 1, p.bh, n, L, per_chunk, ext ? gs : u, x, ext ? dvec : nullptr, states,
-                                 s1b, stats, out_b, nullptr, tc2)))
+                                 s16, stats, out_b, nullptr, tc2)))
         return rc;
     return FASTMAX_OK;
   }
@@ -331,6 +340,29 @@ int moments_forward_total(const Ctx& c, const void* q, const stat_t* stats, cons
 }
 
 // ---- backward ----------------------------------------------------------------------
+// What grad_k and grad_v take from the tokens after a chunk: the states of (q, gradient) become suffix sums (r_base: those
+// of later shards, or null) and are read out in both kinds.  zero_chunk has nothing after it.  Nothing reads r_states after
+// this, so their second-order rows may stay raw (prefix_states).
+static int read_suffix_sums(const Ctx& c, int nchunk, float* r_states, const float* r_base, int zero_chunk, const void* k,
+                            const void* v, const stat_t* stats, void* s16, float* gk_add, float* gv_add) {
+  const fastmax_problem& p = c.p;
+  const StateCopies cp = copies_at(p, 2, s16, gv_add, p.nk, p.bh * nchunk);
+  const Ctx z = zeroing(c, zero_chunk);
+  auto read = [&](int mode, const StateCopies* ready) {
+    return read_states(z, mode, p.nk, 1, k, v, nullptr, nullptr, 0, nullptr, nullptr, r_states, s16, stats, gv_add, nullptr,
+                       gk_add, ready);
+  };
+  bool ready;
+  int rc = prefix_states(c, nchunk, r_states, r_base, 1, true, at_once(cp), &ready);
+  if (rc) return rc;
+  if (!ready) return read(2, nullptr);
+  if (cp.a != cp.b) return read(2, &cp);
+  StateCopies then;
+  then.a = cp.a;
+  if ((rc = read(1, &cp)) || (rc = moments_tc_prefix_convert(c, p.bh, nchunk, r_states, r_base, 1, then))) return rc;
+  return read(0, &cp);
+}
+
 // The part of grad_q that reads the key/value prefixes (everything before a token's own chunk).  It
 // depends on nothing from later shards, so a sequence shard issues it while the query/gradient
 // totals are being exchanged.
@@ -359,12 +391,7 @@ int moments_backward_finish(const Ctx& c, const void* q, const void* k, const vo
       (rc = moments_backward_dq_far(c, q, den, stats, grad_out, delta, dvec, gs, s_states, gq_add, s16)))
     return rc;
   // grad_k and grad_v read the suffix sums of the query/gradient states
-  // (nothing reads r_states after this call, so their second-order rows may stay raw: prefix_states)
-  bool ready;
-  const StateCopies cp = copies_at(p, s16, p.bh * nchunk);
-  if ((rc = prefix_states(c, nchunk, r_states, r_base, 1, true, cp, &ready))) return rc;
-  if ((rc = read_states(zeroing(c, r_base ? -1 : nchunk - 1), 2, p.nk, 1, k, v, nullptr, nullptr, 0, nullptr, nullptr,
-                        r_states, s16, stats, gv_add, nullptr, gk_add, ready ? &cp : nullptr)))
+  if ((rc = read_suffix_sums(c, nchunk, r_states, r_base, r_base ? -1 : nchunk - 1, k, v, stats, s16, gk_add, gv_add)))
     return rc;
   ChunkAdd ca;
   ca.chunk = L;
@@ -440,11 +467,7 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
                           ready ? &kv : nullptr)))
       return rc;
     if ((rc = moments_build_states(skipping(c, 0), p.nq, q, grad_out, den, delta, 1, gs, dvec, states))) return rc;
-    const StateCopies qg = copies_at(p, s16, p.bh * ncq);
-    if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, qg, &ready))) return rc;
-    if ((rc = read_states(zeroing(c, ncq - 1), 2, p.nk, 1, k, v, nullptr, nullptr, 0, nullptr, nullptr, states, s16,
-                          stats, gv_add, nullptr, gk_add, ready ? &qg : nullptr)))
-      return rc;
+    if ((rc = read_suffix_sums(c, ncq, states, nullptr, ncq - 1, k, v, stats, s16, gk_add, gv_add))) return rc;
     ChunkAdd ca;
     ca.chunk = L;
     ca.gq_add = gq_add;

@@ -1,6 +1,7 @@
 """Workspace sizes (host arithmetic, no device).  The operand parts of the float32 score kernels take 6 bytes per element;
 very large problems and the families that name the CUDA cores need none.  The fused first-order path needs room for
-its states and their bf16 copies, and backward for the scaled gradient, but for no fp32 rows."""
+its states and their bf16 copies, and backward for the scaled gradient, but for no fp32 rows.  The second-order moment family
+needs room for its states, result rows and one layout of their bf16 copies."""
 import pytest
 
 from fastmax_b200 import _cabi
@@ -69,3 +70,28 @@ def test_moment_form_forward_only_where_the_terms_hardly_cancel(kw, moment):
     fwd, _ = sizes(**{**dict(bh=heads, bhkv=heads, nq=nq, nk=nk, d=64, mask=0), **kw})
     parts = 6 * 64 * heads * (nq + 2 * nk)
     assert (fwd > parts + 1024) == moment
+
+
+# heads, n, mask, chunk, family (3: moments), bytes of the forward and backward workspace and of the shards' that an earlier
+# layout took: a caller that keeps buffers of those sizes is served
+@pytest.mark.parametrize("heads,n,mask,chunk,impl,most", [
+    (1024, 10000, 1, 0, 0, (12510199808, 19104768000, 5556469760, 12110069760)),
+    (32, 262144, 1, 0, 0, (9168331264, 14570595072, 4496293888, 9865003008)),
+    (64, 6000, 0, 0, 0, (498106368, 745402880, 208367616, 454127616)),
+    (16, 2049, 1, 0, 3, (80937984, 102051328, 26611968, 47593728)),
+    (16, 1, 1, 256, 3, (45265664, 45276416, 9048320, 9058560)),
+    (4, 10000, 1, 256, 3, (286453760, 312214016, 100839680, 126439680)),
+    (4, 300, 0, 256, 3, (18415872, 19188992, 4834048, 5602048)),
+    (3, 2431, 1, 2048, 3, (15474176, 20171264, 5287680, 9955328)),
+    (16, 12001, 1, 1536, 3, (285254144, 408912896, 122276096, 245166336))])
+def test_second_order_moments_need_room_for_one_layout_of_copies(heads, n, mask, chunk, impl, most):
+    prob = _cabi.Problem(dtype=_cabi.BF16, bh=heads, bhkv=heads, nq=n, nk=n, d=64, mask=mask, normalize=1, p=2, impl=impl, a0=1,
+                         a1=1, a2=0.5, lim=1, temperature=1, chunk=chunk)
+    L = _cabi.lib()
+    got = (L.fastmax_b200_forward_workspace_bytes(prob), L.fastmax_b200_backward_workspace_bytes(prob),
+           L.fastmax_b200_shard_forward_workspace_bytes(prob), L.fastmax_b200_shard_backward_workspace_bytes(prob))
+    assert all(g <= m for g, m in zip(got, most)), (got, most)
+    # states of 4161 rows of 68 floats a chunk, a total, rows of 65 floats and copies of 344 064 bytes a state
+    states = heads * -(-n // (chunk or 2048))
+    rows = heads * n * 65 * 4
+    assert got[0] <= states * (4161 * 68 * 4 + 344064) + heads * 4161 * 68 * 4 + rows + 4096
