@@ -347,16 +347,18 @@ int fastmax_b200_profile_get(int i, char* name, int name_len, float* ms) {
 // rebuild from k and v: unmasked, the total key/value state; causal, the exclusive prefixes of the key/value
 // chunk states -- the latter only while they are no larger than twice the tensors autograd holds anyway
 // (q, k, v, out), which is the case for the tensor-core configurations (1.1 MB of state per 2048-token chunk
-// and head at d = 64 against 1 MB of tokens).
+// and head at d = 64 against 1 MB of tokens).  The bf16 copies count with 68 x 64 rows of 64, however they are laid out:
+// what a statistics buffer holds, and with it its size, is not to change with a kernel's layout.
 static size_t stats_words_bytes(const fastmax_problem& p) {
   return align_up(sizeof(stat_t) * (size_t)(p.bh + p.bhkv), 256);
 }
 static size_t kept_bytes(const fastmax_problem& p) {
   if (!p.mask) return moment_total_bytes(p);
-  const size_t states = moment_state_bytes(p, p.nk) + moment_kept16_bytes(p);
+  const size_t states = moment_state_bytes(p, p.nk), copies = moment_kept16_bytes(p);
+  const size_t rows16 = copies ? (size_t)2 * 68 * 64 * 64 * p.bh * ((p.nk + moments_chunk(p) - 1) / moments_chunk(p)) : 0;
   const size_t es = p.dtype == FASTMAX_BF16 ? 2 : 4;
   const size_t held = es * (size_t)p.d * (2 * (size_t)p.bh * p.nq + 2 * (size_t)p.bhkv * p.nk);
-  return states <= 2 * held ? states : 0;
+  return states + rows16 <= 2 * held ? states + copies : 0;
 }
 static bool keeps_total(const fastmax_problem& p, int impl) {
   return impl == FASTMAX_IMPL_MOMENTS && kept_bytes(p) > 0;

@@ -95,3 +95,13 @@ def test_second_order_moments_need_room_for_one_layout_of_copies(heads, n, mask,
     states = heads * -(-n // (chunk or 2048))
     rows = heads * n * 65 * 4
     assert got[0] <= states * (4161 * 68 * 4 + 344064) + heads * 4161 * 68 * 4 + rows + 4096
+
+
+@pytest.mark.parametrize("n,chunk,kept", [(10000, 0, True), (12001, 1536, False), (1649 * 7, 1792, False), (1650 * 7, 1792, True),
+                                          (1500, 1536, False), (1, 256, False)])
+def test_which_states_are_kept_does_not_hang_on_the_layout_of_their_copies(n, chunk, kept):
+    """fp32 states and 68 x 64 rows of 64 bf16 against twice the tensors: from 1650 tokens a chunk on."""
+    heads = 16
+    prob = _cabi.Problem(dtype=_cabi.BF16, bh=heads, bhkv=heads, nq=n, nk=n, d=64, mask=1, normalize=1, p=2, impl=3, a0=1, a1=1,
+                         a2=0.5, lim=1, temperature=1, chunk=chunk)
+    assert (_cabi.lib().fastmax_b200_stats_bytes(prob) > 8 * 2 * heads + 256) == kept
