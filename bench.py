@@ -71,8 +71,6 @@ TRAFFIC_LIB_VERSION = 200
 NCU_BYTES_PER_TOKEN_HEAD = {"fm_dense_tc_fwd": 487.0, "fm_dense_tc_dq": 622.7, "fm_dense_tc_dkdv": 722.1,
                             # per token whose chunk builds a state (profiles/moments_tc_small_case_ncu_full.md)
                             "fm_moments_tc_state": 717.5}
-# Labels that are launches of one kernel function: the roofline record is of the function with the largest share.
-KERNEL_OF_LABEL = {}
 
 
 def cfg_of(name):
@@ -572,30 +570,30 @@ def moment_kernel_flops(name, D, N, mask, chunk):
     return None
 
 
+def score_flops(kind, D, N, mask, chunk):
+    """Products one launch of a score kernel needs, per batch*head unit: q.k and p.v forward; q.k, g.v and e.k for grad_q;
+    q.k, g.v, e.q and p.g for grad_k and grad_v.  Over all pairs of rows that see each other, or (chunk > 0, causal) over those
+    of a chunk, which is what the moment family leaves to these kernels."""
+    L = chunk or max(N, 1)
+    full, rest = divmod(N, L)
+    pairs = full * (L * (L + 1) // 2) + rest * (rest + 1) // 2 if mask else N * N
+    return {"fwd": 4, "dq": 6, "dkdv": 8, "dk": 6, "dv": 4}[kind] * D * pairs
+
+
 def roofline_of(per, cfg, bh, peaks, lib_version, chunk=0):
     """Roofline record of the kernel with the largest share of the timed region."""
     B, H, N, D, dt, mask, p, norm = cfg
     if not per:
         return None
-    share = {}
-    for label, (c_, t_) in per.items():
-        fn = KERNEL_OF_LABEL.get(label, label)
-        share[fn] = share.get(fn, 0.0) + t_
-    dom = max(share, key=share.get)
-    labels = [n for n in per if KERNEL_OF_LABEL.get(n, n) == dom]
-    cnt, tot = sum(per[n][0] for n in labels), sum(per[n][1] for n in labels)
-    ms = tot / cnt
-    mfs = {n: moment_kernel_flops(n, D, N, mask, chunk) for n in labels} if (dt == "bf16" and p == 2) else {}
-    if mfs and all(v is not None for v in mfs.values()):
-        # per launch: the average over this function's launches of the step, of FLOPs and of time alike
-        flops = sum(per[n][0] * mfs[n] for n in labels) * bh / cnt
+    dom = max(per, key=lambda label: per[label][1])
+    ms = per[dom][1] / per[dom][0]
+    flops = moment_kernel_flops(dom, D, N, mask, chunk) if (dt == "bf16" and p == 2) else None
+    if flops is not None:
+        flops *= bh
         achieved = flops / (ms * 1e-3) / 1e12
         traffic = None
-        if all(n in NCU_BYTES_PER_TOKEN_HEAD for n in labels) and D == 64 and lib_version == TRAFFIC_LIB_VERSION:
-            traffic = sum(per[n][0] * NCU_BYTES_PER_TOKEN_HEAD[n] * mfs[n] / moment_kernel_flops(n, D, 1, 0, 1)
-                          for n in labels) * bh / cnt
-        if len(labels) > 1:
-            dom = dom + " (" + ", ".join(sorted(labels)) + ")"
+        if dom in NCU_BYTES_PER_TOKEN_HEAD and D == 64 and lib_version == TRAFFIC_LIB_VERSION:
+            traffic = NCU_BYTES_PER_TOKEN_HEAD[dom] * flops / moment_kernel_flops(dom, D, 1, 0, 1)
         return {"bound": "tensor", "kernel": dom, "achieved": achieved, "peak": peaks["bf16_tflops_sustained"],
                 "unit": "TFLOP/s", "frac": achieved / peaks["bf16_tflops_sustained"], "traffic": traffic,
                 "traffic_source": "ncu dram bytes of a small case scaled by heads x tokens" if traffic else None,
@@ -607,8 +605,14 @@ def roofline_of(per, cfg, bh, peaks, lib_version, chunk=0):
     flops_of = {"fwd": ff, "dq": fq, "dkdv": fkv, "dk": fkv * 2 // 3, "dv": fkv // 3}
     kind = dom.rsplit("_", 1)[-1]
     es = 2 if dt == "bf16" else 4
+    moments = any(n.startswith(("fm_moments", "fm_first")) for n in per)
     if kind in flops_of and (p == 2 or dt != "bf16"):
-        flops = flops_of[kind] * bh * N
+        if moments and mask:
+            flops, note = score_flops(kind, D, N, mask, chunk or 2048) * bh, "products of the chunks' own blocks in score form"
+        else:
+            forms = {"in score form": score_flops(kind, D, N, mask, 0), "factorised": flops_of[kind] * N}
+            form = min(forms, key=forms.get)
+            flops, note = forms[form] * bh, "products of the pass %s, the cheaper one" % form
         achieved = flops / (ms * 1e-3) / 1e12
         if dt == "bf16":
             peak, src, bound = peaks["bf16_tflops_sustained"], peaks["source"] + " (sustained cuBLAS bf16)", "tensor"
@@ -620,13 +624,14 @@ def roofline_of(per, cfg, bh, peaks, lib_version, chunk=0):
         traffic = None
         # the capture is of the wide kernels on whole rows; short rows (at most 1900 columns on average) and the chunks of
         # the moment family run on other kernels under the same labels
-        wide = (N / 2 if mask else N) > 1900 and not any(n.startswith(("fm_moments", "fm_first")) for n in per)
+        wide = (N / 2 if mask else N) > 1900 and not moments
         if dom in NCU_BYTES_PER_TOKEN_HEAD and D == 64 and dt == "bf16" and wide and lib_version == TRAFFIC_LIB_VERSION:
             traffic = NCU_BYTES_PER_TOKEN_HEAD[dom] * bh * N
         return {"bound": bound, "kernel": dom, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": traffic,
                 "traffic_source": "ncu dram bytes of a small case scaled by heads x tokens" if traffic else None,
-                "peak_source": src, "ms_per_launch": ms, "alg_flops_per_launch": flops}
+                "peak_source": src, "ms_per_launch": ms, "alg_flops_per_launch": flops,
+                "note": note}
     nb = 2 * bh * N * D * es     # a streaming kernel of the p = 1 path reads two token tensors once
     achieved = nb / (ms * 1e-3) / 1e9
     return {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
