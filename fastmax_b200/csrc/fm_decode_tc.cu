@@ -162,7 +162,7 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const AppArgs a) {
       for (int h = 0; h < 2; ++h) {
         uint32_t v[16];
         tmem_ld16(tl + hf * 32 + h * 16, v);
-        tmem_wait_ld();
+        tmem_wait_ld(v);
 #pragma unroll
         for (int i = 0; i < 8; ++i) run[8 * h + i] = add2(run[8 * h + i], pack2u(v[2 * i], v[2 * i + 1]));
       }

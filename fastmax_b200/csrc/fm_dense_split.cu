@@ -172,14 +172,14 @@ __device__ __forceinline__ void promote(uint64_t (&run)[D / 4], uint32_t taddr, 
   if constexpr (D == 64) {
     uint32_t a[32];
     tmem_ld32(taddr + cpart * 32, a);
-    tmem_wait_ld();
+    tmem_wait_ld(a);
 #pragma unroll
     for (int e = 0; e < 16; ++e) run[e] = add2(run[e], pack2u(a[2 * e], a[2 * e + 1]));
   } else {
     uint32_t a[16], b[16];
     tmem_ld16(taddr + cpart * 16, a);
     tmem_ld16(taddr + 32 + cpart * 16, b);
-    tmem_wait_ld();
+    tmem_wait_ld(a, b);
 #pragma unroll
     for (int e = 0; e < 8; ++e)
       run[e] = add2(run[e], add2(pack2u(a[2 * e], a[2 * e + 1]), pack2u(b[2 * e], b[2 * e + 1])));
@@ -455,8 +455,12 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       }
       uint32_t sv[32], wv[HAS_U ? 32 : 1];
       tmem_ld32(tl + C::T_S + cpart * 32, sv);
-      if constexpr (HAS_U) tmem_ld32(tl + C::T_W + cpart * 32, wv);
-      tmem_wait_ld();
+      if constexpr (HAS_U) {
+        tmem_ld32(tl + C::T_W + cpart * 32, wv);
+        tmem_wait_ld(sv, wv);
+      } else {
+        tmem_wait_ld(sv);
+      }
       // S and W of this tile are in registers: the next tile's may be issued
       tc_fence_before();
       __syncwarp();

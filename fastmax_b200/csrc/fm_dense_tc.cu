@@ -301,9 +301,13 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         uint32_t sv[BN];
         uint32_t wv[(MODE == OP_B) ? BN : 1];
         tmem_ld64(tg + C::T_S, sv);
-        if constexpr (MODE == OP_A) tmem_ld64(tg + C::T_S + 64, sv + 64);
-        else tmem_ld64(tg + C::T_W, wv);
-        tmem_wait_ld();
+        if constexpr (MODE == OP_A) {
+          tmem_ld64(tg + C::T_S + 64, sv + 64);
+          tmem_wait_ld(sv);
+        } else {
+          tmem_ld64(tg + C::T_W, wv);
+          tmem_wait_ld(sv, wv);
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR_SFREE(g));
@@ -386,7 +390,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         for (int hc = 0; hc < D / 64; ++hc) {      // 64 accumulator columns at a time
           uint32_t ov[64];
           tmem_ld64(tg + C::T_O + hc * 64, ov);
-          tmem_wait_ld();
+          tmem_wait_ld(ov);
           if (row_ok) {
             const size_t orow = (MODE == OP_A && a.fwd_div) ? out_row(head, row, a.nrows, a.o_heads) : grow;
             uint4* dst = (uint4*)((__nv_bfloat16*)a.o + orow * D + hc * 64);

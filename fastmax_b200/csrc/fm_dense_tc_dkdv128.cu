@@ -281,7 +281,7 @@ dkdv128_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         uint32_t sv[32], wv[32];
         tmem_ld32(tl + T_S + cpart * HB + ps * 32, sv);
         tmem_ld32(tl + T_W + cpart * HB + ps * 32, wv);
-        tmem_wait_ld();
+        tmem_wait_ld(sv, wv);
         if (ps + 1 == HB / 32) {
           // S and W of this tile are in registers: the next tile's may be issued
           tc_fence_before();

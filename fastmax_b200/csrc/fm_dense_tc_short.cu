@@ -92,7 +92,7 @@ __device__ __forceinline__ float store_row_vec(uint32_t taddr, bool row_ok, __nv
   for (int c0 = 0; c0 < NC; c0 += 16) {
     uint32_t ov[16];
     tmem_ld16(taddr + c0, ov);
-    tmem_wait_ld();
+    tmem_wait_ld(ov);
     if (row_ok) {
       float f[16];
 #pragma unroll
@@ -324,8 +324,12 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       for (int ps = 0; ps < 2; ++ps) {
         uint32_t sv[16], wv[HAS_U ? 16 : 1];
         tmem_ld16(tl + C::T_S + cpart * 32 + ps * 16, sv);
-        if constexpr (HAS_U) tmem_ld16(tl + C::T_W + cpart * 32 + ps * 16, wv);
-        tmem_wait_ld();
+        if constexpr (HAS_U) {
+          tmem_ld16(tl + C::T_W + cpart * 32 + ps * 16, wv);
+          tmem_wait_ld(sv, wv);
+        } else {
+          tmem_wait_ld(sv);
+        }
         if (!C::INPLACE && ps == 1) {   // S and W of this tile are in registers: the next tile's may be issued
           tc_fence_before();
           __syncwarp();

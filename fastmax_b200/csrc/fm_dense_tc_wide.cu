@@ -430,8 +430,12 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       for (int ps = 0; ps < HB / 32; ++ps) {
         uint32_t sv[32], wv[FWD ? 1 : 32];
         tmem_ld32(TRI ? tset + cpart * HB + ps * 32 : tl + T_S + gp * BN + cpart * HB + ps * 32, sv);
-        if constexpr (!FWD) tmem_ld32(tl + T_W + gp * BN + cpart * HB + ps * 32, wv);
-        tmem_wait_ld();
+        if constexpr (!FWD) {
+          tmem_ld32(tl + T_W + gp * BN + cpart * HB + ps * 32, wv);
+          tmem_wait_ld(sv, wv);
+        } else {
+          tmem_wait_ld(sv);
+        }
         if (!TRI && ps + 1 == HB / 32) {
           // S and W of this tile are in registers: the group's next tile may be issued
           tc_fence_before();

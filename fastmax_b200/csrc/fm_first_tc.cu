@@ -181,7 +181,7 @@ first_state_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constan
       for (int hcol = 0; hcol < DD / 64; ++hcol) {
         uint32_t tv[64];
         tmem_ld64(tmem + ((uint32_t)(qd * 32) << 16) + hcol * 64, tv);
-        tmem_wait_ld();
+        tmem_wait_ld(tv);
 #pragma unroll
         for (int e4 = 0; e4 < 16; ++e4)
           ((float4*)(dst + hcol * 64))[e4] = make_float4(__uint_as_float(tv[4 * e4]), __uint_as_float(tv[4 * e4 + 1]),
@@ -418,7 +418,7 @@ first_readout_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_const
       for (int hcol = 0; hcol < DD / 64; ++hcol) {
         uint32_t tv[64];
         tmem_ld64(tmem + b * DD + ((uint32_t)(qd * 32) << 16) + hcol * 64, tv);
-        tmem_wait_ld();
+        tmem_wait_ld(tv);
         if (hcol + 1 == DD / 64) {   // the accumulator is in registers: the next product may overwrite it
           tc_fence_before();
           __syncwarp();

@@ -321,7 +321,7 @@ state_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__
       uint32_t tv[64];
       if (warp_mine) {
         tmem_ld64(tmem + m * 64 + ((uint32_t)(qd * 32) << 16), tv);
-        tmem_wait_ld();
+        tmem_wait_ld(tv);
       }
       // the pair's row goes to both of its places in the state, (b, other) and (other, b), or to those that are read
       for (int side = 0; mine && side < (o == b ? 1 : 2); ++side) {
@@ -486,7 +486,7 @@ state_ecol_tc_kernel(const __grid_constant__ CUtensorMap tmY, const float* __res
     if (ok && warp < 2) {
       uint32_t tv[64];
       tmem_ld64(tmem + ((uint32_t)(warp * 32) << 16), tv);
-      tmem_wait_ld();
+      tmem_wait_ld(tv);
       // E[a][0..63] as one contiguous row of the scratch block (see the header comment)
       float4* row = (float4*)(state + (size_t)hc * per_state + (size_t)4096 * dvp + (size_t)(warp * 32 + lane) * 64);
 #pragma unroll

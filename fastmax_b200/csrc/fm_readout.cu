@@ -353,13 +353,13 @@ readout_a_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a) {
       full(0);
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        uint32_t tv[32];
+        uint32_t tv[16];
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           uint32_t (&t8)[8] = *(uint32_t(*)[8])(tv + 8 * g);
           tmem_ld8(tb - h * 64 + (2 * (2 * hf + g) + h) * 8, t8);
         }
-        tmem_wait_ld();
+        tmem_wait_ld(tv);
         if (hf == 1) release(0);
 #pragma unroll
         for (int g = 0; g < 2; ++g)
@@ -381,7 +381,7 @@ readout_a_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a) {
       } else {
         uint32_t tv[64];
         tmem_ld64(tb - h * 64 + 128, tv);
-        wait_ld64(tv);
+        tmem_wait_ld(tv);
         release(1);
         uint64_t s4[4] = {0ull, 0ull, 0ull, 0ull};
         float first = 0.f;
@@ -414,7 +414,7 @@ readout_a_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a) {
           tmem_ld64(tb + buf * 128, tv);
           const uint4 xw = lds128(xrow + (((uint32_t)oct << 4) ^ xs));
           const uint32_t ww[4] = {xw.x, xw.y, xw.z, xw.w};
-          wait_ld64(tv);
+          tmem_wait_ld(tv);
           release(buf);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -660,7 +660,7 @@ readout_b_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         tmem_ld64(tb + (st & 1) * 128, tv);
         tmem_ld64(tb + (st & 1) * 128 + 64, tv + 64);
         const uint4 xa0 = words(a0), xb0 = words(b0);
-        wait_ld128(tv);
+        tmem_wait_ld(tv);
         release(st);
         if (n == 5) stage(vecs + (xb ^ 1) * RB_VEC, vnext, qnext, knext, enext);
         block(tv, a0, b0, xa0, xb0);
@@ -672,7 +672,7 @@ readout_b_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         full(st);
         tmem_ld64(tb + (st & 1) * 128, tv);
         tmem_ld64(tb + (st & 1) * 128 + 64, tv + 64);
-        wait_ld128(tv);
+        tmem_wait_ld(tv);
         release(st);
         ++st;
         const float ue = vec[64 + row], c = vec[192], A1 = a.a1 * c, K2 = 2.f * a.a2 * c * c;

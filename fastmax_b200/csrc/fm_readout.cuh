@@ -79,13 +79,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t saddr) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(saddr));
   return r;
 }
-// wait for the loads of tensor memory in flight; the registers they fill pass through, so no use moves ahead of it
-template <int N> __device__ __forceinline__ void pass_through(uint32_t (&r)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
-}
-__device__ __forceinline__ void wait_ld64(uint32_t (&r)[64]) { tmem_wait_ld(); pass_through(r); }
-__device__ __forceinline__ void wait_ld128(uint32_t (&r)[128]) { tmem_wait_ld(); pass_through(r); }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])

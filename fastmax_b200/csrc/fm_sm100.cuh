@@ -122,8 +122,16 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() {
+// Wait for the loads of tensor memory in flight.  It is given the registers that they fill, which pass through it: nothing
+// else keeps the compiler from moving arithmetic on them ahead of the wait.
+template <int N> __device__ __forceinline__ void pass_through(uint32_t (&r)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+template <int... N> __device__ __forceinline__ void tmem_wait_ld(uint32_t (&... r)[N]) {
+  static_assert(sizeof...(N) > 0, "the registers that the loads fill");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  (pass_through(r), ...);
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -510,7 +518,7 @@ __device__ __forceinline__ float store_row(uint32_t taddr, bool row_ok, __nv_bfl
   for (int c0 = 0; c0 < NC; c0 += 32) {
     uint32_t ov[32];
     tmem_ld32(taddr + c0, ov);
-    tmem_wait_ld();
+    tmem_wait_ld(ov);
     if (row_ok) {
 #pragma unroll
       for (int v16 = 0; v16 < 2; ++v16) {

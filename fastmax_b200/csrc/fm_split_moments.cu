@@ -130,7 +130,7 @@ pair_sums_kernel(const __grid_constant__ CUtensorMap tmV, const float* __restric
       for (int h = 0; h < 2; ++h) {
         uint32_t v[16];
         tmem_ld16(tl + hf * 32 + h * 16, v);
-        tmem_wait_ld();
+        tmem_wait_ld(v);
 #pragma unroll
         for (int i = 0; i < 8; ++i) run[8 * h + i] = add2(run[8 * h + i], pack2u(v[2 * i], v[2 * i + 1]));
       }
@@ -471,8 +471,7 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
         const int cc = (2 * i + h) * 8;
         uint32_t t8[8];
         tmem_ld8(tb + cc, t8);
-        tmem_wait_ld();
-        pass_through(t8);
+        tmem_wait_ld(t8);
         if (i == 3) release(0);
 #pragma unroll
         for (int e = 0; e < 8; ++e) t8[e] = __float_as_uint(fmaf(A1, __uint_as_float(t8[e]), a.a0 * vec[cc + e]));
@@ -485,7 +484,7 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
       } else {
         uint32_t tv[64];
         tmem_ld64(tb + 128, tv);
-        wait_ld64(tv);
+        tmem_wait_ld(tv);
         release(1);
         float second[4] = {0.f, 0.f, 0.f, 0.f}, first[2] = {0.f, 0.f};
 #pragma unroll
@@ -516,7 +515,7 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
           tmem_ld64(tb + h * 64 + buf * 128, tv);
           float x[8];
           features(oct, x);
-          wait_ld64(tv);
+          tmem_wait_ld(tv);
           release(buf);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
