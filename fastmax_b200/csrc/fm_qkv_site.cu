@@ -20,8 +20,8 @@
 //   scale_by_noise      y = x * (1 + dropout * noise), the reference's output
 //                       dropout (fastmax_cuda_forward.cu:271-280).
 //
-// All four are HBM-bound copies: 16-byte accesses where the shapes allow (bf16 whose rotated width or head size is only a
-// multiple of 8 falls back to 8-byte accesses, so that a piece never straddles the two halves of the rotation), several
+// All four are HBM-bound copies: 16-byte accesses where the shapes allow (bf16 whose rotated width is an odd multiple
+// of 8 falls back to 8-byte accesses, so that a piece never straddles the two halves of the rotation), several
 // pieces loaded per thread before the first store, grid-stride over a grid sized to the SM count.
 // Measured on B200 in bf16 (B=8, T=4096, H=32, hs=64): split and merge move 806 MB in 0.141 and 0.130 ms (5.7 and
 // 6.2 TB/s; 0.234 and 0.229 ms when a CTA took one token, each piece loaded its partner too and read its table entries
@@ -91,10 +91,11 @@ constexpr int kInFlight = 4;  // vectors a warp loads before it computes and sto
 // With x = (x1, x2) the two halves of the rotated features, cos = (c1, c2), sin = (s1, s2):
 //   y1 = x1 c1 - x2 s1,  y2 = x2 c2 + x1 s2       (model.py:812-825)
 //   gx1 = gy1 c1 + gy2 s2,  gx2 = gy2 c2 - gy1 s1
-// A lane keeps one slot of one token: two pieces of V elements that are rotated with each other, or two pieces that are
-// only copied.  Its table entries stay in registers while the warp walks the vectors (heads) of its tokens, so a vector
-// costs two loads and two stores a lane.  A warp's tokens are neighbours (8 of 64 bf16 features): on the head side it
-// moves a run of 1 KB, and the CTA's warps together take whole tokens of the packed side.
+// A lane keeps one slot of one token: two pieces of V elements that are rotated with each other, or two pieces (of an odd
+// number of them the last slot has one) that are only copied.  Its table entries stay in registers while the warp walks the
+// vectors (heads) of its tokens, so a vector costs two loads and two stores a lane.  A warp's tokens are neighbours (8 of 64
+// bf16 features): on the head side it moves a run of 1 KB, and the CTA's warps together take whole tokens of the packed
+// side.  Vectors of 16 bytes are taken two at a time, side by side, or each would be half a sector of the packed side.
 template <typename T, int V, bool GRAD>
 __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ packed_in, T* __restrict__ packed_out,
                                                           T* __restrict__ q, T* __restrict__ k, T* __restrict__ v,
@@ -102,15 +103,18 @@ __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ 
                                                           const SiteArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int total = a.qper + 2, vecs = a.groups * total;
-  const int slots = a.d / V / 2, width = slots < 32 ? slots : 32, tpw = 32 / width;   // lanes and tokens of a warp
+  const int side = sizeof(T) * a.d < 32 ? 2 : 1;                                      // vectors side by side
+  const int slots = (a.d / V + 1) / 2, width = slots < 32 ? slots : 32, tpw = 32 / (width * side);   // lanes, tokens of a warp
+  const int mine = lane / width % side;
   const int pairs = a.rope / 2 / V, half = a.rope / 2;
   const long long tgroups = (a.n + tpw - 1) / tpw, units = a.batch * tgroups;
   for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
-    const long long b = unit / tgroups, t = (unit - b * tgroups) * tpw + lane / width;
+    const long long b = unit / tgroups, t = (unit - b * tgroups) * tpw + lane / (width * side);
     for (int s0 = 0; s0 < slots; s0 += width) {
       const int slot = s0 + lane % width;
-      const bool ok = t < a.n && lane / width < tpw && slot < slots, rot = ok && slot < pairs;
+      const bool ok = t < a.n && lane / (width * side) < tpw && slot < slots, rot = ok && slot < pairs;
       const int lo = (slot < pairs ? slot : 2 * slot) * V, hi = slot < pairs ? lo + half : lo + V;
+      const bool both = hi < a.d;
       float c1[V], c2[V], s1[V], s2[V];
 #pragma unroll
       for (int e = 0; e < V; e += 4) {
@@ -122,13 +126,13 @@ __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ 
       }
       const long long pbase = (b * a.n + t) * vecs * a.d;
       const int step = 8 * gridDim.y;
-      for (int v0 = warp + 8 * blockIdx.y; v0 < vecs; v0 += kInFlight * step) {
+      for (int v0 = warp + 8 * blockIdx.y; v0 * side < vecs; v0 += kInFlight * step) {
         Pack<T, V> x[kInFlight], y[kInFlight];
         T* dst[kInFlight];
         bool turn[kInFlight];
 #pragma unroll
         for (int u = 0; u < kInFlight; ++u) {
-          const int vec = v0 + u * step;
+          const int vec = (v0 + u * step) * side + mine;
           if (vec >= vecs) continue;
           const int g = vec / total, j = vec - g * total;
           T* hrow = head_row(q, k, v, a, b, t, g, j);
@@ -136,11 +140,12 @@ __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ 
           const T* src = GRAD ? hrow : packed_in + pvec;
           dst[u] = GRAD ? packed_out + pvec : hrow;
           turn[u] = rot && j <= a.qper;
-          if (ok) { x[u].load(src + lo); y[u].load(src + hi); }
+          if (ok) x[u].load(src + lo);
+          if (ok && both) y[u].load(src + hi);
         }
 #pragma unroll
         for (int u = 0; u < kInFlight; ++u) {
-          if (v0 + u * step >= vecs || !ok) continue;
+          if ((v0 + u * step) * side + mine >= vecs || !ok) continue;
           if (turn[u]) {
             float xf[V], yf[V], xo[V], yo[V];
             x[u].get(xf);
@@ -154,7 +159,7 @@ __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ 
             y[u].set(yo);
           }
           x[u].store(dst[u] + lo);
-          y[u].store(dst[u] + hi);
+          if (both) y[u].store(dst[u] + hi);
         }
       }
     }
@@ -274,14 +279,15 @@ int launch_site(const void* packed_in, void* packed_out, void* q, void* k, void*
   }
   SiteArgs a{batch, n, groups, qper, d, rope};
   if (batch * n == 0) return FASTMAX_OK;
-  // 16-byte pieces where a vector has an even number of them and the rotation's halves are whole pieces (bf16: else 8 bytes)
-  const int V = dtype == FASTMAX_F32 ? 4 : (rope % 16 == 0 && d % 16 == 0 ? 8 : 4);
-  const int slots = d / V / 2, tpw = 32 / (slots < 32 ? slots : 32);
+  // 16-byte pieces where the rotation's halves are whole pieces (bf16: else 8 bytes)
+  const int V = dtype == FASTMAX_F32 ? 4 : (rope % 16 == 0 ? 8 : 4);
+  const int side = d * (dtype == FASTMAX_F32 ? 4 : 2) < 32 ? 2 : 1;
+  const int slots = (d / V + 1) / 2, tpw = 32 / ((slots < 32 ? slots : 32) * side);
   const long long units = batch * ((n + tpw - 1) / tpw);
   int blocks;
   if ((rc = grid_for(units * 256, &blocks))) return rc;        // one CTA per group of tokens, grid-stride beyond the cap
   // few tokens: several CTAs share the vectors of a group (a warp keeps at least one)
-  const int vecs8 = (groups * (qper + 2) + 7) / 8;
+  const int vecs8 = (groups * (qper + 2) + 8 * side - 1) / (8 * side);
   int split = (int)(units < 296 ? 296 / units : 1);
   if (split > vecs8) split = vecs8;
   const dim3 grid(blocks, split < 1 ? 1 : split);
