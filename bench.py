@@ -143,8 +143,8 @@ class ClockSampler:
 
 def run_decode(args, world, rank, dev, cfg):
     """One step = one new token for each of the B sequences on every rank (B*H heads, grouped 1:1), added to
-    the per-head moment state and read by its query.  The state (fp32, larger than L2) is read and written once
-    per step: HBM-bound, 2 x state bytes of algorithmic traffic.  Sequences are independent: no collective."""
+    the per-head moment state and read by its query.  The state (fp32, larger than L2) is written once per
+    step and its upper triangle read: HBM-bound.  Sequences are independent: no collective."""
     import torch
     import torch.distributed as dist
 
@@ -204,7 +204,8 @@ def run_decode(args, world, rank, dev, cfg):
         peaks = load_peaks()
         step_ms = sum(t for n, t in recs if n == "fm_decode_step") / max(1, sum(1 for n, _ in recs if n == "fm_decode_step"))
         state_bytes = st.state.numel() * 4
-        ach = 2 * state_bytes / (step_ms * 1e-3) / 1e9
+        moved = decode_step_bytes(D, p) * B * H
+        ach = moved / (step_ms * 1e-3) / 1e9
         nbytes = q.numel() * q.element_size()
         line = {
             "metric": "fastmax_decode_tokens_per_s", "value": B * world * args.steps / (ms * 1e-3), "unit": "tokens/s",
@@ -220,12 +221,23 @@ def run_decode(args, world, rank, dev, cfg):
                     "h2d_bytes_per_step": 3 * nbytes, "d2h_bytes_per_step": nbytes},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": ach / peaks["hbm_gbs"], "traffic": None, "kernel": "fm_decode_step",
-                         "peak_source": peaks["source"]},
+                         "peak_source": peaks["source"], "ms_per_launch": step_ms, "alg_bytes_per_launch": moved,
+                         "note": "state rows that a step reads (of the second order, the tiles of 8 x 8 on and above the "
+                                 "diagonal) and writes (all)"},
         }
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
+
+
+def decode_step_bytes(D, p):
+    """State bytes one decode step moves per key/value head: all rows are written, of the second-order ones only the tiles of
+    8 x 8 features on and above the diagonal are read."""
+    tiles = D // 8
+    read = D + 1 + (tiles * (tiles + 1) // 2 * 64 if p == 2 else 0)
+    written = D + 1 + (D * D if p == 2 else 0)
+    return 4 * (D + 1) * (read + written)
 
 
 def run_site(args, world, rank, dev, cfg):

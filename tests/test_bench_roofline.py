@@ -28,3 +28,8 @@ def test_whole_rows_get_the_cheaper_form():
         cfg = (1, 8, n, 64, "bf16", 1, 2, 1)
         r = bench.roofline_of({"fm_dense_tc_dq": (1, 1.0)}, cfg, 8, PEAKS, 0)
         assert r["alg_flops_per_launch"] == 8 * form
+
+
+def test_decode_step_moves_a_triangle_in_and_a_square_out():
+    assert bench.decode_step_bytes(64, 2) == 4 * 65 * (65 + 36 * 64 + 65 + 4096)
+    assert bench.decode_step_bytes(64, 1) == 4 * 65 * 130
