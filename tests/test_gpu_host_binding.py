@@ -179,3 +179,66 @@ def test_without_the_queries_of_torch_the_python_function_serves(monkeypatch):
     q, k, v, _ = _inputs()
     monkeypatch.setattr(_native, "_queries", None)
     assert torch.equal(fastmax_b200.FASTMultiHeadAttention()(q, k, v, **KW), _python(q, k, v))
+
+
+def test_two_threads_with_streams_of_their_own():
+    import threading
+
+    mod = fastmax_b200.FASTMultiHeadAttention()
+    t = [_inputs(torch.bfloat16, n=300 + 40 * i, d=64) for i in range(2)]
+    want = []
+    for q, k, v, go in t:
+        out = mod(q, k, v, **KW)
+        want.append((out.detach(),) + torch.autograd.grad(out, (q, k, v), go))
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            q, k, v, go = t[i]
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(30):
+                    out = mod(q, k, v, **KW)
+                    got = (out.detach(),) + torch.autograd.grad(out, (q, k, v), go)
+                    torch.cuda.current_stream().synchronize()
+                    # outputs bit for bit; of the gradients, the atomically summed dots may move one row a head
+                    assert torch.equal(got[0], want[i][0]) and torch.equal(got[3], want[i][3])
+                    assert all(torch.allclose(x, y, rtol=0, atol=2e-2) for x, y in zip(got, want[i]))
+        except BaseException as e:          # noqa: BLE001 -- handed to the main thread
+            bad.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    [x.start() for x in threads]
+    [x.join() for x in threads]
+    assert not bad, bad
+
+
+def test_under_graph_capture():
+    """A training step and a decode step captured once and replayed on new inputs."""
+    mod = fastmax_b200.FASTMultiHeadAttention()
+    q, k, v, go = _inputs(torch.bfloat16, n=333, d=64)
+    st = fastmax_b200.FastmaxDecodeState(4, 4, 64, torch.bfloat16, "cuda")
+    row = torch.randn(4, 1, 64, device="cuda").bfloat16()
+
+    def both():
+        out = mod(q, k, v, **KW)
+        return (out.detach(),) + torch.autograd.grad(out, (q, k, v), go) + (st.step(row, row, row),)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        both()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = both()
+    with torch.no_grad():
+        for x in (q, k, v, row):
+            x.copy_(torch.randn_like(x))
+    st.reset()
+    graph.replay()
+    torch.cuda.synchronize()
+    got = [x.clone() for x in got]
+    st.reset()
+    for x, y in zip(got, both()):
+        assert torch.allclose(x, y, rtol=0, atol=2e-2)
