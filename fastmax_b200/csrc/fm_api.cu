@@ -148,12 +148,14 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
     return p.nk > moments_chunk(p) && us_moment < (us_pairs > us_chain ? us_pairs : us_chain);
   }
   const double d = p.d, F = d + (p.p == 2 ? d * d : 0.0);
-  // Constants fitted to this library's kernels on a B200 (bf16, d = 64, p = 2, causal): the score family takes
-  // 5.6 ns per token and head at 10^4 keys; the moment family 4.1 ns for its states and read-outs plus 2.0 ns
-  // for the score kernels of a 2048-token chunk (short rows run at 0.58 of the long-row rate), the former
-  // times the share of chunks that build and read states.  The two families then break even near 9 300 keys,
-  // as measured (score against moment family for the same number of token-heads, 8192 keys: 20.3 / 22.8 ms;
-  // 9216: 22.6 / 23.0; 10000: 60.9 / 54.5).
+  // Rates per token and head (bf16, d = 64, p = 2, causal): the score family 5.6 ns at 10^4 keys; the moment family 4.1 ns for
+  // its states and read-outs plus 2.0 ns for the score kernels of a 2048-token chunk (short rows run at 0.58 of the
+  // long-row rate), the former times the share of chunks that build and read states.  The two then meet at 9 300 keys with any
+  // number of heads.  The states and read-outs have become faster than that (3.7 ns), but where the families meet depends on
+  // the heads, which these rates leave out; the line lies between.  Measured, ms per step, score / moment:
+  //   512 heads: 16.8 / 17.5 at 7500, 20.0 / 18.8 at 8192, 26.1 / 22.0 at 9300, 30.7 / 23.7 at 10 000
+  //   256: 9.74 / 10.0 at 8192, 11.8 / 11.4 at 9150, 14.4 / 13.3 at 10 000; 64: 2.81 / 2.99 at 9150, 3.07 / 2.97 at 9300
+  //   16: 0.72 / 0.95 at 9300, 0.86 / 0.98 at 10 000, 1.09 / 1.09 at 11 500, 1.27 / 1.22 at 12 500
   // float32, second order (fm_dense_split.cu, moment states on the CUDA cores), per token and head and step: the score form
   // takes 4.2 / 5.8 ps per key at d = 32 / 64, the states and read-outs 25 / 190 ns, so the moment family starts near
   // 8 160 unmasked and 13 500 causal keys at d = 32 and beyond 20 000 at d = 64.
@@ -173,7 +175,9 @@ static bool moments_faster(const fastmax_problem& p, bool tc_ok) {
   const double used = p.mask ? 1.0 - 1.0 / (double)((p.nk + L - 1) / L) : 1.0;
   double t_mom = used * 14.0 * F * (d + 1) / rate_state + chunk_keys * per_key / rate_chunk;
   // unmasked: the fp32 result rows take one more pass (5.5 ns per token and head in all), and each head
-  // pays about a third of a chunk's time once, for its totals (break-even measured near 5 500 keys)
+  // pays about a third of a chunk's time once, for its totals.  The line is near 5 400 keys; measured, score / moment:
+  //   512 heads: 8.79 / 9.84 at 4000, 11.7 / 10.8 at 4500, 17.0 / 12.6 at 5500; 256: 5.52 / 5.95 at 4500, 6.93 / 6.23 at 5000
+  //   64: 1.40 / 1.50 at 4500, 1.72 / 1.61 at 5000; 16: 0.55 / 0.62 at 5500, 0.66 / 0.63 at 6000
   if (!p.mask) t_mom *= 1.3 * (1.0 + 0.33 * L / (0.5 * ((double)p.nq + p.nk)));
   return t_mom < t_score && p.nk > moments_chunk(p);
 }
@@ -214,7 +218,7 @@ static bool aligned16(std::initializer_list<const void*> ptrs) {
 
 // bf16 first-order causal problems go to the moment family from some 1000 (d = 64) or 2750 (d = 128) tokens on, where
 // the score form would serve unaligned tensors on the CUDA cores; they go on being served there.  Second-order
-// ones get to the moment family near 9 500 tokens and are refused.
+// ones get to the moment family near 9 300 tokens and are refused.
 static bool first_order_unaligned(const fastmax_problem& p, int impl, std::initializer_list<const void*> ptrs) {
   return p.impl == FASTMAX_IMPL_AUTO && impl == FASTMAX_IMPL_MOMENTS && p.p == 1 && p.mask && dense_tc_supports(p) &&
          !aligned16(ptrs);
@@ -270,7 +274,7 @@ using namespace fm;
 
 extern "C" {
 
-int fastmax_b200_version(void) { return 200; }
+int fastmax_b200_version(void) { return 201; }
 
 const char* fastmax_b200_last_error(void) { return g_err; }
 

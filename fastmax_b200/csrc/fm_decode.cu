@@ -26,9 +26,10 @@
 // Three kernels:
 //   step_kernel    one token and its read-out: bound by the state's traffic with many heads, by a chain of latencies with
 //                  few.  The lower triangle is written but never read: 4 F (d+1) x (1 + 0.56) bytes at d = 64.  Measured, us,
-//                  p = 2: 1024 heads, d = 64, bf16: 350 for 1.73 GB = 4.9 TB/s; 8 key/value heads of 4 query heads 9.3 (11.8
-//                  when the queries were asked for after the update, the arriving CTA fenced its 24 KB of state and the
-//                  last one read the queries' shares in turn); 4 heads, float32: 6.1 (7.0); d = 128, 128 heads: 328 (354).
+//                  events around a launch included, p = 2: 1024 heads, d = 64: 353 for 1.73 GB = 4.9 TB/s in bf16 and float32; 8
+//                  key/value heads of 4 query heads 12.8 (16.8 when the queries were asked for after the update, the
+//                  arriving CTA fenced its 24 KB of state and the last one read the queries' shares in turn); 4 heads, float32,
+//                  10.7 (11.6); 128 heads, d = 128: bf16 336 (353), float32 326 (357).  1024 heads: no change (355).
 //                  Two other arrangements for many heads were slower: several groups of blocks to a CTA 397 us, five CTAs
 //                  to an SM 377.
 //   few_kernel     the same update for a few tokens of a prompt.

@@ -22,9 +22,9 @@ int first_order_chunk(const fastmax_problem& p) {
   return dense_split_supports(p) || (p.d != 32 && p.d != 64) ? 256 : 0;
 }
 
-// Tokens per chunk.  Second order: 2048, measured best for the tensor-core kernels (8.9 ms at 1024, 7.8 at 2048,
-// 8.2 at 4096 per step for 8 heads of 65536 tokens): a chunk's state is as large as its tokens, so fewer, larger
-// chunks mean fewer states to build, scan and convert.  First order, causal: first_order_chunk; unmasked: there is no
+// Tokens per chunk.  Second order: 2048, measured best for the tensor-core kernels (ms per step at 1024 / 1536 / 2048 / 3072 /
+// 4096: 8 heads x 65536 3.63, 3.07, 3.07, 3.36, 3.49; 512 x 10 000 28.3, 24.1, 24.0, 25.9, 26.7): a chunk's state is as large as
+// its tokens, so larger chunks mean fewer states to build, scan and convert, and more in-chunk score work.  First order, causal: first_order_chunk; unmasked: there is no
 // in-chunk part and every chunk only adds a state to sum.
 int moments_chunk(const fastmax_problem& p) {
   int L = p.chunk > 0 ? p.chunk : first_order_chunk(p);

@@ -1,7 +1,9 @@
 // Unmasked second-order forward in float32 on the tensor cores, in moment form (d = 64): the sums over all keys
 //   S2[(a, b)][c] = sum_j k_j[a] k_j[b] (v_j, 1)[c],  S1, S0
 // once per key/value head, then for every query row r = a2 q (x) q . S2 + a1 q . S1 + a0 S0 and out = r[0..63] / r[64].
-// The score form costs 4 n d operations a query, this 4 165 d whatever n is.  Every operand is the exact sum of three bf16
+// The score form costs 4 n d operations a query (a multiply-add counts two); this 2 x 65 for each of 2 560 pairs of features (the
+// blocks of 16 on and below the diagonal) and 65 lower terms, 5 300 d, whatever n is, and for the sums 2 x 65 x 2 145 = 4 400 d a
+// key.  Every operand is the exact sum of three bf16
 // parts (fm_dense_split.cu), every product sum six sums of bf16 products, the small ones first.
 //   pair_sums_kernel   features are formed in fp32 (one rounding), split and put in tensor memory as the A operand, 128
 //                      unordered pairs a tile; B are the value parts.  An accumulator holds 64 tokens and is added to
@@ -10,8 +12,8 @@
 //   copies3_kernel     the type A operand copies (fm_readout.cuh) of the three parts of the sums.
 //   readout3_kernel    the type A read-out with six products to a slice, and the division.  Bound by the products: 504 K
 //                      steps of 128 x 128 x 16 per 128 rows, 32 600 cycles.
-// 64 heads x 10 000: sums 1.32 ms, copies 0.03, read-out 0.90, operand parts 0.12, where the score form takes 7.1 ms; 2-norm
-// error against float64 2.4e-7 (score form 2.6e-7).  The transposed key block written one block ahead: no change.
+// 64 heads x 10 000: sums 1.32 ms, copies 0.03, read-out 0.90, operand parts 0.12, where the score form takes 7.1 ms.  2-norm
+// error against float64 of N(0,1) inputs, normalised, 2.4e-7 (score form 2.6e-7); other inputs at split_moments_faster.  The transposed key block written one block ahead: no change.
 #include "fm_readout.cuh"
 
 namespace fm {

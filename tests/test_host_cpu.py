@@ -48,8 +48,8 @@ def test_version_and_size_queries_need_no_gpu():
 
 def test_family_selection_follows_the_measured_break_even_points():
     """The library's choice of kernel family (host arithmetic, no device): tensor-core score kernels for short
-    rows, the moment family where it was measured faster -- causal bf16 p=2 d=64 from about 9 500 keys on (the
-    headline shape has 10 000), unmasked from about 5 500, p=1 at almost any length -- and never for a few
+    rows, the moment family beyond the rule's lines -- causal bf16 p=2 d=64 from about 9 300 keys on (the
+    headline shape has 10 000), unmasked from about 5 400, p=1 at almost any length -- and never for a few
     query rows against many keys; fp32 stays on the CUDA-core score kernels."""
     def pick(**kw):
         base = dict(dtype=_cabi.BF16, bh=1024, bhkv=1024, nq=10000, nk=10000, d=64, mask=1, normalize=1, p=2,
