@@ -70,6 +70,11 @@ __device__ __forceinline__ float pow2_of(float s) {
   const uint32_t e = __float_as_uint(s) & 0x7F800000u;
   return e == 0u || e == 0x7F800000u ? 1.f : __uint_as_float(e);
 }
+// s / pow2_of(s), exactly
+__device__ __forceinline__ float beyond_pow2(float s) {
+  const uint32_t e = __float_as_uint(s) & 0x7F800000u;
+  return e == 0u || e == 0x7F800000u ? s : __uint_as_float((__float_as_uint(s) & 0x807FFFFFu) | 0x3F800000u);
+}
 
 // Order of the row tiles in a score kernel's grid.  Long grids go head by head, so that a head's column tiles stay in
 // L2.  A causal grid of a few waves goes tile by tile over all heads (`by_tile` = number of row heads): the longest row

@@ -619,6 +619,8 @@ __global__ void __launch_bounds__(256) split3_kernel(const SplitJobs jobs) {
   const int part = (int)(idx % TPR);
   if (row - (size_t)(threadIdx.x & 31) / TPR >= jb.rows) return;      // whole warps leave together
   const bool ok = row < jb.rows;
+  // (rows stay below 2^32: their parts take at most 48 GiB)
+  const stat_t st = jb.stat && ok ? __ldg((const unsigned long long*)jb.stat + (unsigned)row / (unsigned)jb.n) : 0;
   float f[8];
   if (ok) {
     const float4 u = __ldg((const float4*)(jb.src + row * D + part * 8)), w = __ldg((const float4*)(jb.src + row * D + part * 8) + 1);
@@ -644,7 +646,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const SplitJobs jobs) {
   }
   if (!ok) return;
   if (jb.stat) {
-    const float s = pow2_of(stat_scale(jb.stat, (int)(row / jb.n), jb.lim));
+    const float s = pow2_of(stat_scale(&st, 0, jb.lim));
 #pragma unroll
     for (int e = 0; e < 8; ++e) f[e] *= s;
   }

@@ -431,8 +431,9 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
     auto first_rows = [&](const Walk& w) { return a.state + (size_t)(w.head / ratio) * a.per_state + (size_t)(64 * 64) * a.dvp; };
     auto const_of = [&](const Walk& w) { return w.more() && row <= 64 ? __ldg(first_rows(w) + (size_t)64 * a.dvp + row) : 0.f; };
     auto norm_of = [&](const Walk& w) { return w.more() && h && row < 64 ? __ldg(first_rows(w) + (size_t)row * a.dvp + 64) : 0.f; };
-    auto q_of = [&](const Walk& w) { return w.more() ? a.stat_q[w.head] : (stat_t)0; };
-    auto k_of = [&](const Walk& w) { return w.more() ? a.stat_k[w.head / ratio] : (stat_t)0; };
+    // (past the end the last head's words again: without a branch the loop keeps 16 bytes in local memory instead of 132, 1.5 %)
+    auto q_of = [&](const Walk& w) { return a.stat_q[min(w.head, a.heads - 1)]; };
+    auto k_of = [&](const Walk& w) { return a.stat_k[min(w.head, a.heads - 1) / ratio]; };
     Walk w(a);
     float s0next = const_of(w), n1next = norm_of(w);
     stat_t qnext = q_of(w), knext = k_of(w);
@@ -449,8 +450,7 @@ readout3_kernel(const __grid_constant__ CUtensorMap tmX, const RdArgs a, const i
     };
     for (; w.more(); ++k) {
       // what pow2_of has left of the scales of the queries and of the keys
-      const float sq = stat_scale(&qnext, 0, a.lim), sk = stat_scale(&knext, 0, a.lim);
-      const float c = (sq / pow2_of(sq)) * (sk / pow2_of(sk));
+      const float c = beyond_pow2(stat_scale(&qnext, 0, a.lim)) * beyond_pow2(stat_scale(&knext, 0, a.lim));
       const float A1 = a.a1 * c, A2 = a.a2 * c * c;
       const int tok = w.tok0(a) + t * 128 + row;
       const bool tok_ok = tok < a.n;
