@@ -84,6 +84,12 @@ __device__ __forceinline__ T* head_row(T* q, T* k, T* v, const SiteArgs& a, long
   return base + ((b * a.groups + g) * a.n + t) * a.d;
 }
 
+// Vectors that a warp takes side by side: two where a vector is three pieces or less, or its run of the packed side is a
+// part of a sector or a single one.  us, split / merge of 403 MB in bf16 (float32: 805), one / two: d = 8 248 / 525 -> 210 / 189,
+// 16 191 / 228 -> 158 / 158, 24 174 / 224 -> 184 / 181, float32 8 386 / 467 -> 289 / 291; vectors of four pieces: d = 32 145 / 141
+// -> 157 / 150, float32 16 266 / 264 -> 283 / 267.
+__host__ __device__ constexpr int side_by_side(int pieces) { return pieces <= 3 ? 2 : 1; }
+
 constexpr int kInFlight = 4;  // vectors a warp loads before it computes and stores
 
 // GRAD = false: per-head arrays <- packed projection, rotation R(t).
@@ -95,15 +101,16 @@ constexpr int kInFlight = 4;  // vectors a warp loads before it computes and sto
 // number of them the last slot has one) that are only copied.  Its table entries stay in registers while the warp walks the
 // vectors (heads) of its tokens, so a vector costs two loads and two stores a lane.  A warp's tokens are neighbours (8 of 64
 // bf16 features): on the head side it moves a run of 1 KB, and the CTA's warps together take whole tokens of the packed
-// side.  Vectors of 16 bytes are taken two at a time, side by side, or each would be half a sector of the packed side.
-template <typename T, int V, bool GRAD>
+// side.
+// ODD: vectors of an odd number of pieces, or taken two side by side (d = 64 takes 2 us of 147 less without the tests for them).
+template <typename T, int V, bool GRAD, bool ODD>
 __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ packed_in, T* __restrict__ packed_out,
                                                           T* __restrict__ q, T* __restrict__ k, T* __restrict__ v,
                                                           const float* __restrict__ cs, const float* __restrict__ sn,
                                                           const SiteArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int total = a.qper + 2, vecs = a.groups * total;
-  const int side = sizeof(T) * a.d < 32 ? 2 : 1;                                      // vectors side by side
+  const int side = ODD ? side_by_side(a.d / V) : 1;
   const int slots = (a.d / V + 1) / 2, width = slots < 32 ? slots : 32, tpw = 32 / (width * side);   // lanes, tokens of a warp
   const int mine = lane / width % side;
   const int pairs = a.rope / 2 / V, half = a.rope / 2;
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(256, 2) qkv_site_kernel(const T* __restrict__ 
       const int slot = s0 + lane % width;
       const bool ok = t < a.n && lane / (width * side) < tpw && slot < slots, rot = ok && slot < pairs;
       const int lo = (slot < pairs ? slot : 2 * slot) * V, hi = slot < pairs ? lo + half : lo + V;
-      const bool both = hi < a.d;
+      const bool both = !ODD || hi < a.d;
       float c1[V], c2[V], s1[V], s2[V];
 #pragma unroll
       for (int e = 0; e < V; e += 4) {
@@ -281,7 +288,8 @@ int launch_site(const void* packed_in, void* packed_out, void* q, void* k, void*
   if (batch * n == 0) return FASTMAX_OK;
   // 16-byte pieces where the rotation's halves are whole pieces (bf16: else 8 bytes)
   const int V = dtype == FASTMAX_F32 ? 4 : (rope % 16 == 0 ? 8 : 4);
-  const int side = d * (dtype == FASTMAX_F32 ? 4 : 2) < 32 ? 2 : 1;
+  const int side = side_by_side(d / V);
+  const bool odd = side == 2 || d / V % 2;
   const int slots = (d / V + 1) / 2, tpw = 32 / ((slots < 32 ? slots : 32) * side);
   const long long units = batch * ((n + tpw - 1) / tpw);
   int blocks;
@@ -293,14 +301,23 @@ int launch_site(const void* packed_in, void* packed_out, void* q, void* k, void*
   const dim3 grid(blocks, split < 1 ? 1 : split);
   const char* name = GRAD ? "fm_qkv_merge_rope_grad" : "fm_qkv_split_rope";
   typedef __nv_bfloat16 bf;
-  if (dtype == FASTMAX_F32)
-    FM_LAUNCH(name, st, (qkv_site_kernel<float, 4, GRAD><<<grid, 256, 0, st>>>(
+  if (dtype == FASTMAX_F32 && odd)
+    FM_LAUNCH(name, st, (qkv_site_kernel<float, 4, GRAD, true><<<grid, 256, 0, st>>>(
                             (const float*)packed_in, (float*)packed_out, (float*)q, (float*)k, (float*)v, cs, sn, a)));
+  else if (dtype == FASTMAX_F32)
+    FM_LAUNCH(name, st, (qkv_site_kernel<float, 4, GRAD, false><<<grid, 256, 0, st>>>(
+                            (const float*)packed_in, (float*)packed_out, (float*)q, (float*)k, (float*)v, cs, sn, a)));
+  else if (V == 8 && !odd)
+    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 8, GRAD, false><<<grid, 256, 0, st>>>(
+                            (const bf*)packed_in, (bf*)packed_out, (bf*)q, (bf*)k, (bf*)v, cs, sn, a)));
   else if (V == 8)
-    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 8, GRAD><<<grid, 256, 0, st>>>(
+    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 8, GRAD, true><<<grid, 256, 0, st>>>(
+                            (const bf*)packed_in, (bf*)packed_out, (bf*)q, (bf*)k, (bf*)v, cs, sn, a)));
+  else if (!odd)
+    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 4, GRAD, false><<<grid, 256, 0, st>>>(
                             (const bf*)packed_in, (bf*)packed_out, (bf*)q, (bf*)k, (bf*)v, cs, sn, a)));
   else
-    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 4, GRAD><<<grid, 256, 0, st>>>(
+    FM_LAUNCH(name, st, (qkv_site_kernel<bf, 4, GRAD, true><<<grid, 256, 0, st>>>(
                             (const bf*)packed_in, (bf*)packed_out, (bf*)q, (bf*)k, (bf*)v, cs, sn, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;

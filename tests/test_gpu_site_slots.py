@@ -14,7 +14,7 @@ SHAPES = [(2, 9, 2, 1, 24, 8), (1, 7, 3, 3, 40, 24), (1, 8, 1, 1, 544, 544), (2,
           (3, 17, 40, 8, 64, 48), (1, 3, 300, 100, 16, 16), (1, 1001, 2, 1, 128, 64), (2, 5, 2, 2, 8, 8),
           # odd numbers of 16-byte pieces in bf16, one slot more than a warp among them; vectors taken in pairs, an odd number of them
           (1, 13, 2, 1, 24, 16), (3, 70, 4, 2, 72, 16), (2, 33, 3, 3, 88, 64), (1, 5, 1, 1, 520, 16), (1, 37, 5, 5, 8, 8),
-          (2, 300, 3, 1, 8, 8)]
+          (2, 300, 3, 1, 8, 8), (2, 70, 3, 1, 16, 16)]
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["fp32", "bf16"])
