@@ -300,6 +300,9 @@ int first_tc_readout(const Ctx& c, int type_b, int heads, int n, int chunk, int 
                      const void* x, const float* uvec, const float* state, const void* s1b,
                      const stat_t* stats, float* o_add, float* den_add, int accumulate, int final = 0,
                      void* out_final = nullptr, float* den_final = nullptr, float* dots = nullptr);
+int first_tc_total(const Ctx& c, int nchunk, const float* states, float* total, void* s1b);
+int first_tc_grad(const Ctx& c, const void* q, const void* out, const float* den, const void* grad_out, const float* total,
+                  const void* s1b, const stat_t* stats, void* grad_q, float* dots, float* states, int* nruns);
 int first_tc_status(int* out, cudaStream_t stream);
 int first_tc_status_reset(cudaStream_t stream);
 // host orchestration of the moment family (fm_moments.cu)

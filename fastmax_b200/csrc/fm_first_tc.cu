@@ -29,6 +29,18 @@ using namespace sm100;
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_ftc_status, 0, code); }
 
+// 16 bytes from shared memory by shared-window address (keeps the epilogue's vector reads off the generic path)
+__device__ __forceinline__ uint4 lds128u(uint32_t saddr) {
+  uint4 r;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(saddr));
+  return r;
+}
+__device__ __forceinline__ float4 lds128f(uint32_t saddr) {
+  float4 r;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(saddr));
+  return r;
+}
+
 constexpr int F1_THREADS = 192;  // warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: vector sums, epilogue
 
 // =====================================================================================
@@ -227,18 +239,6 @@ struct F1ReadArgs {
   int wide_io;          // out_final / o_add / x are 32-byte aligned: 32-byte accesses in the epilogue
   int zero_chunk;       // per-chunk mode: the tokens of this chunk read an empty state (-1: none)
 };
-
-// 16 bytes from shared memory by shared-window address (keeps the epilogue's vector reads off the generic path)
-__device__ __forceinline__ uint4 lds128u(uint32_t saddr) {
-  uint4 r;
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(saddr));
-  return r;
-}
-__device__ __forceinline__ float4 lds128f(uint32_t saddr) {
-  float4 r;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(saddr));
-  return r;
-}
 
 template <int DD>
 struct F1R {
@@ -506,6 +506,432 @@ __global__ void __launch_bounds__(256) s1_to_bf16_kernel(const float* __restrict
   for (int i = threadIdx.x; i < d * d; i += 256) dst[i] = __float2bfloat16_rn(scale * src[(size_t)(i / d) * dvp + i % d]);
 }
 
+// =====================================================================================
+// unmasked backward of p = 1: grad_q and the states of (q, gs | e) from one read of the query side
+// =====================================================================================
+// What the three passes before it did -- gs = grad_out / den and dvec (fm_gprep), grad_q (read-out type B) and the
+// states (first_state_kernel) -- moved q, grad_out and out once each, gs three times and grad_q once: seven tensors.
+// Here a tile of gs exists in shared memory only, four tensors move.
+//
+//   per 128-token tile   gs = grad_out / den, rounded to bf16, written over the tile TMA delivered; dvec = gs . out
+//                        T = gs S1^T                 grad_q_i[a] = A1 (T_i[a] - dvec_i S1[a][D])
+//                        Q1 += q^T gs                the state's first-order rows; its vectors on the CUDA cores
+//                        grad_q takes the place of gs and leaves by TMA
+//
+// Bound by HBM.  Persistent CTAs, one per SM, walk runs of tiles (one state each), so the loads of the next run's tiles
+// are under way while a run's state is written: warp 0 TMA loads, warp 1 MMA issuer, warp 2 TMA stores, warps 4-19
+// everything else (eight of them spent 7 300 cycles on a tile of d = 128, which HBM delivers in 5 600: 1 026 us for 256 heads
+// x 16384, 780 with sixteen -- 5.5 TB/s; the three passes before took 1 341).  Rows are walked
+// 16 bytes a thread, a row's pieces side by side, so that reads of out coalesce and a thread keeps the sums over its eight
+// features in registers.  TMEM: two accumulators for T, two for Q1.
+struct F1GradArgs {
+  const __nv_bfloat16* out;   // (heads, n, D)
+  const float* den;           // (heads, n)
+  const float* total;         // (heads, rows, dvp): key/value totals
+  float* states;              // (heads, runs, rows, dvp): states of the runs of (q, gs | -dvec)
+  float* dots;                // per head: sum of grad_q . q is added, or null
+  const stat_t* stat_q;
+  const stat_t* stat_k;
+  float a1, lim;
+  int heads, n, dvp, rows, f_lin;
+  int run, runs;              // tiles per run, runs per head
+};
+
+constexpr int FG_THREADS = 640, FG_FIRST = 4, FG_WARPS = 16;   // the first warp of those and their number
+
+template <int DD>
+struct F1G {
+  static constexpr int NSUB = DD / 64;
+  static constexpr int TILE = NSUB * 16384;        // 128 tokens x DD bf16
+  static constexpr int STAGE = 2 * TILE;           // q, then grad_out / gs / grad_q
+  static constexpr int NS = DD == 128 ? 2 : 4;     // 128 KB of tiles
+  static constexpr bool AHEAD = NS > 2;            // gs of the next tile before grad_q of this one
+  static constexpr int SMAT = DD * DD * 2;
+  static constexpr int OFF_S = NS * STAGE;         // bf16 copies of S1 of this run's head and the next one's
+  static constexpr int OFF_NCOL = OFF_S + 2 * SMAT;         // float S1[a][D] of the same
+  static constexpr int OFF_E = OFF_NCOL + 2 * DD * 4;       // float e[NS][128]
+  static constexpr int VROW = 2 * DD + 4;          // a warp's sums: q e [DD], gs [DD], e
+  static constexpr int OFF_VEC = OFF_E + NS * 512;
+  static constexpr int OFF_BAR = OFF_VEC + FG_WARPS * VROW * 4;
+  static constexpr int NBAR = 4 * NS + 8;          // full, gs, grad_q, empty per stage; T, state, S full, S empty twice
+  static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
+  static constexpr int SMEM = OFF_TMEM + 16 + 1024;
+};
+
+// The tiles a CTA walks: runs blockIdx.x, blockIdx.x + gridDim.x, ... of all heads, tile by tile.
+struct F1Walk {
+  int g = 0, m = 0;          // tiles and runs before this one
+  int item, head, first, t, nt;
+  const F1GradArgs& a;
+  __device__ __forceinline__ F1Walk(const F1GradArgs& args) : item((int)blockIdx.x), a(args) { open(); }
+  __device__ __forceinline__ void open() {
+    t = 0;
+    head = item / a.runs;
+    first = (item % a.runs) * a.run;
+    nt = min(a.run, (a.n + 127) / 128 - first);
+  }
+  __device__ __forceinline__ bool live() const { return item < a.heads * a.runs; }
+  __device__ __forceinline__ bool last() const { return t + 1 == nt; }
+  __device__ __forceinline__ int token() const { return (first + t) * 128; }
+  __device__ __forceinline__ void next() {
+    ++g;
+    if (++t == nt) {
+      ++m;
+      item += (int)gridDim.x;
+      open();
+    }
+  }
+};
+
+template <int DD>
+__global__ void __launch_bounds__(FG_THREADS, 1)
+first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
+                  const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmO, const F1GradArgs a) {
+  using C = F1G<DD>;
+  constexpr int NS = C::NS;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t bar0 = sbase + C::OFF_BAR;
+  auto BAR_FULL = [&](int s) { return bar0 + 8u * s; };
+  auto BAR_GS = [&](int s) { return bar0 + 8u * (NS + s); };
+  auto BAR_DQ = [&](int s) { return bar0 + 8u * (2 * NS + s); };
+  auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (3 * NS + s); };
+  auto BAR_T = [&](int b) { return bar0 + 8u * (4 * NS + b); };
+  auto BAR_STATE = [&](int b) { return bar0 + 8u * (4 * NS + 2 + b); };
+  auto BAR_SF = [&](int b) { return bar0 + 8u * (4 * NS + 4 + b); };
+  auto BAR_SE = [&](int b) { return bar0 + 8u * (4 * NS + 6 + b); };
+  volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_TMEM);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(BAR_FULL(s), 1);
+      mbar_init(BAR_GS(s), FG_WARPS);
+      mbar_init(BAR_DQ(s), FG_WARPS);
+      mbar_init(BAR_EMPTY(s), 1);                  // grad_q has left it
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(BAR_T(b), 1);
+      mbar_init(BAR_STATE(b), 1);
+      mbar_init(BAR_SF(b), 1);
+      mbar_init(BAR_SE(b), 1);
+    }
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), 4 * DD);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  F1Walk w(a);
+  if (warp == 0) {
+    // ================= TMA producer =================
+    for (; w.live(); w.next()) {
+      const int s = w.g % NS;
+      if (w.t == 0) {
+        if (!mbar_wait(BAR_SE(w.m & 1), (uint32_t)(((w.m >> 1) & 1) ^ 1))) { report(50); break; }
+        if (lane == 0) {
+          mbar_expect_tx(BAR_SF(w.m & 1), C::SMAT);
+          for (int sub = 0; sub < C::NSUB; ++sub)
+            tma_load_3d(sbase + C::OFF_S + (w.m & 1) * C::SMAT + sub * (DD * 128), &tmS, BAR_SF(w.m & 1), sub * 64, 0, w.head);
+        }
+      }
+      if (!mbar_wait(BAR_EMPTY(s), (uint32_t)(((w.g / NS) & 1) ^ 1))) { report(51); break; }
+      if (lane == 0) {
+        mbar_expect_tx(BAR_FULL(s), C::STAGE);
+        const uint32_t dst = sbase + s * C::STAGE;
+        for (int sub = 0; sub < C::NSUB; ++sub) {
+          tma_load_3d(dst + C::TILE + sub * 16384, &tmG, BAR_FULL(s), sub * 64, w.token(), w.head);
+          tma_load_3d(dst + sub * 16384, &tmQ, BAR_FULL(s), sub * 64, w.token(), w.head);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ================= MMA issuer (whole warp, one elected lane issues) =================
+    for (; w.live(); w.next()) {
+      const int s = w.g % NS, mb = w.m & 1;
+      const uint32_t ph = (uint32_t)((w.g / NS) & 1);
+      if (w.t == 0 && !mbar_wait_warp(BAR_SF(mb), (uint32_t)((w.m >> 1) & 1))) { report(52); break; }
+      // whoever forms gs has waited for the tile, and has read the accumulators that are overwritten here: T of two tiles
+      // ago before this gs, the state of two runs ago before the run's first gs
+      if (!mbar_wait_warp(BAR_FULL(s), ph) || !mbar_wait_warp(BAR_GS(s), ph)) { report(53); break; }
+      tc_fence_after();
+      const uint32_t q_s = sbase + s * C::STAGE, g_s = q_s + C::TILE;
+      if (elect_one()) {
+        // T[i][a] = sum_c gs_i[c] S1[a][c]: S1's rows a are K-major
+        const uint32_t g_lo = desc_lo(g_s, 16), s_lo = desc_lo(sbase + C::OFF_S + mb * C::SMAT, 16);
+#pragma unroll
+        for (int sub = 0; sub < C::NSUB; ++sub)
+          umma_ss_k64(tmem + (w.g & 1) * DD, g_lo + sub * (16384 >> 4), s_lo + sub * ((DD * 128) >> 4),
+                      idesc_bf16(128, DD, 0, 0), sub > 0);
+        // M = 128 feature rows; with D = 64 the second 64 are those of the tile that follows q, never read back
+        umma_ss_mn_steps<8>(tmem + 2 * DD + mb * DD, desc_lo(q_s, 16384), desc_lo(g_s, 16384), idesc_bf16(128, DD, 1, 1),
+                            w.t > 0 ? 1u : 0u);
+        umma_commit(BAR_T(w.g & 1));       // of both products: grad_q is written over gs
+        if (w.last()) {
+          umma_commit(BAR_STATE(mb));
+          umma_commit(BAR_SE(mb));
+        }
+      }
+      __syncwarp();
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // ================= TMA stores of grad_q: rows past the end are left out =================
+    for (; w.live(); w.next()) {
+      const int s = w.g % NS;
+      if (!mbar_wait(BAR_DQ(s), (uint32_t)((w.g / NS) & 1))) { report(58); break; }
+      if (lane == 0) {
+        for (int sub = 0; sub < C::NSUB; ++sub)
+          tma_store_3d(&tmO, sbase + s * C::STAGE + C::TILE + sub * 16384, sub * 64, w.token(), w.head);
+        tma_store_wait_read();
+        mbar_arrive(BAR_EMPTY(s));
+      }
+      __syncwarp();
+    }
+    if (lane == 0) tma_store_wait_all();
+    __syncwarp();
+  } else if (warp >= FG_FIRST) {
+    constexpr int LPR = DD / 8, RPS = 32 * FG_WARPS / LPR, STEPS = 128 / RPS;   // 16-byte pieces of a row; rows per step
+    const int te = tid - 32 * FG_FIRST, sub_r = te / LPR, piece = te % LPR;
+    const uint32_t at0 = (uint32_t)((piece >> 3) * 16384 + sub_r * 128 + (((piece & 7) ^ (sub_r & 7)) << 4));   // in a tile
+    const int qd = warp & 3, cols = (warp - FG_FIRST) >> 2;   // TMEM lane quarter; quarter of the features
+    constexpr int HC = DD / 4;
+    static_assert(RPS % 8 == 0 && STEPS <= LPR, "a thread's rows have one swizzle; a row's threads hold the rows' den");
+    auto sync = []() { asm volatile("bar.sync 2, %0;" ::"n"(32 * FG_WARPS) : "memory"); };
+    // its eight features summed over its rows: q e, gs; e
+    uint64_t sq[4] = {0, 0, 0, 0}, sg[4] = {0, 0, 0, 0};
+    float se = 0.f;
+    uint4 o[STEPS];
+    float den = 1.f;          // of this thread's row `piece`, if it has so many
+    // out and den of a tile, asked for a tile ahead
+    auto fetch = [&](const F1Walk& p) {
+      const int tok = p.token() + sub_r;
+      const size_t row = (size_t)p.head * a.n + tok;
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st)
+        o[st] = p.live() && tok + st * RPS < a.n ? __ldg((const uint4*)(a.out + (row + st * RPS) * DD) + piece)
+                                                 : make_uint4(0u, 0u, 0u, 0u);
+      den = p.live() && piece < STEPS && tok + piece * RPS < a.n ? __ldg(a.den + row + piece * RPS) : 1.f;
+    };
+    auto sts128 = [](uint32_t at, const uint32_t (&v)[4]) {
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+    };
+    // grad_out -> gs in place, e = -dvec (as fm_gprep: dvec from the rounded values, so that both cancel alike)
+    auto form = [&](const F1Walk& p) -> bool {
+      const int s = p.g % NS;
+      if (p.t == 0) {          // the run's normaliser column, once nobody reads that of two runs ago
+        sync();
+        const float* src = a.total + (size_t)p.head * a.rows * a.dvp + (size_t)a.f_lin * a.dvp + DD;
+        if (te < DD) ((float*)(smem + C::OFF_NCOL))[(p.m & 1) * DD + te] = __ldg(src + (size_t)te * a.dvp);
+        sync();
+      }
+      if (!mbar_wait(BAR_FULL(s), (uint32_t)((p.g / NS) & 1))) { report(54); return false; }
+      const uint32_t qt = sbase + s * C::STAGE + at0, gt = qt + C::TILE;
+      const float inv_own = 1.0f / den;
+      float e[STEPS];
+      uint32_t g[STEPS][4];
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) {
+        const uint4 v = lds128u(gt + st * (RPS * 128));
+        g[st][0] = v.x; g[st][1] = v.y; g[st][2] = v.z; g[st][3] = v.w;
+      }
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) {
+        const uint32_t ow[4] = {o[st].x, o[st].y, o[st].z, o[st].w};
+        const float inv = __shfl_sync(0xffffffffu, inv_own, (lane & ~(LPR - 1)) | st);     // (past the end grad_out is 0)
+        const uint64_t inv2 = pack2(inv, inv);
+        uint64_t sum = 0ull;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          g[st][x] = pack_bf16_2(mul2(pack2u(g[st][x] << 16, g[st][x] & 0xFFFF0000u), inv2));
+          const uint64_t gf = pack2u(g[st][x] << 16, g[st][x] & 0xFFFF0000u);
+          sum = fma2(gf, pack2u(ow[x] << 16, ow[x] & 0xFFFF0000u), sum);
+          sg[x] = add2(sg[x], gf);
+        }
+        float lo, hi;
+        unpack2(sum, lo, hi);
+        e[st] = -(lo + hi);
+      }
+#pragma unroll
+      for (int k = LPR / 2; k >= 1; k >>= 1)
+#pragma unroll
+        for (int st = 0; st < STEPS; ++st) e[st] += __shfl_xor_sync(0xffffffffu, e[st], k);
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) {
+        sts128(gt + st * (RPS * 128), g[st]);
+        if (piece == 0) ((float*)(smem + C::OFF_E))[s * 128 + st * RPS + sub_r] = e[st];
+      }
+      fence_proxy_async();
+      // (also orders this warp's earlier reads of the accumulators before the products that overwrite them)
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_GS(s));
+      uint4 qv[STEPS];
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) qv[st] = lds128u(qt + st * (RPS * 128));
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) {
+        const uint32_t qw[4] = {qv[st].x, qv[st].y, qv[st].z, qv[st].w};
+        const uint64_t e2 = pack2(e[st], e[st]);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) sq[x] = fma2(pack2u(qw[x] << 16, qw[x] & 0xFFFF0000u), e2, sq[x]);
+        se += e[st];
+      }
+      return true;
+    };
+    // a run's vectors: column D and the constant row of its state
+    auto write_vectors = [&](const F1Walk& p) {
+      float* const mine = (float*)(smem + C::OFF_VEC) + (warp - FG_FIRST) * C::VROW;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        float f[4];
+        unpack2(sq[x], f[0], f[1]);
+        unpack2(sg[x], f[2], f[3]);
+#pragma unroll
+        for (int k = LPR; k < 32; k <<= 1)          // the warp's other rows of the same features
+#pragma unroll
+          for (int y = 0; y < 4; ++y) f[y] += __shfl_xor_sync(0xffffffffu, f[y], k);
+        if (lane < LPR) {
+          *(float2*)(mine + piece * 8 + 2 * x) = make_float2(f[0], f[1]);
+          *(float2*)(mine + DD + piece * 8 + 2 * x) = make_float2(f[2], f[3]);
+        }
+        sq[x] = sg[x] = 0ull;
+      }
+#pragma unroll
+      for (int k = LPR; k < 32; k <<= 1) se += __shfl_xor_sync(0xffffffffu, se, k);
+      if (lane == 0) mine[2 * DD] = se;
+      se = 0.f;
+      sync();
+      auto total = [&](int i) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < FG_WARPS; ++k) v += ((const float*)(smem + C::OFF_VEC))[k * C::VROW + i];
+        return v;
+      };
+      float* st = a.states + (size_t)p.item * a.rows * a.dvp + (size_t)a.f_lin * a.dvp;
+      if (te < DD) {
+        st[(size_t)te * a.dvp + DD] = total(te);
+        for (int x = DD + 1; x < a.dvp; ++x) st[(size_t)te * a.dvp + x] = 0.f;
+      }
+      for (int x = te; x < a.dvp; x += 32 * FG_WARPS) st[(size_t)DD * a.dvp + x] = x < DD ? total(DD + x) : (x == DD ? total(2 * DD) : 0.f);
+      sync();
+    };
+    float part = 0.f;
+    F1Walk f(a);
+    bool ok = true;
+    auto form_next = [&]() {
+      ok = form(f);
+      if (ok && f.last()) write_vectors(f);
+      f.next();
+      fetch(f);
+    };
+    fetch(f);
+    if (C::AHEAD && f.live()) form_next();
+    for (; ok && w.live(); w.next()) {
+      if (f.live()) form_next();
+      if (!ok) break;
+      const int s = w.g % NS;
+      // (the tile's e come from all the warps that form gs)
+      if (!mbar_wait(BAR_GS(s), (uint32_t)((w.g / NS) & 1)) || !mbar_wait(BAR_T(w.g & 1), (uint32_t)((w.g >> 1) & 1))) {
+        report(55);
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const float c = stat_scale(a.stat_q, w.head, a.lim) * stat_scale(a.stat_k, w.head, a.lim), A1 = a.a1 * c;
+      const int r = qd * 32 + lane;
+      const bool in = w.token() + r < a.n;
+      const float e = ((const float*)(smem + C::OFF_E))[s * 128 + r];
+      const int col = cols * HC;
+      uint32_t tv[HC];
+      const uint32_t t_at = tmem + ((uint32_t)(qd * 32) << 16) + (w.g & 1) * DD + col;
+      if constexpr (HC == 32) tmem_ld32(t_at, tv);
+      else tmem_ld16(t_at, tv);
+      const uint32_t nc = sbase + C::OFF_NCOL + ((w.m & 1) * DD + col) * 4;
+      const uint32_t qrow = sbase + s * C::STAGE + (col >> 6) * 16384 + r * 128, grow = qrow + C::TILE;
+      tmem_wait_ld(tv);
+#pragma unroll
+      for (int b = 0; b < HC / 8; ++b) {
+        const uint32_t pc = (((col & 63) / 8 + b) ^ (r & 7)) << 4;      // 16-byte piece of the row, swizzled
+        const float4 n0 = lds128f(nc + 32 * b), n1 = lds128f(nc + 32 * b + 16);
+        const float cv[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+        float v[8];
+        uint32_t ww[4];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) v[x] = A1 * fmaf(e, cv[x], __uint_as_float(tv[8 * b + x]));
+#pragma unroll
+        for (int x = 0; x < 4; ++x) ww[x] = pack_bf16(v[2 * x], v[2 * x + 1]);
+        sts128(grow + pc, ww);
+        if (a.dots && in) {
+          const uint4 xv = lds128u(qrow + pc);
+          const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            part = fmaf(v[2 * x], __uint_as_float(xw[x] << 16), part);
+            part = fmaf(v[2 * x + 1], __uint_as_float(xw[x] & 0xFFFF0000u), part);
+          }
+        }
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_DQ(s));
+      if (w.last()) {
+        if (a.dots) {
+#pragma unroll
+          for (int k = 16; k >= 1; k >>= 1) part += __shfl_xor_sync(0xffffffffu, part, k);
+          if (lane == 0) atomicAdd(a.dots + w.head, part);
+          part = 0.f;
+        }
+        if (!mbar_wait(BAR_STATE(w.m & 1), (uint32_t)((w.m >> 1) & 1))) { report(56); ok = false; break; }
+        tc_fence_after();
+        if (qd * 32 < DD) {
+          float* dst = a.states + (size_t)w.item * a.rows * a.dvp + (size_t)(a.f_lin + r) * a.dvp + col;
+          uint32_t sv[HC];
+          const uint32_t at = tmem + ((uint32_t)(qd * 32) << 16) + 2 * DD + (w.m & 1) * DD + col;
+          if constexpr (HC == 32) tmem_ld32(at, sv);
+          else tmem_ld16(at, sv);
+          tmem_wait_ld(sv);
+#pragma unroll
+          for (int x = 0; x < HC / 4; ++x)
+            ((float4*)dst)[x] = make_float4(__uint_as_float(sv[4 * x]), __uint_as_float(sv[4 * x + 1]),
+                                            __uint_as_float(sv[4 * x + 2]), __uint_as_float(sv[4 * x + 3]));
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 4 * DD);
+  }
+}
+
+// Sum of a head's chunk states (the first-order rows, all there are when p = 1) and its bf16 first-order block.
+// total: where the sum goes, or null.  Four elements a thread, eight chunks in flight.
+__global__ void __launch_bounds__(256) first_total_kernel(const float* __restrict__ states, int nchunk, int per, int d, int dvp,
+                                                          float* __restrict__ total, __nv_bfloat16* __restrict__ s1b) {
+  const int e = (blockIdx.x * 256 + threadIdx.x) * 4, head = blockIdx.y;
+  if (e >= per) return;
+  const float* src = states + (size_t)head * nchunk * per + e;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i0 = 0; i0 < nchunk; i0 += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      v[u] = i0 + u < nchunk ? __ldcs((const float4*)(src + (size_t)(i0 + u) * per)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) { sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w; }
+  }
+  if (total) *(float4*)(total + (size_t)head * per + e) = sum;
+  const int row = e / dvp, col = e % dvp;
+  if (row < d && col < d)
+    *(uint2*)(s1b + ((size_t)head * d + row) * d + col) = make_uint2(pack_bf16(sum.x, sum.y), pack_bf16(sum.z, sum.w));
+}
+
 }  // namespace
 
 // ---- host side ---------------------------------------------------------------------------
@@ -555,6 +981,71 @@ int first_tc_chunk_state(const Ctx& c, int heads, int n, int chunk, const void* 
   } else {
     FM_CUDA_TRY(cudaFuncSetAttribute(first_state_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, F1S<64>::SMEM));
     FM_LAUNCH("fm_first_tc_state", c.stream, (first_state_kernel<64><<<grid, F1_THREADS, F1S<64>::SMEM, c.stream>>>(ty, tz, a)));
+  }
+  FM_CUDA_TRY(cudaGetLastError());
+  return FASTMAX_OK;
+}
+
+// Totals of a head's chunk states and their bf16 copies (p = 1: the states are the first-order rows).
+int first_tc_total(const Ctx& c, int nchunk, const float* states, float* total, void* s1b) {
+  const fastmax_problem& p = c.p;
+  if (p.bh == 0) return FASTMAX_OK;
+  const MomentDims m = moment_dims(p.d, p.p);
+  const int per = m.f * m.dvp;
+  dim3 grid((unsigned)((per + 1023) / 1024), p.bh);
+  FM_LAUNCH("fm_first_total", c.stream,
+            (first_total_kernel<<<grid, 256, 0, c.stream>>>(states, nchunk, per, p.d, m.dvp, total, (__nv_bfloat16*)s1b)));
+  FM_CUDA_TRY(cudaGetLastError());
+  return FASTMAX_OK;
+}
+
+// Tokens of a run of first_grad_kernel.  A run leaves a state behind (d = 128: 68 KB against 96 KB that a tile moves), and
+// the CTAs, one per SM, each take the same number of runs but for one: the length with the least of both is taken.  At
+// 512 tokens and more the states fit the room of gs (2 d bytes a token: 128 KB a run at d = 128) and one state more.
+static int grad_run(const fastmax_problem& p) {
+  int best = 0;
+  double least = 0;
+  for (int run = 512; run <= 8192; run *= 2) {
+    const double t = (double)(((size_t)p.bh * ((p.nq + run - 1) / run) + 147) / 148) * ((run < p.nq ? run : p.nq) + 160);
+    if (!best || t < least) {
+      best = run;
+      least = t;
+    }
+  }
+  return best;
+}
+
+// Unmasked p = 1: grad_q from the key/value totals (and their bf16 copies), and the states of runs of (q, grad_out/den |
+// -dvec) -- *nruns per head, at `states`, which has room for a state a head and 2 d bytes for every query row.
+int first_tc_grad(const Ctx& c, const void* q, const void* out, const float* den, const void* grad_out, const float* total,
+                  const void* s1b, const stat_t* stats, void* grad_q, float* dots, float* states, int* nruns) {
+  const fastmax_problem& p = c.p;
+  const MomentDims m = moment_dims(p.d, p.p);
+  if ((((uintptr_t)grad_out | (uintptr_t)out) & 15) != 0)
+    return fail(FASTMAX_E_ARG, "the tensor-core family needs 16-byte aligned tensors");
+  CUtensorMap tq, tg, ts, to;
+  int rc;
+  if ((rc = tma_map_bf16(&tq, q, p.bh, p.nq, p.d, 128))) return rc;
+  if ((rc = tma_map_bf16(&tg, grad_out, p.bh, p.nq, p.d, 128))) return rc;
+  if ((rc = tma_map_bf16(&ts, s1b, p.bh, p.d, p.d, p.d))) return rc;
+  if ((rc = tma_map_bf16(&to, grad_q, p.bh, p.nq, p.d, 128))) return rc;
+  F1GradArgs a;
+  a.out = (const __nv_bfloat16*)out; a.den = den; a.total = total; a.states = states; a.dots = dots;
+  a.stat_q = p.normalize ? stats : nullptr;
+  a.stat_k = p.normalize ? stats + p.bh : nullptr;
+  a.a1 = p.a1; a.lim = p.lim;
+  a.heads = p.bh; a.n = p.nq; a.dvp = m.dvp; a.rows = m.f; a.f_lin = p.d * p.d - m.f0;
+  a.run = grad_run(p) / 128;
+  a.runs = ((p.nq + 127) / 128 + a.run - 1) / a.run;
+  *nruns = a.runs;
+  const size_t items = (size_t)p.bh * a.runs;
+  const unsigned grid = (unsigned)(items < 148 ? items : 148);
+  if (p.d == 128) {
+    FM_CUDA_TRY(cudaFuncSetAttribute(first_grad_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, F1G<128>::SMEM));
+    FM_LAUNCH("fm_first_tc_grad", c.stream, (first_grad_kernel<128><<<grid, FG_THREADS, F1G<128>::SMEM, c.stream>>>(tq, tg, ts, to, a)));
+  } else {
+    FM_CUDA_TRY(cudaFuncSetAttribute(first_grad_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, F1G<64>::SMEM));
+    FM_LAUNCH("fm_first_tc_grad", c.stream, (first_grad_kernel<64><<<grid, FG_THREADS, F1G<64>::SMEM, c.stream>>>(tq, tg, ts, to, a)));
   }
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;

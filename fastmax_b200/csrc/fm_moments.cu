@@ -199,15 +199,25 @@ static int read_states(const Ctx& c, int mode, int n, int per_chunk, const void*
 }
 
 // p = 1 on tensor cores without a score-form part: the read-out of the total state is the
-// result, so it is divided / rounded in the read-out kernel itself
+// result, so it is divided / rounded in the read-out kernel itself; s16: the bf16 copies of the totals (first_tc_total)
 static bool first_is_whole(const fastmax_problem& p) { return p.p == 1 && !p.mask && first_tc_supports(p); }
 static int read_first_final(const Ctx& c, int type_b, int n, const void* tile, const void* x, const float* uvec,
-                            const float* total, void* s16, const stat_t* stats, int final, void* out,
+                            const float* total, const void* s16, const stat_t* stats, int final, void* out,
                             float* den_out, float* dots) {
-  int rc;
-  if ((rc = first_tc_convert(c, c.p.bh, total, s16))) return rc;
   return first_tc_readout(c, type_b, c.p.bh, n, moments_chunk(c.p), 0, tile, x, uvec, total, s16, stats, nullptr,
                           nullptr, 0, final, out, den_out, dots);
+}
+
+// grad_k and grad_v from the query/gradient totals
+static int read_first_dkdv(const Ctx& c, const void* k, const void* v, const float* total, const void* s16, const stat_t* stats,
+                           float* dots, void* grad_k, void* grad_v) {
+  int rc;
+  if ((rc = read_first_final(c, 1, c.p.nk, v, k, nullptr, total, s16, stats, 2, grad_k, nullptr, dots))) return rc;
+  return read_first_final(c, 0, c.p.nk, k, k, nullptr, total, s16, stats, 2, grad_v, nullptr, nullptr);
+}
+static int plain_layout(const fastmax_problem& p, const FwdOut& o) {
+  if (!o.out_f32 && o.o_stride == p.d) return FASTMAX_OK;
+  return fail(FASTMAX_E_UNSUPPORTED, "the moment family writes the plain output layout only");
 }
 
 // Exclusive running sums over the chunks of every head (per-chunk mode).  With `fuse` and the tensor-core second-order
@@ -296,6 +306,10 @@ int moments_forward(const Ctx& c, const void* q, const void* k, const void* v, c
   }
   // unmasked: every query reads the total of all keys
   const int nchunk = (p.nk + L - 1) / L;
+  if (first_is_whole(p)) {
+    if ((rc = plain_layout(p, o)) || (rc = first_tc_total(c, nchunk, states, total, s16))) return rc;
+    return read_first_final(c, 0, p.nq, q, q, nullptr, total, s16, stats, 1, o.out, o.den, nullptr);
+  }
   if ((rc = moments_prefix(c, p.bh, nchunk, states, nullptr, total, 0, 0))) return rc;
   return moments_forward_total(c, q, stats, total, o_add, den_add, s16, o);
 }
@@ -329,10 +343,11 @@ int moments_forward_total(const Ctx& c, const void* q, const stat_t* stats, cons
                           float* den_add, void* s16, const FwdOut& o) {
   const fastmax_problem& p = c.p;
   int rc;
-  if (o.out_f32 || o.o_stride != p.d)
-    return fail(FASTMAX_E_UNSUPPORTED, "the moment family writes the plain output layout only");
-  if (first_is_whole(p))
+  if ((rc = plain_layout(p, o))) return rc;
+  if (first_is_whole(p)) {
+    if ((rc = first_tc_total(c, 1, total, nullptr, s16))) return rc;
     return read_first_final(c, 0, p.nq, q, q, nullptr, total, s16, stats, 1, o.out, o.den, nullptr);
+  }
   if ((rc = read_states(c, 0, p.nq, 0, q, nullptr, nullptr, nullptr, 0, nullptr, nullptr, total, s16, stats,
                         o_add, den_add, nullptr)))
     return rc;
@@ -430,7 +445,9 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
   // all read gs / dvec and the pass over grad_out and out is skipped
   const bool all_tc = moments_all_tc(p);
   if (!all_tc && (rc = launch_delta(c, grad_out, out, delta))) return rc;
-  if (tc && (rc = launch_gprep(c, grad_out, out, den, gs, dvec))) return rc;
+  // unmasked p = 1: no score kernel reads gs, and the kernel of grad_q forms it itself
+  const bool whole = first_is_whole(p) && p.nq > 0;
+  if (tc && !whole && (rc = launch_gprep(c, grad_out, out, den, gs, dvec))) return rc;
   const int nck = (p.nk + L - 1) / L, ncq = (p.nq + L - 1) / L;
   if (p.mask) {
     // the key/value prefixes are rebuilt (the forward does not keep them), used for grad_q,
@@ -485,6 +502,18 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
       if ((rc = moments_build_states(c, p.nk, k, v, nullptr, nullptr, 0, nullptr, nullptr, states))) return rc;
       if ((rc = moments_prefix(c, p.bh, nck, states, nullptr, total, 0, 0))) return rc;
     }
+    if (whole) {
+      // one kernel reads the query side; the room for gs and the states behind it take those it leaves, s16 the copies of
+      // either total
+      const float* kv = kv_total_kept ? kv_total_kept : total;
+      int nruns;
+      if ((rc = first_tc_total(c, 1, kv, nullptr, s16))) return rc;
+      if ((rc = first_tc_grad(c, q, out, den, grad_out, kv, s16, stats, grad_q, p.normalize ? dots : nullptr, (float*)gs, &nruns)))
+        return rc;
+      if ((rc = first_tc_total(c, nruns, (const float*)gs, total, s16))) return rc;
+      if ((rc = read_first_dkdv(c, k, v, total, s16, stats, p.normalize ? dots + p.bh : nullptr, grad_k, grad_v))) return rc;
+      return p.normalize ? launch_norm_fixup(c, q, k, stats, dots, grad_q, grad_k) : FASTMAX_OK;
+    }
     if ((rc = moments_backward_total(c, q, k, v, den, stats, grad_out, delta, dvec, gs,
                                      kv_total_kept ? kv_total_kept : total, nullptr, gq_add,
                                      gk_add, gv_add, s16, dots, grad_q, nullptr, nullptr)))
@@ -511,6 +540,7 @@ int moments_backward_total(const Ctx& c, const void* q, const void* k, const voi
   int rc;
   if (kv_total && grad_q) {
     if (first_is_whole(p)) {
+      if ((rc = first_tc_total(c, 1, kv_total, nullptr, s16))) return rc;
       if ((rc = read_first_final(c, 1, p.nq, gs, q, dvec, kv_total, s16, stats, 2, grad_q, nullptr,
                                  p.normalize ? dots : nullptr)))
         return rc;
@@ -525,11 +555,8 @@ int moments_backward_total(const Ctx& c, const void* q, const void* k, const voi
   }
   if (qg_total && grad_k) {
     if (first_is_whole(p)) {
-      if ((rc = read_first_final(c, 1, p.nk, v, k, nullptr, qg_total, s16, stats, 2, grad_k, nullptr,
-                                 p.normalize ? dots + p.bh : nullptr)))
-        return rc;
-      if ((rc = read_first_final(c, 0, p.nk, k, k, nullptr, qg_total, s16, stats, 2, grad_v, nullptr, nullptr)))
-        return rc;
+      if ((rc = first_tc_total(c, 1, qg_total, nullptr, s16))) return rc;
+      if ((rc = read_first_dkdv(c, k, v, qg_total, s16, stats, p.normalize ? dots + p.bh : nullptr, grad_k, grad_v))) return rc;
     } else {
       if ((rc = read_states(c, 2, p.nk, 0, k, v, nullptr, nullptr, 0, nullptr, nullptr, qg_total, s16, stats,
                             gv_add, nullptr, gk_add)))

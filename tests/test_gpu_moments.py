@@ -57,6 +57,26 @@ def test_unmasked_moments_with_more_keys_than_queries():
     assert_close(got, ref, torch.float32, "unmasked nq != nk")
 
 
+@pytest.mark.parametrize("bh,nq,nk,d,normalize", [(1, 1, 300, 64, 1), (3, 127, 127, 128, 1), (2, 128, 300, 64, 0),
+                                                  (1, 513, 513, 128, 0), (150, 640, 129, 64, 1), (2, 2049, 2049, 128, 1),
+                                                  (80, 1300, 1300, 128, 0), (3, 4300, 4300, 64, 1)])
+def test_unmasked_first_order_gradients_at_run_edges(bh, nq, nk, d, normalize):
+    """grad_q and the query/gradient states come from one walk over runs of 128-token tiles."""
+    q, go = randn(1, bh, nq, d, seed=nq), randn(1, bh, nq, d, seed=nq + 1)
+    k, v = randn(1, bh, nk, d, seed=nk + 2), randn(1, bh, nk, d, seed=nk + 3)
+    if not normalize:
+        q, k = q * d ** -0.5, k * d ** -0.5
+    kw = dict(mask=0, normalize=normalize, p=1, a0=1.0, a1=0.9, a2=0.5, lim=1.0)
+    _cabi.profile(True)
+    got, _ = run_cabi(q, k, v, go, torch.bfloat16, impl="moments", **kw)
+    names = [n for n, _ in _cabi.profile_records()]
+    _cabi.profile(False)
+    assert "fm_first_tc_grad" in names and _cabi.device_status() == 0
+    # (relative to the gradients, small as they are at these lengths)
+    assert_close(got, oracle(q, k, v, go, torch.bfloat16, dense=True, **kw), torch.bfloat16, "first-order gradients",
+                 floor=1e-9)
+
+
 @pytest.mark.parametrize("dtype,d,normalize", [(torch.float32, 32, True), (torch.bfloat16, 64, True),
                                                (torch.float32, 16, False)])
 def test_shard_stage_calls_reproduce_the_unsharded_result(dtype, d, normalize):
