@@ -66,8 +66,9 @@ struct F1S {
   static constexpr int SUBTILE = TOK * 128;       // TOK tokens x 64 bf16
   static constexpr int TILE = NSUB * SUBTILE;     // one operand tile: TOK tokens x DD bf16
   static constexpr int STAGE = 2 * TILE;          // Y then Z
-  static constexpr int OFF_VEC = NS * STAGE;      // float sv[DD], se[DD], s_e, pad, e[128]
-  static constexpr int OFF_BAR = OFF_VEC + (2 * DD + 4 + 128) * 4;
+  static constexpr int VROW = 2 * DD + 4;         // a warp's sums: z [DD], y e [DD], e
+  static constexpr int OFF_VEC = NS * STAGE;
+  static constexpr int OFF_BAR = OFF_VEC + 4 * VROW * 4;
   static constexpr int NBAR = 2 * NS + 1;
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_TMEM + 16 + 1024;
@@ -86,7 +87,6 @@ first_state_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constan
   auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (C::NS + s); };
   auto BAR_DONE = [&]() { return bar0 + 8u * (2 * C::NS); };
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_TMEM);
-  float* vsum = (float*)(smem + C::OFF_VEC);      // [0,DD): sum z, [DD,2DD): sum y e, [2DD]: sum e
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hc = blockIdx.x, head = hc / a.nchunk, chunk = hc % a.nchunk;
@@ -97,11 +97,10 @@ first_state_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constan
 
   if (tid == 0) {
     // a stage is free when the MMAs that read it are done and the vector sums have read it
-    for (int s = 0; s < C::NS; ++s) { mbar_init(BAR_FULL(s), 1); mbar_init(BAR_EMPTY(s), 2); }
+    for (int s = 0; s < C::NS; ++s) { mbar_init(BAR_FULL(s), 1); mbar_init(BAR_EMPTY(s), 1 + 4); }
     mbar_init(BAR_DONE(), 1);
     mbar_fence_init();
   }
-  for (int i = tid; i < 2 * DD + 4; i += F1_THREADS) vsum[i] = 0.f;
   if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), 128);
   tc_fence_before();
   __syncthreads();
@@ -142,45 +141,72 @@ first_state_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constan
     __syncwarp();
   } else {
     // ---- vector sums over the chunk's tokens, read from the tiles TMA delivered ----
-    // element (row r, column c) of a 64-column sub-tile sits at r*128 + (((c>>3) ^ (r&7))<<4) + (c&7)*2
+    // 16 bytes a thread, a row's pieces side by side: element (row r, column c) of a 64-column sub-tile sits at
+    // r*128 + (((c>>3) ^ (r&7))<<4) + (c&7)*2.  (A pair of columns a thread through the generic path, the sums of threads
+    // added by atomics, bound the kernel: 404 us for 256 heads x 16384 x 128 and 76 for 256 x 4096 x 64; 356 and 63 now.)
     const int t = tid - 64;                       // 0..127
-    constexpr int HP = DD / 2;                    // bf16 pairs per row
-    constexpr int NPART = 128 / HP;               // threads per column pair, interleaved over rows
-    const int cp = t % HP, part = t / HP;
-    const int sub = (2 * cp) >> 6, cc = (2 * cp) & 63;
+    constexpr int LPR = DD / 8, RPS = 128 / LPR, STEPS = TOK / RPS;
+    static_assert(RPS % 8 == 0, "a thread's rows have one swizzle");
+    const int sub_r = t / LPR, piece = t % LPR;
+    const uint32_t at0 = sbase + (uint32_t)((piece >> 3) * C::SUBTILE + sub_r * 128 + (((piece & 7) ^ (sub_r & 7)) << 4));
     const float* dv = a.dvec ? a.dvec + (size_t)head * a.n : nullptr;
-    float* ebuf = vsum + 2 * DD + 4;
-    float2 sz = make_float2(0.f, 0.f), sye = sz;
-    float se = 0.f;
+    uint64_t sz[4] = {0, 0, 0, 0}, sye[4] = {0, 0, 0, 0};
+    float se = 0.f, ev[STEPS];
+    auto fetch = [&](int k) {                     // e of this thread's rows of tile k, asked for a tile ahead
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) {
+        const int tok = t_begin + k * TOK + st * RPS + sub_r;
+        ev[st] = tok < t_end ? (dv ? -__ldg(dv + tok) : 1.f) : 0.f;
+      }
+    };
+    fetch(0);
     bool ok = true;
     for (int k = 0; k < nblk; ++k) {
       const int s = k % C::NS;
-      const int tok0 = t_begin + k * TOK;
-      if (t < TOK) ebuf[t] = (tok0 + t < t_end) ? (dv ? -__ldg(dv + tok0 + t) : 1.f) : 0.f;
+      float e[STEPS];
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) e[st] = ev[st];
+      fetch(k + 1);
       if (!mbar_wait(BAR_FULL(s), (uint32_t)((k / C::NS) & 1))) { report(46); ok = false; break; }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      const uint8_t* yt = smem + s * C::STAGE + sub * C::SUBTILE;
-      const uint8_t* zt = yt + C::TILE;
-#pragma unroll 4
-      for (int r = part; r < TOK; r += NPART) {
-        const uint32_t off = r * 128 + ((((uint32_t)cc >> 3) ^ (r & 7)) << 4) + (cc & 7) * 2;
-        const float e = ebuf[r];                  // 0 for rows past the end of the chunk
-        const float2 zv = __bfloat1622float2(*(const __nv_bfloat162*)(zt + off));
-        const float2 yv = __bfloat1622float2(*(const __nv_bfloat162*)(yt + off));
-        if (tok0 + r < t_end) { sz.x += zv.x; sz.y += zv.y; }
-        sye.x = fmaf(yv.x, e, sye.x); sye.y = fmaf(yv.y, e, sye.y);
-        se += e;
+      const uint32_t yt = at0 + s * C::STAGE, zt = yt + C::TILE;
+#pragma unroll
+      for (int st = 0; st < STEPS; ++st) {        // (rows past the end of the sequence hold zeros)
+        const uint4 yv = lds128u(yt + st * (RPS * 128)), zv = lds128u(zt + st * (RPS * 128));
+        const uint32_t yw[4] = {yv.x, yv.y, yv.z, yv.w}, zw[4] = {zv.x, zv.y, zv.z, zv.w};
+        const uint64_t e2 = pack2(e[st], e[st]);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          sz[x] = add2(sz[x], pack2u(zw[x] << 16, zw[x] & 0xFFFF0000u));
+          sye[x] = fma2(pack2u(yw[x] << 16, yw[x] & 0xFFFF0000u), e2, sye[x]);
+        }
+        se += e[st];
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (t == 0) mbar_arrive(BAR_EMPTY(s));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_EMPTY(s));
     }
-    atomicAdd(&vsum[2 * cp], sz.x);
-    atomicAdd(&vsum[2 * cp + 1], sz.y);
-    atomicAdd(&vsum[DD + 2 * cp], sye.x);
-    atomicAdd(&vsum[DD + 2 * cp + 1], sye.y);
-    if (cp == 0) atomicAdd(&vsum[2 * DD], se);
+    // the rows of a warp, then (in the epilogue) the warps, in a fixed order
+    float* const sums = (float*)(smem + C::OFF_VEC);
+    float* const mine = sums + (warp - 2) * C::VROW;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      float f[4];
+      unpack2(sz[x], f[0], f[1]);
+      unpack2(sye[x], f[2], f[3]);
+#pragma unroll
+      for (int k = LPR; k < 32; k <<= 1)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) f[y] += __shfl_xor_sync(0xffffffffu, f[y], k);
+      if (lane < LPR) {
+        *(float2*)(mine + piece * 8 + 2 * x) = make_float2(f[0], f[1]);
+        *(float2*)(mine + DD + piece * 8 + 2 * x) = make_float2(f[2], f[3]);
+      }
+    }
+#pragma unroll
+    for (int k = LPR; k < 32; k <<= 1) se += __shfl_xor_sync(0xffffffffu, se, k);
+    if (lane == 0) mine[2 * DD] = se;
     // named barrier among the four epilogue warps only
     asm volatile("bar.sync 1, 128;" ::: "memory");
+    auto vsum = [&](int i) { return (sums[i] + sums[C::VROW + i]) + (sums[2 * C::VROW + i] + sums[3 * C::VROW + i]); };
     // ---- epilogue ----
     if (ok && !mbar_wait(BAR_DONE(), 0)) { report(43); ok = false; }
     tc_fence_after();
@@ -199,12 +225,12 @@ first_state_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constan
           ((float4*)(dst + hcol * 64))[e4] = make_float4(__uint_as_float(tv[4 * e4]), __uint_as_float(tv[4 * e4 + 1]),
                                                          __uint_as_float(tv[4 * e4 + 2]), __uint_as_float(tv[4 * e4 + 3]));
       }
-      dst[DD] = vsum[DD + arow];
+      dst[DD] = vsum(DD + arow);
       for (int cc = DD + 1; cc < a.dvp; ++cc) dst[cc] = 0.f;
     }
     // constant row: [sum z | sum e | 0]
     float* crow = st + (size_t)(a.f_lin + DD) * a.dvp;
-    for (int cc = t; cc < a.dvp; cc += 128) crow[cc] = (cc < DD) ? vsum[cc] : (cc == DD ? vsum[2 * DD] : 0.f);
+    for (int cc = t; cc < a.dvp; cc += 128) crow[cc] = (cc < DD) ? vsum(cc) : (cc == DD ? vsum(2 * DD) : 0.f);
   }
   tc_fence_before();
   __syncthreads();
