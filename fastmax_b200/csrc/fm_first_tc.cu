@@ -1114,17 +1114,19 @@ int first_tc_readout(const Ctx& c, int type_b, int heads, int n, int chunk, int 
   a.final = final; a.out_final = out_final; a.den_final = den_final; a.dots = dots;
   a.wide_io = (((uintptr_t)out_final | (uintptr_t)o_add | (uintptr_t)x) & 31) == 0;
   a.zero_chunk = (per_chunk && !final) ? c.zero_chunk : -1;
-  // runs of up to 8 tiles that never cross a chunk (chunks are multiples of 256 tokens)
-  // a CTA pays for loading the state copy and the vector terms once per run, so runs are as long as
-  // the chunk allows (a run never crosses a chunk; chunks are multiples of 256 tokens), at most 32 tiles --
-  // shortened while that would leave the GPU short of CTAs
+  // A CTA takes a run of tiles that share a state and pays for the copy, the vector terms and its own start once, as much
+  // as two or three tiles; two CTAs run per SM.  The length that gives the shortest sum of waves is taken among those that do
+  // not cross a chunk (256 heads x 16384 x 128: 32 tiles, in 3.5 waves, 409 us type A
+  // and 373 type B; 16, in 6.9, 391 and 366).
   const int tiles = (n + 127) / 128;
-  int run = 32;
-  if (per_chunk) {
-    const int tpc = chunk / 128;
-    while (tpc % run) run >>= 1;
+  int run = 0;
+  for (int r = per_chunk ? min(32, (chunk / 128) & -(chunk / 128)) : 32, least = 0; r >= 1; r >>= 1) {
+    const long long waves = ((long long)heads * ((tiles + r - 1) / r) + 295) / 296, cost = waves * (r + 2);
+    if (run == 0 || cost < least) {
+      run = r;
+      least = (int)(cost < 0x7FFFFFFF ? cost : 0x7FFFFFFF);
+    }
   }
-  while (run > 8 && (size_t)heads * ((tiles + run - 1) / run) < 4 * 148) run >>= 1;
   a.run = run;
   const unsigned grid = (unsigned)((size_t)heads * ((tiles + run - 1) / run));
   const char* name = type_b ? "fm_first_tc_readout_b" : "fm_first_tc_readout_a";
