@@ -235,6 +235,8 @@ int split_moments_forward(const Ctx& c, const void* q, const void* k, const void
                           void* workspace);
 int split_moments_status(int* out, cudaStream_t stream);
 int split_moments_status_reset(cudaStream_t stream);
+int split_rows_status(int* out, cudaStream_t stream);
+int split_rows_status_reset(cudaStream_t stream);
 int split_status(int* out, cudaStream_t stream);
 int split_status_reset(cudaStream_t stream);
 

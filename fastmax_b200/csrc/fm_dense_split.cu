@@ -19,26 +19,27 @@
 // small cross terms are added before the leading ones, and the TMEM accumulators hold ONE 64-column tile; the
 // compute warps add every tile to float32 registers, rounded to nearest.
 //
-// One CTA = one 128-row tile, 352 threads: warps 0-7 compute (warp % 4 = TMEM lane quarter = 32 rows, warp / 4 =
-// half of the tile's 64 columns, and half of the features when accumulators are read), warp 8 loads tiles by
-// TMA, warp 9 issues X Y^T and U Z^T, warp 10 the accumulating products.  S and W are single buffers that are
-// refilled as soon as they are in registers, so the tensor core works on the next tile's scores while the
-// polynomial and the split of this one run on the CUDA cores.  All waits are bounded.
+// The forward and grad_q are in fm_dense_split_rows.cu; here are the preparation of the operands and grad_k + grad_v, one CTA
+// per 128-row tile, 352 threads: warps 0-7 compute (warp % 4 = TMEM lane quarter = 32 rows, warp / 4 = half of the tile's 64
+// columns, and half of the features when accumulators are read), warp 8 loads tiles by TMA, warp 9 issues X Y^T and U Z^T,
+// warp 10 the accumulating products.  S and W are single buffers that are refilled as soon as they are in registers, so the
+// tensor core works on the next tile's scores while the polynomial and the split of this one run on the CUDA cores.  All
+// waits are bounded.
 //
 // Measured (B200, forward / grad_q / grad_k + grad_v, ms; the CUDA-core family on the same inputs in brackets):
-//   512 heads x 1000 causal, d = 32:   0.30 / 0.37 / 0.54  (1.40 / 2.00 / 2.45)
-//    64 heads x 4000 unmasked, d = 64: 1.07 / 1.81 / 3.08  (7.96 / 11.7 / 15.6)
+//   512 heads x 1000 causal, d = 32:   0.22 / 0.29 / 0.53  (1.40 / 2.00 / 2.45)
+//    64 heads x 4000 unmasked, d = 64: 1.07 / 1.81 / 3.05  (7.96 / 11.7 / 15.6)
 // Error against float64 (2-norm, outputs and gradients): 0.8-3.7e-7 for 64 to 10 000 tokens where the CUDA-core
-// family has 0.9e-7 to 2.4e-6.  What bounds it: the chain of hand-offs per 64-column tile (scores -> registers ->
-// operand parts -> products -> sums), 2 000-2 300 cycles at d = 32 against 780 (forward) of tensor-pipe time.  DKDV holds
-// 32 columns of S and W and six arrays of parts at once and is the one that spills at 168 registers (246 bytes of
-// stores at d = 64, 44 at d = 32).
+// family has 0.9e-7 to 2.4e-6.  What bounds grad_k + grad_v: the chain of hand-offs per 64-column tile (scores -> registers ->
+// operand parts -> products -> sums), 2 950 cycles at d = 32 of which the polynomial and the splits take 1 550 and the tensor
+// pipe 1 740, and a row tile's ends, a quarter of its time at 8 column tiles.  It does not gain from what serves the others:
+// walking row tiles in one CTA costs it as much in registers as it saves (533 -> 528 us), sixteen compute warps instead of
+// eight 558, two CTAs per SM with the parts in the place of the scores 607.  32 columns of S and W and six arrays of parts are
+// held at once, and it spills at 168 registers (246 bytes of stores at d = 64, 28 at d = 32).
 //
-// Operands: split3_kernel writes each tensor once as rows of [h | m | l] (3 d bf16); a tile of them in shared
-// memory is a set of 64-element (128-byte) swizzle atoms -- d = 64: one atom per part; d = 32: [h | m] and
-// [l | zero fill].
-#include "fm_common.cuh"
-#include "fm_sm100.cuh"
+// Operands: split3_kernel writes each tensor once as rows of [h | m | l] (3 d bf16); each part of a tile is a tile of its own
+// in shared memory, with rows of d bf16 swizzled over their whole length (128 or 64 bytes).
+#include "fm_dense_split.cuh"
 
 namespace fm {
 
@@ -46,187 +47,35 @@ __device__ int g_split_status = 0;
 
 namespace {
 using namespace sm100;
+using namespace split;
 
-enum { MODE_FWD = 0, MODE_DQ = 1, MODE_DKDV = 2 };
+constexpr int kThreads = 352, kProducerWarp = 8, kIssuerWarp = 9, kAccIssuerWarp = 10;
 
-struct SplitArgs {
-  float* o1;              // out, grad_q or grad_k
-  float* o2;              // grad_v (DKDV)
-  float* den_out;         // FWD
-  const float* o1_add;    // fp32 rows added before the result is divided / stored (may be null)
-  const float* o2_add;
-  const float* den_add;   // FWD
-  const float* x;         // row operand as given (normalisation dot)
-  const float* dvec;      // (query heads, nq)
-  float* dots;            // per row head: sum of o1 . x, or null
-  const stat_t* stat_q;
-  const stat_t* stat_k;
-  int nrows, ncols, off, mask, ntr, chunk, ratio, by_tile;
-  int o_stride, den_stride;   // FWD: floats per row of out and den (the packed layout interleaves them)
-  float a0, a1, a2, lim;
-};
-
-constexpr int BM = 128, BN = 64;
-constexpr int kThreads = 352, kComputeWarps = 8, kProducerWarp = 8, kIssuerWarp = 9, kAccIssuerWarp = 10;
-
-template <int D, int MODE>
+template <int D>
 struct SC {
-  static constexpr int NA = (D == 64) ? 3 : 2;              // 64-element atoms per operand row
-  static constexpr int ROW_SUB = BM * 128, ROW_TILE = NA * ROW_SUB;
-  static constexpr int COL_SUB = BN * 128, COL_TILE = NA * COL_SUB, STAGE = 2 * COL_TILE;
-  static constexpr int OFF_U = ROW_TILE, OFF_ST = (MODE == MODE_FWD ? 1 : 2) * ROW_TILE;
-  static constexpr int NS = (D == 64 && MODE != MODE_FWD) ? 2 : 3;
-  static constexpr int OFF_VEC = OFF_ST + NS * STAGE;       // per compute warp 2 x 32 floats; row-sum exchange
+  static constexpr int ROW_SUB = BM * D * 2, ROW_TILE = 3 * ROW_SUB;
+  static constexpr int COL_SUB = BN * D * 2, COL_TILE = 3 * COL_SUB, STAGE = 2 * COL_TILE;
+  static constexpr int OFF_U = ROW_TILE, OFF_ST = 2 * ROW_TILE;
+  static constexpr int NS = D == 64 ? 2 : 4;
+  static constexpr int OFF_VEC = OFF_ST + NS * STAGE;       // per compute warp 2 x 32 floats
   static constexpr int OFF_BAR = OFF_VEC + kComputeWarps * 2 * 32 * 4;
   static constexpr int NBAR = 3 + 2 * NS + 4;
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_TMEM + 16 + 1024;
-  // TMEM columns: S 64 | W 64 | three parts of 32 packed columns (P, or E and P) | accumulators of 64 columns
-  // (d = 32: leading terms 32, cross terms with ym or yl 32)
-  static constexpr int T_S = 0, T_W = BN, T_E = (MODE == MODE_FWD) ? BN : 2 * BN, T_P = T_E + 96;
-  static constexpr int T_A1 = (MODE == MODE_DKDV) ? T_P + 96 : T_E + 96, T_A2 = T_A1 + 64;
-  // row operands that also lie in tensor memory (3 d / 2 columns each), as far as there is room
-  static constexpr int NT = (MODE == MODE_DKDV) ? (D == 32 ? 1 : 0) : (MODE == MODE_DQ ? 2 : 1);
-  static constexpr int XC = 3 * D / 2;
-  static constexpr int T_X = (MODE == MODE_DKDV) ? T_A2 + 64 : T_A1 + 64, T_U = T_X + XC;
-  static constexpr int T_COLS = 512;
+  // TMEM columns: S 64 | W 64 | three parts of 32 packed columns of E | of P | accumulators of 64 columns (d = 32: leading
+  // terms 32, cross terms with ym or yl 32) | x where there is room (3 d / 2 columns)
+  enum : int { T_S = 0, T_W = BN, T_E = 2 * BN, T_P = T_E + 96, T_A1 = T_P + 96, T_A2 = T_A1 + 64, T_X = T_A2 + 64, T_COLS = 512 };
+  static constexpr bool X_IN_T = D == 32;
 };
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_split_status, 0, code); }
 
-// Offset of part p (0 h, 1 m, 2 l) inside an operand tile, in descriptor units of 16 bytes.
 template <int D>
-__device__ __forceinline__ constexpr uint32_t part_off(int p, int sub) {
-  return D == 64 ? (uint32_t)p * (sub >> 4) : (p == 0 ? 0u : (p == 1 ? 4u : (uint32_t)(sub >> 4)));
-}
-
-// One K = 16 step of D[tmem] (+)= A[smem] B[smem]^T, both K-major.
-__device__ __forceinline__ void umma_ss_1(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .b64 da, db;\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "mov.b64 da, {%1, %3};\n"
-      "mov.b64 db, {%2, %3};\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n"
-      "}\n"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// 128 x 64 scores of a row tile against a column tile: the six part products, small terms first.
-template <int D>
-__device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, int row_sub, int col_sub) {
-  constexpr uint32_t idesc = idesc_bf16(BM, BN, 0, 0);
-  constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
-#pragma unroll
-  for (int t = 0; t < 6; ++t)
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks)
-      umma_ss_1(d_tmem, a_lo + part_off<D>(PA[t], row_sub) + 2 * ks, b_lo + part_off<D>(PB[t], col_sub) + 2 * ks, idesc,
-                (t | ks) ? 1u : 0u);
-}
-
-// The same with the row operand in tensor memory (d / 2 columns per part): a K step then reads only the column
-// tile from shared memory, 32 instead of 49 cycles (128 x 64, the shared-memory port being the limit otherwise).
-template <int D>
-__device__ __forceinline__ void issue_scores_t(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, int col_sub) {
-  constexpr uint32_t idesc = idesc_bf16(BM, BN, 0, 0);
-  constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
-#pragma unroll
-  for (int t = 0; t < 6; ++t)
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks)
-      umma_ts_1(d_tmem, a_tmem + PA[t] * (D / 2) + 8 * ks, b_lo + part_off<D>(PB[t], col_sub) + 2 * ks, idesc,
-                (t | ks) ? 1u : 0u);
-}
-
-// acc = (three parts of a 128 x 64 operand in TMEM) x (column tile, MN-major), small terms first.
-template <int D>
-__device__ __forceinline__ void issue_acc(uint32_t acc, uint32_t a_tmem, uint32_t b_mn, int col_sub) {
-  constexpr uint32_t idesc64 = idesc_bf16(BM, 64, 0, 1);
-  const uint32_t ah = a_tmem, am = a_tmem + 32, al = a_tmem + 64;
-  if constexpr (D == 64) {
-    const uint32_t bh = b_mn, bm = b_mn + (col_sub >> 4), bl = b_mn + 2 * (col_sub >> 4);
-    umma_ts_steps<BN / 16>(acc, am, bm, idesc64, 0u);
-    umma_ts_steps<BN / 16>(acc, ah, bl, idesc64, 1u);
-    umma_ts_steps<BN / 16>(acc, al, bh, idesc64, 1u);
-    umma_ts_steps<BN / 16>(acc, ah, bm, idesc64, 1u);
-    umma_ts_steps<BN / 16>(acc, am, bh, idesc64, 1u);
-    umma_ts_steps<BN / 16>(acc, ah, bh, idesc64, 1u);
-  } else {
-    // columns 0..31 against the h part, 32..63 against the m part; the l part is added to the latter
-    constexpr uint32_t idesc32 = idesc_bf16(BM, 32, 0, 1);
-    umma_ts_steps<BN / 16>(acc, am, b_mn, idesc64, 0u);
-    umma_ts_steps<BN / 16>(acc + 32, ah, b_mn + (col_sub >> 4), idesc32, 1u);
-    umma_ts_steps<BN / 16>(acc, al, b_mn, idesc32, 1u);
-    umma_ts_steps<BN / 16>(acc, ah, b_mn, idesc64, 1u);
-  }
-}
-
-// Adds this warp's half of the features of one tile's accumulator to the running sums (packed pairs).
-template <int D>
-__device__ __forceinline__ void promote(uint64_t (&run)[D / 4], uint32_t taddr, int cpart) {
-  if constexpr (D == 64) {
-    uint32_t a[32];
-    tmem_ld32(taddr + cpart * 32, a);
-    tmem_wait_ld(a);
-#pragma unroll
-    for (int e = 0; e < 16; ++e) run[e] = add2(run[e], pack2u(a[2 * e], a[2 * e + 1]));
-  } else {
-    uint32_t a[16], b[16];
-    tmem_ld16(taddr + cpart * 16, a);
-    tmem_ld16(taddr + 32 + cpart * 16, b);
-    tmem_wait_ld(a, b);
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-      run[e] = add2(run[e], add2(pack2u(a[2 * e], a[2 * e + 1]), pack2u(b[2 * e], b[2 * e + 1])));
-  }
-}
-
-// (sum + add) * scale -> one row's half of the features; returns its dot product with x when wanted.
-template <int D>
-__device__ __forceinline__ float store_half(const uint64_t (&run)[D / 4], float* dst, const float* add, const float* xr,
-                                            float scale) {
-  float part = 0.f;
-  const bool wide = (((uintptr_t)dst | (uintptr_t)add | (uintptr_t)xr) & 31) == 0;
-#pragma unroll
-  for (int b = 0; b < D / 16; ++b) {
-    float f[8];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) unpack2(run[4 * b + e], f[2 * e], f[2 * e + 1]);
-    if (add) {
-      uint32_t aw[8];
-      ldg32(add + 8 * b, aw, wide);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] += __uint_as_float(aw[e]);
-    }
-    uint32_t w[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      f[e] *= scale;
-      w[e] = __float_as_uint(f[e]);
-    }
-    stg32(dst + 8 * b, w, wide);
-    if (xr) {
-      uint32_t xw[8];
-      ldg32(xr + 8 * b, xw, wide);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) part = fmaf(f[e], __uint_as_float(xw[e]), part);
-    }
-  }
-  return part;
-}
-
-template <int D, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
-split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
+split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
              const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmZ, const SplitArgs a) {
-  using C = SC<D, MODE>;
-  constexpr int NS = C::NS, NA = C::NA;
-  constexpr bool rev = MODE == MODE_DKDV, HAS_U = MODE != MODE_FWD;
+  using C = SC<D>;
+  constexpr int NS = C::NS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -241,27 +90,18 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // longest rows first (row_tile_of)
   int head, pidx;
-  row_tile_of(blockIdx.x, a.by_tile, a.ntr, head, pidx);
-  const int r0 = (rev ? pidx : a.ntr - 1 - pidx) * BM;
+  row_tile_of(blockIdx.x, a.order, a.ntr, head, pidx);
+  const int r0 = pidx * BM;
 
   const int ntile = (a.ncols + BN - 1) / BN;
-  int tb = 0, te = ntile;
-  if (a.mask) {
-    if (rev) tb = max(0, r0 - a.off) / BN;
-    else te = min(ntile, (min(r0 + BM - 1, a.nrows - 1) + a.off) / BN + 1);
-  }
-  if (a.chunk > 0) {  // the row tile lies in one chunk (chunk % 256 == 0)
-    const int cb = (r0 / a.chunk) * (a.chunk / BN), ce = cb + a.chunk / BN;
-    if (rev) te = min(te, ce);
-    else tb = cb;
-  }
-  // grouped heads: a key/value head (DKDV rows) walks its tile range once per query head of the group
-  const int Jh = max(te - tb, 0);
-  const int J = rev ? Jh * a.ratio : Jh;
+  const int tb = a.mask ? max(0, r0 - a.off) / BN : 0;
+  const int te = a.chunk > 0 ? min(ntile, (r0 / a.chunk + 1) * (a.chunk / BN)) : ntile;   // the row tile lies in one chunk
+  // grouped heads: a key/value head walks its tile range once per query head of the group
+  const int Jh = max(te - tb, 0), J = Jh * a.ratio;
   struct ColPos { int t, h; };
-  const ColPos pos0 = {tb, rev ? head * a.ratio : head / a.ratio};
+  const ColPos pos0 = {tb, head * a.ratio};
   auto advance = [&](ColPos& cp) {
-    if (++cp.t >= tb + Jh && rev) { cp.t = tb; ++cp.h; }
+    if (++cp.t >= tb + Jh) { cp.t = tb; ++cp.h; }
   };
 
   if (tid == 0) {
@@ -283,23 +123,19 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // where the two column halves of a row exchange their row sums (FWD)
-  float* const rows_sum = (float*)(smem + C::OFF_VEC);
-
-  float rsum = 0.f;
   bool ok_compute = true;
-  uint64_t run1[D / 4], run2[rev ? D / 4 : 1];
+  uint64_t run1[D / 4], run2[D / 4];
   if (warp == kProducerWarp) {
     // ================= TMA producer =================
     if (lane == 0 && J > 0) {
       tma_prefetch_desc(&tmX);
-      if (HAS_U) tma_prefetch_desc(&tmU);
+      tma_prefetch_desc(&tmU);
       tma_prefetch_desc(&tmY);
       tma_prefetch_desc(&tmZ);
-      mbar_expect_tx(BAR_X, (HAS_U ? 2 : 1) * C::ROW_TILE);
-      for (int sub = 0; sub < NA; ++sub) {
-        tma_load_3d(sbase + sub * C::ROW_SUB, &tmX, BAR_X, sub * 64, r0, head);
-        if (HAS_U) tma_load_3d(sbase + C::OFF_U + sub * C::ROW_SUB, &tmU, BAR_X, sub * 64, r0, head);
+      mbar_expect_tx(BAR_X, 2 * C::ROW_TILE);
+      for (int p = 0; p < 3; ++p) {
+        tma_load_3d(sbase + p * C::ROW_SUB, &tmX, BAR_X, p * D, r0, head);
+        tma_load_3d(sbase + C::OFF_U + p * C::ROW_SUB, &tmU, BAR_X, p * D, r0, head);
       }
     }
     ColPos pc = pos0;
@@ -309,9 +145,9 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       if (lane == 0) {
         mbar_expect_tx(BAR_FULL(s), C::STAGE);
         const uint32_t dst = sbase + C::OFF_ST + s * C::STAGE;
-        for (int sub = 0; sub < NA; ++sub) {
-          tma_load_3d(dst + sub * C::COL_SUB, &tmY, BAR_FULL(s), sub * 64, pc.t * BN, pc.h);
-          tma_load_3d(dst + C::COL_TILE + sub * C::COL_SUB, &tmZ, BAR_FULL(s), sub * 64, pc.t * BN, pc.h);
+        for (int p = 0; p < 3; ++p) {
+          tma_load_3d(dst + p * C::COL_SUB, &tmY, BAR_FULL(s), p * D, pc.t * BN, pc.h);
+          tma_load_3d(dst + C::COL_TILE + p * C::COL_SUB, &tmZ, BAR_FULL(s), p * D, pc.t * BN, pc.h);
         }
       }
     }
@@ -321,7 +157,7 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       const uint32_t x_lo = desc_lo(sbase, 16), u_lo = desc_lo(sbase + C::OFF_U, 16);
       const uint32_t st_k = desc_lo(sbase + C::OFF_ST, 16);   // stage 0, K-major view
       bool ok = mbar_wait_warp(BAR_X, 0);
-      if (ok && C::NT > 0) ok = mbar_wait_warp(BAR_XT, 0);
+      if (ok && C::X_IN_T) ok = mbar_wait_warp(BAR_XT, 0);
       if (!ok) report(2);
       tc_fence_after();
       for (int j = 0; ok && j < J; ++j) {
@@ -331,12 +167,8 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         tc_fence_after();
         const uint32_t y_lo = st_k + (uint32_t)s * (C::STAGE >> 4);
         if (elect_one()) {
-          if constexpr (C::NT >= 1) issue_scores_t<D>(tmem + C::T_S, tmem + C::T_X, y_lo, C::COL_SUB);
-          else issue_scores<D>(tmem + C::T_S, x_lo, y_lo, C::ROW_SUB, C::COL_SUB);
-          if constexpr (HAS_U && C::NT >= 2)
-            issue_scores_t<D>(tmem + C::T_W, tmem + C::T_U, y_lo + (C::COL_TILE >> 4), C::COL_SUB);
-          else if constexpr (HAS_U)
-            issue_scores<D>(tmem + C::T_W, u_lo, y_lo + (C::COL_TILE >> 4), C::ROW_SUB, C::COL_SUB);
+          issue_scores<D, C::X_IN_T>(tmem + C::T_S, C::X_IN_T ? tmem + C::T_X : x_lo, y_lo);
+          issue_scores<D, false>(tmem + C::T_W, u_lo, y_lo + (C::COL_TILE >> 4));
           umma_commit(BAR_S);
         }
         __syncwarp();
@@ -346,15 +178,15 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   } else if (warp == kAccIssuerWarp) {
     // ================= MMA issuer of the accumulating products =================
     if (J > 0) {
-      const uint32_t st_mn = desc_lo(sbase + C::OFF_ST, C::COL_SUB);   // stage 0, MN-major view
+      const uint32_t st_mn = desc_mn(sbase + C::OFF_ST, D);   // stage 0, MN-major view
       for (int j = 0; j < J; ++j) {
         const int s = j % NS;
         if (!mbar_wait_warp(BAR_P, (uint32_t)(j & 1))) { report(5); break; }
         tc_fence_after();
         const uint32_t y_mn = st_mn + (uint32_t)s * (C::STAGE >> 4), z_mn = y_mn + (C::COL_TILE >> 4);
         if (elect_one()) {
-          issue_acc<D>(tmem + C::T_A1, tmem + C::T_E, MODE == MODE_FWD ? z_mn : y_mn, C::COL_SUB);
-          if (rev) issue_acc<D>(tmem + C::T_A2, tmem + C::T_P, z_mn, C::COL_SUB);
+          issue_acc<D>(tmem + C::T_A1, tmem + C::T_E, y_mn);
+          issue_acc<D>(tmem + C::T_A2, tmem + C::T_P, z_mn);
           umma_commit(BAR_PV);
           umma_commit(BAR_EMPTY(s));
           if (j + 1 == J) umma_commit(BAR_DONE);
@@ -367,8 +199,7 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     // ================= compute warps =================
     const int cpart = warp >> 2, qd = warp & 3;
     const int row = r0 + qd * 32 + lane;
-    const bool row_ok = row < a.nrows;
-    const float ck = stat_scale(a.stat_k, rev ? head : head / a.ratio, a.lim);
+    const float ck = stat_scale(a.stat_k, head, a.lim);
     const uint64_t A0v = pack2(a.a0, a.a0);
     uint64_t A1v, A2v, A2d;
     auto set_coefficients = [&](int hq) {
@@ -378,17 +209,10 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       A2v = pack2(A2, A2);
       A2d = pack2(2.f * A2, 2.f * A2);
     };
-    int hq_now = rev ? head * a.ratio : head;
+    int hq_now = head * a.ratio;
     set_coefficients(hq_now);
-    int limcol = a.ncols - 1, lowcol = 0;                   // columns kept: lowcol <= col <= limcol
-    if (a.mask) {
-      if (rev) lowcol = row - a.off;
-      else limcol = min(limcol, row + a.off);
-    }
-    const int wrow_lo = r0 + qd * 32, wrow_hi = wrow_lo + 31;
-    float dl_row = 0.f;
-    if (MODE == MODE_DQ && row_ok) dl_row = __ldg(a.dvec + (size_t)head * a.nrows + row);
-    const uint64_t ndl_row = pack2(-dl_row, -dl_row);
+    const int limcol = a.ncols - 1, lowcol = a.mask ? row - a.off : 0;     // columns kept: lowcol <= col <= limcol
+    const int wrow_hi = r0 + qd * 32 + 31;
     const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
     float* myvec = (float*)(smem + C::OFF_VEC) + warp * 64;
     const uint32_t myvec_s = sbase + C::OFF_VEC + warp * 256;
@@ -399,32 +223,23 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       return (col < a.ncols) ? -__ldg(a.dvec + (size_t)cp.h * a.ncols + col) : 0.f;
     };
 #pragma unroll
-    for (int e = 0; e < D / 4; ++e) run1[e] = 0ull;
-    if constexpr (rev) {
-#pragma unroll
-      for (int e = 0; e < D / 4; ++e) run2[e] = 0ull;
-    }
+    for (int e = 0; e < D / 4; ++e) run1[e] = run2[e] = 0ull;
     bool ok = true;
-    if (C::NT > 0 && J > 0) {
-      // copy the row operands to tensor memory: column c of a part holds elements 2c and 2c+1 of the row; the
-      // two warps of a lane quarter take alternate parts
+    if (C::X_IN_T && J > 0) {
+      // copy x to tensor memory: column c of a part holds elements 2c and 2c+1 of the row; the two warps of a lane quarter
+      // take alternate parts.  (16-byte pieces, XOR-swizzled by the row's place in its swizzle atom)
       if (!mbar_wait(BAR_X, 0)) { report(6); ok = false; }
       if (ok) {
-        const int r = qd * 32 + lane;
-        for (int it = cpart; it < 3 * C::NT; it += 2) {
-          const int t = it % 3;
-          const uint32_t src = sbase + (it < 3 ? 0 : C::OFF_U) + (D == 64 ? t : t >> 1) * C::ROW_SUB + r * 128;
-          const int piece0 = (D == 64) ? 0 : (t & 1) * 4;       // 16-byte pieces, XOR-swizzled by the row
-          uint32_t w[D / 2];
+        const int r = qd * 32 + lane, sw = (r >> 1) & 3;
+        for (int p = cpart; p < 3; p += 2) {
+          uint32_t w[16];
 #pragma unroll
-          for (int pc = 0; pc < D / 8; ++pc) {
-            const ulonglong2 v = lds_v2(src + (((piece0 + pc) ^ (r & 7)) << 4));
+          for (int pc = 0; pc < 4; ++pc) {
+            const ulonglong2 v = lds_v2(sbase + p * C::ROW_SUB + r * (D * 2) + ((pc ^ sw) << 4));
             w[4 * pc] = (uint32_t)v.x; w[4 * pc + 1] = (uint32_t)(v.x >> 32);
             w[4 * pc + 2] = (uint32_t)v.y; w[4 * pc + 3] = (uint32_t)(v.y >> 32);
           }
-          const uint32_t dst = tl + (it < 3 ? C::T_X : C::T_U) + t * (D / 2);
-          if constexpr (D == 64) tmem_st32(dst, w);
-          else tmem_st16(dst, w);
+          tmem_st16(tl + C::T_X + p * (D / 2), w);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -432,46 +247,35 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         if (lane == 0) mbar_arrive(BAR_XT);
       }
     }
-    uint64_t rs2 = 0ull;
     ColPos pc = pos0;
-    float nxt = rev ? fetch_vec(0, pc) : 0.f;
+    float nxt = fetch_vec(0, pc);
     for (int j = 0; ok && j < J; ++j, advance(pc)) {
       const float cur = nxt;
-      if (rev) {
-        ColPos pn = pc;
-        advance(pn);
-        nxt = fetch_vec(j + 1, pn);
-        if (pc.h != hq_now) {
-          hq_now = pc.h;
-          set_coefficients(pc.h);
-        }
+      ColPos pn = pc;
+      advance(pn);
+      nxt = fetch_vec(j + 1, pn);
+      if (pc.h != hq_now) {
+        hq_now = pc.h;
+        set_coefficients(pc.h);
       }
       if (!mbar_wait(BAR_S, (uint32_t)(j & 1))) { report(7); ok = false; break; }
       tc_fence_after();
       const uint32_t vec_s = myvec_s + (j & 1) * 128;
-      if (rev) {
-        myvec[(j & 1) * 32 + lane] = cur;
-        __syncwarp();
-      }
-      uint32_t sv[32], wv[HAS_U ? 32 : 1];
+      myvec[(j & 1) * 32 + lane] = cur;
+      __syncwarp();
+      uint32_t sv[32], wv[32];
       tmem_ld32(tl + C::T_S + cpart * 32, sv);
-      if constexpr (HAS_U) {
-        tmem_ld32(tl + C::T_W + cpart * 32, wv);
-        tmem_wait_ld(sv, wv);
-      } else {
-        tmem_wait_ld(sv);
-      }
+      tmem_ld32(tl + C::T_W + cpart * 32, wv);
+      tmem_wait_ld(sv, wv);
       // S and W of this tile are in registers: the next tile's may be issued
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(BAR_SFREE);
       const int c0 = pc.t * BN + cpart * 32;                // first of this warp's 32 columns
-      bool need_mask = (c0 + 32 > a.ncols);
-      if (a.mask) need_mask = need_mask || (rev ? (c0 < wrow_hi - a.off) : (c0 + 31 > wrow_lo + a.off));
-      // E (or P of the forward) and P of the tile as three packed parts each
-      uint32_t e3[3][16], p3[3][rev ? 16 : 1];
+      const bool need_mask = c0 + 32 > a.ncols || (a.mask && c0 < wrow_hi - a.off);
+      // E and P of the tile as three packed parts each
+      uint32_t e3[3][16], p3[3][16];
       ulonglong2 nd2 = make_ulonglong2(0ull, 0ull);
-      uint64_t ts2 = 0ull;                                  // row sums of this tile
       auto element = [&](int e, bool masked) {
         const uint64_t s2 = pack2u(sv[2 * e], sv[2 * e + 1]);
         bool z0 = false, z1 = false;
@@ -486,17 +290,10 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
           unpack2(v, v0, v1);
           return pack2(z0 ? 0.f : v0, z1 ? 0.f : v1);
         };
-        if constexpr (MODE == MODE_FWD) {
-          const uint64_t pv = keep(fma2(fma2(A2v, s2, A1v), s2, A0v));
-          ts2 = add2(ts2, pv);
-          split3(pv, e3[0][e], e3[1][e], e3[2][e]);
-        } else {
-          if (rev && (e & 1) == 0) nd2 = lds_v2(vec_s + (e >> 1) * 16);   // four column values per load
-          const uint64_t ndl = rev ? ((e & 1) ? nd2.y : nd2.x) : ndl_row;
-          const uint64_t ev = keep(mul2(fma2(A2d, s2, A1v), add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl)));
-          split3(ev, e3[0][e], e3[1][e], e3[2][e]);
-          if constexpr (rev) split3(keep(fma2(fma2(A2v, s2, A1v), s2, A0v)), p3[0][e], p3[1][e], p3[2][e]);
-        }
+        if ((e & 1) == 0) nd2 = lds_v2(vec_s + (e >> 1) * 16);   // four column values per load
+        const uint64_t ndl = (e & 1) ? nd2.y : nd2.x;
+        split3(keep(mul2(fma2(A2d, s2, A1v), add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl))), e3[0][e], e3[1][e], e3[2][e]);
+        split3(keep(fma2(fma2(A2v, s2, A1v), s2, A0v)), p3[0][e], p3[1][e], p3[2][e]);
       };
       // the mask test stays outside the element loops so that each is one basic block of independent pairs
       if (!need_mask) {
@@ -506,7 +303,6 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
 #pragma unroll
         for (int e = 0; e < 16; ++e) element(e, true);
       }
-      if (MODE == MODE_FWD) rs2 = add2(rs2, ts2);
       // the previous tile's products must be done before their operands are overwritten; their sums are
       // taken over before the arrival below lets this tile's products replace them
       if (j > 0) {
@@ -516,11 +312,11 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
 #pragma unroll
       for (int t = 0; t < 3; ++t) {
         tmem_st16(tl + C::T_E + 32 * t + cpart * 16, e3[t]);
-        if constexpr (rev) tmem_st16(tl + C::T_P + 32 * t + cpart * 16, p3[t]);
+        tmem_st16(tl + C::T_P + 32 * t + cpart * 16, p3[t]);
       }
       if (j > 0) {
         promote<D>(run1, tl + C::T_A1, cpart);
-        if constexpr (rev) promote<D>(run2, tl + C::T_A2, cpart);
+        promote<D>(run2, tl + C::T_A2, cpart);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -532,16 +328,10 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       else {
         tc_fence_after();
         promote<D>(run1, tl + C::T_A1, cpart);
-        if constexpr (rev) promote<D>(run2, tl + C::T_A2, cpart);
+        promote<D>(run2, tl + C::T_A2, cpart);
       }
     }
     ok_compute = ok;
-    if (MODE == MODE_FWD) {
-      float lo, hi;
-      unpack2(rs2, lo, hi);
-      rsum = lo + hi;
-      rows_sum[cpart * BM + qd * 32 + lane] = rsum;
-    }
   }
 
   tc_fence_before();
@@ -555,35 +345,15 @@ split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
     const int cpart = warp >> 2, rl = (warp & 3) * 32 + lane, row = r0 + rl;
     const bool row_ok = row < a.nrows;
     const size_t grow = (size_t)head * a.nrows + (row_ok ? row : 0), at = grow * D + cpart * (D / 2);
-    if constexpr (MODE == MODE_FWD) {
-      if (row_ok) {
-        const float dsum = rows_sum[rl] + rows_sum[BM + rl] + (a.den_add ? a.den_add[grow] : 0.f);
-        if (cpart == 0) a.den_out[grow * a.den_stride] = dsum;
-        if (a.o_stride == D) {
-          store_half<D>(run1, a.o1 + at, a.o1_add ? a.o1_add + at : nullptr, nullptr, 1.0f / dsum);
-        } else {             // rows of d + 1 floats: no alignment to use
-          const float inv = 1.0f / dsum;
-          float* dst = a.o1 + grow * a.o_stride + cpart * (D / 2);
+    float part = 0.f;
+    if (row_ok) {
+      part = store_half<D>(run1, a.o1 + at, a.o1_add ? a.o1_add + at : nullptr, a.dots ? a.x + at : nullptr, 1.f);
+      store_half<D>(run2, a.o2 + at, a.o2_add ? a.o2_add + at : nullptr, nullptr, 1.f);
+    }
+    if (a.dots) {
 #pragma unroll
-          for (int e = 0; e < D / 4; ++e) {
-            float lo, hi;
-            unpack2(run1[e], lo, hi);
-            dst[2 * e] = lo * inv;
-            dst[2 * e + 1] = hi * inv;
-          }
-        }
-      }
-    } else {
-      float part = 0.f;
-      if (row_ok) {
-        part = store_half<D>(run1, a.o1 + at, a.o1_add ? a.o1_add + at : nullptr, a.dots ? a.x + at : nullptr, 1.f);
-        if constexpr (rev) store_half<D>(run2, a.o2 + at, a.o2_add ? a.o2_add + at : nullptr, nullptr, 1.f);
-      }
-      if (a.dots) {
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
-        if (lane == 0) atomicAdd(a.dots + head, part);
-      }
+      for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
+      if (lane == 0) atomicAdd(a.dots + head, part);
     }
   }
 }
@@ -670,35 +440,23 @@ int launch_split3(const Ctx& c, const SplitJobs& jobs, int count) {
   return FASTMAX_OK;
 }
 
-template <int D, int MODE>
-int launch_mode(const Ctx& c, const char* name, const void* x, const void* u, const void* y, const void* z, int nrows,
-                int ncols, SplitArgs a) {
-  using C = SC<D, MODE>;
-  constexpr bool rev = MODE == MODE_DKDV;
+template <int D>
+int launch_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, SplitArgs a) {
+  using C = SC<D>;
   const fastmax_problem& p = c.p;
-  const int heads = rev ? p.bhkv : p.bh, col_heads = rev ? p.bh : p.bhkv;
-  if (heads == 0 || nrows == 0) return FASTMAX_OK;
+  if (p.bhkv == 0 || p.nk == 0) return FASTMAX_OK;
   CUtensorMap tx, tu, ty, tz;
   int rc;
-  if ((rc = tma_map_bf16(&tx, x, heads, nrows, 3 * D, BM))) return rc;
-  if ((rc = tma_map_bf16(&tu, u, heads, nrows, 3 * D, BM))) return rc;
-  if ((rc = tma_map_bf16(&ty, y, col_heads, ncols, 3 * D, BN))) return rc;
-  if ((rc = tma_map_bf16(&tz, z, col_heads, ncols, 3 * D, BN))) return rc;
-  a.nrows = nrows;
-  a.ncols = ncols;
-  a.ntr = (nrows + BM - 1) / BM;
-  a.by_tile = rows_by_tile(p.mask && a.chunk == 0, heads, a.ntr, 1);
-  a.ratio = p.bh / p.bhkv;
-  a.off = p.nk - p.nq;
-  a.mask = p.mask;
-  a.a0 = p.a0;
-  a.a1 = p.a1;
-  a.a2 = (p.p == 2) ? p.a2 : 0.f;
-  a.lim = p.lim;
-  const long long blocks = (long long)heads * a.ntr;
-  if (blocks > 0x7FFFFFFFLL) return fail(FASTMAX_E_ARG, "heads x row tiles = %lld exceeds the grid limit", blocks);
-  FM_CUDA_TRY(cudaFuncSetAttribute(split_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-  FM_LAUNCH(name, c.stream, (split_kernel<D, MODE><<<(unsigned)blocks, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, a)));
+  if ((rc = split_map<D>(&tx, k, p.bhkv, p.nk, BM))) return rc;
+  if ((rc = split_map<D>(&tu, v, p.bhkv, p.nk, BM))) return rc;
+  if ((rc = split_map<D>(&ty, q, p.bh, p.nq, BN))) return rc;
+  if ((rc = split_map<D>(&tz, gs, p.bh, p.nq, BN))) return rc;
+  long long blocks;
+  if ((rc = set_sizes(p, p.bhkv, p.nk, p.nq, &a, &blocks))) return rc;
+  a.order = rows_by_tile(p.mask && a.chunk == 0, a.heads, a.ntr, 1);
+  FM_CUDA_TRY(cudaFuncSetAttribute(split_dkdv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+  FM_LAUNCH("fm_dense_split_dkdv", c.stream,
+            (split_dkdv_kernel<D><<<(unsigned)blocks, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
@@ -746,8 +504,7 @@ int dense_split_forward(const Ctx& c, const void* q, const void* k, const void* 
   a.o_stride = o.o_stride;
   a.den_stride = o.den_stride;
   if (ca) { a.chunk = ca->chunk; a.o1_add = ca->out_add; a.den_add = ca->den_add; }
-  if (p.d == 32) return launch_mode<32, MODE_FWD>(c, "fm_dense_split_fwd", q3, q3, k3, v3, p.nq, p.nk, a);
-  return launch_mode<64, MODE_FWD>(c, "fm_dense_split_fwd", q3, q3, k3, v3, p.nq, p.nk, a);
+  return split_rows_forward(c, q3, k3, v3, a);
 }
 
 int dense_split_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* out, const float* den,
@@ -779,17 +536,14 @@ int dense_split_backward(const Ctx& c, const void* q, const void* k, const void*
   a.o1_add = ca ? ca->gq_add : nullptr;
   a.x = (const float*)q;
   a.dots = p.normalize ? dots : nullptr;
-  if (p.d == 32) rc = launch_mode<32, MODE_DQ>(c, "fm_dense_split_dq", q3, g3, k3, v3, p.nq, p.nk, a);
-  else rc = launch_mode<64, MODE_DQ>(c, "fm_dense_split_dq", q3, g3, k3, v3, p.nq, p.nk, a);
-  if (rc) return rc;
+  if ((rc = split_rows_dq(c, q3, g3, k3, v3, a))) return rc;
   a.o1 = (float*)grad_k;
   a.o2 = (float*)grad_v;
   a.o1_add = ca ? ca->gk_add : nullptr;
   a.o2_add = ca ? ca->gv_add : nullptr;
   a.x = (const float*)k;
   a.dots = p.normalize ? dots + p.bh : nullptr;
-  if (p.d == 32) return launch_mode<32, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, p.nk, p.nq, a);
-  return launch_mode<64, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, p.nk, p.nq, a);
+  return p.d == 32 ? launch_dkdv<32>(c, k3, v3, q3, g3, a) : launch_dkdv<64>(c, k3, v3, q3, g3, a);
 }
 
 int split3_scaled_q(const Ctx& c, const void* q, void* q3, const void* v, void* v3, const stat_t* stats) {

@@ -167,6 +167,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -487,6 +493,10 @@ __device__ __forceinline__ void split3(uint64_t v, uint32_t& h, uint32_t& m, uin
   m = pack_bf16_2(r);
   l = pack_bf16_2(fma2(pack2u(m << 16, m & 0xFFFF0000u), neg1, r));
 }
+
+// Registers of a warpgroup (four warps, all of whose threads take part), out of those that the block was launched with.
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // 32 bytes to / from global memory in one access where the address allows it (one full sector per lane:
 // a thread owns a whole row here, so its accesses never coalesce with its neighbours'), else two of 16.

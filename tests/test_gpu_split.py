@@ -114,3 +114,24 @@ def test_no_room_for_the_operand_parts(p):
     assert not any("split" in n_ for n_ in names), names
     for x, r, name in zip(got, want, ("out", "dq", "dk", "dv")):
         assert float((x - r).abs().max() / r.abs().max()) < BOUND, name
+
+
+@pytest.mark.parametrize("bh,n,d,mask,chunk", [(40, 700, 32, 1, 0), (200, 900, 32, 1, 0), (420, 640, 32, 1, 0), (500, 641, 32, 1, 0),
+                                               (75, 513, 32, 0, 0), (160, 1000, 64, 1, 0), (330, 520, 64, 1, 0), (60, 650, 64, 0, 0),
+                                               (150, 1100, 32, 1, 256), (600, 600, 32, 1, 256)])
+def test_row_walks_match_the_cuda_cores(bh, n, d, mask, chunk):
+    """Several row tiles to a CTA, in every order they are taken in: head by head, tile by tile, in pairs (even and odd
+    numbers of tiles).  Both families' bounds against float64 add up to 2e-5 of the largest value at these lengths."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v, go = [torch.randn(bh, n, d, generator=g, device="cuda") for _ in range(4)]
+    kw = dict(mask=bool(mask), normalize=True, p=1 if chunk else 2)
+    impl = dict(impl="moments", chunk=chunk) if chunk else {}
+    out, den, st = _cabi.forward(q, k, v, **kw, **impl)
+    got = (out,) + tuple(_cabi.backward(q, k, v, out, den, st, go, **kw, **impl))
+    out, den, st = _cabi.forward(q, k, v, impl="dense_ffma", **kw)
+    want = (out,) + tuple(_cabi.backward(q, k, v, out, den, st, go, impl="dense_ffma", **kw))
+    assert _cabi.device_status() == 0
+    for x, r, name in zip(got, want, ("out", "dq", "dk", "dv")):
+        # per head, so that a row tile that is left out or taken twice shows whatever the other heads' values are
+        err = float(((x - r).abs().amax((1, 2)) / r.abs().amax((1, 2))).max())
+        assert err < BOUND, (name, err)
