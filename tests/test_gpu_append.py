@@ -1,6 +1,6 @@
-"""Prompt processing of the decode state at the sizes where its kernels change: the tensor-core kernel's blocks of 64
-tokens (bf16, d 64 and 128), the CUDA-core kernel's batches, and the few-token kernel (below 24 tokens at p = 1, 64 at
-p = 2 for bf16 with d = 128, else 40); onto an empty and onto a filled state, against float64 sums.
+"""Prompt processing of the decode state at the sizes where its kernels change: the tensor-core kernel's blocks of 128
+tokens and their K steps of 16 (bf16, d 64 and 128), the CUDA-core kernel's batches, and the few-token kernel (below 14 and
+28 tokens at p = 1 and 2 for those, else 24 and 40); onto an empty and onto a filled state, against float64 sums.
 
 Bound: products are exact (bf16) or rounded once (float32) and sums of up to n terms are accumulated in float32, so
 the error of an element is within n * 2^-24 of the sum of its terms' magnitudes; elements of a state of N(0,1) keys
@@ -50,6 +50,13 @@ def test_append_matches_float64_sums(heads, d, p, pieces, dtype):
     if p == 2:       # both places of a pair hold the same bits
         s2 = got[:, :d * d].view(heads, d, d, d + 1)
         assert torch.equal(s2, s2.transpose(1, 2))
+
+
+@pytest.mark.parametrize("heads,d,p,pieces", [
+    (2, 64, 2, (28, 27)), (2, 64, 2, (112, 113)), (3, 64, 2, (128, 127)), (2, 128, 2, (28, 144)), (2, 128, 2, (129, 240)),
+    (2, 64, 1, (14, 128)), (2, 128, 1, (13, 257, 16)), (4, 64, 2, (3000,))])
+def test_append_at_the_edges_of_blocks_and_steps(heads, d, p, pieces):
+    test_append_matches_float64_sums(heads, d, p, pieces, torch.bfloat16)
 
 
 @pytest.mark.parametrize("d,ratio", [(64, 1), (64, 5), (32, 6), (128, 3)])
