@@ -88,6 +88,11 @@ __device__ __forceinline__ float store_row_vec(uint32_t taddr, bool row_ok, __nv
                                                const __nv_bfloat16* xr, float scale) {
   float part = 0.f;
   const bool wide = (((uintptr_t)dst | (uintptr_t)xr) & 31) == 0;
+  uint32_t xw[NC / 16][8];                 // asked for together
+  if (xr && row_ok) {
+#pragma unroll
+    for (int i = 0; i < NC / 16; ++i) ldg32(xr + 16 * i, xw[i], wide);
+  }
 #pragma unroll
   for (int c0 = 0; c0 < NC; c0 += 16) {
     uint32_t ov[16];
@@ -109,12 +114,10 @@ __device__ __forceinline__ float store_row_vec(uint32_t taddr, bool row_ok, __nv
       for (int e = 0; e < 8; ++e) w[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
       stg32(dst + c0, w, wide);
       if (xr) {
-        uint32_t xw[8];
-        ldg32(xr + c0, xw, wide);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          part = fmaf(f[2 * e], __uint_as_float(xw[e] << 16), part);
-          part = fmaf(f[2 * e + 1], __uint_as_float(xw[e] & 0xFFFF0000u), part);
+          part = fmaf(f[2 * e], __uint_as_float(xw[c0 / 16][e] << 16), part);
+          part = fmaf(f[2 * e + 1], __uint_as_float(xw[c0 / 16][e] & 0xFFFF0000u), part);
         }
       }
     }
@@ -451,12 +454,12 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       } else if constexpr (rev) {
         const bool second = cpart == 1;
         const float* add = second ? a.o2_add : a.o1_add;
-        part = store_row<64>(tl + (second ? C::T_A2 : C::T_A1), row_ok, (__nv_bfloat16*)(second ? a.o2 : a.o1) + grow * D,
+        part = store_row<64, 16>(tl + (second ? C::T_A2 : C::T_A1), row_ok, (__nv_bfloat16*)(second ? a.o2 : a.o1) + grow * D,
                              add ? add + grow * D : nullptr, dots_here ? (const __nv_bfloat16*)a.x + grow * D : nullptr, 1.f);
       } else {
         const int cc = cpart * 32;
         const size_t orow = FWD ? out_row(head, row_ok ? row : 0, a.nrows, a.o_heads) : grow;
-        part = store_row<32>(tl + C::T_A1 + cc, row_ok, (__nv_bfloat16*)a.o1 + orow * D + cc,
+        part = store_row<32, 16>(tl + C::T_A1 + cc, row_ok, (__nv_bfloat16*)a.o1 + orow * D + cc,
                              a.o1_add ? a.o1_add + grow * D + cc : nullptr,
                              dots_here ? (const __nv_bfloat16*)a.x + grow * D + cc : nullptr, scale);
         if (FWD && cpart == 0 && row_ok) a.den_out[grow] = rowsum;

@@ -529,8 +529,10 @@ __device__ __forceinline__ ulonglong2 lds_v2(uint32_t saddr) {
 
 // One thread's accumulator row segment (NC fp32 columns from TMEM column tcol) -> bf16 global
 // row: (accumulator * pre + optional fp32 addend) * scale; returns the dot product of what was
-// stored (before rounding) with the x row when wanted.
-template <int NC>
+// stored (before rounding) with the x row when wanted.  The global reads of AHEAD columns are under way together and
+// before the accumulator is read (32, or 16 where registers are short: six to eight rows of 32 bytes, each of which had
+// the wait for HBM to itself before).
+template <int NC, int AHEAD = 32>
 __device__ __forceinline__ float store_row(uint32_t taddr, bool row_ok, __nv_bfloat16* dst,
                                            const float* add, const __nv_bfloat16* xr, float scale,
                                            float pre = 1.f) {
@@ -539,24 +541,28 @@ __device__ __forceinline__ float store_row(uint32_t taddr, bool row_ok, __nv_bfl
   // (whole sectors) where the three addresses allow them
   const bool wide = (((uintptr_t)dst | (uintptr_t)add | (uintptr_t)xr) & 31) == 0;
 #pragma unroll
-  for (int c0 = 0; c0 < NC; c0 += 32) {
-    uint32_t ov[32];
-    tmem_ld32(taddr + c0, ov);
-    tmem_wait_ld(ov);
-    if (row_ok) {
+  for (int c0 = 0; c0 < NC; c0 += AHEAD) {
+    uint32_t aw[AHEAD / 8][8], xw[AHEAD / 16][8];
+    if (add && row_ok) {
 #pragma unroll
-      for (int v16 = 0; v16 < 2; ++v16) {
+      for (int h = 0; h < AHEAD / 8; ++h) ldg32(add + c0 + 8 * h, aw[h], wide);
+    }
+    if (xr && row_ok) {
+#pragma unroll
+      for (int h = 0; h < AHEAD / 16; ++h) ldg32(xr + c0 + 16 * h, xw[h], wide);
+    }
+#pragma unroll
+    for (int v16 = 0; v16 < AHEAD / 16; ++v16) {
+      uint32_t ov[16];
+      tmem_ld16(taddr + c0 + 16 * v16, ov);
+      tmem_wait_ld(ov);
+      if (row_ok) {
         float f[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(ov[v16 * 16 + e]) * pre;   // pre scales the accumulator only
+        for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(ov[e]) * pre;   // pre scales the accumulator only
         if (add) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t aw[8];
-            ldg32(add + c0 + 16 * v16 + 8 * h, aw, wide);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[8 * h + e] += __uint_as_float(aw[e]);
-          }
+          for (int e = 0; e < 16; ++e) f[e] += __uint_as_float(aw[2 * v16 + (e >> 3)][e & 7]);
         }
         uint32_t w[8];
 #pragma unroll
@@ -567,12 +573,10 @@ __device__ __forceinline__ float store_row(uint32_t taddr, bool row_ok, __nv_bfl
         }
         stg32(dst + c0 + 16 * v16, w, wide);
         if (xr) {
-          uint32_t xw[8];
-          ldg32(xr + c0 + 16 * v16, xw, wide);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            part = fmaf(f[2 * e], __uint_as_float(xw[e] << 16), part);
-            part = fmaf(f[2 * e + 1], __uint_as_float(xw[e] & 0xFFFF0000u), part);
+            part = fmaf(f[2 * e], __uint_as_float(xw[v16][e] << 16), part);
+            part = fmaf(f[2 * e + 1], __uint_as_float(xw[v16][e] & 0xFFFF0000u), part);
           }
         }
       }
