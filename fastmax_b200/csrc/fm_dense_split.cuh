@@ -1,7 +1,7 @@
 // What the float32 score kernels on the tensor cores share (fm_dense_split.cu, fm_dense_split_rows.cu).
 #pragma once
 
-#include "fm_common.cuh"
+#include "fm_row_walk.cuh"
 #include "fm_sm100.cuh"
 
 namespace fm {
@@ -32,52 +32,7 @@ struct SplitArgs {
 
 constexpr int BM = 128, BN = 64, kComputeWarps = 8;
 
-// The row tiles that a CTA takes one after the other, and their column tiles.
-//   ORDER_LINEAR   head by head (row tiles of about the same length)
-//   ORDER_TILES    causal grids of a few waves: tile by tile over all heads, the longest first, every other round backwards
-//   ORDER_PAIRS    longer causal grids: head by head, so that a head's column tiles stay in L2, the i-th longest row tile
-//                  together with the i-th shortest, so that every CTA gets the same work
-enum { ORDER_LINEAR = 0, ORDER_TILES = 1, ORDER_PAIRS = 2 };
-struct RowWalk {
-  int turn = 0, second = 0, head, r0;   // position; head and first row
-  int tb, j;                            // first column tile and their number
-  int m = 0;                            // row tiles before this one
-  __device__ __forceinline__ static int units(const SplitArgs& a) {
-    return a.heads * (a.order == ORDER_PAIRS ? (a.ntr + 1) / 2 : a.ntr);
-  }
-  __device__ __forceinline__ int unit(const SplitArgs& a) const {
-    const int b = (int)blockIdx.x, g = (int)gridDim.x;
-    return turn * g + (a.order == ORDER_TILES && (turn & 1) ? g - 1 - b : b);
-  }
-  __device__ __forceinline__ bool live(const SplitArgs& a) const { return unit(a) < units(a); }
-  __device__ __forceinline__ void open(const SplitArgs& a) {
-    const int u = unit(a), per = a.order == ORDER_PAIRS ? (a.ntr + 1) / 2 : a.ntr;
-    head = a.order == ORDER_TILES ? u % a.heads : u / per;
-    int t = a.order == ORDER_TILES ? u / a.heads : u % per;           // 0: the longest
-    if (second) t = a.ntr - 1 - t;
-    r0 = (a.ntr - 1 - t) * BM;
-    int te = (a.ncols + BN - 1) / BN;
-    if (a.mask) te = min(te, (min(r0 + BM - 1, a.nrows - 1) + a.off) / BN + 1);
-    tb = a.chunk > 0 ? (r0 / a.chunk) * (a.chunk / BN) : 0;           // the row tile lies in one chunk (chunk % 256 == 0)
-    j = te - tb;              // at least one: every row sees a column
-  }
-  __device__ __forceinline__ void next(const SplitArgs& a) {
-    ++m;
-    const int per = (a.ntr + 1) / 2, t = unit(a) % per;
-    if (a.order == ORDER_PAIRS && !second && a.ntr - 1 - t != t) {
-      second = 1;
-    } else {
-      second = 0;
-      ++turn;
-    }
-    if (live(a)) open(a);
-  }
-};
-inline int row_order(const fastmax_problem& p, int chunk, long long heads, long long ntr, int ctas_per_sm) {
-  if (!p.mask || heads * ntr <= 148 * ctas_per_sm) return ORDER_LINEAR;
-  if (heads * ntr > 8LL * 148 * ctas_per_sm) return ORDER_PAIRS;
-  return chunk ? ORDER_LINEAR : ORDER_TILES;
-}
+using Rows = RowWalk<SplitArgs, BN, false>;   // of the forward and grad_q
 
 // ---- operands and products ----
 // A tile's part p (0 h, 1 m, 2 l) lies at p * SUB: rows of D bf16, 128 or 64 bytes, swizzled over their whole length.

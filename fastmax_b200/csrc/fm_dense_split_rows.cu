@@ -106,7 +106,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   const uint32_t tmem = *tmem_slot;
 
   // every role walks the same row tiles and counts their column tiles in g
-  RowWalk w;
+  Rows w;
   w.open(a);
   int g = 0;
   bool ok = true;
@@ -194,7 +194,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     // statistics of the next row tile's heads and dvec of its row, asked for early
     stat_t st_q = 0, st_k = 0;
     float dl_next = 0.f;
-    auto ask = [&](const RowWalk& x) {
+    auto ask = [&](const Rows& x) {
       if (a.stat_q) {
         st_q = __ldg(a.stat_q + x.head);
         st_k = __ldg(a.stat_k + x.head / a.ratio);
@@ -289,7 +289,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR_SFREE);
         if (i + 1 == w.j) {          // the row tile's score products are done: the next one's operands take their place
-          RowWalk n = w;
+          Rows n = w;
           n.next(a);
           if (n.live(a)) {
             ask(n);
@@ -385,7 +385,7 @@ int launch_rows(const Ctx& c, const char* name, const void* x, const void* u, co
   if ((rc = split_map<D>(&tz, z, p.bhkv, p.nk, BN))) return rc;
   long long blocks;
   if ((rc = set_sizes(p, p.bh, p.nq, p.nk, &a, &blocks))) return rc;
-  a.order = row_order(p, a.chunk, a.heads, a.ntr, CTAS);
+  a.order = row_order(p, a.heads, a.ntr, CTAS);
   const auto kernel = split_rows_kernel<D, MODE, CTAS>;
   // the compute warps of two CTAs wait for registers that the block must have been launched with
   static const int regs = [&] {
