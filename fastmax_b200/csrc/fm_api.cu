@@ -292,6 +292,7 @@ int fastmax_b200_device_status(int* status, void* stream) {
   if ((rc = first_tc_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = tc_short_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = split_status(&f, (cudaStream_t)stream))) return rc;
+  if (!f && (rc = tc_walk_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = split_rows_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = split_moments_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = readout_status(&f, (cudaStream_t)stream))) return rc;
@@ -308,6 +309,7 @@ int fastmax_b200_device_status_reset(void* stream) {
   if ((rc = tc_dkdv128_status_reset(s))) return rc;
   if ((rc = moments_tc_status_reset(s))) return rc;
   if ((rc = split_status_reset(s))) return rc;
+  if ((rc = tc_walk_status_reset(s))) return rc;
   if ((rc = split_rows_status_reset(s))) return rc;
   if ((rc = split_moments_status_reset(s))) return rc;
   if ((rc = readout_status_reset(s))) return rc;

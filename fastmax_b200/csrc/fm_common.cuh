@@ -185,6 +185,8 @@ int dense_tc_short_forward(const Ctx& c, const void* q, const void* k, const voi
                            void* out, float* den, const ChunkAdd* ca = nullptr, const FirstState* fs = nullptr);
 int tc_short_status(int* out, cudaStream_t stream);
 int tc_short_status_reset(cudaStream_t stream);
+int tc_walk_status(int* out, cudaStream_t stream);
+int tc_walk_status_reset(cudaStream_t stream);
 int tc_wide_status(int* out, cudaStream_t stream);
 int tc_wide_status_reset(cudaStream_t stream);
 // backward for d == 128: grad_q, and grad_k / grad_v in one kernel (fm_dense_tc_dkdv128.cu)

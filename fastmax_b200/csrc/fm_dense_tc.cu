@@ -476,14 +476,14 @@ int make_map(CUtensorMap* m, const void* base, int heads, int n, int box_rows, i
 }  // namespace
 
 static int map_boxes(CUtensorMap* m, const void* base, size_t mats, size_t rows, int d, int box_rows, int box_cols,
-                     CUtensorMapSwizzle swizzle) {
+                     CUtensorMapSwizzle swizzle, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, int es = 2) {
   EncodeFn enc = encode_fn();
   if (!enc) return fail(FASTMAX_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t gdim[3] = {(cuuint64_t)d, (cuuint64_t)rows, (cuuint64_t)mats};
-  cuuint64_t gstr[2] = {(cuuint64_t)d * 2, (cuuint64_t)rows * d * 2};
+  cuuint64_t gstr[2] = {(cuuint64_t)d * es, (cuuint64_t)rows * d * es};
   cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstr, box, estr,
+  CUresult r = enc(m, type, 3, const_cast<void*>(base), gdim, gstr, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(FASTMAX_E_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
@@ -491,6 +491,9 @@ static int map_boxes(CUtensorMap* m, const void* base, size_t mats, size_t rows,
 }
 int tma_map_bf16(CUtensorMap* m, const void* base, size_t mats, size_t rows, int d, int box_rows) {
   return map_boxes(m, base, mats, rows, d, box_rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+int tma_map_f32_rows(CUtensorMap* m, const float* base, size_t mats, size_t rows) {
+  return map_boxes(m, base, mats, rows, 64, 128, 32, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4);
 }
 int tma_map_bf16_half(CUtensorMap* m, const void* base, size_t mats, size_t rows, int d, int box_rows) {
   return map_boxes(m, base, mats, rows, d, box_rows, 32, CU_TENSOR_MAP_SWIZZLE_64B);

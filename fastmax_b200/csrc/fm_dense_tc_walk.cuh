@@ -1,0 +1,38 @@
+// Arguments of the score kernels that walk row tiles (fm_dense_tc_walk.cu).
+#pragma once
+
+#include <cuda.h>
+
+#include "fm_common.cuh"
+
+namespace fm {
+namespace walk {
+
+enum { MODE_FWD = 0, MODE_DKDV = 1 };
+
+struct WalkArgs {
+  void* o;               // (heads, nrows, 64) bf16: out, or grad_k
+  void* o2;              // DKDV: grad_v
+  float* den_out;        // FWD: (heads, nrows) row sums
+  const float* den_add;  // FWD: added to the row sum (may be null)
+  const float* o_add;    // fp32 rows added before the division / rounding (may be null)
+  const float* o2_add;
+  const void* x;         // row operand in global memory (normalisation dots)
+  const float* dvec;     // (heads, nq)
+  float* dots;           // per head sum of o . x, or null
+  const stat_t* stat_q;
+  const stat_t* stat_k;
+  int heads, nrows, ncols, off, mask, ntr, chunk, ratio, order;   // see RowWalk
+  float a0, a1, a2, lim;
+  int o_heads;           // FWD: > 0 writes out as (batch, nrows, o_heads, 64)
+};
+
+}  // namespace walk
+
+// Boxes of 128 rows x 32 of a (mats, rows, 64) float32 array, 128-byte swizzle (fm_dense_tc.cu)
+int tma_map_f32_rows(CUtensorMap* m, const float* base, size_t mats, size_t rows);
+
+int dense_tc_walk_forward(const Ctx& c, const void* q, const void* k, const void* v, const walk::WalkArgs& a);
+int dense_tc_walk_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, const walk::WalkArgs& a);
+
+}  // namespace fm

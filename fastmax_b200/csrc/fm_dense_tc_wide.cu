@@ -1,6 +1,7 @@
 // Score form on the tcgen05 tensor cores, bf16, head dimension 64: one CTA owns ONE
 // 128-row tile and walks column tiles that alternate between two groups of compute warps
-// ("ping-pong"), each with its own S / W / E / P regions in TMEM.
+// ("ping-pong"), each with its own S / W / E / P regions in TMEM.  fm_dense_tc_walk.cu has the same loop in CTAs that go on
+// from one row tile to the next; walk_rows() and short_rows() below say which rows come here.
 //
 //   MODE_DQ    grad_q:  rows = queries (x = q, u = gs), columns = keys (y = k, z = v)
 //              E = f'(x.y) (u.z - dvec_row);          grad_q += E Y
@@ -33,6 +34,7 @@
 #include <type_traits>
 
 #include "fm_common.cuh"
+#include "fm_dense_tc_walk.cuh"
 #include "fm_sm100.cuh"
 
 namespace fm {
@@ -628,8 +630,9 @@ bool dense_tc_wide_supports(const fastmax_problem& p) {
 // causal columns, 211 / 224 at 2048, 668 / 619 at 4096, unmasked 217 / 223 at 1600, 320 / 301 at 2048; grad_q 254 / 291
 // at 2048 causal, 392 / 406 at 2048 unmasked, 826 / 820 at 4096; grad_k + grad_v 179 / 187 at 1200 causal, 271 / 267 at
 // 1600, 264 / 277 at 1200 unmasked, 435 / 410 at 1600 -- but 845 / 921 in the moment family's chunks of 2048, whose
-// epilogues read fp32 rows too.  So the line is drawn at the mean number of columns a row tile walks.  With no more
-// row tiles than SMs there is nothing to overlap and the wide kernels' larger tiles win (8 heads of 1024: 16.3 / 12.4).
+// epilogues read fp32 rows too (of which chunks of grad_q and of grouped heads are left; walk_rows takes the others).
+// So the line is drawn at the mean number of columns a row tile walks.  With no more row tiles than SMs there is nothing
+// to overlap and the wide kernels' larger tiles win (8 heads of 1024: 16.3 / 12.4).
 static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
   const bool chunked = ca && ca->chunk > 0;
   const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
@@ -637,6 +640,38 @@ static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
   const int seen = chunked ? ca->chunk / 2 : (p.mask ? cols / 2 : cols);
   const int most[3] = {1500, 1900, chunked ? 1100 : (p.mask ? 700 : 1300)};
   return seen * (pass == 2 ? p.bh / p.bhkv : 1) <= most[pass];
+}
+
+// Whether the kernels that walk row tiles serve a pass (0 forward, 2 grad_k + grad_v): they cover the ends of a row tile and
+// keep the wide loop's pace, but deal their row tiles out beforehand, so a nearly empty last round costs a whole row tile, and
+// below some columns to a row tile the short kernels' two CTAs hide the ends better.  us, what served it before / walking:
+//   chunks        forward 121 / 111 at 4096 row tiles in chunks of 256, 241 / 190 of 2048, 375 / 302 of 4096, 20.8 / 18.7 at
+//                 320 row tiles of 256; grad_k + grad_v 205 / 166, 449 / 386, but 630 / 642 of 4096, and 29.1 / 24.9; no gain
+//                 of the forward at 200 row tiles
+//   forward       causal, 2048 to 2200 row tiles: 61.8 / 76 at 400 columns, 72.2 / 66.0 at 1000, 170 / 163 at 4600, but
+//                 301 / 313 (3008 row tiles) at 6000; 208 / 176 (4096) at 2000; 480 to 1200 row tiles: 47.6 / 49.5 to
+//                 37.2 / 35.3 at 1000, 45.4 / 41.4 at 1500, 33.2 / 33.2 at 3600; 320 at most: 16.6 / 14.7 at 600 columns,
+//                 26.8 / 18.8 at 2200, 22.9 / 27.0 at 4000.  Unmasked: 47.4 / 45.5 at 450, 94.5 / 82.2 at 1600, 158 / 152
+//                 at 3600, and nothing at two rounds
+//   grad_k+grad_v causal, at most 320 row tiles: 25.0 / 20.9 at 600 columns, 33.2 / 22.9 at 1100, 31.2 / 31.2 (all 320) at
+//                 1000, but 29.1 / 31.1 at 1500; more row tiles: 31.2 / 33.2.  Unmasked: 78.1 / 72.0 at 300, 152 / 134 at
+//                 1200, 158 / 164 at 1600, and nothing at two rounds
+static bool walk_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
+  const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
+  const long long tiles = (long long)p.bh * ((rows + BM - 1) / BM);
+  if (p.bh != p.bhkv || tiles <= 148) return false;
+  if (ca && ca->chunk > 0) return tiles > 2 * 148 && ca->chunk <= (pass == 2 ? 2048 : 4096);
+  const int seen = p.mask ? cols / 2 : cols;
+  if (!p.mask) return tiles > 2 * 148 && (pass == 2 ? seen >= 300 && seen <= 1300 : seen >= 450 && seen <= 3000);
+  if (tiles <= 320) return seen >= 300 && seen <= (pass == 2 ? 550 : 1500);
+  return pass == 0 && seen >= 500 && seen <= (tiles > 8 * 148 ? 2500 : 1900);
+}
+static walk::WalkArgs walk_args(const fastmax_problem& p, const stat_t* stats, const ChunkAdd* ca) {
+  walk::WalkArgs a = {};
+  a.stat_q = p.normalize ? stats : nullptr;
+  a.stat_k = p.normalize ? stats + p.bh : nullptr;
+  a.chunk = ca ? ca->chunk : 0;
+  return a;
 }
 
 int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* gs,
@@ -662,6 +697,16 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
   if (short_rows(p, ca, 1)) rc = dense_tc_short_dq(c, q, k, v, gs, dvec, stats, dots, grad_q, ca);
   else rc = launch_wide<MODE_DQ>(c, "fm_dense_tc_dq", q, gs, k, v, p.nq, p.nk, a);
   if (rc) return rc;
+  if (walk_rows(p, ca, 2)) {
+    walk::WalkArgs b = walk_args(p, stats, ca);
+    b.dvec = dvec;
+    b.o = grad_k;
+    b.o2 = grad_v;
+    b.dots = p.normalize ? dots + p.bh : nullptr;
+    b.o_add = ca ? ca->gk_add : nullptr;
+    b.o2_add = ca ? ca->gv_add : nullptr;
+    return dense_tc_walk_dkdv(c, k, v, q, gs, b);
+  }
   if (short_rows(p, ca, 2)) return dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, ca);
   // grad_k and grad_v: rows = keys, columns = queries
   a.o = grad_k;
@@ -675,6 +720,14 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
 int dense_tc_wide_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                           void* out, float* den, const ChunkAdd* ca) {
   const fastmax_problem& p = c.p;
+  if (walk_rows(p, ca, 0)) {
+    walk::WalkArgs a = walk_args(p, stats, ca);
+    a.o = out;
+    a.den_out = den;
+    a.o_heads = c.out_heads;
+    if (ca) { a.o_add = ca->out_add; a.den_add = ca->den_add; }
+    return dense_tc_walk_forward(c, q, k, v, a);
+  }
   if (short_rows(p, ca, 0)) return dense_tc_short_forward(c, q, k, v, stats, out, den, ca);
   WArgs a = {};
   a.stat_q = p.normalize ? stats : nullptr;
