@@ -23,15 +23,18 @@
 // running step (0 between calls), 0} per key/value head.  S2 is symmetric in (a, b), so only its
 // upper triangle of tiles is computed; every result is written to both of its rows.
 //
-// Three kernels:
+// The kernels:
 //   step_kernel    one token and its read-out: bound by the state's traffic with many heads, by a chain of latencies with
 //                  few.  The lower triangle is written but never read: 4 F (d+1) x (1 + 0.56) bytes at d = 64.  Measured, us,
-//                  events around a launch included, p = 2: 1024 heads, d = 64: 353 for 1.73 GB = 4.9 TB/s in bf16 and float32; 8
-//                  key/value heads of 4 query heads 12.8 (16.8 when the queries were asked for after the update, the
-//                  arriving CTA fenced its 24 KB of state and the last one read the queries' shares in turn); 4 heads, float32,
-//                  10.7 (11.6); 128 heads, d = 128: bf16 336 (353), float32 326 (357).  1024 heads: no change (355).
-//                  Two other arrangements for many heads were slower: several groups of blocks to a CTA 397 us, five CTAs
-//                  to an SM 377.
+//                  events around a launch included, p = 2: 1024 heads, d = 64: 312 for 1.73 GB = 5.5 TB/s (352 when every thread
+//                  fenced and each CTA waited for its arrival, 330 with one thread's fence); 8 key/value heads of 4 query heads
+//                  12.3 (12.8, and 16.8 when the queries were asked for after the update, the arriving CTA fenced its 24 KB of
+//                  state and the last one read the queries' shares in turn); 4 heads, float32, 10.5 (11.6); 128 heads, d = 128:
+//                  305 (334).  The same bytes in 2 KB runs, without the arithmetic: 258.  Other arrangements for 1024 heads:
+//                  several groups of blocks to a CTA 397, five CTAs to an SM 377 (both before the above); tiles by bulk copies
+//                  through shared memory, CTAs as here 366 / 291 (one kernel / without the sums; d = 128 319 / 264), persistent
+//                  with 1 to 4 CTAs an SM 338 to 403.
+//   sum_kernel     the heads' sums, where step_kernel leaves them out (kSharesFrom).
 //   few_kernel     the same update for a few tokens of a prompt.
 //   append_kernel  many tokens (prompt), float32 or d = 32: bound by the FMA pipe; see there.  bf16 prompts of
 //                  d 64 and 128 go to the tensor cores (fm_decode_tc.cu).
@@ -215,7 +218,8 @@ template <int D> struct Block {
 // One token per head and its read-out.  A CTA takes one group of RPB blocks of its head and leaves their share of the
 // read-out in scratch[query head][CTA][column]; the CTA of a head that arrives last (a counter in the head's header) adds
 // the shares in CTA order, divides and writes the output row.
-template <typename T, int D>
+// SHARES: that is all; sum_kernel does the rest.
+template <typename T, int D, bool SHARES>
 __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_kernel(const DecArgs a, const T* __restrict__ q,
                                                                   const T* __restrict__ k, const T* __restrict__ v,
                                                                   float* __restrict__ state, float* __restrict__ scratch,
@@ -299,9 +303,14 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
       __stcg(scratch + ((qh + g) * gridDim.x + blockIdx.x) * C::DV + cc, tot);
     }
   }
-  __threadfence();
+  if constexpr (SHARES) {
+    blk.store();
+    return;
+  }
   __syncthreads();
-  if (tid == 0) {
+  // one thread's fence, for all of the CTA: the others go on to their stores.  One in the last warp, which has fewest
+  if (tid == C::THREADS - 1) {
+    __threadfence();
     const int before = atomicAdd(reinterpret_cast<int*>(hs + 2), 1);
     s_last = before == (int)gridDim.x - 1;
   }
@@ -348,6 +357,46 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
       stf(out + qh * D + x, num / den);
     }
     __syncthreads();
+  }
+}
+
+// The shares that step_kernel's CTAs left in the scratch, in their order: a CTA per query row, which it divides and writes; the
+// first one of a key/value head also counts the token.
+template <typename T, int D>
+__global__ void __launch_bounds__(DecCfg<D>::THREADS) sum_kernel(const DecArgs a, int shares, const T* __restrict__ k,
+                                                                 float* __restrict__ state, const float* __restrict__ scratch,
+                                                                 T* __restrict__ out) {
+  typedef DecCfg<D> C;
+  __shared__ float red[C::RPB][C::DV];
+  const int tid = threadIdx.x, r = tid / C::DV, c = tid - r * C::DV, lane = tid & 31;
+  const int qh = blockIdx.x, head = qh / a.ratio;
+  const float* src = scratch + (long long)qh * shares * C::DV + c;
+  float tot = 0.0f;
+#pragma unroll 10
+  for (int b = r; b < shares; b += C::RPB) tot += __ldcg(src + (long long)b * C::DV);
+  if (qh % a.ratio == 0 && tid < 32) {
+    float n2 = 0.0f;
+#pragma unroll
+    for (int e = lane; e < D; e += 32) {
+      const float x = ldf(k + (long long)head * D + e);
+      n2 = fmaf(x, x, n2);
+    }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, m);
+    if (lane == 0) {
+      float* hs = state + head * a.head_floats;
+      hs[0] = fmaxf(hs[0], n2);
+      // the token count is an integer bit pattern in the float slot: exact past 2^24 tokens
+      hs[1] = __int_as_float(__float_as_int(hs[1]) + 1);
+    }
+  }
+  red[r][c] = tot;
+  __syncthreads();
+  if (tid < D) {
+    float num = 0.0f, den = 0.0f;
+#pragma unroll
+    for (int rr = 0; rr < C::RPB; ++rr) { num += red[rr][tid]; den += red[rr][D]; }
+    stf(out + (long long)qh * D + tid, num / den);
   }
 }
 
@@ -590,6 +639,12 @@ long long append_min(const fastmax_problem& p) {
   return p.p == 1 ? (tc ? 14 : 24) : (tc ? 28 : 40);
 }
 
+// From how many CTAs on a step leaves the heads' sums to sum_kernel: a CTA then ends without a fence and an atomic's way to
+// memory and back, but the sums cost a kernel that starts when everything has been written, 9 to 13 us.  Measured, us a step, one
+// kernel / two: d = 64 88.1 / 88.3 at 6400 CTAs (256 heads), 330 / 312 at 25600; d = 128 165.6 / 160.4 at 8896 (64 heads), 321 /
+// 305 at 17792, 49.9 / 51.3 at 2224; d = 32 11.7 / 11.5 at 512 (128 heads), 29.5 / 26.8 at 2048, 117 / 101 at 8192.
+template <int D> constexpr long long kSharesFrom = D == 32 ? 2048 : 8192;
+
 template <typename T, int D, bool READ>
 int launch_decode(const fastmax_problem& p, const void* q, const void* k, const void* v, long long n_new,
                   float* state, float* scratch, void* out, cudaStream_t st) {
@@ -606,11 +661,20 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
     }
   } else {
     const dim3 grid(DecCfg<D>::ctas(p.p), p.bhkv);
-    if constexpr (READ)
-      FM_LAUNCH("fm_decode_step", st,
-                (step_kernel<T, D><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
-                                                                        scratch, (T*)out)));
-    else
+    if constexpr (READ) {
+      if (grid.x * (long long)p.bhkv >= kSharesFrom<D>) {
+        FM_LAUNCH("fm_decode_step", st,
+                  (step_kernel<T, D, true><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
+                                                                                scratch, (T*)out)));
+        FM_CUDA_TRY(cudaGetLastError());
+        FM_LAUNCH("fm_decode_sum", st,
+                  (sum_kernel<T, D><<<p.bh, DecCfg<D>::THREADS, 0, st>>>(a, (int)grid.x, (const T*)k, state, scratch, (T*)out)));
+      } else {
+        FM_LAUNCH("fm_decode_step", st,
+                  (step_kernel<T, D, false><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
+                                                                                 scratch, (T*)out)));
+      }
+    } else
       FM_LAUNCH("fm_decode_append", st,
                 (few_kernel<T, D><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)k, (const T*)v, state)));
   }

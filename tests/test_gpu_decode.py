@@ -92,3 +92,23 @@ def test_steps_match_the_oracle_recurrence_with_other_coefficients(p):
         got = st.step(q[:, sl].contiguous().cuda(), k[:, sl].contiguous().cuda(), v[:, sl].contiguous().cuda())
         err = float((got.double().cpu() - want).abs().max() / want.abs().max())
         assert err < TOL[torch.float32], (t, err)
+
+
+@pytest.mark.parametrize("heads,ratio,d", [(512, 1, 32), (513, 5, 32), (328, 1, 64), (59, 4, 128)])
+def test_steps_of_many_heads_equal_those_of_few(heads, ratio, d):
+    """From some number of CTAs on a second kernel adds up a step's shares, in the order of the first one's last CTA: the state
+    must be the same to the bit, the rows up to the order of at most 139 additions per column."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    mk = lambda n: torch.randn(n, 1, d, generator=g, device="cuda").bfloat16()  # noqa: E731
+    whole = FastmaxDecodeState(heads * ratio, heads, d, device="cuda:0")
+    cut = heads // 3
+    parts = [FastmaxDecodeState(n * ratio, n, d, device="cuda:0") for n in (cut, heads - 2 * cut, cut)]
+    for _ in range(3):
+        q, k, v = mk(heads * ratio), mk(heads), mk(heads)
+        out, lo = whole.step(q, k, v), 0
+        for p in parts:
+            n = p.bhkv
+            want = p.step(q[lo * ratio:(lo + n) * ratio].contiguous(), k[lo:lo + n].contiguous(), v[lo:lo + n].contiguous())
+            assert torch.allclose(out[lo * ratio:(lo + n) * ratio].float(), want.float(), rtol=2 ** -7, atol=1e-4)
+            lo += n
+    assert torch.equal(whole.state.view(-1), torch.cat([p.state.view(-1) for p in parts]))
