@@ -183,6 +183,9 @@ int dense_tc_short_dkdv(const Ctx& c, const void* q, const void* k, const void* 
                         const FirstState* fs = nullptr);
 int dense_tc_short_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                            void* out, float* den, const ChunkAdd* ca = nullptr, const FirstState* fs = nullptr);
+// grad_k and grad_v of the first-order chunks, by those kernels or the ones that walk row tiles
+int dense_tc_first_dkdv(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
+                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd& ca, const FirstState& fs);
 int tc_short_status(int* out, cudaStream_t stream);
 int tc_short_status_reset(cudaStream_t stream);
 int tc_walk_status(int* out, cudaStream_t stream);

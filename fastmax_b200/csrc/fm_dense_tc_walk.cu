@@ -8,7 +8,9 @@
 // tile are loaded meanwhile, its first scores follow the last ones of this, the float32 rows that a chunk adds to its result come
 // by TMA while the columns pass, and the forward, which has room for two row tiles' accumulators, reads and stores a row tile's
 // result when the next one's columns are done.  32 heads of 32768 in chunks of 2048, us, short-row kernels / this: forward
-// 469 / 377, grad_k + grad_v 874 / 787; 240 heads of 2000, causal: forward 208 / 176.  What bounds it is the loop: TMEM loads,
+// 469 / 361, grad_k + grad_v 874 / 787; 240 heads of 2000, causal: forward 208 / 176.  A second buffer for the row operands and
+// shorter rings pay in the forward (32 heads of 16384 in chunks of 2048 189 / 181, 160 heads of 1600 86 / 83) and not in DKDV
+// (387 / 394).  What bounds it is the loop: TMEM loads,
 // polynomial and TMEM stores of sixteen warps.  grad_q the same way was slower than its short kernel (0.78 to 0.98 of it):
 // its S, W, E and two accumulators leave one set of each, so the warps wait for every tile's scores.
 //
@@ -21,6 +23,11 @@
 //   DKDV     S[2] 0 | W[2] 128 | E[2] 256 (bf16 pairs) | P[2] 320 | accumulators 384, 448
 //   forward  three sets of 128 score columns at 0, 128, 256 (tile g in set g % 3), P over the S columns it came from;
 //            accumulators of alternate row tiles 384, 448
+// FIRST (DKDV): the first-order moment family's chunks, as in fm_dense_tc_short.cu: what a chunk's keys take from all tokens
+// after it is one more product with the d x d state before the chunk's own, and its vectors are added at the end.  256 heads of
+// 4096 in chunks of 512, us: 365 / 351; 64 of 2000 57.8 / 53.8; 80 of 600 31 / 27.  The forward of these chunks, tried in the
+// same way, was slower than the short kernel's (232 / 247): its row tiles have 2.5 column
+// tiles.
 // All waits are bounded; a wait that gives up records a status and the CTA winds down.
 #include <type_traits>
 
@@ -44,7 +51,7 @@ constexpr int kRegsLaunch = 96, kRegsCompute = 104, kRegsOther = 64;
 static_assert(32 * kComputeWarps * kRegsCompute + (kThreads - 32 * kComputeWarps) * kRegsOther <= kThreads * kRegsLaunch,
               "the shares of the warpgroups add up to what the block is launched with");
 
-template <int MODE>
+template <int MODE, bool FIRST>
 struct WK {
   static constexpr bool FWD = MODE == MODE_FWD, FUSED = MODE == MODE_DKDV;
   static constexpr int BN = FWD ? 128 : 64;                  // columns of a tile
@@ -52,21 +59,26 @@ struct WK {
   static constexpr int ROWS = (FWD ? 1 : 2) * ROW_TILE;
   // Rings of Y and Z tiles.  DKDV: an even number, so that each barrier is waited on by one of the two groups' issuers, phase
   // after phase.
-  static constexpr int NY = FWD ? 4 : 6, NZ = 6;
-  static constexpr int OFF_Y = ROWS, OFF_Z = OFF_Y + NY * COL_TILE;
+  static constexpr int NX = FUSED && !FIRST ? 1 : 2, NY = FWD ? 4 : 6, NZ = FWD ? 5 : 6;
+  static constexpr int OFF_Y = NX * ROWS, OFF_Z = OFF_Y + NY * COL_TILE;
   static constexpr int ADD_HALF = 128 * 128;                 // 128 rows of 32 floats
   static constexpr int OFF_ADD = OFF_Z + NZ * COL_TILE, ADDS = (FUSED ? 2 : 1) * 2 * ADD_HALF;
-  static constexpr int OFF_VEC = OFF_ADD + ADDS;             // per compute warp 2 x 32 floats; FWD: row sums, [4][4][128]
+  // FIRST, in place of rows to add: the state copy of the row tile's chunk, and of eight row tiles the state's normaliser column
+  // (64) and constant row (65)
+  static constexpr int S1_TILE = 8192, OFF_S1 = OFF_ADD, OFF_STV = OFF_S1 + NX * S1_TILE, STV = 132 * 4;
+  // per compute warp 2 x 32 floats; FWD: row sums, [4][4][128]
+  static constexpr int OFF_VEC = FIRST ? OFF_STV + 8 * STV : OFF_ADD + ADDS;
   static constexpr int OFF_ITEM = OFF_VEC + (FWD ? 4 * 4 * 128 : kComputeWarps * 64) * 4;   // eight row tiles (Item)
   static constexpr int OFF_BAR = OFF_ITEM + 8 * 32;
-  static constexpr int NBAR = 13 + 2 * NY + 2 * NZ + 9;
+  static constexpr int NBAR = 15 + 2 * NY + 2 * NZ + 9;
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_TMEM + 16 + 1024;
   static_assert(SMEM <= 227 * 1024, "shared memory");
   static constexpr int T_S = 0, T_W = 128, T_E = 256, T_P = 320, T_A = 384, SETS = 3, SET_COLS = 128;
   static constexpr int ACCS = FUSED ? 1 : 2;                 // row tiles whose accumulators there is room for
   static constexpr int FC = FUSED ? 32 : 16;                 // accumulator columns that a warp stores
-  static constexpr int X_READERS = (FWD ? 1 : 2) + kComputeWarps;   // issuers; the compute warps have seen the row tile
+  // readers of a row tile's operands: issuers; the compute warps have seen which row tile it is
+  static constexpr int X_READERS = (FWD ? 1 : 2) + (FIRST ? 1 : 0) + kComputeWarps;
 };
 
 // A row tile as the producer hands it to the compute warps: also the coefficients of its head's polynomial.
@@ -80,12 +92,12 @@ __device__ __forceinline__ void report(int code) { atomicCAS(&g_walk_status, 0, 
 // SQ (DKDV, a2 > 0): the polynomial in completed-square form, f(s) = A2 ((s + b)^2 + c), f'(s) = 2 A2 (s + b), with
 // b = A1 / (2 A2), c = A0 / A2 - b^2: a pair of scores costs t = s + b, P' = t t + c, E' = t (w - dvec), four packed operations
 // instead of five; A2 (grad_v) and 2 A2 (grad_k) multiply the accumulators in the end.
-template <int MODE, bool SQ>
+template <int MODE, bool SQ, bool FIRST>
 __global__ void __launch_bounds__(kThreads, 1)
 walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
             const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmZ,
             const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const WalkArgs a) {
-  using C = WK<MODE>;
+  using C = WK<MODE, FIRST>;
   constexpr bool FWD = C::FWD, FUSED = C::FUSED, rev = FUSED;
   constexpr int BN = C::BN, HB = BN / 2;         // HB: columns of one compute warp = packed columns of a group
   using Rows = RowWalk<WalkArgs, BN, rev>;
@@ -93,19 +105,22 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bar0 = sbase + C::OFF_BAR;
-  // barrier map: x | x free | rows to add | products of a row tile done[2] | accumulators read[2] | row sums[4] | y_full |
+  // barrier map: x[2] | x free[2] | rows to add | products of a row tile done[2] | accumulators read[2] | row sums[4] | y_full |
   // y_empty | z_full | z_empty | s_full[2] | s_free[2] | p_full[2] | pv_done[2]; forward: s_full[set] | p_full[set] |
   // set_free[set]
   constexpr int NY = C::NY, NZ = C::NZ;
-  const uint32_t BAR_X = bar0, BAR_XE = bar0 + 8, BAR_ADD = bar0 + 16;
-  auto BAR_DN = [&](int b) { return bar0 + 8u * (3 + b); };
-  auto BAR_AF = [&](int b) { return bar0 + 8u * (5 + b); };
-  auto BAR_RS = [&](int b) { return bar0 + 8u * (7 + b); };
-  auto BAR_YF = [&](int s) { return bar0 + 8u * (11 + s); };
-  auto BAR_YE = [&](int s) { return bar0 + 8u * (11 + NY + s); };
-  auto BAR_ZF = [&](int s) { return bar0 + 8u * (11 + 2 * NY + s); };
-  auto BAR_ZE = [&](int s) { return bar0 + 8u * (11 + 2 * NY + NZ + s); };
-  const uint32_t bar1 = bar0 + 8u * (11 + 2 * NY + 2 * NZ);
+  auto BAR_X = [&](int m) { return bar0 + 8u * (m % C::NX); };
+  auto BAR_XE = [&](int m) { return bar0 + 8u * (2 + m % C::NX); };
+  auto XPHASE = [&](int m) { return (uint32_t)(m / C::NX & 1); };
+  const uint32_t BAR_ADD = bar0 + 32;
+  auto BAR_DN = [&](int b) { return bar0 + 8u * (5 + b); };
+  auto BAR_AF = [&](int b) { return bar0 + 8u * (7 + b); };
+  auto BAR_RS = [&](int b) { return bar0 + 8u * (9 + b); };
+  auto BAR_YF = [&](int s) { return bar0 + 8u * (13 + s); };
+  auto BAR_YE = [&](int s) { return bar0 + 8u * (13 + NY + s); };
+  auto BAR_ZF = [&](int s) { return bar0 + 8u * (13 + 2 * NY + s); };
+  auto BAR_ZE = [&](int s) { return bar0 + 8u * (13 + 2 * NY + NZ + s); };
+  const uint32_t bar1 = bar0 + 8u * (13 + 2 * NY + 2 * NZ);
   auto BAR_S = [&](int q) { return bar1 + 8u * q; };
   auto BAR_SFREE = [&](int q) { return bar1 + 8u * (2 + q); };
   auto BAR_P = [&](int q) { return bar1 + 8u * (4 + q); };
@@ -117,8 +132,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    mbar_init(BAR_X, 1);
-    mbar_init(BAR_XE, C::X_READERS);
+    for (int b = 0; b < C::NX; ++b) { mbar_init(BAR_X(b), 1); mbar_init(BAR_XE(b), C::X_READERS); }
     mbar_init(BAR_ADD, 1);
     for (int b = 0; b < 2; ++b) { mbar_init(BAR_DN(b), 1); mbar_init(BAR_AF(b), kComputeWarps); }
     for (int b = 0; b < 4; ++b) mbar_init(BAR_RS(b), kComputeWarps);
@@ -147,6 +161,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   const uint32_t tmem = *tmem_slot;
 
   // every role walks the same row tiles; g counts their column tiles
+  auto has_state = [&](int r0) { return FIRST && r0 / a.chunk != a.zero_chunk; };
   Rows w;
   w.open(a);
   int g = 0;
@@ -175,16 +190,36 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         st_k = __ldg(a.stat_k + head);
       };
       if (w.live(a)) ask(w.head);
+      // FIRST: the state's vectors, asked for with the row tile
+      auto vectors = [&](int m, int r0, int head) {
+        const float* st = a.st + (size_t)(head * a.nchunk + r0 / a.chunk) * (D + 1) * a.dvp;
+        float x[5];
+        const bool some = has_state(r0);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          const int e = lane + 32 * i;
+          x[i] = !some || e > 128 ? 0.f : (e < 64 ? __ldg(st + (size_t)e * a.dvp + D) : __ldg(st + (size_t)D * a.dvp + (e - 64)));
+        }
+        float* to = (float*)(smem + C::OFF_STV + (m & 7) * C::STV);
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+          if (lane + 32 * i <= 128) to[lane + 32 * i] = x[i];
+        __syncwarp();
+      };
       int last_r0 = 0, last_head = 0;
       for (; ok && w.live(a); w.next(a)) {
         const float c = a.stat_q ? stat_scale(&st_q, 0, a.lim) * stat_scale(&st_k, 0, a.lim) : 1.f;
-        if (!mbar_wait(BAR_XE, (uint32_t)((w.m & 1) ^ 1))) { report(1); break; }
+        if (!mbar_wait(BAR_XE(w.m), XPHASE(w.m) ^ 1u)) { report(1); break; }
+        if constexpr (FIRST) vectors(w.m, w.r0, w.head);
         if (lane == 0) {
           const Item it = {w.head, w.r0, w.tb, w.j, a.a1 * c, a.a2 * c * c};
           *(Item*)(smem + C::OFF_ITEM + (w.m & 7) * 32) = it;
-          mbar_expect_tx(BAR_X, C::ROWS);
-          tma_load_3d(sbase, &tmX, BAR_X, 0, w.r0, w.head);
-          if (!FWD) tma_load_3d(sbase + ROW_TILE, &tmU, BAR_X, 0, w.r0, w.head);
+          const uint32_t bar = BAR_X(w.m), to = sbase + w.m % C::NX * C::ROWS;
+          mbar_expect_tx(bar, C::ROWS + (has_state(w.r0) ? C::S1_TILE : 0));
+          if (has_state(w.r0))
+            tma_load_3d(sbase + C::OFF_S1 + w.m % C::NX * C::S1_TILE, &tmA, bar, 0, 0, w.head * a.nchunk + w.r0 / a.chunk);
+          tma_load_3d(to, &tmX, bar, 0, w.r0, w.head);
+          if (!FWD) tma_load_3d(to + ROW_TILE, &tmU, bar, 0, w.r0, w.head);
         }
         {
           Rows x = w;
@@ -216,9 +251,9 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         last_head = w.head;
       }
       // no more row tiles
-      if (ok && mbar_wait(BAR_XE, (uint32_t)((w.m & 1) ^ 1)) && lane == 0) {
+      if (ok && mbar_wait(BAR_XE(w.m), XPHASE(w.m) ^ 1u) && lane == 0) {
         ((Item*)(smem + C::OFF_ITEM + (w.m & 7) * 32))->j = 0;
-        mbar_arrive(BAR_X);
+        mbar_arrive(BAR_X(w.m));
       }
       __syncwarp();
       if (ok && FWD && w.m > 0) load_add(w.m - 1, last_r0, last_head);
@@ -238,10 +273,10 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       // ================= issuers of the S / W products (whole warp, one elected lane issues) =================
       constexpr uint32_t idescS = idesc_bf16(128, BN, 0, 0);
       const uint32_t y_k = desc_lo(sbase + C::OFF_Y, 16), z_k = desc_lo(sbase + C::OFF_Z, 16);      // K-major views
-      const uint32_t x_lo = desc_lo(sbase, 16), u_lo = x_lo + (ROW_TILE >> 4);
       const int q = warp - kIssuerWarp;
       for (; ok && w.live(a); g += w.j, w.next(a)) {
-        if (!mbar_wait_warp(BAR_X, (uint32_t)(w.m & 1))) { report(2); break; }
+        if (!mbar_wait_warp(BAR_X(w.m), XPHASE(w.m))) { report(2); break; }
+        const uint32_t x_lo = desc_lo(sbase + w.m % C::NX * C::ROWS, 16), u_lo = x_lo + (ROW_TILE >> 4);
         for (int gi = FWD ? g : g + ((g ^ q) & 1); gi < g + w.j; gi += FWD ? 1 : 2) {
           const int s = gi % NY;
           // the tiles have normally been loaded long ago: checking them first keeps that check out of the way from the score
@@ -275,7 +310,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
           }
           __syncwarp();
         }
-        if (ok && elect_one()) umma_commit(BAR_XE);
+        if (ok && elect_one()) umma_commit(BAR_XE(w.m));
         __syncwarp();
       }
       __syncwarp();
@@ -286,6 +321,24 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       for (; ok && w.live(a); w.next(a)) {
         if (w.m >= C::ACCS && !__all_sync(0xffffffffu, read(w.m - C::ACCS))) { report(6); break; }
         const uint32_t acc = tmem + C::T_A + w.m % C::ACCS * D;
+        const uint32_t state = has_state(w.r0) ? 1u : 0u;
+        if constexpr (FIRST) {
+          // what the chunk's keys take from all tokens after it: u S1^T and x S1
+          if (state) {
+            if (!mbar_wait_warp(BAR_X(w.m), XPHASE(w.m))) { report(6); break; }
+            tc_fence_after();
+            const uint32_t s1 = sbase + C::OFF_S1 + w.m % C::NX * C::S1_TILE;
+            const uint32_t x_lo = desc_lo(sbase + w.m % C::NX * C::ROWS, 16), s_mn = desc_lo(s1, 8192);
+            if (elect_one()) {
+              umma_ss_k64(acc, x_lo + (ROW_TILE >> 4), desc_lo(s1, 16), idesc_bf16(128, D, 0, 0));
+              umma_ss_kmn_steps<4>(acc + D, x_lo, s_mn, idescO, 0u);
+              umma_commit(BAR_XE(w.m));
+            }
+          } else if (elect_one()) {
+            mbar_arrive(BAR_XE(w.m));
+          }
+          __syncwarp();
+        }
         for (int i = 0; i < w.j; ++i, ++g) {
           const int s = g % NZ, q = g & 1, set = g % C::SETS;
           if (!mbar_wait_warp(BAR_ZF(s), (uint32_t)((g / NZ) & 1)) ||
@@ -303,11 +356,12 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
 #pragma unroll
               for (int ks = 0; ks < BN / 16; ++ks)
                 umma_ts_1(acc, tmem + set * C::SET_COLS + (ks >> 1) * 32 + (ks & 1) * 8, z_lo + ks * 128, idescO,
-                          (i > 0 || ks > 0) ? 1u : 0u);
+                          (i > 0 || ks > 0) ? 1u : state);
               umma_commit(BAR_TF(set));
             } else {
-              umma_ts_steps<BN / 16>(acc, tmem + C::T_E + q * HB, y_mn + (uint32_t)s * (C::COL_TILE >> 4), idescO, i > 0 ? 1u : 0u);
-              umma_ts_steps<BN / 16>(acc + D, tmem + C::T_P + q * HB, z_lo, idescO, i > 0 ? 1u : 0u);
+              umma_ts_steps<BN / 16>(acc, tmem + C::T_E + q * HB, y_mn + (uint32_t)s * (C::COL_TILE >> 4), idescO,
+                                     i > 0 ? 1u : state);
+              umma_ts_steps<BN / 16>(acc + D, tmem + C::T_P + q * HB, z_lo, idescO, i > 0 ? 1u : state);
               umma_commit(BAR_PV(q));
               umma_commit(BAR_YE(s));
             }
@@ -340,14 +394,14 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
               __uint_as_float((uint32_t)(f.x >> 32))};
     };
     auto open = [&](int m, Item& it) -> bool {
-      if (!mbar_wait(BAR_X, (uint32_t)(m & 1))) { report(11); return false; }
+      if (!mbar_wait(BAR_X(m), XPHASE(m))) { report(11); return false; }
       it = item(m);
       __syncwarp();
-      if (lane == 0) mbar_arrive(BAR_XE);
+      if (lane == 0) mbar_arrive(BAR_XE(m));
       return true;
     };
     // The result of a row tile: this warp's FC accumulator columns.
-    auto finish = [&](int m, int head, int r0, float pre) -> bool {
+    auto finish = [&](int m, int head, int r0, float pre, float A1) -> bool {
       const int ab = m % C::ACCS, row = r0 + rl;
       const bool row_ok = row < a.nrows, second = FUSED && part4 >= 2;
       const int cc = FUSED ? (part4 & 1) * 32 : part4 * 16;
@@ -381,7 +435,20 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       float f[C::FC];
 #pragma unroll
       for (int e = 0; e < C::FC; ++e) f[e] = FUSED ? __uint_as_float(ov[e]) * pre : __uint_as_float(ov[e]);
-      if (a.o_add) {
+      if constexpr (FIRST) {
+        // grad_k: normaliser column, grad_v: constant row
+        const uint32_t vec = sbase + C::OFF_STV + (m & 7) * C::STV + (second ? 256 : 0) + cc * 4;
+        const float mul = second ? a.a0 : A1;
+#pragma unroll
+        for (int e = 0; e < C::FC / 4; ++e) {
+          const ulonglong2 v = lds_v2(vec + 16 * e);
+          float x[4];
+          unpack2(v.x, x[0], x[1]);
+          unpack2(v.y, x[2], x[3]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) f[4 * e + i] = fmaf(mul, x[i], f[4 * e + i]);
+        }
+      } else if (a.o_add) {
         const uint32_t row_s = sbase + C::OFF_ADD + (second ? 2 * C::ADD_HALF : 0) + (cc >> 5) * C::ADD_HALF + rl * 128;
 #pragma unroll
         for (int p = 0; p < C::FC / 4; ++p) {
@@ -542,10 +609,10 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       if (rev && (((g + it.j) ^ gp) & 1) < next.j) nxt_raw = fetch_vec(next.tb + (((g + it.j) ^ gp) & 1), next.head);
       // completed square: the factor left out of E' and P'
       if (FUSED) {
-        ok = finish(m, it.head, it.r0, SQ ? (part4 >= 2 ? A2 : 2.f * A2) : 1.f);
+        ok = finish(m, it.head, it.r0, SQ ? (part4 >= 2 ? A2 : 2.f * A2) : 1.f, A1);
       } else if (m > 0) {
         const Item before = item(m - 1);
-        ok = finish(m - 1, before.head, before.r0, 1.f);
+        ok = finish(m - 1, before.head, before.r0, 1.f, 0.f);
       }
       g += it.j;
       it = next;
@@ -553,7 +620,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     }
     if (ok && !FUSED && m > 0) {
       const Item before = item(m - 1);
-      finish(m - 1, before.head, before.r0, 1.f);
+      finish(m - 1, before.head, before.r0, 1.f, 0.f);
     }
   }
 
@@ -565,37 +632,47 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   }
 }
 
-template <int MODE, bool SQ>
+template <int MODE, bool SQ, bool FIRST>
 int start(const Ctx& c, const char* name, unsigned grid, const CUtensorMap& tx, const CUtensorMap& tu, const CUtensorMap& ty,
           const CUtensorMap& tz, const CUtensorMap& ta, const CUtensorMap& tb, const WalkArgs& a) {
-  using C = WK<MODE>;
+  using C = WK<MODE, FIRST>;
   // the compute warps wait for registers that the block must have been launched with
   static const int regs = [] {
     cudaFuncAttributes at;
-    return cudaFuncGetAttributes(&at, walk_kernel<MODE, SQ>) == cudaSuccess ? at.numRegs : 0;
+    return cudaFuncGetAttributes(&at, walk_kernel<MODE, SQ, FIRST>) == cudaSuccess ? at.numRegs : 0;
   }();
   if (regs < kRegsLaunch)
     return fail(FASTMAX_E_UNSUPPORTED, "%s: %d registers a thread at launch instead of %d", name, regs, kRegsLaunch);
-  FM_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<MODE, SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-  FM_LAUNCH(name, c.stream, (walk_kernel<MODE, SQ><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, ta, tb, a)));
+  FM_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<MODE, SQ, FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+  FM_LAUNCH(name, c.stream, (walk_kernel<MODE, SQ, FIRST><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, ta, tb, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
 
 template <int MODE>
 int launch(const Ctx& c, const char* name, const void* x, const void* u, const void* y, const void* z, int nrows, int ncols,
-           WalkArgs a) {
+           WalkArgs a, const FirstState* fs) {
   const fastmax_problem& p = c.p;
   if (p.bh == 0 || nrows == 0) return FASTMAX_OK;
   CUtensorMap tx, tu, ty, tz, ta, tb;
   int rc;
   if ((rc = tma_map_bf16(&tx, x, p.bh, nrows, D, 128))) return rc;
   if ((rc = tma_map_bf16(&tu, u ? u : x, p.bh, nrows, D, 128))) return rc;
-  if ((rc = tma_map_bf16(&ty, y, p.bh, ncols, D, WK<MODE>::BN))) return rc;
-  if ((rc = tma_map_bf16(&tz, z, p.bh, ncols, D, WK<MODE>::BN))) return rc;
+  if ((rc = tma_map_bf16(&ty, y, p.bh, ncols, D, WK<MODE, false>::BN))) return rc;
+  if ((rc = tma_map_bf16(&tz, z, p.bh, ncols, D, WK<MODE, false>::BN))) return rc;
   ta = tb = tx;
   if (a.o_add && (rc = tma_map_f32_rows(&ta, a.o_add, p.bh, nrows))) return rc;
   if (a.o2_add && (rc = tma_map_f32_rows(&tb, a.o2_add, p.bh, nrows))) return rc;
+  if (fs) {
+    // the first-order chunks come here without passing dense_tc_forward / _backward, which check this for the others
+    const uintptr_t bases = (uintptr_t)x | (uintptr_t)u | (uintptr_t)y | (uintptr_t)z | (uintptr_t)a.o | (uintptr_t)a.o2;
+    if (bases & 15) return fail(FASTMAX_E_ARG, "the tensor-core family needs 16-byte aligned tensors");
+    a.nchunk = (nrows + a.chunk - 1) / a.chunk;
+    a.st = fs->states;
+    a.dvp = moment_dims(D, 1).dvp;
+    a.zero_chunk = fs->zero_chunk;
+    if ((rc = tma_map_bf16(&ta, fs->s1b, (size_t)p.bh * a.nchunk, D, D, D))) return rc;
+  }
   a.x = x;
   a.heads = p.bh;
   a.nrows = nrows;
@@ -612,17 +689,19 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
   const long long blocks = (long long)a.heads * a.ntr;
   if (blocks > 0x7FFF0000LL) return fail(FASTMAX_E_ARG, "heads x row tiles = %lld exceeds the grid limit", blocks);
   const unsigned grid = (unsigned)(blocks < 148 ? blocks : 148);
-  if (MODE == MODE_DKDV && a.a2 > 0.f) return start<MODE, MODE == MODE_DKDV>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
-  return start<MODE, false>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
+  if (fs) return start<MODE, false, MODE == MODE_DKDV>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
+  if (MODE == MODE_DKDV && a.a2 > 0.f) return start<MODE, MODE == MODE_DKDV, false>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
+  return start<MODE, false, false>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
 }
 
 }  // namespace
 
 int dense_tc_walk_forward(const Ctx& c, const void* q, const void* k, const void* v, const WalkArgs& a) {
-  return launch<MODE_FWD>(c, "fm_dense_tc_fwd", q, nullptr, k, v, c.p.nq, c.p.nk, a);
+  return launch<MODE_FWD>(c, "fm_dense_tc_fwd", q, nullptr, k, v, c.p.nq, c.p.nk, a, nullptr);
 }
-int dense_tc_walk_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, const WalkArgs& a) {
-  return launch<MODE_DKDV>(c, "fm_dense_tc_dkdv", k, v, q, gs, c.p.nk, c.p.nq, a);
+int dense_tc_walk_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, const WalkArgs& a,
+                       const FirstState* fs) {
+  return launch<MODE_DKDV>(c, "fm_dense_tc_dkdv", k, v, q, gs, c.p.nk, c.p.nq, a, fs);
 }
 
 int tc_walk_status(int* out, cudaStream_t stream) {

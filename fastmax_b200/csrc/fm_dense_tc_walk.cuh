@@ -24,6 +24,9 @@ struct WalkArgs {
   const stat_t* stat_k;
   int heads, nrows, ncols, off, mask, ntr, chunk, ratio, order;   // see RowWalk
   float a0, a1, a2, lim;
+  // first-order chunks: running sums of the states, rows [y_a | 1] of `dvp` floats, d + 1 rows per (head, chunk)
+  const float* st;
+  int dvp, nchunk, zero_chunk;   // zero_chunk: the chunk whose running sum is empty (-1: none)
   int o_heads;           // FWD: > 0 writes out as (batch, nrows, o_heads, 64)
 };
 
@@ -33,6 +36,7 @@ struct WalkArgs {
 int tma_map_f32_rows(CUtensorMap* m, const float* base, size_t mats, size_t rows);
 
 int dense_tc_walk_forward(const Ctx& c, const void* q, const void* k, const void* v, const walk::WalkArgs& a);
-int dense_tc_walk_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, const walk::WalkArgs& a);
+int dense_tc_walk_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, const walk::WalkArgs& a,
+                       const FirstState* fs = nullptr);
 
 }  // namespace fm

@@ -645,9 +645,10 @@ static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
 // Whether the kernels that walk row tiles serve a pass (0 forward, 2 grad_k + grad_v): they cover the ends of a row tile and
 // keep the wide loop's pace, but deal their row tiles out beforehand, so a nearly empty last round costs a whole row tile, and
 // below some columns to a row tile the short kernels' two CTAs hide the ends better.  us, what served it before / walking:
-//   chunks        forward 121 / 111 at 4096 row tiles in chunks of 256, 241 / 190 of 2048, 375 / 302 of 4096, 20.8 / 18.7 at
+//   chunks        forward 121 / 115 at 4096 row tiles in chunks of 256, 241 / 181 of 2048, 375 / 302 of 4096, 20.8 / 18.7 at
 //                 320 row tiles of 256; grad_k + grad_v 205 / 166, 449 / 386, but 630 / 642 of 4096, and 29.1 / 24.9; no gain
-//                 of the forward at 200 row tiles
+//                 of the forward at 200 row tiles.  First-order chunks (grad_k + grad_v): 189 / 183 of 512, 155 / 148 of 256,
+//                 27.3 / 25.1 at 320 row tiles of 512
 //   forward       causal, 2048 to 2200 row tiles: 61.8 / 76 at 400 columns, 72.2 / 66.0 at 1000, 170 / 163 at 4600, but
 //                 301 / 313 (3008 row tiles) at 6000; 208 / 176 (4096) at 2000; 480 to 1200 row tiles: 47.6 / 49.5 to
 //                 37.2 / 35.3 at 1000, 45.4 / 41.4 at 1500, 33.2 / 33.2 at 3600; 320 at most: 16.6 / 14.7 at 600 columns,
@@ -673,6 +674,31 @@ static walk::WalkArgs walk_args(const fastmax_problem& p, const stat_t* stats, c
   a.chunk = ca ? ca->chunk : 0;
   return a;
 }
+static int walk_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats, void* out, float* den,
+                        const ChunkAdd* ca) {
+  walk::WalkArgs a = walk_args(c.p, stats, ca);
+  a.o = out;
+  a.den_out = den;
+  a.o_heads = c.out_heads;
+  if (ca) { a.o_add = ca->out_add; a.den_add = ca->den_add; }
+  return dense_tc_walk_forward(c, q, k, v, a);
+}
+static int walk_dkdv(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
+                     const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd* ca, const FirstState* fs) {
+  walk::WalkArgs a = walk_args(c.p, stats, ca);
+  a.dvec = dvec;
+  a.o = grad_k;
+  a.o2 = grad_v;
+  a.dots = c.p.normalize ? dots + c.p.bh : nullptr;
+  if (ca) { a.o_add = ca->gk_add; a.o2_add = ca->gv_add; }
+  return dense_tc_walk_dkdv(c, k, v, q, gs, a, fs);
+}
+
+int dense_tc_first_dkdv(const Ctx& c, const void* q, const void* k, const void* v, const void* gs, const float* dvec,
+                        const stat_t* stats, float* dots, void* grad_k, void* grad_v, const ChunkAdd& ca, const FirstState& fs) {
+  if (walk_rows(c.p, &ca, 2)) return walk_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, &ca, &fs);
+  return dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, &ca, &fs);
+}
 
 int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* gs,
                            const float* dvec, const stat_t* stats, float* dots, void* grad_q,
@@ -697,16 +723,7 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
   if (short_rows(p, ca, 1)) rc = dense_tc_short_dq(c, q, k, v, gs, dvec, stats, dots, grad_q, ca);
   else rc = launch_wide<MODE_DQ>(c, "fm_dense_tc_dq", q, gs, k, v, p.nq, p.nk, a);
   if (rc) return rc;
-  if (walk_rows(p, ca, 2)) {
-    walk::WalkArgs b = walk_args(p, stats, ca);
-    b.dvec = dvec;
-    b.o = grad_k;
-    b.o2 = grad_v;
-    b.dots = p.normalize ? dots + p.bh : nullptr;
-    b.o_add = ca ? ca->gk_add : nullptr;
-    b.o2_add = ca ? ca->gv_add : nullptr;
-    return dense_tc_walk_dkdv(c, k, v, q, gs, b);
-  }
+  if (walk_rows(p, ca, 2)) return walk_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, ca, nullptr);
   if (short_rows(p, ca, 2)) return dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, ca);
   // grad_k and grad_v: rows = keys, columns = queries
   a.o = grad_k;
@@ -720,14 +737,7 @@ int dense_tc_wide_backward(const Ctx& c, const void* q, const void* k, const voi
 int dense_tc_wide_forward(const Ctx& c, const void* q, const void* k, const void* v, const stat_t* stats,
                           void* out, float* den, const ChunkAdd* ca) {
   const fastmax_problem& p = c.p;
-  if (walk_rows(p, ca, 0)) {
-    walk::WalkArgs a = walk_args(p, stats, ca);
-    a.o = out;
-    a.den_out = den;
-    a.o_heads = c.out_heads;
-    if (ca) { a.o_add = ca->out_add; a.den_add = ca->den_add; }
-    return dense_tc_walk_forward(c, q, k, v, a);
-  }
+  if (walk_rows(p, ca, 0)) return walk_forward(c, q, k, v, stats, out, den, ca);
   if (short_rows(p, ca, 0)) return dense_tc_short_forward(c, q, k, v, stats, out, den, ca);
   WArgs a = {};
   a.stat_q = p.normalize ? stats : nullptr;

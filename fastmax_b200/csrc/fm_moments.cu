@@ -474,7 +474,7 @@ int moments_backward(const Ctx& c, const void* q, const void* k, const void* v, 
       if ((rc = prefix_states(c, ncq, states, nullptr, 1, true, kv, &ready))) return rc;
       if ((rc = first_tc_convert(c, p.bh * ncq, states, s16, ncq, stats))) return rc;
       const FirstState after = {states, s16, ncq - 1};
-      if ((rc = dense_tc_short_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, &own, &after))) return rc;
+      if ((rc = dense_tc_first_dkdv(c, q, k, v, gs, dvec, stats, dots, grad_k, grad_v, own, after))) return rc;
       return p.normalize ? launch_norm_fixup(c, q, k, stats, dots, grad_q, grad_k) : FASTMAX_OK;
     }
     // grad_q: the first chunk's tokens have no keys before their chunk; grad_k, grad_v: the last chunk's

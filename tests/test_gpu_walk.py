@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 # bh, nq, nk, mask, p, normalize, chunk, walking kernels (forward; grad_k and grad_v)
 CASES = [(19, 1000, 1000, 1, 2, 1, 0, 2), (20, 1030, 1030, 1, 1, 0, 0, 2), (38, 1000, 1129, 1, 2, 1, 0, 1), (55, 690, 650, 0, 2, 1, 0, 2),
          (60, 650, 520, 0, 1, 1, 0, 2), (75, 515, 515, 1, 2, 1, 256, 2), (34, 1281, 1281, 1, 2, 0, 512, 2), (240, 641, 641, 1, 2, 1, 256, 2),
-         (150, 1031, 1031, 1, 2, 1, 0, 1)]
+         (150, 1031, 1031, 1, 2, 1, 0, 1), (75, 515, 515, 1, 1, 1, 256, 1), (34, 1281, 1281, 1, 1, 0, 512, 1),
+         (240, 641, 641, 1, 1, 1, 256, 1)]
 
 
 @pytest.mark.parametrize("cfg", CASES, ids=["bh%dnq%dnk%dm%dp%dz%dc%dw%d" % c for c in CASES])
