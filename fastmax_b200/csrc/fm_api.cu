@@ -297,6 +297,7 @@ int fastmax_b200_device_status(int* status, void* stream) {
   if (!f && (rc = split_moments_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = readout_status(&f, (cudaStream_t)stream))) return rc;
   if (!f && (rc = decode_tc_status(&f, (cudaStream_t)stream))) return rc;
+  if (!f && (rc = decode_step_status(&f, (cudaStream_t)stream))) return rc;
   *status = a ? a : (b ? b : f);
   return FASTMAX_OK;
 }
@@ -315,6 +316,7 @@ int fastmax_b200_device_status_reset(void* stream) {
   if ((rc = readout_status_reset(s))) return rc;
   if ((rc = tc_short_status_reset(s))) return rc;
   if ((rc = decode_tc_status_reset(s))) return rc;
+  if ((rc = decode_step_status_reset(s))) return rc;
   return first_tc_status_reset(s);
 }
 

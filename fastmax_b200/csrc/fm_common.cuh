@@ -250,6 +250,8 @@ int decode_append_tc(const fastmax_problem& p, const void* k, const void* v, lon
                      cudaStream_t st);
 int decode_tc_status(int* out, cudaStream_t stream);
 int decode_tc_status_reset(cudaStream_t stream);
+int decode_step_status(int* out, cudaStream_t stream);
+int decode_step_status_reset(cudaStream_t stream);
 
 // ---- moment-state form (fm_moments_ffma.cu) ---------------------------------------
 struct MomentDims {

@@ -30,10 +30,10 @@
 //                  fenced and each CTA waited for its arrival, 330 with one thread's fence); 8 key/value heads of 4 query heads
 //                  12.3 (12.8, and 16.8 when the queries were asked for after the update, the arriving CTA fenced its 24 KB of
 //                  state and the last one read the queries' shares in turn); 4 heads, float32, 10.5 (11.6); 128 heads, d = 128:
-//                  305 (334).  The same bytes in 2 KB runs, without the arithmetic: 258.  Other arrangements for 1024 heads:
+//                  271 (334).  The same bytes in 2 KB runs, without the arithmetic: 258.  Other arrangements for 1024 heads:
 //                  several groups of blocks to a CTA 397, five CTAs to an SM 377 (both before the above); tiles by bulk copies
-//                  through shared memory, CTAs as here 366 / 291 (one kernel / without the sums; d = 128 319 / 264), persistent
-//                  with 1 to 4 CTAs an SM 338 to 403.
+//                  through shared memory, CTAs as here 366 / 291 (one kernel / without the sums; d = 128 319 / 264, kept),
+//                  persistent with 1 to 4 CTAs an SM 338 to 403.
 //   sum_kernel     the heads' sums, where step_kernel leaves them out (kSharesFrom).
 //   few_kernel     the same update for a few tokens of a prompt.
 //   append_kernel  many tokens (prompt), float32 or d = 32: bound by the FMA pipe; see there.  bf16 prompts of
@@ -42,7 +42,11 @@
 #include "fm_sm100.cuh"
 
 namespace fm {
+
+__device__ int g_step_status = 0;
+
 namespace {
+using namespace sm100;
 
 constexpr int kTile = 8;        // step_kernel: a thread's block is half (4 x 8) of an 8 x 8 tile of second-order rows ...
 constexpr int kHalf = 4;
@@ -67,6 +71,12 @@ template <int D> struct DecCfg {
   static constexpr int NB2 = NT * (NT + 1);                       // second-order half tiles per head
   static constexpr int NB1 = (D + kLinear - 1) / kLinear;         // first-order blocks per head
   __host__ __device__ static constexpr int ctas(int p) { return ((p == 2 ? NB2 : 0) + NB1 + 1 + RPB - 1) / RPB; }
+};
+
+// A tile of step_kernel in shared memory: its rows are kTile runs of kTile * DV contiguous floats, each kept from the 16-byte
+// boundary before it on; its mirror image's rows are kTile more.
+template <int D> struct RunCfg {
+  static constexpr int RUN = kTile * DecCfg<D>::DV, LD = RUN + 4, TILE = kTile * LD, SMEM = 2 * TILE * 4;
 };
 
 // Sum of squares of x[0..D) by one warp; the result is valid in every lane.
@@ -154,6 +164,39 @@ template <int D> struct Block {
 #pragma unroll
       for (int i = 0; i < kTile; ++i) s[u][i] = (u * kTile + i < live) ? base[u * ustride + i * C::DV] : 0.0f;
   }
+  // The same from and to shared memory (kind 2): the half tile's rows (half * kHalf + u, i) at column c of the tile's runs,
+  // which start x floats behind a 16-byte boundary, and of its mirror image's.
+  __device__ __forceinline__ void load_staged(const float* tile, int half, int x, int c) {
+#pragma unroll
+    for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+      for (int i = 0; i < kTile; ++i) s[u][i] = tile[(half * kHalf + u) * RunCfg<D>::LD + x + i * C::DV + c];
+  }
+  __device__ __forceinline__ void store_staged(float* tile, int half, int x, int c) const {
+    typedef RunCfg<D> S;
+#pragma unroll
+    for (int u = 0; u < kHalf; ++u)
+#pragma unroll
+      for (int i = 0; i < kTile; ++i) {
+        tile[(half * kHalf + u) * S::LD + x + i * C::DV + c] = s[u][i];
+        if (!diagonal) tile[S::TILE + i * S::LD + x + (half * kHalf + u) * C::DV + c] = s[u][i];
+      }
+  }
+  // what bulk copies leave out: a run's first floats up to a 16-byte boundary and its last ones after one
+  __device__ __forceinline__ void store_edges(int half, int x, int c) const {
+    const bool head = x > 0 && c < 4 - x, tail = c >= C::DV - x;
+#pragma unroll
+    for (int u = 0; u < kHalf; ++u) {
+      if (head) base[u * ustride] = s[u][0];
+      if (tail) base[u * ustride + (kTile - 1) * C::DV] = s[u][kTile - 1];
+    }
+    if (diagonal) return;
+#pragma unroll
+    for (int i = 0; i < kTile; ++i) {
+      if (head && half == 0) base2[i * D * C::DV] = s[0][i];
+      if (tail && half == 1) base2[(i * D + kHalf - 1) * C::DV] = s[kHalf - 1][i];
+    }
+  }
   // one token: k, and this column's value
   __device__ __forceinline__ void add(const float* k, float vc) {
     if (kind == 2) {
@@ -225,6 +268,12 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
                                                                   float* __restrict__ state, float* __restrict__ scratch,
                                                                   T* __restrict__ out) {
   typedef DecCfg<D> C;
+  typedef RunCfg<D> R;
+  // With d = 128 a CTA has one tile, which bulk copies bring and take back: 264 instead of 295 us for 128 heads, the sums apart.
+  // (With d = 64 291 instead of 294, with d = 32 107 instead of 99.)
+  constexpr bool BULK = SHARES && D == 128;
+  extern __shared__ __align__(16) float tile[];    // BULK
+  __shared__ __align__(8) uint64_t tile_here;
   __shared__ float ks[D], vs[D + 1];       // the token; (v, 1)
   __shared__ float qs[kQueries][D];
   __shared__ float red[kQueries][C::RPB][C::DV];
@@ -244,6 +293,29 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
     }
   };
 
+  // BULK: lane l of the first warp copies run l of the tile.  x: floats from a 16-byte boundary to a run, the same for all of a
+  // head, whose tiles start at multiples of four rows
+  const int x = BULK ? (int)((uintptr_t)(hs + kHeader) >> 2 & 3) : 0;
+  const bool copies = BULK && (int)blockIdx.x < C::NB2 / 2 && tid < kTile;
+  float *own = nullptr, *image = nullptr;
+  if constexpr (BULK) {
+    static_assert(C::RPB == 2, "a tile, two halves, to a CTA");
+    if (copies) {
+      int ta, tb;
+      upper_tile(blockIdx.x, C::NT, ta, tb);
+      own = hs + kHeader + (long long)C::DV * ((ta * kTile + tid) * D + tb * kTile);
+      image = ta == tb ? nullptr : hs + kHeader + (long long)C::DV * ((tb * kTile + tid) * D + ta * kTile);
+      const uint32_t bytes = 4 * R::RUN + (x ? 16 : 0);
+      if (tid == 0) {
+        mbar_init(smem_u32(&tile_here), 1);
+        mbar_fence_init();
+        mbar_expect_tx(smem_u32(&tile_here), kTile * bytes);
+      }
+      __syncwarp((1u << kTile) - 1u);
+      bulk_load(smem_u32(tile + tid * R::LD), own - x, bytes, smem_u32(&tile_here));
+    }
+  }
+
   // the token and the first queries travel with the block's rows (a step of one sequence is a chain of latencies)
   static_assert(C::THREADS >= 2 * D, "a thread an element of the token");
   const int ng0 = a.ratio < kQueries ? a.ratio : kQueries;
@@ -258,7 +330,8 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
   const float kmax2 = hs[0];
   Block<D> blk;
   blk.place(blockIdx.x * C::RPB + r, a.p, hs + kHeader, c);
-  blk.load();
+  const bool bulk = BULK && blk.kind == 2;
+  if (!bulk) blk.load();
   if (tid < D) ks[tid] = tok;
   else if (tid < 2 * D) vs[tid - D] = tok;
   if (tid == 0) vs[D] = 1.0f;
@@ -274,8 +347,24 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
     const float n2 = warp_norm2<D>(ks, lane);
     if (lane == 0) s_kmax2 = fmaxf(kmax2, n2);
   }
+  bool here = true;
+  if (bulk) {
+    here = mbar_wait(smem_u32(&tile_here), 0);
+    if (!here) atomicCAS(&g_step_status, 0, 1);
+    blk.load_staged(tile, r, x, c);
+  }
   blk.add(ks, vs[c]);
+  if (bulk) {
+    blk.store_staged(tile, r, x, c);
+    fence_proxy_async();
+  }
   __syncthreads();
+  if (copies && here) {
+    const int skip = (4 - x) & 3;
+    const uint32_t from = smem_u32(tile + tid * R::LD + x + skip), bytes = 4 * (R::RUN - (x ? 4 : 0));
+    bulk_store(own + skip, from, bytes);
+    if (image) bulk_store(image + skip, from + 4 * R::TILE, bytes);
+  }
   auto scale = [&](int g) {
     return a.normalize ? (a.lim * rsqrtf(s_q2[g])) * (a.lim * rsqrtf(s_kmax2)) : 1.0f;
   };
@@ -304,7 +393,9 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
     }
   }
   if constexpr (SHARES) {
-    blk.store();
+    if (!bulk) blk.store();
+    else if (here) blk.store_edges(r, x, c);
+    if (copies) tma_store_wait_read();     // the bulk copies have read this CTA's shared memory
     return;
   }
   __syncthreads();
@@ -472,7 +563,6 @@ template <typename T, int D>
 __global__ void __launch_bounds__(AppCfg<D>::THREADS, 2) append_kernel(const DecArgs a, const T* __restrict__ k,
                                                                        const T* __restrict__ v,
                                                                        float* __restrict__ state) {
-  using namespace sm100;
   typedef AppCfg<D> C;
   constexpr int DV = D + 1, KS = D + 4;
   constexpr int TB = 64 / (int)sizeof(T) * (D >= 128 ? 1 : 2) / 2;      // tokens per batch: bf16 32, float32 16 (D = 128: 8)
@@ -641,9 +731,10 @@ long long append_min(const fastmax_problem& p) {
 
 // From how many CTAs on a step leaves the heads' sums to sum_kernel: a CTA then ends without a fence and an atomic's way to
 // memory and back, but the sums cost a kernel that starts when everything has been written, 9 to 13 us.  Measured, us a step, one
-// kernel / two: d = 64 88.1 / 88.3 at 6400 CTAs (256 heads), 330 / 312 at 25600; d = 128 165.6 / 160.4 at 8896 (64 heads), 321 /
-// 305 at 17792, 49.9 / 51.3 at 2224; d = 32 11.7 / 11.5 at 512 (128 heads), 29.5 / 26.8 at 2048, 117 / 101 at 8192.
-template <int D> constexpr long long kSharesFrom = D == 32 ? 2048 : 8192;
+// kernel / two: d = 64 88.1 / 88.3 at 6400 CTAs (256 heads), 330 / 312 at 25600; d = 128, whose two kernels use bulk copies, 49.9
+// / 48.9 (with the state out of L2 55.2 / 56.3) at 2224 (16 heads), 69.9 / 64.4 at 3336, 165.6 / 144 at 8896, 321 / 271 at
+// 17792, 4 query heads each 102 / 86.7 at 4448; d = 32 17.5 / 16.7 (24.8 / 25.6) at 1024, 24.3 / 22.3 at 1600, 117 / 101 at 8192.
+template <int D> constexpr long long kSharesFrom = D == 32 ? 1600 : D == 64 ? 8192 : 3072;
 
 template <typename T, int D, bool READ>
 int launch_decode(const fastmax_problem& p, const void* q, const void* k, const void* v, long long n_new,
@@ -662,10 +753,12 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
   } else {
     const dim3 grid(DecCfg<D>::ctas(p.p), p.bhkv);
     if constexpr (READ) {
-      if (grid.x * (long long)p.bhkv >= kSharesFrom<D>) {
+      if (p.p == 2 && grid.x * (long long)p.bhkv >= kSharesFrom<D>) {
+        const int smem = D == 128 ? RunCfg<D>::SMEM : 0;
+        FM_CUDA_TRY(cudaFuncSetAttribute(step_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         FM_LAUNCH("fm_decode_step", st,
-                  (step_kernel<T, D, true><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
-                                                                                scratch, (T*)out)));
+                  (step_kernel<T, D, true><<<grid, DecCfg<D>::THREADS, smem, st>>>(a, (const T*)q, (const T*)k, (const T*)v,
+                                                                                   state, scratch, (T*)out)));
         FM_CUDA_TRY(cudaGetLastError());
         FM_LAUNCH("fm_decode_sum", st,
                   (sum_kernel<T, D><<<p.bh, DecCfg<D>::THREADS, 0, st>>>(a, (int)grid.x, (const T*)k, state, scratch, (T*)out)));
@@ -732,3 +825,17 @@ int fastmax_b200_decode_step(const fastmax_problem* prob, const void* q, const v
   if (((uintptr_t)k | (uintptr_t)v) & 15) return fail(FASTMAX_E_ARG, "k and v must be 16-byte aligned");
   return dispatch_decode<true>(*prob, q, k, v, 1, (float*)state, (float*)scratch, out, (cudaStream_t)stream);
 }
+
+namespace fm {
+int decode_step_status(int* out, cudaStream_t stream) {
+  FM_CUDA_TRY(cudaMemcpyFromSymbolAsync(out, g_step_status, sizeof(int), 0, cudaMemcpyDeviceToHost, stream));
+  FM_CUDA_TRY(cudaStreamSynchronize(stream));
+  return FASTMAX_OK;
+}
+int decode_step_status_reset(cudaStream_t stream) {
+  const int zero = 0;
+  FM_CUDA_TRY(cudaMemcpyToSymbolAsync(g_step_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
+  FM_CUDA_TRY(cudaStreamSynchronize(stream));
+  return FASTMAX_OK;
+}
+}  // namespace fm

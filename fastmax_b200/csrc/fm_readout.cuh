@@ -68,12 +68,6 @@ struct Walk {
     return a.chunk > 0 ? head * a.nchunk + (a.first + grp) / a.per_chunk : head;
   }
 };
-// contiguous global -> shared copy (both 16-byte aligned, size a multiple of 16)
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
 __device__ __forceinline__ uint4 lds128(uint32_t saddr) {
   uint4 r;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(saddr));
