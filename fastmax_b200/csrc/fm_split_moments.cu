@@ -32,7 +32,7 @@ constexpr int TB = 64;                                  // tokens per block
 constexpr int PS_GEN = 512, PS_THREADS = 19 * 32;       // 16 generator warps, producer, two issuers
 constexpr int PS_NS = 3;
 constexpr int PS_STAGE = 3 * TB * D * 2;                // value parts of a block
-constexpr int PS_ROWS = D + 2, PS_YT = PS_ROWS * TB * 4;
+constexpr int PS_ROWS = D + 2, PS_LD = TB * 4 + 16, PS_YT = PS_ROWS * PS_LD;
 constexpr int PS_TILES = 17;
 constexpr int PS_OFF_Y = PS_NS * PS_STAGE;              // two transposed blocks, fp32
 constexpr int PS_OFF_EP = PS_OFF_Y + 2 * PS_YT;         // float ep[2][128][65], then the second share of the last column
@@ -43,8 +43,10 @@ constexpr int PS_OFF_TMEM = PS_OFF_BAR + PS_NBAR * 8;
 constexpr int PS_SMEM = PS_OFF_TMEM + 16 + 1024;
 static_assert(PS_SMEM <= 227 * 1024, "shared memory");
 constexpr int PS_TM = 256;                              // tensor memory columns of a tile: sums 64, two operands of 3 x 32
-// byte offset of token chunk c (4 tokens) of row f inside a transposed block
-__device__ __forceinline__ uint32_t yt_off(int f, int c) { return (uint32_t)(f * 256 + ((c ^ (f & 7) ^ ((f >> 3) & 7)) << 4)); }
+// byte offset of token chunk c (4 tokens) of row f inside a transposed block: 16 bytes between rows, so that any eight
+// neighbouring rows (a lane's second one is its own plus the tile's distance) are read from different banks
+// (64 heads of 10000 keys 1152 us; 1320 with the pieces of 256-byte rows permuted, which suits aligned eights only)
+__device__ __forceinline__ uint32_t yt_off(int f, int c) { return (uint32_t)(f * PS_LD + c * 16); }
 
 __global__ void __launch_bounds__(PS_THREADS, 1)
 pair_sums_kernel(const __grid_constant__ CUtensorMap tmV, const float* __restrict__ k, const stat_t* __restrict__ stat_k, float lim,
@@ -67,7 +69,7 @@ pair_sums_kernel(const __grid_constant__ CUtensorMap tmV, const float* __restric
     mbar_fence_init();
   }
   if (warp == 17) tmem_alloc(smem_u32((const void*)tmem_slot), 512);
-  for (int i = tid; i < 2 * TB; i += PS_THREADS) *(float*)(smem + PS_OFF_Y + (i / TB) * PS_YT + (D + 1) * 256 + (i % TB) * 4) = 0.f;
+  for (int i = tid; i < 2 * TB; i += PS_THREADS) *(float*)(smem + PS_OFF_Y + (i / TB) * PS_YT + (D + 1) * PS_LD + (i % TB) * 4) = 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -155,9 +157,14 @@ pair_sums_kernel(const __grid_constant__ CUtensorMap tmV, const float* __restric
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int idx = tid + i * PS_GEN, tok = idx / 16, f0 = (idx % 16) * 4;
-        const float w[4] = {ks * kr[i].x, ks * kr[i].y, ks * kr[i].z, ks * kr[i].w};
+        // lane pairs begin at different features, or the sixteen of a token would meet two banks
+        const float4 w = kr[i];
+        const bool r1 = (idx >> 1) & 1, r2 = (idx >> 2) & 1;
+        const float a0 = r1 ? w.y : w.x, a1 = r1 ? w.z : w.y, a2 = r1 ? w.w : w.z, a3 = r1 ? w.x : w.w;
+        const float v[4] = {r2 ? a2 : a0, r2 ? a3 : a1, r2 ? a0 : a2, r2 ? a1 : a3};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) *(float*)(yt + yt_off(f0 + e, tok >> 2) + (tok & 3) * 4) = w[e];
+        for (int e = 0; e < 4; ++e)
+          *(float*)(yt + yt_off(f0 + ((e + (idx >> 1)) & 3), tok >> 2) + (tok & 3) * 4) = ks * v[e];
       }
       if (tid < TB) *(float*)(yt + yt_off(D, tid >> 2) + (tid & 3) * 4) = j * TB + tid < n ? 1.f : 0.f;
       asm volatile("bar.sync 1, 512;" ::: "memory");
