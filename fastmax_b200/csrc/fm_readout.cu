@@ -112,16 +112,20 @@ __global__ void __launch_bounds__(256) copies_kernel(const float* __restrict__ s
 // Running sum over the chunks of a head and the copies in one pass, second-order rows only: the copies of chunk m get
 // base + the sum of the raw states of the chunks before m (after m when reverse).  One CTA per (head, b) keeps its block
 // of the running sum in registers, in fp32, and reads rows (b, a) with block(a) <= block(b) of every raw chunk state
-// once; the fp32 states are left as they are.  The first chunk in scan order has nothing before it: without a base no
-// read-out asks for its copies and they are not written (skip_first).  The CTA with b == 64 copies the first-order rows (already summed in place).
-// Bound by HBM: 0.71 MB read and up to 0.66 MB written per chunk state; 1.2 ms a launch for 1024 heads of five chunks
-// (5.0 TB/s; all rows read and one layout of 0.56 MB written a word at a time: 1.4 ms).
-__global__ void __launch_bounds__(256, 3) prefix_copies_kernel(const float* __restrict__ state,
+// once, two chunks ahead by bulk copies; the fp32 states are left as they are.  The first chunk in scan order has nothing
+// before it: without a base no read-out asks for its copies and they are not written (skip_first).  The CTA with b == 64
+// copies the first-order rows (already summed in place).
+// Bound by HBM: 0.71 MB read and up to 0.66 MB written per chunk state; 0.98 ms a launch for 1024 heads of five chunks
+// (6.1 TB/s; 1.30 with one chunk ahead in registers and three CTAs an SM), 131 us for 32 heads of sixteen (156).
+constexpr int PC_NS = 2, PC_BLK = 64 * BLK_LD * 4;      // chunk states in flight; bytes of a block
+__global__ void __launch_bounds__(256, 4) prefix_copies_kernel(const float* __restrict__ state,
                                                             const float* __restrict__ base, char* __restrict__ ca,
                                                             char* __restrict__ cb, int nchunk, int dvp,
                                                             size_t per_state, int reverse, int skip_first) {
-  __shared__ __align__(16) float blk[64][BLK_LD];
-  const int head = blockIdx.y, b = blockIdx.x, t = threadIdx.x;
+  extern __shared__ __align__(128) uint8_t blocks[];
+  __shared__ __align__(8) uint64_t bars[PC_NS];
+  float(*blk)[BLK_LD] = (float(*)[BLK_LD])(blocks + PC_NS * PC_BLK);
+  const int head = blockIdx.y, b = 64 - (int)blockIdx.x, t = threadIdx.x;     // the longest first
   auto at_a = [&](int c) { return ca ? ca + (size_t)(head * nchunk + c) * A_BYTES : nullptr; };
   auto at_b = [&](int c) { return cb ? cb + (size_t)(head * nchunk + c) * B_BYTES : nullptr; };
   if (b == 64) {
@@ -133,43 +137,47 @@ __global__ void __launch_bounds__(256, 3) prefix_copies_kernel(const float* __re
   }
   const int NV = 16 * ((b >> 4) + 1) * 68 / 4;       // float4 pieces of the rows (b, a) that are read (dvp == 68)
   const size_t blk_off = (size_t)b * 64 * dvp;       // rows (b, a = 0..63) are contiguous
-  float4 run[5], nxt[5];
+  const uint32_t bar = smem_u32(bars);
+  // the last chunk in scan order is never added to anything that is written (and may not have been built)
+  auto load = [&](int i) {
+    if (i + 1 >= nchunk) return;
+    const int c = reverse ? nchunk - 1 - i : i, s = i % PC_NS;
+    mbar_expect_tx(bar + 8 * s, NV * 16);
+    bulk_load(smem_u32(blocks) + s * PC_BLK, state + (size_t)(head * nchunk + c) * per_state + blk_off, NV * 16, bar + 8 * s);
+  };
+  if (t == 0) {
+    for (int s = 0; s < PC_NS; ++s) mbar_init(bar + 8 * s, 1);
+    mbar_fence_init();
+    for (int i = 0; i < PC_NS; ++i) load(i);
+  }
+  float4 run[5];
 #pragma unroll
   for (int u = 0; u < 5; ++u) {
     const int v = t + u * 256;
     run[u] = (base && v < NV) ? *(const float4*)(base + (size_t)head * per_state + blk_off + 4 * v)
                               : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  auto load = [&](int i, float4 (&r)[5]) {
-    const int c = reverse ? nchunk - 1 - i : i;
-    const float* src = state + (size_t)(head * nchunk + c) * per_state + blk_off;
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-      const int v = t + u * 256;
-      // the last chunk in scan order is never added to anything that is written (and may not have been built)
-      r[u] = (i + 1 < nchunk && v < NV) ? __ldcs((const float4*)(src + 4 * v)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  load(0, nxt);
+  __syncthreads();
+  bool ok = true;
   for (int i = 0; i < nchunk; ++i) {
-    const int c = reverse ? nchunk - 1 - i : i;
+    const int c = reverse ? nchunk - 1 - i : i, s = i % PC_NS;
     const bool wanted = i >= skip_first;
     // the exclusive running sum of this chunk, transposed through shared memory
+    if (ok && i + 1 < nchunk && !mbar_wait(bar + 8 * s, (uint32_t)((i / PC_NS) & 1))) { report(91); ok = false; }
 #pragma unroll
     for (int u = 0; u < 5; ++u) {
       const int v = t + u * 256;
-      if (v < NV) *(float4*)(&blk[0][0] + 4 * v) = run[u];
+      if (v < NV) {
+        *(float4*)(&blk[0][0] + 4 * v) = run[u];
+        if (i + 1 < nchunk) {
+          const float4 x = *(const float4*)(blocks + s * PC_BLK + 16 * v);
+          run[u].x += x.x; run[u].y += x.y; run[u].z += x.z; run[u].w += x.w;
+        }
+      }
     }
-    float4 cur[5];
-#pragma unroll
-    for (int u = 0; u < 5; ++u) cur[u] = nxt[u];
-    load(i + 1, nxt);                                  // in flight during the transposed write
     __syncthreads();
+    if (t == 0 && ok) load(i + PC_NS);
     if (wanted) write_feature(blk, b, at_a(c), at_b(c), t);
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-      run[u].x += cur[u].x; run[u].y += cur[u].y; run[u].z += cur[u].z; run[u].w += cur[u].w;
-    }
     __syncthreads();
   }
 }
@@ -743,8 +751,9 @@ int moments_tc_prefix_convert(const Ctx& c, int heads, int nchunk, const float* 
   if ((((uintptr_t)state | (uintptr_t)base | (uintptr_t)to.a | (uintptr_t)to.b) & 15) != 0)
     return fail(FASTMAX_E_ARG, "moment states, totals and copies must be 16-byte aligned");
   dim3 grid(65, heads);
+  FM_CUDA_TRY(cudaFuncSetAttribute(prefix_copies_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (PC_NS + 1) * PC_BLK));
   FM_LAUNCH("fm_moments_prefix_bf16", c.stream,
-            (prefix_copies_kernel<<<grid, 256, 0, c.stream>>>(state, base, (char*)to.a, (char*)to.b, nchunk, m.dvp,
+            (prefix_copies_kernel<<<grid, 256, (PC_NS + 1) * PC_BLK, c.stream>>>(state, base, (char*)to.a, (char*)to.b, nchunk, m.dvp,
                                                               (size_t)m.f * m.dvp, reverse, base ? 0 : 1)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;

@@ -230,3 +230,21 @@ def test_more_heads_than_a_grid_dimension():
         s = slice(lo, lo + 4)
         for a, b, name in zip(got, run(*[t[s].contiguous() for t in (q, k, v, go)], impl="moments"), ("out", "dq", "dk", "dv")):
             assert float((a[s] - b).abs().max() / b.abs().max()) < 1e-4, (lo, name)
+
+
+@pytest.mark.parametrize("n,chunk", [(250, 256), (512, 256), (700, 256), (1100, 256), (2600, 256), (4700, 512)])
+def test_running_sums_over_few_and_many_chunks(n, chunk):
+    """One chunk to eleven: the running sums read their states two chunks ahead.  Tolerance: the bf16 one of the other tests."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v, go = [torch.randn(3, n, 64, generator=g, device="cuda").bfloat16() for _ in range(4)]
+    kw = dict(mask=True, normalize=True, p=2)
+
+    def run(*t, **impl):
+        out, den, st = _cabi.forward(*t[:3], **kw, **impl)
+        return (out,) + tuple(_cabi.backward(*t[:3], out, den, st, t[3], **kw, **impl))
+
+    got = run(q, k, v, go, impl="moments", chunk=chunk)
+    want = run(*[t.float() for t in (q, k, v, go)], impl="dense_ffma")
+    assert _cabi.device_status() == 0
+    for x, r, name in zip(got, want, ("out", "dq", "dk", "dv")):
+        assert float((x.float() - r).abs().max() / r.abs().max()) < 2e-2, name
