@@ -19,12 +19,15 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // covers 32*VEC/D rows per load and every load is a full 128-byte line; UNROLL
 // independent loads per lane are in flight, because one at a time left HBM at
 // 45 % (256 heads x 4096 x 64 bf16: 45.5 us per tensor before, 134 MB each).
-// q and k go in one launch (blockIdx.x: query heads, then key heads).  A head that one CTA covers
-// is written directly, so small problems need no zero fill either.
+// q and k go in one launch (query heads, then key heads), a head's CTAs side by side: with neighbours on different heads
+// at the same row, the strides of long sequences met few memory channels.  Four rounds of CTAs, or a last one of a few
+// CTAs costs as much as a full one.  A head that one CTA covers is written directly, so small problems need no zero fill
+// either.  32 heads of 262144 x 64 bf16, q and k: 334 us = 6.4 TB/s (476 heads first and one round, 339 when that round
+// was never passed); 64 heads of 10000 in float32 74 (80).
 struct RowmaxArgs {
   const void* q;
   const void* k;
-  int bh, nq, nk, rows_per_block, row_offset, direct;
+  int bh, nq, nk, rows_per_block, row_offset, direct, splits;
 };
 
 template <typename T, int D, bool WIDE>
@@ -36,13 +39,13 @@ __global__ void __launch_bounds__(256) rowmax_kernel(const RowmaxArgs a, stat_t*
   constexpr int RPW = 32 / LPR;                // rows per warp per load
   constexpr int UNROLL = 4;
   static_assert(D % VEC == 0 && LPR <= 32 && 32 % LPR == 0, "bad head dimension");
-  const int head = blockIdx.x;
+  const int head = blockIdx.x / a.splits;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / LPR, off = (lane % LPR) * VEC;
   const bool is_q = head < a.bh;
   const int n = is_q ? a.nq : a.nk;
   const T* base = is_q ? (const T*)a.q + (size_t)head * n * D : (const T*)a.k + (size_t)(head - a.bh) * n * D;
-  const int row0 = blockIdx.y * a.rows_per_block;
+  const int row0 = (blockIdx.x % a.splits) * a.rows_per_block;
   const int row1 = min(n, row0 + a.rows_per_block);
   float best = -1.0f;
   int best_row = 0;
@@ -114,7 +117,7 @@ __global__ void __launch_bounds__(256) rowmax_kernel(const RowmaxArgs a, stat_t*
 
 template <typename T>
 static int rowmax_both(const Ctx& c, const RowmaxArgs& a, int heads, int splits, stat_t* stats) {
-  dim3 grid(heads, splits);
+  const unsigned grid = (unsigned)heads * splits;
   const bool wide = (((uintptr_t)a.q | (uintptr_t)a.k) & 15) == 0;
   switch (c.p.d) {
 #define FM_CASE(DD) \
@@ -136,9 +139,9 @@ int launch_rowmax(const Ctx& c, const void* q, const void* k, stat_t* stats, int
   const fastmax_problem& p = c.p;
   const int heads = p.bh + p.bhkv, n = p.nq > p.nk ? p.nq : p.nk;
   if (heads == 0) return FASTMAX_OK;
-  // enough blocks per head to fill the GPU, at least 512 rows each
-  int splits = max(1, min((n + 511) / 512, (148 * 8 + heads - 1) / heads));
-  RowmaxArgs a{q, k, p.bh, p.nq, p.nk, (n + splits - 1) / splits, row_offset, splits == 1};
+  // enough blocks per head to fill the GPU four times, at least 512 rows each
+  int splits = max(1, min((n + 511) / 512, (4 * 148 * 8 + heads - 1) / heads));
+  RowmaxArgs a{q, k, p.bh, p.nq, p.nk, (n + splits - 1) / splits, row_offset, splits == 1, splits};
   if (n == 0 || splits > 1) FM_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(stat_t) * (size_t)heads, c.stream));
   if (n == 0) return FASTMAX_OK;
   if (p.dtype == FASTMAX_F32) return rowmax_both<float>(c, a, heads, splits, stats);
