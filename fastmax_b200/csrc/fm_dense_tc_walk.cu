@@ -81,7 +81,8 @@ struct WK {
   static constexpr int X_READERS = (FWD ? 1 : 2) + (FIRST ? 1 : 0) + kComputeWarps;
 };
 
-// A row tile as the producer hands it to the compute warps: also the coefficients of its head's polynomial.
+// A row tile as the producer hands it to the compute warps: also the coefficients of its head's polynomial (SQ: A2 is the
+// root times the scale).
 struct Item {
   int head, r0, tb, j;
   float A1, A2;
@@ -89,9 +90,7 @@ struct Item {
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_walk_status, 0, code); }
 
-// SQ (DKDV, a2 > 0): the polynomial in completed-square form, f(s) = A2 ((s + b)^2 + c), f'(s) = 2 A2 (s + b), with
-// b = A1 / (2 A2), c = A0 / A2 - b^2: a pair of scores costs t = s + b, P' = t t + c, E' = t (w - dvec), four packed operations
-// instead of five; A2 (grad_v) and 2 A2 (grad_k) multiply the accumulators in the end.
+// SQ (DKDV): the polynomial as a square and a rest (fm_square.cuh).
 template <int MODE, bool SQ, bool FIRST>
 __global__ void __launch_bounds__(kThreads, 1)
 walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
@@ -212,7 +211,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         if (!mbar_wait(BAR_XE(w.m), XPHASE(w.m) ^ 1u)) { report(1); break; }
         if constexpr (FIRST) vectors(w.m, w.r0, w.head);
         if (lane == 0) {
-          const Item it = {w.head, w.r0, w.tb, w.j, a.a1 * c, a.a2 * c * c};
+          const Item it = {w.head, w.r0, w.tb, w.j, a.a1 * c, SQ ? a.sq.root * c : a.a2 * c * c};
           *(Item*)(smem + C::OFF_ITEM + (w.m & 7) * 32) = it;
           const uint32_t bar = BAR_X(w.m), to = sbase + w.m % C::NX * C::ROWS;
           mbar_expect_tx(bar, C::ROWS + (has_state(w.r0) ? C::S1_TILE : 0));
@@ -431,7 +430,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       if constexpr (FUSED) tmem_ld32(at, ov);
       else tmem_ld16(at, ov);
       tmem_wait_ld(ov);
-      // (accumulator * factor left out of E' and P' + row to add), forward: (accumulator + row to add) / row sum
+      // (accumulator * factor left out of E' + row to add), forward: (accumulator + row to add) / row sum
       float f[C::FC];
 #pragma unroll
       for (int e = 0; e < C::FC; ++e) f[e] = FUSED ? __uint_as_float(ov[e]) * pre : __uint_as_float(ov[e]);
@@ -500,8 +499,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       const int first = (g ^ gp) & 1;              // the group's first column tile of this row tile
       const float A1 = it.A1, A2 = it.A2;
       const uint64_t A1v = pack2(A1, A1), A2v = pack2(A2, A2), A2d = pack2(2.f * A2, 2.f * A2);
-      const float sq_b = SQ ? A1 / (2.f * A2) : 0.f, sq_c = SQ ? a.a0 / A2 - sq_b * sq_b : 0.f;
-      const uint64_t Bv = pack2(sq_b, sq_b), Cv = pack2(sq_c, sq_c);
+      const uint64_t Bv = pack2(a.sq.shift, a.sq.shift), Cv = pack2(a.sq.rest, a.sq.rest);
       const int row = it.r0 + rl;
       int limcol = a.ncols - 1, lowcol = 0;        // columns kept for this row: lowcol <= col <= limcol
       if (a.mask) {
@@ -569,7 +567,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
             } else {
               if ((e & 1) == 0) nd2 = lds_v2(vec_s + (e >> 1) * 16);   // four column values per load
               const uint64_t ndl = (e & 1) ? nd2.y : nd2.x;
-              const uint64_t t2 = SQ ? add2(s2, Bv) : fma2(A2d, s2, A1v);
+              const uint64_t t2 = SQ ? fma2(s2, A2v, Bv) : fma2(A2d, s2, A1v);
               pe[e] = round2(mul2(t2, add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl)));
               pp[e] = round2(SQ ? fma2(t2, t2, Cv) : fma2(fma2(A2v, s2, A1v), s2, A0v));
             }
@@ -607,9 +605,9 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       Item next;
       if (!(ok = open(m + 1, next))) break;
       if (rev && (((g + it.j) ^ gp) & 1) < next.j) nxt_raw = fetch_vec(next.tb + (((g + it.j) ^ gp) & 1), next.head);
-      // completed square: the factor left out of E' and P'
+      // SQ: the factor left out of E'
       if (FUSED) {
-        ok = finish(m, it.head, it.r0, SQ ? (part4 >= 2 ? A2 : 2.f * A2) : 1.f, A1);
+        ok = finish(m, it.head, it.r0, SQ && part4 < 2 ? 2.f * A2 : 1.f, A1);
       } else if (m > 0) {
         const Item before = item(m - 1);
         ok = finish(m - 1, before.head, before.r0, 1.f, 0.f);
@@ -690,7 +688,7 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
   if (blocks > 0x7FFF0000LL) return fail(FASTMAX_E_ARG, "heads x row tiles = %lld exceeds the grid limit", blocks);
   const unsigned grid = (unsigned)(blocks < 148 ? blocks : 148);
   if (fs) return start<MODE, false, MODE == MODE_DKDV>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
-  if (MODE == MODE_DKDV && a.a2 > 0.f) return start<MODE, MODE == MODE_DKDV, false>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
+  if (MODE == MODE_DKDV && square_form(a.a0, a.a1, a.a2, &a.sq)) return start<MODE, MODE == MODE_DKDV, false>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
   return start<MODE, false, false>(c, name, grid, tx, tu, ty, tz, ta, tb, a);
 }
 

@@ -3,7 +3,7 @@
 
 #include <cuda.h>
 
-#include "fm_common.cuh"
+#include "fm_square.cuh"
 
 namespace fm {
 namespace walk {
@@ -24,6 +24,7 @@ struct WalkArgs {
   const stat_t* stat_k;
   int heads, nrows, ncols, off, mask, ntr, chunk, ratio, order;   // see RowWalk
   float a0, a1, a2, lim;
+  Square sq;             // DKDV, where square_form() gives one
   // first-order chunks: running sums of the states, rows [y_a | 1] of `dvp` floats, d + 1 rows per (head, chunk)
   const float* st;
   int dvp, nchunk, zero_chunk;   // zero_chunk: the chunk whose running sum is empty (-1: none)

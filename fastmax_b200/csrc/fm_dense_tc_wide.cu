@@ -36,6 +36,7 @@
 #include "fm_common.cuh"
 #include "fm_dense_tc_walk.cuh"
 #include "fm_sm100.cuh"
+#include "fm_square.cuh"
 
 namespace fm {
 
@@ -58,6 +59,7 @@ struct WArgs {
   const stat_t* stat_k;
   int nrows, ncols, off, mask, ntr, chunk, by_tile;
   float a0, a1, a2, lim;
+  Square sq;             // SQ
   int o_heads;           // MODE_FWD: > 0 writes out as (batch, nrows, o_heads, 64)
 };
 
@@ -96,10 +98,7 @@ struct WCfg {
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_wtc_status, 0, code); }
 
 // GQ: grouped k/v heads (bh > bhkv); the plain case compiles without the head walk.
-// SQ (MODE_DKDV without grouped heads, a2 > 0): the polynomial in completed-square form,
-//   f(s) = A2 ((s + b)^2 + c),  f'(s) = 2 A2 (s + b),  b = A1 / (2 A2),  c = A0 / A2 - b^2,
-// so that a pair of scores costs t = s + b, P' = t t + c, E' = t (w - dvec): four packed operations
-// instead of five.  The factors A2 (grad_v) and 2 A2 (grad_k) multiply the accumulators in the epilogue.
+// SQ (MODE_DKDV without grouped heads): the polynomial as a square and a rest (fm_square.cuh).
 template <int MODE, bool GQ, bool SQ = false>
 __global__ void __launch_bounds__(kThreads, 1)
 dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
@@ -347,8 +346,8 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     const uint64_t A0v = pack2(A0, A0);
     using coef_t = typename std::conditional<GQ, uint64_t, const uint64_t>::type;   // fixed unless heads are grouped
     coef_t A1v = pack2(A1, A1), A2v = pack2(A2, A2), A2d = pack2(2.f * A2, 2.f * A2);
-    const float sq_b = SQ ? A1 / (2.f * A2) : 0.f, sq_c = SQ ? A0 / A2 - sq_b * sq_b : 0.f;
-    const uint64_t Bv = pack2(sq_b, sq_b), Cv = pack2(sq_c, sq_c);
+    const float root = a.sq.root * c;
+    const uint64_t Rv = pack2(root, root), Bv = pack2(a.sq.shift, a.sq.shift), Cv = pack2(a.sq.rest, a.sq.rest);
     int limcol = a.ncols - 1, lowcol = 0;   // columns kept for this row: lowcol <= col <= limcol
     if (a.mask) {
       if (rev) lowcol = row - a.off;
@@ -483,7 +482,7 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             if (rev && (e & 1) == 0) nd2 = lds_v2(vec_s + (e >> 1) * 16);   // four column values per load
             const uint64_t ndl = rev ? ((e & 1) ? nd2.y : nd2.x) : ndl_row;
             if constexpr (SQ) {
-              const uint64_t t2 = add2(s2, Bv);
+              const uint64_t t2 = fma2(s2, Rv, Bv);
               pe[e] = pack_bf16_2(mul2(t2, add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl)));
               pp[e] = pack_bf16_2(fma2(t2, t2, Cv));
             } else {
@@ -500,7 +499,7 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             const int col = c0 + 2 * e;
             const bool z0 = col > limcol || col < lowcol, z1 = col + 1 > limcol || col + 1 < lowcol;
             float v0, v1;
-            const uint64_t t2 = SQ ? add2(s2, Bv) : fma2(A2d, s2, A1v);
+            const uint64_t t2 = SQ ? fma2(s2, Rv, Bv) : fma2(A2d, s2, A1v);
             unpack2(mul2(t2, add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl)), v0, v1);
             pe[e] = pack_bf16(z0 ? 0.f : v0, z1 ? 0.f : v1);
             if (FUSED) {
@@ -548,7 +547,7 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       const int cc = (part4 & 1) * 32;
       const bool dots_here = !FWD && !second && a.dots != nullptr;
       const float* add = second ? a.o2_add : a.o_add;
-      const float pre = SQ ? (second ? A2 : 2.f * A2) : 1.f;   // completed square: the factor left out of E' and P'
+      const float pre = SQ && !second ? 2.f * root : 1.f;      // the factor left out of E'
       const size_t orow = FWD ? out_row(head, row_ok ? row : 0, a.nrows, a.o_heads) : grow;
       const float part = store_row<32>(tl + (second ? T_O2 : T_O) + cc, row_ok,
                                        (__nv_bfloat16*)(second ? a.o2 : a.o) + orow * D + cc,
@@ -592,7 +591,7 @@ int launch_wide(const Ctx& c, const char* name, const void* x, const void* u, co
   a.ntr = (nrows + BM - 1) / BM;
   a.by_tile = rows_by_tile(a.mask && a.chunk == 0, heads, a.ntr, 1);
   dim3 grid((unsigned)((size_t)heads * a.ntr));
-  if (MODE == MODE_DKDV && kv_ratio == 1 && a.a2 > 0.f) {
+  if (MODE == MODE_DKDV && kv_ratio == 1 && square_form(a.a0, a.a1, a.a2, &a.sq)) {
     FM_CUDA_TRY(cudaFuncSetAttribute(dense_tc_wide_kernel<MODE, false, MODE == MODE_DKDV>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, WCfg<MODE>::SMEM));
     FM_LAUNCH(name, c.stream,
