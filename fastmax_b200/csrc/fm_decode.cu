@@ -717,16 +717,16 @@ int step_ctas(const fastmax_problem& p) {
 }
 
 // From how many tokens on a prompt's kernels beat few_kernel, which reads and writes whole rows but walks the tokens
-// one by one.  Measured, us, few_kernel / prompt kernel:
+// one by one.  Measured, us, few_kernel / prompt kernel (p = 1 stays below its line on tensor cores, whose sums truncate: error
+// 1.1 to 1.4 times few_kernel's at 14 to 23 tokens, for 12.4 / 10.5 at 16):
 //   CUDA cores (float32, d = 32), 64 heads: d = 64, p = 2: 69 / 70 at 44 tokens; p = 1: 15.0 / 10.4 at 33, 10.4 / 10.4 at 20;
 //                                 d = 128, p = 2: 462 / 391 at 44
 //   fm_decode_tc.cu   d = 64, p = 2: 8 heads 12.7 / 14.7 at 16, 16.7 / 14.7 at 24; 64: 43.5 / 43.3 at 24, 49.5 / 43.3 at 28;
 //                                    512: 277 / 324 at 24, 346 / 324 at 32
 //                     d = 128, p = 2: 8 heads 37 / 43 at 16, 47 / 44 at 24; 64: 277 / 319 at 24, 336 / 320 at 32
-//                     p = 1, 64 heads: d = 64 10.6 / 10.6 at 12, 12.4 / 10.5 at 16; d = 128 12.7 / 12.6 at 12
 long long append_min(const fastmax_problem& p) {
   const bool tc = p.dtype == FASTMAX_BF16 && p.d >= 64;
-  return p.p == 1 ? (tc ? 14 : 24) : (tc ? 28 : 40);
+  return p.p == 1 ? 24 : (tc ? 28 : 40);
 }
 
 // From how many CTAs on a step leaves the heads' sums to sum_kernel: a CTA then ends without a fence and an atomic's way to

@@ -5,11 +5,11 @@
 // The product of two bf16 numbers has at most 16 significand bits, so it is EXACTLY the sum of two bf16 numbers, its
 // rounding to bf16 and what that leaves, which one multiplication and one fused multiply-add on bf16 pairs deliver;
 // with the values as they are (bf16) every product the tensor core forms is exact, and what is rounded is the
-// float32 summation only: the accumulators hold 128 tokens at a time and are then added to float32 registers,
-// rounded to nearest.  (Finite keys and values: an infinite value times a low part that is exactly zero is NaN where a
+// float32 summation only: an accumulator holds 64 tokens and is then added to float32 registers, rounded to nearest.
+// (Finite keys and values: an infinite value times a low part that is exactly zero is NaN where a
 // plain sum would stay infinite; a row of the state that holds either gives NaN when it is read.)  Measured, 2-norm error
-// of the state against float64 after 4000 tokens: 1.6e-7, where the CUDA-core kernel, token by token, has 2.8e-6 (and this
-// one 9.3e-7 while the normaliser column was a running sum on the CUDA cores).
+// of the state against float64, N(0,1) keys, d = 64: 0.9e-7 after 64 and 128 tokens, 1.1e-7 after 1000, 1.5e-7 after 4000, and of
+// its normaliser column 0.4e-7 to 0.8e-7 (few_kernel, token by token: 0.9e-7 and 0.4e-7 after 28, append_kernel 2.8e-6 after 4000).
 //
 // Rows.  128 lanes of tensor memory are one tile of pairs (b, b + s mod d) at a fixed distance s around the ring
 // of features: d = 64 has two distances per tile (s = 0..32, every unordered pair once; half of s = 32 is left over),
@@ -20,14 +20,20 @@
 // loads the value and key tiles by TMA, warps 17 and 18 issue the products of the two tiles.  Per block of 128 tokens the
 // sixteen warps write the keys transposed to shared memory (yT[feature][token]; 16-byte chunks XOR-swizzled so that
 // the transposed stores and the row reads are both free of bank conflicts), then a thread forms its lane's 64 products
-// (half of the block: two warps share a lane quarter), sixteen at a time, and stores their parts as the A operand in tensor
-// memory; B is the value tile as TMA delivered it and, sixteen columns more, a column of ones that makes the normaliser.
-//   Measured, 64 heads, d = 64, p = 2: 4000 tokens 396 -> 281 us through the public entry, 40 tokens 64 -> 43 us of kernel
-// (append_kernel: 2.22 ms for the former).  Of it: products as bf16 pairs instead of eleven instructions on unpacked
-// float32, normaliser from the tensor core: 396 -> 351; blocks of 128 tokens instead of 64: 321; keys by TMA: 317; rows of the
-// state asked for seven at a time: 281.  What bounds it: a block's chain -- transposed stores, barrier, row reads,
-// products, tcgen05.st -- 3 700 cycles, of which the shared-memory port is busy for some 2 200 (row reads 1 000, the tensor
-// core's reads of B 640) and the tensor pipe for 1 300.  The transposition one block ahead with barriers of its own: 351.
+// (half of the block's: two warps share a lane quarter), sixteen at a time, and stores their parts as the A operand in tensor
+// memory; B is the value tile as TMA delivered it and, sixteen columns more, ones that make the normaliser: every K step's high
+// parts have a column of their own there, and its low parts another, so that the tensor core adds sixteen numbers of eight bits
+// to each and everything else is added in float32, rounded to nearest.  The two halves of a block have an accumulator each, because the tensor core truncates what it adds: 128 tokens in one had 1.5 to 2
+// times the error of 64.  There is no room for both beside the parts, so the second one lies over the parts of the first half,
+// and its products wait for the first half's; the other tile's are issued meanwhile.
+//   Measured, 64 heads, d = 64, p = 2: 4000 tokens 388 -> 284 us of kernel, 40 tokens 61 -> 40 (append_kernel: 2.22 ms for the
+// former).  Of it: products as bf16 pairs instead of eleven instructions on unpacked float32 and the normaliser from the tensor core
+// take off a ninth, blocks of 128 tokens instead of 64 8 %, keys by TMA 1 %, rows of the state asked for seven at a time 11 %; an
+// accumulator to either half of a block costs 9 % (261 with one, at up to twice the error; 292 when both halves' sums are taken
+// over before the parts are formed, 303 with the first half's products issued ahead of the second half's parts).  What bounds it: a
+// block's chain -- transposed stores, barrier, row reads, products, tcgen05.st, sums -- 4 000 cycles, of which the shared-memory port
+// is busy for some 2 200 (row reads 1 000, the tensor core's reads of B 640) and the tensor pipe for 1 300.  The transposition one
+// block ahead with barriers of its own was slower by a tenth.
 // The result goes through shared memory, because a lane is a row of 65 floats: whole rows are read, added and written
 // to both places of the pair.
 #include "fm_common.cuh"
@@ -46,7 +52,11 @@ constexpr int kGenWarps = 16, kGenThreads = kGenWarps * 32;
 constexpr int kProducerWarp = 16, kIssuerWarp = 17;     // and 18
 constexpr int kThreads = 19 * 32;
 constexpr int VT = TB * 128;                            // bytes of a tile of 64 columns
-constexpr int kTileCols = 256, kHi = 96, kLo = kHi + TB / 2;   // TMEM columns of a tile: accumulator (80), high parts, low parts
+// TMEM columns of a tile: the accumulator of half h of a block is at 80 h (64 value columns, 16 of the normaliser), the parts of
+// its K steps at 80 (h + 1).  So the second accumulator's value columns are where the first half's parts were: those of a lane
+// quarter's two warps (32 columns each: two steps' low, two steps' high parts) under the columns that the same warp reads.
+constexpr int kTileCols = 256, kHalfCols = 80, kHiOff = 16;
+__device__ __forceinline__ constexpr int part_col(int half, int warp, int step) { return kHalfCols * (half + 1) + 32 * warp + 8 * step; }
 
 template <int D>
 struct AT {
@@ -55,11 +65,12 @@ struct AT {
   static constexpr int NS = D == 64 ? 3 : 2;            // stages: a value tile and the key tiles
   static constexpr int STAGE = VT + D / 64 * VT;
   static constexpr int OFF_ONE = NS * STAGE;            // the TMA tiles stay on 1024-byte boundaries
-  static constexpr int OFF_Y = OFF_ONE + VT;
+  static constexpr int OFF_Y = OFF_ONE + 2 * VT;
   static constexpr int OFF_EP = 0;                      // float ep[2][128][65], where the stages were
+  static constexpr int OFF_E = 2 * 128 * 65 * 4;        // float e[2][128]: the second halves' part of the last column
   static constexpr int OFF_BAR = OFF_Y + 2 * YT;
-  static_assert(NS * STAGE >= 2 * 128 * 65 * 4, "room for the results");
-  static constexpr int NBAR = 2 * NS + 4;               // full, empty, a_full[2], done[2]
+  static_assert(NS * STAGE >= OFF_E + 2 * 128 * 4, "room for the results");
+  static constexpr int NBAR = 2 * NS + 6;               // full, empty, a_full[2], first half done[2], done[2]
   static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;   // TMEM address, max |k|^2 bits
   static constexpr int SMEM = OFF_MISC + 16 + 1024;
   static constexpr int TILES = (D == 64) ? 17 : 66;
@@ -82,11 +93,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t saddr) {
 }
 __device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); }
 __device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
-// One TMEM column.
-__device__ __forceinline__ void tmem_ld1(uint32_t taddr, uint32_t (&r)[1]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r[0]) : "r"(taddr) : "memory");
-}
-
 // Byte offset of token chunk c (8 tokens) of row f inside a transposed block.
 __device__ __forceinline__ uint32_t yt_off(int f, int c) { return (uint32_t)(f * (TB * 2) + ((c ^ (f & 7) ^ ((f >> 3) & 7)) << 4)); }
 
@@ -103,7 +109,8 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
   auto BAR_VF = [&](int s) { return bar0 + 8u * s; };
   auto BAR_VE = [&](int s) { return bar0 + 8u * (NS + s); };
   auto BAR_A = [&](int t) { return bar0 + 8u * (2 * NS + t); };
-  auto BAR_DONE = [&](int t) { return bar0 + 8u * (2 * NS + 2 + t); };
+  auto BAR_HALF = [&](int t) { return bar0 + 8u * (2 * NS + 2 + t); };
+  auto BAR_DONE = [&](int t) { return bar0 + 8u * (2 * NS + 4 + t); };
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_MISC);
   int* kmax_bits = (int*)(smem + C::OFF_MISC + 4);
 
@@ -115,15 +122,23 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
 
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) { mbar_init(BAR_VF(s), 1); mbar_init(BAR_VE(s), active + kGenWarps); }
-    for (int t = 0; t < 2; ++t) { mbar_init(BAR_A(t), kGenWarps / 2); mbar_init(BAR_DONE(t), 1); }
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(BAR_A(t), kGenWarps / 2);
+      mbar_init(BAR_HALF(t), 1);
+      mbar_init(BAR_DONE(t), 1);
+    }
     mbar_fence_init();
     *kmax_bits = __float_as_int(hs[0]);
   }
   if (warp == kIssuerWarp) tmem_alloc(smem_u32((const void*)tmem_slot), 512);
-  // the second block of B: a column of ones and fifteen of zeros (16-byte pieces, XOR-swizzled by the row); its other columns
-  // are not read
-  for (int i = tid; i < 2 * TB; i += kThreads)
-    *(uint4*)(smem + C::OFF_ONE + (i >> 1) * 128 + (((i & 1) ^ ((i >> 1) & 7)) << 4)) = make_uint4((i & 1) ? 0u : 0x3F80u, 0u, 0u, 0u);
+  // the second block of B, for high and for low parts: sixteen columns (two 16-byte pieces, XOR-swizzled by the row), of which
+  // one is one and the others zero -- the row's K step of its half, low parts four columns on; its other columns are not read
+  for (int i = tid; i < 4 * TB; i += kThreads) {
+    const int r = (i >> 1) % TB, low = i / (2 * TB), x = 4 * low + ((r >> 4) & 3);
+    const uint32_t one = i & 1 ? 0u : 0x3F80u << (16 * (x & 1));
+    *(uint4*)(smem + C::OFF_ONE + low * VT + r * 128 + (((i & 1) ^ (r & 7)) << 4)) =
+        make_uint4(x >> 1 == 0 ? one : 0u, x >> 1 == 1 ? one : 0u, x >> 1 == 2 ? one : 0u, x >> 1 == 3 ? one : 0u);
+  }
   fence_proxy_async();
   // the zero row of both buffers
   for (int i = tid; i < TB; i += kThreads)
@@ -156,17 +171,32 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
         if (!mbar_wait_warp(BAR_VF(s), (uint32_t)((j / NS) & 1))) { report(62); break; }
         if (!mbar_wait_warp(BAR_A(t), (uint32_t)(j & 1))) { report(63); break; }
         tc_fence_after();
-        const uint32_t b = desc_lo(sbase + s * C::STAGE, C::OFF_ONE - s * C::STAGE);   // the second block: the ones
-        if (elect_one()) {
-          // low parts first
-          if (a.n_new - (long long)j * TB >= TB) {
-            umma_ts_steps<TB / 16>(acc, acc + kLo, b, idesc, 0u);
-            umma_ts_steps<TB / 16>(acc, acc + kHi, b, idesc, 1u);
-          } else {
-            const int steps = (int)(a.n_new - (long long)j * TB + 15) / 16;
-            for (int x = 0; x < 2 * steps; ++x)
-              umma_ts_1(acc, acc + (x < steps ? kLo + 8 * x : kHi + 8 * (x - steps)), b + (x < steps ? x : x - steps) * 128, idesc, x > 0);
+        const uint32_t b_hi = desc_lo(sbase + s * C::STAGE, C::OFF_ONE - s * C::STAGE);   // the second block: the ones
+        const uint32_t b_lo = desc_lo(sbase + s * C::STAGE, C::OFF_ONE + VT - s * C::STAGE);
+        const int left = (int)(a.n_new - (long long)j * TB < TB ? a.n_new - (long long)j * TB : TB);
+        // the K steps of half h that hold tokens, low parts first
+        auto issue = [&](int h) {
+          const int steps = min((left - h * (TB / 2) + 15) / 16, TB / 32);
+#pragma unroll
+          for (int x = 0; x < TB / 16; ++x) {
+            const int ks = x % (TB / 32);
+            if (ks < steps)
+              umma_ts_1(acc + kHalfCols * h, acc + part_col(h, ks >> 1, ks & 1) + (x < TB / 32 ? 0 : kHiOff),
+                        (x < TB / 32 ? b_lo : b_hi) + (h * (TB / 32) + ks) * 128, idesc, x > 0);
           }
+        };
+        const bool two = left > TB / 2;
+        if (elect_one()) {
+          issue(0);
+          umma_commit(two ? BAR_HALF(t) : BAR_DONE(t));
+          if (!two) umma_commit(BAR_VE(s));
+        }
+        __syncwarp();
+        if (!two) continue;                              // (the last block)
+        if (!mbar_wait_warp(BAR_HALF(t), (uint32_t)(j & 1))) { report(67); break; }
+        tc_fence_after();
+        if (elect_one()) {
+          issue(1);
           umma_commit(BAR_DONE(t));
           umma_commit(BAR_VE(s));
         }
@@ -191,24 +221,31 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
     }
     const uint32_t tl = tmem + t * kTileCols + ((uint32_t)(qd * 32) << 16);
     uint64_t run[16];
-    float run_e = 0.f;                                   // normaliser column (hf == 0)
+    float run_e[4] = {0.f, 0.f, 0.f, 0.f};              // normaliser column: K steps of this warp's half of a block (0: the first)
 #pragma unroll
     for (int i = 0; i < 16; ++i) run[i] = 0ull;
-    auto promote = [&]() {
+    // the sums of half h of a block: this warp's 32 value columns, and for one half the normaliser's K steps
+    auto take = [&](int h) {
+      const uint32_t from = tl + h * kHalfCols;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int x = 0; x < 2; ++x) {
         uint32_t v[16];
-        tmem_ld16(tl + hf * 32 + h * 16, v);
+        tmem_ld16(from + hf * 32 + x * 16, v);
         tmem_wait_ld(v);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) run[8 * h + i] = add2(run[8 * h + i], pack2u(v[2 * i], v[2 * i + 1]));
+        for (int i = 0; i < 8; ++i) run[8 * x + i] = add2(run[8 * x + i], pack2u(v[2 * i], v[2 * i + 1]));
       }
-      if (hf == 0) {
-        uint32_t v[1];
-        tmem_ld1(tl + 64, v);
-        tmem_wait_ld(v);
-        run_e += __uint_as_float(v[0]);
+      if (h == hf) {
+        uint32_t e[8];
+        tmem_ld8(from + 64, e);
+        tmem_wait_ld(e);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) run_e[i] += __uint_as_float(e[i]) + __uint_as_float(e[4 + i]);
       }
+    };
+    auto done = [&](uint32_t bar, int j) {
+      if (ok && !mbar_wait(bar, (uint32_t)(j & 1))) { report(64); ok = false; }
+      tc_fence_after();
     };
     // 16 bytes (8 features) of one token per thread and load, from the key tiles (16-byte pieces, XOR-swizzled by the row;
     // zeros past the end).  Read at the end of the block before: in global loads, the wait for the row reads below was one
@@ -278,16 +315,17 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
         fetch(j + 1);
         continue;
       }
-      // K steps of this warp's half of the block that hold tokens (the last block's others are not multiplied)
-      const int steps = (int)(a.n_new - (long long)j * TB - hf * (TB / 2) + 15) >> 4;
-      // two chunks of 8 tokens at a time: their 16 operand words and the 32 running sums fit the registers
+      const long long left = a.n_new - (long long)j * TB;
+      // Two K steps of either half of the block, those that hold tokens (the others are not multiplied); two chunks of 8 tokens
+      // at a time: their 16 operand words and the 32 running sums fit the registers
 #pragma unroll
       for (int step = 0; step < TB / 32; ++step) {
-        if (step > 0 && step >= steps) break;
+        const int half = step >> 1, tok0 = half * (TB / 2) + hf * 32 + (step & 1) * 16;
+        if (step > 0 && tok0 >= left) break;
         uint32_t hi[8], lo[8];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          const uint32_t at = (uint32_t)(hf * (TB / 16) + step * 2 + c) << 4;
+          const uint32_t at = (uint32_t)(tok0 / 8 + c) << 4;
           const ulonglong2 x = lds_v2(xr ^ at), y = lds_v2(yr ^ at);
           const uint32_t xw[4] = {(uint32_t)x.x, (uint32_t)(x.x >> 32), (uint32_t)x.y, (uint32_t)(x.y >> 32)};
           const uint32_t yw[4] = {(uint32_t)y.x, (uint32_t)(y.x >> 32), (uint32_t)y.y, (uint32_t)(y.y >> 32)};
@@ -298,14 +336,15 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
             lo[4 * c + q] = as_u32(__hfma2(xv, yv, __hneg2(h)));      // exact: what rounding to eight bits left
           }
         }
-        if (step == 0 && j > 0) {     // the previous block's products are done: take its sums over, reuse the operand
-          if (ok && !mbar_wait(BAR_DONE(t), (uint32_t)((j - 1) & 1))) { report(64); ok = false; }
-          tc_fence_after();
-          promote();
+        if (step == 0 && j > 0) {     // the previous block's products are done: take the second half's sums over, reuse the operands
+          done(BAR_DONE(t), j - 1);
+          take(1);
         }
-        tmem_st8(tl + kHi + hf * (TB / 4) + step * 8, hi);
-        tmem_st8(tl + kLo + hf * (TB / 4) + step * 8, lo);
+        const uint32_t to = tl + part_col(half, hf, step & 1);
+        tmem_st8(to + kHiOff, hi);
+        tmem_st8(to, lo);
       }
+      if (j > 0) take(0);             // the first half's, while the parts are on their way
       fetch(j + 1);
       tmem_wait_st();
       tc_fence_before();
@@ -313,16 +352,18 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
       if (lane == 0) mbar_arrive(BAR_A(t));
     }
     if (on) {
-      if (ok && !mbar_wait(BAR_DONE(t), (uint32_t)((nblk - 1) & 1))) { report(65); ok = false; }
-      tc_fence_after();
-      promote();
+      done(BAR_DONE(t), nblk - 1);
+      take(0);
+      if (a.n_new - (long long)(nblk - 1) * TB > TB / 2) take(1);
     }
     asm volatile("bar.sync 1, 512;" ::: "memory");       // both tiles' products have read their stages
     if (on) {
       float* ep = (float*)(smem + C::OFF_EP) + (t * 128 + L) * 65;
 #pragma unroll
       for (int i = 0; i < 16; ++i) unpack2(run[i], ep[hf * 32 + 2 * i], ep[hf * 32 + 2 * i + 1]);
-      if (hf == 0) ep[64] = run_e;
+      const float e = (run_e[0] + run_e[1]) + (run_e[2] + run_e[3]);
+      if (hf == 0) ep[64] = e;
+      else ((float*)(smem + C::OFF_E))[t * 128 + L] = e;
     }
     if (blockIdx.x == 0 && kmax > 0.f) atomicMax(kmax_bits, __float_as_int(kmax));
   }
@@ -384,7 +425,7 @@ append_tc_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant_
         if (row2[i] != row1[i]) r2[c] = f;
       }
       if (cb == 0 && lane == 0) {
-        const float f = old[i][2] + ep[64];
+        const float f = old[i][2] + (ep[64] + ((const float*)(smem + C::OFF_E))[r0 + i * kWarps]);
         r1[D] = f;
         if (row2[i] != row1[i]) r2[D] = f;
       }

@@ -1,6 +1,6 @@
 """Prompt processing of the decode state at the sizes where its kernels change: the tensor-core kernel's blocks of 128
-tokens and their K steps of 16 (bf16, d 64 and 128), the CUDA-core kernel's batches, and the few-token kernel (below 14 and
-28 tokens at p = 1 and 2 for those, else 24 and 40); onto an empty and onto a filled state, against float64 sums.
+tokens and their K steps of 16 (bf16, d 64 and 128), the CUDA-core kernel's batches, and the few-token kernel (below 24
+tokens at p = 1; at p = 2 below 28 for those, else 40); onto an empty and onto a filled state, against float64 sums.
 
 Bound: products are exact (bf16) or rounded once (float32) and sums of up to n terms are accumulated in float32, so
 the error of an element is within n * 2^-24 of the sum of its terms' magnitudes; elements of a state of N(0,1) keys
@@ -57,6 +57,21 @@ def test_append_matches_float64_sums(heads, d, p, pieces, dtype):
     (2, 64, 1, (14, 128)), (2, 128, 1, (13, 257, 16)), (4, 64, 2, (3000,))])
 def test_append_at_the_edges_of_blocks_and_steps(heads, d, p, pieces):
     test_append_matches_float64_sums(heads, d, p, pieces, torch.bfloat16)
+
+
+@pytest.mark.parametrize("n", [64, 65, 100, 128, 200, 1000])
+def test_sums_of_a_prompt_stay_short_in_the_tensor_core(n):
+    """Its accumulators cut off what they add, by 2^-23 of the partial sum at most and by a third of that on average, always
+    towards zero.  With keys and values of one sign an accumulator of 64 tokens, four steps that see a quarter to all of its sum,
+    loses 2.5 x 2^-23 / 3 = 1.0e-7 (one of 128 tokens 1.8e-7); everything else is rounded to nearest.  The normaliser adds a step's
+    sixteen numbers only: roundings to nearest of random sign, which stay below 2^-24 of the sum."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    k, v = [torch.randn(4, n, 64, generator=g, device="cuda").abs().bfloat16() for _ in range(2)]
+    st = fastmax_b200.FastmaxDecodeState(4, 4, 64, dtype=torch.bfloat16, device="cuda:0")
+    st.append(k, v)
+    got, ref = rows_of(st.state, 4, 64, 2)[1], want(k, v, 2).cpu()
+    err = [float((a - b).norm() / b.norm()) for a, b in ((got[..., :64], ref[..., :64]), (got[..., 64], ref[..., 64]))]
+    assert err[0] < 1.4e-7 and err[1] < 2.0 ** -24, err
 
 
 @pytest.mark.parametrize("d,ratio", [(64, 1), (64, 5), (32, 6), (128, 3)])
