@@ -43,7 +43,7 @@ struct SR {
   static constexpr int NS = HAS_U ? (D == 64 ? 2 : 4) : 3;  // (two stages leave the next scores waiting for their tile)
   static constexpr int OFF_VEC = OFF_ST + NS * STAGE;       // row-sum exchange
   static constexpr int OFF_BAR = OFF_VEC + 2 * 2 * BM * 4;
-  static constexpr int NBAR = 2 * NXB + 1 + 2 * NS + 4;
+  static constexpr int NBAR = 2 * NXB + 1 + 2 * NS + 5;
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_TMEM + 16 + 1024;
   static_assert(CTAS * (SMEM + 1024) <= 228 * 1024, "shared memory of an SM");
@@ -73,13 +73,13 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bar0 = sbase + C::OFF_BAR;
-  // barrier map: x[NXB] | x free[NXB] | x in tensor memory | full[NS] | empty[NS] | s_full | s_free | p_full | pv_done
+  // barrier map: x[NXB] | x free[NXB] | x in tensor memory | full[NS] | empty[NS] | s_full | s_free | p_full | pv_done | row sums
   auto BAR_X = [&](int b) { return bar0 + 8u * b; };
   auto BAR_XE = [&](int b) { return bar0 + 8u * (NXB + b); };
   const uint32_t BAR_XT = bar0 + 8u * (2 * NXB);
   auto BAR_FULL = [&](int s) { return bar0 + 8u * (2 * NXB + 1 + s); };
   auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (2 * NXB + 1 + NS + s); };
-  const uint32_t BAR_S = bar0 + 8u * (2 * NXB + 1 + 2 * NS), BAR_SFREE = BAR_S + 8, BAR_P = BAR_S + 16, BAR_PV = BAR_S + 24;
+  const uint32_t BAR_S = bar0 + 8u * (2 * NXB + 1 + 2 * NS), BAR_SFREE = BAR_S + 8, BAR_P = BAR_S + 16, BAR_PV = BAR_S + 24, BAR_RS = BAR_S + 32;
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_TMEM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -97,6 +97,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     mbar_init(BAR_SFREE, kComputeWarps);
     mbar_init(BAR_P, kComputeWarps);
     mbar_init(BAR_PV, 1);
+    mbar_init(BAR_RS, kComputeWarps);
     mbar_fence_init();
   }
   if (warp == kIssuerWarp) tmem_alloc(smem_u32((const void*)tmem_slot), C::T_COLS);
@@ -238,7 +239,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     };
     clear();
     // a finished row tile: each compute thread owns half of the features of one row
-    auto finish = [&](int m, int head, int r0, uint64_t sums) {
+    auto finish = [&](int m, int head, int r0, uint64_t sums) -> bool {
       const int row = r0 + rl;
       const bool row_ok = row < a.nrows;
       const size_t grow = (size_t)head * a.nrows + (row_ok ? row : 0), at = grow * D + cpart * (D / 2);
@@ -247,7 +248,10 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         float lo, hi;
         unpack2(sums, lo, hi);
         rows_sum[cpart * BM + rl] = lo + hi;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        // (a warp that gave up is not waited for without a limit; the next sums go to the other buffer)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR_RS);
+        if (!mbar_wait(BAR_RS, (uint32_t)(m & 1))) { report(11); return false; }
         if (row_ok)
           store_forward<D>(a, run, grow, cpart, rows_sum[rl] + rows_sum[BM + rl] + (a.den_add ? a.den_add[grow] : 0.f));
       } else {
@@ -260,6 +264,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
       clear();
+      return true;
     };
     // the row tile whose last products are still under way: its head, first row and row sums
     int last_head = -1, last_r0 = 0;
@@ -347,7 +352,7 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR_P);
-        if (i == 0 && last_head >= 0) finish(w.m - 1, last_head, last_r0, last_sums);
+        if (i == 0 && last_head >= 0 && !(ok = finish(w.m - 1, last_head, last_r0, last_sums))) break;
       }
       last_head = w.head;
       last_r0 = w.r0;

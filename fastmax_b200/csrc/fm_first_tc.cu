@@ -579,7 +579,7 @@ struct F1G {
   static constexpr int VROW = 2 * DD + 4;          // a warp's sums: q e [DD], gs [DD], e
   static constexpr int OFF_VEC = OFF_E + NS * 512;
   static constexpr int OFF_BAR = OFF_VEC + FG_WARPS * VROW * 4;
-  static constexpr int NBAR = 4 * NS + 8;          // full, gs, grad_q, empty per stage; T, state, S full, S empty twice
+  static constexpr int NBAR = 4 * NS + 9;          // full, gs, grad_q, empty per stage; T, state, S full, S empty twice; meet
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_TMEM + 16 + 1024;
 };
@@ -627,6 +627,7 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   auto BAR_STATE = [&](int b) { return bar0 + 8u * (4 * NS + 2 + b); };
   auto BAR_SF = [&](int b) { return bar0 + 8u * (4 * NS + 4 + b); };
   auto BAR_SE = [&](int b) { return bar0 + 8u * (4 * NS + 6 + b); };
+  const uint32_t BAR_MEET = bar0 + 8u * (4 * NS + 8);
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem + C::OFF_TMEM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -643,6 +644,7 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       mbar_init(BAR_SF(b), 1);
       mbar_init(BAR_SE(b), 1);
     }
+    mbar_init(BAR_MEET, FG_WARPS);
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(smem_u32((const void*)tmem_slot), 4 * DD);
@@ -726,7 +728,15 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const int qd = warp & 3, cols = (warp - FG_FIRST) >> 2;   // TMEM lane quarter; quarter of the features
     constexpr int HC = DD / 4;
     static_assert(RPS % 8 == 0 && STEPS <= LPR, "a thread's rows have one swizzle; a row's threads hold the rows' den");
-    auto sync = []() { asm volatile("bar.sync 2, %0;" ::"n"(32 * FG_WARPS) : "memory"); };
+    // all of these warps, in the same order; one that gave up is not waited for without a limit
+    uint32_t met = 0;
+    auto meet = [&]() -> bool {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_MEET);
+      if (mbar_wait(BAR_MEET, met++ & 1u)) return true;
+      report(57);
+      return false;
+    };
     // its eight features summed over its rows: q e, gs; e
     uint64_t sq[4] = {0, 0, 0, 0}, sg[4] = {0, 0, 0, 0};
     float se = 0.f;
@@ -749,10 +759,10 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     auto form = [&](const F1Walk& p) -> bool {
       const int s = p.g % NS;
       if (p.t == 0) {          // the run's normaliser column, once nobody reads that of two runs ago
-        sync();
+        if (!meet()) return false;
         const float* src = a.total + (size_t)p.head * a.rows * a.dvp + (size_t)a.f_lin * a.dvp + DD;
         if (te < DD) ((float*)(smem + C::OFF_NCOL))[(p.m & 1) * DD + te] = __ldg(src + (size_t)te * a.dvp);
-        sync();
+        if (!meet()) return false;
       }
       if (!mbar_wait(BAR_FULL(s), (uint32_t)((p.g / NS) & 1))) { report(54); return false; }
       const uint32_t qt = sbase + s * C::STAGE + at0, gt = qt + C::TILE;
@@ -809,7 +819,7 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       return true;
     };
     // a run's vectors: column D and the constant row of its state
-    auto write_vectors = [&](const F1Walk& p) {
+    auto write_vectors = [&](const F1Walk& p) -> bool {
       float* const mine = (float*)(smem + C::OFF_VEC) + (warp - FG_FIRST) * C::VROW;
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
@@ -830,7 +840,7 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       for (int k = LPR; k < 32; k <<= 1) se += __shfl_xor_sync(0xffffffffu, se, k);
       if (lane == 0) mine[2 * DD] = se;
       se = 0.f;
-      sync();
+      if (!meet()) return false;
       auto total = [&](int i) {
         float v = 0.f;
 #pragma unroll
@@ -843,14 +853,14 @@ first_grad_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         for (int x = DD + 1; x < a.dvp; ++x) st[(size_t)te * a.dvp + x] = 0.f;
       }
       for (int x = te; x < a.dvp; x += 32 * FG_WARPS) st[(size_t)DD * a.dvp + x] = x < DD ? total(DD + x) : (x == DD ? total(2 * DD) : 0.f);
-      sync();
+      return meet();
     };
     float part = 0.f;
     F1Walk f(a);
     bool ok = true;
     auto form_next = [&]() {
       ok = form(f);
-      if (ok && f.last()) write_vectors(f);
+      if (ok && f.last()) ok = write_vectors(f);
       f.next();
       fetch(f);
     };
