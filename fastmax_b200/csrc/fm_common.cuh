@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "fastmax_b200.h"
 
 namespace fm {
@@ -58,6 +60,19 @@ __host__ __device__ __forceinline__ float stat_norm2(stat_t s) {
 }
 __host__ __device__ __forceinline__ int stat_row(stat_t s) {
   return (int)(0xFFFFFFFFu - (unsigned)(s & 0xFFFFFFFFull));
+}
+// Registers a thread that a kernel is launched with, asked for once (0 where the question fails, which is not an error of the call).
+template <class Kernel>
+int launch_registers(Kernel kernel, std::atomic<int>* known) {
+  int regs = known->load(std::memory_order_relaxed);
+  if (regs > 0) return regs;
+  cudaFuncAttributes at;
+  if (cudaFuncGetAttributes(&at, kernel) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  known->store(at.numRegs, std::memory_order_relaxed);
+  return at.numRegs;
 }
 // lim / max_n ||x_n||  (1 when the problem is not normalised: st == nullptr)
 __device__ __forceinline__ float stat_scale(const stat_t* st, int head, float lim) {

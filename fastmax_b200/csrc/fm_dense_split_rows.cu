@@ -392,12 +392,6 @@ int launch_rows(const Ctx& c, const char* name, const void* x, const void* u, co
   if ((rc = set_sizes(p, p.bh, p.nq, p.nk, &a, &blocks))) return rc;
   a.order = row_order(p, a.heads, a.ntr, CTAS);
   const auto kernel = split_rows_kernel<D, MODE, CTAS>;
-  // the compute warps of two CTAs wait for registers that the block must have been launched with
-  static const int regs = [&] {
-    cudaFuncAttributes at;
-    return cudaFuncGetAttributes(&at, kernel) == cudaSuccess ? at.numRegs : 0;
-  }();
-  if (CTAS == 2 && regs < C::REGS) return fail(FASTMAX_E_UNSUPPORTED, "%s: %d registers a thread at launch instead of %d", name, regs, C::REGS);
   FM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   const unsigned grid = (unsigned)(blocks < 148 * CTAS ? blocks : 148 * CTAS);
   FM_LAUNCH(name, c.stream, (kernel<<<grid, C::THREADS, C::SMEM, c.stream>>>(tx, tu, ty, tz, a)));
@@ -411,7 +405,11 @@ int split_rows_forward(const Ctx& c, const void* q, const void* k, const void* v
   if (c.p.d == 64) return launch_rows<64, MODE_FWD, 1>(c, "fm_dense_split_fwd", q, q, k, v, a);
   // where there is a second row tile for an SM: 512 heads x 1000 causal 220 us instead of 242, 60 x 4000 unmasked 607 instead
   // of 627; a single one takes a tenth longer without x in tensor memory
-  if ((long long)c.p.bh * ((c.p.nq + BM - 1) / BM) > 148) return launch_rows<32, MODE_FWD, 2>(c, "fm_dense_split_fwd", q, q, k, v, a);
+  // (the compute warps of two CTAs wait for registers that the block must have been launched with)
+  static std::atomic<int> regs{0};
+  if ((long long)c.p.bh * ((c.p.nq + BM - 1) / BM) > 148 &&
+      launch_registers(split_rows_kernel<32, MODE_FWD, 2>, &regs) >= SR<32, MODE_FWD, 2>::REGS)
+    return launch_rows<32, MODE_FWD, 2>(c, "fm_dense_split_fwd", q, q, k, v, a);
   return launch_rows<32, MODE_FWD, 1>(c, "fm_dense_split_fwd", q, q, k, v, a);
 }
 int split_rows_dq(const Ctx& c, const void* q, const void* gs, const void* k, const void* v, const SplitArgs& a) {

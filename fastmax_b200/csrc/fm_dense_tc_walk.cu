@@ -630,17 +630,17 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
   }
 }
 
+// the compute warps wait for registers that the block must have been launched with
+template <int MODE, bool SQ, bool FIRST>
+bool has_registers() {
+  static std::atomic<int> regs{0};
+  return launch_registers(walk_kernel<MODE, SQ, FIRST>, &regs) >= kRegsLaunch;
+}
+
 template <int MODE, bool SQ, bool FIRST>
 int start(const Ctx& c, const char* name, unsigned grid, const CUtensorMap& tx, const CUtensorMap& tu, const CUtensorMap& ty,
           const CUtensorMap& tz, const CUtensorMap& ta, const CUtensorMap& tb, const WalkArgs& a) {
   using C = WK<MODE, FIRST>;
-  // the compute warps wait for registers that the block must have been launched with
-  static const int regs = [] {
-    cudaFuncAttributes at;
-    return cudaFuncGetAttributes(&at, walk_kernel<MODE, SQ, FIRST>) == cudaSuccess ? at.numRegs : 0;
-  }();
-  if (regs < kRegsLaunch)
-    return fail(FASTMAX_E_UNSUPPORTED, "%s: %d registers a thread at launch instead of %d", name, regs, kRegsLaunch);
   FM_CUDA_TRY(cudaFuncSetAttribute(walk_kernel<MODE, SQ, FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   FM_LAUNCH(name, c.stream, (walk_kernel<MODE, SQ, FIRST><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, ta, tb, a)));
   FM_CUDA_TRY(cudaGetLastError());
@@ -693,6 +693,11 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
 }
 
 }  // namespace
+
+bool dense_tc_walk_runs(bool forward) {
+  if (forward) return has_registers<MODE_FWD, false, false>();
+  return has_registers<MODE_DKDV, false, false>() && has_registers<MODE_DKDV, true, false>() && has_registers<MODE_DKDV, false, true>();
+}
 
 int dense_tc_walk_forward(const Ctx& c, const void* q, const void* k, const void* v, const WalkArgs& a) {
   return launch<MODE_FWD>(c, "fm_dense_tc_fwd", q, nullptr, k, v, c.p.nq, c.p.nk, a, nullptr);

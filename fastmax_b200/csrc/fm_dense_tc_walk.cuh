@@ -36,6 +36,9 @@ struct WalkArgs {
 // Boxes of 128 rows x 32 of a (mats, rows, 64) float32 array, 128-byte swizzle (fm_dense_tc.cu)
 int tma_map_f32_rows(CUtensorMap* m, const float* base, size_t mats, size_t rows);
 
+// Whether the kernels have the registers that their warpgroups exchange, which the compiler decides; where not, the short and wide
+// kernels serve their rows.
+bool dense_tc_walk_runs(bool forward);
 int dense_tc_walk_forward(const Ctx& c, const void* q, const void* k, const void* v, const walk::WalkArgs& a);
 int dense_tc_walk_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, const walk::WalkArgs& a,
                        const FirstState* fs = nullptr);

@@ -659,7 +659,7 @@ static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
 static bool walk_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
   const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
   const long long tiles = (long long)p.bh * ((rows + BM - 1) / BM);
-  if (p.bh != p.bhkv || tiles <= 148) return false;
+  if (p.bh != p.bhkv || tiles <= 148 || !dense_tc_walk_runs(pass == 0)) return false;
   if (ca && ca->chunk > 0) return tiles > 2 * 148 && ca->chunk <= (pass == 2 ? 2048 : 4096);
   const int seen = p.mask ? cols / 2 : cols;
   if (!p.mask) return tiles > 2 * 148 && (pass == 2 ? seen >= 300 && seen <= 1300 : seen >= 450 && seen <= 3000);

@@ -86,3 +86,14 @@ def test_the_reading_finds_what_it_looks_for():
     assert not barriers_in_loops_that_warps_leave(leave + "while (more()) { if (ok && !mbar_wait(b, 0)) ok = false; meet(); } }")
     assert not barriers_in_loops_that_warps_leave(leave + "while (more()) { meet(); for (;;) { if (!ok) break; } } }")
     assert not barriers_in_loops_that_warps_leave(leave + "for (; ok && more(); next()) { } meet(); }")
+
+
+# Warpgroups that take registers wait for them until the block has them, so the block must have been launched with enough: the
+# compiler decides, and where it gave fewer another kernel serves the call.  A call that other kernels can serve is not refused.
+@pytest.mark.parametrize("name", ["fm_dense_tc_walk.cu", "fm_dense_split_rows.cu"])
+def test_missing_registers_choose_another_kernel(name):
+    with open(os.path.join(CSRC, name)) as f:
+        s = re.sub(r"//[^\n]*", "", f.read())
+    assert "regs_up<" in s
+    assert re.search(r"launch_registers\([^;]*>=", s)
+    assert not [c for c in re.findall(r"\bfail\([^;]*;", s) if re.search(r"\bregs|registers", c, re.I)]
