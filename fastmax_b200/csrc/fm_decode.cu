@@ -26,11 +26,11 @@
 // The kernels:
 //   step_kernel    one token and its read-out: bound by the state's traffic with many heads, by a chain of latencies with
 //                  few.  The lower triangle is written but never read: 4 F (d+1) x (1 + 0.56) bytes at d = 64.  Measured, us,
-//                  events around a launch included, p = 2: 1024 heads, d = 64: 312 for 1.73 GB = 5.5 TB/s (352 when every thread
-//                  fenced and each CTA waited for its arrival, 330 with one thread's fence); 8 key/value heads of 4 query heads
-//                  12.3 (12.8, and 16.8 when the queries were asked for after the update, the arriving CTA fenced its 24 KB of
-//                  state and the last one read the queries' shares in turn); 4 heads, float32, 10.5 (11.6); 128 heads, d = 128:
-//                  271 (334).  The same bytes in 2 KB runs, without the arithmetic: 258.  Other arrangements for 1024 heads:
+//                  p = 2: 1024 heads, d = 64: 312 for 1.73 GB = 5.5 TB/s (352 when every thread fenced and each CTA waited for its
+//                  arrival, 330 with one thread's fence); 128 heads, d = 128: 271 (334).  Steps one after another in a graph: 8
+//                  key/value heads of 4 query heads 8.9 (9.2 when every thread fenced), 4 heads, float32, 6.1 (6.3), 64 heads 22.8
+//                  (24.3); p = 1, whose head is one CTA at d 32 and 64, 64 heads of d = 32 3.8 (5.6 with a fence and a counter).
+//                  The same bytes in 2 KB runs, without the arithmetic: 258.  Other arrangements for 1024 heads:
 //                  several groups of blocks to a CTA 397, five CTAs to an SM 377 (both before the above); tiles by bulk copies
 //                  through shared memory, CTAs as here 366 / 291 (one kernel / without the sums; d = 128 319 / 264, kept),
 //                  persistent with 1 to 4 CTAs an SM 338 to 403.
@@ -261,8 +261,10 @@ template <int D> struct Block {
 // One token per head and its read-out.  A CTA takes one group of RPB blocks of its head and leaves their share of the
 // read-out in scratch[query head][CTA][column]; the CTA of a head that arrives last (a counter in the head's header) adds
 // the shares in CTA order, divides and writes the output row.
-// SHARES: that is all; sum_kernel does the rest.
-template <typename T, int D, bool SHARES>
+// SUMS says how: the last CTA to arrive; SUMS_APART: none, sum_kernel does the rest; SUMS_ALONE: the head is one CTA, which needs
+// neither fence nor counter.
+enum { SUMS_LAST = 0, SUMS_APART = 1, SUMS_ALONE = 2 };
+template <typename T, int D, int SUMS>
 __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_kernel(const DecArgs a, const T* __restrict__ q,
                                                                   const T* __restrict__ k, const T* __restrict__ v,
                                                                   float* __restrict__ state, float* __restrict__ scratch,
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
   typedef RunCfg<D> R;
   // With d = 128 a CTA has one tile, which bulk copies bring and take back: 264 instead of 295 us for 128 heads, the sums apart.
   // (With d = 64 291 instead of 294, with d = 32 107 instead of 99.)
-  constexpr bool BULK = SHARES && D == 128;
+  constexpr bool BULK = SUMS == SUMS_APART && D == 128;
   extern __shared__ __align__(16) float tile[];    // BULK
   __shared__ __align__(8) uint64_t tile_here;
   __shared__ float ks[D], vs[D + 1];       // the token; (v, 1)
@@ -392,24 +394,33 @@ __global__ void __launch_bounds__(DecCfg<D>::THREADS, DecCfg<D>::PER_SM) step_ke
       __stcg(scratch + ((qh + g) * gridDim.x + blockIdx.x) * C::DV + cc, tot);
     }
   }
-  if constexpr (SHARES) {
+  if constexpr (SUMS == SUMS_APART) {
     if (!bulk) blk.store();
     else if (here) blk.store_edges(r, x, c);
     if (copies) tma_store_wait_read();     // the bulk copies have read this CTA's shared memory
     return;
   }
-  __syncthreads();
-  // one thread's fence, for all of the CTA: the others go on to their stores.  One in the last warp, which has fewest
-  if (tid == C::THREADS - 1) {
-    __threadfence();
-    const int before = atomicAdd(reinterpret_cast<int*>(hs + 2), 1);
-    s_last = before == (int)gridDim.x - 1;
+  if constexpr (SUMS == SUMS_LAST) {
+    // One thread's fence, for all of the CTA: the others go on to their stores.  With few CTAs that leave several queries' shares
+    // each, every thread fences its own ahead of the barrier.  us, every thread / the last one / the first one: 8 heads 7.47 / 7.55 /
+    // 7.39, 9 heads 7.43 / 7.65 / 7.29, 20 heads 10.94 / 10.54 / 10.58, 64 heads of d = 32 7.73 / 7.47 / 7.21; 2 key/value heads of 4
+    // queries 7.20 / 7.26 / 7.25, 16 of 4 11.73 / 10.99 / 11.00
+    const bool each = a.ratio > 1 && gridDim.x * gridDim.y <= 100;
+    if (each) __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      if (!each) __threadfence();
+      const int before = atomicAdd(reinterpret_cast<int*>(hs + 2), 1);
+      s_last = before == (int)gridDim.x - 1;
+    }
   }
   // The block is written only now: the fence above need not wait for it, and a CTA leaves with its stores in flight.
   blk.store();
   __syncthreads();
-  if (!s_last) return;
-  __threadfence();
+  if constexpr (SUMS == SUMS_LAST) {
+    if (!s_last) return;
+    __threadfence();
+  }
   if (tid == 0) {
     hs[0] = s_kmax2;
     // the token count is an integer bit pattern in the float slot: exact past 2^24 tokens
@@ -755,17 +766,21 @@ int launch_decode(const fastmax_problem& p, const void* q, const void* k, const 
     if constexpr (READ) {
       if (p.p == 2 && grid.x * (long long)p.bhkv >= kSharesFrom<D>) {
         const int smem = D == 128 ? RunCfg<D>::SMEM : 0;
-        FM_CUDA_TRY(cudaFuncSetAttribute(step_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        FM_CUDA_TRY(cudaFuncSetAttribute(step_kernel<T, D, SUMS_APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         FM_LAUNCH("fm_decode_step", st,
-                  (step_kernel<T, D, true><<<grid, DecCfg<D>::THREADS, smem, st>>>(a, (const T*)q, (const T*)k, (const T*)v,
+                  (step_kernel<T, D, SUMS_APART><<<grid, DecCfg<D>::THREADS, smem, st>>>(a, (const T*)q, (const T*)k, (const T*)v,
                                                                                    state, scratch, (T*)out)));
         FM_CUDA_TRY(cudaGetLastError());
         FM_LAUNCH("fm_decode_sum", st,
                   (sum_kernel<T, D><<<p.bh, DecCfg<D>::THREADS, 0, st>>>(a, (int)grid.x, (const T*)k, state, scratch, (T*)out)));
+      } else if (grid.x == 1) {
+        FM_LAUNCH("fm_decode_step", st,
+                  (step_kernel<T, D, SUMS_ALONE><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
+                                                                                     scratch, (T*)out)));
       } else {
         FM_LAUNCH("fm_decode_step", st,
-                  (step_kernel<T, D, false><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
-                                                                                 scratch, (T*)out)));
+                  (step_kernel<T, D, SUMS_LAST><<<grid, DecCfg<D>::THREADS, 0, st>>>(a, (const T*)q, (const T*)k, (const T*)v, state,
+                                                                                    scratch, (T*)out)));
       }
     } else
       FM_LAUNCH("fm_decode_append", st,

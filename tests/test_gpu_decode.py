@@ -94,21 +94,43 @@ def test_steps_match_the_oracle_recurrence_with_other_coefficients(p):
         assert err < TOL[torch.float32], (t, err)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("normalize", [True, False], ids=["norm", "plain"])
 @pytest.mark.parametrize("heads,ratio,d", [(400, 1, 32), (513, 5, 32), (328, 1, 64), (23, 4, 128), (26, 1, 128)])
-def test_steps_of_many_heads_equal_those_of_few(heads, ratio, d):
+def test_steps_of_many_heads_equal_those_of_few(heads, ratio, d, normalize, dtype):
     """From some number of CTAs on a second kernel adds up a step's shares, in the order of the first one's last CTA: the state
-    must be the same to the bit, the rows up to the order of at most 139 additions per column."""
+    must be the same to the bit, the rows up to the order of at most 139 additions per column (139 x 2^-24 of the sum of the
+    magnitudes, which is within a few times the largest value).  One head's rows against float64."""
     g = torch.Generator(device="cuda").manual_seed(d)
-    mk = lambda n: torch.randn(n, 1, d, generator=g, device="cuda").bfloat16()  # noqa: E731
-    whole = FastmaxDecodeState(heads * ratio, heads, d, device="cuda:0")
-    cut = heads // 3
-    parts = [FastmaxDecodeState(n * ratio, n, d, device="cuda:0") for n in (cut, heads - 2 * cut, cut)]
+    scale = 1.0 if normalize else d ** -0.5
+    mk = lambda n, c: (torch.randn(n, 1, d, generator=g, device="cuda") * c).to(dtype)  # noqa: E731
+    state = lambda n: FastmaxDecodeState(n * ratio, n, d, dtype=dtype, device="cuda:0", normalize=normalize)  # noqa: E731
+    whole, cut, seen = state(heads), heads // 3, []
+    parts = [state(n) for n in (cut, heads - 2 * cut, cut)]
+
+    def step(st, *t):
+        _cabi.profile(True)
+        out = st.step(*t)
+        names = [n for n, _ in _cabi.profile_records()]
+        _cabi.profile(False)
+        return out, names
+
     for _ in range(3):
-        q, k, v = mk(heads * ratio), mk(heads), mk(heads)
-        out, lo = whole.step(q, k, v), 0
+        q, k, v = mk(heads * ratio, scale), mk(heads, scale), mk(heads, 1.0)
+        (out, names), lo = step(whole, q, k, v), 0
+        assert names == ["fm_decode_step", "fm_decode_sum"]
         for p in parts:
             n = p.bhkv
-            want = p.step(q[lo * ratio:(lo + n) * ratio].contiguous(), k[lo:lo + n].contiguous(), v[lo:lo + n].contiguous())
-            assert torch.allclose(out[lo * ratio:(lo + n) * ratio].float(), want.float(), rtol=2 ** -7, atol=1e-4)
+            want, names = step(p, q[lo * ratio:(lo + n) * ratio].contiguous(), k[lo:lo + n].contiguous(), v[lo:lo + n].contiguous())
+            assert names == ["fm_decode_step"]
+            assert torch.allclose(out[lo * ratio:(lo + n) * ratio].float(), want.float(), atol=1e-4,
+                                  rtol=2 ** -7 if dtype == torch.bfloat16 else 1e-5)
             lo += n
+        seen.append((k[cut].cpu(), v[cut].cpu()))
+        ks, vs = [torch.cat(t)[None, None].double().expand(1, ratio, -1, -1) for t in zip(*seen)]
+        row = q[cut * ratio:(cut + 1) * ratio].cpu().double()[None]
+        ref = fastmax_dense(row, ks, vs, mask=1, normalize=int(normalize), p=2, a0=1.0, a1=1.0, a2=0.5, lim=1.0)[0]
+        got = out[cut * ratio:(cut + 1) * ratio].double().cpu()
+        assert float((got - ref).abs().max() / ref.abs().max()) < TOL[dtype]
     assert torch.equal(whole.state.view(-1), torch.cat([p.state.view(-1) for p in parts]))
+    assert _cabi.device_status() == 0
