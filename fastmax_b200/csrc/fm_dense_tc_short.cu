@@ -480,6 +480,16 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   }
 }
 
+// Whether the forward, whose registers and shared memory leave room for a third CTA on an SM, is to run with two.  The third
+// one waits for the tensor memory of a CTA of its own SM, so its start is covered, but it is bound to that SM, which evens
+// out over many row tiles only.  us, two / three: 322 row tiles of 800 causal columns 13.4 / 15.4, 357 14.9 / 16.6, 600 of 3000 8 %
+// slower, 720 1 % faster, 2048 of 450 52.4 / 49.4; rows of 150 columns 303 to 600 row tiles 7 to 11 % faster.
+constexpr int kTwoFit = 80 * 1024;
+bool two_ctas(long long tiles, int ncols, const ShortArgs& a) {
+  const int seen = a.chunk > 0 ? a.chunk / 2 : (a.mask ? ncols / 2 : ncols);
+  return tiles <= 666 && seen > 160;
+}
+
 template <int MODE>
 int launch(const Ctx& c, const char* name, const void* x, const void* u, const void* y, const void* z, int nrows,
            int ncols, ShortArgs a, const FirstState* fs = nullptr) {
@@ -521,8 +531,11 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
     FM_LAUNCH(name, c.stream, (short_kernel<MODE, true><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, ts, a)));
   } else {
     using C = SH<MODE, false>;
-    FM_CUDA_TRY(cudaFuncSetAttribute(short_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    FM_LAUNCH(name, c.stream, (short_kernel<MODE, false><<<grid, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, tx, a)));
+    // (the limit is the same for all calls: another thread may be between these two lines)
+    constexpr int most = MODE == MODE_FWD && C::SMEM < kTwoFit ? kTwoFit : C::SMEM;
+    const int smem = MODE == MODE_FWD && two_ctas(grid.x, ncols, a) ? most : C::SMEM;
+    FM_CUDA_TRY(cudaFuncSetAttribute(short_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    FM_LAUNCH(name, c.stream, (short_kernel<MODE, false><<<grid, kThreads, smem, c.stream>>>(tx, tu, ty, tz, tx, a)));
   }
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
