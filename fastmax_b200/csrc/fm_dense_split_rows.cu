@@ -390,7 +390,7 @@ int launch_rows(const Ctx& c, const char* name, const void* x, const void* u, co
   if ((rc = split_map<D>(&tz, z, p.bhkv, p.nk, BN))) return rc;
   long long blocks;
   if ((rc = set_sizes(p, p.bh, p.nq, p.nk, &a, &blocks))) return rc;
-  a.order = row_order(p, a.heads, a.ntr, CTAS);
+  a.order = row_order(p, a.heads, a.ntr, CTAS, a.chunk);
   const auto kernel = split_rows_kernel<D, MODE, CTAS>;
   FM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   const unsigned grid = (unsigned)(blocks < 148 * CTAS ? blocks : 148 * CTAS);

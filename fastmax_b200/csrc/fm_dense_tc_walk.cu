@@ -683,7 +683,7 @@ int launch(const Ctx& c, const char* name, const void* x, const void* u, const v
   a.a1 = p.a1;
   a.a2 = p.p == 2 ? p.a2 : 0.f;
   a.lim = p.lim;
-  a.order = row_order(p, a.heads, a.ntr, 1);
+  a.order = row_order(p, a.heads, a.ntr, 1, a.chunk);
   const long long blocks = (long long)a.heads * a.ntr;
   if (blocks > 0x7FFF0000LL) return fail(FASTMAX_E_ARG, "heads x row tiles = %lld exceeds the grid limit", blocks);
   const unsigned grid = (unsigned)(blocks < 148 ? blocks : 148);

@@ -7,15 +7,22 @@ namespace fm {
 
 // In which order row tiles are dealt out to the CTAs of a grid:
 //   ORDER_LINEAR   head by head (row tiles of the same length, or one to a CTA)
-//   ORDER_TILES    causal grids of a few waves: tile by tile over all chunks and heads, the longest first, every other round
-//                  backwards.  (Chunks head by head instead, float32 forward / grad_q, us: 8 heads of 8192 in chunks of 2048
-//                  111 / 187, so 94 / 150; 24 heads of 5000, d 32, in chunks of 1024 92 / 105, so 72 / 90)
-//   ORDER_PAIRS    longer causal grids: head by head, so that a head's column tiles stay in L2, the i-th longest row tile
-//                  together with the i-th shortest, so that every CTA gets the same work
+//   ORDER_TILES    causal: tile by tile over all chunks and heads, the longest first, every other round backwards
+//   ORDER_PAIRS    causal: head by head, so that a head's column tiles stay in L2, the i-th longest row tile of a head together
+//                  with the i-th shortest, so that every pair is the same work
+// A grid of up to eight waves goes by tiles.  (Chunks head by head instead, float32 forward / grad_q, us: 8 heads of 8192 in
+// chunks of 2048 111 / 187, so 94 / 150.)  Longer ones go in pairs where pairs fill their rounds, and in any case beyond
+// forty waves.  bf16 forward, tiles / pairs, as parts of what a CTA per row tile takes: 1300 causal columns (pairs fill 86 % of
+// theirs) 0.92 / 1.08 at 1188 row tiles, 0.90 / 1.05 at 2046, 0.85 / 1.01 at 3003; 2200 columns 0.88 / 0.97 at 1188 (80 %), 0.87 / 0.86 at
+// 2052 (99 %), 0.82 / 0.81 at 4104; chunks of 2048 0.82 / 0.75 at 2048 row tiles of whole chunks, 0.81 / 0.93 (grad_k + grad_v 0.86 / 1.24) at
+// 2106 where the last chunk is shorter.
 enum { ORDER_LINEAR = 0, ORDER_TILES = 1, ORDER_PAIRS = 2 };
-inline int row_order(const fastmax_problem& p, long long heads, long long ntr, int ctas_per_sm) {
-  if (!p.mask || heads * ntr <= 148 * ctas_per_sm) return ORDER_LINEAR;
-  return heads * ntr > 8LL * 148 * ctas_per_sm ? ORDER_PAIRS : ORDER_TILES;
+inline int row_order(const fastmax_problem& p, long long heads, long long ntr, int ctas_per_sm, int chunk) {
+  const long long ctas = 148LL * ctas_per_sm, tiles = heads * ntr, units = heads * ((ntr + 1) / 2), rounds = (units + ctas - 1) / ctas;
+  if (!p.mask || tiles <= ctas) return ORDER_LINEAR;
+  if (tiles <= 8 * ctas) return ORDER_TILES;
+  const bool even = chunk == 0 || ntr % (chunk / 128) == 0;
+  return tiles > 40 * ctas || (even && 100 * tiles >= 93 * 2 * ctas * rounds) ? ORDER_PAIRS : ORDER_TILES;
 }
 
 // Args: heads (row heads), ntr (row tiles of a head), order, nrows, ncols, off, mask, chunk, ratio.  REV: rows are keys, whose
