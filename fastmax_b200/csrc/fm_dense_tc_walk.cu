@@ -171,6 +171,11 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     auto read = [&](int m) { return mbar_wait(BAR_AF(m % C::ACCS), (uint32_t)((m / C::ACCS) & 1)); };
     if (warp == kProducerWarp) {
       // ================= TMA loads: row operands, Y tiles (DKDV: and Z tiles), rows to add =================
+      if (lane == 0) {
+        tma_prefetch_desc(&tmX);
+        tma_prefetch_desc(&tmY);
+        if (!FWD) { tma_prefetch_desc(&tmU); tma_prefetch_desc(&tmZ); }
+      }
       // the fp32 rows to add to the result of row tile x, once those of the one before have been read
       auto load_add = [&](int m, int r0, int head) -> bool {
         if (!a.o_add) return true;
@@ -259,6 +264,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       __syncwarp();
     } else if (FWD && warp == kIssuerWarp + 1) {
       // ================= TMA loads of the forward's Z tiles =================
+      if (lane == 0) tma_prefetch_desc(&tmZ);
       for (; ok && w.live(a); w.next(a))
         for (int i = 0; i < w.j; ++i, ++g) {
           const int s = g % NZ;

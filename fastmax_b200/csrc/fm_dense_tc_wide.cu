@@ -642,29 +642,38 @@ static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
 }
 
 // Whether the kernels that walk row tiles serve a pass (0 forward, 2 grad_k + grad_v): they cover the ends of a row tile and
-// keep the wide loop's pace, but deal their row tiles out beforehand, so a nearly empty last round costs a whole row tile, and
-// below some columns to a row tile the short kernels' two CTAs hide the ends better.  us, what served it before / walking:
-//   chunks        forward 121 / 115 at 4096 row tiles in chunks of 256, 241 / 181 of 2048, 375 / 302 of 4096, 20.8 / 18.7 at
-//                 320 row tiles of 256; grad_k + grad_v 205 / 166, 449 / 386, but 630 / 642 of 4096, and 29.1 / 24.9; no gain
-//                 of the forward at 200 row tiles.  First-order chunks (grad_k + grad_v): 189 / 183 of 512, 155 / 148 of 256,
-//                 27.3 / 25.1 at 320 row tiles of 512
-//   forward       causal, 2048 to 2200 row tiles: 61.8 / 76 at 400 columns, 72.2 / 66.0 at 1000, 170 / 163 at 4600, but
-//                 301 / 313 (3008 row tiles) at 6000; 208 / 176 (4096) at 2000; 480 to 1200 row tiles: 47.6 / 49.5 to
-//                 37.2 / 35.3 at 1000, 45.4 / 41.4 at 1500, 33.2 / 33.2 at 3600; 320 at most: 16.6 / 14.7 at 600 columns,
-//                 26.8 / 18.8 at 2200, 22.9 / 27.0 at 4000.  Unmasked: 47.4 / 45.5 at 450, 94.5 / 82.2 at 1600, 158 / 152
-//                 at 3600, and nothing at two rounds
-//   grad_k+grad_v causal, at most 320 row tiles: 25.0 / 20.9 at 600 columns, 33.2 / 22.9 at 1100, 31.2 / 31.2 (all 320) at
-//                 1000, but 29.1 / 31.1 at 1500; more row tiles: 31.2 / 33.2.  Unmasked: 78.1 / 72.0 at 300, 152 / 134 at
-//                 1200, 158 / 164 at 1600, and nothing at two rounds
+// keep the wide loop's pace, but deal their row tiles out beforehand, one CTA to an SM where the short kernels have two, so that
+// rounds which the row tiles do not fill cost more.  Time walking as part of what a CTA per row tile takes (the better of the
+// other kernels), B200:
+//   chunks        second order: forward 0.70 to 0.99 from 300 row tiles on, 1.00 at 200; chunks of 4096 0.76 to 0.95.  grad_k + grad_v
+//                 0.63 to 0.97 up to chunks of 2048, 0.87 to 1.04 for 3072, 0.97 to 1.23 for 4096.  First order (grad_k + grad_v only):
+//                 chunks of 512 0.86 to 0.99, but 1.09 at 300 row tiles; of 256 0.94 to 1.08
+//   forward       causal, up to two rounds of row tiles: 0.90 to 1.01 at 600 columns, 0.79 to 0.92 at 1000, 0.58 to 0.69 at 3000, 1.02 to
+//                 1.13 at 3800.  Up to four: 1.00 to 1.11 at 800 to 1300 columns, 0.92 to 1.00 from 1900 on.  More: 0.94 to 1.05 (others
+//                 0.92 to 0.96) at 600, 0.86 to 1.00 at 1000, 0.79 to 0.93 from 1900 on, 0.96 to 1.04 at 5200.
+//                 Unmasked: 1.00 to 1.24 up to 400 columns and at any number within two rounds; 0.92 to 1.04 at 650 and 800 below
+//                 eight rounds, 0.91 to 0.98 above; 0.82 to 0.98 from 1000 on
+//   grad_k+grad_v causal, up to two rounds: 0.75 to 0.92 at 600 columns, 0.71 to 0.84 at 1000, 1.06 to 1.22 at 1900; with a third
+//                 one 1.09 at 600, 1.03 at 1000.  Unmasked: 0.80 to 1.00 at 300 to 1300 columns, 1.03 to 1.25 from 1600 on; without
+//                 normalisation (whose dots the short kernel waits for) 1.00 to 1.07 in four rounds, where the short kernel's two CTAs
+//                 have two full ones
 static bool walk_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
   const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
-  const long long tiles = (long long)p.bh * ((rows + BM - 1) / BM);
-  if (p.bh != p.bhkv || tiles <= 148 || !dense_tc_walk_runs(pass == 0)) return false;
-  if (ca && ca->chunk > 0) return tiles > 2 * 148 && ca->chunk <= (pass == 2 ? 2048 : 4096);
+  const long long tiles = (long long)p.bh * ((rows + BM - 1) / BM), rounds = (tiles + 147) / 148;
+  if (p.bh != p.bhkv || rounds <= 1 || !dense_tc_walk_runs(pass == 0)) return false;
+  if (ca && ca->chunk > 0) {
+    if (p.p == 1) return tiles > 320 && ca->chunk >= 512 && ca->chunk <= 2048;
+    return rounds > 2 && ca->chunk <= (pass == 2 ? 2048 : 4096);
+  }
   const int seen = p.mask ? cols / 2 : cols;
-  if (!p.mask) return tiles > 2 * 148 && (pass == 2 ? seen >= 300 && seen <= 1300 : seen >= 450 && seen <= 3000);
-  if (tiles <= 320) return seen >= 300 && seen <= (pass == 2 ? 550 : 1500);
-  return pass == 0 && seen >= 500 && seen <= (tiles > 8 * 148 ? 2500 : 1900);
+  if (!p.mask) {
+    if (rounds <= 2) return false;
+    if (pass == 0) return seen >= (rounds > 8 ? 600 : 900) && seen <= 3000;
+    return seen >= 300 && seen <= 1300 && (p.normalize || rounds % 2 == 1 || rounds > 6);
+  }
+  // (a few row tiles more from 500 columns on: 0.92 to 1.05 there, and 20 and 40 heads of 1000 then give the same bits)
+  if (rounds <= 2 || (tiles <= 320 && seen >= 500)) return seen >= 300 && seen <= (pass == 2 ? 550 : 1500);
+  return pass == 0 && seen >= (rounds <= 4 ? 950 : 500) && seen <= 1900;
 }
 static walk::WalkArgs walk_args(const fastmax_problem& p, const stat_t* stats, const ChunkAdd* ca) {
   walk::WalkArgs a = {};

@@ -10,10 +10,12 @@ from fastmax_b200 import _cabi
 pytestmark = pytest.mark.gpu
 
 # bh, nq, nk, mask, p, normalize, chunk, walking kernels (forward; grad_k and grad_v)
-CASES = [(19, 1000, 1000, 1, 2, 1, 0, 2), (20, 1030, 1030, 1, 1, 0, 0, 2), (38, 1000, 1129, 1, 2, 1, 0, 1), (55, 690, 650, 0, 2, 1, 0, 2),
-         (60, 650, 520, 0, 1, 1, 0, 2), (75, 515, 515, 1, 2, 1, 256, 2), (34, 1281, 1281, 1, 2, 0, 512, 2), (240, 641, 641, 1, 2, 1, 256, 2),
-         (150, 1031, 1031, 1, 2, 1, 0, 1), (75, 515, 515, 1, 1, 1, 256, 1), (34, 1281, 1281, 1, 1, 0, 512, 1),
-         (240, 641, 641, 1, 1, 1, 256, 1)]
+CASES = [(19, 1000, 1000, 1, 2, 1, 0, 2), (20, 1030, 1030, 1, 1, 0, 0, 2), (38, 1900, 2029, 1, 2, 1, 0, 1), (55, 690, 650, 0, 2, 1, 0, 1),
+         (44, 900, 930, 0, 2, 1, 0, 2), (60, 650, 520, 0, 1, 1, 0, 1), (200, 650, 640, 0, 1, 0, 0, 2), (75, 515, 515, 1, 2, 1, 256, 2),
+         (34, 1281, 1281, 1, 2, 0, 512, 2), (240, 641, 641, 1, 2, 1, 256, 2), (150, 1031, 1031, 1, 2, 1, 0, 1), (75, 515, 515, 1, 1, 1, 512, 1),
+         (34, 1281, 1281, 1, 1, 0, 512, 1), (240, 641, 641, 1, 1, 1, 512, 1),
+         # in pairs: even and odd numbers of row tiles, whole chunks, a shorter last one
+         (185, 1024, 1024, 1, 2, 1, 0, 1), (185, 1900, 1900, 1, 2, 1, 0, 1), (185, 1024, 1024, 1, 2, 1, 512, 2), (560, 1281, 1281, 1, 2, 0, 512, 2)]
 
 
 @pytest.mark.parametrize("cfg", CASES, ids=["bh%dnq%dnk%dm%dp%dz%dc%dw%d" % c for c in CASES])
@@ -37,7 +39,7 @@ def test_row_walks_match_the_cuda_cores(cfg):
             got = run(q, k, v, go, **impl)
         torch.cuda.synchronize()
     names = [e.key for e in prof.key_averages()]
-    assert not names or sum("walk_kernel<" in n for n in names) == walking, names
+    assert sum("walk_kernel<" in n for n in names) == walking, names
     assert _cabi.device_status() == 0
     want = run(*[t.float() for t in (q, k, v, go)], impl="dense_ffma")
     for x, r, name in zip(got, want, ("out", "dq", "dk", "dv")):
@@ -45,5 +47,7 @@ def test_row_walks_match_the_cuda_cores(cfg):
         err = float(((x.float() - r).abs().amax((1, 2)) / r.abs().amax((1, 2))).max())
         assert err < 2e-2, (name, err)
     bt, _, _ = _cabi.forward_bt(q, k, v, bh // 2 if bh % 2 == 0 else bh, **kw, **impl)
-    # (chunks: the states are summed by atomics, so two calls may round differently)
-    torch.testing.assert_close(bt.transpose(1, 2).reshape(got[0].shape), got[0], rtol=2 ** -7 if chunk else 0, atol=2e-3 if chunk else 0)
+    if chunk and p == 2:         # (two issuers add the halves of a block to these chunks' states, in the order they come)
+        torch.testing.assert_close(bt.transpose(1, 2).reshape(got[0].shape), got[0], rtol=2 ** -7, atol=2e-3)
+    else:
+        assert torch.equal(bt.transpose(1, 2).reshape(got[0].shape), got[0])
