@@ -19,8 +19,9 @@
 // small cross terms are added before the leading ones, and the TMEM accumulators hold ONE 64-column tile; the
 // compute warps add every tile to float32 registers, rounded to nearest.
 //
-// The forward and grad_q are in fm_dense_split_rows.cu; here are the preparation of the operands and grad_k + grad_v, one CTA
-// per 128-row tile, 352 threads: warps 0-7 compute (warp % 4 = TMEM lane quarter = 32 rows, warp / 4 = half of the tile's 64
+// Here are the preparation of the operands and the kernels of one CTA per 128-row tile: grad_k + grad_v, and the forward and
+// grad_q of grids that those of fm_dense_split_rows.cu, whose CTAs go on from row tile to row tile, do not serve
+// (split_rows_serve).  352 threads: warps 0-7 compute (warp % 4 = TMEM lane quarter = 32 rows, warp / 4 = half of the tile's 64
 // columns, and half of the features when accumulators are read), warp 8 loads tiles by TMA, warp 9 issues X Y^T and U Z^T,
 // warp 10 the accumulating products.  S and W are single buffers that are refilled as soon as they are in registers, so the
 // tensor core works on the next tile's scores while the polynomial and the split of this one run on the CUDA cores.  All
@@ -51,31 +52,36 @@ using namespace split;
 
 constexpr int kThreads = 352, kProducerWarp = 8, kIssuerWarp = 9, kAccIssuerWarp = 10;
 
-template <int D>
+template <int D, int MODE>
 struct SC {
+  static constexpr bool rev = MODE == MODE_DKDV, HAS_U = MODE != MODE_FWD;
   static constexpr int ROW_SUB = BM * D * 2, ROW_TILE = 3 * ROW_SUB;
   static constexpr int COL_SUB = BN * D * 2, COL_TILE = 3 * COL_SUB, STAGE = 2 * COL_TILE;
-  static constexpr int OFF_U = ROW_TILE, OFF_ST = 2 * ROW_TILE;
-  static constexpr int NS = D == 64 ? 2 : 4;
-  static constexpr int OFF_VEC = OFF_ST + NS * STAGE;       // per compute warp 2 x 32 floats
+  static constexpr int OFF_U = ROW_TILE, OFF_ST = (HAS_U ? 2 : 1) * ROW_TILE;
+  static constexpr int NS = HAS_U ? (D == 64 ? 2 : 4) : 3;
+  static constexpr int OFF_VEC = OFF_ST + NS * STAGE;       // per compute warp 2 x 32 floats; row-sum exchange
   static constexpr int OFF_BAR = OFF_VEC + kComputeWarps * 2 * 32 * 4;
   static constexpr int NBAR = 3 + 2 * NS + 4;
   static constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
   static constexpr int SMEM = OFF_TMEM + 16 + 1024;
-  // TMEM columns: S 64 | W 64 | three parts of 32 packed columns of E | of P | accumulators of 64 columns (d = 32: leading
-  // terms 32, cross terms with ym or yl 32) | x where there is room (3 d / 2 columns)
-  enum : int { T_S = 0, T_W = BN, T_E = 2 * BN, T_P = T_E + 96, T_A1 = T_P + 96, T_A2 = T_A1 + 64, T_X = T_A2 + 64, T_COLS = 512 };
-  static constexpr bool X_IN_T = D == 32;
+  // TMEM columns: S 64 | W 64 | three parts of 32 packed columns (P, or E and P) | accumulators of 64 columns (d = 32: leading
+  // terms 32, cross terms with ym or yl 32) | row operands as far as there is room (3 d / 2 columns each)
+  enum : int {
+    T_S = 0, T_W = BN, T_E = HAS_U ? 2 * BN : BN, T_P = T_E + 96, T_A1 = rev ? T_P + 96 : T_E + 96, T_A2 = T_A1 + 64,
+    T_X = rev ? T_A2 + 64 : T_A1 + 64, T_U = T_X + 3 * D / 2, T_COLS = 512
+  };
+  static constexpr bool X_IN_T = !rev || D == 32, U_IN_T = MODE == MODE_DQ;
 };
 
 __device__ __forceinline__ void report(int code) { atomicCAS(&g_split_status, 0, code); }
 
-template <int D>
+template <int D, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
-split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
+split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
              const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmZ, const SplitArgs a) {
-  using C = SC<D>;
+  using C = SC<D, MODE>;
   constexpr int NS = C::NS;
+  constexpr bool rev = C::rev, HAS_U = C::HAS_U;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -91,17 +97,24 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   // longest rows first (row_tile_of)
   int head, pidx;
   row_tile_of(blockIdx.x, a.order, a.ntr, head, pidx);
-  const int r0 = pidx * BM;
+  const int r0 = (rev ? pidx : a.ntr - 1 - pidx) * BM;
 
-  const int ntile = (a.ncols + BN - 1) / BN;
-  const int tb = a.mask ? max(0, r0 - a.off) / BN : 0;
-  const int te = a.chunk > 0 ? min(ntile, (r0 / a.chunk + 1) * (a.chunk / BN)) : ntile;   // the row tile lies in one chunk
+  int tb = 0, te = (a.ncols + BN - 1) / BN;
+  if (a.mask) {
+    if (rev) tb = max(0, r0 - a.off) / BN;
+    else te = min(te, (min(r0 + BM - 1, a.nrows - 1) + a.off) / BN + 1);
+  }
+  if (a.chunk > 0) {        // the row tile lies in one chunk (chunk % 256 == 0)
+    const int cb = (r0 / a.chunk) * (a.chunk / BN);
+    if (rev) te = min(te, cb + a.chunk / BN);
+    else tb = cb;
+  }
   // grouped heads: a key/value head walks its tile range once per query head of the group
-  const int Jh = max(te - tb, 0), J = Jh * a.ratio;
+  const int Jh = max(te - tb, 0), J = rev ? Jh * a.ratio : Jh;
   struct ColPos { int t, h; };
-  const ColPos pos0 = {tb, head * a.ratio};
+  const ColPos pos0 = {tb, rev ? head * a.ratio : head / a.ratio};
   auto advance = [&](ColPos& cp) {
-    if (++cp.t >= tb + Jh) { cp.t = tb; ++cp.h; }
+    if (++cp.t >= tb + Jh && rev) { cp.t = tb; ++cp.h; }
   };
 
   if (tid == 0) {
@@ -123,19 +136,21 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // where the two column halves of a row exchange their row sums (FWD)
+  float* const rows_sum = (float*)(smem + C::OFF_VEC);
   bool ok_compute = true;
-  uint64_t run1[D / 4], run2[D / 4];
+  uint64_t run1[D / 4], run2[rev ? D / 4 : 1];
   if (warp == kProducerWarp) {
     // ================= TMA producer =================
     if (lane == 0 && J > 0) {
       tma_prefetch_desc(&tmX);
-      tma_prefetch_desc(&tmU);
+      if (HAS_U) tma_prefetch_desc(&tmU);
       tma_prefetch_desc(&tmY);
       tma_prefetch_desc(&tmZ);
-      mbar_expect_tx(BAR_X, 2 * C::ROW_TILE);
+      mbar_expect_tx(BAR_X, (HAS_U ? 2 : 1) * C::ROW_TILE);
       for (int p = 0; p < 3; ++p) {
         tma_load_3d(sbase + p * C::ROW_SUB, &tmX, BAR_X, p * D, r0, head);
-        tma_load_3d(sbase + C::OFF_U + p * C::ROW_SUB, &tmU, BAR_X, p * D, r0, head);
+        if (HAS_U) tma_load_3d(sbase + C::OFF_U + p * C::ROW_SUB, &tmU, BAR_X, p * D, r0, head);
       }
     }
     ColPos pc = pos0;
@@ -168,7 +183,8 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const uint32_t y_lo = st_k + (uint32_t)s * (C::STAGE >> 4);
         if (elect_one()) {
           issue_scores<D, C::X_IN_T>(tmem + C::T_S, C::X_IN_T ? tmem + C::T_X : x_lo, y_lo);
-          issue_scores<D, false>(tmem + C::T_W, u_lo, y_lo + (C::COL_TILE >> 4));
+          if constexpr (HAS_U)
+            issue_scores<D, C::U_IN_T>(tmem + C::T_W, C::U_IN_T ? tmem + C::T_U : u_lo, y_lo + (C::COL_TILE >> 4));
           umma_commit(BAR_S);
         }
         __syncwarp();
@@ -185,8 +201,8 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         tc_fence_after();
         const uint32_t y_mn = st_mn + (uint32_t)s * (C::STAGE >> 4), z_mn = y_mn + (C::COL_TILE >> 4);
         if (elect_one()) {
-          issue_acc<D>(tmem + C::T_A1, tmem + C::T_E, y_mn);
-          issue_acc<D>(tmem + C::T_A2, tmem + C::T_P, z_mn);
+          issue_acc<D>(tmem + C::T_A1, tmem + C::T_E, HAS_U ? y_mn : z_mn);
+          if (rev) issue_acc<D>(tmem + C::T_A2, tmem + C::T_P, z_mn);
           umma_commit(BAR_PV);
           umma_commit(BAR_EMPTY(s));
           if (j + 1 == J) umma_commit(BAR_DONE);
@@ -199,7 +215,8 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     // ================= compute warps =================
     const int cpart = warp >> 2, qd = warp & 3;
     const int row = r0 + qd * 32 + lane;
-    const float ck = stat_scale(a.stat_k, head, a.lim);
+    const bool row_ok = row < a.nrows;
+    const float ck = stat_scale(a.stat_k, rev ? head : head / a.ratio, a.lim);
     const uint64_t A0v = pack2(a.a0, a.a0);
     uint64_t A1v, A2v, A2d;
     auto set_coefficients = [&](int hq) {
@@ -209,10 +226,16 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       A2v = pack2(A2, A2);
       A2d = pack2(2.f * A2, 2.f * A2);
     };
-    int hq_now = head * a.ratio;
+    int hq_now = rev ? head * a.ratio : head;
     set_coefficients(hq_now);
-    const int limcol = a.ncols - 1, lowcol = a.mask ? row - a.off : 0;     // columns kept: lowcol <= col <= limcol
-    const int wrow_hi = r0 + qd * 32 + 31;
+    int limcol = a.ncols - 1, lowcol = 0;                   // columns kept: lowcol <= col <= limcol
+    if (a.mask) {
+      if (rev) lowcol = row - a.off;
+      else limcol = min(limcol, row + a.off);
+    }
+    const int wrow_lo = r0 + qd * 32, wrow_hi = wrow_lo + 31;
+    const float dl_row = MODE == MODE_DQ && row_ok ? __ldg(a.dvec + (size_t)head * a.nrows + row) : 0.f;
+    const uint64_t ndl_row = pack2(-dl_row, -dl_row);
     const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
     float* myvec = (float*)(smem + C::OFF_VEC) + warp * 64;
     const uint32_t myvec_s = sbase + C::OFF_VEC + warp * 256;
@@ -223,23 +246,28 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       return (col < a.ncols) ? -__ldg(a.dvec + (size_t)cp.h * a.ncols + col) : 0.f;
     };
 #pragma unroll
-    for (int e = 0; e < D / 4; ++e) run1[e] = run2[e] = 0ull;
+    for (int e = 0; e < D / 4; ++e) {
+      run1[e] = 0ull;
+      if constexpr (rev) run2[e] = 0ull;
+    }
     bool ok = true;
     if (C::X_IN_T && J > 0) {
-      // copy x to tensor memory: column c of a part holds elements 2c and 2c+1 of the row; the two warps of a lane quarter
-      // take alternate parts.  (16-byte pieces, XOR-swizzled by the row's place in its swizzle atom)
+      // copy the row operands to tensor memory: column c of a part holds elements 2c and 2c+1 of the row; the two warps of a
+      // lane quarter take alternate parts.  (16-byte pieces, XOR-swizzled by the row's place in its swizzle atom)
       if (!mbar_wait(BAR_X, 0)) { report(6); ok = false; }
       if (ok) {
-        const int r = qd * 32 + lane, sw = (r >> 1) & 3;
-        for (int p = cpart; p < 3; p += 2) {
-          uint32_t w[16];
+        const int r = qd * 32 + lane, sw = D == 64 ? (r & 7) : ((r >> 1) & 3);
+        for (int it = cpart; it < (C::U_IN_T ? 6 : 3); it += 2) {
+          const uint32_t src = sbase + it * C::ROW_SUB + r * (D * 2), dst = tl + C::T_X + it * (D / 2);
+          uint32_t w[D / 2];
 #pragma unroll
-          for (int pc = 0; pc < 4; ++pc) {
-            const ulonglong2 v = lds_v2(sbase + p * C::ROW_SUB + r * (D * 2) + ((pc ^ sw) << 4));
+          for (int pc = 0; pc < D / 8; ++pc) {
+            const ulonglong2 v = lds_v2(src + ((pc ^ sw) << 4));
             w[4 * pc] = (uint32_t)v.x; w[4 * pc + 1] = (uint32_t)(v.x >> 32);
             w[4 * pc + 2] = (uint32_t)v.y; w[4 * pc + 3] = (uint32_t)(v.y >> 32);
           }
-          tmem_st16(tl + C::T_X + p * (D / 2), w);
+          if constexpr (D == 64) tmem_st32(dst, w);
+          else tmem_st16(dst, w);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -247,35 +275,46 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         if (lane == 0) mbar_arrive(BAR_XT);
       }
     }
+    uint64_t rs2 = 0ull;
     ColPos pc = pos0;
-    float nxt = fetch_vec(0, pc);
+    float nxt = rev ? fetch_vec(0, pc) : 0.f;
     for (int j = 0; ok && j < J; ++j, advance(pc)) {
       const float cur = nxt;
-      ColPos pn = pc;
-      advance(pn);
-      nxt = fetch_vec(j + 1, pn);
-      if (pc.h != hq_now) {
-        hq_now = pc.h;
-        set_coefficients(pc.h);
+      if (rev) {
+        ColPos pn = pc;
+        advance(pn);
+        nxt = fetch_vec(j + 1, pn);
+        if (pc.h != hq_now) {
+          hq_now = pc.h;
+          set_coefficients(pc.h);
+        }
       }
       if (!mbar_wait(BAR_S, (uint32_t)(j & 1))) { report(7); ok = false; break; }
       tc_fence_after();
       const uint32_t vec_s = myvec_s + (j & 1) * 128;
-      myvec[(j & 1) * 32 + lane] = cur;
-      __syncwarp();
-      uint32_t sv[32], wv[32];
+      if (rev) {
+        myvec[(j & 1) * 32 + lane] = cur;
+        __syncwarp();
+      }
+      uint32_t sv[32], wv[HAS_U ? 32 : 1];
       tmem_ld32(tl + C::T_S + cpart * 32, sv);
-      tmem_ld32(tl + C::T_W + cpart * 32, wv);
-      tmem_wait_ld(sv, wv);
+      if constexpr (HAS_U) {
+        tmem_ld32(tl + C::T_W + cpart * 32, wv);
+        tmem_wait_ld(sv, wv);
+      } else {
+        tmem_wait_ld(sv);
+      }
       // S and W of this tile are in registers: the next tile's may be issued
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(BAR_SFREE);
       const int c0 = pc.t * BN + cpart * 32;                // first of this warp's 32 columns
-      const bool need_mask = c0 + 32 > a.ncols || (a.mask && c0 < wrow_hi - a.off);
-      // E and P of the tile as three packed parts each
-      uint32_t e3[3][16], p3[3][16];
+      bool need_mask = c0 + 32 > a.ncols;
+      if (a.mask) need_mask = need_mask || (rev ? c0 < wrow_hi - a.off : c0 + 31 > wrow_lo + a.off);
+      // E (or P of the forward) and P of the tile as three packed parts each
+      uint32_t e3[3][16], p3[3][rev ? 16 : 1];
       ulonglong2 nd2 = make_ulonglong2(0ull, 0ull);
+      uint64_t ts2 = 0ull;                                  // row sums of this tile
       auto element = [&](int e, bool masked) {
         const uint64_t s2 = pack2u(sv[2 * e], sv[2 * e + 1]);
         bool z0 = false, z1 = false;
@@ -290,10 +329,16 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           unpack2(v, v0, v1);
           return pack2(z0 ? 0.f : v0, z1 ? 0.f : v1);
         };
-        if ((e & 1) == 0) nd2 = lds_v2(vec_s + (e >> 1) * 16);   // four column values per load
-        const uint64_t ndl = (e & 1) ? nd2.y : nd2.x;
-        split3(keep(mul2(fma2(A2d, s2, A1v), add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl))), e3[0][e], e3[1][e], e3[2][e]);
-        split3(keep(fma2(fma2(A2v, s2, A1v), s2, A0v)), p3[0][e], p3[1][e], p3[2][e]);
+        if constexpr (!HAS_U) {
+          const uint64_t pv = keep(fma2(fma2(A2v, s2, A1v), s2, A0v));
+          ts2 = add2(ts2, pv);
+          split3(pv, e3[0][e], e3[1][e], e3[2][e]);
+        } else {
+          if (rev && (e & 1) == 0) nd2 = lds_v2(vec_s + (e >> 1) * 16);   // four column values per load
+          const uint64_t ndl = rev ? ((e & 1) ? nd2.y : nd2.x) : ndl_row;
+          split3(keep(mul2(fma2(A2d, s2, A1v), add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl))), e3[0][e], e3[1][e], e3[2][e]);
+          if constexpr (rev) split3(keep(fma2(fma2(A2v, s2, A1v), s2, A0v)), p3[0][e], p3[1][e], p3[2][e]);
+        }
       };
       // the mask test stays outside the element loops so that each is one basic block of independent pairs
       if (!need_mask) {
@@ -303,6 +348,7 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 #pragma unroll
         for (int e = 0; e < 16; ++e) element(e, true);
       }
+      if (!HAS_U) rs2 = add2(rs2, ts2);
       // the previous tile's products must be done before their operands are overwritten; their sums are
       // taken over before the arrival below lets this tile's products replace them
       if (j > 0) {
@@ -312,11 +358,11 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 #pragma unroll
       for (int t = 0; t < 3; ++t) {
         tmem_st16(tl + C::T_E + 32 * t + cpart * 16, e3[t]);
-        tmem_st16(tl + C::T_P + 32 * t + cpart * 16, p3[t]);
+        if constexpr (rev) tmem_st16(tl + C::T_P + 32 * t + cpart * 16, p3[t]);
       }
       if (j > 0) {
         promote<D>(run1, tl + C::T_A1, cpart);
-        promote<D>(run2, tl + C::T_A2, cpart);
+        if constexpr (rev) promote<D>(run2, tl + C::T_A2, cpart);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -328,10 +374,15 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       else {
         tc_fence_after();
         promote<D>(run1, tl + C::T_A1, cpart);
-        promote<D>(run2, tl + C::T_A2, cpart);
+        if constexpr (rev) promote<D>(run2, tl + C::T_A2, cpart);
       }
     }
     ok_compute = ok;
+    if (!HAS_U) {
+      float lo, hi;
+      unpack2(rs2, lo, hi);
+      rows_sum[cpart * BM + qd * 32 + lane] = lo + hi;
+    }
   }
 
   tc_fence_before();
@@ -345,15 +396,20 @@ split_dkdv_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     const int cpart = warp >> 2, rl = (warp & 3) * 32 + lane, row = r0 + rl;
     const bool row_ok = row < a.nrows;
     const size_t grow = (size_t)head * a.nrows + (row_ok ? row : 0), at = grow * D + cpart * (D / 2);
-    float part = 0.f;
-    if (row_ok) {
-      part = store_half<D>(run1, a.o1 + at, a.o1_add ? a.o1_add + at : nullptr, a.dots ? a.x + at : nullptr, 1.f);
-      store_half<D>(run2, a.o2 + at, a.o2_add ? a.o2_add + at : nullptr, nullptr, 1.f);
-    }
-    if (a.dots) {
+    if constexpr (!HAS_U) {
+      if (row_ok)
+        store_forward<D>(a, run1, grow, cpart, rows_sum[rl] + rows_sum[BM + rl] + (a.den_add ? a.den_add[grow] : 0.f));
+    } else {
+      float part = 0.f;
+      if (row_ok) {
+        part = store_half<D>(run1, a.o1 + at, a.o1_add ? a.o1_add + at : nullptr, a.dots ? a.x + at : nullptr, 1.f);
+        if constexpr (rev) store_half<D>(run2, a.o2 + at, a.o2_add ? a.o2_add + at : nullptr, nullptr, 1.f);
+      }
+      if (a.dots) {
 #pragma unroll
-      for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
-      if (lane == 0) atomicAdd(a.dots + head, part);
+        for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(0xffffffffu, part, m);
+        if (lane == 0) atomicAdd(a.dots + head, part);
+      }
     }
   }
 }
@@ -440,23 +496,25 @@ int launch_split3(const Ctx& c, const SplitJobs& jobs, int count) {
   return FASTMAX_OK;
 }
 
-template <int D>
-int launch_dkdv(const Ctx& c, const void* k, const void* v, const void* q, const void* gs, SplitArgs a) {
-  using C = SC<D>;
+template <int D, int MODE>
+int launch_tiles(const Ctx& c, const char* name, const void* x, const void* u, const void* y, const void* z, SplitArgs a) {
+  using C = SC<D, MODE>;
   const fastmax_problem& p = c.p;
-  if (p.bhkv == 0 || p.nk == 0) return FASTMAX_OK;
+  const int heads = C::rev ? p.bhkv : p.bh, col_heads = C::rev ? p.bh : p.bhkv;
+  const int nrows = C::rev ? p.nk : p.nq, ncols = C::rev ? p.nq : p.nk;
+  if (heads == 0 || nrows == 0) return FASTMAX_OK;
   CUtensorMap tx, tu, ty, tz;
   int rc;
-  if ((rc = split_map<D>(&tx, k, p.bhkv, p.nk, BM))) return rc;
-  if ((rc = split_map<D>(&tu, v, p.bhkv, p.nk, BM))) return rc;
-  if ((rc = split_map<D>(&ty, q, p.bh, p.nq, BN))) return rc;
-  if ((rc = split_map<D>(&tz, gs, p.bh, p.nq, BN))) return rc;
+  if ((rc = split_map<D>(&tx, x, heads, nrows, BM))) return rc;
+  if ((rc = split_map<D>(&tu, u, heads, nrows, BM))) return rc;
+  if ((rc = split_map<D>(&ty, y, col_heads, ncols, BN))) return rc;
+  if ((rc = split_map<D>(&tz, z, col_heads, ncols, BN))) return rc;
   long long blocks;
-  if ((rc = set_sizes(p, p.bhkv, p.nk, p.nq, &a, &blocks))) return rc;
+  if ((rc = set_sizes(p, heads, nrows, ncols, &a, &blocks))) return rc;
   a.order = rows_by_tile(p.mask && a.chunk == 0, a.heads, a.ntr, 1);
-  FM_CUDA_TRY(cudaFuncSetAttribute(split_dkdv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-  FM_LAUNCH("fm_dense_split_dkdv", c.stream,
-            (split_dkdv_kernel<D><<<(unsigned)blocks, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, a)));
+  const auto kernel = split_kernel<D, MODE>;
+  FM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+  FM_LAUNCH(name, c.stream, (kernel<<<(unsigned)blocks, kThreads, C::SMEM, c.stream>>>(tx, tu, ty, tz, a)));
   FM_CUDA_TRY(cudaGetLastError());
   return FASTMAX_OK;
 }
@@ -504,7 +562,9 @@ int dense_split_forward(const Ctx& c, const void* q, const void* k, const void* 
   a.o_stride = o.o_stride;
   a.den_stride = o.den_stride;
   if (ca) { a.chunk = ca->chunk; a.o1_add = ca->out_add; a.den_add = ca->den_add; }
-  return split_rows_forward(c, q3, k3, v3, a);
+  if (split_rows_serve(p, MODE_FWD, a.chunk)) return split_rows_forward(c, q3, k3, v3, a);
+  if (p.d == 32) return launch_tiles<32, MODE_FWD>(c, "fm_dense_split_fwd", q3, q3, k3, v3, a);
+  return launch_tiles<64, MODE_FWD>(c, "fm_dense_split_fwd", q3, q3, k3, v3, a);
 }
 
 int dense_split_backward(const Ctx& c, const void* q, const void* k, const void* v, const void* out, const float* den,
@@ -536,14 +596,17 @@ int dense_split_backward(const Ctx& c, const void* q, const void* k, const void*
   a.o1_add = ca ? ca->gq_add : nullptr;
   a.x = (const float*)q;
   a.dots = p.normalize ? dots : nullptr;
-  if ((rc = split_rows_dq(c, q3, g3, k3, v3, a))) return rc;
+  if (split_rows_serve(p, MODE_DQ, a.chunk)) rc = split_rows_dq(c, q3, g3, k3, v3, a);
+  else rc = launch_tiles<64, MODE_DQ>(c, "fm_dense_split_dq", q3, g3, k3, v3, a);
+  if (rc) return rc;
   a.o1 = (float*)grad_k;
   a.o2 = (float*)grad_v;
   a.o1_add = ca ? ca->gk_add : nullptr;
   a.o2_add = ca ? ca->gv_add : nullptr;
   a.x = (const float*)k;
   a.dots = p.normalize ? dots + p.bh : nullptr;
-  return p.d == 32 ? launch_dkdv<32>(c, k3, v3, q3, g3, a) : launch_dkdv<64>(c, k3, v3, q3, g3, a);
+  if (p.d == 32) return launch_tiles<32, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, a);
+  return launch_tiles<64, MODE_DKDV>(c, "fm_dense_split_dkdv", k3, v3, q3, g3, a);
 }
 
 int split3_scaled_q(const Ctx& c, const void* q, void* q3, const void* v, void* v3, const stat_t* stats) {

@@ -25,14 +25,14 @@ struct SplitArgs {
   const stat_t* stat_q;
   const stat_t* stat_k;
   int heads, nrows, ncols, off, mask, ntr, chunk, ratio;   // heads: row heads
-  int order;              // FWD, DQ: see RowWalk; DKDV: see rows_by_tile
+  int order;              // row walks: see RowWalk; a CTA per row tile: see rows_by_tile
   int o_stride, den_stride;   // FWD: floats per row of out and den (the packed layout interleaves them)
   float a0, a1, a2, lim;
 };
 
 constexpr int BM = 128, BN = 64, kComputeWarps = 8;
 
-using Rows = RowWalk<SplitArgs, BN, false>;   // of the forward and grad_q
+using Rows = RowWalk<SplitArgs, BN, false>;   // of the forward's and grad_q's walks
 
 // ---- operands and products ----
 // A tile's part p (0 h, 1 m, 2 l) lies at p * SUB: rows of D bf16, 128 or 64 bytes, swizzled over their whole length.
@@ -216,6 +216,7 @@ inline int set_sizes(const fastmax_problem& p, int heads, int nrows, int ncols, 
 }  // namespace split
 
 // fm_dense_split_rows.cu; q, gs, k, v: parts
+bool split_rows_serve(const fastmax_problem& p, int mode, int chunk);
 int split_rows_forward(const Ctx& c, const void* q, const void* k, const void* v, const split::SplitArgs& a);
 int split_rows_dq(const Ctx& c, const void* q, const void* gs, const void* k, const void* v, const split::SplitArgs& a);
 

@@ -55,6 +55,9 @@ struct SR {
     T_S = 0, T_W = BN, T_E = HAS_U ? 2 * BN : BN, T_A = T_E + 96, T_X = T_A + 64, T_U = T_X + 3 * D / 2, T_COLS = 512 / CTAS
   };
   static constexpr int CH = CTAS == 2 ? 8 : 16;             // pairs of columns whose parts a thread holds at once
+  // Whether a pair is formed and split in one go.  us, d = 64: forward 269 instead of 277 (448 row tiles of 4000 columns), grad_q 483
+  // instead of 495; but grad_q of d = 32 198 instead of 190 (2400 of 1000)
+  static constexpr bool AT_ONCE = CTAS == 1 && D == 64;
 };
 
 __device__ __forceinline__ void put(uint32_t taddr, const uint32_t (&r)[8]) { tmem_st8(taddr, r); }
@@ -115,6 +118,12 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     if constexpr (CTAS == 2) regs_down<C::REGS_OTHER>();
     if (warp == kProducerWarp) {
       // ================= TMA producer =================
+      if (lane == 0) {
+        tma_prefetch_desc(&tmX);
+        if (HAS_U) tma_prefetch_desc(&tmU);
+        tma_prefetch_desc(&tmY);
+        tma_prefetch_desc(&tmZ);
+      }
       for (; ok && w.live(a); w.next(a)) {
         const int b = w.m % NXB;
         if (!mbar_wait(BAR_XE(b), (uint32_t)(((w.m / NXB) & 1) ^ 1))) { report(1); break; }
@@ -303,48 +312,75 @@ split_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
         const int c0 = (w.tb + i) * BN + cpart * 32;          // first of this warp's 32 columns
         const bool need_mask = c0 + 32 > a.ncols || (a.mask && c0 + 31 > w.r0 + qd * 32 + a.off);
-        // P or E in the place of the scores.  The mask test stays outside the loops so that each is one basic block of
-        // independent pairs
+        // P or E of a pair of columns.  The mask test stays outside the loops so that each is one basic block of independent
+        // pairs
         auto value = [&](int e) {
           const uint64_t s2 = pack2u(sv[2 * e], sv[2 * e + 1]), f = fma2(A2v, s2, A1v);
           if constexpr (HAS_U) return mul2(f, add2(pack2u(wv[2 * e], wv[2 * e + 1]), ndl_row));
           else return fma2(f, s2, A0v);
         };
-        auto keep = [&](int e, float lo, float hi) { sv[2 * e] = __float_as_uint(lo); sv[2 * e + 1] = __float_as_uint(hi); };
-        float lo, hi;
-        if (!need_mask) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            unpack2(value(e), lo, hi);
-            keep(e, lo, hi);
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            unpack2(value(e), lo, hi);
-            keep(e, c0 + 2 * e > limcol ? 0.f : lo, c0 + 2 * e + 1 > limcol ? 0.f : hi);
-          }
-        }
+        auto zero = [&](int e) { return c0 + e > limcol; };
         uint64_t ts2 = 0ull;                                  // row sums of this tile
-#pragma unroll
-        for (int k = 0; k < 16 / C::CH; ++k) {
-          uint32_t e3[3][C::CH];                              // three packed parts each of CH pairs
-#pragma unroll
-          for (int e = 0; e < C::CH; ++e) {
-            const int x = 2 * (C::CH * k + e);
-            const uint64_t v = pack2u(sv[x], sv[x + 1]);
+        if constexpr (C::AT_ONCE) {
+          uint32_t e3[3][16];
+          auto split = [&](int e, uint64_t v) {
             if constexpr (!HAS_U) ts2 = add2(ts2, v);
             split3(v, e3[0][e], e3[1][e], e3[2][e]);
+          };
+          if (!need_mask) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) split(e, value(e));
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              float lo, hi;
+              unpack2(value(e), lo, hi);
+              split(e, pack2(zero(2 * e) ? 0.f : lo, zero(2 * e + 1) ? 0.f : hi));
+            }
           }
           // the previous tile's products must be done before their operands are overwritten
-          if (k == 0 && g > 0) {
+          if (g > 0) {
             if (!mbar_wait(BAR_PV, (uint32_t)((g - 1) & 1))) { report(9); ok = false; break; }
             tc_fence_after();
           }
 #pragma unroll
-          for (int p = 0; p < 3; ++p) put(tl + C::T_E + 32 * p + cpart * 16 + C::CH * k, e3[p]);
+          for (int p = 0; p < 3; ++p) tmem_st16(tl + C::T_E + 32 * p + cpart * 16, e3[p]);
+        } else {
+          // in the place of the scores first
+          auto keep = [&](int e, float lo, float hi) { sv[2 * e] = __float_as_uint(lo); sv[2 * e + 1] = __float_as_uint(hi); };
+          float lo, hi;
+          if (!need_mask) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              unpack2(value(e), lo, hi);
+              keep(e, lo, hi);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              unpack2(value(e), lo, hi);
+              keep(e, zero(2 * e) ? 0.f : lo, zero(2 * e + 1) ? 0.f : hi);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 16 / C::CH; ++k) {
+            uint32_t e3[3][C::CH];                            // three packed parts each of CH pairs
+#pragma unroll
+            for (int e = 0; e < C::CH; ++e) {
+              const int x = 2 * (C::CH * k + e);
+              const uint64_t v = pack2u(sv[x], sv[x + 1]);
+              if constexpr (!HAS_U) ts2 = add2(ts2, v);
+              split3(v, e3[0][e], e3[1][e], e3[2][e]);
+            }
+            if (k == 0 && g > 0) {                            // (as above)
+              if (!mbar_wait(BAR_PV, (uint32_t)((g - 1) & 1))) { report(9); ok = false; break; }
+              tc_fence_after();
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p) put(tl + C::T_E + 32 * p + cpart * 16 + C::CH * k, e3[p]);
+          }
+          if (!ok) break;
         }
-        if (!ok) break;
         if (MODE == MODE_FWD) rs2 = add2(rs2, ts2);
         // its sums are taken over before the arrival below lets this tile's products replace them
         if (g > 0) promote<D>(run, tl + C::T_A, cpart);
@@ -401,16 +437,28 @@ int launch_rows(const Ctx& c, const char* name, const void* x, const void* u, co
 
 }  // namespace
 
-int split_rows_forward(const Ctx& c, const void* q, const void* k, const void* v, const SplitArgs& a) {
-  if (c.p.d == 64) return launch_rows<64, MODE_FWD, 1>(c, "fm_dense_split_fwd", q, q, k, v, a);
-  // where there is a second row tile for an SM: 512 heads x 1000 causal 220 us instead of 242, 60 x 4000 unmasked 607 instead
-  // of 627; a single one takes a tenth longer without x in tensor memory
-  // (the compute warps of two CTAs wait for registers that the block must have been launched with)
+// Which problems' forward (MODE_FWD) and grad_q (MODE_DQ) walk row tiles; fm_dense_split.cu has a CTA per row tile for the others.
+// Measured, walk as part of that:
+//   d = 32  forward (two CTAs per SM; one walking is 0 to 10 % slower than none): causal 0.78 to 0.93 from 300 row tiles of up to 1000
+//           columns on, but with 2100 to 4000 columns 1.08 to 1.12 at 310 row tiles, 1.00 to 1.04 at 340, 0.92 to 0.98 from 370
+//           on; up to 296 1.1 to 1.6.  Unmasked 0.75 to 1.00 from 300 on, 1.03 to 1.04 for 350 to 380 of 4000.  grad_q 0.80 to 1.00
+//           everywhere
+//   d = 64  forward 0.97 to 1.06 up to 296 row tiles, 0.84 to 1.01 above.  grad_q 1.00 to 1.07 up to 296, 0.82 to 1.01 above, but 1.00
+//           to 1.04 (unmasked, 3000 columns and more)
+bool split_rows_serve(const fastmax_problem& p, int mode, int chunk) {
+  const long long tiles = (long long)p.bh * ((p.nq + BM - 1) / BM);
+  const int most = chunk > 0 ? chunk : p.nk;         // columns of the longest row
+  if (p.d == 32 && mode == MODE_DQ) return true;
+  if (p.d == 64) return tiles > 2 * 148 && (mode == MODE_FWD || (p.mask ? most / 2 : most) <= 2000);
+  // the compute warps of two CTAs wait for registers that the block must have been launched with
   static std::atomic<int> regs{0};
-  if ((long long)c.p.bh * ((c.p.nq + BM - 1) / BM) > 148 &&
-      launch_registers(split_rows_kernel<32, MODE_FWD, 2>, &regs) >= SR<32, MODE_FWD, 2>::REGS)
-    return launch_rows<32, MODE_FWD, 2>(c, "fm_dense_split_fwd", q, q, k, v, a);
-  return launch_rows<32, MODE_FWD, 1>(c, "fm_dense_split_fwd", q, q, k, v, a);
+  const bool few = p.mask ? most > 1400 && tiles <= 370 : most > 2800 && tiles <= 400;
+  return tiles > 2 * 148 && !few &&
+         launch_registers(split_rows_kernel<32, MODE_FWD, 2>, &regs) >= SR<32, MODE_FWD, 2>::REGS;
+}
+int split_rows_forward(const Ctx& c, const void* q, const void* k, const void* v, const SplitArgs& a) {
+  if (c.p.d == 32) return launch_rows<32, MODE_FWD, 2>(c, "fm_dense_split_fwd", q, q, k, v, a);
+  return launch_rows<64, MODE_FWD, 1>(c, "fm_dense_split_fwd", q, q, k, v, a);
 }
 int split_rows_dq(const Ctx& c, const void* q, const void* gs, const void* k, const void* v, const SplitArgs& a) {
   if (c.p.d == 32) return launch_rows<32, MODE_DQ, 1>(c, "fm_dense_split_dq", q, gs, k, v, a);
