@@ -77,6 +77,35 @@ def test_unmasked_first_order_gradients_at_run_edges(bh, nq, nk, d, normalize):
                  floor=1e-9)
 
 
+def test_unmasked_first_order_gradients_over_long_runs():
+    """148 heads of 8192 tokens are one run each, so a state is one chain of 512 steps in the tensor core's accumulator, which
+    truncates: within 512 x 2^-23 of a sum of positive terms (6e-5), far below the bf16 copies that the read-outs multiply.  The
+    scaled upstream gradient, the copy and the result are each rounded once, 2^-9 at most: 2-norm error within 3 x 2^-9 (+ 6e-5),
+    against float64 sums of the inputs as they are."""
+    heads, n, d = 148, 8192, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, go = [torch.randn(heads, n, d, generator=g, device="cuda") for _ in range(4)]
+    q, k, v, go = (q.abs() / 8).bfloat16(), (k.abs() / 8).bfloat16(), v.bfloat16(), go.abs().bfloat16()
+    kw = dict(mask=False, normalize=False, p=1, a0=1.0, a1=0.9, a2=0.5, lim=1.0, impl="moments")
+    out, den, st = _cabi.forward(q, k, v, **kw)
+    _cabi.profile(True)
+    got = _cabi.backward(q, k, v, out, den, st, go, **kw)
+    names = [name for name, _ in _cabi.profile_records()]
+    _cabi.profile(False)
+    assert "fm_first_tc_grad" in names and _cabi.device_status() == 0
+    for h in (0, 77, 147):
+        Q, K, V, G = [t[h].double() for t in (q, k, v, go)]
+        dn = n + 0.9 * (Q @ K.sum(0))
+        o = (V.sum(0) + 0.9 * (Q @ (K.T @ V))) / dn[:, None]
+        gs = G / dn[:, None]
+        dv = (gs * o).sum(1)
+        want = (0.9 * (gs @ (V.T @ K) - dv[:, None] * K.sum(0)), 0.9 * (V @ (gs.T @ Q) - (dv[:, None] * Q).sum(0)),
+                gs.sum(0) + 0.9 * (K @ (Q.T @ gs)))
+        for name, x, r in zip(("dq", "dk", "dv"), got, want):
+            err = float((x[h].double() - r).norm() / r.norm())
+            assert err < 3 * 2.0 ** -9 + 6e-5, (h, name, err)
+
+
 @pytest.mark.parametrize("dtype,d,normalize", [(torch.float32, 32, True), (torch.bfloat16, 64, True),
                                                (torch.float32, 16, False)])
 def test_shard_stage_calls_reproduce_the_unsharded_result(dtype, d, normalize):
