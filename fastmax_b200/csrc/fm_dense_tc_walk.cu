@@ -505,7 +505,7 @@ walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
       const int first = (g ^ gp) & 1;              // the group's first column tile of this row tile
       const float A1 = it.A1, A2 = it.A2;
       const uint64_t A1v = pack2(A1, A1), A2v = pack2(A2, A2), A2d = pack2(2.f * A2, 2.f * A2);
-      const uint64_t Bv = pack2(a.sq.shift, a.sq.shift), Cv = pack2(a.sq.rest, a.sq.rest);
+      const uint64_t Bv = a.sq.shift, Cv = a.sq.rest;
       const int row = it.r0 + rl;
       int limcol = a.ncols - 1, lowcol = 0;        // columns kept for this row: lowcol <= col <= limcol
       if (a.mask) {

@@ -347,7 +347,7 @@ dense_tc_wide_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     using coef_t = typename std::conditional<GQ, uint64_t, const uint64_t>::type;   // fixed unless heads are grouped
     coef_t A1v = pack2(A1, A1), A2v = pack2(A2, A2), A2d = pack2(2.f * A2, 2.f * A2);
     const float root = a.sq.root * c;
-    const uint64_t Rv = pack2(root, root), Bv = pack2(a.sq.shift, a.sq.shift), Cv = pack2(a.sq.rest, a.sq.rest);
+    const uint64_t Rv = pack2(root, root), Bv = a.sq.shift, Cv = a.sq.rest;
     int limcol = a.ncols - 1, lowcol = 0;   // columns kept for this row: lowcol <= col <= limcol
     if (a.mask) {
       if (rev) lowcol = row - a.off;

@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cmath>
+#include <cstdint>
+#include <cstring>
 
 #include "fm_common.cuh"
 
@@ -11,9 +13,13 @@ namespace fm {
 // pair of scores costs t = fma(s, root c, shift), P = fma(t, t, rest), E' = t (w - dvec): four packed operations where the
 // polynomial and its derivative cost five.  P is what is multiplied, so it is rounded to bf16 where f lies; 2 root c multiplies
 // grad_k's accumulator in the end.  (With a2 c^2 left out of P as well, it was rounded where f / (a2 c^2) lies: the error of
-// grad_v was 2.75e-3 to 3.07e-3, by the mantissa of a2 c^2, instead of 2.75e-3.)
+// grad_v was 2.75e-3 to 3.07e-3, by the mantissa of a2 c^2, instead of 2.75e-3, and
+// inputs 1e10 apart overflowed.  Then t is an addition: the wide kernel took 60.0 us instead of 62.3 for 168 row tiles of 3500
+// unmasked columns, 154 / 154 for 1176 causal ones, 252.7 / 249.7 for 1176 unmasked ones.)
+// shift and rest stand twice in 64 bits, as packed operations take them from a kernel's parameters, without a register.
 struct Square {
-  float root, shift, rest;
+  uint64_t shift, rest;
+  float root;
 };
 
 // Whether t^2 and the rest cancel by less than a factor of 16 (four of float32's 24 bits), which does not depend on the scale: a2 has
@@ -24,7 +30,13 @@ inline bool square_form(float a0, float a1, float a2, Square* sq) {
   const double b = a1, a = a2, lift = b * b / (4.0 * a);
   if (!(a > 0.0) || !(lift <= 16.0 * std::fabs((double)a0)) || !std::isfinite(a) || !std::isfinite(a0)) return false;
   const double root = std::sqrt(a);
-  *sq = {(float)root, (float)(b / (2.0 * root)), (float)(a0 - lift)};
+  const auto twice = [](double x) {
+    const float f = (float)x;
+    uint32_t bits;
+    std::memcpy(&bits, &f, sizeof bits);
+    return (uint64_t)bits << 32 | bits;
+  };
+  *sq = {twice(b / (2.0 * root)), twice(a0 - lift), (float)root};
   return true;
 }
 
