@@ -483,11 +483,12 @@ short_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
 // Whether the forward, whose registers and shared memory leave room for a third CTA on an SM, is to run with two.  The third
 // one waits for the tensor memory of a CTA of its own SM, so its start is covered, but it is bound to that SM, which evens
 // out over many row tiles only.  us, two / three: 322 row tiles of 800 causal columns 13.4 / 15.4, 357 14.9 / 16.6, 600 of 3000 8 %
-// slower, 720 1 % faster, 2048 of 450 52.4 / 49.4; rows of 150 columns 303 to 600 row tiles 7 to 11 % faster.
+// slower, 720 1 % faster, 2048 of 450 52.4 / 49.4; causal rows of 300 columns and unmasked ones of 300 5 %
+// faster at 300 to 600.
 constexpr int kTwoFit = 80 * 1024;
 bool two_ctas(long long tiles, int ncols, const ShortArgs& a) {
   const int seen = a.chunk > 0 ? a.chunk / 2 : (a.mask ? ncols / 2 : ncols);
-  return tiles <= 666 && seen > 160;
+  return tiles <= 666 && seen > (a.mask ? 160 : 320);
 }
 
 template <int MODE>

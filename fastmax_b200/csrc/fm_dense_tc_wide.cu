@@ -632,11 +632,17 @@ bool dense_tc_wide_supports(const fastmax_problem& p) {
 // epilogues read fp32 rows too (of which chunks of grad_q and of grouped heads are left; walk_rows takes the others).
 // So the line is drawn at the mean number of columns a row tile walks.  With no more row tiles than SMs there is nothing
 // to overlap and the wide kernels' larger tiles win (8 heads of 1024: 16.3 / 12.4).
+//   Causal rows of two rounds of row tiles leave the second one to the short ones, so there is little to overlap either: forward, short /
+// wide, 14.2 / 10.6 at 160 row tiles of 1000 columns, 15.8 / 13.5 at 288, 11.3 / 10.3 and 12.3 / 12.5 of 700, 16.6 / 10.6 and 20.5 / 15.3 of
+// 1500; grad_k + grad_v 20.8 / 11.7 and 22.0 / 17.6 of 700, 29.1 / 16.5 and 33.6 / 22.4 of 1300, and with a few row tiles more (320) 20.1 /
+// 20.8 of 700, 24.7 / 23.4 of 900, 28.3 / 26.2 of 1100.
 static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
   const bool chunked = ca && ca->chunk > 0;
   const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
-  if ((long long)(pass == 2 ? p.bhkv : p.bh) * ((rows + BM - 1) / BM) <= 148) return false;
+  const long long tiles = (long long)(pass == 2 ? p.bhkv : p.bh) * ((rows + BM - 1) / BM);
+  if (tiles <= 148) return false;
   const int seen = chunked ? ca->chunk / 2 : (p.mask ? cols / 2 : cols);
+  if (p.mask && !chunked && p.bh == p.bhkv && pass != 1 && tiles <= (pass == 2 && seen >= 450 ? 320 : 2 * 148) && seen >= 300) return false;
   const int most[3] = {1500, 1900, chunked ? 1100 : (p.mask ? 700 : 1300)};
   return seen * (pass == 2 ? p.bh / p.bhkv : 1) <= most[pass];
 }
@@ -648,15 +654,15 @@ static bool short_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
 //   chunks        second order: forward 0.70 to 0.99 from 300 row tiles on, 1.00 at 200; chunks of 4096 0.76 to 0.95.  grad_k + grad_v
 //                 0.63 to 0.97 up to chunks of 2048, 0.87 to 1.04 for 3072, 0.97 to 1.23 for 4096.  First order (grad_k + grad_v only):
 //                 chunks of 512 0.86 to 0.99, but 1.09 at 300 row tiles; of 256 0.94 to 1.08
-//   forward       causal, up to two rounds of row tiles: 0.90 to 1.01 at 600 columns, 0.79 to 0.92 at 1000, 0.58 to 0.69 at 3000, 1.02 to
-//                 1.13 at 3800.  Up to four: 1.00 to 1.11 at 800 to 1300 columns, 0.92 to 1.00 from 1900 on.  More: 0.94 to 1.05 (others
-//                 0.92 to 0.96) at 600, 0.86 to 1.00 at 1000, 0.79 to 0.93 from 1900 on, 0.96 to 1.04 at 5200.
-//                 Unmasked: 1.00 to 1.24 up to 400 columns and at any number within two rounds; 0.92 to 1.04 at 650 and 800 below
-//                 eight rounds, 0.91 to 0.98 above; 0.82 to 0.98 from 1000 on
-//   grad_k+grad_v causal, up to two rounds: 0.75 to 0.92 at 600 columns, 0.71 to 0.84 at 1000, 1.06 to 1.22 at 1900; with a third
-//                 one 1.09 at 600, 1.03 at 1000.  Unmasked: 0.80 to 1.00 at 300 to 1300 columns, 1.03 to 1.25 from 1600 on; without
-//                 normalisation (whose dots the short kernel waits for) 1.00 to 1.07 in four rounds, where the short kernel's two CTAs
-//                 have two full ones
+//   forward       causal, up to two rounds of row tiles: 0.98 to 1.17.  Of 300 to 320: 1.07 to 1.10 at 700 to 1100 columns, 1.00 at 1300
+//                 and 1500, 0.85 at 2100.  Up to four rounds: 1.00 to 1.11 at 800 to 1300, 0.92 to 1.00 from 1900 on.  More: 0.94 to
+//                 1.05 (others 0.92 to 0.96) at 600, 0.86 to 1.00 at 1000, 0.79 to 0.93 from 1900 on, 0.96 to 1.04 at 5200.
+//                 Unmasked, two rounds: 1.00 at any number.  Three: 0.95 to 1.01 at 450 columns, 0.93 to 0.98 at 500 to 800, 0.82 to
+//                 0.98 from 1000 on; four (whose two full ones the short kernel's two CTAs have) 1.06 to 1.09, 1.00 to 1.05, 0.91 to
+//                 0.95; five and more 0.92 to 1.05, 0.87 to 0.96, 0.80 to 0.92
+//   grad_k+grad_v causal 1.02 to 1.23 up to 320 row tiles of 700 to 1500 columns, and above.  Unmasked: 0.80 to 1.00 at 300 to 1300
+//                 columns, 1.03 to 1.25 from 1600 on; without normalisation (whose dots the short kernel waits for) 1.00 to 1.07 in
+//                 four rounds
 static bool walk_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
   const int rows = pass == 2 ? p.nk : p.nq, cols = pass == 2 ? p.nq : p.nk;
   const long long tiles = (long long)p.bh * ((rows + BM - 1) / BM), rounds = (tiles + 147) / 148;
@@ -666,14 +672,13 @@ static bool walk_rows(const fastmax_problem& p, const ChunkAdd* ca, int pass) {
     return rounds > 2 && ca->chunk <= (pass == 2 ? 2048 : 4096);
   }
   const int seen = p.mask ? cols / 2 : cols;
+  if (rounds <= 2) return false;
   if (!p.mask) {
-    if (rounds <= 2) return false;
-    if (pass == 0) return seen >= (rounds > 8 ? 600 : 900) && seen <= 3000;
+    if (pass == 0) return seen >= (rounds == 4 ? 900 : 500) && seen <= 3000;
     return seen >= 300 && seen <= 1300 && (p.normalize || rounds % 2 == 1 || rounds > 6);
   }
-  // (a few row tiles more from 500 columns on: 0.92 to 1.05 there, and 20 and 40 heads of 1000 then give the same bits)
-  if (rounds <= 2 || (tiles <= 320 && seen >= 500)) return seen >= 300 && seen <= (pass == 2 ? 550 : 1500);
-  return pass == 0 && seen >= (rounds <= 4 ? 950 : 500) && seen <= 1900;
+  // (up to 320 from 500 columns on: 20 heads of 1000 in the wide kernel and 40 here then give the same bits)
+  return pass == 0 && seen >= (tiles > 320 && rounds <= 4 ? 950 : 500) && seen <= (tiles <= 320 ? 1500 : 1900);
 }
 static walk::WalkArgs walk_args(const fastmax_problem& p, const stat_t* stats, const ChunkAdd* ca) {
   walk::WalkArgs a = {};
