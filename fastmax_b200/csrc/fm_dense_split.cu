@@ -597,6 +597,7 @@ int dense_split_backward(const Ctx& c, const void* q, const void* k, const void*
   a.x = (const float*)q;
   a.dots = p.normalize ? dots : nullptr;
   if (split_rows_serve(p, MODE_DQ, a.chunk)) rc = split_rows_dq(c, q3, g3, k3, v3, a);
+  else if (p.d == 32) rc = launch_tiles<32, MODE_DQ>(c, "fm_dense_split_dq", q3, g3, k3, v3, a);
   else rc = launch_tiles<64, MODE_DQ>(c, "fm_dense_split_dq", q3, g3, k3, v3, a);
   if (rc) return rc;
   a.o1 = (float*)grad_k;

@@ -439,21 +439,30 @@ int launch_rows(const Ctx& c, const char* name, const void* x, const void* u, co
 
 // Which problems' forward (MODE_FWD) and grad_q (MODE_DQ) walk row tiles; fm_dense_split.cu has a CTA per row tile for the others.
 // Measured, walk as part of that:
-//   d = 32  forward (two CTAs per SM; one walking is 0 to 10 % slower than none): causal 0.78 to 0.93 from 300 row tiles of up to 1000
-//           columns on, but with 2100 to 4000 columns 1.08 to 1.12 at 310 row tiles, 1.00 to 1.04 at 340, 0.92 to 0.98 from 370
-//           on; up to 296 1.1 to 1.6.  Unmasked 0.75 to 1.00 from 300 on, 1.03 to 1.04 for 350 to 380 of 4000.  grad_q 0.80 to 1.00
-//           everywhere
-//   d = 64  forward 0.97 to 1.06 up to 296 row tiles, 0.84 to 1.01 above.  grad_q 1.00 to 1.07 up to 296, 0.82 to 1.01 above, but 1.00
-//           to 1.04 (unmasked, 3000 columns and more)
+//   d = 32  forward (two CTAs per SM; one walking is 0 to 10 % slower than none): up to 148 row tiles 1.10 to 1.26.  Causal, up to 296: 0.76
+//           to 0.99 of 128 to 300 columns, 1.03 to 1.16 of 384, 1.06 to 1.33 of 474, 1.1 to 1.7 above.  From 300 on 0.78 to 0.93 of up
+//           to 1000 columns, but with 2100 to 4000 1.08 to 1.12 at 310 row tiles, 1.00 to 1.04 at 340, 0.92 to 0.98 from 370 on.
+//           Unmasked 0.75 to 1.00, but 1.03 to 1.04 for 350 to 380 row tiles of 4000.
+//           grad_q: up to 148 1.06 to 1.14 of 128 to 384 columns, 1.01 to 1.04 of 474 to 1000, 0.95 of 2000; above 0.77 to 1.03
+//   d = 64  up to 148 row tiles 1.03 to 1.07.  Up to 296, causal: forward 0.88 to 0.98, grad_q 0.89 to 0.99 at 200 to 296 row tiles of 212
+//           and 474 columns; of 1000 columns 1.03 at 200, 0.95 to 0.97 from 224 on; of 2000 1.05 and 1.03 at 224, 0.99 to 1.00 from 256
+//           on; 160 row tiles 0.88 and 0.93 of 212 columns, 1.00 and 1.04 of 474, 1.07 and 1.04 of 1000.  Unmasked: forward 0.90 to
+//           0.96 of 212 and 474, 0.97 to 0.98 of 1000, 1.00 to 1.02 of 2000; grad_q 0.92 to 0.99, 0.99 to 1.01, 1.02 to 1.05.  Above 296
+//           0.84 to 1.01, but grad_q 1.00 to 1.04 unmasked, 3000 columns and more
 bool split_rows_serve(const fastmax_problem& p, int mode, int chunk) {
   const long long tiles = (long long)p.bh * ((p.nq + BM - 1) / BM);
   const int most = chunk > 0 ? chunk : p.nk;         // columns of the longest row
-  if (p.d == 32 && mode == MODE_DQ) return true;
-  if (p.d == 64) return tiles > 2 * 148 && (mode == MODE_FWD || (p.mask ? most / 2 : most) <= 2000);
+  if (p.d == 32 && mode == MODE_DQ) return tiles > 148 || most > 1000;
+  if (p.d == 64) {
+    const int seen = p.mask ? most / 2 : most;       // mean columns of a row tile
+    if (tiles > 2 * 148) return mode == MODE_FWD || seen <= 2000;
+    return tiles > 148 && (p.mask ? 8 * (tiles - 148) >= seen : seen <= (mode == MODE_FWD ? 1000 : 500));
+  }
   // the compute warps of two CTAs wait for registers that the block must have been launched with
   static std::atomic<int> regs{0};
-  const bool few = p.mask ? most > 1400 && tiles <= 370 : most > 2800 && tiles <= 400;
-  return tiles > 2 * 148 && !few &&
+  const bool second = tiles <= 2 * 148;
+  const bool few = p.mask ? (second ? most > 320 : most > 1400 && tiles <= 370) : !second && most > 2800 && tiles <= 400;
+  return tiles > 148 && !few &&
          launch_registers(split_rows_kernel<32, MODE_FWD, 2>, &regs) >= SR<32, MODE_FWD, 2>::REGS;
 }
 int split_rows_forward(const Ctx& c, const void* q, const void* k, const void* v, const SplitArgs& a) {
