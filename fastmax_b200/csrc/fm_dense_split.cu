@@ -28,7 +28,7 @@
 // waits are bounded.
 //
 // Measured (B200, forward / grad_q / grad_k + grad_v, ms; the CUDA-core family on the same inputs in brackets):
-//   512 heads x 1000 causal, d = 32:   0.22 / 0.29 / 0.53  (1.40 / 2.00 / 2.45)
+//   512 heads x 1000 causal, d = 32:   0.22 / 0.29 / 0.53  (1.40 / 2.00 / 2.45); one after another in a step 0.24 / 0.29 / 0.54
 //    64 heads x 4000 unmasked, d = 64: 1.07 / 1.81 / 3.05  (7.96 / 11.7 / 15.6)
 // Error against float64 (2-norm, outputs and gradients): 0.8-3.7e-7 for 64 to 10 000 tokens where the CUDA-core
 // family has 0.9e-7 to 2.4e-6.  What bounds grad_k + grad_v: the chain of hand-offs per 64-column tile (scores -> registers ->

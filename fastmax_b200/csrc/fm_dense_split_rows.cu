@@ -13,7 +13,8 @@
 // products.  S and W are refilled as soon as they are in registers.  The forward at d = 32 needs so little that two CTAs
 // share an SM, and one's chain from scores to sums runs under the other's.  All waits are bounded.
 //
-// Measured (B200, us, a CTA per row tile / now): 512 heads x 1000 causal, d = 32: forward 303 / 220, grad_q 370 / 295; 60 heads x
+// Measured (B200, us, a CTA per row tile / now): 512 heads x 1000 causal, d = 32: forward 303 / 220 (after the
+// operands' preparation, as in a step, 304 / 241), grad_q 370 / 290; 60 heads x
 // 4000 unmasked, d = 32: 687 / 605, 815 / 735; 64 heads x 1000 causal, d = 64: 60 / 54, 97 / 89.  What bounds it: tensor pipe
 // and CUDA cores (ALU) are each busy for half of the time (forward at d = 32: 780 and 620 of 1 400 cycles a tile).
 #include "fm_dense_split.cuh"

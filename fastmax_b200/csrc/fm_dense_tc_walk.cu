@@ -8,7 +8,7 @@
 // tile are loaded meanwhile, its first scores follow the last ones of this, the float32 rows that a chunk adds to its result come
 // by TMA while the columns pass, and the forward, which has room for two row tiles' accumulators, reads and stores a row tile's
 // result when the next one's columns are done.  32 heads of 32768 in chunks of 2048, us, short-row kernels / this: forward
-// 469 / 361, grad_k + grad_v 874 / 787; 240 heads of 2000, causal: forward 208 / 176.  A second buffer for the row operands and
+// 468 / 356, grad_k + grad_v 871 / 758; 240 heads of 2000, causal: forward 200 / 161.  A second buffer for the row operands and
 // shorter rings pay in the forward (32 heads of 16384 in chunks of 2048 189 / 181, 160 heads of 1600 86 / 83) and not in DKDV
 // (387 / 394).  What bounds it is the loop: TMEM loads,
 // polynomial and TMEM stores of sixteen warps.  grad_q the same way was slower than its short kernel (0.78 to 0.98 of it):
