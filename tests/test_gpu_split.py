@@ -120,7 +120,8 @@ def test_no_room_for_the_operand_parts(p):
                                                (75, 513, 32, 0, 0), (160, 1000, 64, 1, 0), (330, 520, 64, 1, 0), (60, 650, 64, 0, 0),
                                                (150, 1100, 32, 1, 256), (600, 600, 32, 1, 256), (40, 900, 64, 1, 256), (16, 1281, 64, 1, 512),
                                                (30, 500, 64, 1, 512), (370, 500, 64, 1, 0), (370, 512, 32, 1, 0), (740, 512, 32, 1, 0),
-                                               (30, 1500, 32, 1, 0), (34, 1000, 64, 1, 0), (20, 2100, 64, 0, 0)])
+                                               (30, 1500, 32, 1, 0), (34, 1000, 64, 1, 0), (20, 2100, 64, 0, 0),
+                                               (80, 212, 32, 0, 0), (80, 212, 32, 1, 0), (37, 1000, 32, 0, 0), (80, 212, 64, 1, 0), (72, 474, 64, 0, 0)])
 def test_row_walks_match_the_cuda_cores(bh, n, d, mask, chunk):
     """Several row tiles to a CTA, in every order they are taken in: head by head, tile by tile, in pairs (even and odd
     numbers of tiles).  Both families' bounds against float64 add up to 2e-5 of the largest value at these lengths."""
